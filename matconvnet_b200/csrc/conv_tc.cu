@@ -121,7 +121,20 @@ struct Params {
   int smemSum;            // conv_ts_kernel, kMode 0 / 1: keep the running sum of a tile in shared memory even for the tile widths that fit the
                           // drain warps' registers (tiles of a few k-blocks, where the stores dominate; test switch bit 3)
   int plane;              // row mode: reduction indices per image in the tile images -- the plane's pixels rounded up to whole k-blocks
+  // conv_ts_gen_kernel (general gather).  The reduction runs over units of `unit` channels of one filter tap, upk = 32 / unit of
+  // them per k-block: unit number = tap + taps * (channel / unit).  Column tile nt belongs to filter group nt / tilesPerGroup;
+  // a group has `cols` columns and reads a.C channels, aGroup elements further on.  Row (i, j) of an image is the output pixel
+  // (oy + oys * i, ox + oxs * j) of a plane of outH x outW.  shufY > 0: column n of a group is channel n / (shufY * shufX) at the
+  // output pixel moved by (n % shufY, n / shufY % shufX), outC channels per group.  ctaBeg, ctas: the CTAs that walk this problem.
+  int unit, upk, tilesPerGroup, cols;
+  int groups;             // tc_gemm_kernel, filter gradient: filter groups (0 counts as one), M rows and N columns each
+  long long aGroup;
+  int oy, ox, oys, oxs, outH, outW, shufY, shufX, outC, ctaBeg, ctas;
 };
+
+// Several contractions in one launch of conv_ts_gen_kernel (the residue classes of a strided data gradient), each with CTAs of its own.
+constexpr int kMaxTsProblems = 16;
+struct TsProblems { int n; Params p[kMaxTsProblems]; };
 
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(void const* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -513,7 +526,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
   uint32_t const tmemCols = kSplit ? (uint32_t)(4 * BN) : (BN < 32 ? 32u : (uint32_t)BN);
 
   int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int const m0 = blockIdx.x * BM, n0 = blockIdx.y * BN, split = blockIdx.z;
+  // filter groups (WGATHER): gridDim.x = groups x row tiles of a group
+  int const fgrp = kAMode == OP_WGATHER ? (int)blockIdx.x / p.tilesM : 0;
+  int const m0 = ((int)blockIdx.x - fgrp * p.tilesM) * BM, n0 = blockIdx.y * BN, split = blockIdx.z;
   int const kbBeg = split * p.kbPerSplit;
   int const kbEnd = min(p.numKb, kbBeg + p.kbPerSplit);
   int const numIter = max(kbEnd - kbBeg, 0);
@@ -534,7 +549,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
   }
   if (kAMode == OP_WGATHER && p.pipelined && threadIdx.x < BM) {
     TapCtx tc = tap_ctx(p.a, m0 + (int)threadIdx.x);
-    tapTab[threadIdx.x] = make_int4((int)tc.coff + tc.dw * p.a.H + tc.dh, tc.dh, tc.dw, tc.valid ? 1 : 0);
+    tapTab[threadIdx.x] = make_int4((int)(tc.coff + fgrp * p.aGroup) + tc.dw * p.a.H + tc.dh, tc.dh, tc.dw, tc.valid ? 1 : 0);
   }
   tc_fence_before();
   __syncthreads();
@@ -813,7 +828,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
         if (tg == 0) {
           mbar_expect_tx(smem_u32(&fullBar[s]), bBytes);
           bulk_copy_g2s(smem_u32(base + (kSplit ? 2u : 1u) * aTileBytes),
-                        p.bTiles + ((size_t)blockIdx.y * p.numKb + (size_t)(kbBeg + it)) * (bBytes / 4), bBytes, smem_u32(&fullBar[s]));
+                        p.bTiles + (((size_t)fgrp * gridDim.y + blockIdx.y) * p.numKb + (size_t)(kbBeg + it)) * (bBytes / 4), bBytes, smem_u32(&fullBar[s]));
         }
 #pragma unroll
         for (int j = 0; j < CHG; ++j) {
@@ -919,7 +934,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
       int const m = m0 + quarter * 32 + lane;
       long long rowBase = 0;
       if (kEpi == EPI_CONV) { int pix = m % p.e.P, img = m / p.e.P; rowBase = (long long)img * p.e.Ktot * p.e.P + pix; }
-      else rowBase = m + (long long)split * p.e.splitStride;
+      else rowBase = m + (long long)split * p.e.splitStride + (long long)fgrp * p.N * p.e.ldd;      // (groups: p.N columns each)
       uint32_t const lastT = (uint32_t)(((numChunks - 1) & 1) * BN);
       for (int c0 = 16 * rank; c0 < BN; c0 += 16 * group) {
         uint32_t const laneBase = tmemAcc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
@@ -1063,11 +1078,23 @@ __device__ __forceinline__ float lds32(uint32_t addr)
 // Where row `row` (0..127, = TMEM lane) of row tile `tm` lies in the output: image, pixel ho + Ho*wo, and whether it exists.
 // Linear mode: the tile is 128 consecutive output pixels (ho fastest, images following one another).  Box mode (p.tma):
 // the tile is a box of bh x bw pixels of one image, row = dh + bh*dw.
-struct RowPos { int img, pix, split; bool valid; };
+struct RowPos { int img, pix, split; bool valid; int h, w; };
 
+template <bool kGen>
 __device__ __forceinline__ RowPos row_pos(Params const& p, int tm, int row)
 {
   RowPos r;
+  r.h = r.w = 0;
+  if (kGen) {
+    r.split = tm / p.tilesM; tm -= r.split * p.tilesM;
+    int const m = tm * BM + row;
+    r.valid = m < p.M;
+    int const mm = min(m, p.M - 1), t = mm / p.a.Ho;
+    r.img = t / p.a.Wo;
+    r.h = p.oy + p.oys * (mm - t * p.a.Ho); r.w = p.ox + p.oxs * (t - r.img * p.a.Wo);
+    r.pix = r.h + p.outH * r.w;
+    return r;
+  }
   if (p.wg) {
     // tm = row tile + tilesM * reduction range; row tile = tap group + tapGroups * channel block; row = local tap * cPer + channel.
     // The "pixel" is the element of dF the row belongs to, fh + FH*(fw + FW*c), plus the offset of the range's partial result.
@@ -1095,19 +1122,56 @@ __device__ __forceinline__ RowPos row_pos(Params const& p, int tm, int row)
   return r;
 }
 
+// The columns of column tile nt: the first one among the output's columns, and how many of the tile's columns exist.
+struct TileCols { int n0, cnt, grp; };
+
+template <bool kGen>
+__device__ __forceinline__ TileCols tile_cols(Params const& p, int nt)
+{
+  TileCols c;
+  if (kGen) {
+    c.grp = nt / p.tilesPerGroup;
+    int const local = (nt - c.grp * p.tilesPerGroup) * p.BN;
+    c.n0 = c.grp * p.cols + local; c.cnt = min(p.BN, p.cols - local);
+  } else {
+    c.grp = 0; c.n0 = nt * p.BN; c.cnt = min(p.BN, p.N - c.n0);
+  }
+  return c;
+}
+
 // Epilogue of conv_ts_kernel: the finished tile sits in shared memory, P[column][row]; this warp stores the rows of its
 // TMEM lane quarter for the columns rank, rank + nranks, ...: out[(image*Ktot + n)*P + pixel] = inMult*acc + bias[n] + outMult*old.
 // P holds the columns cBeg .. cBeg + cCnt - 1 of the tile (cCnt = BN: all of it).
-__device__ __forceinline__ void ts_store_tile(Params const& p, float const* P, int quarter, int lane, int rank, int nranks, int tm, int n0,
+template <bool kGen>
+__device__ __forceinline__ void ts_store_tile(Params const& p, float const* P, int quarter, int lane, int rank, int nranks, int tm, TileCols const& tc,
                                               uint32_t const* maskBits = nullptr, int cBeg = 0, int cCnt = 1 << 20)
 {
-  int const row = quarter * 32 + lane;
-  RowPos const rp = row_pos(p, tm, row);
+  int const row = quarter * 32 + lane, n0 = tc.n0;
+  RowPos const rp = row_pos<kGen>(p, tm, row);
   if (!rp.valid) return;
   int const pix = rp.pix, img = rp.img;
   float* const dst0 = p.e.out + ((long long)rp.split * p.e.splitStride + (long long)img * p.e.Ktot * p.e.P + pix);
-  int const nEnd = min(min(p.BN, cBeg + cCnt), p.N - n0);
+  int const nEnd = min(cBeg + cCnt, tc.cnt);
   P -= (size_t)cBeg * BM;                              // column c of the tile sits at P[(c - cBeg) * BM + row]
+  if (kGen && p.shufY > 0) {
+    // column n = moved by (ry, rx), channel c: the pixel is (h + ry, w + rx) where that lies inside the plane
+    int const first = n0 - tc.grp * p.cols + cBeg + rank, per = p.shufY * p.shufX;
+    int c = first / per, ry = (first - c * per) % p.shufY, rx = (first - c * per) / p.shufY;
+    long long const plane = ((long long)img * p.e.Ktot + tc.grp * p.outC) * p.e.P;
+    float* const out = p.e.out + (long long)rp.split * p.e.splitStride;
+    for (int k = cBeg + rank; k < nEnd; k += nranks) {
+      int const h = rp.h + ry, w = rp.w + rx;
+      if ((unsigned)h < (unsigned)p.outH && (unsigned)w < (unsigned)p.outW) {
+        long long const at = plane + (long long)c * p.e.P + (h + (long long)p.outH * w);
+        float o = P[k * BM + row] + (p.e.bias ? p.e.bias[tc.grp * p.outC + c] : 0.f);
+        if (p.e.mask && !(__ldg(p.e.mask + at) > 0.f)) o = 0.f;
+        out[at] = o;
+      }
+      for (int s = 0; s < nranks; ++s)
+        if (++ry == p.shufY) { ry = 0; if (++rx == p.shufX) { rx = 0; ++c; } }
+    }
+    return;
+  }
   if (maskBits) {
     // the mask of this row was fetched while the tile was being computed: bit c = the mask is positive in column c
     uint32_t const b0 = maskBits[0], b1 = maskBits[1], b2 = maskBits[2], b3 = maskBits[3];
@@ -1177,6 +1241,7 @@ constexpr int kTsXStages = 6;                           // at most
 // was tried first: with six filter stages and four A stages the loader fell a whole phase behind on conv1_2 at batch 64 and then
 // waited for a completion that needed its own copies -- the bounded wait ran out.)
 constexpr int kTsDoneRing = 8;
+constexpr int kMaxGenTaps = 128;                        // of the general gather (11 x 11 filters)
 static_assert(kTsBStages < kTsDoneRing, "the loader must not be able to fall a whole ring behind");
 
 // Registers (kMode 0, 1): 128 per thread at launch (512 threads: the whole register file, one CTA per SM); then the warps 4-7
@@ -1190,15 +1255,17 @@ static_assert(kTsBStages < kTsDoneRing, "the loader must not be able to fall a w
 // bound by shared-memory bandwidth (per k-block about 150 KB of tile copies, operand reads by the tensor core, runs read by the
 // producers and 32 KB of running sum read and rewritten, against 128 bytes per clock).
 // kNarrow: tiles of 64 columns or fewer (kMode 0, 1), which get more accumulators and A stages (below).
-template <bool kSplit, int kMode, bool kNarrow>
-__global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) conv_ts_kernel(Params p, const __grid_constant__ CUtensorMap xmap)
+// kGen: the general gather (below) instead of the one that needs whole blocks of 32 channels.  cta, ctas: this CTA's place among
+// those that walk the problem's tiles.
+template <bool kSplit, int kMode, bool kNarrow, bool kGen>
+__device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const* xmap, int const cta, int const ctas)
 {
   constexpr bool kTma = kMode == 1, kWg = kMode == 2;
   extern __shared__ uint8_t smemRaw[];
   __shared__ __align__(8) uint64_t fullA[4], doneK[kTsDoneRing], fullB[kTsBStages], emptyB[kTsBStages];
   __shared__ __align__(8) uint64_t tFull[4], tFree[4], tileDone, turn[2], fullX[kTsXStages], emptyX[kTsXStages];
   __shared__ uint32_t tmemBase;
-  __shared__ int2 tapLut[64];       // per filter tap fh + FH*fw: {element offset of the tap (in the input window when kTma), fh | fw << 5}
+  __shared__ int2 tapLut[kGen ? kMaxGenTaps : 64];       // per filter tap fh + FH*fw: {element offset of the tap (in the input window when kTma), fh | fw << 5}
 
   uint8_t* smem = smemRaw + ((1024u - (smem_u32(smemRaw) & 1023u)) & 1023u);
   int const BN = p.BN;
@@ -1231,9 +1298,9 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
   int const numIter = p.kbPerSplit;                      // k-blocks per tile (work item: one range of the reduction of one output tile)
   int const chunksPerTile = kSplit ? (numIter + kTsDrainEvery - 1) / kTsDrainEvery : 1;
   int const numTiles = p.tilesM * p.tilesN * p.splits;
-  // this CTA's tiles: blockIdx.x, blockIdx.x + gridDim.x, ...; tile t = (row tile t / tilesN, column tile t % tilesN)
-  int const myTiles = (int)blockIdx.x < numTiles ? (numTiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  bool const singleTile = (int)gridDim.x == numTiles;      // launched with one CTA per tile (long reductions)
+  // this CTA's tiles: cta, cta + ctas, ...; tile t = (row tile t / tilesN, column tile t % tilesN)
+  int const myTiles = cta < numTiles ? (numTiles - 1 - cta) / ctas + 1 : 0;
+  bool const singleTile = ctas == numTiles;      // launched with one CTA per tile (long reductions)
 
   if (threadIdx.x == 0) {
     // an A stage is full when its four producer warps and the forwarder (filter tile landed) have arrived
@@ -1271,15 +1338,17 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
     asm volatile("setmaxnreg.inc.sync.aligned.u32 200;" ::: "memory");
     uint32_t const lanes = tmemAcc + ((uint32_t)(warp * 32) << 16);
     float* const Prow = Psm + warp * 32 + lane;       // this thread's row of P: Prow[column * BM]
-    bool const preMask = p.e.mask != nullptr && !singleTile;
+    bool const preMask = p.e.mask != nullptr && !singleTile && !(kGen && p.shufY > 0);
     auto drain = [&](auto kRegsTag) {
       constexpr int kRegs = decltype(kRegsTag)::value;          // columns of the running sum held in registers (0: none, shared memory)
       float Pr[kRegs > 0 ? kRegs : 1];
       int g = 0;                                        // chains in the order they are drained, over the CTA's life: chain g sits in T[g % 3]
       bool ok = true;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
-        int const tile = (int)blockIdx.x + ts * (int)gridDim.x;
-        int const tm = tile / p.tilesN, n0 = (tile % p.tilesN) * BN;
+        int const tile = cta + ts * ctas;
+        int const tm = tile / p.tilesN;
+        TileCols const tc = tile_cols<kGen>(p, tile - tm * p.tilesN);
+        int const n0 = tc.n0;
         int const chainsF = ts_chains<kSplit>(numIter, 0), chainsS = ts_chains<kSplit>(numIter, 1);   // of the issuer that owns the tile's first k-block, of the other
         bool fresh = true;                              // P holds nothing of this tile yet
         if (kRegs > 0) {
@@ -1289,10 +1358,10 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
         // ReLU mask of this thread's output row (persistent mode): sixteen columns are fetched before each of the tile's
         // first chain waits, so that their latency passes while the chain is being computed, and kept as one bit each
         uint32_t mbits[4] = {0u, 0u, 0u, 0u};
-        int const nEndT = min(BN, p.N - n0);
+        int const nEndT = tc.cnt;
         float const* mkRow = p.e.mask;
         if (preMask) {
-          RowPos const rp = row_pos(p, tm, warp * 32 + lane);     // a row that does not exist reads (and discards) the mask of a pixel that does
+          RowPos const rp = row_pos<kGen>(p, tm, warp * 32 + lane);     // a row that does not exist reads (and discards) the mask of a pixel that does
           mkRow += ((long long)rp.img * p.e.Ktot + n0) * p.e.P + rp.pix;      // (a masked data gradient is never cut into ranges)
         }
         int lc = 0;                                     // batches of sixteen mask columns fetched so far
@@ -1371,18 +1440,18 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
             if (c0 < nEndT) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) Prow[j * BM] = Pr[c0 + j];
-              ts_store_tile(p, Psm, warp, lane, 0, 1, tm, n0, preMask ? mbits : nullptr, c0, 32);
+              ts_store_tile<kGen>(p, Psm, warp, lane, 0, 1, tm, tc, preMask ? mbits : nullptr, c0, 32);
             }
           }
         } else if (singleTile) {
           // one tile per CTA: the producers have nothing left to do and share the stores
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&tileDone));
-          ts_store_tile(p, Psm, warp, lane, 0, 1 + kTsGroups, tm, n0);
+          ts_store_tile<kGen>(p, Psm, warp, lane, 0, 1 + kTsGroups, tm, tc);
         } else {
           // the tile is complete in P: store it while the tensor core works on the next tile (its chains wait in
           // their T buffers until this is through)
-          ts_store_tile(p, Psm, warp, lane, 0, 1, tm, n0, preMask ? mbits : nullptr);
+          ts_store_tile<kGen>(p, Psm, warp, lane, 0, 1, tm, tc, preMask ? mbits : nullptr);
         }
       }
     };
@@ -1497,7 +1566,7 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
       bool ok = true;
       long long gk = 0;                                  // k-blocks numbered over the CTA's life
       for (int ts = 0; ts < myTiles && ok; ++ts) {
-        int const tile = (int)blockIdx.x + ts * (int)gridDim.x;
+        int const tile = cta + ts * ctas;
         int const nt = tile % p.tilesN;
         float const* src = p.bTiles + ((size_t)nt * p.kbTot + (size_t)(tile / p.tilesN / p.tilesM) * numIter) * (bBytes / 4);
         for (int it = 0; it < numIter; ++it, ++gk) {
@@ -1538,14 +1607,14 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
           long long const wpos = wxs < nXb ? 0 : (wxs - nXb + 1) * taps + 1;
           if (wpos > gpos) break;
           if (!mbar_wait(smem_u32(&emptyX[wbuf]), wph)) { atomicExch(p.status, 12); return false; }
-          int const tmf = ((int)blockIdx.x + wts * (int)gridDim.x) / p.tilesN;
+          int const tmf = (cta + wts * ctas) / p.tilesN;
           int const split = tmf / p.tilesM, tm = tmf - split * p.tilesM;
           {
             int const per = p.tilesH * p.tilesW;
             int const n = tm / per, t = tm - n * per, wb = t / p.tilesH, hb = t - wb * p.tilesH;
             int const c0 = hb * p.bh - p.a.pt - p.rowOff, c1 = wb * p.bw - p.a.pl;      // c0 is a multiple of four: bh and pt + rowOff are
             mbar_arrive_expect_tx(smem_u32(&fullX[wbuf]), xTileBytes);
-            tma_load_4d(xTile0 + (uint32_t)wbuf * xTileBytes, &xmap, c0, c1, (split * perTile + wsub) * 32, n, smem_u32(&fullX[wbuf]));   // a range of the reduction is whole channel blocks
+            tma_load_4d(xTile0 + (uint32_t)wbuf * xTileBytes, xmap, c0, c1, (split * perTile + wsub) * 32, n, smem_u32(&fullX[wbuf]));   // a range of the reduction is whole channel blocks
           }
           ++wxs;
           if (++wbuf == nXb) { wbuf = 0; wph ^= 1u; }
@@ -1580,7 +1649,7 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
       int buf = 0; uint32_t ph = 1;                        // first use of a buffer: nothing to wait for
       bool ok = true;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
-        int const tmf = ((int)blockIdx.x + ts * (int)gridDim.x) / p.tilesN;
+        int const tmf = (cta + ts * ctas) / p.tilesN;
         int const split = tmf / p.tilesM, t = tmf - split * p.tilesM, cb = t / p.tapGroups, tg = t - cb * p.tapGroups;
         int const tap0 = tg * p.tapsPerTile, nTaps = min(p.tapsPerTile, taps - tap0);
         long long const r0 = (long long)split * numIter * BK;
@@ -1589,7 +1658,7 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
           if (!mbar_wait(smem_u32(&emptyX[buf]), ph)) { atomicExch(p.status, 12); ok = false; break; }
           mbar_arrive_expect_tx(smem_u32(&fullX[buf]), (uint32_t)(nTaps * p.cPer * kWgRowBytes));
           for (int tl = 0; tl < nTaps; ++tl)
-            tma_load_3d(xTile0 + (uint32_t)buf * xTileBytes + (uint32_t)(tl * p.cPer * kWgRowBytes), &xmap,
+            tma_load_3d(xTile0 + (uint32_t)buf * xTileBytes + (uint32_t)(tl * p.cPer * kWgRowBytes), xmap,
                         pix0 + (tapLut[tap0 + tl].x & ~3), cb * p.cPer, img, smem_u32(&fullX[buf]));
           if (++buf == nX) { buf = 0; ph ^= 1u; }
           pix0 += BK; if (pix0 >= P) { pix0 -= P; ++img; }
@@ -1640,7 +1709,7 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
       int const tl = (quarter * 32) / p.cPer;
       int const H = p.a.H, P = p.plane, nX = p.xStages;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
-        int const tmf = ((int)blockIdx.x + ts * (int)gridDim.x) / p.tilesN;
+        int const tmf = (cta + ts * ctas) / p.tilesN;
         int const split = tmf / p.tilesM, t = tmf - split * p.tilesM, tg = t % p.tapGroups;
         int const tap = tg * p.tapsPerTile + tl;
         bool const active = tap < taps;                                   // a tap the filter does not have: rows of zeros, never stored
@@ -1722,7 +1791,7 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
       }
     } else {
       for (int ts = 0; ts < myTiles && ok; ++ts) {
-        int const tile = (int)blockIdx.x + ts * (int)gridDim.x;
+        int const tile = cta + ts * ctas;
         int const tmf = tile / p.tilesN, split = tmf / p.tilesM, kb0 = split * numIter;     // this item's range starts at k-block kb0
         int const m = (tmf - split * p.tilesM) * BM + quarter * 32 + lane;
         uint32_t hm = 0, wm = 0;                          // tap rows / columns inside the image for this pixel
@@ -1733,39 +1802,72 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
           for (int fh = 0; fh < p.a.FH; ++fh) { int h = ho * p.a.sy + fh * p.a.dy - p.a.pt; if (h >= 0 && h < p.a.H) hm |= 1u << fh; }
           for (int fw = 0; fw < p.a.FW; ++fw) { int w = wo * p.a.sx + fw * p.a.dx - p.a.pl; if (w >= 0 && w < p.a.W) wm |= 1u << fw; }
         }
+        if constexpr (kGen) {
+          int const grpC = (tile - tmf * p.tilesN) / p.tilesPerGroup;
+          xq += (long long)grpC * p.aGroup;
+          // A k-block is upk units of kU channels of one tap: one table look-up and validity test per unit, kU loads a constant stride
+          // apart.  Small units are for few channels (kU = 32 would gather zeros), large ones keep the look-ups off the issue slots.
+          auto gather = [&](auto kUnitTag) {
+            constexpr int kU = decltype(kUnitTag)::value, kPer = 32 / kU;
+            for (int it = (int)((gi ^ grp) & 1); it < numIter; it += kTsGroups) {
+              float v[32];
+              int const u0 = (kb0 + it) * kPer;
+              int cb = u0 / taps, tap = u0 - cb * taps;
+#pragma unroll
+              for (int u = 0; u < kPer; ++u) {
+                int2 const te = tapLut[tap];
+                uint32_t const e = (uint32_t)te.y;
+                int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
+                bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
+                float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;
+                if (left >= kU) {
+                  long long const step = on ? (long long)HW : 0;
+#pragma unroll
+                  for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + k * step);
+                  if (!on) {
+#pragma unroll
+                    for (int k = 0; k < kU; ++k) v[u * kU + k] = 0.f;
+                  }
+                } else {
+#pragma unroll
+                  for (int k = 0; k < kU; ++k) { v[u * kU + k] = 0.f; ldg32_if(v[u * kU + k], q + (long long)k * HW, on && k < left); }
+                }
+                if (++tap == taps) { tap = 0; ++cb; }
+              }
+#pragma unroll
+              for (int k = kPer * kU; k < 32; ++k) v[k] = 0.f;
+              if (!hand_over(v, it)) { ok = false; break; }
+            }
+          };
+          switch (p.unit) {
+            case 32: gather(std::integral_constant<int, 32>{}); break;
+            case 16: gather(std::integral_constant<int, 16>{}); break;
+            case 8:  gather(std::integral_constant<int, 8>{}); break;
+            case 4:  gather(std::integral_constant<int, 4>{}); break;
+            case 3:  gather(std::integral_constant<int, 3>{}); break;
+            default: gather(std::integral_constant<int, 1>{}); break;
+          }
+        } else {
         for (int it = (int)((gi ^ grp) & 1); it < numIter; it += kTsGroups) {
-          int const r = (kb0 + it) * BK;
           float v[32];
-          if (p.chanFast) {
-            // the whole k-block is one filter tap and 32 consecutive channels: one validity test, constant stride.  The taps
-            // of a channel block follow one another, so that the lines fetched for one tap are still in L1 for the next.
-            int const tp = (kb0 + it) % taps, c0 = ((kb0 + it) / taps) * 32;
-            int2 const te = tapLut[tp];
-            uint32_t const e = (uint32_t)te.y;
-            bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && c0 < p.a.C;      // (c0 >= C: padding of the last range)
-            // unconditional loads (a pixel outside the image reads the start of the tensor instead and discards it):
-            // nothing for the compiler to predicate or branch around, all 32 in flight together
-            float const* const q = on ? xq + ((long long)c0 * HW + te.x) : p.a.ptr;
-            long long const step = on ? (long long)HW : 0;
+          // the whole k-block is one filter tap and 32 consecutive channels: one validity test, constant stride.  The taps
+          // of a channel block follow one another, so that the lines fetched for one tap are still in L1 for the next.
+          int const tp = (kb0 + it) % taps, c0 = ((kb0 + it) / taps) * 32;
+          int2 const te = tapLut[tp];
+          uint32_t const e = (uint32_t)te.y;
+          bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && c0 < p.a.C;      // (c0 >= C: padding of the last range)
+          // unconditional loads (a pixel outside the image reads the start of the tensor instead and discards it):
+          // nothing for the compiler to predicate or branch around, all 32 in flight together
+          float const* const q = on ? xq + ((long long)c0 * HW + te.x) : p.a.ptr;
+          long long const step = on ? (long long)HW : 0;
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = __ldg(q + k * step);
-            if (!on) {
+          for (int k = 0; k < 32; ++k) v[k] = __ldg(q + k * step);
+          if (!on) {
 #pragma unroll
-              for (int k = 0; k < 32; ++k) v[k] = 0.f;
-            }
-          } else {
-            int tap = r % taps, ch = r / taps;
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              int2 const te = tapLut[tap];
-              uint32_t const e = (uint32_t)te.y;
-              bool const on = ((r + k < p.R ? 1u : 0u) & (hm >> (e & 31u)) & (wm >> (e >> 5))) != 0;
-              v[k] = 0.f;
-              ldg32_if(v[k], xq + (ch * HW + te.x), on);
-              if (++tap == taps) { tap = 0; ++ch; }
-            }
+            for (int k = 0; k < 32; ++k) v[k] = 0.f;
           }
           if (!hand_over(v, it)) { ok = false; break; }
+        }
         }
         gi += numIter;
       }
@@ -1776,8 +1878,8 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
       tc_fence_after();
       if (!done) { if (lane == 0) atomicExch(p.status, 3); }
       else {
-        int const tile = (int)blockIdx.x;
-        ts_store_tile(p, Psm, quarter, lane, 1 + grp, 1 + kTsGroups, tile / p.tilesN, (tile % p.tilesN) * BN);
+        int const tile = cta;
+        ts_store_tile<kGen>(p, Psm, quarter, lane, 1 + grp, 1 + kTsGroups, tile / p.tilesN, tile_cols<kGen>(p, tile % p.tilesN));
       }
       tc_fence_before();
     }
@@ -1786,6 +1888,23 @@ __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1) c
   __syncthreads();
   tc_fence_after();
   if (warp == kEpilogueWarps) tmem_dealloc(tmemAcc, tmemCols);
+}
+
+template <bool kSplit, int kMode, bool kNarrow>
+__global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1)
+conv_ts_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap xmap)
+{
+  conv_ts_body<kSplit, kMode, kNarrow, false>(p, &xmap, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// The same for what the plain kernel's gather does not cover: channels that are no multiple of 32, filter groups, and the residue
+// classes of a strided data gradient (several problems in one launch, so that a small layer's classes share the chip).
+template <bool kSplit, bool kNarrow>
+__global__ void __launch_bounds__(kTsThreads, 1) conv_ts_gen_kernel(const __grid_constant__ TsProblems b)
+{
+  int i = 0;
+  while (i + 1 < b.n && (int)blockIdx.x >= b.p[i + 1].ctaBeg) ++i;
+  conv_ts_body<kSplit, 0, kNarrow, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
 }
 
 // out[e] = sum over splits (ascending) of part[s*stride + e]
@@ -1866,6 +1985,56 @@ __global__ void prep_b_tiles_kernel(float* __restrict__ out, float const* __rest
   }
 }
 
+// Filter tile images for conv_ts_gen_kernel: like prep_b_tiles_kernel's, for the units of channels, filter groups, tap subsets
+// (residue classes of a strided data gradient) and shuffled columns of the general gather.  Row n of a tile is column n of its
+// group; tap (fh', fw') of the problem is tap (bh + ah*fh', bw + aw*fw') of the filter bank, zero where that does not exist; the
+// filter of (column channel n, reduction channel q) starts at F + FH*FW * (gs*group + sn*n + sq*q).
+// grid (rows / 32, k-blocks / per, problems): a thread owns four consecutive reduction indices of one row (one swizzled 16-byte
+// chunk of the hi and of the lo tile) and walks `per` k-blocks, the taps of one block of 32 channels where there are that many: the
+// lines read for one tap are still in L1 for the next, and the stores of a warp are whole lines.
+struct PrepFilters {
+  float* out;
+  float const* f;
+  int BN, numKb, rows, tilesPerGroup, cols, unit, upk, tapsH, tapsW, C, FH, FW, bh, ah, bw, aw, shufY, shufX, per;
+  long long sn, sq, gs;
+};
+struct PrepBatch { PrepFilters p[kMaxTsProblems]; };
+
+template <bool kSplit>
+__global__ void __launch_bounds__(256) prep_filters_kernel(const __grid_constant__ PrepBatch b)
+{
+  PrepFilters const& p = b.p[blockIdx.z];
+  int const row = (int)blockIdx.x * 32 + ((int)threadIdx.x >> 3), chunk = (int)threadIdx.x & 7;
+  if (row >= p.rows) return;
+  int const tile = row / p.BN, inTile = row - tile * p.BN, grp = tile / p.tilesPerGroup;
+  int const col = (tile - grp * p.tilesPerGroup) * p.BN + inTile;
+  int ry = 0, rx = 0, n = col;
+  if (p.shufY > 0) { n = col / (p.shufY * p.shufX); int const t = col - n * p.shufY * p.shufX; rx = t / p.shufY; ry = t - rx * p.shufY; }
+  int const taps = p.tapsH * p.tapsW, FT = p.FH * p.FW;
+  float const* const f = p.f + (long long)FT * (p.gs * grp + p.sn * n);
+  int const kbEnd = min(p.numKb, ((int)blockIdx.y + 1) * p.per);
+  for (int kb = (int)blockIdx.y * p.per; kb < kbEnd; ++kb) {
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      int const kk = chunk * 4 + e, u = kk / p.unit;
+      int const un = kb * p.upk + u, cb = un / taps, tap = un - cb * taps, q = cb * p.unit + (kk - u * p.unit);
+      int const tw = tap / p.tapsH, th = tap - tw * p.tapsH;
+      int const fh = p.bh + p.ah * th + ry, fw = p.bw + p.aw * tw + rx;
+      bool const on = u < p.upk && q < p.C && col < p.cols && (unsigned)fh < (unsigned)p.FH && (unsigned)fw < (unsigned)p.FW;
+      v[e] = on ? __ldg(f + (long long)FT * p.sq * q + (fh + p.FH * fw)) : 0.f;
+    }
+    float* const base = p.out + ((size_t)tile * p.numKb + kb) * (kSplit ? 2 : 1) * (size_t)p.BN * 32 + (size_t)inTile * 32 + ((chunk ^ (inTile & 7)) << 2);
+    if (kSplit) {
+      float4 const h = make_float4(tf32_hi(v[0]), tf32_hi(v[1]), tf32_hi(v[2]), tf32_hi(v[3]));
+      *reinterpret_cast<float4*>(base) = h;
+      *reinterpret_cast<float4*>(base + (size_t)p.BN * 32) = make_float4(v[0] - h.x, v[1] - h.y, v[2] - h.z, v[3] - h.w);
+    } else {
+      *reinterpret_cast<float4*>(base) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
 // dY of a filter gradient as tile images (mode 2 of prep_b_tiles_kernel) for planes that are a multiple of
 // four pixels: 16-byte loads along the pixels, 16-byte stores of the swizzled chunks, and -- dY being read
 // anyway -- the bias gradient db[n] = sum of dY over pixels and images (reference bits/nnconv.cu:141-149) on
@@ -1874,14 +2043,18 @@ __global__ void prep_b_tiles_kernel(float* __restrict__ out, float const* __rest
 // grid (blocks per channel, channels rounded up to the tile), kPrepThreads threads, kPrepIters float4 per thread.
 constexpr int kPrepThreads = 256, kPrepIters = 4;
 
-template <bool kSplit>
+// Filter groups: the Kg channels of a group start a new column tile (tilesPerGroup of them; one group: Kg = N).
+// kVec: planes of a multiple of four pixels on a 16-byte boundary; otherwise (13 x 13, 27 x 27 maps) four scalar loads.
+template <bool kSplit, bool kVec>
 __global__ void __launch_bounds__(kPrepThreads)
 prep_dy_tiles_kernel(float* __restrict__ out, float const* __restrict__ dy, int N, int R, int P, int Pp, int BN, int numKb,
-                     float* __restrict__ db, float* __restrict__ dbPart, unsigned* __restrict__ tickets)
+                     float* __restrict__ db, float* __restrict__ dbPart, unsigned* __restrict__ tickets, int Kg, int tilesPerGroup)
 {
   __shared__ float red[kPrepThreads / 32];
   __shared__ bool last;
-  int const n = blockIdx.y, tile = n / BN, row = n % BN;
+  int const tile = blockIdx.y / BN, row = blockIdx.y - tile * BN, grp = tile / tilesPerGroup;
+  int const local = (tile - grp * tilesPerGroup) * BN + row;
+  int const n = local < Kg ? grp * Kg + local : N;         // N: a column that does not exist
   int const Rp = numKb * 32;
   float sum = 0.f;
 #pragma unroll
@@ -1891,7 +2064,20 @@ prep_dy_tiles_kernel(float* __restrict__ out, float const* __restrict__ dy, int 
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       // reduction index r = pixel + Pp * image (Pp >= P: planes padded to whole k-blocks read as zeros); R = P * images
       int const img = r / Pp, pix = r - img * Pp;
-      if (n < N && pix < P && img * P + pix < R) v = *reinterpret_cast<float4 const*>(dy + ((size_t)img * N + n) * P + pix);
+      if (kVec) {
+        if (n < N && pix < P && img * P + pix < R) v = *reinterpret_cast<float4 const*>(dy + ((size_t)img * N + n) * P + pix);
+      } else if (n < N) {
+        // (planes that are no multiple of four pixels are never padded: Pp == P)
+        float w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          int const over = pix + e >= P ? 1 : 0;               // the four indices may run into the next images' planes
+          int pe = pix + e - (over ? P : 0), ie = img + over;
+          while (pe >= P) { pe -= P; ++ie; }
+          w[e] = r + e < R ? dy[((size_t)ie * N + n) * P + pe] : 0.f;
+        }
+        v = make_float4(w[0], w[1], w[2], w[3]);
+      }
       sum += (v.x + v.y) + (v.z + v.w);
       int const kb = r >> 5, kk = r & 31;
       size_t const base = ((size_t)tile * numKb + kb) * (kSplit ? 2 : 1) * (size_t)BN * 32;
@@ -1964,13 +2150,16 @@ float const* prep_b_tiles(vlb_ctx* ctx, float const* f, int N, int R, int BN, in
   return tiles;
 }
 
-// dY tile images with 16-byte accesses and, when db is given, the bias gradient from the same sweep.
+// dY tile images and, when db is given, the bias gradient from the same sweep; K channels in `groups` filter groups.
 // Scratch layout: [tiles][extraBytes for the caller][per-block partial sums of db].
-float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, int BN, int numKb, size_t extraBytes, float* db, int Pp = 0)
+float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, int BN, int numKb, size_t extraBytes, float* db, int Pp = 0,
+                           int groups = 1)
 {
   if (Pp == 0) Pp = P;
   bool split3 = ctx->precision == VLB_PRECISION_3XTF32;
-  size_t const tileBytes = b_tiles_bytes(ctx, K, BN, numKb);
+  int const Kg = K / groups, tpg = vlb::ceil_div(Kg, BN), rows = groups * tpg * BN;
+  bool const vec = P % 4 == 0 && (((uintptr_t)dY) & 15) == 0;
+  size_t const tileBytes = b_tiles_bytes(ctx, rows, BN, numKb);
   int const perBlock = kPrepThreads * 4 * kPrepIters;
   unsigned const bx = (unsigned)vlb::ceil_div((long long)numKb * 32, perBlock);
   size_t const partBytes = db ? sizeof(float) * (size_t)K * bx : 0;
@@ -1980,9 +2169,11 @@ float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, i
   float* tiles = (float*)ws;
   float* dbPart = db ? (float*)(ws + tileBytes + extraBytes) : nullptr;
   unsigned* tickets = (unsigned*)((char*)ctx->deviceStatus + 256);
-  dim3 grid(bx, (unsigned)(vlb::ceil_div(K, BN) * BN));
-  if (split3) prep_dy_tiles_kernel<true><<<grid, kPrepThreads, 0, ctx->stream>>>(tiles, dY, K, R, P, Pp, BN, numKb, db, dbPart, tickets);
-  else        prep_dy_tiles_kernel<false><<<grid, kPrepThreads, 0, ctx->stream>>>(tiles, dY, K, R, P, Pp, BN, numKb, db, dbPart, tickets);
+  dim3 grid(bx, (unsigned)rows);
+#define VLB_PDY(split, v) prep_dy_tiles_kernel<split, v><<<grid, kPrepThreads, 0, ctx->stream>>>(tiles, dY, K, R, P, Pp, BN, numKb, db, dbPart, tickets, Kg, tpg)
+  if (split3) { if (vec) VLB_PDY(true, true); else VLB_PDY(true, false); }
+  else        { if (vec) VLB_PDY(false, true); else VLB_PDY(false, false); }
+#undef VLB_PDY
   VLB_LAUNCHED(ctx, 1);
   return tiles;
 }
@@ -2002,6 +2193,10 @@ template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 0, true>>() { retu
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 0, false>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 1, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 1, false>>() { return 128; }
+template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<true, true>>() { return 128; }
+template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<true, false>>() { return 128; }
+template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<false, true>>() { return 128; }
+template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<false, false>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 2, false>>() { return 96; }
 
@@ -2035,7 +2230,8 @@ int launch(vlb_ctx* ctx, Params& p, int splits, char const* where)
   p.status = ctx->deviceStatus;
   p.drainEvery = kDrainEvery;
   size_t smemBytes = (size_t)stages * stageBytes + 1024;
-  dim3 grid(vlb::ceil_div(p.M, BM), vlb::ceil_div(p.N, p.BN), splits);
+  p.tilesM = vlb::ceil_div(p.M, BM);
+  dim3 grid(p.tilesM * std::max(p.groups, 1), vlb::ceil_div(p.N, p.BN), splits);
   if (grid.y > 65535u || grid.z > 65535u) return VLB_Unsupported;
   cudaError_t e;
   vlb_ctx::ProfRec rec;
@@ -2446,6 +2642,246 @@ int fc_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, floa
   return launch_ts(ctx, p, "fc_wgrad_ts");
 }
 
+// ------------------------------------------------------------------ general gather: host side
+// Channels per unit of the general gather: the least work, counting the gathered zeros (channels rounded up to units; kU = 3 leaves two of
+// a k-block's 32 places empty) and the look-ups of small units (relative cost of a k-block, measured on 56 x 56 maps).
+int gen_unit(int C)
+{
+  static int const unit[] = {32, 16, 8, 4, 3, 1};
+  static double const cost[] = {1.0, 1.03, 1.1, 1.25, 1.35, 2.0};
+  int best = 1; double bestCost = 1e30;
+  for (int i = 0; i < 6; ++i) {
+    double const c = cost[i] * (vlb::ceil_div(C, unit[i]) * unit[i]) * (32.0 / (32 / unit[i] * unit[i])) / C;
+    if (c < bestCost) { bestCost = c; best = unit[i]; }
+  }
+  return best;
+}
+
+// Filter groups narrower than this (depthwise convolutions) leave a tensor-core tile nearly empty: CUDA cores.
+constexpr int kMinGroupCols = 4;
+
+bool gen_taps_ok(int FH, int FW) { return FH <= 32 && FW <= 32 && FH * FW <= kMaxGenTaps; }
+
+// One contraction of conv_ts_gen_kernel: the stride / pad / dilation geometry t over src, `groups` groups of chPerGroup channels
+// and `cols` output columns each.
+void gen_problem(Params& p, ConvGeom const& t, float const* src, int chPerGroup, int groups, int cols, int BN)
+{
+  conv_operand(p.a, t, src, chPerGroup * groups);
+  p.a.C = chPerGroup; p.aGroup = (long long)t.H * t.W * chPerGroup;
+  p.M = t.Ho * t.Wo * t.N; p.N = cols * groups; p.R = t.FH * t.FW * chPerGroup; p.a.rows = p.M;
+  p.unit = gen_unit(chPerGroup); p.upk = 32 / p.unit;
+  p.numKb = vlb::ceil_div(t.FH * t.FW * vlb::ceil_div(chPerGroup, p.unit), p.upk);
+  p.BN = BN; p.cols = cols; p.tilesPerGroup = vlb::ceil_div(cols, BN); p.tilesN = groups * p.tilesPerGroup; p.tilesM = vlb::ceil_div(p.M, BM);
+  p.splits = 1; p.kbPerSplit = p.kbTot = p.numKb;
+  p.oy = p.ox = 0; p.oys = p.oxs = 1; p.outH = t.Ho; p.outW = t.Wo; p.shufY = p.shufX = 0; p.outC = cols;
+}
+
+// The part of the filter tile images' description that follows from the problem.
+PrepFilters gen_prep(Params const& p, ConvGeom const& g, float const* f)
+{
+  PrepFilters q = {};
+  q.f = f; q.BN = p.BN; q.numKb = p.numKb; q.rows = p.tilesN * p.BN; q.tilesPerGroup = p.tilesPerGroup; q.cols = p.cols;
+  q.unit = p.unit; q.upk = p.upk; q.tapsH = p.a.FH; q.tapsW = p.a.FW; q.C = p.a.C; q.FH = g.FH; q.FW = g.FW;
+  q.ah = q.aw = 1; q.shufY = p.shufY; q.shufX = p.shufX;
+  q.per = p.unit == 32 ? std::max(4, std::min(16, q.tapsH * q.tapsW)) : 8;
+  return q;
+}
+
+// Time of a problem's k-blocks in units of a 128-column k-block, for comparing routes: narrower tiles save less than they drop columns.
+double gen_cost(int tiles, int numKb, int BN)
+{
+  double const kb = BN == 128 ? 1.0 : (BN == 64 ? 0.62 : 0.5);
+  return (double)tiles * (numKb + 6) * kb;
+}
+
+// Builds the tile images of all problems (one launch) and runs them (one launch).  The problems share the tile width.
+int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, char const* where)
+{
+  bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
+  int const BN = b.p[0].BN;
+  size_t const stageBytes = (split3 ? 2u : 1u) * (size_t)BN * BK * 4;
+  size_t total = 0, sumBytes = 0;
+  long long tiles = 0;
+  int rows = 0, kbGroups = 0;
+  double work = 0;
+  for (int i = 0; i < b.n; ++i) {
+    Params& p = b.p[i];
+    prep.p[i].out = (float*)total;                 // offset for now
+    total += (sizeof(float) * (size_t)p.tilesN * BN * (size_t)p.numKb * 32 * (split3 ? 2 : 1) + 255) & ~(size_t)255;
+    rows = std::max(rows, prep.p[i].rows); kbGroups = std::max(kbGroups, vlb::ceil_div(prep.p[i].numKb, prep.p[i].per));
+    p.smemSum = ((ctx->testSwitch & 8) || p.kbPerSplit < 8) ? 1 : 0;
+    sumBytes = std::max(sumBytes, p_bytes(BN, p.smemSum));
+    long long const t = (long long)p.tilesM * p.tilesN;
+    tiles += t;
+    work += (double)t * (p.numKb + 6);
+    if (t >= (1LL << 31)) return VLB_Unsupported;
+  }
+  char* const ws = (char*)vlb::workspace(ctx, total);
+  if (!ws) return ctx->lastError;
+  // CTAs per problem: one per tile when all tiles fit, else shares of the chip in proportion to the work, the rest to the longest queues
+  int given = 0;
+  for (int i = 0; i < b.n; ++i) {
+    Params& p = b.p[i];
+    long long const t = (long long)p.tilesM * p.tilesN;
+    p.ctas = tiles <= ctx->smCount ? (int)t
+             : (int)std::min<long long>(t, std::max(1, (int)((double)ctx->smCount * (double)t * (p.numKb + 6) / work)));
+    given += p.ctas;
+  }
+  while (tiles > ctx->smCount && given < ctx->smCount) {
+    int worst = -1; double most = 0;
+    for (int i = 0; i < b.n; ++i) {
+      Params const& p = b.p[i];
+      long long const t = (long long)p.tilesM * p.tilesN;
+      double const queue = (double)((t + p.ctas - 1) / p.ctas) * (p.numKb + 6);
+      if (p.ctas < t && queue > most) { most = queue; worst = i; }
+    }
+    if (worst < 0) break;
+    ++b.p[worst].ctas; ++given;
+  }
+  int const stages = (int)std::min<size_t>(kTsBStages, (227 * 1024 - 1536 - 1024 - sumBytes) / stageBytes);
+  for (int i = 0, beg = 0; i < b.n; ++i) {
+    Params& p = b.p[i];
+    p.ctaBeg = beg; beg += p.ctas;
+    prep.p[i].out = (float*)(ws + (size_t)prep.p[i].out);
+    p.bTiles = prep.p[i].out;
+    p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;
+  }
+  dim3 const pgrid(vlb::ceil_div(rows, 32), kbGroups, b.n);
+  if (pgrid.y > 65535u) return VLB_Unsupported;
+  if (split3) prep_filters_kernel<true><<<pgrid, 256, 0, ctx->stream>>>(prep);
+  else        prep_filters_kernel<false><<<pgrid, 256, 0, ctx->stream>>>(prep);
+  size_t const smemBytes = std::max<size_t>((size_t)stages * stageBytes + sumBytes + 1024, 120u * 1024u);      // two CTAs never share an SM
+  cudaError_t e;
+  auto go = [&](auto kernel) {
+    e = allow_large_smem<decltype(kernel)::value>(ctx->device);
+    if (e == cudaSuccess) decltype(kernel)::value<<<given, kTsThreads, smemBytes, ctx->stream>>>(b);
+  };
+#define VLB_TSG(split, nar) go(std::integral_constant<decltype(&conv_ts_gen_kernel<split, nar>), &conv_ts_gen_kernel<split, nar>>{})
+  if (split3) { if (BN <= 64) VLB_TSG(true, true); else VLB_TSG(true, false); }
+  else        { if (BN <= 64) VLB_TSG(false, true); else VLB_TSG(false, false); }
+#undef VLB_TSG
+  if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
+  VLB_LAUNCHED(ctx, 2);
+  return vlb::check_launch(ctx, where);
+}
+
+// Forward convolution through the general gather: any channel count, stride, dilation, filter groups.
+int conv_fprop_gen(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, float const* X, float inMult, float const* F, float const* b)
+{
+  TsProblems ts = {};
+  PrepBatch prep = {};
+  ts.n = 1;
+  Params& p = ts.p[0];
+  gen_problem(p, g, X, g.FC, g.G, g.Kg, pick_bn(g.Kg));
+  p.e.out = Y; p.e.bias = b; p.e.inMult = inMult; p.e.outMult = outMult; p.e.P = g.Ho * g.Wo; p.e.Ktot = g.K;
+  p.e.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
+  PrepFilters& q = prep.p[0] = gen_prep(p, g, F);
+  q.sn = g.FC; q.sq = 1; q.gs = (long long)g.FC * g.Kg;
+  return launch_ts_gen(ctx, ts, prep, "conv_fprop_gen");
+}
+
+// One dimension of a data gradient's residue class: the input positions h with (h + pad) % stride == r, and the filter taps that reach
+// them.  Positions are h0 + stride * i, i < count; tap f0 + step * (taps - 1 - f') of the filter meets position i at output
+// position i + f' * dil - pad: a stride-1 convolution of the output derivative with `taps` taps.
+struct ClassDim { int h0, count, taps, f0, step, dil, pad; };
+
+ClassDim class_dim(int r, int H, int FH, int stride, int pad, int dilate)
+{
+  ClassDim c = {};
+  c.h0 = ((r - pad) % stride + stride) % stride;
+  c.count = c.h0 < H ? (H - 1 - c.h0) / stride + 1 : 0;
+  int a = stride, d = dilate;
+  while (d) { int const t = a % d; a = d; d = t; }                   // a = gcd(stride, dilate)
+  c.step = stride / a; c.dil = dilate / a;
+  c.f0 = -1;
+  for (int f = 0; f < c.step && f < FH; ++f) if ((f * dilate) % stride == r) c.f0 = f;
+  c.taps = c.f0 < 0 ? 0 : (FH - 1 - c.f0) / c.step + 1;
+  // output position of tap f0 + step*j at position h: (h + pad - (f0 + step*j)*dilate) / stride = i + first - j*dil
+  int const first = c.f0 < 0 ? 0 : (c.h0 + pad - c.f0 * dilate) / stride;          // exact: the numerator is a multiple of the stride
+  c.pad = (c.taps - 1) * c.dil - first;
+  return c;
+}
+
+// Data gradient of a strided or grouped convolution, or one whose filters are no multiple of 32, through the general gather.  Two forms:
+//   classes   one problem per residue class of the input pixel modulo the stride, each a stride-1 convolution of dY with the taps that
+//             reach the class: no product with a structural zero, but C columns each;
+//   shuffled  (dilation 1) one problem over the stride-sized blocks of input pixels whose columns are (pixel of the block, channel):
+//             the classes' taps padded to the largest class, C * strideY * strideX columns -- for few channels, whose class
+//             tiles would be mostly empty columns (11 x 11 stride 4 onto 3 channels: one 48-column problem instead of 16 with 3).
+int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
+{
+  int const C = g.FC, nc = g.sy * g.sx;
+  ConvGeom t = g;
+  t.H = g.Ho; t.W = g.Wo; t.N = g.N; t.sy = t.sx = 1;
+  ClassDim ch[kMaxTsProblems], cw[kMaxTsProblems];
+  bool const classesOk = g.sy <= kMaxTsProblems && g.sx <= kMaxTsProblems && nc <= kMaxTsProblems;
+  double classCost = 1e30;
+  bool holes = false;               // classes that no tap reaches: zeros
+  int const unit = gen_unit(g.Kg), upk = 32 / unit;
+  auto kblocks = [&](int taps) { return vlb::ceil_div(taps * vlb::ceil_div(g.Kg, unit), upk); };
+  if (classesOk) {
+    classCost = 0;
+    for (int r = 0; r < g.sy; ++r) ch[r] = class_dim(r, g.H, g.FH, g.sy, g.pt, g.dy);
+    for (int r = 0; r < g.sx; ++r) cw[r] = class_dim(r, g.W, g.FW, g.sx, g.pl, g.dx);
+    int const BN = pick_bn(C);
+    for (int y = 0; y < g.sy; ++y)
+      for (int x = 0; x < g.sx; ++x) {
+        int const taps = ch[y].taps * cw[x].taps, pix = ch[y].count * cw[x].count;
+        if (pix == 0) continue;
+        if (taps == 0) { holes = true; continue; }
+        classCost += gen_cost(vlb::ceil_div((long long)pix * g.N, BM) * g.G * vlb::ceil_div(C, BN), kblocks(taps), BN);
+      }
+  }
+  TsProblems ts = {};
+  PrepBatch prep = {};
+  // shuffled form
+  int const FHm = vlb::ceil_div(g.FH, g.sy), FWm = vlb::ceil_div(g.FW, g.sx);
+  int const iy = g.pt / g.sy, ix = g.pl / g.sx, Hm = (g.H - 1 + g.pt) / g.sy - iy + 1, Wm = (g.W - 1 + g.pl) / g.sx - ix + 1;
+  if (nc > 1 && g.dy == 1 && g.dx == 1 && gen_taps_ok(FHm, FWm)) {
+    int const cols = C * nc, BN = pick_bn(cols);
+    double const cost = gen_cost(vlb::ceil_div((long long)Hm * Wm * g.N, BM) * g.G * vlb::ceil_div(cols, BN), kblocks(FHm * FWm), BN);
+    if (cost < classCost) {
+      t.FH = FHm; t.FW = FWm; t.Ho = Hm; t.Wo = Wm; t.pt = FHm - 1 - iy; t.pl = FWm - 1 - ix;
+      ts.n = 1;
+      Params& p = ts.p[0];
+      gen_problem(p, t, dY, g.Kg, g.G, cols, BN);
+      p.oys = g.sy; p.oxs = g.sx; p.oy = g.sy * iy - g.pt; p.ox = g.sx * ix - g.pl; p.outH = g.H; p.outW = g.W;
+      p.shufY = g.sy; p.shufX = g.sx; p.outC = C;
+      p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C; p.e.mask = ctx->reluMask;
+      ctx->maskDone = ctx->reluMask != nullptr;
+      PrepFilters& q = prep.p[0] = gen_prep(p, g, F);
+      q.bh = g.sy * (FHm - 1); q.ah = -g.sy; q.bw = g.sx * (FWm - 1); q.aw = -g.sx;
+      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
+      return launch_ts_gen(ctx, ts, prep, "conv_dgrad_gen");
+    }
+  }
+  if (!classesOk) return VLB_Unsupported;
+  for (int y = 0; y < g.sy; ++y) for (int x = 0; x < g.sx; ++x) if (ch[y].taps * cw[x].taps > 0 && !gen_taps_ok(ch[y].taps, cw[x].taps)) return VLB_Unsupported;
+  if (holes) {
+    cudaError_t const e = cudaMemsetAsync(dX, 0, sizeof(float) * (size_t)g.H * g.W * g.C * g.N, ctx->stream);
+    if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
+  }
+  ts.n = 0;
+  for (int y = 0; y < g.sy; ++y)
+    for (int x = 0; x < g.sx; ++x) {
+      ClassDim const& h = ch[y];
+      ClassDim const& w = cw[x];
+      if (h.taps * w.taps == 0 || h.count * w.count == 0) continue;
+      t.FH = h.taps; t.FW = w.taps; t.Ho = h.count; t.Wo = w.count; t.pt = h.pad; t.pl = w.pad; t.dy = h.dil; t.dx = w.dil;
+      Params& p = ts.p[ts.n];
+      gen_problem(p, t, dY, g.Kg, g.G, C, pick_bn(C));
+      p.oys = g.sy; p.oxs = g.sx; p.oy = h.h0; p.ox = w.h0; p.outH = g.H; p.outW = g.W;
+      p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C; p.e.mask = ctx->reluMask;
+      PrepFilters& q = prep.p[ts.n] = gen_prep(p, g, F);
+      q.bh = h.f0 + h.step * (h.taps - 1); q.ah = -h.step; q.bw = w.f0 + w.step * (w.taps - 1); q.aw = -w.step;
+      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
+      ++ts.n;
+    }
+  ctx->maskDone = ctx->reluMask != nullptr;
+  if (ts.n == 0) return VLB_Success;                // no tap reaches any pixel: all zeros, written above
+  return launch_ts_gen(ctx, ts, prep, "conv_dgrad_gen");
+}
+
 bool is_fc(ConvGeom const& g)
 {
   return g.Ho == 1 && g.Wo == 1 && g.FH == g.H && g.FW == g.W && g.FC == g.C && g.sy == 1 && g.sx == 1 && g.pt == 0 &&
@@ -2459,7 +2895,7 @@ namespace vlb {
 int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, float const* X, float inMult,
                   float const* F, float const* b)
 {
-  if (g.G != 1 || !fits32(g)) return VLB_Unsupported;
+  if (!fits32(g)) return VLB_Unsupported;
   int const V = g.FH * g.FW * g.FC;
   Params p = {};
   if (is_fc(g)) {
@@ -2500,6 +2936,10 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
   long long M = (long long)g.Ho * g.Wo * g.N;
   ProfScope prof(ctx, kProfFprop);
   prof.rec.flops = 2.0 * (double)M * (double)g.K * (double)V;
+  // whole blocks of 32 channels and one group: the plain kernel; everything else through the general gather
+  if ((g.G != 1 || g.C % 32 != 0 || g.FH * g.FW > 64) && gen_taps_ok(g.FH, g.FW) && (g.G == 1 || g.Kg >= kMinGroupCols))
+    return conv_fprop_gen(ctx, g, Y, outMult, X, inMult, F, b);
+  if (g.G != 1) { prof.rec.flops = 0; return VLB_Unsupported; }
   p.M = (int)M; p.N = g.K; p.R = V;
   conv_operand(p.a, g, X, g.C);
   p.a.rows = p.M;
@@ -2508,9 +2948,9 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
   p.numKb = ceil_div(p.R, BK); p.kbPerSplit = p.numKb;
   p.e = Epilogue{}; p.e.out = Y; p.e.bias = b; p.e.inMult = inMult; p.e.outMult = outMult; p.e.P = g.Ho * g.Wo; p.e.Ktot = g.K;
   p.e.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
-  if (p.a.fast) {
-    p.chanFast = g.C % 32 == 0;
-    p.bTiles = prep_b_tiles(ctx, F, g.K, V, p.BN, p.numKb, p.chanFast ? 3 : 0, g);
+  if (p.a.fast && g.C % 32 == 0) {
+    p.chanFast = 1;
+    p.bTiles = prep_b_tiles(ctx, F, g.K, V, p.BN, p.numKb, 3, g);
     if (!p.bTiles) return ctx->lastError;
     p.pipelined = 1;
     return launch_ts(ctx, p, "conv_fprop_ts");
@@ -2520,7 +2960,7 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
 
 int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
 {
-  if (g.G != 1 || !fits32(g)) return VLB_Unsupported;
+  if (!fits32(g)) return VLB_Unsupported;
   Params p = {};
   if (is_fc(g)) {
     // dX(V x N) = F(V x K) dY(K x N)  (reference bits/nnfullyconnected.cu:139-151): rows = input elements
@@ -2539,7 +2979,14 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     p.e = Epilogue{}; p.e.out = dX; p.e.ldd = V;
     return launch<OP_DENSE_MN, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "fc_dgrad_tc");
   }
-  if (g.sy != 1 || g.sx != 1) return VLB_Unsupported;
+  if (g.G != 1 || g.sy != 1 || g.sx != 1 || g.K % 32 != 0 || g.FH * g.FW > 64) {
+    ProfScope prof(ctx, kProfDgrad);
+    prof.rec.flops = 2.0 * (double)g.Ho * g.Wo * g.N * (double)g.K * g.FH * g.FW * g.FC;
+    int const rc = g.FC >= kMinGroupCols || g.G == 1 ? conv_dgrad_gen(ctx, g, dX, F, dY) : VLB_Unsupported;
+    if (rc != VLB_Unsupported) return rc;
+    prof.rec.flops = 0;
+  }
+  if (g.G != 1 || g.sy != 1 || g.sx != 1) return VLB_Unsupported;
   // dX = conv(dY, flipped and transposed filters) with padding (F-1)*dilate - pad
   ConvGeom t = g;
   t.H = g.Ho; t.W = g.Wo; t.C = g.K; t.FC = g.K; t.K = g.C; t.Ho = g.H; t.Wo = g.W;
@@ -2554,9 +3001,9 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
   p.BN = pick_bn(p.N);
   p.numKb = ceil_div(p.R, BK); p.kbPerSplit = p.numKb;
   p.b = Operand{}; p.b.ld = V; p.b.rows = g.C;
-  if (p.a.fast) {
-    p.chanFast = g.K % 32 == 0;
-    p.bTiles = prep_b_tiles(ctx, F, g.C, V, p.BN, p.numKb, p.chanFast ? 4 : 1, g);
+  if (p.a.fast && g.K % 32 == 0) {
+    p.chanFast = 1;
+    p.bTiles = prep_b_tiles(ctx, F, g.C, V, p.BN, p.numKb, 4, g);
     if (!p.bTiles) return ctx->lastError;
     p.b.ptr = p.bTiles;          // not read by the pipelined producers
     p.pipelined = 1;
@@ -2579,7 +3026,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
 int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float const* X, float const* dY, bool* dbDone)
 {
   *dbDone = false;
-  if (g.G != 1 || !fits32(g)) return VLB_Unsupported;
+  if (!fits32(g) || (g.G > 1 && g.Kg < kMinGroupCols)) return VLB_Unsupported;
   int const V = g.FH * g.FW * g.FC;
   Params p = {};
   if (is_fc(g)) {
@@ -2598,49 +3045,40 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
     p.e = Epilogue{}; p.e.out = dF; p.e.ldd = V;
     return launch<OP_DENSE_MN, OP_DENSE_MN, EPI_PLAIN>(ctx, p, 1, "fc_wgrad_tc");
   }
-  {
+  if (g.G == 1) {
     int const rc = conv_wgrad_ts(ctx, g, dF, db, X, dY, dbDone);
     if (rc >= 0) return rc;
   }
   long long R = (long long)g.Ho * g.Wo * g.N;
   ProfScope prof(ctx, kProfWgrad);      // includes the dY tile images (with the bias gradient) and the sum of the split partial results
   prof.rec.flops = 2.0 * (double)V * (double)g.K * (double)R;
-  p.M = V; p.N = g.K; p.R = (int)R;
+  p.M = V; p.N = g.Kg; p.R = (int)R; p.groups = g.G; p.aGroup = (long long)g.H * g.W * g.FC;
   conv_operand(p.a, g, X, g.C);
   p.a.rows = V;
+  if (!p.a.fast) p.a.fast = 2;            // (the tap table of this mode has no limit on the filter's size)
   int const P = g.Ho * g.Wo;
-  p.b = Operand{}; p.b.ptr = dY; p.b.ld = P; p.b.bs = (long long)P * g.K; p.b.P = P; p.b.rows = g.K;
-  p.b.vec = (P % 4 == 0) && aligned16(dY);
   p.BN = pick_bn(p.N);
   p.numKb = ceil_div(p.R, BK);
-  int tiles = ceil_div(p.M, BM) * ceil_div(p.N, p.BN);
+  int const tpg = ceil_div(p.N, p.BN), tiles = ceil_div(p.M, BM) * tpg * g.G;
+  if (tpg * p.BN * g.G > 65535) return VLB_Unsupported;
   int splits = pick_splits(ctx, tiles, p.numKb, 8);
   p.kbPerSplit = ceil_div(p.numKb, splits);
   splits = ceil_div(p.numKb, p.kbPerSplit);
   p.e = Epilogue{}; p.e.ldd = V;
   size_t nF = (size_t)V * g.K;
-  size_t partBytes = splits > 1 ? sizeof(float) * nF * splits : 0;
-  size_t tileBytes = 0;
-  if (p.a.fast) {
-    // dY is split into hi / lo once and laid out as tile images, like the filters of fprop
-    tileBytes = b_tiles_bytes(ctx, g.K, p.BN, p.numKb);
-    partBytes = (partBytes + 255) & ~(size_t)255;
-    if (P % 4 == 0 && aligned16(dY) && g.K <= 4096 && vlb::ceil_div(g.K, p.BN) * p.BN <= 65535) {
-      p.bTiles = prep_dy_tiles(ctx, dY, g.K, p.R, P, p.BN, p.numKb, partBytes, db);
-      *dbDone = db != nullptr;
-    } else {
-      p.bTiles = prep_b_tiles(ctx, dY, g.K, p.R, p.BN, p.numKb, 2, g, partBytes, P);
-    }
-    if (!p.bTiles) return ctx->lastError;
-    p.pipelined = 1;
-  }
+  size_t const partBytes = splits > 1 ? (sizeof(float) * nF * splits + 255) & ~(size_t)255 : 0;
+  // dY is split into hi / lo once and laid out as tile images, like the filters of fprop
+  size_t const tileBytes = b_tiles_bytes(ctx, tpg * p.BN * g.G, p.BN, p.numKb);
+  float* const dbHere = g.K <= 4096 ? db : nullptr;      // (a ticket counter per channel)
+  p.bTiles = prep_dy_tiles(ctx, dY, g.K, p.R, P, p.BN, p.numKb, partBytes, dbHere, 0, g.G);
+  if (!p.bTiles) return ctx->lastError;
+  *dbDone = dbHere != nullptr;
+  p.pipelined = 1;
   if (splits == 1) {
     p.e.out = dF;
     return launch<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "conv_wgrad_tc");
   }
-  char* ws = (char*)workspace(ctx, tileBytes + partBytes);
-  float* part = ws ? (float*)(ws + tileBytes) : nullptr;
-  if (!part) return ctx->lastError;
+  float* const part = (float*)((char*)p.bTiles + tileBytes);
   p.e.out = part; p.e.splitStride = (long long)nF;
   int rc = launch<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "conv_wgrad_tc");
   if (rc) return rc;

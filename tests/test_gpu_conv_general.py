@@ -1,0 +1,59 @@
+"""The general gather of the tensor-memory convolution kernel against the CPU checker: channel counts that are no multiple of
+32 (every unit size), filter groups, and strided data gradients in both forms -- one problem per residue class of the input pixel, and
+the shuffled form for few channels -- with dilation, uneven padding, classes that no filter tap reaches, and the ReLU mask."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# x, filters (FH, FW, C / groups, K), stride, pad (top bottom left right), dilate
+CASES = {
+    "unit1_c1": ((17, 15, 1, 3), (5, 4, 1, 20), (1, 1), (2, 1, 0, 2), (1, 1)),
+    "unit3_rgb_11x11_s4": ((67, 59, 3, 3), (11, 11, 3, 24), (4, 4), (0, 0, 0, 0), (1, 1)),         # shuffled: 48 columns, ragged classes
+    "unit4_c20": ((12, 12, 20, 7), (5, 5, 20, 50), (1, 1), (0, 0, 0, 0), (1, 1)),
+    "unit16_c48": ((13, 9, 48, 5), (3, 3, 48, 70), (2, 1), (1, 1, 0, 1), (1, 1)),
+    "unit32_tail_c90": ((29, 22, 90, 3), (3, 3, 90, 150), (2, 2), (1, 1, 1, 1), (1, 1)),           # classes of 4, 2, 2, 1 taps
+    "one_by_one_s2": ((15, 16, 64, 4), (1, 1, 64, 96), (2, 2), (0, 0, 0, 0), (1, 1)),              # three classes without a tap
+    "one_by_one_s2_narrow": ((14, 13, 8, 4), (1, 1, 8, 40), (2, 2), (0, 0, 0, 0), (1, 1)),         # the same, shuffled
+    "s3_f2": ((16, 17, 32, 2), (2, 2, 32, 33), (3, 3), (0, 1, 1, 0), (1, 1)),                      # classes without a tap in each dimension
+    "s2_dilate2": ((20, 18, 24, 2), (3, 3, 24, 40), (2, 2), (2, 2, 2, 2), (2, 2)),                 # taps reach even positions only
+    "s3_dilate2_uneven": ((21, 23, 40, 2), (4, 3, 40, 36), (3, 2), (3, 0, 1, 4), (2, 3)),
+    "pad_beyond_filter": ((9, 10, 33, 2), (2, 3, 33, 34), (2, 2), (4, 4, 5, 3), (1, 1)),
+    "groups2": ((14, 13, 96, 3), (5, 5, 48, 128), (1, 1), (2, 2, 2, 2), (1, 1)),
+    "groups2_wide_s2": ((15, 11, 80, 2), (3, 3, 40, 300), (2, 2), (1, 1, 1, 1), (1, 1)),           # several column tiles per group
+    "groups4_narrow": ((12, 12, 24, 4), (3, 3, 6, 20), (1, 2), (1, 1, 1, 1), (1, 1)),
+    "many_tiles_s2": ((96, 90, 40, 6), (3, 3, 40, 72), (2, 2), (1, 1, 1, 1), (1, 1)),              # more tiles than SMs: CTAs shared out
+    "s5_falls_back": ((23, 24, 8, 2), (3, 3, 8, 16), (5, 5), (1, 1, 1, 1), (2, 2)),                # 25 classes: more than one launch holds
+}
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 1e-5), (1, 2e-3)])
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_general_gather_vs_oracle(gpu, oracle, case, precision, tol):
+    nn, mat, ctx = gpu
+    xs, fs, stride, pad, dilate = CASES[case]
+    kw = dict(stride=stride, pad=pad, dilate=dilate)
+    rng = np.random.default_rng(sum(xs) + 7 * sum(fs))
+    x = np.asfortranarray(np.maximum(rng.standard_normal(xs), -0.3).astype(np.float32))
+    f = np.asfortranarray((rng.standard_normal(fs) * np.sqrt(2.0 / np.prod(fs[:3]))).astype(np.float32))
+    b = (rng.standard_normal(fs[3]) * 0.1).astype(np.float32)
+    x64, f64, b64 = (a.astype(np.float64) for a in (x, f, b))
+    y_ref = oracle.conv_forward(x64, f64, b64, **kw)
+    dy = np.asfortranarray(rng.standard_normal(y_ref.shape).astype(np.float32))
+    dx_ref, df_ref, db_ref = oracle.conv_backward(x64, f64, dy.astype(np.float64), **kw)
+    xd, fd, bd, dyd = (mat.from_numpy(a) for a in (x, f, b, dy))
+    ctx.set_precision(precision)
+    try:
+        y = nn.vl_nnconv(xd, fd, bd, ctx=ctx, **kw)
+        yr = nn.vl_nnconv(xd, fd, bd, relu=True, ctx=ctx, **kw)
+        dx, df, db = nn.vl_nnconv(xd, fd, bd, dyd, ctx=ctx, **kw)
+        dxm = nn.vl_nnconv(xd, fd, bd, dyd, through_relu=True, no_der_filters=True, no_der_biases=True, ctx=ctx, **kw)[0]
+        assert ctx.device_status() == 0
+        for got, want, name in ((y, y_ref, "y"), (dx, dx_ref, "dx"), (df, df_ref, "df"), (db, db_ref, "db")):
+            assert rel_l2(mat.to_numpy(got).ravel(), np.asarray(want).ravel()) < tol, name
+        assert np.array_equal(mat.to_numpy(yr), np.maximum(mat.to_numpy(y), 0))
+        assert rel_l2(mat.to_numpy(dxm), np.where(x > 0, dx_ref, 0)) < tol
+    finally:
+        ctx.set_precision(0)
