@@ -307,6 +307,15 @@ typedef struct { double rho, epsilon, beta1, beta2; } vlb_solver_opts;
 int vlb_solver_update(vlb_ctx* ctx, int solver, float* W, float* S1, float* S2, float const* G, size_t n, double gradMult,
                       double decay, double lr, vlb_solver_opts const* opts, long long t);
 
+/* The trainer's update of several parameter tensors in one launch (the loop over layers and parameters of
+ * examples/cnn_train.m:451-507), each element as vlb_sgd_update / vlb_solver_update computes it.  The tensors of a list must not
+ * overlap.  S2 is used by adadelta and adam only, t (the step count after this step) by adam only; S1 is the momentum state of
+ * vlb_sgd_update_many. */
+typedef struct { float *W, *S1, *S2; float const* G; size_t n; double decay, lr; long long t; } vlb_param_update;
+int vlb_sgd_update_many(vlb_ctx* ctx, int count, vlb_param_update const* u, double gradMult, double momentum, int nesterov);
+int vlb_solver_update_many(vlb_ctx* ctx, int solver, int count, vlb_param_update const* u, double gradMult,
+                           vlb_solver_opts const* opts);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,7 +1,7 @@
-"""Builds libvlb.so, the C-ABI engine, for sm_100a with nvcc.
+"""Builds libvlb.so, the C-ABI engine, for sm_100a with nvcc, and _hostpath.so, the native host side of nn.py, with g++.
 
-The shared library is written next to this file (in-tree) so that it travels
-with the source tree; it is never installed into site-packages.  There is no
+Both shared libraries are written next to this file (in-tree) so that they travel
+with the source tree; they are never installed into site-packages.  There is no
 fallback of any kind: if nvcc fails, building fails.
 """
 import os
@@ -13,6 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libvlb.so")
+HOST = os.path.join(HERE, "_hostpath.so")
 
 SOURCES = ["ctx.cu", "elementwise.cu", "normalize.cu", "pool.cu", "bnorm.cu", "roipool.cu", "sampler.cu",
            "conv.cu", "conv_simt.cu", "conv_small.cu", "conv_tc.cu"]
@@ -56,8 +57,30 @@ def _compile(src, verbose):
     return obj, log
 
 
+def _build_hostpath(force):
+    """The CPython module of csrc/hostpath.cpp: torch's C++ API for the tensors, libvlb.so (found beside it) for the work."""
+    src = os.path.join(CSRC, "hostpath.cpp")
+    if not force and not _stale(HOST, [src, os.path.join(HERE, "..", "include", "vlb.h")]):
+        return HOST
+    import sysconfig
+    import torch
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    lib = os.path.join(root, "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-attributes",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), src, "-o", HOST]
+    cmd += [f for d in inc for f in ("-isystem", d)]
+    cmd += ["-L" + lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-L" + HERE, "-l:libvlb.so",
+            "-Wl,-rpath," + "$ORIGIN", "-Wl,-rpath," + lib]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError("g++ failed for hostpath.cpp:\n%s\n%s" % (p.stdout, p.stderr))
+    return HOST
+
+
 def build(force=False, verbose=False):
-    """Compile every CUDA source for sm_100a and link libvlb.so; returns its path."""
+    """Compile every CUDA source for sm_100a and link libvlb.so, then the host module; returns the library's path."""
     os.makedirs(OBJ, exist_ok=True)
     if force:
         for f in os.listdir(OBJ):
@@ -75,6 +98,7 @@ def build(force=False, verbose=False):
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (p.stdout, p.stderr))
+    _build_hostpath(force)
     return LIB
 
 

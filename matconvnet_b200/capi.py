@@ -46,6 +46,11 @@ SOLVERS = {"adagrad": 0, "adadelta": 1, "adam": 2, "rmsprop": 3}
 SOLVER_DEFAULTS = {"adagrad": dict(epsilon=1e-10, rho=1.0), "adadelta": dict(epsilon=1e-6, rho=0.9),
                    "adam": dict(beta1=0.9, beta2=0.999, epsilon=1e-8), "rmsprop": dict(epsilon=1e-8, rho=0.99)}
 
+class ParamUpdate(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("W", "S1", "S2", "G")] + [("n", C.c_size_t), ("decay", C.c_double), ("lr", C.c_double),
+                                                                    ("t", C.c_longlong)]
+
+
 _P = C.c_void_p
 _I = C.c_int
 _D = C.c_double
@@ -114,6 +119,8 @@ SIGNATURES = {
     "vlb_softmax_backward": (_I, [_P, _P, _P, _P, _I, _I, _I, _I]),
     "vlb_dropout_mask": (_I, [_P, _P, _Z, _D, C.c_ulonglong]),
     "vlb_mul": (_I, [_P, _P, _P, _P, _Z]),
+    "vlb_sgd_update_many": (_I, [_P, _I, C.POINTER(ParamUpdate), _D, _D, _I]),
+    "vlb_solver_update_many": (_I, [_P, _I, _I, C.POINTER(ParamUpdate), _D, C.POINTER(SolverOpts)]),
     "vlb_solver_update": (_I, [_P, _I, _P, _P, _P, _P, _Z, _D, _D, _D, C.POINTER(SolverOpts), C.c_longlong]),
 }
 
@@ -146,6 +153,7 @@ class Context:
         if rc != 0:
             raise VlbError(rc, "vlb_ctx_create failed (is a B200 the current CUDA device?)")
         self.handle = h
+        self._h = h.value              # the same pointer as the native host side (csrc/hostpath.cpp) takes it
         if stream is not None:
             self.set_stream(stream)
         if precision is not None:
@@ -155,6 +163,7 @@ class Context:
         if getattr(self, "handle", None):
             self.lib.vlb_ctx_destroy(self.handle)
             self.handle = None
+            self._h = 0
 
     def __del__(self):
         try:

@@ -24,32 +24,33 @@ def accumulate_gradients(net, res, state, params, num_workers=1, pulled=None, ct
     res[l]['dzdw'][j] is used as it is (cnn_train.m:459-464).  This function is the one place that divides by
     num_workers (cnn_train.m:455,482), so an exchange built with average=True must not be combined with num_workers > 1."""
     layers = net["layers"]
+    solver, base_lr, base_wd = params.get("solver"), params["learning_rate"], params["weight_decay"]
+    updates = []                      # all parameter tensors of the network are updated by one launch
     for l in range(len(layers) - 1, -1, -1):
         dzdw = res[l]["dzdw"]
         if dzdw is None:
             continue
         layer = layers[l]
+        lr_mults, wd_mults = layer.get("learningRate"), layer.get("weightDecay")
         for j in range(len(dzdw) - 1, -1, -1):
             der = pulled[(l, j)] if pulled is not None and (l, j) in pulled else dzdw[j]
             if der is None:
                 continue
             w = layer["weights"][j]
-            lr_mult = layer.get("learningRate", [1.0] * len(dzdw))[j]
-            wd_mult = layer.get("weightDecay", [1.0] * len(dzdw))[j]
+            lr_mult = lr_mults[j] if lr_mults is not None else 1.0
             if j == 2 and layer["type"] == "bnorm":
                 # moments: w = (1 - lr) * w + lr / numWorkers * der   (cnn_train.m:468-476)
                 nn.vl_taccum(1.0 - lr_mult, w, lr_mult / num_workers, der, out=w, ctx=ctx)
                 continue
-            decay = params["weight_decay"] * wd_mult
-            lr = params["learning_rate"] * lr_mult
+            decay = base_wd * (wd_mults[j] if wd_mults is not None else 1.0)
+            lr = base_lr * lr_mult
             if lr > 0 or decay > 0:
                 key = (l, j)
-                if params.get("solver"):
-                    nn.solver_update_(params["solver"], w, state.setdefault(key, {}), der, 1.0 / num_workers, decay, lr,
-                                      params.get("solver_opts"), ctx=ctx)
-                    continue
                 if key not in state:
-                    state[key] = torch.zeros_like(w)
-                nn.sgd_update_(w, state[key], der, 1.0 / num_workers, decay, params["momentum"], lr,
-                               params.get("nesterov_update", False), ctx=ctx)
+                    state[key] = {} if solver else torch.zeros_like(w)
+                updates.append((w, state[key], der, decay, lr))
+    if updates and solver:
+        nn.solver_update_many_(solver, updates, 1.0 / num_workers, params.get("solver_opts"), ctx)
+    elif updates:
+        nn.sgd_update_many_(updates, 1.0 / num_workers, params["momentum"], params.get("nesterov_update", False), ctx)
     return state
