@@ -6,12 +6,14 @@
 //    VGG-16): each thread owns whole windows, so the backward pass REPLAYS the argmax
 //    scan and overwrites dx with 64/128-bit stores -- no atomics, no zero fill, no
 //    scratch; algorithmic traffic 4*(2*in + out) bytes is also the real traffic.
-//  * everything else: forward = one thread per output; backward = one thread per
-//    INPUT element gathering from the windows that cover it, visited in the
+//  * everything else: tiles in shared memory (pool_fwd_tiled, pool_bwd_tiled); backward is a gather, every
+//    INPUT element visiting the windows that cover it in the
 //    reference's order (wo outer, ho inner), so sums are formed in the same order as
-//    on the CPU and the result is bit-identical and run-to-run deterministic.
+//    on the CPU and the result is bit-identical and run-to-run deterministic.  Columns too long
+//    for a tile take the thread-per-element kernels.
 #include "common.cuh"
 #include <math.h>
+#include <algorithm>
 
 namespace {
 
@@ -102,6 +104,312 @@ __global__ void pool_bwd_generic(float* __restrict__ dx, float const* __restrict
     if (relu) acc = xz[(size_t)u * p.H + v] > 0.f ? acc : 0.f;
     dx[i] = acc;
   }
+}
+
+// ------------------------------------------------------------------ overlapping windows: tiles in shared memory
+// A block takes whole planes, or a strip of columns of one plane, that fit its shared memory: the input is read once, coalesced; a
+// window's arg-max is found once, by one thread, instead of once per input element that the window covers (a 3x3 / stride-2 backward pass
+// scanned every window nine times: 1273 us on 55x55x96x128 where its 334 MB take 51 us; this kernel: 292 us); then every
+// input element adds the derivatives of the windows that chose it, in the reference's order (wo outer, ho inner).
+// Division by a plane extent with a multiply: exact for i * d < 2^32.
+struct FastDiv {
+  unsigned d, m;
+  __host__ FastDiv(int v = 1) : d((unsigned)v), m(v > 1 ? (unsigned)((0x100000000ull + v - 1) / (unsigned)v) : 0u) {}
+  __device__ __forceinline__ int operator()(int i) const { return d == 1 ? i : (int)__umulhi((unsigned)i, m); }
+};
+
+struct TileParams {
+  PoolParams p;
+  int planesPerTile, cols, tilesPerPlane;     // one plane and `cols` columns per tile (backward: of the input, forward: of the output), or several whole planes
+  int xCols, winCols;                         // columns of the input / of windows that a tile holds at most
+  FastDiv H, Ho, sy, sx, xPlane, winPlane, blkPlane, blkRows;    // ..Plane: elements of a tile per plane (planesPerTile > 1)
+};
+
+// A tile's place: first plane, planes, its range of windows [w0, w1) and of input columns [c0, c1).
+struct Tile { size_t z0; int planes, u0, u1, w0, w1, c0, c1; };
+
+__device__ __forceinline__ Tile tile_of(TileParams const& t, bool backward)
+{
+  Tile r;
+  PoolParams const& p = t.p;
+  if (t.planesPerTile > 1) {
+    r.z0 = (size_t)blockIdx.x * t.planesPerTile;
+    r.planes = (int)min((size_t)t.planesPerTile, p.planes - r.z0);
+    r.u0 = 0; r.u1 = p.W; r.w0 = 0; r.w1 = p.Wo; r.c0 = 0; r.c1 = p.W;
+    return r;
+  }
+  r.z0 = blockIdx.x / t.tilesPerPlane;
+  r.planes = 1;
+  int const s = (int)(blockIdx.x - r.z0 * t.tilesPerPlane) * t.cols;
+  if (backward) {
+    r.u0 = s; r.u1 = min(s + t.cols, p.W);
+    r.w0 = max(ceil_div_i(r.u0 + p.padLeft - p.poolW + 1, p.strideX), 0);
+    r.w1 = min((r.u1 - 1 + p.padLeft) / p.strideX + 1, p.Wo);
+  } else {
+    r.w0 = s; r.w1 = min(s + t.cols, p.Wo);
+    r.u0 = r.u1 = 0;
+  }
+  r.c0 = max(r.w0 * p.strideX - p.padLeft, 0);
+  r.c1 = max(r.c0, min((r.w1 - 1) * p.strideX - p.padLeft + p.poolW, p.W));
+  if (backward && r.w1 > r.w0) { r.c0 = min(r.c0, r.u0); r.c1 = max(r.c1, r.u1); }      // (the ReLU mask reads the tile's own elements too)
+  if (r.w1 <= r.w0) { r.w1 = r.w0; r.c0 = r.u0; r.c1 = r.u1; }
+  return r;
+}
+
+// The columns [c0, c1) of `planes` planes of x into shared memory.  Whole planes are one contiguous run.
+__device__ __forceinline__ void load_tile(float* xs, float const* __restrict__ x, TileParams const& t, Tile const& r)
+{
+  size_t const plane = (size_t)t.p.H * t.p.W;
+  int const n = t.planesPerTile > 1 ? r.planes * (int)plane : (r.c1 - r.c0) * t.p.H;
+  float const* const src = x + r.z0 * plane + (size_t)r.c0 * t.p.H;
+  for (int i = threadIdx.x; i < n; i += 4 * kThreads) {
+    float v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = i + k * kThreads < n ? __ldg(src + i + k * kThreads) : 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) if (i + k * kThreads < n) xs[i + k * kThreads] = v[k];
+  }
+}
+
+struct Window { int x1, x2, y1, y2; };
+
+__device__ __forceinline__ Window window_of(PoolParams const& p, int ho, int wo)
+{
+  Window w;
+  w.x1 = wo * p.strideX - p.padLeft; w.y1 = ho * p.strideY - p.padTop;
+  w.x2 = min(w.x1 + p.poolW, p.W); w.y2 = min(w.y1 + p.poolH, p.H);
+  w.x1 = max(w.x1, 0); w.y1 = max(w.y1, 0);
+  return w;
+}
+
+template <bool kMax>
+__global__ void __launch_bounds__(kThreads) pool_fwd_tiled(float* __restrict__ y, float const* __restrict__ x, const __grid_constant__ TileParams t)
+{
+  extern __shared__ float xs[];
+  PoolParams const& p = t.p;
+  Tile const r = tile_of(t, false);
+  load_tile(xs, x, t, r);
+  __syncthreads();
+  int const wp = (r.w1 - r.w0) * p.Ho, n = r.planes * wp;
+  float* const yp = y + (r.z0 * p.Wo + r.w0) * (size_t)p.Ho;              // (several planes: w0 = 0, so the outputs are contiguous too)
+  for (int i = threadIdx.x; i < n; i += kThreads) {
+    int const pl = t.planesPerTile > 1 ? t.winPlane(i) : 0, q = i - pl * wp, wl = t.Ho(q), ho = q - wl * p.Ho;
+    Window const w = window_of(p, ho, r.w0 + wl);
+    float const* const xp = xs + (t.planesPerTile > 1 ? pl * p.H * p.W : 0);
+    if (kMax) {
+      float best = -INFINITY;
+      for (int u = w.x1; u < w.x2; ++u)
+        for (int v = w.y1; v < w.y2; ++v) { float const a = xp[(u - r.c0) * p.H + v]; best = (best < a) ? a : best; }
+      yp[i] = best;
+    } else {
+      float s = 0.f;
+      for (int u = w.x1; u < w.x2; ++u)
+        for (int v = w.y1; v < w.y2; ++v) s = __fadd_rn(s, xp[(u - r.c0) * p.H + v]);
+      yp[i] = __fmul_rn(s, __fdiv_rn(1.f, (float)((w.y2 - w.y1) * (w.x2 - w.x1))));
+    }
+  }
+}
+
+// relu: as for pool_bwd_generic.
+template <bool kMax>
+__global__ void __launch_bounds__(kThreads) pool_bwd_tiled(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ dy,
+                                                           const __grid_constant__ TileParams t, bool relu)
+{
+  extern __shared__ float smem[];
+  PoolParams const& p = t.p;
+  Tile const r = tile_of(t, true);
+  bool const needX = kMax || relu;
+  float* const xs = smem;                                               // [planes][columns][H]
+  float* const ds = smem + (needX ? t.planesPerTile * t.xCols * p.H : 0);      // derivative of each window (average: times its scale)
+  int* const arg = reinterpret_cast<int*>(ds + t.planesPerTile * t.winCols * p.Ho);      // arg-max of each window, as an index into the plane's part of xs
+  if (needX) load_tile(xs, x, t, r);
+  if (kMax) __syncthreads();
+  int const wp = (r.w1 - r.w0) * p.Ho, nWin = r.planes * wp;
+  float const* const dyp = dy + (r.z0 * p.Wo + r.w0) * (size_t)p.Ho;
+  for (int i = threadIdx.x; i < nWin; i += kThreads) {
+    float const d = __ldg(dyp + i);
+    int const pl = t.planesPerTile > 1 ? t.winPlane(i) : 0, q = i - pl * wp, wl = t.Ho(q), ho = q - wl * p.Ho;
+    Window const w = window_of(p, ho, r.w0 + wl);
+    if (kMax) {
+      float const* const xp = xs + (t.planesPerTile > 1 ? pl * p.H * p.W : 0);
+      // the reference's scan: column-outer, row-inner, first strictly greater wins
+      float best = -INFINITY;
+      int at = -1;
+      for (int u = w.x1; u < w.x2; ++u)
+        for (int v = w.y1; v < w.y2; ++v) {
+          int const k = (u - r.c0) * p.H + v;
+          float const a = xp[k];
+          if (a > best) { best = a; at = k; }
+        }
+      ds[i] = d;
+      arg[i] = at;
+    } else {
+      ds[i] = __fmul_rn(d, __fdiv_rn(1.f, (float)((w.y2 - w.y1) * (w.x2 - w.x1))));
+    }
+  }
+  __syncthreads();
+  int const xp = (r.u1 - r.u0) * p.H, n = r.planes * xp;
+  float* const out = dx + (r.z0 * p.W + r.u0) * (size_t)p.H;
+  for (int i = threadIdx.x; i < n; i += kThreads) {
+    int const pl = t.planesPerTile > 1 ? t.xPlane(i) : 0, q = i - pl * xp, ul = t.H(q), v = q - ul * p.H, u = r.u0 + ul;
+    int const self = (u - r.c0) * p.H + v;
+    int const hb = v + p.padTop - p.poolH + 1, wb = u + p.padLeft - p.poolW + 1;
+    int const ho0 = hb > 0 ? t.sy(hb + p.strideY - 1) : 0, ho1 = min(t.sy(v + p.padTop), p.Ho - 1);
+    int const wo0 = wb > 0 ? t.sx(wb + p.strideX - 1) : 0, wo1 = min(t.sx(u + p.padLeft), p.Wo - 1);
+    float acc = 0.f;
+    for (int wo = wo0; wo <= wo1; ++wo)
+      for (int ho = ho0; ho <= ho1; ++ho) {
+        int const k = pl * wp + (wo - r.w0) * p.Ho + ho;
+        if (!kMax || arg[k] == self) acc = __fadd_rn(acc, ds[k]);
+      }
+    if (relu) acc = xs[(t.planesPerTile > 1 ? pl * p.H * p.W : 0) + self] > 0.f ? acc : 0.f;
+    out[i] = acc;
+  }
+}
+
+// 3x3 windows two apart (AlexNet, CIFAR, ResNet): pool_bwd_tiled's general loops cost about 130 instructions per element there.  A
+// thread finds a window's arg-max with the nine reads unrolled; then it takes the 2 x 2 elements around (2k - padTop, 2l - padLeft),
+// which only the windows (k-1..k, l-1..l) reach -- four arg-maxima and four derivatives for four elements -- from tables with a border of
+// "no window", and the result leaves through shared memory in whole lines.  55x55x96x128: 1273 us (generic), 292 (tiled), 132 (this).
+template <bool kMax>
+__global__ void __launch_bounds__(kThreads) pool33_bwd_tiled(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ dy,
+                                                             const __grid_constant__ TileParams t, bool relu)
+{
+  extern __shared__ float smem[];
+  PoolParams const& p = t.p;
+  Tile const r = tile_of(t, true);
+  int const H = p.H, Ho = p.Ho, Hw = Ho + 2;                             // window tables: rows -1 .. Ho, columns w0-1 .. w1
+  int const xPer = t.planesPerTile > 1 ? H * p.W : 0, wCols = r.w1 - r.w0, tab = (wCols + 2) * Hw;
+  float* const xs = smem;
+  float* const ds = smem + t.planesPerTile * t.xCols * H;
+  int* const arg = reinterpret_cast<int*>(ds + t.planesPerTile * (t.winCols + 2) * Hw);
+  if (kMax || relu) load_tile(xs, x, t, r);
+  for (int i = threadIdx.x; i < r.planes * tab; i += kThreads) { ds[i] = 0.f; if (kMax) arg[i] = -1; }
+  __syncthreads();
+  int const wp = wCols * Ho, nWin = r.planes * wp;
+  float const* const dyp = dy + (r.z0 * p.Wo + r.w0) * (size_t)Ho;
+  for (int i = threadIdx.x; i < nWin; i += kThreads) {
+    float const d = __ldg(dyp + i);
+    int const pl = t.planesPerTile > 1 ? t.winPlane(i) : 0, q = i - pl * wp, wl = t.Ho(q), ho = q - wl * Ho;
+    int const x1 = 2 * (r.w0 + wl) - p.padLeft, y1 = 2 * ho - p.padTop, k = pl * tab + (wl + 1) * Hw + ho + 1;
+    if (kMax) {
+      float const* const xp = xs + pl * xPer;
+      float best = -INFINITY;
+      int at = -1;
+      int const base = (x1 - r.c0) * H + y1;
+      if (x1 >= 0 && y1 >= 0 && x1 + 3 <= p.W && y1 + 3 <= H) {
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+#pragma unroll
+          for (int v = 0; v < 3; ++v) {
+            float const a = xp[base + u * H + v];
+            if (a > best) { best = a; at = base + u * H + v; }
+          }
+      } else {
+        for (int u = max(-x1, 0); u < min(3, p.W - x1); ++u)
+          for (int v = max(-y1, 0); v < min(3, H - y1); ++v) {
+            float const a = xp[base + u * H + v];
+            if (a > best) { best = a; at = base + u * H + v; }
+          }
+      }
+      ds[k] = d;
+      arg[k] = at;
+    } else {
+      int const n = (min(x1 + 3, p.W) - max(x1, 0)) * (min(y1 + 3, H) - max(y1, 0));
+      ds[k] = __fmul_rn(d, __fdiv_rn(1.f, (float)n));
+    }
+  }
+  __syncthreads();
+  // blocks of 2 x 2 elements: rows 2k - padTop + {0, 1}, columns 2l - padLeft + {0, 1}, from the first block that touches the tile
+  int const k0 = p.padTop >> 1, kN = ((H - 1 + p.padTop) >> 1) - k0 + 1;
+  int const l0 = (r.u0 + p.padLeft) >> 1, lN = ((r.u1 - 1 + p.padLeft) >> 1) - l0 + 1, blk = kN * lN;
+  for (int i = threadIdx.x; i < r.planes * blk; i += kThreads) {
+    int const pl = t.planesPerTile > 1 ? t.blkPlane(i) : 0, q = i - pl * blk, ll = t.blkRows(q), k = k0 + q - ll * kN, l = l0 + ll;
+    int const v0 = 2 * k - p.padTop, u0 = 2 * l - p.padLeft;
+    // table entries of the windows (k-1, k) x (l-1, l); windows below or right of the last one are border
+    int const ka = min(k - 1, Ho) + 1, kb = min(k, Ho) + 1, la = min(max(l - 1 - r.w0, -1), wCols) + 1, lb = min(max(l - r.w0, -1), wCols) + 1;
+    int const w00 = pl * tab + la * Hw + ka, w01 = pl * tab + la * Hw + kb, w10 = pl * tab + lb * Hw + ka, w11 = pl * tab + lb * Hw + kb;
+    float const d00 = ds[w00], d01 = ds[w01], d10 = ds[w10], d11 = ds[w11];
+    int a00 = 0, a01 = 0, a10 = 0, a11 = 0;
+    if (kMax) { a00 = arg[w00]; a01 = arg[w01]; a10 = arg[w10]; a11 = arg[w11]; }
+    float* const xp = xs + pl * xPer;
+    int const s = (u0 - r.c0) * H + v0;
+    // (the order of the reference: wo outer, ho inner; an absent window of an average adds its zero, which changes no sum)
+    auto put = [&](int u, int v, int self, float acc) {
+      if ((unsigned)v < (unsigned)H && u >= r.u0 && u < r.u1) xp[self] = relu && !(xp[self] > 0.f) ? 0.f : acc;
+    };
+    float acc = 0.f;
+    if (!kMax || a00 == s) acc = __fadd_rn(acc, d00);
+    if (!kMax || a01 == s) acc = __fadd_rn(acc, d01);
+    if (!kMax || a10 == s) acc = __fadd_rn(acc, d10);
+    if (!kMax || a11 == s) acc = __fadd_rn(acc, d11);
+    put(u0, v0, s, acc);
+    acc = 0.f;
+    if (!kMax || a01 == s + 1) acc = __fadd_rn(acc, d01);
+    if (!kMax || a11 == s + 1) acc = __fadd_rn(acc, d11);
+    put(u0, v0 + 1, s + 1, acc);
+    acc = 0.f;
+    if (!kMax || a10 == s + H) acc = __fadd_rn(acc, d10);
+    if (!kMax || a11 == s + H) acc = __fadd_rn(acc, d11);
+    put(u0 + 1, v0, s + H, acc);
+    acc = 0.f;
+    if (!kMax || a11 == s + H + 1) acc = __fadd_rn(acc, d11);
+    put(u0 + 1, v0 + 1, s + H + 1, acc);
+  }
+  __syncthreads();
+  int const n = r.planes * (r.u1 - r.u0) * H, off = (r.u0 - r.c0) * H;
+  float* const out = dx + (r.z0 * p.W + r.u0) * (size_t)H;
+  for (int i = threadIdx.x; i < n; i += kThreads) out[i] = xs[off + i];
+}
+
+// Tile sizes for a shared-memory budget that leaves six blocks of 256 threads per SM; false when not even the narrowest strip fits it
+// (columns of thousands of rows: the generic kernels).
+constexpr size_t kTileBytes = 36 * 1024;
+
+bool is_33s2(PoolParams const& p) { return p.poolH == 3 && p.poolW == 3 && p.strideY == 2 && p.strideX == 2; }
+
+bool plan_tiles(PoolParams const& p, bool backward, bool needX, bool max, TileParams* t, size_t* smem, unsigned* grid)
+{
+  bool const t33 = backward && is_33s2(p);         // (its result passes through the x tile, its window tables have a border)
+  if (t33) needX = true;
+  size_t const winBytes = backward ? (max ? 8 : 4) : 0;
+  // (planned as if x were always loaded, which also bounds the elements per tile)
+  auto bytes = [&](int xCols, int winCols) { return (size_t)xCols * p.H * 4 + (t33 ? (size_t)(winCols + 2) * (p.Ho + 2) : (size_t)winCols * p.Ho) * winBytes; };
+  t->p = p;
+  // the multiply-for-division of the stride: positions reach H + padTop and W + padLeft
+  auto divides = [](long long extent, long long pad, long long pool, long long stride) { return (extent + pad + pool + stride) * stride < (1LL << 31); };
+  if (!divides(p.H, p.padTop, p.poolH, p.strideY) || !divides(p.W, p.padLeft, p.poolW, p.strideX)) return false;
+  size_t const whole = bytes(p.W, p.Wo);
+  t->cols = backward ? p.W : p.Wo; t->tilesPerPlane = 1; t->xCols = p.W; t->winCols = p.Wo;
+  t->planesPerTile = 1;
+  if (whole <= kTileBytes) {
+    // several small planes per block: at least 1024 elements of work, as long as there are blocks enough for the chip
+    size_t const elems = (size_t)(backward ? p.H * p.W : p.Ho * p.Wo);
+    size_t n = std::min<size_t>(kTileBytes / std::max<size_t>(whole, 1), std::max<size_t>(1, 2048 / elems));
+    while (n > 1 && (p.planes + n - 1) / n < 148 * 4) n = (n + 1) / 2;
+    if (n * std::max((size_t)p.H * p.W, (size_t)p.Ho * p.Wo) < 65536) t->planesPerTile = (int)std::max<size_t>(1, n);
+  } else {
+    auto fits = [&](int cols, int* xc, int* wc) {
+      if (backward) { *wc = std::min(p.Wo, (cols + p.poolW - 2) / p.strideX + 2); *xc = std::min(p.W, cols + 2 * (p.poolW - 1)); }
+      else          { *wc = cols; *xc = std::min(p.W, (cols - 1) * p.strideX + p.poolW); }
+      return bytes(*xc, *wc) <= kTileBytes;
+    };
+    int cols = t->cols, xc = 0, wc = 0;
+    while (cols > 1 && !fits(cols, &xc, &wc)) cols = (cols + 1) / 2;
+    if (!fits(cols, &xc, &wc)) return false;
+    t->cols = cols; t->xCols = xc; t->winCols = wc;
+    t->tilesPerPlane = ((backward ? p.W : p.Wo) + cols - 1) / cols;
+  }
+  size_t const blocks = t->planesPerTile > 1 ? (p.planes + t->planesPerTile - 1) / t->planesPerTile : p.planes * t->tilesPerPlane;
+  if (blocks >= (1u << 31) || (long long)t->winCols * p.Ho * p.Ho >= (1LL << 32)) return false;
+  *grid = (unsigned)blocks;
+  *smem = (bytes(t->xCols, t->winCols) - (needX ? 0 : (size_t)t->xCols * p.H * 4)) * t->planesPerTile;
+  // the 2 x 2 blocks of pool33_bwd_tiled (the plane's decomposition is only used with whole planes)
+  int const kN = ((p.H - 1 + p.padTop) >> 1) - (p.padTop >> 1) + 1, lN = ((p.W - 1 + p.padLeft) >> 1) - (p.padLeft >> 1) + 1;
+  t->blkRows = FastDiv(kN); t->blkPlane = FastDiv(kN * lN);
+  t->H = FastDiv(p.H); t->Ho = FastDiv(p.Ho); t->sy = FastDiv(p.strideY); t->sx = FastDiv(p.strideX);
+  t->xPlane = FastDiv(p.H * p.W); t->winPlane = FastDiv(p.Ho * p.Wo);
+  return true;
 }
 
 // ------------------------------------------------------------------ 2x2 / stride 2 fast path
@@ -266,7 +574,19 @@ int pool_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, vlb_
               else       launch2x2_bwd<1, false>(ctx, grid, dX, X, dY, d->H, d->W, planes, relu); }
   } else {
     PoolParams p = {d->H, d->W, Ho, Wo, d->poolH, d->poolW, d->strideY, d->strideX, d->padTop, d->padLeft, planes};
-    unsigned grid = vlb::grid_for(planes * (size_t)d->H * d->W, kThreads, ctx->smCount * 16);
+    TileParams t;
+    size_t smem = 0;
+    unsigned grid = 0;
+    if (plan_tiles(p, true, isMax || relu, isMax, &t, &smem, &grid)) {
+      bool const t33 = is_33s2(p);
+      if (t33 && isMax) pool33_bwd_tiled<true><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
+      else if (t33)     pool33_bwd_tiled<false><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
+      else if (isMax)   pool_bwd_tiled<true><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
+      else              pool_bwd_tiled<false><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
+      VLB_LAUNCHED(ctx, 1);
+      return vlb::check_launch(ctx, where);
+    }
+    grid = vlb::grid_for(planes * (size_t)d->H * d->W, kThreads, ctx->smCount * 16);
     if (isMax) pool_bwd_generic<true><<<grid, kThreads, 0, ctx->stream>>>(dX, X, dY, p, relu);
     else       pool_bwd_generic<false><<<grid, kThreads, 0, ctx->stream>>>(dX, X, dY, p, relu);
   }
@@ -305,7 +625,16 @@ int vlb_pool_forward(vlb_ctx* ctx, float* Y, float const* X, vlb_pool_desc const
               else       pool2x2_fwd<1, false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, d->H, d->W, planes); }
   } else {
     PoolParams p = {d->H, d->W, Ho, Wo, d->poolH, d->poolW, d->strideY, d->strideX, d->padTop, d->padLeft, planes};
-    unsigned grid = vlb::grid_for(planes * (size_t)Ho * Wo, kThreads, ctx->smCount * 16);
+    TileParams t;
+    size_t smem = 0;
+    unsigned grid = 0;
+    if (plan_tiles(p, false, true, isMax, &t, &smem, &grid)) {
+      if (isMax) pool_fwd_tiled<true><<<grid, kThreads, smem, ctx->stream>>>(Y, X, t);
+      else       pool_fwd_tiled<false><<<grid, kThreads, smem, ctx->stream>>>(Y, X, t);
+      VLB_LAUNCHED(ctx, 1);
+      return vlb::check_launch(ctx, "vlb_pool_forward");
+    }
+    grid = vlb::grid_for(planes * (size_t)Ho * Wo, kThreads, ctx->smCount * 16);
     if (isMax) pool_fwd_generic<true><<<grid, kThreads, 0, ctx->stream>>>(Y, X, p);
     else       pool_fwd_generic<false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, p);
   }
