@@ -34,6 +34,10 @@ struct vlb_ctx {
   // where reluMask (the convolution's input, a ReLU's output) is not positive and says so, otherwise the caller masks dX
   float const* reluMask = nullptr;
   bool maskDone = false;
+  // set by vlb_convt_forward around its call of the data gradient that computes it: the path that ran adds this bias per channel of dX
+  // in its epilogue and says so, otherwise the caller adds it in a pass of its own
+  float const* dgradBias = nullptr;
+  bool biasDone = false;
   bool profiling = false;
   std::vector<ProfRec> prof;
   // vlb_ctx_set_test_switch: bit 0 makes the filter-tile loader of the tensor-memory convolution kernel stay idle, so that

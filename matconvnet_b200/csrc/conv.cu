@@ -58,24 +58,9 @@ conv_dbias_kernel(float* __restrict__ db, float const* __restrict__ dy, int P, i
   cluster.sync();
 }
 
-// The same for 1x1 outputs (fully connected layers): db[k] = sum over images of dy[k + K*n]; one thread per
-// filter, reads coalesced across the filters, images added in order.
-__global__ void conv_dbias_p1_kernel(float* __restrict__ db, float const* __restrict__ dy, int K, int N)
-{
-  int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= K) return;
-  float s = 0.f;
-  for (int n = 0; n < N; ++n) s += dy[(size_t)n * K + k];
-  db[k] = s;
-}
-
 int launch_dbias(vlb_ctx* ctx, float* db, float const* dY, int P, int K, int N)
 {
-  if (P == 1) {
-    conv_dbias_p1_kernel<<<vlb::ceil_div(K, 128), 128, 0, ctx->stream>>>(db, dY, K, N);
-    VLB_LAUNCHED(ctx, 1);
-    return vlb::check_launch(ctx, "conv_dbias");
-  }
+  if (P == 1) return vlb::sum_parts(ctx, db, dY, K, K, N);      // 1x1 outputs (fully connected layers): db[k] = sum over images of dy[k + K*n]
   bool vec = (P % 4 == 0) && ((((uintptr_t)dY) & 15) == 0);
   dim3 grid(K, kCluster);
   if (vec) conv_dbias_kernel<true><<<grid, kThreads, 0, ctx->stream>>>(db, dY, P, K, N);
@@ -260,8 +245,11 @@ int vlb_convt_forward(vlb_ctx* ctx, float* Y, float const* X, float const* F, fl
   VLB_REQUIRE(ctx, Y && X && F, "convt_forward: null tensor");
   // the whole batch in one call: this engine's data gradient writes every image's own slice (the reference loops over
   // the images because its row2im accumulates, bits/nnconv.cu:338-367)
+  ctx->dgradBias = b; ctx->biasDone = false;
   rc = vlb_conv_backward(ctx, Y, nullptr, nullptr, nullptr, F, X, &c);
-  if (rc || !b) return rc;
+  bool const done = ctx->biasDone;
+  ctx->dgradBias = nullptr; ctx->biasDone = false;
+  if (rc || !b || done) return rc;
   return vlb_bias_forward(ctx, Y, 1.0, nullptr, 0.0, b, 1.0, c.H, c.W, c.C, c.N);       // bits/nnconv.cu:368-370
 }
 
@@ -283,7 +271,7 @@ int vlb_convt_backward(vlb_ctx* ctx, float* dX, float* dF, float* db, float cons
     rc = vlb_conv_backward(ctx, nullptr, dF, nullptr, dY, nullptr, X, &c);
     if (rc) return rc;
   }
-  if (db) return vlb_bias_backward(ctx, nullptr, 0.0, db, 0.0, 0.0, 1.0, dY, c.H, c.W, c.C, c.N);      // :411-414
+  if (db) return launch_dbias(ctx, db, dY, c.H * c.W, c.C, c.N);      // :411-414
   return VLB_Success;
 }
 

@@ -13,6 +13,17 @@ struct ConvGeom {
   int G, Kg;        // groups = C / FC, filters per group = K / G
 };
 
+// out[i] = act(inMult * (sum over k ascending of part[k*stride + i]) + bias[i/P % K] + outMult*out[i]), zeroed where mask is not
+// positive (reduce.cu); the defaults are the plain sum.
+struct SumEpilogue {
+  float const* bias = nullptr;
+  int P = 1, K = 1;
+  float inMult = 1.f, outMult = 0.f;
+  int relu = 0;
+  float const* mask = nullptr;
+};
+int sum_parts(vlb_ctx* ctx, float* out, float const* part, size_t n, size_t stride, int parts, SumEpilogue const& e = SumEpilogue());
+
 // CUDA-core implicit GEMM (conv_simt.cu): every configuration, exact fp32 products.
 int conv_fprop_simt(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, float const* X, float inMult,
                     float const* F, float const* b);
@@ -25,6 +36,9 @@ int conv_fprop_small(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, f
                      float const* F, float const* b);
 int conv_dgrad_small(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY);
 int conv_wgrad_small(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float const* X, float const* dY, bool* dbDone);
+
+// Fully connected forward pass of at most 8 images on CUDA cores (fc_small.cu).
+int fc_fprop_small(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float const* F, float const* b);
 
 // tcgen05 implicit GEMM (conv_tc.cu).  Each returns VLB_Unsupported -- without touching
 // the context's error state -- when the configuration is outside what the tensor-core

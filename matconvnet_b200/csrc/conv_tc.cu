@@ -1907,17 +1907,6 @@ __global__ void __launch_bounds__(kTsThreads, 1) conv_ts_gen_kernel(const __grid
   conv_ts_body<kSplit, 0, kNarrow, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
 }
 
-// out[e] = sum over splits (ascending) of part[s*stride + e]
-__global__ void tc_splitk_reduce_kernel(float* __restrict__ out, float const* __restrict__ part, size_t n, size_t stride, int splits)
-{
-  size_t step = (size_t)gridDim.x * blockDim.x;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += step) {
-    float s = part[e];
-    for (int k = 1; k < splits; ++k) s += part[(size_t)k * stride + e];
-    out[e] = s;
-  }
-}
-
 // Ft[fh', fw', k, c] = F[FH-1-fh', FW-1-fw', c, k]: the filter bank whose forward convolution
 // over dY is the data gradient of a stride-1 convolution.
 __global__ void flip_filters_kernel(float* __restrict__ ft, float const* __restrict__ f, int FH, int FW, int C, int K)
@@ -2417,6 +2406,16 @@ int pick_wg_splits(int smCount, int tiles, int numKb, int* kbPerSplit, int minKb
   return vlb::ceil_div(numKb, *kbPerSplit);
 }
 
+// A forward or data-gradient contraction with fewer output tiles than SMs leaves most of the chip idle for the length of its whole reduction
+// (one image through VGG-16's 28 x 28 layers: 28 tiles of 144 k-blocks): its reduction is cut into ranges as the filter gradients' are,
+// and sum_parts adds them and applies the epilogue.  Returns the number of ranges; 1: left alone.
+int split_few_tiles(int smCount, int tiles, int numKb, int* kbPerSplit)
+{
+  *kbPerSplit = numKb;
+  if (tiles * 4 > smCount * 5 || numKb < 12) return 1;
+  return pick_wg_splits(smCount, tiles, numKb, kbPerSplit, 6);
+}
+
 void conv_operand(Operand& o, ConvGeom const& g, float const* ptr, int channels)
 {
   o.ptr = ptr;
@@ -2533,11 +2532,7 @@ int conv_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
   p.e.out = part ? part : dF; p.e.splitStride = part ? (long long)nF : 0; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.K;
   int const rc = launch_rows(ctx, p, map, "conv_wgrad_ts");
   if (rc) return rc;
-  if (part) {
-    tc_splitk_reduce_kernel<<<vlb::grid_for(nF, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(dF, part, nF, nF, p.splits);
-    VLB_LAUNCHED(ctx, 1);
-  }
-  return vlb::check_launch(ctx, "conv_wgrad_ts");
+  return part ? vlb::sum_parts(ctx, dF, part, nF, nF, p.splits) : VLB_Success;
 }
 
 // The geometry of a 1 x 1 convolution over a "plane" of `pixels` elements with `channels` channels (channel stride = pixels).
@@ -2583,12 +2578,10 @@ int fc_fprop_ts(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float
   p.e.out = part ? part : Y; p.e.splitStride = part ? (long long)nOut : 0; p.e.inMult = 1.f; p.e.P = g.K; p.e.Ktot = g.N;
   int rc = launch_rows(ctx, p, map, "fc_fprop_ts");
   if (rc) return rc;
-  if (part) {
-    tc_splitk_reduce_kernel<<<vlb::grid_for(nOut, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(Y, part, nOut, nOut, p.splits);
-    VLB_LAUNCHED(ctx, 1);
-  }
-  if (b) return vlb_bias_forward(ctx, Y, 1.0, nullptr, 0.0, b, 1.0, 1, 1, g.K, g.N);
-  return vlb::check_launch(ctx, "fc_fprop_ts");
+  if (!part) return b ? vlb_bias_forward(ctx, Y, 1.0, nullptr, 0.0, b, 1.0, 1, 1, g.K, g.N) : VLB_Success;
+  vlb::SumEpilogue epi;
+  epi.bias = b; epi.K = g.K; epi.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
+  return vlb::sum_parts(ctx, Y, part, nOut, nOut, p.splits, epi);
 }
 
 int fc_dgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
@@ -2614,11 +2607,10 @@ int fc_dgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, floa
   float* const part = p.splits > 1 ? (float*)((char*)p.bTiles + b_tiles_bytes(ctx, g.N, p.BN, p.numKb)) : nullptr;
   p.e = Epilogue{};
   p.e.out = part ? part : dX; p.e.splitStride = part ? (long long)nOut : 0; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.N;
+  vlb::SumEpilogue epi;
+  (part ? epi.mask : p.e.mask) = ctx->reluMask; ctx->maskDone = ctx->reluMask != nullptr;
   int rc = launch_ts(ctx, p, "fc_dgrad_ts");
-  if (rc || !part) return rc;
-  tc_splitk_reduce_kernel<<<vlb::grid_for(nOut, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(dX, part, nOut, nOut, p.splits);
-  VLB_LAUNCHED(ctx, 1);
-  return vlb::check_launch(ctx, "fc_dgrad_ts");
+  return rc || !part ? rc : vlb::sum_parts(ctx, dX, part, nOut, nOut, p.splits, epi);
 }
 
 int fc_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, float const* dY)
@@ -2695,7 +2687,10 @@ double gen_cost(int tiles, int numKb, int BN)
 }
 
 // Builds the tile images of all problems (one launch) and runs them (one launch).  The problems share the tile width.
-int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, char const* where)
+// Where the problems' tiles are too few for the chip the reductions are cut, all into the same number of ranges, and `fin` (the epilogue,
+// which the problems then do not apply themselves) goes to the sum over the ranges; they cover every element of the output then
+// (`covered`).
+int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size_t nOut, vlb::SumEpilogue const& fin, bool covered, char const* where)
 {
   bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
   int const BN = b.p[0].BN;
@@ -2704,35 +2699,51 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, char const* wher
   long long tiles = 0;
   int rows = 0, kbGroups = 0;
   double work = 0;
+  int splits = 1;
+  {
+    long long t = 0, kb = 0;
+    for (int i = 0; i < b.n; ++i) { long long const ti = (long long)b.p[i].tilesM * b.p[i].tilesN; t += ti; kb += ti * b.p[i].numKb; }
+    int per;
+    if (covered && t < (1 << 20)) splits = split_few_tiles(ctx->smCount, (int)t, (int)(kb / t), &per);
+  }
   for (int i = 0; i < b.n; ++i) {
     Params& p = b.p[i];
+    p.splits = splits; p.kbPerSplit = vlb::ceil_div(p.numKb, splits);
+    p.numKb = p.kbTot = p.splits * p.kbPerSplit;
+    prep.p[i].numKb = p.numKb;
+    // few blocks of many k-blocks each would be all latency
+    while (prep.p[i].per > 1 && (long long)vlb::ceil_div(prep.p[i].rows, 32) * vlb::ceil_div(p.numKb, prep.p[i].per) * b.n < 2 * ctx->smCount) prep.p[i].per = (prep.p[i].per + 1) / 2;
+    p.e.out = out;
+    if (splits > 1) p.e.splitStride = (long long)nOut;
+    else { p.e.bias = fin.bias; p.e.inMult = fin.inMult; p.e.outMult = fin.outMult; p.e.relu = fin.relu; p.e.mask = fin.mask; }
     prep.p[i].out = (float*)total;                 // offset for now
     total += (sizeof(float) * (size_t)p.tilesN * BN * (size_t)p.numKb * 32 * (split3 ? 2 : 1) + 255) & ~(size_t)255;
     rows = std::max(rows, prep.p[i].rows); kbGroups = std::max(kbGroups, vlb::ceil_div(prep.p[i].numKb, prep.p[i].per));
     p.smemSum = ((ctx->testSwitch & 8) || p.kbPerSplit < 8) ? 1 : 0;
     sumBytes = std::max(sumBytes, p_bytes(BN, p.smemSum));
-    long long const t = (long long)p.tilesM * p.tilesN;
+    long long const t = (long long)p.tilesM * p.tilesN * p.splits;
     tiles += t;
-    work += (double)t * (p.numKb + 6);
+    work += (double)t * (p.kbPerSplit + 6);
     if (t >= (1LL << 31)) return VLB_Unsupported;
   }
-  char* const ws = (char*)vlb::workspace(ctx, total);
+  char* const ws = (char*)vlb::workspace(ctx, total + (splits > 1 ? sizeof(float) * nOut * splits : 0));
   if (!ws) return ctx->lastError;
+  float* const part = (float*)(ws + total);
   // CTAs per problem: one per tile when all tiles fit, else shares of the chip in proportion to the work, the rest to the longest queues
   int given = 0;
   for (int i = 0; i < b.n; ++i) {
     Params& p = b.p[i];
-    long long const t = (long long)p.tilesM * p.tilesN;
+    long long const t = (long long)p.tilesM * p.tilesN * p.splits;
     p.ctas = tiles <= ctx->smCount ? (int)t
-             : (int)std::min<long long>(t, std::max(1, (int)((double)ctx->smCount * (double)t * (p.numKb + 6) / work)));
+             : (int)std::min<long long>(t, std::max(1, (int)((double)ctx->smCount * (double)t * (p.kbPerSplit + 6) / work)));
     given += p.ctas;
   }
   while (tiles > ctx->smCount && given < ctx->smCount) {
     int worst = -1; double most = 0;
     for (int i = 0; i < b.n; ++i) {
       Params const& p = b.p[i];
-      long long const t = (long long)p.tilesM * p.tilesN;
-      double const queue = (double)((t + p.ctas - 1) / p.ctas) * (p.numKb + 6);
+      long long const t = (long long)p.tilesM * p.tilesN * p.splits;
+      double const queue = (double)((t + p.ctas - 1) / p.ctas) * (p.kbPerSplit + 6);
       if (p.ctas < t && queue > most) { most = queue; worst = i; }
     }
     if (worst < 0) break;
@@ -2744,6 +2755,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, char const* wher
     p.ctaBeg = beg; beg += p.ctas;
     prep.p[i].out = (float*)(ws + (size_t)prep.p[i].out);
     p.bTiles = prep.p[i].out;
+    if (splits > 1) p.e.out = part;
     p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;
   }
   dim3 const pgrid(vlb::ceil_div(rows, 32), kbGroups, b.n);
@@ -2762,7 +2774,8 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, char const* wher
 #undef VLB_TSG
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 2);
-  return vlb::check_launch(ctx, where);
+  int const rc = vlb::check_launch(ctx, where);
+  return rc || splits == 1 ? rc : vlb::sum_parts(ctx, out, part, nOut, nOut, splits, fin);
 }
 
 // Forward convolution through the general gather: any channel count, stride, dilation, filter groups.
@@ -2773,11 +2786,12 @@ int conv_fprop_gen(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, flo
   ts.n = 1;
   Params& p = ts.p[0];
   gen_problem(p, g, X, g.FC, g.G, g.Kg, pick_bn(g.Kg));
-  p.e.out = Y; p.e.bias = b; p.e.inMult = inMult; p.e.outMult = outMult; p.e.P = g.Ho * g.Wo; p.e.Ktot = g.K;
-  p.e.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
+  p.e.inMult = 1.f; p.e.P = g.Ho * g.Wo; p.e.Ktot = g.K;
+  vlb::SumEpilogue fin;
+  fin.bias = b; fin.P = p.e.P; fin.K = g.K; fin.inMult = inMult; fin.outMult = outMult; fin.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
   PrepFilters& q = prep.p[0] = gen_prep(p, g, F);
   q.sn = g.FC; q.sq = 1; q.gs = (long long)g.FC * g.Kg;
-  return launch_ts_gen(ctx, ts, prep, "conv_fprop_gen");
+  return launch_ts_gen(ctx, ts, prep, Y, (size_t)p.M * g.K, fin, true, "conv_fprop_gen");
 }
 
 // One dimension of a data gradient's residue class: the input positions h with (h + pad) % stride == r, and the filter taps that reach
@@ -2834,6 +2848,10 @@ int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, f
   }
   TsProblems ts = {};
   PrepBatch prep = {};
+  size_t const nOut = (size_t)g.H * g.W * g.C * g.N;
+  vlb::SumEpilogue fin;
+  fin.mask = ctx->reluMask;
+  fin.bias = ctx->dgradBias; fin.P = g.H * g.W; fin.K = g.C;
   // shuffled form
   int const FHm = vlb::ceil_div(g.FH, g.sy), FWm = vlb::ceil_div(g.FW, g.sx);
   int const iy = g.pt / g.sy, ix = g.pl / g.sx, Hm = (g.H - 1 + g.pt) / g.sy - iy + 1, Wm = (g.W - 1 + g.pl) / g.sx - ix + 1;
@@ -2847,12 +2865,12 @@ int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, f
       gen_problem(p, t, dY, g.Kg, g.G, cols, BN);
       p.oys = g.sy; p.oxs = g.sx; p.oy = g.sy * iy - g.pt; p.ox = g.sx * ix - g.pl; p.outH = g.H; p.outW = g.W;
       p.shufY = g.sy; p.shufX = g.sx; p.outC = C;
-      p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C; p.e.mask = ctx->reluMask;
-      ctx->maskDone = ctx->reluMask != nullptr;
+      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
+      ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true;
       PrepFilters& q = prep.p[0] = gen_prep(p, g, F);
       q.bh = g.sy * (FHm - 1); q.ah = -g.sy; q.bw = g.sx * (FWm - 1); q.aw = -g.sx;
       q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
-      return launch_ts_gen(ctx, ts, prep, "conv_dgrad_gen");
+      return launch_ts_gen(ctx, ts, prep, dX, nOut, fin, true, "conv_dgrad_gen");
     }
   }
   if (!classesOk) return VLB_Unsupported;
@@ -2871,15 +2889,16 @@ int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, f
       Params& p = ts.p[ts.n];
       gen_problem(p, t, dY, g.Kg, g.G, C, pick_bn(C));
       p.oys = g.sy; p.oxs = g.sx; p.oy = h.h0; p.ox = w.h0; p.outH = g.H; p.outW = g.W;
-      p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C; p.e.mask = ctx->reluMask;
+      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
       PrepFilters& q = prep.p[ts.n] = gen_prep(p, g, F);
       q.bh = h.f0 + h.step * (h.taps - 1); q.ah = -h.step; q.bw = w.f0 + w.step * (w.taps - 1); q.aw = -w.step;
       q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
       ++ts.n;
     }
-  ctx->maskDone = ctx->reluMask != nullptr;
+  if (holes) fin.bias = nullptr;                    // (the zeros of the classes without a tap would miss it)
+  ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = !holes;
   if (ts.n == 0) return VLB_Success;                // no tap reaches any pixel: all zeros, written above
-  return launch_ts_gen(ctx, ts, prep, "conv_dgrad_gen");
+  return launch_ts_gen(ctx, ts, prep, dX, nOut, fin, !holes, "conv_dgrad_gen");
 }
 
 bool is_fc(ConvGeom const& g)
@@ -2901,6 +2920,10 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
   if (is_fc(g)) {
     // Y(K x N) = F'(K x V) X(V x N) + b 1'  (reference bits/nnfullyconnected.cu:45-70): rows = filters
     if (outMult != 0.f || inMult != 1.f) return VLB_Unsupported;
+    {
+      int const rc = fc_fprop_small(ctx, g, Y, X, F, b);
+      if (rc != VLB_Unsupported) return rc;
+    }
     {
       int const rc = fc_fprop_ts(ctx, g, Y, X, F, b);
       if (rc >= 0) return rc;
@@ -2928,10 +2951,9 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
     p.e.out = part; p.e.splitStride = (long long)nOut;
     int rc = launch<OP_DENSE_K, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "fc_fprop_tc");
     if (rc) return rc;
-    tc_splitk_reduce_kernel<<<grid_for(nOut, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(Y, part, nOut, nOut, splits);
-    VLB_LAUNCHED(ctx, 1);
-    if (b) return vlb_bias_forward(ctx, Y, 1.0, nullptr, 0.0, b, 1.0, 1, 1, g.K, g.N);
-    return check_launch(ctx, "fc_fprop_tc");
+    SumEpilogue epi;
+    epi.bias = b; epi.K = g.K; epi.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
+    return sum_parts(ctx, Y, part, nOut, nOut, splits, epi);
   }
   long long M = (long long)g.Ho * g.Wo * g.N;
   ProfScope prof(ctx, kProfFprop);
@@ -2950,10 +2972,19 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
   p.e.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
   if (p.a.fast && g.C % 32 == 0) {
     p.chanFast = 1;
-    p.bTiles = prep_b_tiles(ctx, F, g.K, V, p.BN, p.numKb, 3, g);
+    p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit);
+    p.numKb = p.splits * p.kbPerSplit;
+    size_t const nOut = (size_t)p.M * g.K, partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
+    p.bTiles = prep_b_tiles(ctx, F, g.K, V, p.BN, p.numKb, 3, g, partBytes);
     if (!p.bTiles) return ctx->lastError;
     p.pipelined = 1;
-    return launch_ts(ctx, p, "conv_fprop_ts");
+    if (p.splits == 1) return launch_ts(ctx, p, "conv_fprop_ts");
+    SumEpilogue epi;
+    epi.bias = b; epi.P = p.e.P; epi.K = g.K; epi.inMult = inMult; epi.outMult = outMult; epi.relu = ctx->fuseRelu;
+    float* const part = (float*)((char*)p.bTiles + b_tiles_bytes(ctx, g.K, p.BN, p.numKb));
+    p.e.out = part; p.e.splitStride = (long long)nOut; p.e.bias = nullptr; p.e.inMult = 1.f; p.e.outMult = 0.f; p.e.relu = 0;
+    int const rc = launch_ts(ctx, p, "conv_fprop_ts");
+    return rc ? rc : sum_parts(ctx, Y, part, nOut, nOut, p.splits, epi);
   }
   return launch<OP_IM2COL, OP_DENSE_K, EPI_CONV>(ctx, p, 1, "conv_fprop_tc");
 }
@@ -3003,7 +3034,9 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
   p.b = Operand{}; p.b.ld = V; p.b.rows = g.C;
   if (p.a.fast && g.K % 32 == 0) {
     p.chanFast = 1;
-    p.bTiles = prep_b_tiles(ctx, F, g.C, V, p.BN, p.numKb, 4, g);
+    p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit);
+    p.numKb = p.splits * p.kbPerSplit;
+    p.bTiles = prep_b_tiles(ctx, F, g.C, V, p.BN, p.numKb, 4, g, p.splits > 1 ? sizeof(float) * (size_t)p.M * g.C * p.splits : 0);
     if (!p.bTiles) return ctx->lastError;
     p.b.ptr = p.bTiles;          // not read by the pipelined producers
     p.pipelined = 1;
@@ -3017,8 +3050,15 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
   }
   p.e = Epilogue{}; p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
   if (p.pipelined) {
-    p.e.mask = ctx->reluMask; ctx->maskDone = ctx->reluMask != nullptr;
-    return launch_ts(ctx, p, "conv_dgrad_ts");
+    ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true;
+    if (p.splits == 1) { p.e.mask = ctx->reluMask; p.e.bias = ctx->dgradBias; return launch_ts(ctx, p, "conv_dgrad_ts"); }
+    SumEpilogue epi;
+    epi.mask = ctx->reluMask; epi.bias = ctx->dgradBias; epi.P = p.e.P; epi.K = g.C;
+    size_t const nOut = (size_t)p.M * g.C;
+    float* const part = (float*)((char*)p.bTiles + b_tiles_bytes(ctx, g.C, p.BN, p.numKb));
+    p.e.out = part; p.e.splitStride = (long long)nOut;
+    int const rc = launch_ts(ctx, p, "conv_dgrad_ts");
+    return rc ? rc : sum_parts(ctx, dX, part, nOut, nOut, p.splits, epi);
   }
   return launch<OP_IM2COL, OP_DENSE_K, EPI_CONV>(ctx, p, 1, "conv_dgrad_tc");
 }
@@ -3082,9 +3122,7 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
   p.e.out = part; p.e.splitStride = (long long)nF;
   int rc = launch<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "conv_wgrad_tc");
   if (rc) return rc;
-  tc_splitk_reduce_kernel<<<grid_for(nF, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(dF, part, nF, nF, splits);
-  VLB_LAUNCHED(ctx, 1);
-  return check_launch(ctx, "conv_wgrad_tc");
+  return sum_parts(ctx, dF, part, nF, nF, splits);
 }
 
 }  // namespace vlb

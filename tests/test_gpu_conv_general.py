@@ -57,3 +57,40 @@ def test_general_gather_vs_oracle(gpu, oracle, case, precision, tol):
         assert rel_l2(mat.to_numpy(dxm), np.where(x > 0, dx_ref, 0)) < tol
     finally:
         ctx.set_precision(0)
+
+
+# the fully connected forward pass for few images, and reductions cut into ranges because the output tiles are few
+FEW = {
+    "fc_n1": ((7, 7, 64, 1), (7, 7, 64, 130), 0), "fc_n3_ragged": ((5, 3, 23, 3), (5, 3, 23, 1201), 0), "fc_n8": ((1, 1, 512, 8), (1, 1, 512, 67), 0),
+    "few_tiles_plain": ((14, 14, 256, 1), (3, 3, 256, 160), 1), "few_tiles_windows": ((32, 16, 64, 1), (5, 5, 64, 48), 2),
+    "few_tiles_general": ((8, 8, 50, 5), (5, 5, 50, 70), 0),
+}
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 1e-5), (1, 2e-3)])
+@pytest.mark.parametrize("case", sorted(FEW))
+def test_few_images_and_few_tiles_vs_oracle(gpu, oracle, case, precision, tol):
+    nn, mat, ctx = gpu
+    xs, fs, pad = FEW[case]
+    rng = np.random.default_rng(len(case))
+    x = np.asfortranarray(np.maximum(rng.standard_normal(xs), -0.3).astype(np.float32))
+    f = np.asfortranarray((rng.standard_normal(fs) * np.sqrt(2.0 / np.prod(fs[:3]))).astype(np.float32))
+    b = (rng.standard_normal(fs[3]) * 0.1).astype(np.float32)
+    x64, f64, b64 = (a.astype(np.float64) for a in (x, f, b))
+    kw = dict(pad=(pad,) * 4)
+    y_ref = oracle.conv_forward(x64, f64, b64, **kw)
+    dy = np.asfortranarray(rng.standard_normal(y_ref.shape).astype(np.float32))
+    dx_ref, df_ref, db_ref = oracle.conv_backward(x64, f64, dy.astype(np.float64), **kw)
+    xd, fd, bd, dyd = (mat.from_numpy(a) for a in (x, f, b, dy))
+    ctx.set_precision(precision)
+    try:
+        y, yr = nn.vl_nnconv(xd, fd, bd, ctx=ctx, **kw), nn.vl_nnconv(xd, fd, bd, relu=True, ctx=ctx, **kw)
+        dx, df, db = nn.vl_nnconv(xd, fd, bd, dyd, ctx=ctx, **kw)
+        dxm = nn.vl_nnconv(xd, fd, bd, dyd, through_relu=True, ctx=ctx, **kw)[0]
+        assert ctx.device_status() == 0
+        for got, want, name in ((y, y_ref, "y"), (dx, dx_ref, "dx"), (df, df_ref, "df"), (db, db_ref, "db")):
+            assert rel_l2(mat.to_numpy(got).ravel(), np.asarray(want).ravel()) < tol, name
+        assert np.array_equal(mat.to_numpy(yr), np.maximum(mat.to_numpy(y), 0))
+        assert rel_l2(mat.to_numpy(dxm), np.where(x > 0, dx_ref, 0)) < tol
+    finally:
+        ctx.set_precision(0)
