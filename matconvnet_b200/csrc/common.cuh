@@ -107,6 +107,13 @@ inline unsigned grid_for(size_t n, int threads, int maxBlocks = 148 * 16)
 
 #ifdef __CUDACC__
 namespace vlb {
+// Division by a small number with a multiply: exact for i * d < 2^32.
+struct FastDiv {
+  unsigned d, m;
+  __host__ FastDiv(int v = 1) : d((unsigned)v), m(v > 1 ? (unsigned)((0x100000000ull + v - 1) / (unsigned)v) : 0u) {}
+  __device__ __forceinline__ int operator()(int i) const { return d == 1 ? i : (int)__umulhi((unsigned)i, m); }
+};
+
 // Exclusive prefix sum of v[0..n) in place by a whole block of kThreads threads (a multiple of 32, at most 1024);
 // warpSums: 32 ints of shared memory.  Ends with a block barrier.
 template <int kThreads>

@@ -316,6 +316,107 @@ __global__ void __launch_bounds__(kThreads) conv_small_n4_kernel(SmallParams p)
   }
 }
 
+// Data gradient onto at most 4 channels, tiles of dY in shared memory: a block computes 4*quads rows x cols columns of dX, a thread four
+// vertically adjacent pixels of up to four channels.  dY is staged kSnChunk channels at a time by asynchronous copies (zero-filled
+// outside the plane) while the previous channels are used: per channel and filter column a thread reads its FH + 3 rows with 16-byte
+// loads and FH broadcast filter values for 4 * FH * channels FMAs.  (One pixel per thread from global memory, the form this replaces for
+// filters of 3 and 5 rows, was bound by load latency: LeNet's first layer at batch 100 39.6 us, 16.8 here; CIFAR's 50 us, 33 here.)
+constexpr int kSnThreads = 128, kSnChunk = 4;
+
+__device__ __forceinline__ void sn_cp_async4(float* dst, float const* src, bool on)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 4 : 0) : "memory");
+}
+
+template <int kFH, int kC>
+__global__ void __launch_bounds__(kSnThreads) conv_small_n_tile_kernel(SmallParams p, int quads, int cols, int tilesH, int tilesW, int vec)
+{
+  extern __shared__ float4 smem4[];
+  int const pitch = 4 * quads + 4, width = cols + p.FW - 1, plane = pitch * width;      // rows of a tile: 4*quads + kFH - 1 <= pitch (kFH <= 5)
+  float4* const ws = smem4;                                                               // [channel][fw][fh], four output channels
+  float* const xs = reinterpret_cast<float*>(smem4 + (size_t)p.Cin * p.FW * kFH);         // two buffers of kSnChunk planes
+  int const tid = threadIdx.x;
+  for (int i = tid; i < p.Cin * p.FW * kFH; i += kSnThreads) {
+    int const fh = i % kFH, t = i / kFH, fw = t % p.FW, c = t / p.FW;
+    float w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = k < kC && k < p.Kout ? filter_at(p, fh, fw, c, k) : 0.f;
+    ws[i] = make_float4(w[0], w[1], w[2], w[3]);
+  }
+  int const th = (int)blockIdx.x % tilesH, t1 = (int)blockIdx.x / tilesH, tw = t1 % tilesW, n = t1 / tilesW;
+  int const h0 = th * 4 * quads, w0 = tw * cols;
+  float const* const img = p.x + (long long)n * p.H * p.W * p.Cin;
+  int const rows = 4 * quads + kFH - 1, count = rows * width;
+  auto stage = [&](int c0, int buf) {
+    float* const dst = xs + buf * kSnChunk * plane;
+    // (row, column) of this thread's next element, advanced without divisions
+    int col = tid / rows, row = tid - col * rows;
+    int const dc = kSnThreads / rows, dr = kSnThreads - dc * rows;
+    for (int i = tid; i < count; i += kSnThreads) {
+      int const h = h0 + row - p.pt, w = w0 + col - p.pl;
+      bool const in = (unsigned)h < (unsigned)p.H && (unsigned)w < (unsigned)p.W;
+      float const* const src = img + (in ? (long long)w * p.H + h : 0);
+#pragma unroll
+      for (int c = 0; c < kSnChunk; ++c) {
+        bool const on = in && c0 + c < p.Cin;
+        sn_cp_async4(dst + c * plane + col * pitch + row, on ? src + (long long)(c0 + c) * p.H * p.W : p.x, on);
+      }
+      col += dc; row += dr;
+      if (row >= rows) { row -= rows; ++col; }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int const q = tid % quads, lc = tid / quads;
+  bool const active = lc < cols;
+  float acc[4][kC];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int k = 0; k < kC; ++k) acc[j][k] = 0.f;
+  stage(0, 0);
+  for (int c0 = 0, buf = 0; c0 < p.Cin; c0 += kSnChunk, buf ^= 1) {
+    if (c0 + kSnChunk < p.Cin) { stage(c0 + kSnChunk, buf ^ 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+    else                       asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (active) {
+      int const cn = min(kSnChunk, p.Cin - c0);
+      for (int c = 0; c < cn; ++c) {
+        float const* const xp = xs + (buf * kSnChunk + c) * plane + lc * pitch + 4 * q;
+        float4 const* const wp = ws + (size_t)(c0 + c) * p.FW * kFH;
+        for (int fw = 0; fw < p.FW; ++fw) {
+          float v[8];
+          *reinterpret_cast<float4*>(&v[0]) = *reinterpret_cast<float4 const*>(xp + fw * pitch);
+          *reinterpret_cast<float4*>(&v[4]) = *reinterpret_cast<float4 const*>(xp + fw * pitch + 4);
+#pragma unroll
+          for (int fh = 0; fh < kFH; ++fh) {
+            float4 const w = wp[fw * kFH + fh];
+            float const wk[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int k = 0; k < kC; ++k) acc[j][k] = fmaf(v[j + fh], wk[k], acc[j][k]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  int const h = h0 + 4 * q, w = w0 + lc;
+  if (!active || w >= p.Wo || h >= p.Ho) return;
+  long long const P = (long long)p.Ho * p.Wo;
+  float* const dst = p.out + ((long long)n * p.Kout * P + (long long)w * p.Ho + h);
+#pragma unroll
+  for (int k = 0; k < kC; ++k) {
+    if (k < p.Kout) {
+      if (vec) *reinterpret_cast<float4*>(dst + k * P) = make_float4(acc[0][k], acc[1][k], acc[2][k], acc[3][k]);
+      else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (h + j < p.Ho) dst[k * P + j] = acc[j][k];
+      }
+    }
+  }
+}
+
 // ---- filter (and bias) gradient with few inputs per pixel (R = FH*FW*C <= 27): dF[r][k] = sum over output pixels of
 // x(pixel, r) * dY(pixel, k).  A block walks chunks of 256 consecutive output pixels: it stages the chunk's input windows
 // (256 x R values, gathered once and then shared by all filters) and its 64 x 256 tile of dY in shared memory, both loaded
@@ -544,6 +645,22 @@ int conv_dgrad_small(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F,
     conv_small_n4_kernel<3><<<(unsigned)ceil_div(M / 4, kThreads), kThreads, smem, ctx->stream>>>(p);      // (one group of quads per block measured faster here than a bounded grid)
     VLB_LAUNCHED(ctx, 1);
     return check_launch(ctx, "conv_dgrad_small");
+  }
+  // (three rows, one row of padding, aligned: the kernel above, 474 us on VGG-16's first layer where this one takes 563)
+  if ((g.FH == 3 || g.FH == 5) && g.dy == 1 && g.dx == 1) {
+    int const allQuads = ceil_div(g.H, 4), tilesH = ceil_div(allQuads, 8), quads = ceil_div(allQuads, tilesH);
+    int const cols = std::min(kSnThreads / quads, g.W), tilesW = ceil_div(g.W, cols);
+    size_t const tile = sizeof(float4) * (size_t)g.K * g.FW * g.FH + sizeof(float) * 2 * kSnChunk * (size_t)(4 * quads + 4) * (cols + g.FW - 1);
+    long long const blocks = (long long)tilesH * tilesW * g.N;
+    if (tile <= 48 * 1024 && blocks < (1LL << 31)) {
+      int const vec = g.H % 4 == 0 && (((uintptr_t)dX) & 15) == 0;
+#define VLB_SN(fh, c) conv_small_n_tile_kernel<fh, c><<<(unsigned)blocks, kSnThreads, tile, ctx->stream>>>(p, quads, cols, tilesH, tilesW, vec)
+      if (g.FH == 3) { if (g.C == 1) VLB_SN(3, 1); else if (g.C <= 3) VLB_SN(3, 3); else VLB_SN(3, 4); }
+      else           { if (g.C == 1) VLB_SN(5, 1); else if (g.C <= 3) VLB_SN(5, 3); else VLB_SN(5, 4); }
+#undef VLB_SN
+      VLB_LAUNCHED(ctx, 1);
+      return check_launch(ctx, "conv_dgrad_small");
+    }
   }
   conv_small_n_kernel<4><<<(unsigned)ceil_div(M, kThreads), kThreads, smem, ctx->stream>>>(p);
   VLB_LAUNCHED(ctx, 1);

@@ -1921,46 +1921,19 @@ __global__ void flip_filters_kernel(float* __restrict__ ft, float const* __restr
   }
 }
 
-// The B operand of fprop / dgrad is the filter bank: small, and the same for every CTA.  It is split
-// into hi / lo once and laid out as ready-made shared-memory tile images -- for n-tile t and k-block
-// kb: [hi tile BN x 32][lo tile BN x 32], K-major with the 128-byte swizzle -- so that a producer
-// fetches a whole stage of B with one bulk copy.
-// modes 3 / 4: as 0 / 1 with the reduction index in blocks of 32 channels, all filter taps of a block one after the other.
-// mode 5: B(n, r) = F[n + N*r].
-// mode 0: B(n, r) = F[n*R + r].  mode 2: B(n, r) = dY[pixel, n, image] with r = pixel + P*image.  mode 1 (data gradient of a stride-1 convolution): n = channel c,
-// r = fh' + FH*(fw' + FW*k), B = F[FH-1-fh', FW-1-fw', c, k].
-template <bool kSplit>
-__global__ void prep_b_tiles_kernel(float* __restrict__ out, float const* __restrict__ f, int N, int R, int BN, int numKb,
-                                    int mode, int FH, int FW, int C, int K)
+// The B operand of a contraction is small and the same for every CTA: it is split into hi / lo once and laid out as ready-made
+// shared-memory tile images -- for n-tile t and k-block kb: [hi tile BN x 32][lo tile BN x 32], K-major with the 128-byte swizzle --
+// so that a stage of B is one bulk copy.  Dense operands here, filter banks below:
+// kRows: B(n, r) = f[n*R + r]; else B(n, r) = f[n + N*r].
+template <bool kSplit, bool kRows>
+__global__ void prep_dense_tiles_kernel(float* __restrict__ out, float const* __restrict__ f, int N, int R, int BN, int numKb)
 {
   size_t const Rp = (size_t)numKb * 32;
   size_t const total = (size_t)((N + BN - 1) / BN) * BN * Rp;
   size_t const step = (size_t)gridDim.x * blockDim.x;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += step) {
     int const r = (int)(idx % Rp), n = (int)(idx / Rp);
-    float val = 0.f;
-    if (n < N && r < R) {
-      if (mode == 0) val = f[(size_t)n * R + r];
-      else if (mode == 2) {
-        // filter gradient: n = filter, r = pixel + P*image of dY (FH carries P here)
-        int img = r / FH, pix = r - img * FH;
-        val = f[((size_t)img * N + n) * FH + pix];
-      } else if (mode == 5) {
-        // B(n, r) = f[n + N*r]: rows contiguous (dY of a fully connected layer as the filters of its weight gradient)
-        val = f[(size_t)r * N + n];
-      } else if (mode == 3) {
-        // forward filters, reduction in blocks of 32 channels: r = c%32 + 32*(tap + taps*(c/32))
-        int taps = FH * FW, t = r >> 5, tap = t % taps, c = (t / taps) * 32 + (r & 31);
-        val = f[(size_t)n * R + tap + (size_t)taps * c];
-      } else if (mode == 4) {
-        // data gradient, reduction in blocks of 32 filters: r = k%32 + 32*(tap' + taps*(k/32)), tap' = fh' + FH*fw'
-        int taps = FH * FW, t = r >> 5, tap = t % taps, k = (t / taps) * 32 + (r & 31), fh = tap % FH, fw = tap / FH;
-        val = f[(FH - 1 - fh) + (size_t)FH * ((FW - 1 - fw) + (size_t)FW * (n + (size_t)C * k))];
-      } else {
-        int fh = r % FH, t = r / FH, fw = t % FW, k = t / FW;
-        val = f[(FH - 1 - fh) + (size_t)FH * ((FW - 1 - fw) + (size_t)FW * (n + (size_t)C * k))];
-      }
-    }
+    float const val = n < N && r < R ? f[kRows ? (size_t)n * R + r : (size_t)r * N + n] : 0.f;
     int const tile = n / BN, row = n % BN, kb = r >> 5, kk = r & 31;
     size_t const base = ((size_t)tile * numKb + kb) * (kSplit ? 2 : 1) * (size_t)BN * 32;
     size_t const off = (size_t)row * 32 + ((((kk >> 2) ^ (row & 7)) << 2) | (kk & 3));
@@ -1974,7 +1947,7 @@ __global__ void prep_b_tiles_kernel(float* __restrict__ out, float const* __rest
   }
 }
 
-// Filter tile images for conv_ts_gen_kernel: like prep_b_tiles_kernel's, for the units of channels, filter groups, tap subsets
+// Filter tile images for conv_ts_kernel and conv_ts_gen_kernel, for the units of channels, filter groups, tap subsets
 // (residue classes of a strided data gradient) and shuffled columns of the general gather.  Row n of a tile is column n of its
 // group; tap (fh', fw') of the problem is tap (bh + ah*fh', bw + aw*fw') of the filter bank, zero where that does not exist; the
 // filter of (column channel n, reduction channel q) starts at F + FH*FW * (gs*group + sn*n + sq*q).
@@ -1986,6 +1959,7 @@ struct PrepFilters {
   float const* f;
   int BN, numKb, rows, tilesPerGroup, cols, unit, upk, tapsH, tapsW, C, FH, FW, bh, ah, bw, aw, shufY, shufX, per;
   long long sn, sq, gs;
+  vlb::FastDiv divRun, divFT;       // by 8 * FH*FW and FH*FW (set by launch_prep)
 };
 struct PrepBatch { PrepFilters p[kMaxTsProblems]; };
 
@@ -2024,7 +1998,123 @@ __global__ void __launch_bounds__(256) prep_filters_kernel(const __grid_constant
   }
 }
 
-// dY of a filter gradient as tile images (mode 2 of prep_b_tiles_kernel) for planes that are a multiple of
+// The same for units of 32 channels, through shared memory.  The direct kernel reads a value at a time, a tap (36 bytes) or a filter apart:
+// every 32-byte sector is fetched for four useful bytes (512 -> 512 channels, 3x3: 16.8 us for 28 MB; this one 9 us).  A block takes eight rows
+// and one block of 32 channels, reads whole runs -- forward: the 32 * FH*FW floats of a row; data gradient: for each of 32 filters the
+// 8 * FH*FW floats of its eight channels -- and writes every tap's 128-byte rows, four taps at a time.  Shared memory: element
+// (row, q, tap) at row * (32 * FTp + 1) + q * FTp + tap, FTp odd: the reads of a warp (four rows x eight chunks) fall into 32 banks.
+constexpr int kPrepRows = 8, kMaxPrepTaps = 45;
+
+template <bool kSplit>
+__global__ void __launch_bounds__(256) prep_filters_tile_kernel(const __grid_constant__ PrepBatch b)
+{
+  extern __shared__ float prepSmem[];
+  PrepFilters const& p = b.p[blockIdx.z];
+  int const r0 = (int)blockIdx.x * kPrepRows, cb = (int)blockIdx.y, taps = p.tapsH * p.tapsW, FT = p.FH * p.FW, FTp = FT | 1;
+  if (r0 >= p.rows || cb * taps >= p.numKb) return;
+  int const tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int const tile = r0 / p.BN, inTile0 = r0 - tile * p.BN, grp = tile / p.tilesPerGroup;
+  int const col0 = (tile - grp * p.tilesPerGroup) * p.BN + inTile0;
+  constexpr int kLoads = 12;                           // in flight per thread: one round for 3x3 filters (nine)
+  int const rowPitch = 32 * FTp + 1, q0 = cb * 32, nq = min(32, p.C - q0), per = p.shufY > 0 ? p.shufY * p.shufX : 1;
+  if (p.sq == 1) {
+    // a warp per row: nq * FT consecutive floats
+    int const col = col0 + warp;
+    if (col < p.cols) {
+      float const* const src = p.f + (long long)FT * (p.gs * grp + p.sn * (col / per) + q0);
+      float* const dst = prepSmem + warp * rowPitch;
+      int const n = nq * FT;
+      for (int i = lane; i < n; i += 32 * kLoads) {
+        float v[kLoads];
+#pragma unroll
+        for (int k = 0; k < kLoads; ++k) v[k] = i + 32 * k < n ? __ldg(src + i + 32 * k) : 0.f;
+#pragma unroll
+        for (int k = 0; k < kLoads; ++k) { int const e = i + 32 * k; if (e < n) dst[FT == FTp ? e : e + e / FT] = v[k]; }
+      }
+    }
+  } else {
+    // runs of the FT taps of this block's rows, consecutive channels (shuffled columns: a channel serves several rows)
+    int const nr = min(kPrepRows, p.cols - col0);
+    float const* const src = p.f + (long long)FT * (p.gs * grp + p.sq * q0);
+    int const run = kPrepRows * FT, n = nq * run;
+    for (int i = tid; i < n; i += 256 * kLoads) {
+      float v[kLoads];
+      int at[kLoads];
+#pragma unroll
+      for (int k = 0; k < kLoads; ++k) {
+        int const e = i + 256 * k;
+        v[k] = 0.f; at[k] = -1;
+        if (e < n) {
+          int const q = p.divRun(e), u = e - q * run, row = p.divFT(u), t = u - row * FT;
+          if (row >= nr) continue;
+          at[k] = row * rowPitch + q * FTp + t;
+          v[k] = __ldg(src + (long long)FT * (p.sq * q + p.sn * (per == 1 ? col0 + row : (col0 + row) / per)) + t);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kLoads; ++k) if (at[k] >= 0) prepSmem[at[k]] = v[k];
+    }
+  }
+  __syncthreads();
+  int const row = (tid >> 3) & 7, chunk = tid & 7, col = col0 + row;
+  int ry = 0, rx = 0;
+  if (p.shufY > 0) { int const t = col % per; rx = t / p.shufY; ry = t - rx * p.shufY; }
+  float const* const s = prepSmem + row * rowPitch + chunk * 4 * FTp;
+  size_t const tileFloats = (size_t)(kSplit ? 2 : 1) * p.BN * 32;
+  float* const out = p.out + ((size_t)tile * p.numKb + (size_t)cb * taps) * tileFloats + (size_t)(inTile0 + row) * 32 + ((chunk ^ ((inTile0 + row) & 7)) << 2);
+  for (int tap = tid >> 6; tap < taps && cb * taps + tap < p.numKb; tap += 4) {
+    int const tw = tap / p.tapsH, th = tap - tw * p.tapsH, fh = p.bh + p.ah * th + ry, fw = p.bw + p.aw * tw + rx;
+    bool const on = col < p.cols && (unsigned)fh < (unsigned)p.FH && (unsigned)fw < (unsigned)p.FW;
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = on && chunk * 4 + e < nq ? s[e * FTp + fh + p.FH * fw] : 0.f;
+    float* const base = out + (size_t)tap * tileFloats;
+    if (kSplit) {
+      float4 const h = make_float4(tf32_hi(v[0]), tf32_hi(v[1]), tf32_hi(v[2]), tf32_hi(v[3]));
+      *reinterpret_cast<float4*>(base) = h;
+      *reinterpret_cast<float4*>(base + (size_t)p.BN * 32) = make_float4(v[0] - h.x, v[1] - h.y, v[2] - h.z, v[3] - h.w);
+    } else {
+      *reinterpret_cast<float4*>(base) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
+// Launches the tile-image kernel for n problems whose output pointers are set.
+void launch_prep(vlb_ctx* ctx, PrepBatch& prep, int n)
+{
+  bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
+  int rows = 0, groups = 0, blocks = 0, FT = 0;
+  bool whole = true;
+  long long elements = 0;
+  for (int i = 0; i < n; ++i) {
+    PrepFilters& q = prep.p[i];
+    q.divFT = vlb::FastDiv(q.FH * q.FW); q.divRun = vlb::FastDiv(kPrepRows * q.FH * q.FW);
+    rows = std::max(rows, q.rows);
+    blocks = std::max(blocks, vlb::ceil_div(q.numKb, q.tapsH * q.tapsW)); FT = std::max(FT, q.FH * q.FW);
+    whole = whole && q.unit == 32;
+    elements += (long long)q.rows * q.numKb * 32;
+  }
+  // few blocks of many k-blocks each would be all latency
+  for (int i = 0; i < n; ++i) {
+    PrepFilters& q = prep.p[i];
+    while (q.per > 1 && (long long)vlb::ceil_div(q.rows, 32) * vlb::ceil_div(q.numKb, q.per) * n < 2 * ctx->smCount) q.per = (q.per + 1) / 2;
+    groups = std::max(groups, vlb::ceil_div(q.numKb, q.per));
+  }
+  VLB_LAUNCHED(ctx, 1);
+  // the tiled kernel's two phases cost more than they save on banks of less than about 600,000 elements (256 -> 256 channels, 3x3: 6.3 us both ways; 64 -> 64: 4.2 against 2.6)
+  if (whole && FT <= kMaxPrepTaps && elements >= 600000) {
+    dim3 const grid(vlb::ceil_div(rows, kPrepRows), blocks, n);
+    size_t const smem = sizeof(float) * kPrepRows * (32 * (size_t)(FT | 1) + 1);
+    if (split3) prep_filters_tile_kernel<true><<<grid, 256, smem, ctx->stream>>>(prep);
+    else        prep_filters_tile_kernel<false><<<grid, 256, smem, ctx->stream>>>(prep);
+    return;
+  }
+  dim3 const grid(vlb::ceil_div(rows, 32), groups, n);
+  if (split3) prep_filters_kernel<true><<<grid, 256, 0, ctx->stream>>>(prep);
+  else        prep_filters_kernel<false><<<grid, 256, 0, ctx->stream>>>(prep);
+}
+
+// dY of a filter gradient as tile images, B(n, r) = dY[pixel, n, image] with r = pixel + P*image, for planes that are a multiple of
 // four pixels: 16-byte loads along the pixels, 16-byte stores of the swizzled chunks, and -- dY being read
 // anyway -- the bias gradient db[n] = sum of dY over pixels and images (reference bits/nnconv.cu:141-149) on
 // the way: per-block partial sums, and the block that takes a channel's last ticket adds them in block order,
@@ -2118,24 +2208,35 @@ size_t b_tiles_bytes(vlb_ctx* ctx, int N, int BN, int numKb)
 }
 
 // `extraBytes` of scratch are reserved behind the tiles for the caller (split-K partials).
-float const* prep_b_tiles(vlb_ctx* ctx, float const* f, int N, int R, int BN, int numKb, int mode, vlb::ConvGeom const& g,
-                          size_t extraBytes = 0, int P = 0)
+float const* prep_dense_tiles(vlb_ctx* ctx, float const* f, int N, int R, int BN, int numKb, bool rows, size_t extraBytes = 0)
 {
-  bool split3 = ctx->precision == VLB_PRECISION_3XTF32;
-  size_t total = (size_t)vlb::ceil_div(N, BN) * BN * (size_t)numKb * 32;
+  bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
+  size_t const total = (size_t)vlb::ceil_div(N, BN) * BN * (size_t)numKb * 32;
   float* tiles = (float*)vlb::workspace(ctx, b_tiles_bytes(ctx, N, BN, numKb) + extraBytes);
   if (!tiles) return nullptr;
-  if (mode == 2) {
-    unsigned grid2 = vlb::grid_for(total, 256, ctx->smCount * 16);
-    if (split3) prep_b_tiles_kernel<true><<<grid2, 256, 0, ctx->stream>>>(tiles, f, N, R, BN, numKb, 2, P, 0, 0, 0);
-    else        prep_b_tiles_kernel<false><<<grid2, 256, 0, ctx->stream>>>(tiles, f, N, R, BN, numKb, 2, P, 0, 0, 0);
-    VLB_LAUNCHED(ctx, 1);
-    return tiles;
-  }
-  unsigned grid = vlb::grid_for(total, 256, ctx->smCount * 8);
-  if (split3) prep_b_tiles_kernel<true><<<grid, 256, 0, ctx->stream>>>(tiles, f, N, R, BN, numKb, mode, g.FH, g.FW, g.C, g.K);
-  else        prep_b_tiles_kernel<false><<<grid, 256, 0, ctx->stream>>>(tiles, f, N, R, BN, numKb, mode, g.FH, g.FW, g.C, g.K);
+  unsigned const grid = vlb::grid_for(total, 256, ctx->smCount * 8);
+#define VLB_PD(split, r) prep_dense_tiles_kernel<split, r><<<grid, 256, 0, ctx->stream>>>(tiles, f, N, R, BN, numKb)
+  if (split3) { if (rows) VLB_PD(true, true); else VLB_PD(true, false); }
+  else        { if (rows) VLB_PD(false, true); else VLB_PD(false, false); }
+#undef VLB_PD
   VLB_LAUNCHED(ctx, 1);
+  return tiles;
+}
+
+// The filter bank of one group, reduction in blocks of 32 channels (conv_ts_kernel): forward, or flipped and transposed for the data gradient
+// of a stride-1 convolution.
+float const* prep_conv_tiles(vlb_ctx* ctx, float const* f, vlb::ConvGeom const& g, int BN, int numKb, bool dgrad, size_t extraBytes)
+{
+  int const N = dgrad ? g.C : g.K;
+  float* tiles = (float*)vlb::workspace(ctx, b_tiles_bytes(ctx, N, BN, numKb) + extraBytes);
+  if (!tiles) return nullptr;
+  PrepBatch prep = {};
+  PrepFilters& q = prep.p[0];
+  q.out = tiles; q.f = f; q.BN = BN; q.numKb = numKb; q.tilesPerGroup = vlb::ceil_div(N, BN); q.rows = q.tilesPerGroup * BN; q.cols = N;
+  q.unit = 32; q.upk = 1; q.tapsH = q.FH = g.FH; q.tapsW = q.FW = g.FW; q.C = dgrad ? g.K : g.C;
+  q.bh = dgrad ? g.FH - 1 : 0; q.bw = dgrad ? g.FW - 1 : 0; q.ah = q.aw = dgrad ? -1 : 1;
+  q.sn = dgrad ? 1 : g.C; q.sq = dgrad ? g.C : 1; q.per = 8;
+  launch_prep(ctx, prep, 1);
   return tiles;
 }
 
@@ -2602,7 +2703,7 @@ int fc_dgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, floa
   size_t const partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
   ProfScope prof(ctx, kProfFc);
   prof.rec.flops = 2.0 * (double)V * (double)g.N * (double)g.K;
-  p.bTiles = prep_b_tiles(ctx, dY, g.N, g.K, p.BN, p.numKb, 0, t, partBytes);            // B(n, k) = dY[k + K n]
+  p.bTiles = prep_dense_tiles(ctx, dY, g.N, g.K, p.BN, p.numKb, true, partBytes);            // B(n, k) = dY[k + K n]
   if (!p.bTiles) return ctx->lastError;
   float* const part = p.splits > 1 ? (float*)((char*)p.bTiles + b_tiles_bytes(ctx, g.N, p.BN, p.numKb)) : nullptr;
   p.e = Epilogue{};
@@ -2627,7 +2728,7 @@ int fc_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, floa
   p.chanFast = 1; p.pipelined = 1;
   ProfScope prof(ctx, kProfFc);
   prof.rec.flops = 2.0 * (double)V * (double)g.K * (double)g.N;
-  p.bTiles = prep_b_tiles(ctx, dY, g.K, g.N, p.BN, p.numKb, 5, t);                       // B(k, n) = dY[k + K n]
+  p.bTiles = prep_dense_tiles(ctx, dY, g.K, g.N, p.BN, p.numKb, false);                       // B(k, n) = dY[k + K n]
   if (!p.bTiles) return ctx->lastError;
   p.e = Epilogue{};
   p.e.out = dF; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.K;
@@ -2675,7 +2776,7 @@ PrepFilters gen_prep(Params const& p, ConvGeom const& g, float const* f)
   q.f = f; q.BN = p.BN; q.numKb = p.numKb; q.rows = p.tilesN * p.BN; q.tilesPerGroup = p.tilesPerGroup; q.cols = p.cols;
   q.unit = p.unit; q.upk = p.upk; q.tapsH = p.a.FH; q.tapsW = p.a.FW; q.C = p.a.C; q.FH = g.FH; q.FW = g.FW;
   q.ah = q.aw = 1; q.shufY = p.shufY; q.shufX = p.shufX;
-  q.per = p.unit == 32 ? std::max(4, std::min(16, q.tapsH * q.tapsW)) : 8;
+  q.per = 8;
   return q;
 }
 
@@ -2697,7 +2798,6 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
   size_t const stageBytes = (split3 ? 2u : 1u) * (size_t)BN * BK * 4;
   size_t total = 0, sumBytes = 0;
   long long tiles = 0;
-  int rows = 0, kbGroups = 0;
   double work = 0;
   int splits = 1;
   {
@@ -2711,14 +2811,12 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     p.splits = splits; p.kbPerSplit = vlb::ceil_div(p.numKb, splits);
     p.numKb = p.kbTot = p.splits * p.kbPerSplit;
     prep.p[i].numKb = p.numKb;
-    // few blocks of many k-blocks each would be all latency
-    while (prep.p[i].per > 1 && (long long)vlb::ceil_div(prep.p[i].rows, 32) * vlb::ceil_div(p.numKb, prep.p[i].per) * b.n < 2 * ctx->smCount) prep.p[i].per = (prep.p[i].per + 1) / 2;
     p.e.out = out;
     if (splits > 1) p.e.splitStride = (long long)nOut;
     else { p.e.bias = fin.bias; p.e.inMult = fin.inMult; p.e.outMult = fin.outMult; p.e.relu = fin.relu; p.e.mask = fin.mask; }
     prep.p[i].out = (float*)total;                 // offset for now
     total += (sizeof(float) * (size_t)p.tilesN * BN * (size_t)p.numKb * 32 * (split3 ? 2 : 1) + 255) & ~(size_t)255;
-    rows = std::max(rows, prep.p[i].rows); kbGroups = std::max(kbGroups, vlb::ceil_div(prep.p[i].numKb, prep.p[i].per));
+    if (p.numKb > 65535) return VLB_Unsupported;
     p.smemSum = ((ctx->testSwitch & 8) || p.kbPerSplit < 8) ? 1 : 0;
     sumBytes = std::max(sumBytes, p_bytes(BN, p.smemSum));
     long long const t = (long long)p.tilesM * p.tilesN * p.splits;
@@ -2758,10 +2856,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     if (splits > 1) p.e.out = part;
     p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;
   }
-  dim3 const pgrid(vlb::ceil_div(rows, 32), kbGroups, b.n);
-  if (pgrid.y > 65535u) return VLB_Unsupported;
-  if (split3) prep_filters_kernel<true><<<pgrid, 256, 0, ctx->stream>>>(prep);
-  else        prep_filters_kernel<false><<<pgrid, 256, 0, ctx->stream>>>(prep);
+  launch_prep(ctx, prep, b.n);
   size_t const smemBytes = std::max<size_t>((size_t)stages * stageBytes + sumBytes + 1024, 120u * 1024u);      // two CTAs never share an SM
   cudaError_t e;
   auto go = [&](auto kernel) {
@@ -2773,7 +2868,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
   else        { if (BN <= 64) VLB_TSG(false, true); else VLB_TSG(false, false); }
 #undef VLB_TSG
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
-  VLB_LAUNCHED(ctx, 2);
+  VLB_LAUNCHED(ctx, 1);
   int const rc = vlb::check_launch(ctx, where);
   return rc || splits == 1 ? rc : vlb::sum_parts(ctx, out, part, nOut, nOut, splits, fin);
 }
@@ -2975,7 +3070,7 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
     p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit);
     p.numKb = p.splits * p.kbPerSplit;
     size_t const nOut = (size_t)p.M * g.K, partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
-    p.bTiles = prep_b_tiles(ctx, F, g.K, V, p.BN, p.numKb, 3, g, partBytes);
+    p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, false, partBytes);
     if (!p.bTiles) return ctx->lastError;
     p.pipelined = 1;
     if (p.splits == 1) return launch_ts(ctx, p, "conv_fprop_ts");
@@ -3036,7 +3131,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     p.chanFast = 1;
     p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit);
     p.numKb = p.splits * p.kbPerSplit;
-    p.bTiles = prep_b_tiles(ctx, F, g.C, V, p.BN, p.numKb, 4, g, p.splits > 1 ? sizeof(float) * (size_t)p.M * g.C * p.splits : 0);
+    p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, true, p.splits > 1 ? sizeof(float) * (size_t)p.M * g.C * p.splits : 0);
     if (!p.bTiles) return ctx->lastError;
     p.b.ptr = p.bTiles;          // not read by the pipelined producers
     p.pipelined = 1;

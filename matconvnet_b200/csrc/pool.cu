@@ -19,6 +19,8 @@ namespace {
 
 constexpr int kThreads = 256;
 
+using vlb::FastDiv;
+
 struct PoolParams {
   int H, W, Ho, Wo;
   int poolH, poolW, strideY, strideX, padTop, padLeft;
@@ -111,13 +113,6 @@ __global__ void pool_bwd_generic(float* __restrict__ dx, float const* __restrict
 // window's arg-max is found once, by one thread, instead of once per input element that the window covers (a 3x3 / stride-2 backward pass
 // scanned every window nine times: 1273 us on 55x55x96x128 where its 334 MB take 51 us; this kernel: 292 us); then every
 // input element adds the derivatives of the windows that chose it, in the reference's order (wo outer, ho inner).
-// Division by a plane extent with a multiply: exact for i * d < 2^32.
-struct FastDiv {
-  unsigned d, m;
-  __host__ FastDiv(int v = 1) : d((unsigned)v), m(v > 1 ? (unsigned)((0x100000000ull + v - 1) / (unsigned)v) : 0u) {}
-  __device__ __forceinline__ int operator()(int i) const { return d == 1 ? i : (int)__umulhi((unsigned)i, m); }
-};
-
 struct TileParams {
   PoolParams p;
   int planesPerTile, cols, tilesPerPlane;     // one plane and `cols` columns per tile (backward: of the input, forward: of the output), or several whole planes

@@ -25,6 +25,8 @@ CASES = {
     "groups2_wide_s2": ((15, 11, 80, 2), (3, 3, 40, 300), (2, 2), (1, 1, 1, 1), (1, 1)),           # several column tiles per group
     "groups4_narrow": ((12, 12, 24, 4), (3, 3, 6, 20), (1, 2), (1, 1, 1, 1), (1, 1)),
     "many_tiles_s2": ((96, 90, 40, 6), (3, 3, 40, 72), (2, 2), (1, 1, 1, 1), (1, 1)),              # more tiles than SMs: CTAs shared out
+    "two_channels_5x3": ((71, 29, 2, 3), (5, 3, 2, 30), (1, 1), (4, 0, 1, 2), (1, 1)),             # tiled CUDA-core data gradient, ragged quads and chunks
+    "four_channels_3x5": ((33, 66, 4, 2), (3, 5, 4, 9), (1, 1), (0, 2, 2, 2), (1, 1)),
     "s5_falls_back": ((23, 24, 8, 2), (3, 3, 8, 16), (5, 5), (1, 1, 1, 1), (2, 2)),                # 25 classes: more than one launch holds
 }
 
