@@ -44,6 +44,7 @@ bnorm_reduce_kernel(float* __restrict__ momentsOut,   // 2*C or nullptr
                     float const* __restrict__ x, float const* __restrict__ dy,
                     int WH, int C, int N, float eps)
 {
+  vlb::pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float part[4];
   __shared__ float warpRed[kThreads / 32][4];
@@ -140,6 +141,7 @@ bnorm_fused_kernel(float* __restrict__ out,            // y or dx
                    float const* __restrict__ g, float const* __restrict__ b,
                    int WH, int C, int N, float eps, int relu)      // relu (forward): the stored value is max(y, 0)
 {
+  vlb::pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float part[4];
   __shared__ float coef[4];
@@ -276,8 +278,8 @@ void launch_fused(vlb_ctx* ctx, bool vec, float* out, float* momOut, float* dg, 
                   float const* x, float const* dy, float const* g, float const* b, int WH, int C, int N, float eps, int relu = 0)
 {
   dim3 grid(C, kCluster);
-  if (vec) bnorm_fused_kernel<kMode, true><<<grid, kThreads, 0, ctx->stream>>>(out, momOut, dg, db, momIn, x, dy, g, b, WH, C, N, eps, relu);
-  else     bnorm_fused_kernel<kMode, false><<<grid, kThreads, 0, ctx->stream>>>(out, momOut, dg, db, momIn, x, dy, g, b, WH, C, N, eps, relu);
+  if (vec) vlb::launch(ctx->stream, bnorm_fused_kernel<kMode, true>, grid, kThreads, 0, out, momOut, dg, db, momIn, x, dy, g, b, WH, C, N, eps, relu);
+  else     vlb::launch(ctx->stream, bnorm_fused_kernel<kMode, false>, grid, kThreads, 0, out, momOut, dg, db, momIn, x, dy, g, b, WH, C, N, eps, relu);
   VLB_LAUNCHED(ctx, 1);
 }
 
@@ -288,6 +290,7 @@ __global__ void bnorm_coef_kernel(float4* __restrict__ cf, float const* __restri
                                   float const* __restrict__ g, float const* __restrict__ b,
                                   float const* __restrict__ dg, float const* __restrict__ db, int C, float mass)
 {
+  vlb::pdl_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   float mean = moments[c], sigma = moments[c + C];
@@ -306,6 +309,7 @@ template <bool kVec>
 __global__ void bnorm_fwd_apply_kernel(float* __restrict__ y, float const* __restrict__ x,
                                        float4 const* __restrict__ cf, int WH, int C, size_t total)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   if (kVec) {
     size_t total4 = total >> 2;
@@ -335,6 +339,7 @@ __global__ void bnorm_bwd_apply_kernel(float* __restrict__ dx, float const* __re
                                        float const* __restrict__ dy, float4 const* __restrict__ cf,
                                        int WH, int C, size_t total)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   if (kVec) {
     size_t total4 = total >> 2;
@@ -378,8 +383,8 @@ void launch_reduce(vlb_ctx* ctx, bool vec, float* momOut, float* dg, float* db, 
                    float const* x, float const* dy, int WH, int C, int N, float eps)
 {
   dim3 grid(C, kCluster);
-  if (vec) bnorm_reduce_kernel<kMode, true><<<grid, kThreads, 0, ctx->stream>>>(momOut, dg, db, momIn, x, dy, WH, C, N, eps);
-  else     bnorm_reduce_kernel<kMode, false><<<grid, kThreads, 0, ctx->stream>>>(momOut, dg, db, momIn, x, dy, WH, C, N, eps);
+  if (vec) vlb::launch(ctx->stream, bnorm_reduce_kernel<kMode, true>, grid, kThreads, 0, momOut, dg, db, momIn, x, dy, WH, C, N, eps);
+  else     vlb::launch(ctx->stream, bnorm_reduce_kernel<kMode, false>, grid, kThreads, 0, momOut, dg, db, momIn, x, dy, WH, C, N, eps);
   VLB_LAUNCHED(ctx, 1);
 }
 
@@ -411,12 +416,12 @@ static int forward_common(vlb_ctx* ctx, float* Y, float* momOut, float const* mo
     launch_fused<0>(ctx, vec_ok(WH, Y, X, X), Y, momOut, nullptr, nullptr, nullptr, X, nullptr, g, b, WH, C, N, (float)eps, relu);
     return vlb::check_launch(ctx, where);
   }
-  bnorm_coef_kernel<<<vlb::ceil_div(C, 256), 256, 0, ctx->stream>>>(cf, mom, g, b, nullptr, nullptr, C, 0.f);
+  vlb::launch(ctx->stream, bnorm_coef_kernel, vlb::ceil_div(C, 256), 256, 0, cf, mom, g, b, nullptr, nullptr, C, 0.f);
   size_t total = (size_t)WH * C * N;
   bool vec = vec_ok(WH, Y, X, X);
   unsigned grid = vlb::grid_for(vec ? total / 4 : total, kThreads, ctx->smCount * 16);
-  if (vec) bnorm_fwd_apply_kernel<true><<<grid, kThreads, 0, ctx->stream>>>(Y, X, cf, WH, C, total);
-  else     bnorm_fwd_apply_kernel<false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, cf, WH, C, total);
+  if (vec) vlb::launch(ctx->stream, bnorm_fwd_apply_kernel<true>, grid, kThreads, 0, Y, X, cf, WH, C, total);
+  else     vlb::launch(ctx->stream, bnorm_fwd_apply_kernel<false>, grid, kThreads, 0, Y, X, cf, WH, C, total);
   VLB_LAUNCHED(ctx, 2);
   return vlb::check_launch(ctx, where);
 }
@@ -552,14 +557,14 @@ extern "C" int vlb_bnorm_backward_noalloc(void* cudaStream, float* dX, float* dG
   int WH = H * W;
   bool vec = vec_ok(WH, X, dY, dX);
   dim3 grid(C, kCluster);
-  if (vec) bnorm_reduce_kernel<1, true><<<grid, kThreads, 0, stream>>>(mom, dG, dB, nullptr, X, dY, WH, C, N, (float)eps);
-  else     bnorm_reduce_kernel<1, false><<<grid, kThreads, 0, stream>>>(mom, dG, dB, nullptr, X, dY, WH, C, N, (float)eps);
+  if (vec) vlb::launch(stream, bnorm_reduce_kernel<1, true>, grid, kThreads, 0, mom, dG, dB, nullptr, X, dY, WH, C, N, (float)eps);
+  else     vlb::launch(stream, bnorm_reduce_kernel<1, false>, grid, kThreads, 0, mom, dG, dB, nullptr, X, dY, WH, C, N, (float)eps);
   float mass = (float)((long long)WH * N);
-  bnorm_coef_kernel<<<vlb::ceil_div(C, 256), 256, 0, stream>>>(cf, mom, g, nullptr, dG, dB, C, mass);
+  vlb::launch(stream, bnorm_coef_kernel, vlb::ceil_div(C, 256), 256, 0, cf, mom, g, nullptr, dG, dB, C, mass);
   size_t total = (size_t)WH * C * N;
   unsigned blocks = vlb::grid_for(vec ? total / 4 : total, kThreads, 148 * 16);
-  if (vec) bnorm_bwd_apply_kernel<true><<<blocks, kThreads, 0, stream>>>(dX, X, dY, cf, WH, C, total);
-  else     bnorm_bwd_apply_kernel<false><<<blocks, kThreads, 0, stream>>>(dX, X, dY, cf, WH, C, total);
+  if (vec) vlb::launch(stream, bnorm_bwd_apply_kernel<true>, blocks, kThreads, 0, dX, X, dY, cf, WH, C, total);
+  else     vlb::launch(stream, bnorm_bwd_apply_kernel<false>, blocks, kThreads, 0, dX, X, dY, cf, WH, C, total);
   e = cudaPeekAtLastError();
   if (e != cudaSuccess) {
     report(errbuf, errlen, cudaGetErrorString(e));

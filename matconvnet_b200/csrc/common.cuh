@@ -107,6 +107,28 @@ inline unsigned grid_for(size_t n, int threads, int maxBlocks = 148 * 16)
 
 #ifdef __CUDACC__
 namespace vlb {
+// Programmatic dependent launch.  Every kernel of the library is launched with leave to start before the kernel in front of it in the
+// stream has finished, and waits, before its first access to memory, until everything in front of it has completed and is visible.  The
+// kernels give no early sign of their own: a successor's blocks take the places of finished ones during the last of this kernel's blocks,
+// so its launch and prologue overlap that tail -- 1 to 2.8 us per kernel otherwise, a fifth of the time of the small networks.  (With the
+// sign given at the start of every kernel -- successors placed as soon as all blocks of this kernel are -- waiting blocks hold the
+// places that running ones would have used: LeNet block 172 us, CIFAR step 492, residual block 1215, VGG-16 step 37.0 ms; without it 137, 466,
+// 1140, 36.3 ms; without any of this 168, 563, 1199, 36.5 ms.)  Kernels of other libraries in the stream are launched without that leave
+// and see no difference.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch errors are sticky until read: the callers' check_launch reports them.
+template <class... E, class... A>
+inline void launch(cudaStream_t stream, void (*kernel)(E...), dim3 grid, dim3 block, size_t smem, A&&... args)
+{
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = &attr; cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<E>(args)...);
+}
+
 // Division by a small number with a multiply: exact for i * d < 2^32.
 struct FastDiv {
   unsigned d, m;

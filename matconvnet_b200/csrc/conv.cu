@@ -21,6 +21,7 @@ template <bool kVec>
 __global__ void __cluster_dims__(1, kCluster, 1) __launch_bounds__(kThreads)
 conv_dbias_kernel(float* __restrict__ db, float const* __restrict__ dy, int P, int K, int N)
 {
+  vlb::pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float part;
   __shared__ float warpRed[kThreads / 32];
@@ -63,14 +64,15 @@ int launch_dbias(vlb_ctx* ctx, float* db, float const* dY, int P, int K, int N)
   if (P == 1) return vlb::sum_parts(ctx, db, dY, K, K, N);      // 1x1 outputs (fully connected layers): db[k] = sum over images of dy[k + K*n]
   bool vec = (P % 4 == 0) && ((((uintptr_t)dY) & 15) == 0);
   dim3 grid(K, kCluster);
-  if (vec) conv_dbias_kernel<true><<<grid, kThreads, 0, ctx->stream>>>(db, dY, P, K, N);
-  else     conv_dbias_kernel<false><<<grid, kThreads, 0, ctx->stream>>>(db, dY, P, K, N);
+  if (vec) vlb::launch(ctx->stream, conv_dbias_kernel<true>, grid, kThreads, 0, db, dY, P, K, N);
+  else     vlb::launch(ctx->stream, conv_dbias_kernel<false>, grid, kThreads, 0, db, dY, P, K, N);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "conv_dbias");
 }
 
 __global__ void copy_kernel(float* dst, float const* src, size_t n)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = src[i];
 }
@@ -282,7 +284,7 @@ int vlb_fc_forward(vlb_ctx* ctx, float* Y, float const* X, float const* F, float
     // null filters: copy (reference bits/nnfullyconnected.cu:71-76), then the bias
     VLB_REQUIRE(ctx, d && Y && X, "fc_forward: null tensor");
     size_t n = (size_t)d->H * d->W * d->C * d->N;
-    copy_kernel<<<vlb::grid_for(n, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(Y, X, n);
+    vlb::launch(ctx->stream, copy_kernel, vlb::grid_for(n, 256, ctx->smCount * 8), 256, 0, Y, X, n);
     VLB_LAUNCHED(ctx, 1);
     if (b) return vlb_bias_forward(ctx, Y, 1.0, nullptr, 0.0, b, 1.0, 1, 1, d->H * d->W * d->C, d->N);
     return vlb::check_launch(ctx, "vlb_fc_forward");
@@ -301,7 +303,7 @@ int vlb_fc_backward(vlb_ctx* ctx, float* dX, float* dF, float* db, float const* 
     VLB_REQUIRE(ctx, d && dY, "fc_backward: null tensor");
     size_t n = (size_t)d->H * d->W * d->C * d->N;
     if (dX) {
-      copy_kernel<<<vlb::grid_for(n, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(dX, dY, n);
+      vlb::launch(ctx->stream, copy_kernel, vlb::grid_for(n, 256, ctx->smCount * 8), 256, 0, dX, dY, n);
       VLB_LAUNCHED(ctx, 1);
     }
     if (db) return launch_dbias(ctx, db, dY, 1, d->H * d->W * d->C, d->N);

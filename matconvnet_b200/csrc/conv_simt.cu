@@ -144,6 +144,7 @@ struct WgradOp {
 template <class Op>
 __global__ void __launch_bounds__(kThreads) igemm_simt_kernel(Op op)
 {
+  vlb::pdl_wait();
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
   int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(kThreads) igemm_simt_kernel(Op op)
 // dF[e] = sum over splits (ascending) of partial[s][e]
 __global__ void splitk_reduce_kernel(float* __restrict__ out, float const* __restrict__ part, size_t n, int splits)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
     float s = part[e];
@@ -229,7 +231,7 @@ int conv_fprop_simt(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, fl
   op.M = (int)M; op.Nn = g.Kg; op.R = g.FH * g.FW * g.FC; op.splits = 1;
   dim3 grid(ceil_div(op.M, BM), ceil_div(op.Nn, BN), g.G);
   VLB_REQUIRE(ctx, grid.y <= 65535 && grid.z <= 65535, "conv: too many filters or groups");
-  igemm_simt_kernel<FpropOp><<<grid, kThreads, 0, ctx->stream>>>(op);
+  vlb::launch(ctx->stream, igemm_simt_kernel<FpropOp>, grid, kThreads, 0, op);
   VLB_LAUNCHED(ctx, 1);
   return check_launch(ctx, "conv_fprop_simt");
 }
@@ -243,7 +245,7 @@ int conv_dgrad_simt(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, 
   op.M = (int)M; op.Nn = g.FC; op.R = g.FH * g.FW * g.Kg; op.splits = 1;
   dim3 grid(ceil_div(op.M, BM), ceil_div(op.Nn, BN), g.G);
   VLB_REQUIRE(ctx, grid.y <= 65535 && grid.z <= 65535, "conv: too many channels or groups");
-  igemm_simt_kernel<DgradOp><<<grid, kThreads, 0, ctx->stream>>>(op);
+  vlb::launch(ctx->stream, igemm_simt_kernel<DgradOp>, grid, kThreads, 0, op);
   VLB_LAUNCHED(ctx, 1);
   return check_launch(ctx, "conv_dgrad_simt");
 }
@@ -275,10 +277,10 @@ int conv_wgrad_simt(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, 
   }
   dim3 grid(ceil_div(op.M, BM), ceil_div(op.Nn, BN), g.G * splits);
   VLB_REQUIRE(ctx, grid.y <= 65535 && grid.z <= 65535, "conv: too many filters or groups");
-  igemm_simt_kernel<WgradOp><<<grid, kThreads, 0, ctx->stream>>>(op);
+  vlb::launch(ctx->stream, igemm_simt_kernel<WgradOp>, grid, kThreads, 0, op);
   VLB_LAUNCHED(ctx, 1);
   if (splits > 1) {
-    splitk_reduce_kernel<<<grid_for(nF, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(dF, op.out, nF, splits);
+    vlb::launch(ctx->stream, splitk_reduce_kernel, grid_for(nF, 256, ctx->smCount * 8), 256, 0, dF, op.out, nF, splits);
     VLB_LAUNCHED(ctx, 1);
   }
   return check_launch(ctx, "conv_wgrad_simt");

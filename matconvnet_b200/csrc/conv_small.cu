@@ -61,6 +61,7 @@ __device__ __forceinline__ float filter_at(SmallParams const& p, int fh, int fw,
 template <int KC>
 __global__ void __launch_bounds__(kThreads) conv_small_r_kernel(SmallParams p)
 {
+  vlb::pdl_wait();
   extern __shared__ float4 smem4[];
   float* fs = reinterpret_cast<float*>(smem4);                 // [R][KC]
   int const taps = p.FH * p.FW, R = taps * p.Cin;
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(kThreads) conv_small_r_kernel(SmallParams p)
 template <int KC, int FH>
 __global__ void __launch_bounds__(kThreads) conv_small_r4_kernel(SmallParams p)
 {
+  vlb::pdl_wait();
   extern __shared__ float4 smem4[];
   float* fs = reinterpret_cast<float*>(smem4);                 // [R][KC], r = fh + FH*(fw + FW*c)
   int const taps = FH * p.FW, R = taps * p.Cin;
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(kThreads) conv_small_r4_kernel(SmallParams p)
 template <int NC>
 __global__ void __launch_bounds__(kThreads) conv_small_n_kernel(SmallParams p)
 {
+  vlb::pdl_wait();
   extern __shared__ float4 smem4[];
   float* fs = reinterpret_cast<float*>(smem4);                 // [taps][Cin][NC]
   int const taps = p.FH * p.FW;
@@ -252,6 +255,7 @@ __global__ void __launch_bounds__(kThreads) conv_small_n_kernel(SmallParams p)
 template <int NC>
 __global__ void __launch_bounds__(kThreads) conv_small_n4_kernel(SmallParams p)
 {
+  vlb::pdl_wait();
   extern __shared__ float4 smem4[];
   float* fs = reinterpret_cast<float*>(smem4);                 // [tap][cin][4]
   int const taps = 3 * p.FW;
@@ -331,6 +335,7 @@ __device__ __forceinline__ void sn_cp_async4(float* dst, float const* src, bool 
 template <int kFH, int kC>
 __global__ void __launch_bounds__(kSnThreads) conv_small_n_tile_kernel(SmallParams p, int quads, int cols, int tilesH, int tilesW, int vec)
 {
+  vlb::pdl_wait();
   extern __shared__ float4 smem4[];
   int const pitch = 4 * quads + 4, width = cols + p.FW - 1, plane = pitch * width;      // rows of a tile: 4*quads + kFH - 1 <= pitch (kFH <= 5)
   float4* const ws = smem4;                                                               // [channel][fw][fh], four output channels
@@ -436,6 +441,7 @@ __device__ __forceinline__ void ws_cp_async_wait() { asm volatile("cp.async.comm
 __global__ void __launch_bounds__(kWsThreads)
 conv_wgrad_small_kernel(SmallParams p, float const* __restrict__ dy, float* __restrict__ part, long long M, int chunksPerBlock)
 {
+  vlb::pdl_wait();
   extern __shared__ __align__(16) float wsSmem[];
   float (*xs)[kWsRP] = reinterpret_cast<float (*)[kWsRP]>(wsSmem);                                  // [chunk][28]: the chunk's windows
   float (*dys)[kWsChunk + 1] = reinterpret_cast<float (*)[kWsChunk + 1]>(wsSmem + kWsChunk * kWsRP); // [filter][chunk + 1]: dY of the chunk
@@ -523,6 +529,7 @@ conv_wgrad_small_kernel(SmallParams p, float const* __restrict__ dy, float* __re
 __global__ void conv_wgrad_small_finish_kernel(float* __restrict__ dF, float* __restrict__ db, float const* __restrict__ part,
                                                int R, int K, int blocks)
 {
+  vlb::pdl_wait();
   // 32 values per block, every eighth partial result to each of its eight warps (one thread per value was 10.8 us of load latency)
   __shared__ float red[8][32];
   int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = (int)blockIdx.x * 32 + lane, total = K * kWsRP;
@@ -576,17 +583,17 @@ int conv_fprop_small(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, f
     constexpr int KC = 16;
     dim3 grid4((unsigned)std::min<long long>(ceil_div(M / 4, kThreads), (long long)ctx->smCount * 8), (unsigned)ceil_div(g.K, KC));
     size_t const smem4 = sizeof(float) * (size_t)R * KC;
-    if (g.FH == 3) conv_small_r4_kernel<KC, 3><<<grid4, kThreads, smem4, ctx->stream>>>(p);
-    else           conv_small_r4_kernel<KC, 5><<<grid4, kThreads, smem4, ctx->stream>>>(p);
+    if (g.FH == 3) vlb::launch(ctx->stream, conv_small_r4_kernel<KC, 3>, grid4, kThreads, smem4, p);
+    else           vlb::launch(ctx->stream, conv_small_r4_kernel<KC, 5>, grid4, kThreads, smem4, p);
     VLB_LAUNCHED(ctx, 1);
     return check_launch(ctx, "conv_fprop_small");
   }
   int const KC = g.K > 32 ? 64 : (g.K > 16 ? 32 : 16);
   dim3 grid((unsigned)ceil_div(M, kThreads), (unsigned)ceil_div(g.K, KC));
   size_t const smem = sizeof(float) * (size_t)R * KC + sizeof(int2) * (size_t)R;
-  if (KC == 64) conv_small_r_kernel<64><<<grid, kThreads, smem, ctx->stream>>>(p);
-  else if (KC == 32) conv_small_r_kernel<32><<<grid, kThreads, smem, ctx->stream>>>(p);
-  else conv_small_r_kernel<16><<<grid, kThreads, smem, ctx->stream>>>(p);
+  if (KC == 64) vlb::launch(ctx->stream, conv_small_r_kernel<64>, grid, kThreads, smem, p);
+  else if (KC == 32) vlb::launch(ctx->stream, conv_small_r_kernel<32>, grid, kThreads, smem, p);
+  else vlb::launch(ctx->stream, conv_small_r_kernel<16>, grid, kThreads, smem, p);
   VLB_LAUNCHED(ctx, 1);
   return check_launch(ctx, "conv_fprop_small");
 }
@@ -615,9 +622,9 @@ int conv_wgrad_small(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, floa
     if (e != cudaSuccess) { cudaGetLastError(); return set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
     if (ctx->device >= 0 && ctx->device < 64) attrDone[ctx->device] = true;
   }
-  conv_wgrad_small_kernel<<<dim3((unsigned)blocksX, (unsigned)kGroups), kWsThreads, smem, ctx->stream>>>(p, dY, part, M, chunksPerBlock);
+  vlb::launch(ctx->stream, conv_wgrad_small_kernel, dim3((unsigned)blocksX, (unsigned)kGroups), kWsThreads, smem, p, dY, part, M, chunksPerBlock);
   int const n = g.K * kWsRP;
-  conv_wgrad_small_finish_kernel<<<ceil_div(n, 32), 256, 0, ctx->stream>>>(dF, db, part, R, g.K, blocksX);
+  vlb::launch(ctx->stream, conv_wgrad_small_finish_kernel, ceil_div(n, 32), 256, 0, dF, db, part, R, g.K, blocksX);
   VLB_LAUNCHED(ctx, 2);
   *dbDone = db != nullptr;
   return check_launch(ctx, "conv_wgrad_small");
@@ -642,7 +649,7 @@ int conv_dgrad_small(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F,
   // filter rows: fh' = 0..2 with pt' = 1 row of padding above; the input (dY) and the output (dX) have the same height
   if (g.FH == 3 && p.pt == 1 && g.dy == 1 && g.dx == 1 && g.Ho == g.H && g.H % 4 == 0 && g.C <= 3 &&
       (((uintptr_t)dX) & 15) == 0 && (((uintptr_t)dY) & 15) == 0) {
-    conv_small_n4_kernel<3><<<(unsigned)ceil_div(M / 4, kThreads), kThreads, smem, ctx->stream>>>(p);      // (one group of quads per block measured faster here than a bounded grid)
+    vlb::launch(ctx->stream, conv_small_n4_kernel<3>, (unsigned)ceil_div(M / 4, kThreads), kThreads, smem, p);      // (one group of quads per block measured faster here than a bounded grid)
     VLB_LAUNCHED(ctx, 1);
     return check_launch(ctx, "conv_dgrad_small");
   }
@@ -654,7 +661,7 @@ int conv_dgrad_small(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F,
     long long const blocks = (long long)tilesH * tilesW * g.N;
     if (tile <= 48 * 1024 && blocks < (1LL << 31)) {
       int const vec = g.H % 4 == 0 && (((uintptr_t)dX) & 15) == 0;
-#define VLB_SN(fh, c) conv_small_n_tile_kernel<fh, c><<<(unsigned)blocks, kSnThreads, tile, ctx->stream>>>(p, quads, cols, tilesH, tilesW, vec)
+#define VLB_SN(fh, c) vlb::launch(ctx->stream, conv_small_n_tile_kernel<fh, c>, (unsigned)blocks, kSnThreads, tile, p, quads, cols, tilesH, tilesW, vec)
       if (g.FH == 3) { if (g.C == 1) VLB_SN(3, 1); else if (g.C <= 3) VLB_SN(3, 3); else VLB_SN(3, 4); }
       else           { if (g.C == 1) VLB_SN(5, 1); else if (g.C <= 3) VLB_SN(5, 3); else VLB_SN(5, 4); }
 #undef VLB_SN
@@ -662,7 +669,7 @@ int conv_dgrad_small(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F,
       return check_launch(ctx, "conv_dgrad_small");
     }
   }
-  conv_small_n_kernel<4><<<(unsigned)ceil_div(M, kThreads), kThreads, smem, ctx->stream>>>(p);
+  vlb::launch(ctx->stream, conv_small_n_kernel<4>, (unsigned)ceil_div(M, kThreads), kThreads, smem, p);
   VLB_LAUNCHED(ctx, 1);
   return check_launch(ctx, "conv_dgrad_small");
 }

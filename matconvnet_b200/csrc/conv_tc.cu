@@ -497,6 +497,7 @@ __device__ __forceinline__ void issue_window2(float const* __restrict__ a, int o
 template <int kAMode, int kBMode, int kEpi, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
 {
+  vlb::pdl_wait();
   extern __shared__ uint8_t smemRaw[];
   __shared__ __align__(8) uint64_t fullBar[kMaxStages];
   __shared__ __align__(8) uint64_t emptyBar[kMaxStages];
@@ -1323,6 +1324,7 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
     else           tapLut[threadIdx.x] = make_int2((fw * p.a.dx - p.a.pl) * p.a.H + fh * p.a.dy - p.a.pt, fh | (fw << 5));
   }
   tc_fence_before();
+  vlb::pdl_wait();        // (everything above touches this CTA's own shared and tensor memory only)
   __syncthreads();
   tc_fence_after();
   uint32_t const tmemAcc = tmemBase;
@@ -1911,6 +1913,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) conv_ts_gen_kernel(const __grid
 // over dY is the data gradient of a stride-1 convolution.
 __global__ void flip_filters_kernel(float* __restrict__ ft, float const* __restrict__ f, int FH, int FW, int C, int K)
 {
+  vlb::pdl_wait();
   size_t total = (size_t)FH * FW * C * K;
   size_t step = (size_t)gridDim.x * blockDim.x;
   for (size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x; o < total; o += step) {
@@ -1928,6 +1931,7 @@ __global__ void flip_filters_kernel(float* __restrict__ ft, float const* __restr
 template <bool kSplit, bool kRows>
 __global__ void prep_dense_tiles_kernel(float* __restrict__ out, float const* __restrict__ f, int N, int R, int BN, int numKb)
 {
+  vlb::pdl_wait();
   size_t const Rp = (size_t)numKb * 32;
   size_t const total = (size_t)((N + BN - 1) / BN) * BN * Rp;
   size_t const step = (size_t)gridDim.x * blockDim.x;
@@ -1966,6 +1970,7 @@ struct PrepBatch { PrepFilters p[kMaxTsProblems]; };
 template <bool kSplit>
 __global__ void __launch_bounds__(256) prep_filters_kernel(const __grid_constant__ PrepBatch b)
 {
+  vlb::pdl_wait();
   PrepFilters const& p = b.p[blockIdx.z];
   int const row = (int)blockIdx.x * 32 + ((int)threadIdx.x >> 3), chunk = (int)threadIdx.x & 7;
   if (row >= p.rows) return;
@@ -2008,6 +2013,7 @@ constexpr int kPrepRows = 8, kMaxPrepTaps = 45;
 template <bool kSplit>
 __global__ void __launch_bounds__(256) prep_filters_tile_kernel(const __grid_constant__ PrepBatch b)
 {
+  vlb::pdl_wait();
   extern __shared__ float prepSmem[];
   PrepFilters const& p = b.p[blockIdx.z];
   int const r0 = (int)blockIdx.x * kPrepRows, cb = (int)blockIdx.y, taps = p.tapsH * p.tapsW, FT = p.FH * p.FW, FTp = FT | 1;
@@ -2105,13 +2111,13 @@ void launch_prep(vlb_ctx* ctx, PrepBatch& prep, int n)
   if (whole && FT <= kMaxPrepTaps && elements >= 600000) {
     dim3 const grid(vlb::ceil_div(rows, kPrepRows), blocks, n);
     size_t const smem = sizeof(float) * kPrepRows * (32 * (size_t)(FT | 1) + 1);
-    if (split3) prep_filters_tile_kernel<true><<<grid, 256, smem, ctx->stream>>>(prep);
-    else        prep_filters_tile_kernel<false><<<grid, 256, smem, ctx->stream>>>(prep);
+    if (split3) vlb::launch(ctx->stream, prep_filters_tile_kernel<true>, grid, 256, smem, prep);
+    else        vlb::launch(ctx->stream, prep_filters_tile_kernel<false>, grid, 256, smem, prep);
     return;
   }
   dim3 const grid(vlb::ceil_div(rows, 32), groups, n);
-  if (split3) prep_filters_kernel<true><<<grid, 256, 0, ctx->stream>>>(prep);
-  else        prep_filters_kernel<false><<<grid, 256, 0, ctx->stream>>>(prep);
+  if (split3) vlb::launch(ctx->stream, prep_filters_kernel<true>, grid, 256, 0, prep);
+  else        vlb::launch(ctx->stream, prep_filters_kernel<false>, grid, 256, 0, prep);
 }
 
 // dY of a filter gradient as tile images, B(n, r) = dY[pixel, n, image] with r = pixel + P*image, for planes that are a multiple of
@@ -2129,6 +2135,7 @@ __global__ void __launch_bounds__(kPrepThreads)
 prep_dy_tiles_kernel(float* __restrict__ out, float const* __restrict__ dy, int N, int R, int P, int Pp, int BN, int numKb,
                      float* __restrict__ db, float* __restrict__ dbPart, unsigned* __restrict__ tickets, int Kg, int tilesPerGroup)
 {
+  vlb::pdl_wait();
   __shared__ float red[kPrepThreads / 32];
   __shared__ bool last;
   int const tile = blockIdx.y / BN, row = blockIdx.y - tile * BN, grp = tile / tilesPerGroup;
@@ -2215,7 +2222,7 @@ float const* prep_dense_tiles(vlb_ctx* ctx, float const* f, int N, int R, int BN
   float* tiles = (float*)vlb::workspace(ctx, b_tiles_bytes(ctx, N, BN, numKb) + extraBytes);
   if (!tiles) return nullptr;
   unsigned const grid = vlb::grid_for(total, 256, ctx->smCount * 8);
-#define VLB_PD(split, r) prep_dense_tiles_kernel<split, r><<<grid, 256, 0, ctx->stream>>>(tiles, f, N, R, BN, numKb)
+#define VLB_PD(split, r) vlb::launch(ctx->stream, prep_dense_tiles_kernel<split, r>, grid, 256, 0, tiles, f, N, R, BN, numKb)
   if (split3) { if (rows) VLB_PD(true, true); else VLB_PD(true, false); }
   else        { if (rows) VLB_PD(false, true); else VLB_PD(false, false); }
 #undef VLB_PD
@@ -2260,7 +2267,7 @@ float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, i
   float* dbPart = db ? (float*)(ws + tileBytes + extraBytes) : nullptr;
   unsigned* tickets = (unsigned*)((char*)ctx->deviceStatus + 256);
   dim3 grid(bx, (unsigned)rows);
-#define VLB_PDY(split, v) prep_dy_tiles_kernel<split, v><<<grid, kPrepThreads, 0, ctx->stream>>>(tiles, dY, K, R, P, Pp, BN, numKb, db, dbPart, tickets, Kg, tpg)
+#define VLB_PDY(split, v) vlb::launch(ctx->stream, prep_dy_tiles_kernel<split, v>, grid, kPrepThreads, 0, tiles, dY, K, R, P, Pp, BN, numKb, db, dbPart, tickets, Kg, tpg)
   if (split3) { if (vec) VLB_PDY(true, true); else VLB_PDY(true, false); }
   else        { if (vec) VLB_PDY(false, true); else VLB_PDY(false, false); }
 #undef VLB_PDY
@@ -2309,7 +2316,7 @@ cudaError_t allow_large_smem(int device)
 }
 
 template <int kAMode, int kBMode, int kEpi>
-int launch(vlb_ctx* ctx, Params& p, int splits, char const* where)
+int launch_gemm(vlb_ctx* ctx, Params& p, int splits, char const* where)
 {
   bool split3 = ctx->precision == VLB_PRECISION_3XTF32;
   uint32_t stageBytes = (split3 ? 2u : 1u) * (BM * BK * 4 + (uint32_t)p.BN * BK * 4);
@@ -2333,10 +2340,10 @@ int launch(vlb_ctx* ctx, Params& p, int splits, char const* where)
   }
   if (split3) {
     e = allow_large_smem<tc_gemm_kernel<kAMode, kBMode, kEpi, true>>(ctx->device);
-    if (e == cudaSuccess) tc_gemm_kernel<kAMode, kBMode, kEpi, true><<<grid, kThreads, smemBytes, ctx->stream>>>(p);
+    if (e == cudaSuccess) vlb::launch(ctx->stream, tc_gemm_kernel<kAMode, kBMode, kEpi, true>, grid, kThreads, smemBytes, p);
   } else {
     e = allow_large_smem<tc_gemm_kernel<kAMode, kBMode, kEpi, false>>(ctx->device);
-    if (e == cudaSuccess) tc_gemm_kernel<kAMode, kBMode, kEpi, false><<<grid, kThreads, smemBytes, ctx->stream>>>(p);
+    if (e == cudaSuccess) vlb::launch(ctx->stream, tc_gemm_kernel<kAMode, kBMode, kEpi, false>, grid, kThreads, smemBytes, p);
   }
   if (record) { cudaEventRecord(rec.stop, ctx->stream); ctx->prof.push_back(rec); }
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
@@ -2458,7 +2465,7 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
   bool const narrow = p.BN <= 64;
   auto go = [&](auto kernel) {
     e = allow_large_smem<decltype(kernel)::value>(ctx->device);
-    if (e == cudaSuccess) decltype(kernel)::value<<<grid, kTsThreads, smemBytes, ctx->stream>>>(p, map);
+    if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, grid, kTsThreads, smemBytes, p, map);
   };
 #define VLB_TS(split, mode, nar) go(std::integral_constant<decltype(&conv_ts_kernel<split, mode, nar>), &conv_ts_kernel<split, mode, nar>>{})
   if (split3) {
@@ -2562,10 +2569,10 @@ int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* whe
   cudaError_t e;
   if (split3) {
     e = allow_large_smem<conv_ts_kernel<true, 2, false>>(ctx->device);
-    if (e == cudaSuccess) conv_ts_kernel<true, 2, false><<<grid, kTsThreadsRows, smemBytes, ctx->stream>>>(p, map);
+    if (e == cudaSuccess) vlb::launch(ctx->stream, conv_ts_kernel<true, 2, false>, grid, kTsThreadsRows, smemBytes, p, map);
   } else {
     e = allow_large_smem<conv_ts_kernel<false, 2, false>>(ctx->device);
-    if (e == cudaSuccess) conv_ts_kernel<false, 2, false><<<grid, kTsThreadsRows, smemBytes, ctx->stream>>>(p, map);
+    if (e == cudaSuccess) vlb::launch(ctx->stream, conv_ts_kernel<false, 2, false>, grid, kTsThreadsRows, smemBytes, p, map);
   }
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
@@ -2861,7 +2868,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
   cudaError_t e;
   auto go = [&](auto kernel) {
     e = allow_large_smem<decltype(kernel)::value>(ctx->device);
-    if (e == cudaSuccess) decltype(kernel)::value<<<given, kTsThreads, smemBytes, ctx->stream>>>(b);
+    if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, given, kTsThreads, smemBytes, b);
   };
 #define VLB_TSG(split, nar) go(std::integral_constant<decltype(&conv_ts_gen_kernel<split, nar>), &conv_ts_gen_kernel<split, nar>>{})
   if (split3) { if (BN <= 64) VLB_TSG(true, true); else VLB_TSG(true, false); }
@@ -3038,13 +3045,13 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
     if (splits == 1) {
       p.e.out = Y; p.e.bias = b;
       p.e.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
-      return launch<OP_DENSE_K, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "fc_fprop_tc");
+      return launch_gemm<OP_DENSE_K, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "fc_fprop_tc");
     }
     size_t nOut = (size_t)g.K * g.N;
     float* part = (float*)workspace(ctx, sizeof(float) * nOut * splits);
     if (!part) return ctx->lastError;
     p.e.out = part; p.e.splitStride = (long long)nOut;
-    int rc = launch<OP_DENSE_K, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "fc_fprop_tc");
+    int rc = launch_gemm<OP_DENSE_K, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "fc_fprop_tc");
     if (rc) return rc;
     SumEpilogue epi;
     epi.bias = b; epi.K = g.K; epi.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
@@ -3081,7 +3088,7 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
     int const rc = launch_ts(ctx, p, "conv_fprop_ts");
     return rc ? rc : sum_parts(ctx, Y, part, nOut, nOut, p.splits, epi);
   }
-  return launch<OP_IM2COL, OP_DENSE_K, EPI_CONV>(ctx, p, 1, "conv_fprop_tc");
+  return launch_gemm<OP_IM2COL, OP_DENSE_K, EPI_CONV>(ctx, p, 1, "conv_fprop_tc");
 }
 
 int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
@@ -3103,7 +3110,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     p.BN = pick_bn(p.N);
     p.numKb = ceil_div(p.R, BK); p.kbPerSplit = p.numKb;
     p.e = Epilogue{}; p.e.out = dX; p.e.ldd = V;
-    return launch<OP_DENSE_MN, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "fc_dgrad_tc");
+    return launch_gemm<OP_DENSE_MN, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "fc_dgrad_tc");
   }
   if (g.G != 1 || g.sy != 1 || g.sx != 1 || g.K % 32 != 0 || g.FH * g.FW > 64) {
     ProfScope prof(ctx, kProfDgrad);
@@ -3139,7 +3146,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     size_t nF = (size_t)g.FH * g.FW * g.FC * g.K;
     float* ft = (float*)workspace(ctx, sizeof(float) * nF);
     if (!ft) return ctx->lastError;
-    flip_filters_kernel<<<grid_for(nF, 256, ctx->smCount * 8), 256, 0, ctx->stream>>>(ft, F, g.FH, g.FW, g.C, g.K);
+    vlb::launch(ctx->stream, flip_filters_kernel, grid_for(nF, 256, ctx->smCount * 8), 256, 0, ft, F, g.FH, g.FW, g.C, g.K);
     VLB_LAUNCHED(ctx, 1);
     p.b.ptr = ft; p.b.vec = (V % 4 == 0);
   }
@@ -3155,7 +3162,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     int const rc = launch_ts(ctx, p, "conv_dgrad_ts");
     return rc ? rc : sum_parts(ctx, dX, part, nOut, nOut, p.splits, epi);
   }
-  return launch<OP_IM2COL, OP_DENSE_K, EPI_CONV>(ctx, p, 1, "conv_dgrad_tc");
+  return launch_gemm<OP_IM2COL, OP_DENSE_K, EPI_CONV>(ctx, p, 1, "conv_dgrad_tc");
 }
 
 int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float const* X, float const* dY, bool* dbDone)
@@ -3178,7 +3185,7 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
     p.BN = p.N > 64 ? 128 : (p.N > 32 ? 64 : 32);     // MN-major tiles are built from 32-column atoms
     p.numKb = ceil_div(p.R, BK); p.kbPerSplit = p.numKb;
     p.e = Epilogue{}; p.e.out = dF; p.e.ldd = V;
-    return launch<OP_DENSE_MN, OP_DENSE_MN, EPI_PLAIN>(ctx, p, 1, "fc_wgrad_tc");
+    return launch_gemm<OP_DENSE_MN, OP_DENSE_MN, EPI_PLAIN>(ctx, p, 1, "fc_wgrad_tc");
   }
   if (g.G == 1) {
     int const rc = conv_wgrad_ts(ctx, g, dF, db, X, dY, dbDone);
@@ -3211,11 +3218,11 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
   p.pipelined = 1;
   if (splits == 1) {
     p.e.out = dF;
-    return launch<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "conv_wgrad_tc");
+    return launch_gemm<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "conv_wgrad_tc");
   }
   float* const part = (float*)((char*)p.bTiles + tileBytes);
   p.e.out = part; p.e.splitStride = (long long)nF;
-  int rc = launch<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "conv_wgrad_tc");
+  int rc = launch_gemm<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "conv_wgrad_tc");
   if (rc) return rc;
   return sum_parts(ctx, dF, part, nF, nF, splits);
 }

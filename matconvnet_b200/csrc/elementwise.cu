@@ -15,6 +15,7 @@ inline bool aligned16(void const* p) { return (((uintptr_t)p) & 15) == 0; }
 // y and x may be the same array (element i is read before it is written)
 __global__ void relu_fwd_kernel(float* y, float const* x, size_t n, bool vec)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x, i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (vec) {
     size_t n4 = n >> 2;
@@ -34,6 +35,7 @@ __global__ void relu_fwd_kernel(float* y, float const* x, size_t n, bool vec)
 // dx may be dy (every element is read before it is written, by the same thread)
 __global__ void relu_bwd_kernel(float* dx, float const* __restrict__ x, float const* dy, size_t n, bool vec)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x, i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (vec) {
     size_t n4 = n >> 2;
@@ -56,6 +58,7 @@ __device__ __forceinline__ float taccum1(float alpha, float a, float beta, float
 
 __global__ void taccum_kernel(float* y, float alpha, float const* a, float beta, float const* b, size_t n, bool vec)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x, i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (vec) {
     size_t n4 = n >> 2;
@@ -129,6 +132,7 @@ struct UpdateBatch { int count, solver; SgdParams sgd; SolverParams so; UpdateIt
 template <bool kSgd, bool kTwo>
 __global__ void __launch_bounds__(kThreads) update_kernel(const __grid_constant__ UpdateBatch b)
 {
+  vlb::pdl_wait();
   int lo = 0, hi = b.count - 1;               // the last item whose first block is not behind this one
   while (lo < hi) {
     int const mid = (lo + hi + 1) >> 1;
@@ -177,8 +181,8 @@ int launch_updates(vlb_ctx* ctx, UpdateBatch& b, bool two, int count, vlb_param_
   b.count = 0;
   auto flush = [&] {
     if (b.count == 0) return;
-    if (two) update_kernel<kSgd, true><<<blocks, kThreads, 0, ctx->stream>>>(b);
-    else     update_kernel<kSgd, false><<<blocks, kThreads, 0, ctx->stream>>>(b);
+    if (two) vlb::launch(ctx->stream, update_kernel<kSgd, true>, blocks, kThreads, 0, b);
+    else     vlb::launch(ctx->stream, update_kernel<kSgd, false>, blocks, kThreads, 0, b);
     VLB_LAUNCHED(ctx, 1);
     b.count = 0; blocks = 0;
   };
@@ -199,6 +203,7 @@ int launch_updates(vlb_ctx* ctx, UpdateBatch& b, bool two, int count, vlb_param_
 
 __global__ void sum_kernel(float* y, float const* a, float const* b, size_t n, bool vec)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x, i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (vec) {
     size_t n4 = n >> 2;
@@ -215,6 +220,7 @@ __global__ void sum_kernel(float* y, float const* a, float const* b, size_t n, b
 
 __global__ void scale_kernel(float* x, float alpha, size_t n, bool vec)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x, i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (vec) {
     size_t n4 = n >> 2;
@@ -235,6 +241,7 @@ __global__ void scale_kernel(float* x, float alpha, size_t n, bool vec)
 __global__ void bias_fwd_kernel(float* __restrict__ y, float ym, float const* __restrict__ x, float xm,
                                 float const* __restrict__ b, float bm, int P, int K, size_t planes, int mode)
 {
+  vlb::pdl_wait();
   for (size_t plane = blockIdx.y; plane < planes; plane += gridDim.y) {
     int k = (int)(plane % K);
     float bv = (mode == 2) ? 0.f : __fmul_rn(bm, b[k]);
@@ -253,6 +260,7 @@ __global__ void bias_fwd_kernel(float* __restrict__ y, float ym, float const* __
 __global__ void bias_fwd_flat_kernel(float* __restrict__ y, float ym, float const* __restrict__ x, float xm,
                                      float const* __restrict__ b, float bm, int P, int K, size_t total, int mode)
 {
+  vlb::pdl_wait();
   size_t const step = (size_t)gridDim.x * blockDim.x;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += step) {
     int const k = (int)((e / P) % K);
@@ -267,6 +275,7 @@ __global__ void bias_fwd_flat_kernel(float* __restrict__ y, float ym, float cons
 __global__ void bias_bwd_db_kernel(float* __restrict__ db, float beta, float bm, float const* __restrict__ dy,
                                    int P, int K, int N)
 {
+  vlb::pdl_wait();
   __shared__ float red[32];
   int k = blockIdx.x;
   float s = 0.f;
@@ -288,6 +297,7 @@ __global__ void bias_bwd_db_kernel(float* __restrict__ db, float beta, float bm,
 // dx = dxm*dx + xm*dy ; dxm == 0 means overwrite
 __global__ void axpby_kernel(float* dx, float dxm, float xm, float const* dy, size_t n)
 {
+  vlb::pdl_wait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     float v = __fmul_rn(xm, dy[i]);
@@ -326,6 +336,7 @@ __device__ float block_reduce(float v, bool isMax, float* red)
 __global__ void softmaxloss_kernel(float* __restrict__ terms, float* __restrict__ dx, float const* __restrict__ x,
                                    float const* __restrict__ labels, float scale, int P, int C, int* __restrict__ status)
 {
+  vlb::pdl_wait();
   __shared__ float red[32];
   int p = blockIdx.x, n = blockIdx.y;
   float const* xp = x + p + (size_t)P * C * n;
@@ -358,6 +369,7 @@ __global__ void softmaxloss_kernel(float* __restrict__ terms, float* __restrict_
 // loss = (sum of terms) / N, one block, fixed order.
 __global__ void loss_finish_kernel(float* loss, float const* terms, int count, float invN)
 {
+  vlb::pdl_wait();
   __shared__ float red[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < count; i += blockDim.x) s += terms[i];
@@ -375,7 +387,7 @@ int vlb_relu_forward(vlb_ctx* ctx, float* Y, float const* X, size_t n)
   VLB_REQUIRE(ctx, Y && X, "relu_forward: null tensor");
   if (n == 0) return VLB_Success;
   bool vec = aligned16(Y) && aligned16(X);
-  relu_fwd_kernel<<<vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(Y, X, n, vec);
+  vlb::launch(ctx->stream, relu_fwd_kernel, vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, Y, X, n, vec);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_relu_forward");
 }
@@ -386,7 +398,7 @@ int vlb_relu_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, 
   VLB_REQUIRE(ctx, dX && X && dY, "relu_backward: null tensor");
   if (n == 0) return VLB_Success;
   bool vec = aligned16(dX) && aligned16(X) && aligned16(dY);
-  relu_bwd_kernel<<<vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(dX, X, dY, n, vec);
+  vlb::launch(ctx->stream, relu_bwd_kernel, vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, dX, X, dY, n, vec);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_relu_backward");
 }
@@ -397,7 +409,7 @@ int vlb_sum(vlb_ctx* ctx, float* Y, float const* A, float const* B, size_t n)
   VLB_REQUIRE(ctx, Y && A && B, "sum: null tensor");
   if (n == 0) return VLB_Success;
   bool vec = aligned16(Y) && aligned16(A) && aligned16(B);
-  sum_kernel<<<vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(Y, A, B, n, vec);
+  vlb::launch(ctx->stream, sum_kernel, vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, Y, A, B, n, vec);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_sum");
 }
@@ -408,7 +420,7 @@ int vlb_scale(vlb_ctx* ctx, float* x, double alpha, size_t n)
   VLB_REQUIRE(ctx, x, "scale: null tensor");
   if (n == 0) return VLB_Success;
   bool vec = aligned16(x);
-  scale_kernel<<<vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(x, (float)alpha, n, vec);
+  vlb::launch(ctx->stream, scale_kernel, vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, x, (float)alpha, n, vec);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_scale");
 }
@@ -419,7 +431,7 @@ int vlb_taccum(vlb_ctx* ctx, float* Y, double alpha, float const* A, double beta
   VLB_REQUIRE(ctx, Y && A && B, "taccum: null tensor");
   if (n == 0) return VLB_Success;
   bool vec = aligned16(Y) && aligned16(A) && aligned16(B);
-  taccum_kernel<<<vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(
+  vlb::launch(ctx->stream, taccum_kernel, vlb::grid_for(vec ? n / 4 + 1 : n, kThreads, ctx->smCount * 8), kThreads, 0, 
       Y, (float)alpha, A, (float)beta, B, n, vec);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_taccum");
@@ -490,13 +502,13 @@ int vlb_bias_forward(vlb_ctx* ctx, float* Y, double yMult, float const* X, doubl
   size_t planes = (size_t)K * N;
   if (P < 64) {
     size_t total = planes * (size_t)P;
-    bias_fwd_flat_kernel<<<vlb::grid_for(total, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(
+    vlb::launch(ctx->stream, bias_fwd_flat_kernel, vlb::grid_for(total, kThreads, ctx->smCount * 8), kThreads, 0, 
         Y, (float)yMult, xin, (float)xMult, b, (float)bMult, P, K, total, mode);
     VLB_LAUNCHED(ctx, 1);
     return vlb::check_launch(ctx, "vlb_bias_forward");
   }
   dim3 grid(vlb::ceil_div(P, kThreads) > 64 ? 64 : vlb::ceil_div(P, kThreads), (unsigned)(planes > 32768 ? 32768 : planes));
-  bias_fwd_kernel<<<grid, kThreads, 0, ctx->stream>>>(Y, (float)yMult, xin, (float)xMult, b, (float)bMult, P, K, planes, mode);
+  vlb::launch(ctx->stream, bias_fwd_kernel, grid, kThreads, 0, Y, (float)yMult, xin, (float)xMult, b, (float)bMult, P, K, planes, mode);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_bias_forward");
 }
@@ -509,12 +521,12 @@ int vlb_bias_backward(vlb_ctx* ctx, float* dX, double dXMult, float* db, double 
   VLB_REQUIRE(ctx, H > 0 && W > 0 && K > 0 && N > 0, "bias_backward: empty tensor");
   int P = H * W;
   if (db) {
-    bias_bwd_db_kernel<<<K, 256, 0, ctx->stream>>>(db, (float)dbMult, (float)bMult, dY, P, K, N);
+    vlb::launch(ctx->stream, bias_bwd_db_kernel, K, 256, 0, db, (float)dbMult, (float)bMult, dY, P, K, N);
     VLB_LAUNCHED(ctx, 1);
   }
   if (dX) {
     size_t n = (size_t)P * K * N;
-    axpby_kernel<<<vlb::grid_for(n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(dX, (float)dXMult, (float)xMult, dY, n);
+    vlb::launch(ctx->stream, axpby_kernel, vlb::grid_for(n, kThreads, ctx->smCount * 8), kThreads, 0, dX, (float)dXMult, (float)xMult, dY, n);
     VLB_LAUNCHED(ctx, 1);
   }
   return vlb::check_launch(ctx, "vlb_bias_backward");
@@ -529,8 +541,8 @@ int vlb_softmaxloss_forward(vlb_ctx* ctx, float* loss, float const* X, float con
   float* terms = (float*)vlb::workspace(ctx, sizeof(float) * (size_t)P * N);
   if (!terms) return vlb::pass_error(ctx, ctx->lastError, "vlb_softmaxloss_forward");
   int threads = C >= 256 ? 256 : (C >= 64 ? 64 : 32);
-  softmaxloss_kernel<<<dim3(P, N), threads, 0, ctx->stream>>>(terms, nullptr, X, labels, 0.f, P, C, ctx->deviceStatus);
-  loss_finish_kernel<<<1, 256, 0, ctx->stream>>>(loss, terms, P * N, 1.f / (float)N);
+  vlb::launch(ctx->stream, softmaxloss_kernel, dim3(P, N), threads, 0, terms, nullptr, X, labels, 0.f, P, C, ctx->deviceStatus);
+  vlb::launch(ctx->stream, loss_finish_kernel, 1, 256, 0, loss, terms, P * N, 1.f / (float)N);
   VLB_LAUNCHED(ctx, 2);
   return vlb::check_launch(ctx, "vlb_softmaxloss_forward");
 }
@@ -543,7 +555,7 @@ int vlb_softmaxloss_backward(vlb_ctx* ctx, float* dX, float const* X, float cons
   VLB_REQUIRE(ctx, H > 0 && W > 0 && C > 0 && N > 0 && N <= 65535, "softmaxloss_backward: bad shape");
   int P = H * W;
   int threads = C >= 256 ? 256 : (C >= 64 ? 64 : 32);
-  softmaxloss_kernel<<<dim3(P, N), threads, 0, ctx->stream>>>(nullptr, dX, X, labels, (float)dzdy / (float)N, P, C, ctx->deviceStatus);
+  vlb::launch(ctx->stream, softmaxloss_kernel, dim3(P, N), threads, 0, nullptr, dX, X, labels, (float)dzdy / (float)N, P, C, ctx->deviceStatus);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_softmaxloss_backward");
 }

@@ -14,6 +14,7 @@ template <int kN, int kRows, bool kVec>
 __global__ void __launch_bounds__(kThreads) fc_rows_kernel(float* __restrict__ y, float const* __restrict__ x, float const* __restrict__ f,
                                                            float const* __restrict__ bias, int V, int K, int N, int relu)
 {
+  vlb::pdl_wait();
   __shared__ float red[kThreads / 32][kRows * kN];
   int const k0 = (int)blockIdx.x * kRows;
   float acc[kRows][kN];
@@ -81,12 +82,12 @@ __global__ void __launch_bounds__(kThreads) fc_rows_kernel(float* __restrict__ y
 }
 
 template <int kN, int kRows>
-void launch(vlb_ctx* ctx, float* Y, float const* X, float const* F, float const* b, int V, int K, int N)
+void run(vlb_ctx* ctx, float* Y, float const* X, float const* F, float const* b, int V, int K, int N)
 {
   bool const vec = V % 4 == 0 && ((((uintptr_t)X) | ((uintptr_t)F)) & 15) == 0;
   unsigned const grid = (unsigned)vlb::ceil_div(K, kRows);
-  if (vec) fc_rows_kernel<kN, kRows, true><<<grid, kThreads, 0, ctx->stream>>>(Y, X, F, b, V, K, N, ctx->fuseRelu);
-  else     fc_rows_kernel<kN, kRows, false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, F, b, V, K, N, ctx->fuseRelu);
+  if (vec) vlb::launch(ctx->stream, fc_rows_kernel<kN, kRows, true>, grid, kThreads, 0, Y, X, F, b, V, K, N, ctx->fuseRelu);
+  else     vlb::launch(ctx->stream, fc_rows_kernel<kN, kRows, false>, grid, kThreads, 0, Y, X, F, b, V, K, N, ctx->fuseRelu);
 }
 
 }  // namespace
@@ -100,10 +101,10 @@ int fc_fprop_small(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, fl
   int const V = g.FH * g.FW * g.FC, N = g.N;
   if (N > 8 || V < 256) return VLB_Unsupported;
   bool const few = g.K < 8 * ctx->smCount;
-  if (N == 1)      { if (few) launch<1, 2>(ctx, Y, X, F, b, V, g.K, N); else launch<1, 4>(ctx, Y, X, F, b, V, g.K, N); }
-  else if (N == 2) { if (few) launch<2, 2>(ctx, Y, X, F, b, V, g.K, N); else launch<2, 4>(ctx, Y, X, F, b, V, g.K, N); }
-  else if (N <= 4) { if (few) launch<4, 2>(ctx, Y, X, F, b, V, g.K, N); else launch<4, 4>(ctx, Y, X, F, b, V, g.K, N); }
-  else             { if (few) launch<8, 2>(ctx, Y, X, F, b, V, g.K, N); else launch<8, 4>(ctx, Y, X, F, b, V, g.K, N); }
+  if (N == 1)      { if (few) run<1, 2>(ctx, Y, X, F, b, V, g.K, N); else run<1, 4>(ctx, Y, X, F, b, V, g.K, N); }
+  else if (N == 2) { if (few) run<2, 2>(ctx, Y, X, F, b, V, g.K, N); else run<2, 4>(ctx, Y, X, F, b, V, g.K, N); }
+  else if (N <= 4) { if (few) run<4, 2>(ctx, Y, X, F, b, V, g.K, N); else run<4, 4>(ctx, Y, X, F, b, V, g.K, N); }
+  else             { if (few) run<8, 2>(ctx, Y, X, F, b, V, g.K, N); else run<8, 4>(ctx, Y, X, F, b, V, g.K, N); }
   ctx->reluDone = ctx->fuseRelu;
   VLB_LAUNCHED(ctx, 1);
   return check_launch(ctx, "fc_fprop_small");

@@ -21,6 +21,7 @@ struct LrnParams { int P, C, N, m1, m2; float kappa, alpha, beta; };
 
 __global__ void lrn_forward_kernel(float* __restrict__ y, float const* __restrict__ x, LrnParams p)
 {
+  vlb::pdl_wait();
   size_t const total = (size_t)p.P * p.N, step = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
     size_t const n = i / p.P, pix = i - n * p.P;
@@ -39,6 +40,7 @@ __global__ void lrn_forward_kernel(float* __restrict__ y, float const* __restric
 __global__ void lrn_backward_kernel(float* __restrict__ dx, float* __restrict__ integral, float const* __restrict__ x,
                                     float const* __restrict__ dz, LrnParams p)
 {
+  vlb::pdl_wait();
   size_t const total = (size_t)p.P * p.N, step = (size_t)gridDim.x * blockDim.x;
   float const ab2 = 2.f * p.alpha * p.beta;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
@@ -100,6 +102,7 @@ __device__ __forceinline__ Powers powers_of(float L, float beta)
 template <int kD, bool kThreeQuarters>
 __global__ void __launch_bounds__(128) lrn_forward_window_kernel(float* __restrict__ y, float const* __restrict__ x, LrnParams p, int per, int segments)
 {
+  vlb::pdl_wait();
   constexpr int m1 = (kD - 1) / 2, m2 = kD - m1 - 1;
   size_t const i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, total = (size_t)p.P * p.N;
   if (i >= total * segments) return;
@@ -128,6 +131,7 @@ template <int kD, bool kThreeQuarters>
 __global__ void __launch_bounds__(128) lrn_backward_window_kernel(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ dz,
                                                                   LrnParams p, int per, int segments)
 {
+  vlb::pdl_wait();
   constexpr int m1 = (kD - 1) / 2, m2 = kD - m1 - 1;
   size_t const i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, total = (size_t)p.P * p.N;
   if (i >= total * segments) return;
@@ -184,10 +188,10 @@ bool launch_lrn_window(vlb_ctx* ctx, float* out, float const* x, float const* dz
   bool const tq = p.beta == 0.75f;
 #define VLB_LRN(d) \
   case d: \
-    if (kBackward) { if (tq) lrn_backward_window_kernel<d, true><<<(unsigned)blocks, 128, 0, ctx->stream>>>(out, x, dz, p, per, segments); \
-                     else    lrn_backward_window_kernel<d, false><<<(unsigned)blocks, 128, 0, ctx->stream>>>(out, x, dz, p, per, segments); } \
-    else           { if (tq) lrn_forward_window_kernel<d, true><<<(unsigned)blocks, 128, 0, ctx->stream>>>(out, x, p, per, segments); \
-                     else    lrn_forward_window_kernel<d, false><<<(unsigned)blocks, 128, 0, ctx->stream>>>(out, x, p, per, segments); } \
+    if (kBackward) { if (tq) vlb::launch(ctx->stream, lrn_backward_window_kernel<d, true>, (unsigned)blocks, 128, 0, out, x, dz, p, per, segments); \
+                     else    vlb::launch(ctx->stream, lrn_backward_window_kernel<d, false>, (unsigned)blocks, 128, 0, out, x, dz, p, per, segments); } \
+    else           { if (tq) vlb::launch(ctx->stream, lrn_forward_window_kernel<d, true>, (unsigned)blocks, 128, 0, out, x, p, per, segments); \
+                     else    vlb::launch(ctx->stream, lrn_forward_window_kernel<d, false>, (unsigned)blocks, 128, 0, out, x, p, per, segments); } \
     break;
   switch (depth) {
     VLB_LRN(3) VLB_LRN(5) VLB_LRN(7) VLB_LRN(9)
@@ -225,6 +229,7 @@ __device__ float block_reduce(float v, bool isMax, float* red)
 // forward: y = exp(x - max) / sum; backward (dz != nullptr): out = y .* (dz - sum(dz .* y))   (matlab/vl_nnsoftmax.m:24-29)
 __global__ void softmax_kernel(float* __restrict__ out, float const* __restrict__ x, float const* __restrict__ dz, int P, int C)
 {
+  vlb::pdl_wait();
   __shared__ float red[32];
   size_t const off = blockIdx.x + (size_t)P * C * blockIdx.y;
   float const* xp = x + off;
@@ -258,6 +263,7 @@ __device__ __forceinline__ uint32_t mix(uint32_t a, uint32_t b, uint32_t c)
 
 __global__ void dropout_mask_kernel(float* __restrict__ mask, size_t n, float rate, float scale, uint32_t seedLo, uint32_t seedHi)
 {
+  vlb::pdl_wait();
   size_t const step = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
     uint32_t const h = mix((uint32_t)i, (uint32_t)(i >> 32) ^ seedLo, seedHi);
@@ -268,6 +274,7 @@ __global__ void dropout_mask_kernel(float* __restrict__ mask, size_t n, float ra
 
 __global__ void mul_kernel(float* y, float const* a, float const* b, size_t n)
 {
+  vlb::pdl_wait();
   size_t const step = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) y[i] = a[i] * b[i];
 }
@@ -295,7 +302,7 @@ int vlb_lrn_forward(vlb_ctx* ctx, float* Y, float const* X, int H, int W, int C,
   if (rc) return rc;
   VLB_REQUIRE(ctx, Y && X, "lrn_forward: null tensor");
   if (launch_lrn_window<false>(ctx, Y, X, nullptr, p, normDepth)) return vlb::check_launch(ctx, "vlb_lrn_forward");
-  lrn_forward_kernel<<<vlb::grid_for((size_t)p.P * N, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(Y, X, p);
+  vlb::launch(ctx->stream, lrn_forward_kernel, vlb::grid_for((size_t)p.P * N, kThreads, ctx->smCount * 8), kThreads, 0, Y, X, p);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_lrn_forward");
 }
@@ -311,7 +318,7 @@ int vlb_lrn_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, i
   if (launch_lrn_window<true>(ctx, dX, X, dY, p, normDepth)) return vlb::check_launch(ctx, "vlb_lrn_backward");
   float* integral = (float*)vlb::workspace(ctx, sizeof(float) * (size_t)p.P * C * N);
   if (!integral) return vlb::pass_error(ctx, ctx->lastError, "vlb_lrn_backward");
-  lrn_backward_kernel<<<vlb::grid_for((size_t)p.P * N, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(dX, integral, X, dY, p);
+  vlb::launch(ctx->stream, lrn_backward_kernel, vlb::grid_for((size_t)p.P * N, kThreads, ctx->smCount * 8), kThreads, 0, dX, integral, X, dY, p);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_lrn_backward");
 }
@@ -322,7 +329,7 @@ int vlb_softmax_forward(vlb_ctx* ctx, float* Y, float const* X, int H, int W, in
   VLB_REQUIRE(ctx, Y && X, "softmax_forward: null tensor");
   VLB_REQUIRE(ctx, H > 0 && W > 0 && C > 0 && N > 0 && N <= 65535, "softmax_forward: bad shape");
   int const threads = C >= 256 ? 256 : (C >= 64 ? 64 : 32);
-  softmax_kernel<<<dim3(H * W, N), threads, 0, ctx->stream>>>(Y, X, nullptr, H * W, C);
+  vlb::launch(ctx->stream, softmax_kernel, dim3(H * W, N), threads, 0, Y, X, nullptr, H * W, C);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_softmax_forward");
 }
@@ -333,7 +340,7 @@ int vlb_softmax_backward(vlb_ctx* ctx, float* dX, float const* X, float const* d
   VLB_REQUIRE(ctx, dX && X && dY, "softmax_backward: null tensor");
   VLB_REQUIRE(ctx, H > 0 && W > 0 && C > 0 && N > 0 && N <= 65535, "softmax_backward: bad shape");
   int const threads = C >= 256 ? 256 : (C >= 64 ? 64 : 32);
-  softmax_kernel<<<dim3(H * W, N), threads, 0, ctx->stream>>>(dX, X, dY, H * W, C);
+  vlb::launch(ctx->stream, softmax_kernel, dim3(H * W, N), threads, 0, dX, X, dY, H * W, C);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_softmax_backward");
 }
@@ -345,7 +352,7 @@ int vlb_dropout_mask(vlb_ctx* ctx, float* mask, size_t n, double rate, unsigned 
   VLB_REQUIRE(ctx, rate >= 0.0 && rate < 1.0, "dropout_mask: RATE must be in [0, 1)");
   if (n == 0) return VLB_Success;
   float const scale = (float)(1.0 / (1.0 - rate));         // scale = 1 / (1 - rate), converted to single (matlab/vl_nndropout.m:44-56)
-  dropout_mask_kernel<<<vlb::grid_for(n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(
+  vlb::launch(ctx->stream, dropout_mask_kernel, vlb::grid_for(n, kThreads, ctx->smCount * 8), kThreads, 0, 
       mask, n, (float)rate, scale, (uint32_t)seed, (uint32_t)(seed >> 32));
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_dropout_mask");
@@ -356,7 +363,7 @@ int vlb_mul(vlb_ctx* ctx, float* Y, float const* A, float const* B, size_t n)
   if (!ctx) return VLB_IllegalArgument;
   VLB_REQUIRE(ctx, Y && A && B, "mul: null tensor");
   if (n == 0) return VLB_Success;
-  mul_kernel<<<vlb::grid_for(n, kThreads, ctx->smCount * 8), kThreads, 0, ctx->stream>>>(Y, A, B, n);
+  vlb::launch(ctx->stream, mul_kernel, vlb::grid_for(n, kThreads, ctx->smCount * 8), kThreads, 0, Y, A, B, n);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_mul");
 }

@@ -31,6 +31,7 @@ struct PoolParams {
 template <bool kMax>
 __global__ void pool_fwd_generic(float* __restrict__ y, float const* __restrict__ x, PoolParams p)
 {
+  vlb::pdl_wait();
   size_t total = p.planes * (size_t)p.Ho * p.Wo;
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -68,6 +69,7 @@ template <bool kMax>
 __global__ void pool_bwd_generic(float* __restrict__ dx, float const* __restrict__ x,
                                  float const* __restrict__ dy, PoolParams p, bool relu)
 {
+  vlb::pdl_wait();
   size_t total = p.planes * (size_t)p.H * p.W;
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -180,6 +182,7 @@ __device__ __forceinline__ Window window_of(PoolParams const& p, int ho, int wo)
 template <bool kMax>
 __global__ void __launch_bounds__(kThreads) pool_fwd_tiled(float* __restrict__ y, float const* __restrict__ x, const __grid_constant__ TileParams t)
 {
+  vlb::pdl_wait();
   extern __shared__ float xs[];
   PoolParams const& p = t.p;
   Tile const r = tile_of(t, false);
@@ -210,6 +213,7 @@ template <bool kMax>
 __global__ void __launch_bounds__(kThreads) pool_bwd_tiled(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ dy,
                                                            const __grid_constant__ TileParams t, bool relu)
 {
+  vlb::pdl_wait();
   extern __shared__ float smem[];
   PoolParams const& p = t.p;
   Tile const r = tile_of(t, true);
@@ -270,6 +274,7 @@ template <bool kMax>
 __global__ void __launch_bounds__(kThreads) pool33_bwd_tiled(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ dy,
                                                              const __grid_constant__ TileParams t, bool relu)
 {
+  vlb::pdl_wait();
   extern __shared__ float smem[];
   PoolParams const& p = t.p;
   Tile const r = tile_of(t, true);
@@ -423,6 +428,7 @@ __device__ __forceinline__ void pack(float& v, float const* o) { v = o[0]; }
 template <int kV, bool kMax>
 __global__ void pool2x2_fwd(float* __restrict__ y, float const* __restrict__ x, int H, int W, size_t planes)
 {
+  vlb::pdl_wait();
   typedef typename VecT<kV>::in_t in_t;
   typedef typename VecT<kV>::out_t out_t;
   int Ho = H >> 1, Wo = W >> 1, Hv = Ho / kV;
@@ -461,6 +467,7 @@ template <int kV, bool kMax, bool kRelu>
 __global__ void pool2x2_bwd(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ dy,
                             int H, int W, size_t planes)
 {
+  vlb::pdl_wait();
   typedef typename VecT<kV>::in_t in_t;
   typedef typename VecT<kV>::out_t out_t;
   int Ho = H >> 1, Wo = W >> 1, Hv = Ho / kV;
@@ -546,8 +553,8 @@ namespace {
 template <int kV, bool kMax>
 void launch2x2_bwd(vlb_ctx* ctx, unsigned grid, float* dX, float const* X, float const* dY, int H, int W, size_t planes, bool relu)
 {
-  if (relu) pool2x2_bwd<kV, kMax, true><<<grid, kThreads, 0, ctx->stream>>>(dX, X, dY, H, W, planes);
-  else      pool2x2_bwd<kV, kMax, false><<<grid, kThreads, 0, ctx->stream>>>(dX, X, dY, H, W, planes);
+  if (relu) vlb::launch(ctx->stream, pool2x2_bwd<kV, kMax, true>, grid, kThreads, 0, dX, X, dY, H, W, planes);
+  else      vlb::launch(ctx->stream, pool2x2_bwd<kV, kMax, false>, grid, kThreads, 0, dX, X, dY, H, W, planes);
 }
 
 int pool_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, vlb_pool_desc const* d, bool relu, char const* where)
@@ -574,16 +581,16 @@ int pool_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, vlb_
     unsigned grid = 0;
     if (plan_tiles(p, true, isMax || relu, isMax, &t, &smem, &grid)) {
       bool const t33 = is_33s2(p);
-      if (t33 && isMax) pool33_bwd_tiled<true><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
-      else if (t33)     pool33_bwd_tiled<false><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
-      else if (isMax)   pool_bwd_tiled<true><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
-      else              pool_bwd_tiled<false><<<grid, kThreads, smem, ctx->stream>>>(dX, X, dY, t, relu);
+      if (t33 && isMax) vlb::launch(ctx->stream, pool33_bwd_tiled<true>, grid, kThreads, smem, dX, X, dY, t, relu);
+      else if (t33)     vlb::launch(ctx->stream, pool33_bwd_tiled<false>, grid, kThreads, smem, dX, X, dY, t, relu);
+      else if (isMax)   vlb::launch(ctx->stream, pool_bwd_tiled<true>, grid, kThreads, smem, dX, X, dY, t, relu);
+      else              vlb::launch(ctx->stream, pool_bwd_tiled<false>, grid, kThreads, smem, dX, X, dY, t, relu);
       VLB_LAUNCHED(ctx, 1);
       return vlb::check_launch(ctx, where);
     }
     grid = vlb::grid_for(planes * (size_t)d->H * d->W, kThreads, ctx->smCount * 16);
-    if (isMax) pool_bwd_generic<true><<<grid, kThreads, 0, ctx->stream>>>(dX, X, dY, p, relu);
-    else       pool_bwd_generic<false><<<grid, kThreads, 0, ctx->stream>>>(dX, X, dY, p, relu);
+    if (isMax) vlb::launch(ctx->stream, pool_bwd_generic<true>, grid, kThreads, 0, dX, X, dY, p, relu);
+    else       vlb::launch(ctx->stream, pool_bwd_generic<false>, grid, kThreads, 0, dX, X, dY, p, relu);
   }
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, where);
@@ -614,24 +621,24 @@ int vlb_pool_forward(vlb_ctx* ctx, float* Y, float const* X, vlb_pool_desc const
     bool v2 = (d->H % 4 == 0);
     size_t total = planes * (size_t)Wo * (v2 ? Ho / 2 : Ho);
     unsigned grid = vlb::grid_for(total, kThreads, ctx->smCount * 16);
-    if (v2) { if (isMax) pool2x2_fwd<2, true><<<grid, kThreads, 0, ctx->stream>>>(Y, X, d->H, d->W, planes);
-              else       pool2x2_fwd<2, false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, d->H, d->W, planes); }
-    else    { if (isMax) pool2x2_fwd<1, true><<<grid, kThreads, 0, ctx->stream>>>(Y, X, d->H, d->W, planes);
-              else       pool2x2_fwd<1, false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, d->H, d->W, planes); }
+    if (v2) { if (isMax) vlb::launch(ctx->stream, pool2x2_fwd<2, true>, grid, kThreads, 0, Y, X, d->H, d->W, planes);
+              else       vlb::launch(ctx->stream, pool2x2_fwd<2, false>, grid, kThreads, 0, Y, X, d->H, d->W, planes); }
+    else    { if (isMax) vlb::launch(ctx->stream, pool2x2_fwd<1, true>, grid, kThreads, 0, Y, X, d->H, d->W, planes);
+              else       vlb::launch(ctx->stream, pool2x2_fwd<1, false>, grid, kThreads, 0, Y, X, d->H, d->W, planes); }
   } else {
     PoolParams p = {d->H, d->W, Ho, Wo, d->poolH, d->poolW, d->strideY, d->strideX, d->padTop, d->padLeft, planes};
     TileParams t;
     size_t smem = 0;
     unsigned grid = 0;
     if (plan_tiles(p, false, true, isMax, &t, &smem, &grid)) {
-      if (isMax) pool_fwd_tiled<true><<<grid, kThreads, smem, ctx->stream>>>(Y, X, t);
-      else       pool_fwd_tiled<false><<<grid, kThreads, smem, ctx->stream>>>(Y, X, t);
+      if (isMax) vlb::launch(ctx->stream, pool_fwd_tiled<true>, grid, kThreads, smem, Y, X, t);
+      else       vlb::launch(ctx->stream, pool_fwd_tiled<false>, grid, kThreads, smem, Y, X, t);
       VLB_LAUNCHED(ctx, 1);
       return vlb::check_launch(ctx, "vlb_pool_forward");
     }
     grid = vlb::grid_for(planes * (size_t)Ho * Wo, kThreads, ctx->smCount * 16);
-    if (isMax) pool_fwd_generic<true><<<grid, kThreads, 0, ctx->stream>>>(Y, X, p);
-    else       pool_fwd_generic<false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, p);
+    if (isMax) vlb::launch(ctx->stream, pool_fwd_generic<true>, grid, kThreads, 0, Y, X, p);
+    else       vlb::launch(ctx->stream, pool_fwd_generic<false>, grid, kThreads, 0, Y, X, p);
   }
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_pool_forward");

@@ -34,6 +34,7 @@ __device__ __forceinline__ float finish(SumParams const& p, float s, size_t i)
 template <bool kVec, bool kPlain>
 __global__ void __launch_bounds__(kThreads) sum_parts_wide_kernel(SumParams p)
 {
+  vlb::pdl_wait();
   constexpr int V = kVec ? 4 : 1;
   size_t const step = (size_t)gridDim.x * kThreads;
   for (size_t q = (size_t)blockIdx.x * kThreads + threadIdx.x; q * V < p.n; q += step) {
@@ -72,6 +73,7 @@ __global__ void __launch_bounds__(kThreads) sum_parts_wide_kernel(SumParams p)
 
 __global__ void __launch_bounds__(kThreads) sum_parts_narrow_kernel(SumParams p)
 {
+  vlb::pdl_wait();
   __shared__ float red[kThreads / 32][32];
   int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   size_t const i = (size_t)blockIdx.x * 32 + lane;
@@ -108,14 +110,14 @@ int sum_parts(vlb_ctx* ctx, float* out, float const* part, size_t n, size_t stri
   SumParams p = {out, part, n, stride, parts, e};
   bool const plain = !e.bias && e.outMult == 0.f && e.inMult == 1.f && !e.relu && !e.mask;
   if (parts >= 12 && n < (size_t)ctx->smCount * 1024) {
-    sum_parts_narrow_kernel<<<(unsigned)((n + 31) / 32), kThreads, 0, ctx->stream>>>(p);
+    vlb::launch(ctx->stream, sum_parts_narrow_kernel, (unsigned)((n + 31) / 32), kThreads, 0, p);
   } else {
     bool const vec = n % 4 == 0 && stride % 4 == 0 && ((((uintptr_t)out) | ((uintptr_t)part)) & 15) == 0;
     unsigned const grid = grid_for(vec ? n / 4 : n, kThreads, ctx->smCount * 8);
-    if (vec) { if (plain) sum_parts_wide_kernel<true, true><<<grid, kThreads, 0, ctx->stream>>>(p);
-               else       sum_parts_wide_kernel<true, false><<<grid, kThreads, 0, ctx->stream>>>(p); }
-    else     { if (plain) sum_parts_wide_kernel<false, true><<<grid, kThreads, 0, ctx->stream>>>(p);
-               else       sum_parts_wide_kernel<false, false><<<grid, kThreads, 0, ctx->stream>>>(p); }
+    if (vec) { if (plain) vlb::launch(ctx->stream, sum_parts_wide_kernel<true, true>, grid, kThreads, 0, p);
+               else       vlb::launch(ctx->stream, sum_parts_wide_kernel<true, false>, grid, kThreads, 0, p); }
+    else     { if (plain) vlb::launch(ctx->stream, sum_parts_wide_kernel<false, true>, grid, kThreads, 0, p);
+               else       vlb::launch(ctx->stream, sum_parts_wide_kernel<false, false>, grid, kThreads, 0, p); }
   }
   VLB_LAUNCHED(ctx, 1);
   return check_launch(ctx, "sum_parts");

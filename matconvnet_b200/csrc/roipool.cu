@@ -68,6 +68,7 @@ __device__ __forceinline__ void roi_bin(int q, float bin, int start, int extent,
 __global__ void roipool_bounds_kernel(int* __restrict__ bounds, int* __restrict__ images,
                                       float const* __restrict__ rois, RoiParams p)
 {
+  vlb::pdl_wait();
   int total = p.S0 * p.S1 * p.numROIs;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     int ph = i % p.S0, pw = (i / p.S0) % p.S1, r = i / (p.S0 * p.S1);
@@ -86,6 +87,7 @@ template <bool kMax, bool kBackward>
 __global__ void roipool_kernel(float* __restrict__ out, float const* __restrict__ x,
                                float const* __restrict__ rois, float const* __restrict__ dy, RoiParams p)
 {
+  vlb::pdl_wait();
   size_t total = (size_t)p.S0 * p.S1 * p.C * p.numROIs;
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(kGatherThreads, 1)
 roipool_bwd_gather_kernel(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ rois,
                           float const* __restrict__ dy, RoiParams p, int CH, int RB, int chunks)
 {
+  vlb::pdl_wait();
   extern __shared__ __align__(16) uint8_t sm[];
   __shared__ int sCount, sNext;
   int const HW = p.H * p.W, bins = p.S0 * p.S1, words = (RB + 31) / 32;
@@ -337,6 +340,7 @@ __global__ void __launch_bounds__(kOrdThreads)
 roipool_bwd_ordered_kernel(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ rois,
                            float const* __restrict__ dy, RoiParams p, int G, int RB, int groups)
 {
+  vlb::pdl_wait();
   extern __shared__ __align__(16) uint8_t sm[];
   __shared__ int sCount, sNext;
   int const HW = p.H * p.W, bins = p.S0 * p.S1;
@@ -485,7 +489,7 @@ int vlb_roipool_bounds(vlb_ctx* ctx, int* bounds, int* images, float const* rois
   if (rc) return rc;
   VLB_REQUIRE(ctx, bounds && rois, "roipool_bounds: null tensor");
   if (numROIs == 0) return VLB_Success;
-  roipool_bounds_kernel<<<vlb::grid_for((size_t)S0 * S1 * numROIs, kThreads), kThreads, 0, ctx->stream>>>(bounds, images, rois, p);
+  vlb::launch(ctx->stream, roipool_bounds_kernel, vlb::grid_for((size_t)S0 * S1 * numROIs, kThreads), kThreads, 0, bounds, images, rois, p);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_roipool_bounds");
 }
@@ -501,8 +505,8 @@ int vlb_roipool_forward(vlb_ctx* ctx, float* Y, float const* X, float const* roi
   if (numROIs == 0) return VLB_Success;
   size_t total = (size_t)S0 * S1 * C * numROIs;
   unsigned grid = vlb::grid_for(total, kThreads, ctx->smCount * 16);
-  if (method == VLB_POOL_MAX) roipool_kernel<true, false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, rois, nullptr, p);
-  else                        roipool_kernel<false, false><<<grid, kThreads, 0, ctx->stream>>>(Y, X, rois, nullptr, p);
+  if (method == VLB_POOL_MAX) vlb::launch(ctx->stream, roipool_kernel<true, false>, grid, kThreads, 0, Y, X, rois, nullptr, p);
+  else                        vlb::launch(ctx->stream, roipool_kernel<false, false>, grid, kThreads, 0, Y, X, rois, nullptr, p);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_roipool_forward");
 }
@@ -542,7 +546,7 @@ int vlb_roipool_backward(vlb_ctx* ctx, float* dX, float const* X, float const* r
           if (ea != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(ea)); }
           if (ctx->device < 64) attrDone[ctx->device] = true;
         }
-        roipool_bwd_ordered_kernel<<<(unsigned)(N * groups), kOrdThreads, smem, ctx->stream>>>(dX, X, rois, dY, p, G, (int)RB, groups);
+        vlb::launch(ctx->stream, roipool_bwd_ordered_kernel, (unsigned)(N * groups), kOrdThreads, smem, dX, X, rois, dY, p, G, (int)RB, groups);
         VLB_LAUNCHED(ctx, 1);
         return vlb::check_launch(ctx, "vlb_roipool_backward");
       }
@@ -567,8 +571,8 @@ int vlb_roipool_backward(vlb_ctx* ctx, float* dX, float const* X, float const* r
             if (ctx->device < 64) attrDone[isMax][ctx->device] = true;
           }
           unsigned const grid = (unsigned)(N * chunks);
-          if (isMax) roipool_bwd_gather_kernel<true><<<grid, kGatherThreads, smem, ctx->stream>>>(dX, X, rois, dY, p, CH, (int)RB, chunks);
-          else       roipool_bwd_gather_kernel<false><<<grid, kGatherThreads, smem, ctx->stream>>>(dX, X, rois, dY, p, CH, (int)RB, chunks);
+          if (isMax) vlb::launch(ctx->stream, roipool_bwd_gather_kernel<true>, grid, kGatherThreads, smem, dX, X, rois, dY, p, CH, (int)RB, chunks);
+          else       vlb::launch(ctx->stream, roipool_bwd_gather_kernel<false>, grid, kGatherThreads, smem, dX, X, rois, dY, p, CH, (int)RB, chunks);
           VLB_LAUNCHED(ctx, 1);
           return vlb::check_launch(ctx, "vlb_roipool_backward");
         }
@@ -581,8 +585,8 @@ int vlb_roipool_backward(vlb_ctx* ctx, float* dX, float const* X, float const* r
   if (numROIs == 0) return VLB_Success;
   size_t total = (size_t)S0 * S1 * C * numROIs;
   unsigned grid = vlb::grid_for(total, kThreads, ctx->smCount * 16);
-  if (method == VLB_POOL_MAX) roipool_kernel<true, true><<<grid, kThreads, 0, ctx->stream>>>(dX, X, rois, dY, p);
-  else                        roipool_kernel<false, true><<<grid, kThreads, 0, ctx->stream>>>(dX, X, rois, dY, p);
+  if (method == VLB_POOL_MAX) vlb::launch(ctx->stream, roipool_kernel<true, true>, grid, kThreads, 0, dX, X, rois, dY, p);
+  else                        vlb::launch(ctx->stream, roipool_kernel<false, true>, grid, kThreads, 0, dX, X, rois, dY, p);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_roipool_backward");
 }

@@ -62,6 +62,7 @@ __global__ void sampler_kernel(float* __restrict__ y, float* __restrict__ dx, fl
                                float const* __restrict__ x, float const* __restrict__ grid,
                                float const* __restrict__ dy, int H, int W, int C, int N, int Q, int Ng)
 {
+  vlb::pdl_wait();
   int group = Ng / N;
   size_t total = (size_t)Q * Ng;
   size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -172,6 +173,7 @@ sampler_bwd_gather_kernel(float* __restrict__ dx, float* __restrict__ dgrid, flo
                           float const* __restrict__ grid, float const* __restrict__ dy, int H, int W, int C, int N, int Q, int Ng,
                           int chunks, int CH)
 {
+  vlb::pdl_wait();
   extern __shared__ __align__(16) uint8_t sm[];
   __shared__ int warpSums[32];
   int const HW = H * W, tid = threadIdx.x;
@@ -438,7 +440,7 @@ int vlb_sampler_forward(vlb_ctx* ctx, float* Y, float const* X, float const* gri
   VLB_REQUIRE(ctx, Y && X && grid, "sampler_forward: null tensor");
   VLB_REQUIRE(ctx, (((uintptr_t)grid) & 7) == 0, "sampler_forward: grid must be 8-byte aligned");
   size_t total = (size_t)Ho * Wo * Ng;
-  sampler_kernel<0><<<vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, ctx->stream>>>(
+  vlb::launch(ctx->stream, sampler_kernel<0>, vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, 
       Y, nullptr, nullptr, X, grid, nullptr, H, W, C, N, Ho * Wo, Ng);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_sampler_forward");
@@ -472,12 +474,12 @@ int vlb_sampler_backward(vlb_ctx* ctx, float* dX, float* dGrid, float const* X, 
     }
     size_t const smem = gather_smem(HWi, Qo);
     unsigned const blocks = (unsigned)(N * chunks);
-    if (fusedGrid) sampler_bwd_gather_kernel<true><<<blocks, kGatherThreads, smem, ctx->stream>>>(dX, dGrid, X, grid, dY, H, W, C, N, Qo, Ng, chunks, CH);
-    else           sampler_bwd_gather_kernel<false><<<blocks, kGatherThreads, smem, ctx->stream>>>(dX, nullptr, X, grid, dY, H, W, C, N, Qo, Ng, chunks, CH);
+    if (fusedGrid) vlb::launch(ctx->stream, sampler_bwd_gather_kernel<true>, blocks, kGatherThreads, smem, dX, dGrid, X, grid, dY, H, W, C, N, Qo, Ng, chunks, CH);
+    else           vlb::launch(ctx->stream, sampler_bwd_gather_kernel<false>, blocks, kGatherThreads, smem, dX, nullptr, X, grid, dY, H, W, C, N, Qo, Ng, chunks, CH);
     VLB_LAUNCHED(ctx, 1);
     if (dGrid && !fusedGrid) {
       size_t total = (size_t)Qo * Ng;
-      sampler_kernel<1><<<vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, ctx->stream>>>(
+      vlb::launch(ctx->stream, sampler_kernel<1>, vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, 
           nullptr, nullptr, dGrid, X, grid, dY, H, W, C, N, Qo, Ng);
       VLB_LAUNCHED(ctx, 1);
     }
@@ -488,7 +490,7 @@ int vlb_sampler_backward(vlb_ctx* ctx, float* dX, float* dGrid, float const* X, 
     if (e != cudaSuccess) return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e));
   }
   size_t total = (size_t)Ho * Wo * Ng;
-  sampler_kernel<1><<<vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, ctx->stream>>>(
+  vlb::launch(ctx->stream, sampler_kernel<1>, vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, 
       nullptr, dX, dGrid, X, grid, dY, H, W, C, N, Ho * Wo, Ng);
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, "vlb_sampler_backward");
