@@ -117,6 +117,20 @@ namespace vlb {
 // and see no difference.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Quotient of any 31-bit number by a fixed one with a multiply and a shift (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", PLDI 1994: with 2^s >= d and m = ceil(2^(31+s) / d), floor(n / d) = n*m >> (31+s) for n < 2^31).
+struct FastDiv31 {
+  unsigned m, s;
+  __host__ __device__ FastDiv31() : m(0), s(0) {}
+  __host__ explicit FastDiv31(int d)
+  {
+    s = 0;
+    while ((1ull << s) < (unsigned)d) ++s;
+    m = (unsigned)(((1ull << (31 + s)) + (unsigned)d - 1) / (unsigned)d);
+  }
+  __device__ __forceinline__ int operator()(int n) const { return (int)(((unsigned long long)(unsigned)n * m) >> (31 + s)); }
+};
+
 // Launch errors are sticky until read: the callers' check_launch reports them.
 template <class... E, class... A>
 inline void launch(cudaStream_t stream, void (*kernel)(E...), dim3 grid, dim3 block, size_t smem, A&&... args)

@@ -121,6 +121,7 @@ struct Params {
   int vecStore;           // conv_ts_kernel: four consecutive rows of a tile are four consecutive pixels on a 16-byte boundary of the output (and of the mask)
   int smemSum;            // conv_ts_kernel, kMode 0 / 1: keep the running sum of a tile in shared memory even for the tile widths that fit the
                           // drain warps' registers (one short tile per CTA, whose stores all warps share; test switch bit 3)
+  vlb::FastDiv31 dHo, dWo, dTilesN, dTilesM;      // conv_ts_kernel: by a.Ho, a.Wo, tilesN, tilesM (set by ts_divisors)
   int plane;              // row mode: reduction indices per image in the tile images -- the plane's pixels rounded up to whole k-blocks
   // conv_ts_gen_kernel (general gather).  The reduction runs over units of `unit` channels of one filter tap, upk = 32 / unit of
   // them per k-block: unit number = tap + taps * (channel / unit).  Column tile nt belongs to filter group nt / tilesPerGroup;
@@ -1077,6 +1078,18 @@ __device__ __forceinline__ float lds32(uint32_t addr)
   return v;
 }
 
+// Bit f is set when position at + f * dilate lies inside [0, extent), f < taps (at most 32).
+__device__ __forceinline__ uint32_t taps_inside(int at, int taps, int dilate, int extent)
+{
+  if (dilate == 1) {
+    int const lo = max(-at, 0), hi = min(extent - at, taps);          // f in [lo, hi)
+    return hi <= lo ? 0u : (0xffffffffu >> (32 - hi)) & (0xffffffffu << lo);
+  }
+  uint32_t m = 0;
+  for (int f = 0; f < taps; ++f) if ((unsigned)(at + f * dilate) < (unsigned)extent) m |= 1u << f;
+  return m;
+}
+
 // Where row `row` (0..127, = TMEM lane) of row tile `tm` lies in the output: image, pixel ho + Ho*wo, and whether it exists.
 // Linear mode: the tile is 128 consecutive output pixels (ho fastest, images following one another).  Box mode (p.tma):
 // the tile is a box of bh x bw pixels of one image, row = dh + bh*dw.
@@ -1088,11 +1101,11 @@ __device__ __forceinline__ RowPos row_pos(Params const& p, int tm, int row)
   RowPos r;
   r.h = r.w = 0;
   if (kGen) {
-    r.split = tm / p.tilesM; tm -= r.split * p.tilesM;
+    r.split = p.dTilesM(tm); tm -= r.split * p.tilesM;
     int const m = tm * BM + row;
     r.valid = m < p.M;
-    int const mm = min(m, p.M - 1), t = mm / p.a.Ho;
-    r.img = t / p.a.Wo;
+    int const mm = min(m, p.M - 1), t = p.dHo(mm);
+    r.img = p.dWo(t);
     r.h = p.oy + p.oys * (mm - t * p.a.Ho); r.w = p.ox + p.oxs * (t - r.img * p.a.Wo);
     r.pix = r.h + p.outH * r.w;
     return r;
@@ -1107,12 +1120,12 @@ __device__ __forceinline__ RowPos row_pos(Params const& p, int tm, int row)
     return r;
   }
   // tm = row tile + tilesM * reduction range (one range unless the caller cut the reduction)
-  r.split = tm / p.tilesM; tm -= r.split * p.tilesM;
+  r.split = p.dTilesM(tm); tm -= r.split * p.tilesM;
   if (!p.tma) {
     int const m = tm * BM + row;
     r.valid = m < p.M;
     int const mm = min(m, p.M - 1);
-    r.img = mm / p.e.P; r.pix = mm - r.img * p.e.P;
+    r.img = p.dWo(p.dHo(mm)); r.pix = mm - r.img * p.e.P;          // (a plane is a.Ho x a.Wo pixels)
   } else {
     int const per = p.tilesH * p.tilesW;
     int const n = tm / per, t = tm - n * per, wb = t / p.tilesH, hb = t - wb * p.tilesH;
@@ -1387,7 +1400,7 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
       bool ok = true;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
         int const tile = cta + ts * ctas;
-        int const tm = tile / p.tilesN;
+        int const tm = p.dTilesN(tile);
         TileCols const tc = tile_cols<kGen>(p, tile - tm * p.tilesN);
         int const n0 = tc.n0;
         int const chainsF = ts_chains<kSplit>(numIter, 0), chainsS = ts_chains<kSplit>(numIter, 1);   // of the issuer that owns the tile's first k-block, of the other
@@ -1843,15 +1856,14 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
     } else {
       for (int ts = 0; ts < myTiles && ok; ++ts) {
         int const tile = cta + ts * ctas;
-        int const tmf = tile / p.tilesN, split = tmf / p.tilesM, kb0 = split * numIter;     // this item's range starts at k-block kb0
+        int const tmf = p.dTilesN(tile), split = p.dTilesM(tmf), kb0 = split * numIter;     // this item's range starts at k-block kb0
         int const m = (tmf - split * p.tilesM) * BM + quarter * 32 + lane;
         uint32_t hm = 0, wm = 0;                          // tap rows / columns inside the image for this pixel
         float const* xq = p.a.ptr;
         if (m < p.M) {
-          int const ho = m % p.a.Ho, q = m / p.a.Ho, wo = q % p.a.Wo, n = q / p.a.Wo;
+          int const q = p.dHo(m), n = p.dWo(q), ho = m - q * p.a.Ho, wo = q - n * p.a.Wo;
           xq += (long long)n * p.a.imgStride + (long long)wo * p.a.sx * p.a.H + ho * p.a.sy;
-          for (int fh = 0; fh < p.a.FH; ++fh) { int h = ho * p.a.sy + fh * p.a.dy - p.a.pt; if (h >= 0 && h < p.a.H) hm |= 1u << fh; }
-          for (int fw = 0; fw < p.a.FW; ++fw) { int w = wo * p.a.sx + fw * p.a.dx - p.a.pl; if (w >= 0 && w < p.a.W) wm |= 1u << fw; }
+          hm = taps_inside(ho * p.a.sy - p.a.pt, p.a.FH, p.a.dy, p.a.H); wm = taps_inside(wo * p.a.sx - p.a.pl, p.a.FW, p.a.dx, p.a.W);
         }
         if constexpr (kGen) {
           int const grpC = (tile - tmf * p.tilesN) / p.tilesPerGroup;
@@ -1864,26 +1876,62 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
               float v[32];
               int const u0 = (kb0 + it) * kPer;
               int cb = u0 / taps, tap = u0 - cb * taps;
+              if constexpr (kU <= 3) {
+                // First every load of the k-block, then the zeros: a value tested as soon as it is asked for would make the thread wait for
+                // memory once per unit.
+                uint32_t off = 0;                                  // units that are padding for this pixel
+                int const cb0 = cb, tap0 = tap;
 #pragma unroll
-              for (int u = 0; u < kPer; ++u) {
-                int2 const te = tapLut[tap];
-                uint32_t const e = (uint32_t)te.y;
-                int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
-                bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
-                float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;
-                if (left >= kU) {
+                for (int u = 0; u < kPer; ++u) {
+                  int2 const te = tapLut[tap];
+                  uint32_t const e = (uint32_t)te.y;
+                  int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
+                  bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
+                  off |= on ? 0u : 1u << u;
+                  // (unconditional loads: what is padding reads the start of the tensor, channels that do not exist the first of the unit)
+                  float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;
                   long long const step = on ? (long long)HW : 0;
+                  if (kU == 1 || left >= kU) {
 #pragma unroll
-                  for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + k * step);
-                  if (!on) {
+                    for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + k * step);
+                  } else {
 #pragma unroll
-                    for (int k = 0; k < kU; ++k) v[u * kU + k] = 0.f;
+                    for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + (k < left ? k : 0) * step);
                   }
-                } else {
-#pragma unroll
-                  for (int k = 0; k < kU; ++k) { v[u * kU + k] = 0.f; ldg32_if(v[u * kU + k], q + (long long)k * HW, on && k < left); }
+                  if (++tap == taps) { tap = 0; ++cb; }
                 }
-                if (++tap == taps) { tap = 0; ++cb; }
+                cb = cb0; tap = tap0;
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                  int const left = ((off >> u) & 1u) ? 0 : p.a.C - cb * kU;
+                  if (left < kU) {
+#pragma unroll
+                    for (int k = 0; k < kU; ++k) v[u * kU + k] = k < left ? v[u * kU + k] : 0.f;
+                  }
+                  if (kU > 1 && ++tap == taps) { tap = 0; ++cb; }
+                }
+              } else {
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                  int2 const te = tapLut[tap];
+                  uint32_t const e = (uint32_t)te.y;
+                  int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
+                  bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
+                  float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;
+                  if (left >= kU) {
+                    long long const step = on ? (long long)HW : 0;
+#pragma unroll
+                    for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + k * step);
+                    if (!on) {
+#pragma unroll
+                      for (int k = 0; k < kU; ++k) v[u * kU + k] = 0.f;
+                    }
+                  } else {
+#pragma unroll
+                    for (int k = 0; k < kU; ++k) { v[u * kU + k] = 0.f; ldg32_if(v[u * kU + k], q + (long long)k * HW, on && k < left); }
+                  }
+                  if (++tap == taps) { tap = 0; ++cb; }
+                }
               }
 #pragma unroll
               for (int k = kPer * kU; k < 32; ++k) v[k] = 0.f;
@@ -2480,6 +2528,14 @@ bool plan_windows(vlb_ctx* ctx, Params& p, CUtensorMap* map, size_t* smemBytes, 
   return true;
 }
 
+// The multiply-for-division constants of a launch, once its tiling is known: a thread's tile set-up (four divisions, a test per filter row and
+// column) otherwise took the producers 2800 cycles per tile, in which the tensor core runs dry.
+void ts_divisors(Params& p)
+{
+  p.dHo = vlb::FastDiv31(std::max(p.a.Ho, 1)); p.dWo = vlb::FastDiv31(std::max(p.a.Wo, 1));
+  p.dTilesN = vlb::FastDiv31(p.tilesN); p.dTilesM = vlb::FastDiv31(p.tilesM);
+}
+
 // Whether four rows of a tile, the first a multiple of four, lie next to each other in the output: planes of a multiple of four pixels
 // (linear tiles), columns of one (boxes), pixels one apart, everything on 16-byte boundaries.
 bool rows_contiguous(Params const& p)
@@ -2506,6 +2562,7 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
   memset(&map, 0, sizeof(map));
   bool const windows = plan_windows(ctx, p, &map, &smemBytes, split3);
   p.vecStore = rows_contiguous(p) && (!windows || p.a.Ho % 4 == 0);
+  ts_divisors(p);
   if (smemBytes < 120u * 1024u) smemBytes = 120u * 1024u;
   long long const numTiles = (long long)p.tilesM * p.tilesN * p.splits;
   if (numTiles >= (1LL << 31)) return VLB_Unsupported;
@@ -2620,6 +2677,7 @@ int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* whe
   if (smemBytes < 120u * 1024u) smemBytes = 120u * 1024u;      // two CTAs (each allocating all 512 TMEM columns) never share an SM
   p.wg = 1;
   p.vecStore = rows_contiguous(p) && p.a.FH * p.a.FW == 1;
+  ts_divisors(p);
   p.status = ctx->deviceStatus;
   p.testSwitch = ctx->testSwitch;
   p.chanFast = 1;
@@ -2922,6 +2980,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     p.bTiles = prep.p[i].out;
     if (splits > 1) p.e.out = part;
     p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;
+    ts_divisors(p);
     p.vecStore = rows_contiguous(p) && p.shufY == 0 && p.oys == 1 && p.oxs == 1 && p.outH == p.a.Ho && p.outW == p.a.Wo;
   }
   launch_prep(ctx, prep, b.n);
