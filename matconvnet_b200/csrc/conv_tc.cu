@@ -118,7 +118,7 @@ struct Params {
   // reduction (output pixels of the whole batch, kbTot k-blocks in the dY tile images) is cut into `splits` ranges of kbPerSplit
   // k-blocks, one work item per (range, row tile, column tile); the x runs arrive by tensor-map copies, xStages buffers.
   int wg, cPer, tapsPerTile, tapGroups, kbTot, splits, xStages;
-  int vecStore;           // conv_ts_kernel: four consecutive rows of a tile are four consecutive pixels on a 16-byte boundary of the output (and of the mask)
+  int biasFirst;          // conv_ts_kernel: a tile's running sum starts at the bias (16-byte loads of it legal, no multiplier, columns in order)
   int smemSum;            // conv_ts_kernel, kMode 0 / 1: keep the running sum of a tile in shared memory even for the tile widths that fit the
                           // drain warps' registers (one short tile per CTA, whose stores all warps share; test switch bit 3)
   vlb::FastDiv31 dHo, dWo, dTilesN, dTilesM;      // conv_ts_kernel: by a.Ho, a.Wo, tilesN, tilesM (set by ts_divisors)
@@ -1154,31 +1154,25 @@ __device__ __forceinline__ TileCols tile_cols(Params const& p, int nt)
   return c;
 }
 
-// Epilogue of conv_ts_kernel: a finished tile, or 32 columns of it, sits in shared memory, P[column][row]; a warp stores the rows of its
-// TMEM lane quarter: out[(image*Ktot + n)*P + pixel] = inMult*acc + bias[n] + outMult*old, then ReLU / mask.
-//
-// This is the serial part of a tile: while the drain warps store, the tensor core gets at most two chains ahead and then waits, and the
-// drain warps share their schedulers with the producers.  So it is counted in instructions: where rows are consecutive pixels and
-// 16-byte stores are legal (p.vecStore), a lane takes four rows of every fourth column -- 8 loads and 8 stores of 16 bytes per 32 columns,
-// no test of an option inside the loop; elsewhere a lane keeps its own row, eight columns in flight.  Against one 4-byte load, the option
-// tests and one 4-byte store per column (about 130 cycles, 9 us per 128-column tile): 1x1 layer 512 -> 128 on 28 x 28 x 64 83 -> 61 us, its data
-// gradient 107 -> 86 us, VGG-16 step batch 64 36.2 -> 34.7 ms.
+// Where the row of a tile that a thread stores goes.
 struct TsDst { long long at; int row; bool valid; int h, w, img, split; };
 
 template <bool kGen>
-__device__ __forceinline__ TsDst ts_dst(Params const& p, int tm, int quarter, int lane)
+__device__ __forceinline__ TsDst ts_dst(Params const& p, int tm, int row)
 {
   TsDst d;
-  d.row = quarter * 32 + (p.vecStore ? 4 * (lane & 7) : lane);
-  RowPos const rp = row_pos<kGen>(p, tm, d.row);
+  d.row = row;
+  RowPos const rp = row_pos<kGen>(p, tm, row);
   d.valid = rp.valid; d.h = rp.h; d.w = rp.w; d.img = rp.img; d.split = rp.split;
   d.at = (long long)rp.split * p.e.splitStride + (long long)rp.img * p.e.Ktot * p.e.P + rp.pix;
   return d;
 }
 
-// P holds the columns cBeg .. cBeg + cCnt - 1 of the tile.  masked: the mask has been applied to P already.
+// Epilogue of conv_ts_kernel for what the direct store of the registers does not cover: the columns cBeg .. cBeg + cCnt - 1 of a tile from
+// shared memory, P[column][row]: out[(image*Ktot + n)*P + pixel] = inMult*acc + bias[n] + outMult*old, then ReLU / mask.  Eight columns in flight.
+// masked: the mask has been applied to P already.
 template <bool kGen>
-__device__ __forceinline__ void ts_store_cols(Params const& p, float const* P, int lane, TsDst const& d, TileCols const& tc, int cBeg, int cCnt, bool masked)
+__device__ __forceinline__ void ts_store_cols(Params const& p, float const* P, TsDst const& d, TileCols const& tc, int cBeg, int cCnt, bool masked)
 {
   int const nEnd = min(cCnt, tc.cnt - cBeg), n0 = tc.n0 + cBeg;
   if (!d.valid) return;
@@ -1204,73 +1198,31 @@ __device__ __forceinline__ void ts_store_cols(Params const& p, float const* P, i
     }
     return;
   }
-  float const inMult = p.e.inMult;
-  bool const relu = p.e.relu != 0, hasBias = p.e.bias != nullptr;
-  if (p.e.outMult == 0.f && mask == nullptr) {
-    // the usual case, as few instructions as it takes: the drain warps share their schedulers with the producers
-    if (p.vecStore) {
-      float* o0 = out + (long long)(n0 + (lane >> 3)) * p.e.P;
-      long long const step = 4LL * p.e.P;
-      float const* b0 = p.e.bias + n0;
-      for (int c0 = lane >> 3; c0 < nEnd; c0 += 16, o0 += 4 * step) {
-        float4 v[4];
-        float b[4] = {0.f, 0.f, 0.f, 0.f};
+  bool const hasBias = p.e.bias != nullptr && !p.biasFirst, hasOld = p.e.outMult != 0.f;
+  float* o0 = out + (long long)n0 * p.e.P;
+  for (int c0 = 0; c0 < nEnd; c0 += 8, o0 += 8LL * p.e.P) {
+    float v[8], b[8], old[8], mk[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<float4 const*>(P + min(c0 + 4 * i, nEnd - 1) * BM);
-        if (hasBias) {
+    for (int i = 0; i < 8; ++i) { v[i] = P[min(c0 + i, nEnd - 1) * BM] * p.e.inMult; b[i] = 0.f; old[i] = 0.f; mk[i] = 1.f; }
+    if (hasBias) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) b[i] = __ldg(b0 + min(c0 + 4 * i, nEnd - 1));
-        }
-        if (inMult != 1.f) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) { v[i].x *= inMult; v[i].y *= inMult; v[i].z *= inMult; v[i].w *= inMult; }
-        }
-        if (hasBias) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) { v[i].x += b[i]; v[i].y += b[i]; v[i].z += b[i]; v[i].w += b[i]; }
-        }
-        if (relu) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) { v[i].x = v[i].x > 0.f ? v[i].x : 0.f; v[i].y = v[i].y > 0.f ? v[i].y : 0.f; v[i].z = v[i].z > 0.f ? v[i].z : 0.f; v[i].w = v[i].w > 0.f ? v[i].w : 0.f; }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) if (c0 + 4 * i < nEnd) *reinterpret_cast<float4*>(o0 + i * step) = v[i];
-      }
-    } else {
-      float* o0 = out + (long long)n0 * p.e.P;
-      for (int c0 = 0; c0 < nEnd; c0 += 8, o0 += 8LL * p.e.P) {
-        float v[8], b[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { v[i] = P[min(c0 + i, nEnd - 1) * BM] * inMult; b[i] = 0.f; }
-        if (hasBias) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) b[i] = __ldg(p.e.bias + n0 + min(c0 + i, nEnd - 1));
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] += b[i];
-        }
-        if (relu) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = v[i] > 0.f ? v[i] : 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) if (c0 + i < nEnd) o0[(long long)i * p.e.P] = v[i];
-      }
+      for (int i = 0; i < 8; ++i) b[i] = __ldg(p.e.bias + n0 + min(c0 + i, nEnd - 1));
     }
-    return;
-  }
-  for (int c0 = p.vecStore ? lane >> 3 : 0; c0 < nEnd; c0 += p.vecStore ? 4 : 1) {
-    // accumulation onto the old output, or a mask that could not be fetched ahead
-    long long const off = (long long)(n0 + c0) * p.e.P;
-    float const b = hasBias ? __ldg(p.e.bias + n0 + c0) : 0.f;
+    if (hasOld) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (e > 0 && !p.vecStore) break;
-      float o = inMult * P[c0 * BM + e];
-      if (hasBias) o += b;
-      if (p.e.outMult != 0.f) o += p.e.outMult * out[off + e];
-      if (relu) o = o > 0.f ? o : 0.f;
-      if (mask && !(__ldg(mask + d.at + off + e) > 0.f)) o = 0.f;
-      out[off + e] = o;
+      for (int i = 0; i < 8; ++i) if (c0 + i < nEnd) old[i] = o0[(long long)i * p.e.P];
+    }
+    if (mask) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) if (c0 + i < nEnd) mk[i] = __ldg(mask + d.at + (long long)(n0 + c0 + i) * p.e.P);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float o = v[i];
+      if (hasBias) o += b[i];
+      if (hasOld) o += p.e.outMult * old[i];
+      if (p.e.relu) o = o > 0.f ? o : 0.f;
+      if (c0 + i < nEnd) o0[(long long)i * p.e.P] = mk[i] > 0.f ? o : 0.f;
     }
   }
 }
@@ -1344,8 +1296,8 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
   float* const Psm = reinterpret_cast<float*>(smem + (size_t)nB * bBytes);      // [BN][BM]
   // input windows (kTma): two buffers of boxH*boxW*32 floats behind P
   uint32_t const xPlane = (uint32_t)(p.boxH * p.boxW), xTileBytes = kWg ? (uint32_t)kWgStageBytes : xPlane * 32u * 4u;
-  bool const regsP = (kWg ? (BN == 128 || BN == 64) : (kNarrow ? BN == 64 : BN == 128)) && !p.smemSum;      // the running sum of a tile lives in the drain warps' registers
-  uint32_t const xTile0 = smem_u32(Psm) + (regsP ? 32u : (uint32_t)BN) * BM * 4u;      // (registers: a patch of 32 columns for the stores)
+  bool const regsP = (kWg ? (BN == 128 || BN == 64) : (kNarrow || BN == 128)) && !p.smemSum;      // the running sum of a tile lives in the drain warps' registers
+  uint32_t const xTile0 = smem_u32(Psm) + (regsP && BN > 32 ? 32u : (uint32_t)BN) * BM * 4u;      // (registers: a patch of 32 columns for the stores)
 
   int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int const numIter = p.kbPerSplit;                      // k-blocks per tile (work item: one range of the reduction of one output tile)
@@ -1407,7 +1359,11 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
         bool fresh = true;                              // P holds nothing of this tile yet
         if (kRegs > 0) {
 #pragma unroll
-          for (int j = 0; j < kRegs; ++j) Pr[j] = 0.f;
+          for (int j = 0; j < kRegs; j += 4) {
+            // (the bias is there long before the first chain is)
+            float4 const b = p.biasFirst && j < tc.cnt ? __ldg(reinterpret_cast<float4 const*>(p.e.bias + n0 + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            Pr[j] = b.x; Pr[j + 1] = b.y; Pr[j + 2] = b.z; Pr[j + 3] = b.w;
+          }
         }
         // ReLU mask of this thread's output row (persistent mode): sixteen columns are fetched before each of the tile's
         // first chain waits, so that their latency passes while the chain is being computed, and kept as one bit each
@@ -1438,12 +1394,16 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
               // P += T in fp32, in registers
 #pragma unroll
               for (int c0 = 0; c0 < kRegs; c0 += 32) {
+                constexpr bool two = kRegs > 16;
                 uint32_t t0[16], t1[16];
                 tmem_ld16_issue(lanes + (uint32_t)(t * kRegs + c0), t0);
-                tmem_ld16_issue(lanes + (uint32_t)(t * kRegs + c0 + 16), t1);
+                if (two) tmem_ld16_issue(lanes + (uint32_t)(t * kRegs + c0 + 16), t1);
                 tmem_ld_wait();
 #pragma unroll
-                for (int j = 0; j < 16; ++j) { Pr[c0 + j] += __uint_as_float(t0[j]); Pr[c0 + 16 + j] += __uint_as_float(t1[j]); }
+                for (int j = 0; j < 16; ++j) {
+                  Pr[c0 + j] += __uint_as_float(t0[j]);
+                  if (two) Pr[(c0 + 16 + j) % (kRegs > 0 ? kRegs : 1)] += __uint_as_float(t1[j]);
+                }
               }
             } else {
               // P = T (first chain of the tile) or P += T in fp32, in shared memory
@@ -1457,6 +1417,7 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                   float v0 = __uint_as_float(t0[j]), v1 = __uint_as_float(t1[j]);
+                  if (fresh && p.biasFirst) { v0 += __ldg(p.e.bias + n0 + min(c0 + j, nEndT - 1)); v1 += __ldg(p.e.bias + n0 + min(c0 + 16 + j, nEndT - 1)); }
                   if (!fresh) { v0 += pc[j * BM]; if (two) v1 += pc[(16 + j) * BM]; }
                   pc[j * BM] = v0;
                   if (two) pc[(16 + j) * BM] = v1;
@@ -1485,37 +1446,46 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
           b <<= 16 * (lc & 1);
           if (lc < 2) mbits[0] |= b; else if (lc < 4) mbits[1] |= b; else if (lc < 6) mbits[2] |= b; else mbits[3] |= b;
         }
-        TsDst const dst = ts_dst<kGen>(p, tm, warp, lane);
+        TsDst const dst = ts_dst<kGen>(p, tm, warp * 32 + lane);
         if (kRegs > 0) {
-          // The finished tile, 32 columns at a time: registers -> P[column][row] (a 16 KB patch of shared memory, this warp's 32 rows of it
-          // its own) -> global memory, while the tensor core works on the next tile.  (The loop over the columns has to run over shared
-          // memory: registers cannot be indexed.)
+          // The finished tile while the tensor core works on the next one.  Straight from the registers, a 4-byte store per column and
+          // thread, coalesced along the rows: nothing here waits for anything.  (Every load of this phase -- a patch of shared memory, a
+          // bias -- cost the drain warps its full latency plus a queue behind the producers' gathers: 4.4k cycles per 128-column tile through
+          // 16-byte stores from a patch, 13k to 20k where planes of 13 x 13 or 27 x 27 pixels rule those out.)
+          bool const direct = p.e.inMult == 1.f && p.e.outMult == 0.f && (p.e.bias == nullptr || p.biasFirst) && (p.e.mask == nullptr || preMask) && !(kGen && p.shufY > 0);
+          if (preMask) {
 #pragma unroll
-          for (int c0 = 0; c0 < kRegs; c0 += 32) {
-            if (c0 < nEndT) {
-              if (preMask) {
+            for (int j = 0; j < kRegs; ++j) Pr[j] = ((mbits[j / 32] >> (j & 31)) & 1u) ? Pr[j] : 0.f;
+          }
+          if (direct) {
+            if (p.e.relu) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) Prow[j * BM] = ((mbits[c0 / 32] >> j) & 1u) ? Pr[c0 + j] : 0.f;
-              } else {
+              for (int j = 0; j < kRegs; ++j) Pr[j] = Pr[j] > 0.f ? Pr[j] : 0.f;
+            }
+            float* o = p.e.out + dst.at + (long long)n0 * p.e.P;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) Prow[j * BM] = Pr[c0 + j];
+            for (int j = 0; j < kRegs; ++j, o += p.e.P) if (dst.valid && j < nEndT) *o = Pr[j];
+          } else {
+            // 32 columns at a time: registers -> P[column][row] (a patch of shared memory, every thread its own row) -> global memory
+            // (the loop over the columns has to run over shared memory: registers cannot be indexed)
+#pragma unroll
+            for (int c0 = 0; c0 < kRegs; c0 += 32) {
+              if (c0 < nEndT) {
+#pragma unroll
+                for (int j = 0; j < (kRegs < 32 ? kRegs : 32); ++j) Prow[j * BM] = Pr[c0 + j];
+                ts_store_cols<kGen>(p, Psm, dst, tc, c0, 32, preMask);
               }
-              __syncwarp();
-              ts_store_cols<kGen>(p, Psm, lane, dst, tc, c0, 32, preMask);
-              __syncwarp();
             }
           }
         } else if (singleTile) {
           // one tile per CTA: the producers have nothing left to do and share the stores, 32 columns at a time
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&tileDone));
-          for (int c0 = 0; c0 < nEndT; c0 += 32 * (1 + kTsGroups)) ts_store_cols<kGen>(p, Psm + (size_t)c0 * BM, lane, dst, tc, c0, 32, false);
+          for (int c0 = 0; c0 < nEndT; c0 += 32 * (1 + kTsGroups)) ts_store_cols<kGen>(p, Psm + (size_t)c0 * BM, dst, tc, c0, 32, false);
         } else {
           // the tile is complete in P: store it while the tensor core works on the next tile (its chains wait in
           // their T buffers until this is through)
-          __syncwarp();
-          ts_store_cols<kGen>(p, Psm, lane, dst, tc, 0, BN, false);
-          __syncwarp();
+          ts_store_cols<kGen>(p, Psm, dst, tc, 0, BN, false);
         }
       }
     };
@@ -1527,6 +1497,8 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
       else drain(std::integral_constant<int, 0>{});
     } else if constexpr (kNarrow) {
       if (regsP && BN == 64) drain(std::integral_constant<int, 64>{});
+      else if (regsP && BN == 32) drain(std::integral_constant<int, 32>{});
+      else if (regsP) drain(std::integral_constant<int, 16>{});
       else drain(std::integral_constant<int, 0>{});
     } else {
       if (regsP && BN == 128) drain(std::integral_constant<int, 128>{});
@@ -1978,9 +1950,9 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
       if (!done) { if (lane == 0) atomicExch(p.status, 3); }
       else {
         int const tile = cta;
-        TsDst const dst = ts_dst<kGen>(p, tile / p.tilesN, quarter, lane);
+        TsDst const dst = ts_dst<kGen>(p, tile / p.tilesN, quarter * 32 + lane);
         TileCols const tc = tile_cols<kGen>(p, tile % p.tilesN);
-        for (int c0 = 32 * (1 + grp); c0 < tc.cnt; c0 += 32 * (1 + kTsGroups)) ts_store_cols<kGen>(p, Psm + (size_t)c0 * BM, lane, dst, tc, c0, 32, false);
+        for (int c0 = 32 * (1 + grp); c0 < tc.cnt; c0 += 32 * (1 + kTsGroups)) ts_store_cols<kGen>(p, Psm + (size_t)c0 * BM, dst, tc, c0, 32, false);
       }
       tc_fence_before();
     }
@@ -2479,7 +2451,7 @@ EncodeTiledFn encode_tiled()
 // the per-thread gather is the faster route by 10-15%; on 224 x 224 and 112 x 112 maps the copies win by up to 20% on
 // 64-column tiles and draw level on 128-column tiles), and room in shared memory for two windows.
 // Shared memory of conv_ts_kernel for the running sum of a tile: a patch of 32 columns for the tile widths whose sum lives in registers.
-size_t p_bytes(int BN, int smemSum) { return sizeof(float) * (size_t)(((BN == 128 || BN == 64) && !smemSum) ? 32 : BN) * BM; }
+size_t p_bytes(int BN, int smemSum) { return sizeof(float) * (size_t)(((BN == 128 || BN == 64) && !smemSum) ? 32 : BN) * BM; }      // (narrower tiles: their own width)
 
 bool plan_windows(vlb_ctx* ctx, Params& p, CUtensorMap* map, size_t* smemBytes, bool split3)
 {
@@ -2536,13 +2508,6 @@ void ts_divisors(Params& p)
   p.dTilesN = vlb::FastDiv31(p.tilesN); p.dTilesM = vlb::FastDiv31(p.tilesM);
 }
 
-// Whether four rows of a tile, the first a multiple of four, lie next to each other in the output: planes of a multiple of four pixels
-// (linear tiles), columns of one (boxes), pixels one apart, everything on 16-byte boundaries.
-bool rows_contiguous(Params const& p)
-{
-  return p.e.P % 4 == 0 && aligned16(p.e.out) && p.e.splitStride % 4 == 0 && (p.e.mask == nullptr || aligned16(p.e.mask));
-}
-
 // fprop / stride-1 dgrad with the gathered operand in tensor memory (p.bTiles set, p.a a convolution operand).
 int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
 {
@@ -2561,7 +2526,7 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   bool const windows = plan_windows(ctx, p, &map, &smemBytes, split3);
-  p.vecStore = rows_contiguous(p) && (!windows || p.a.Ho % 4 == 0);
+  p.biasFirst = p.e.bias != nullptr && aligned16(p.e.bias) && p.N % 4 == 0 && p.e.inMult == 1.f && p.e.outMult == 0.f;
   ts_divisors(p);
   if (smemBytes < 120u * 1024u) smemBytes = 120u * 1024u;
   long long const numTiles = (long long)p.tilesM * p.tilesN * p.splits;
@@ -2676,7 +2641,6 @@ int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* whe
   size_t smemBytes = (size_t)p.bStages * bBytes + pBytes + (size_t)p.xStages * kWgStageBytes + 1024;
   if (smemBytes < 120u * 1024u) smemBytes = 120u * 1024u;      // two CTAs (each allocating all 512 TMEM columns) never share an SM
   p.wg = 1;
-  p.vecStore = rows_contiguous(p) && p.a.FH * p.a.FW == 1;
   ts_divisors(p);
   p.status = ctx->deviceStatus;
   p.testSwitch = ctx->testSwitch;
@@ -2981,7 +2945,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     if (splits > 1) p.e.out = part;
     p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;
     ts_divisors(p);
-    p.vecStore = rows_contiguous(p) && p.shufY == 0 && p.oys == 1 && p.oxs == 1 && p.outH == p.a.Ho && p.outW == p.a.Wo;
+    p.biasFirst = p.e.bias != nullptr && aligned16(p.e.bias) && p.cols % 4 == 0 && p.shufY == 0 && p.e.inMult == 1.f && p.e.outMult == 0.f;
   }
   launch_prep(ctx, prep, b.n);
   size_t const smemBytes = std::max<size_t>((size_t)stages * stageBytes + sumBytes + 1024, 120u * 1024u);      // two CTAs never share an SM
