@@ -1848,61 +1848,32 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
               float v[32];
               int const u0 = (kb0 + it) * kPer;
               int cb = u0 / taps, tap = u0 - cb * taps;
-              if constexpr (kU <= 3) {
-                // First every load of the k-block, then the zeros: a value tested as soon as it is asked for would make the thread wait for
-                // memory once per unit.
-                uint32_t off = 0;                                  // units that are padding for this pixel
-                int const cb0 = cb, tap0 = tap;
+              // First every load of the k-block, then the zeros of what is padding: a register overwritten while its load is on the way
+              // makes the thread wait for memory, once per unit.
+              uint32_t off = 0;
 #pragma unroll
-                for (int u = 0; u < kPer; ++u) {
-                  int2 const te = tapLut[tap];
-                  uint32_t const e = (uint32_t)te.y;
-                  int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
-                  bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
-                  off |= on ? 0u : 1u << u;
-                  // (unconditional loads: what is padding reads the start of the tensor, channels that do not exist the first of the unit)
-                  float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;
+              for (int u = 0; u < kPer; ++u) {
+                int2 const te = tapLut[tap];
+                uint32_t const e = (uint32_t)te.y;
+                int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
+                bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
+                off |= on ? 0u : 1u << u;
+                float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;      // (padding reads the start of the tensor and discards it)
+                if (kU == 1 || left >= kU) {
                   long long const step = on ? (long long)HW : 0;
-                  if (kU == 1 || left >= kU) {
 #pragma unroll
-                    for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + k * step);
-                  } else {
+                  for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + k * step);
+                } else {
 #pragma unroll
-                    for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + (k < left ? k : 0) * step);
-                  }
-                  if (++tap == taps) { tap = 0; ++cb; }
+                  for (int k = 0; k < kU; ++k) { v[u * kU + k] = 0.f; ldg32_if(v[u * kU + k], q + (long long)k * HW, on && k < left); }
                 }
-                cb = cb0; tap = tap0;
+                if (++tap == taps) { tap = 0; ++cb; }
+              }
+              if (off != 0) {
 #pragma unroll
                 for (int u = 0; u < kPer; ++u) {
-                  int const left = ((off >> u) & 1u) ? 0 : p.a.C - cb * kU;
-                  if (left < kU) {
 #pragma unroll
-                    for (int k = 0; k < kU; ++k) v[u * kU + k] = k < left ? v[u * kU + k] : 0.f;
-                  }
-                  if (kU > 1 && ++tap == taps) { tap = 0; ++cb; }
-                }
-              } else {
-#pragma unroll
-                for (int u = 0; u < kPer; ++u) {
-                  int2 const te = tapLut[tap];
-                  uint32_t const e = (uint32_t)te.y;
-                  int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
-                  bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
-                  float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;
-                  if (left >= kU) {
-                    long long const step = on ? (long long)HW : 0;
-#pragma unroll
-                    for (int k = 0; k < kU; ++k) v[u * kU + k] = __ldg(q + k * step);
-                    if (!on) {
-#pragma unroll
-                      for (int k = 0; k < kU; ++k) v[u * kU + k] = 0.f;
-                    }
-                  } else {
-#pragma unroll
-                    for (int k = 0; k < kU; ++k) { v[u * kU + k] = 0.f; ldg32_if(v[u * kU + k], q + (long long)k * HW, on && k < left); }
-                  }
-                  if (++tap == taps) { tap = 0; ++cb; }
+                  for (int k = 0; k < kU; ++k) v[u * kU + k] = ((off >> u) & 1u) ? 0.f : v[u * kU + k];
                 }
               }
 #pragma unroll
