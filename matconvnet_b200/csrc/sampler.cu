@@ -1,12 +1,10 @@
 // Bilinear sampler (vl::nn::BilinearSampler, reference bits/nnbilinearsampler.hpp:21-36;
 // CPU definition bits/nnbilinearsampler.cu:32-149).
 //
-// Forward and backward-to-grid: one thread per output pixel (q = ho + Ho*wo, grid n) walks the C
-// channels: the grid entry and the four tap weights are computed once and reused for every
-// channel; reads of dy and writes of y are contiguous across the warp; x taps of neighbouring
-// output pixels fall in the same or adjacent 32-byte sectors.  Backward-to-grid accumulates the
-// channels in ascending order in a register, the order of the CPU loop, and writes each grid
-// entry once.
+// Forward and backward-to-grid stage the planes of a few channels in shared memory and walk the output
+// pixels (q = ho + Ho*wo, grid n); where that does not pay, one thread per output pixel reads its taps
+// from global memory.  The tap weights are formed once per pixel and the channels of the grid derivative
+// added in ascending order, as in the CPU loop; each grid entry is written once.
 //
 // Backward-to-data is a gather, not the reference GPU code's four atomicAdds per output element
 // (bits/impl/nnbilinearsampler_gpu.cu:38-118).  Which output pixels touch an input pixel depends
@@ -14,14 +12,10 @@
 // memory: it counts the taps that land on every input pixel, prefix-sums the counts, fills one
 // list (output pixel, tap) per input pixel and sorts each list by output pixel.  Then every
 // input pixel adds up its list in ascending output-pixel order -- the order in which the CPU loop
-// reaches that element (bits/nnbilinearsampler.cu:72-131) -- for four channels per walk of the
-// list (the dY planes of four channels wait in shared memory, the next four travel meanwhile;
-// decoding an entry and forming its weight is paid once for the four), and writes dX once: no
-// atomics, no zero fill, the CPU's result bit for bit, identical from run to run.  The grid
-// derivative is a second sweep of the same CTA over the channels, two at a time, with the x
-// planes staged beside the dY planes (dY is read a second time), every output pixel adding its
-// channels' terms in ascending channel order.  A grid that sends more than kMaxList taps to one
-// input pixel, and planes too large for the lists, take the atomic scatter instead.
+// reaches that element (bits/nnbilinearsampler.cu:72-131) -- for eight channels per walk of the
+// list, and writes dX once: no atomics, no zero fill, the CPU's result bit for bit, identical from
+// run to run.  A grid that sends more than kMaxList taps to one input pixel, and planes too large for
+// the lists, take the atomic scatter instead.
 //
 // Boundary rule of the CPU reference, kept as it is: the taps are guarded by
 // `-1 <= sy && sy < inHeight` with inHeight a size_t (bits/nnbilinearsampler.cu:92), so
@@ -29,6 +23,7 @@
 // in either coordinate contribute nothing.
 #include "common.cuh"
 #include <math.h>
+#include <type_traits>
 
 namespace {
 
@@ -89,6 +84,40 @@ __global__ void sampler_kernel(float* __restrict__ y, float* __restrict__ dx, fl
     float* dxz = (kMode == 1 && dx) ? dx + imgOff : nullptr;
     size_t outOff = (size_t)q + (size_t)Q * C * (size_t)n;
     float accGy = 0.f, accGx = 0.f;
+    if (kMode == 0) {
+      // Four channels at a time, all sixteen loads on the way before the first is used: one channel at a time the thread waited for memory
+      // once per channel (64 x 64 x 32 x 256: 140 us -> 79 us; 41 us at copy speed).  A tap outside the plane reads the plane's first
+      // element and its product is dropped; adding the +0 in its place changes no sum, none of which is ever -0.
+      float wt[4];
+      int at[4];
+      bool on[4];
+#pragma unroll
+      for (int t4 = 0; t4 < 4; ++t4) {
+        on[t4] = ok[t4 >> 1][t4 & 1];
+        wt[t4] = __fmul_rn(wwx[t4 >> 1], wwy[t4 & 1]);
+        at[t4] = on[t4] ? idx[t4 >> 1][t4 & 1] : 0;
+      }
+      int const HW = H * W;
+      float* o = y + outOff;
+      for (int c = 0; c < C; c += 4) {
+        float v[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float const* const xk = xz + (size_t)min(k, C - 1 - c) * HW;
+#pragma unroll
+          for (int t4 = 0; t4 < 4; ++t4) v[k][t4] = __ldg(xk + at[t4]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float acc = 0.f;
+#pragma unroll
+          for (int t4 = 0; t4 < 4; ++t4) acc = __fadd_rn(acc, on[t4] ? __fmul_rn(wt[t4], v[k][t4]) : 0.f);
+          if (c + k < C) o[(size_t)k * Q] = acc;
+        }
+        xz += 4 * (size_t)HW; o += 4 * (size_t)Q;
+      }
+      continue;
+    }
     for (int c = 0; c < C; ++c) {
       if (kMode == 0) {
         float acc = 0.f;
@@ -127,60 +156,225 @@ __global__ void sampler_kernel(float* __restrict__ y, float* __restrict__ dx, fl
   }
 }
 
-// ---- backward-to-data as a gather (see the header comment) ----
-constexpr int kGatherThreads = 1024;
-constexpr int kMaxList = 48;          // taps of one grid on one input pixel beyond which the scatter path is used
-constexpr int kMaxQPerThread = 4;     // output pixels per thread whose taps and grid derivative are kept in registers
-constexpr int kCB = 4;                // channels per stage: one walk of a pixel's list serves four channels
+// ---- forward and grid derivative with the planes of four channels in shared memory, one float4 per pixel ----
+// The direct kernel above is bound by the tags of L1: the 32 output pixels of a warp lie on a slanted line of the input, so that every
+// load touches up to seven lines.  From shared memory a tap of four channels is one 16-byte read that the banks serve in four passes.
+// B200, 64 x 64 x 32 x 256: forward 79 -> 61 us; 41 us at copy speed, the issue of
+// instructions 71 % busy.
+constexpr int kPlaneThreads = 512;
+constexpr int kGridThreads = 512;
+constexpr int kPlaneQ = 2;             // output pixels per thread of the grid derivative
+constexpr int kGridCh = 2;             // channels per stage of the grid derivative
 
-// Shared memory (bytes): the stage buffers -- float[2][4][Q] (dY planes of four channels, double buffered) for the data gradient,
-// float[2][2 x HW + 2 x Q] (x and dY planes of two channels, double buffered) for the grid derivative -- | wq float2[Q] (the two
-// fractions of every output pixel) | cur int[HW] | ent uint16[4Q] (list entries: output pixel << 2 | tap)
-__host__ __device__ inline size_t gather_smem(int HW, int Q)
+struct PixTaps { int at, ok; float wx, wy; };      // first tap's offset; bit ii + 2*j: tap (row offset ii, column offset j) exists
+
+__device__ __forceinline__ PixTaps pix_taps(float2 gv, int H, int W)
 {
-  size_t const stageFloats = 8 * (size_t)Q > 4 * ((size_t)HW + Q) ? 8 * (size_t)Q : 4 * ((size_t)HW + Q);
-  return sizeof(float) * stageFloats + sizeof(int) * (size_t)HW + (sizeof(float2) + 4 * sizeof(uint16_t)) * (size_t)Q + 64;
+  Taps const t = make_taps(gv.x, gv.y, H, W);
+  PixTaps r;
+  r.wx = t.wx; r.wy = t.wy;
+  r.at = t.inside ? t.sy + t.sx * H : 0;
+  r.ok = t.inside ? (1 | (t.sy + 1 < H ? 2 : 0) | (t.sx + 1 < W ? 4 : 0) | ((t.sy + 1 < H && t.sx + 1 < W) ? 8 : 0)) : 0;
+  return r;
 }
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, void const* src)
 { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory"); }
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, void const* src)
 { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory"); }
 
 // n floats global -> shared by the whole block, asynchronously (16-byte pieces when both sides allow; copies of four bytes
-// keep the load/store unit busy four times as long and were measured to slow the whole stage down)
+// keep the load/store unit busy four times as long)
 __device__ __forceinline__ void stage_plane(float* dst, float const* src, int n)
 {
   uint32_t const d = (uint32_t)__cvta_generic_to_shared(dst);
   if ((n & 3) == 0 && ((((uintptr_t)src) | d) & 15) == 0) {
-    for (int i = threadIdx.x; i < n / 4; i += kGatherThreads) cp_async16(d + 16u * i, src + 4 * i);
+    for (int i = threadIdx.x; i < n / 4; i += blockDim.x) cp_async16(d + 16u * i, src + 4 * i);
   } else {
-    for (int i = threadIdx.x; i < n; i += kGatherThreads) cp_async4(d + 4u * i, src + i);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) cp_async4(d + 4u * i, src + i);
   }
 }
 
-// dY of the channels c .. c + nst - 1 (nst <= 4) of one grid, Q floats per channel, as nst planes of Q floats
-__device__ __forceinline__ void stage_dy4(float* dst, float const* src, int Q, int nst)
+// n pixels of nc <= 4 planes (HW apart) into xs; every thread has up to sixteen loads on the way
+__device__ __forceinline__ void stage_planes(float4* xs, float const* x, int HW, int nc)
 {
-  for (int j = 0; j < nst; ++j) stage_plane(dst + (size_t)Q * j, src + (size_t)Q * j, Q);
+  int const T = blockDim.x;
+  int const o1 = nc > 1 ? HW : 0, o2 = nc > 2 ? 2 * HW : 0, o3 = nc > 3 ? 3 * HW : 0;
+  for (int i = threadIdx.x; i < HW; i += 4 * T) {
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float const* const q = x + min(i + k * T, HW - 1);
+      v[k] = make_float4(__ldg(q), __ldg(q + o1), __ldg(q + o2), __ldg(q + o3));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * T < HW) xs[i + k * T] = v[k];
+  }
 }
 
-template <bool kWantGrid>
+__device__ __forceinline__ void add_tap(float4& a, float w, float4 v)
+{
+  a.x = __fadd_rn(a.x, __fmul_rn(w, v.x)); a.y = __fadd_rn(a.y, __fmul_rn(w, v.y));
+  a.z = __fadd_rn(a.z, __fmul_rn(w, v.z)); a.w = __fadd_rn(a.w, __fmul_rn(w, v.w));
+}
+
+// One block: one image, four channels, all output pixels of its grids.
+__global__ void __launch_bounds__(kPlaneThreads)
+sampler_fwd_planes_kernel(float* __restrict__ y, float const* __restrict__ x, float const* __restrict__ grid, int H, int W, int C, int Q, int group,
+                          int quads)
+{
+  vlb::pdl_wait();
+  extern __shared__ float4 xs[];
+  int const img = blockIdx.x / quads, c0 = (blockIdx.x - img * quads) * 4, nc = min(4, C - c0), HW = H * W;
+  stage_planes(xs, x + (size_t)HW * ((size_t)C * img + c0), HW, nc);
+  __syncthreads();
+  for (int gi = 0; gi < group; ++gi) {
+    int const n = img * group + gi;
+    float2 const* const gr = reinterpret_cast<float2 const*>(grid) + (size_t)Q * n;
+    float* const o = y + (size_t)Q * ((size_t)C * n + c0);
+    int q = threadIdx.x;
+    float2 next = q < Q ? __ldg(gr + q) : make_float2(0.f, 0.f);
+    for (; q < Q; q += kPlaneThreads) {
+      PixTaps const t = pix_taps(next, H, W);
+      if (q + kPlaneThreads < Q) next = __ldg(gr + q + kPlaneThreads);
+      float const wx0 = __fadd_rn(1.f, -t.wx), wy0 = __fadd_rn(1.f, -t.wy);
+      float4 const* const p0 = xs + t.at;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t.ok & 1) add_tap(a, __fmul_rn(wx0, wy0), p0[0]);
+      if (t.ok & 2) add_tap(a, __fmul_rn(wx0, t.wy), p0[1]);
+      if (t.ok & 4) add_tap(a, __fmul_rn(t.wx, wy0), p0[H]);
+      if (t.ok & 8) add_tap(a, __fmul_rn(t.wx, t.wy), p0[H + 1]);
+      o[q] = a.x;
+      if (nc == 4) {
+        o[q + Q] = a.y; o[q + 2 * Q] = a.z; o[q + 3 * Q] = a.w;
+      } else {
+        if (nc > 1) o[q + Q] = a.y;
+        if (nc > 2) o[q + 2 * Q] = a.z;
+      }
+    }
+  }
+}
+
+// One channel's terms of an output pixel, the taps in the CPU loop's order (column offset j outer, row offset i inner;
+// bits/nnbilinearsampler.cu:98-128).  (2j-1)*wwy*dy*x is evaluated left to right there; a negation is exact, so the two magnitudes
+// wwy0*dy and wwy1*dy serve all four taps.
+__device__ __forceinline__ void grid_terms(float& accGy, float& accGx, int ok, float wx0, float wx1, float wy0, float wy1, float d,
+                                           float x00, float x10, float x01, float x11, float sclY, float sclX)
+{
+  float const ty0 = __fmul_rn(wy0, d), ty1 = __fmul_rn(wy1, d), tx0 = __fmul_rn(wx0, d), tx1 = __fmul_rn(wx1, d);
+  float dgx = __fsub_rn(0.f, __fmul_rn(ty0, x00)), dgy = __fsub_rn(0.f, __fmul_rn(tx0, x00));
+  if (ok & 2) { dgx = __fsub_rn(dgx, __fmul_rn(ty1, x10)); dgy = __fadd_rn(dgy, __fmul_rn(tx0, x10)); }
+  if (ok & 4) { dgx = __fadd_rn(dgx, __fmul_rn(ty0, x01)); dgy = __fsub_rn(dgy, __fmul_rn(tx1, x01)); }
+  if (ok & 8) { dgx = __fadd_rn(dgx, __fmul_rn(ty1, x11)); dgy = __fadd_rn(dgy, __fmul_rn(tx1, x11)); }
+  accGy = __fadd_rn(accGy, __fmul_rn(sclY, dgy));
+  accGx = __fadd_rn(accGx, __fmul_rn(sclX, dgx));
+}
+
+// Grid derivative.  One block: one grid and QP <= kGridThreads * kPlaneQ of its output pixels, all channels in ascending order, kGridCh per
+// stage.  Bound by the issue of instructions, hence three blocks per SM
+// (64 x 64 x 32 x 256, two channels of two pixels per thread: 129 us; four channels or four pixels, with fewer warps: 137 to 160).  The x planes of the next stage travel by asynchronous copies, its dY
+// through registers: an output pixel's values are asked for as soon as those of this stage are used.
+__global__ void __launch_bounds__(kGridThreads, 3)
+sampler_grid_planes_kernel(float* __restrict__ dgrid, float const* __restrict__ x, float const* __restrict__ grid, float const* __restrict__ dy,
+                           int H, int W, int C, int Q, int group, int parts, int QP)
+{
+  vlb::pdl_wait();
+  extern __shared__ float4 xsm[];
+  int const n = blockIdx.x / parts, q0 = (blockIdx.x - n * parts) * QP, qEnd = min(Q, q0 + QP), HW = H * W;
+  float* const xs = reinterpret_cast<float*>(xsm);          // [2][kGridCh][HW]
+  float const* const xi = x + (size_t)HW * C * (n / group);
+  float2 const* const gr = reinterpret_cast<float2 const*>(grid) + (size_t)Q * n;
+  float const* const dyn = dy + (size_t)Q * C * n;
+  float const sclY = __fmul_rn(0.5f, (float)(H - 1)), sclX = __fmul_rn(0.5f, (float)(W - 1));
+  stage_plane(xs, xi, HW * min(kGridCh, C));
+  float accGy[kPlaneQ], accGx[kPlaneQ], wx[kPlaneQ], wy[kPlaneQ], d[kPlaneQ][kGridCh];
+  int at[kPlaneQ];                                          // first tap | which taps exist << 28
+#pragma unroll
+  for (int k = 0; k < kPlaneQ; ++k) {
+    int const q = q0 + threadIdx.x + k * kGridThreads;
+    accGy[k] = accGx[k] = 0.f;
+#pragma unroll
+    for (int j = 0; j < kGridCh; ++j) d[k][j] = 0.f;
+    at[k] = 0; wx[k] = wy[k] = 0.f;
+    if (q < qEnd) {
+      PixTaps const t = pix_taps(__ldg(gr + q), H, W);
+      at[k] = t.at | (t.ok << 28); wx[k] = t.wx; wy[k] = t.wy;
+#pragma unroll
+      for (int j = 0; j < kGridCh; ++j)
+        if (j < C) d[k][j] = __ldg(dyn + (size_t)Q * j + q);
+    }
+  }
+  int buf = 0;
+  for (int c0 = 0; c0 < C; c0 += kGridCh, buf ^= 1) {
+    int const nc = min(kGridCh, C - c0), left = C - c0 - kGridCh;
+    float const* const xc = xs + (size_t)(buf * kGridCh) * HW;
+    cp_async_wait_all();
+    __syncthreads();                    // this stage's planes have landed; the other buffer is no longer read
+    if (left > 0) stage_plane(xs + (size_t)((buf ^ 1) * kGridCh) * HW, xi + (size_t)HW * (c0 + kGridCh), HW * min(kGridCh, left));
+    float const* const dn = dyn + (size_t)Q * (c0 + kGridCh) + q0 + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < kPlaneQ; ++k) {
+      int const ok = (int)((unsigned)at[k] >> 28);
+      if (ok) {
+        float const wx0 = __fadd_rn(1.f, -wx[k]), wy0 = __fadd_rn(1.f, -wy[k]);
+        float const* p0 = xc + (at[k] & 0x0fffffff);
+        float v[kGridCh][4];
+#pragma unroll
+        for (int j = 0; j < kGridCh; ++j) {
+          v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
+          if (j < nc) {
+            v[j][0] = p0[0];
+            if (ok & 2) v[j][1] = p0[1];
+            if (ok & 4) v[j][2] = p0[H];
+            if (ok & 8) v[j][3] = p0[H + 1];
+          }
+          p0 += HW;
+        }
+#pragma unroll
+        for (int j = 0; j < kGridCh; ++j)
+          if (j < nc) grid_terms(accGy[k], accGx[k], ok, wx0, wx[k], wy0, wy[k], d[k][j], v[j][0], v[j][1], v[j][2], v[j][3], sclY, sclX);
+#pragma unroll
+        for (int j = 0; j < kGridCh; ++j)
+          if (j < left) d[k][j] = __ldg(dn + Q * j + k * kGridThreads);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kPlaneQ; ++k) {
+    int const q = q0 + threadIdx.x + k * kGridThreads;
+    if (q < qEnd) reinterpret_cast<float2*>(dgrid)[(size_t)Q * n + q] = make_float2(accGy[k], accGx[k]);
+  }
+}
+
+// ---- backward-to-data as a gather (see the header comment) ----
+constexpr int kGatherThreads = 1024;
+constexpr int kMaxList = 48;          // taps of one grid on one input pixel beyond which the scatter path is used
+constexpr int kMaxQPerThread = 4;     // output pixels per thread
+constexpr int kCB = 8;                // channels per stage: one walk of a pixel's list serves eight channels
+
+// Shared memory (bytes): dys float4[2][Q] (dY of eight channels, four side by side) | wq float2[Q] (the two fractions of every output pixel) |
+// ent uint16[4Q] (list entries: output pixel << 2 | tap) | cur int[HW + 1] (where every input pixel's list begins)
+__host__ __device__ inline size_t gather_smem(int HW, int Q)
+{ return (2 * sizeof(float4) + sizeof(float2) + 4 * sizeof(uint16_t)) * (size_t)Q + sizeof(int) * ((size_t)HW + 1) + 64; }
+
+// Bound by shared memory: an entry of a list costs one 2-byte, one 8-byte and two 16-byte reads for eight channels, the last two bank passes
+// per channel.  dY travels through registers (it has to be laid side by side), asked for one stage ahead.
+// B200, 64 x 64 x 32 x 256, both derivatives: 268 us with four channels per walk and the grid derivative in the same
+// block, 255 us now; half of that is the data gradient, for which 256 images on 148 SMs are two rounds, the second not full.
 __global__ void __launch_bounds__(kGatherThreads, 1)
-sampler_bwd_gather_kernel(float* __restrict__ dx, float* __restrict__ dgrid, float const* __restrict__ x,
-                          float const* __restrict__ grid, float const* __restrict__ dy, int H, int W, int C, int N, int Q, int Ng,
+sampler_bwd_gather_kernel(float* __restrict__ dx, float const* __restrict__ grid, float const* __restrict__ dy, int H, int W, int C, int N, int Q, int Ng,
                           int chunks, int CH)
 {
   vlb::pdl_wait();
   extern __shared__ __align__(16) uint8_t sm[];
   __shared__ int warpSums[32];
   int const HW = H * W, tid = threadIdx.x;
-  float* dy4 = reinterpret_cast<float*>(sm);                              // [2][4][Q]
-  float2* wq = reinterpret_cast<float2*>(dy4 + (2 * kCB * (size_t)Q > 4 * ((size_t)HW + Q) ? 2 * kCB * (size_t)Q : 4 * ((size_t)HW + Q)));            // [Q]   (wx, wy) of every output pixel
-  int* cur = reinterpret_cast<int*>(wq + Q);                              // [HW]  list ends (starts before the fill)
-  uint16_t* ent = reinterpret_cast<uint16_t*>(cur + HW);                  // [4Q]  output pixel << 2 | tap (tap = 2*column offset + row offset)
+  float4* dys = reinterpret_cast<float4*>(sm);                              // [2][Q]
+  float2* wq = reinterpret_cast<float2*>(dys + 2 * (size_t)Q);              // [Q]   (wx, wy) of every output pixel
+  uint16_t* ent = reinterpret_cast<uint16_t*>(wq + Q);                      // [4Q]  output pixel << 2 | tap (tap = 2*column offset + row offset)
+  int* cur = reinterpret_cast<int*>(ent + 4 * (size_t)Q);                   // [HW + 1]
   int const group = Ng / N;
   int const img = blockIdx.x / chunks, c0 = (blockIdx.x % chunks) * CH, nch = min(CH, C - c0);
   int const nStages = (nch + kCB - 1) / kCB;
@@ -190,23 +384,22 @@ sampler_bwd_gather_kernel(float* __restrict__ dx, float* __restrict__ dgrid, flo
     int const n = img * group + gi;
     float2 const* gr = reinterpret_cast<float2 const*>(grid) + (size_t)Q * n;
     float const* const dyn = dy + (size_t)Q * C * (size_t)n;
-    // the first stage's dY starts travelling while the grid is inverted
-    stage_dy4(dy4, dyn + (size_t)Q * c0, Q, min(kCB, nch));
     // ---- invert the grid: count, scan, fill, sort
-    for (int i = tid; i < HW; i += kGatherThreads) cur[i] = 0;
+    for (int i = tid; i <= HW; i += kGatherThreads) cur[i] = 0;
     __syncthreads();
-    for (int q = tid; q < Q; q += kGatherThreads) {
-      float2 const gv = gr[q];
-      Taps t = make_taps(gv.x, gv.y, H, W);
-      wq[q] = make_float2(t.wx, t.wy);
-      if (t.inside) {
+    int at[kMaxQPerThread];               // first tap of this thread's output pixels | which taps exist << 28
+    uint32_t rank[kMaxQPerThread];        // its four taps' places in their lists, a byte each
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+    for (int k = 0; k < kMaxQPerThread; ++k) {
+      int const q = tid + k * kGatherThreads;
+      at[k] = 0; rank[k] = 0;
+      if (q < Q) {
+        PixTaps const t = pix_taps(__ldg(gr + q), H, W);
+        wq[q] = make_float2(t.wx, t.wy);
+        at[k] = t.at | (t.ok << 28);
 #pragma unroll
-          for (int ii = 0; ii < 2; ++ii) {
-            int const ssy = t.sy + ii, ssx = t.sx + j;
-            if (ssy < H && ssx < W) atomicAdd(&cur[ssy + ssx * H], 1);
-          }
+        for (int b = 0; b < 4; ++b)
+          if (t.ok & (1 << b)) rank[k] |= ((uint32_t)atomicAdd(&cur[t.at + (b & 1) + (b >> 1) * H], 1) & 255u) << (8 * b);
       }
     }
     __syncthreads();
@@ -214,27 +407,34 @@ sampler_bwd_gather_kernel(float* __restrict__ dx, float* __restrict__ dgrid, flo
     for (int i = tid; i < HW; i += kGatherThreads) tooLong |= cur[i] > kMaxList;
     bool const scatter = __syncthreads_or(tooLong) != 0;
     if (!scatter) {
-      vlb::block_exclusive_scan<kGatherThreads>(cur, HW, warpSums);
-      for (int q = tid; q < Q; q += kGatherThreads) {
-        float2 const gv = gr[q];
-        Taps t = make_taps(gv.x, gv.y, H, W);
-        if (t.inside) {
+      vlb::block_exclusive_scan<kGatherThreads>(cur, HW + 1, warpSums);
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
+      for (int k = 0; k < kMaxQPerThread; ++k) {
+        int const q = tid + k * kGatherThreads, ok = (int)((unsigned)at[k] >> 28), first = at[k] & 0x0fffffff;
 #pragma unroll
-            for (int ii = 0; ii < 2; ++ii) {
-              int const ssy = t.sy + ii, ssx = t.sx + j;
-              if (ssy < H && ssx < W) {
-                int const pos = atomicAdd(&cur[ssy + ssx * H], 1);
-                ent[pos] = (uint16_t)((q << 2) | (2 * j + ii));
-              }
-            }
-        }
+        for (int b = 0; b < 4; ++b)
+          if (ok & (1 << b)) ent[cur[first + (b & 1) + (b >> 1) * H] + (int)((rank[k] >> (8 * b)) & 255u)] = (uint16_t)((q << 2) | b);
       }
+      // the dY of the stage that comes next, on its way while this one is computed
+      float v[kMaxQPerThread][kCB] = {};
+      auto ask = [&](int cs) {
+        int const left = c0 + nch - cs;
+#pragma unroll
+        for (int k = 0; k < kMaxQPerThread; ++k) {
+          int const q = tid + k * kGatherThreads;
+          if (q < Q) {
+            float const* const d = dyn + (size_t)Q * cs + q;
+#pragma unroll
+            for (int j = 0; j < kCB; ++j)
+              if (j < left) v[k][j] = __ldg(d + (size_t)Q * j);
+          }
+        }
+      };
+      ask(c0);
       __syncthreads();
       // every input pixel sorts its list by output pixel (an output pixel reaches an input pixel with one tap at most)
       for (int pix = tid; pix < HW; pix += kGatherThreads) {
-        int const beg = pix == 0 ? 0 : cur[pix - 1], end = cur[pix];
+        int const beg = cur[pix], end = cur[pix + 1];
         for (int a = beg + 1; a < end; ++a) {
           uint16_t const kq = ent[a];
           int b = a - 1;
@@ -242,180 +442,100 @@ sampler_bwd_gather_kernel(float* __restrict__ dx, float* __restrict__ dgrid, flo
           ent[b + 1] = kq;
         }
       }
-      // ---- data gradient, four channels at a time from shared memory: the dY of stage s + 1 travels while stage s is computed
       for (int st = 0; st < nStages; ++st) {
         int const cs = c0 + st * kCB, nst = min(kCB, c0 + nch - cs);
-        float const* const ds = dy4 + (size_t)(st & 1) * kCB * Q;
-        cp_async_wait_all();
-        __syncthreads();                    // this stage's dY has landed (and the lists are sorted); the other buffer is no longer read
-        if (st + 1 < nStages) stage_dy4(dy4 + (size_t)((st + 1) & 1) * kCB * Q, dyn + (size_t)Q * (cs + kCB), Q, min(kCB, c0 + nch - cs - kCB));
-        // every input pixel adds up its list in output-pixel order, four channels per walk.  The weight of an entry
-        // is wwx[j] * wwy[i] as the CPU loop forms it (bits/nnbilinearsampler.cu:108-110), from the output pixel's two fractions.
-        float* const dxc = dx + imgOff + (size_t)HW * cs;
-        for (int pix = tid; pix < HW; pix += kGatherThreads) {
-          int const beg = pix == 0 ? 0 : cur[pix - 1], end = cur[pix];
-          float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-          if (gi > 0) {
-            a0 = dxc[pix];
-            if (nst > 1) a1 = dxc[pix + (size_t)HW];
-            if (nst > 2) a2 = dxc[pix + 2 * (size_t)HW];
-            if (nst > 3) a3 = dxc[pix + 3 * (size_t)HW];
-          }
-          for (int e = beg; e < end; ++e) {
-            unsigned const en = ent[e];
-            unsigned const q = en >> 2;
-            float2 const f = wq[q];
-            float const wx = (en & 2u) ? f.x : __fadd_rn(1.f, -f.x), wy = (en & 1u) ? f.y : __fadd_rn(1.f, -f.y);
-            float const w = __fmul_rn(wx, wy);
-            float const* const d = ds + q;
-            a0 = __fadd_rn(a0, __fmul_rn(w, d[0])); a1 = __fadd_rn(a1, __fmul_rn(w, d[Q]));
-            a2 = __fadd_rn(a2, __fmul_rn(w, d[2 * Q])); a3 = __fadd_rn(a3, __fmul_rn(w, d[3 * Q]));
-          }
-          dxc[pix] = a0;
-          if (nst > 1) dxc[pix + (size_t)HW] = a1;
-          if (nst > 2) dxc[pix + 2 * (size_t)HW] = a2;
-          if (nst > 3) dxc[pix + 3 * (size_t)HW] = a3;
-        }
-      }
-      // ---- grid derivative: a second sweep over the channels, two at a time, with the x planes beside the dY planes in the
-      // stage buffers (dY is read a second time).  Every output pixel adds its channels' terms in ascending channel order, the
-      // taps in the CPU loop's order (column offset j outer, row offset i inner; bits/nnbilinearsampler.cu:98-128).
-      // (2j-1)*wwy*dy*x is evaluated left to right there; a negation is exact, so the two magnitudes wwy0*dy and wwy1*dy serve
-      // all four taps.
-      if (kWantGrid) {
-        float accGy[kMaxQPerThread], accGx[kMaxQPerThread];
-        // this thread's output pixels: first tap's offset in the plane | which of the four taps exist << 28, the two fractions
-        int tapInfo[kMaxQPerThread];
-        float tapWx[kMaxQPerThread], tapWy[kMaxQPerThread];
+        if (st > 0) __syncthreads();        // the previous stage is no longer read
 #pragma unroll
         for (int k = 0; k < kMaxQPerThread; ++k) {
-          accGy[k] = 0.f; accGx[k] = 0.f;
-          tapInfo[k] = 0; tapWx[k] = 0.f; tapWy[k] = 0.f;
           int const q = tid + k * kGatherThreads;
           if (q < Q) {
-            float2 const gv = gr[q];
-            Taps t = make_taps(gv.x, gv.y, H, W);
-            tapWx[k] = t.wx; tapWy[k] = t.wy;
-            if (t.inside)
-              tapInfo[k] = (t.sy + t.sx * H) |
-                           ((1 | (t.sy + 1 < H ? 2 : 0) | (t.sx + 1 < W ? 4 : 0) | ((t.sy + 1 < H && t.sx + 1 < W) ? 8 : 0)) << 28);   // bit ii + 2*j
+            dys[q] = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+            if (nst > 4) dys[Q + q] = make_float4(v[k][4], v[k][5], v[k][6], v[k][7]);
           }
         }
-        float const sclY = __fmul_rn(0.5f, (float)(H - 1)), sclX = __fmul_rn(0.5f, (float)(W - 1));
-        // buffer b: x planes of two channels, then their dY planes
-        size_t const bufFloats = 2 * ((size_t)HW + Q);
-        auto stage2 = [&](int b, int cs, int n2) {
-          float* const base = dy4 + (size_t)b * bufFloats;
-          for (int j = 0; j < n2; ++j) {
-            stage_plane(base + (size_t)HW * j, x + imgOff + (size_t)HW * (cs + j), HW);
-            stage_plane(base + 2 * (size_t)HW + (size_t)Q * j, dyn + (size_t)Q * (cs + j), Q);
+        __syncthreads();                    // (and the lists are sorted)
+        if (st + 1 < nStages) ask(cs + kCB);
+        // every input pixel adds up its list in output-pixel order.  The weight of an entry is wwx[j] * wwy[i] as the CPU loop
+        // forms it (bits/nnbilinearsampler.cu:108-110), from the output pixel's two fractions.
+        float* const dxc = dx + imgOff + (size_t)HW * cs;
+        auto walk = [&](auto full) {
+          int const m = decltype(full)::value ? kCB : nst;       // (a constant in all stages but the last)
+          for (int pix = tid; pix < HW; pix += kGatherThreads) {
+            int const beg = cur[pix], end = cur[pix + 1];
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            float* const o = dxc + pix;
+            if (gi > 0) {
+              a.x = o[0];
+              if (m > 1) a.y = o[HW];
+              if (m > 2) a.z = o[2 * HW];
+              if (m > 3) a.w = o[3 * HW];
+              if (m > 4) b.x = o[4 * HW];
+              if (m > 5) b.y = o[5 * HW];
+              if (m > 6) b.z = o[6 * HW];
+              if (m > 7) b.w = o[7 * HW];
+            }
+#pragma unroll 2
+            for (int e = beg; e < end; ++e) {
+              unsigned const en = ent[e];
+              unsigned const q = en >> 2;
+              float2 const f = wq[q];
+              float4 const da = dys[q], db = m > 4 ? dys[Q + q] : da;
+              float const wx = (en & 2u) ? f.x : __fadd_rn(1.f, -f.x), wy = (en & 1u) ? f.y : __fadd_rn(1.f, -f.y);
+              float const w = __fmul_rn(wx, wy);
+              add_tap(a, w, da);
+              if (m > 4) add_tap(b, w, db);
+            }
+            o[0] = a.x;
+            if (m > 1) o[HW] = a.y;
+            if (m > 2) o[2 * HW] = a.z;
+            if (m > 3) o[3 * HW] = a.w;
+            if (m > 4) o[4 * HW] = b.x;
+            if (m > 5) o[5 * HW] = b.y;
+            if (m > 6) o[6 * HW] = b.z;
+            if (m > 7) o[7 * HW] = b.w;
           }
         };
-        int const nStages2 = (nch + 1) / 2;
-        __syncthreads();                    // the last stage's dY is no longer read
-        stage2(0, c0, min(2, nch));
-        for (int st = 0; st < nStages2; ++st) {
-          int const cs = c0 + 2 * st, n2 = min(2, c0 + nch - cs);
-          float const* const xs = dy4 + (size_t)(st & 1) * bufFloats;
-          float const* const ds = xs + 2 * (size_t)HW;
-          cp_async_wait_all();
-          __syncthreads();
-          if (st + 1 < nStages2) stage2((st + 1) & 1, cs + 2, min(2, c0 + nch - cs - 2));
-#pragma unroll
-          for (int k = 0; k < kMaxQPerThread; ++k) {
-            int const q = tid + k * kGatherThreads;
-            int const ok = (int)((unsigned)tapInfo[k] >> 28);
-            if (q < Q && ok) {
-              float const wx1 = tapWx[k], wy1 = tapWy[k], wx0 = __fadd_rn(1.f, -wx1), wy0 = __fadd_rn(1.f, -wy1);
-              float const* p0 = xs + (tapInfo[k] & 0x0fffffff);      // taps (i = 0, 1; j = 0), and H further on (j = 1)
-              float const* dq = ds + q;
-              for (int j = 0; j < n2; ++j) {
-                float const d = dq[0];
-                float const ty0 = __fmul_rn(wy0, d), ty1 = __fmul_rn(wy1, d), tx0 = __fmul_rn(wx0, d), tx1 = __fmul_rn(wx1, d);
-                float dgx, dgy;
-                if (ok == 15) {
-                  float const x00 = p0[0], x10 = p0[1], x01 = p0[H], x11 = p0[H + 1];
-                  dgx = __fsub_rn(0.f, __fmul_rn(ty0, x00)); dgy = __fsub_rn(0.f, __fmul_rn(tx0, x00));
-                  dgx = __fsub_rn(dgx, __fmul_rn(ty1, x10)); dgy = __fadd_rn(dgy, __fmul_rn(tx0, x10));
-                  dgx = __fadd_rn(dgx, __fmul_rn(ty0, x01)); dgy = __fsub_rn(dgy, __fmul_rn(tx1, x01));
-                  dgx = __fadd_rn(dgx, __fmul_rn(ty1, x11)); dgy = __fadd_rn(dgy, __fmul_rn(tx1, x11));
-                } else {
-                  {                                         // j = 0, i = 0: dgx -= wwy0*d*x, dgy -= wwx0*d*x
-                    float const xv = p0[0];
-                    dgx = __fsub_rn(0.f, __fmul_rn(ty0, xv)); dgy = __fsub_rn(0.f, __fmul_rn(tx0, xv));
-                  }
-                  if (ok & 2) {                             // j = 0, i = 1: dgx -= wwy1*d*x, dgy += wwx0*d*x
-                    float const xv = p0[1];
-                    dgx = __fsub_rn(dgx, __fmul_rn(ty1, xv)); dgy = __fadd_rn(dgy, __fmul_rn(tx0, xv));
-                  }
-                  if (ok & 4) {                             // j = 1, i = 0: dgx += wwy0*d*x, dgy -= wwx1*d*x
-                    float const xv = p0[H];
-                    dgx = __fadd_rn(dgx, __fmul_rn(ty0, xv)); dgy = __fsub_rn(dgy, __fmul_rn(tx1, xv));
-                  }
-                  if (ok & 8) {                             // j = 1, i = 1: dgx += wwy1*d*x, dgy += wwx1*d*x
-                    float const xv = p0[H + 1];
-                    dgx = __fadd_rn(dgx, __fmul_rn(ty1, xv)); dgy = __fadd_rn(dgy, __fmul_rn(tx1, xv));
-                  }
-                }
-                accGy[k] = __fadd_rn(accGy[k], __fmul_rn(sclY, dgy));
-                accGx[k] = __fadd_rn(accGx[k], __fmul_rn(sclX, dgx));
-                p0 += HW; dq += Q;
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < kMaxQPerThread; ++k) {
-          int const q = tid + k * kGatherThreads;
-          if (q < Q) reinterpret_cast<float2*>(dgrid)[(size_t)Q * n + q] = make_float2(accGy[k], accGx[k]);
-        }
+        if (nst == kCB) walk(std::integral_constant<bool, true>{});
+        else            walk(std::integral_constant<bool, false>{});
       }
     } else {
       // a grid that piles its taps on a few input pixels: zero (first grid of the image) and scatter with atomics, from
       // global memory
-      cp_async_wait_all();
       if (gi == 0) {
         for (size_t i = tid; i < (size_t)HW * nch; i += kGatherThreads) dx[imgOff + (size_t)HW * c0 + i] = 0.f;
       }
       __syncthreads();
       for (int q = tid; q < Q; q += kGatherThreads) {
-        float2 const gv = gr[q];
-        Taps t = make_taps(gv.x, gv.y, H, W);
+        PixTaps const t = pix_taps(__ldg(gr + q), H, W);
         float const wwx[2] = {__fadd_rn(1.f, -t.wx), t.wx};
         float const wwy[2] = {__fadd_rn(1.f, -t.wy), t.wy};
-        float accGy = 0.f, accGx = 0.f;
-        for (int c = 0; c < (kWantGrid ? C : nch); ++c) {
-          int const ch = kWantGrid ? c : c0 + c;
-          float const d = dyn[q + (size_t)Q * ch];
-          float* const dxz = dx + imgOff + (size_t)HW * ch;
-          float const* const xz = x + imgOff + (size_t)HW * ch;
-          bool const mine = ch >= c0 && ch < c0 + nch;
-          float dgx = 0.f, dgy = 0.f;
+        for (int c = c0; c < c0 + nch; ++c) {
+          float const d = dyn[q + (size_t)Q * c];
+          float* const dxz = dx + imgOff + (size_t)HW * c + t.at;
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int ii = 0; ii < 2; ++ii) {
-              int const ssy = t.sy + ii, ssx = t.sx + j;
-              if (t.inside && ssy < H && ssx < W) {
-                if (mine) atomicAdd(dxz + ssy + ssx * H, __fmul_rn(__fmul_rn(wwx[j], wwy[ii]), d));
-                if (kWantGrid) {
-                  float const xv = __ldg(xz + ssy + ssx * H);
-                  float const sj = j ? 1.f : -1.f, si = ii ? 1.f : -1.f;
-                  dgx = __fadd_rn(dgx, __fmul_rn(__fmul_rn(__fmul_rn(sj, wwy[ii]), d), xv));
-                  dgy = __fadd_rn(dgy, __fmul_rn(__fmul_rn(__fmul_rn(si, wwx[j]), d), xv));
-                }
-              }
-            }
-          if (kWantGrid) {
-            accGy = __fadd_rn(accGy, __fmul_rn(__fmul_rn(0.5f, (float)(H - 1)), dgy));
-            accGx = __fadd_rn(accGx, __fmul_rn(__fmul_rn(0.5f, (float)(W - 1)), dgx));
-          }
+          for (int b = 0; b < 4; ++b)
+            if (t.ok & (1 << b)) atomicAdd(dxz + (b & 1) + (b >> 1) * H, __fmul_rn(__fmul_rn(wwx[b >> 1], wwy[b & 1]), d));
         }
-        if (kWantGrid) reinterpret_cast<float2*>(dgrid)[(size_t)Q * n + q] = make_float2(accGy, accGx);
       }
     }
     __syncthreads();       // this grid's additions to dX are visible to the block, and the lists free, before the next grid
   }
+}
+
+// The planes of four channels in shared memory (pixels: of the plane or planes that a block holds at a time), where an image fills a good part of
+// the chip with blocks, a stage of x is not mostly unread (Q at least half of a plane), and the planes fit.
+bool planes_apply(vlb_ctx* ctx, long long pixels, bool readsMost, int C, long long blocks)
+{ return C >= 3 && (long long)sizeof(float4) * pixels <= 220 * 1024 && readsMost && blocks >= ctx->smCount; }
+
+// the three kernels above take as much shared memory as an SM has; false with a CUDA error pending
+bool allow_smem(vlb_ctx* ctx)
+{
+  static bool done[64] = {};
+  if (ctx->device < 64 && done[ctx->device]) return true;
+  bool const ok = vlb::allow_max_dynamic_smem(sampler_fwd_planes_kernel) == cudaSuccess && vlb::allow_max_dynamic_smem(sampler_grid_planes_kernel) == cudaSuccess &&
+                  vlb::allow_max_dynamic_smem(sampler_bwd_gather_kernel) == cudaSuccess;
+  if (ok && ctx->device < 64) done[ctx->device] = true;
+  return ok;
 }
 
 int validate(vlb_ctx* ctx, int H, int W, int C, int N, int Ho, int Wo, int Ng)
@@ -439,6 +559,13 @@ int vlb_sampler_forward(vlb_ctx* ctx, float* Y, float const* X, float const* gri
   if (rc) return rc;
   VLB_REQUIRE(ctx, Y && X && grid, "sampler_forward: null tensor");
   VLB_REQUIRE(ctx, (((uintptr_t)grid) & 7) == 0, "sampler_forward: grid must be 8-byte aligned");
+  int const Q = Ho * Wo, quads = vlb::ceil_div(C, 4);
+  if (planes_apply(ctx, (long long)H * W, 2LL * Q >= (long long)H * W, C, (long long)N * quads)) {
+    if (!allow_smem(ctx)) return vlb::check_launch(ctx, "vlb_sampler_forward");
+    vlb::launch(ctx->stream, sampler_fwd_planes_kernel, (unsigned)(N * quads), kPlaneThreads, sizeof(float4) * (size_t)H * W, Y, X, grid, H, W, C, Q, Ng / N, quads);
+    VLB_LAUNCHED(ctx, 1);
+    return vlb::check_launch(ctx, "vlb_sampler_forward");
+  }
   size_t total = (size_t)Ho * Wo * Ng;
   vlb::launch(ctx->stream, sampler_kernel<0>, vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, 
       Y, nullptr, nullptr, X, grid, nullptr, H, W, C, N, Ho * Wo, Ng);
@@ -458,32 +585,30 @@ int vlb_sampler_backward(vlb_ctx* ctx, float* dX, float* dGrid, float const* X, 
   if (!dX && !dGrid) return VLB_Success;
   int const Qo = Ho * Wo, HWi = H * W;
   if (dX && Qo <= kMaxQPerThread * kGatherThreads && HWi < (1 << 28) && gather_smem(HWi, Qo) <= 226 * 1024) {
-    // gather: one CTA per image; with fewer images than SMs the channels are shared out among several CTAs per image,
-    // and the grid derivative (which runs over all channels of an output pixel in order) is left to the other kernel
+    // gather: one CTA per image; with fewer images than SMs the channels are shared out among several CTAs per image
     int chunks = 1;
     if (N < ctx->smCount) chunks = vlb::ceil_div(ctx->smCount, N);
     int CH = vlb::ceil_div(C, chunks);
     chunks = vlb::ceil_div(C, CH);
-    bool const fusedGrid = dGrid != nullptr && chunks == 1;
-    static bool attrDone[64] = {};
-    if (!(ctx->device < 64 && attrDone[ctx->device])) {
-      cudaError_t ea = vlb::allow_max_dynamic_smem(sampler_bwd_gather_kernel<true>);
-      if (ea == cudaSuccess) ea = vlb::allow_max_dynamic_smem(sampler_bwd_gather_kernel<false>);
-      if (ea != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(ea)); }
-      if (ctx->device < 64) attrDone[ctx->device] = true;
-    }
+    if (!allow_smem(ctx)) return vlb::check_launch(ctx, "vlb_sampler_backward");
     size_t const smem = gather_smem(HWi, Qo);
     unsigned const blocks = (unsigned)(N * chunks);
-    if (fusedGrid) vlb::launch(ctx->stream, sampler_bwd_gather_kernel<true>, blocks, kGatherThreads, smem, dX, dGrid, X, grid, dY, H, W, C, N, Qo, Ng, chunks, CH);
-    else           vlb::launch(ctx->stream, sampler_bwd_gather_kernel<false>, blocks, kGatherThreads, smem, dX, nullptr, X, grid, dY, H, W, C, N, Qo, Ng, chunks, CH);
+    vlb::launch(ctx->stream, sampler_bwd_gather_kernel, blocks, kGatherThreads, smem, dX, grid, dY, H, W, C, N, Qo, Ng, chunks, CH);
     VLB_LAUNCHED(ctx, 1);
-    if (dGrid && !fusedGrid) {
-      size_t total = (size_t)Qo * Ng;
-      vlb::launch(ctx->stream, sampler_kernel<1>, vlb::grid_for(total, kThreads, ctx->smCount * 32), kThreads, 0, 
-          nullptr, nullptr, dGrid, X, grid, dY, H, W, C, N, Qo, Ng);
+    dX = nullptr;
+    if (!dGrid) return vlb::check_launch(ctx, "vlb_sampler_backward");
+  }
+  if (!dX) {
+    // the grid derivative alone: blocks of at most kGridThreads * kPlaneQ output pixels (each reads the whole image, from L2 all but once)
+    int const parts = vlb::ceil_div(Qo, kGridThreads * kPlaneQ);
+    if (planes_apply(ctx, 2LL * HWi * kGridCh / 4, 2LL * Qo >= HWi, C, (long long)Ng * parts)) {
+      int const QP = vlb::ceil_div(Qo, parts);
+      if (!allow_smem(ctx)) return vlb::check_launch(ctx, "vlb_sampler_backward");
+      vlb::launch(ctx->stream, sampler_grid_planes_kernel, (unsigned)(Ng * parts), kGridThreads, 2 * kGridCh * sizeof(float) * (size_t)HWi, dGrid, X, grid, dY, H, W, C, Qo,
+          Ng / N, parts, QP);
       VLB_LAUNCHED(ctx, 1);
+      return vlb::check_launch(ctx, "vlb_sampler_backward");
     }
-    return vlb::check_launch(ctx, "vlb_sampler_backward");
   }
   if (dX) {
     cudaError_t e = cudaMemsetAsync(dX, 0, sizeof(float) * (size_t)H * W * C * N, ctx->stream);
