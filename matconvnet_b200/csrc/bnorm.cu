@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include <cooperative_groups.h>
 #include <math.h>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -125,14 +126,73 @@ bnorm_reduce_kernel(float* __restrict__ momentsOut,   // 2*C or nullptr
   cluster.sync();   // keep every CTA's shared memory alive until rank 0 has read it
 }
 
+// Position of a thread in its channel's items (float4s or floats: item i is element i % per of image i / per), moved by a fixed stride without
+// dividing.
+struct Walk {
+  size_t off;                        // of the item, in floats
+  size_t stride, wrap;               // of one move, and what is added when that leaves the plane
+  int q, dq, per;
+  __device__ Walk(int first, int step, int per_, int width, int c, int C, int WH) : per(per_)
+  {
+    int const n = first / per;
+    q = first - n * per;
+    off = ((size_t)n * C + c) * (size_t)WH + (size_t)width * q;
+    int const dn = step / per;
+    dq = step - dn * per;
+    stride = (size_t)dn * C * WH + (size_t)width * dq;
+    wrap = (size_t)C * WH - (size_t)width * per;
+  }
+  __device__ __forceinline__ void move()
+  {
+    q += dq; off += stride;
+    if (q >= per) { q -= per; off += wrap; }
+  }
+};
+
+template <int kMode> __device__ __forceinline__ void add_item(float (&acc)[4], float x, float dy)
+{
+  if (kMode == 2) { acc[2] = fmaf(dy, x, acc[2]); acc[3] += dy; }
+  else accumulate<kMode == 0 ? 2 : 4>(acc, x, dy);
+}
+template <int kMode> __device__ __forceinline__ void add_item(float (&acc)[4], float4 x, float4 dy)
+{
+  if (kMode == 2) {
+    acc[2] = fmaf(dy.x, x.x, acc[2]); acc[2] = fmaf(dy.y, x.y, acc[2]);
+    acc[2] = fmaf(dy.z, x.z, acc[2]); acc[2] = fmaf(dy.w, x.w, acc[2]);
+    acc[3] += (dy.x + dy.y) + (dy.z + dy.w);
+  } else {
+    accumulate<kMode == 0 ? 2 : 4>(acc, x.x, dy.x);
+    accumulate<kMode == 0 ? 2 : 4>(acc, x.y, dy.y);
+    accumulate<kMode == 0 ? 2 : 4>(acc, x.z, dy.z);
+    accumulate<kMode == 0 ? 2 : 4>(acc, x.w, dy.w);
+  }
+}
+// kMode 0: k = {mean, G1, b, -}; else {mean, db/m, G1, G2}
+template <int kMode> __device__ __forceinline__ float apply_item(float x, float dy, float4 k, int relu)
+{
+  if (kMode != 0) return __fadd_rn(__fmul_rn(k.z, __fadd_rn(dy, -k.y)), -__fmul_rn(k.w, __fadd_rn(x, -k.x)));
+  float const o = __fadd_rn(__fmul_rn(k.y, __fadd_rn(x, -k.x)), k.z);
+  return relu && !(o > 0.f) ? 0.f : o;
+}
+template <int kMode> __device__ __forceinline__ float4 apply_item(float4 x, float4 dy, float4 k, int relu)
+{
+  return make_float4(apply_item<kMode>(x.x, dy.x, k, relu), apply_item<kMode>(x.y, dy.y, k, relu), apply_item<kMode>(x.z, dy.z, k, relu),
+                     apply_item<kMode>(x.w, dy.w, k, relu));
+}
+
 // One launch for the whole operator: the cluster that reduced a channel also applies it.
 // After the reduction rank 0 derives the channel's coefficients into its shared memory, the other
 // CTAs read them through distributed shared memory, and every CTA sweeps the same items again --
 // they are still in L2 (a channel's x and dy, 8*m bytes, times the clusters in flight), so DRAM sees
-// x and dy once and the result once: 12*m*C bytes backward, 8*m*C forward.
+// x and dy once and the result once: 12*m*C bytes backward, 8*m*C forward.  What binds beside the traffic is the two
+// meetings of a cluster, and the issue of instructions: a block must have enough to do between the meetings, and no item divides.
+// Clusters of eight with a 64-bit division per item: 28 x 28 x 512 x 64 took 70 us forward and 89 us backward, x 32 images 43 and 66, 28 x 28 x 128 x 64
+// 21 and 26; now 60 and 83, 22 and 44, 12 and 18 (at copy speed 31 and 47, 16 and 24, 8 and 12).  Holding the items in registers or shared memory between
+// the two sweeps was slower: it costs the blocks that hide one another's meetings.
+constexpr int kFusedThreads = 256;
 // kMode 0: forward, moments computed.  1: backward, moments computed.  2: backward, moments given.
-template <int kMode, bool kVec>
-__global__ void __cluster_dims__(1, kCluster, 1) __launch_bounds__(kThreads)
+template <int kMode, bool kVec, int kCl>
+__global__ void __cluster_dims__(1, kCl, 1) __launch_bounds__(kFusedThreads)
 bnorm_fused_kernel(float* __restrict__ out,            // y or dx
                    float* __restrict__ momentsOut,     // 2*C or nullptr
                    float* __restrict__ dgOut, float* __restrict__ dbOut,
@@ -145,42 +205,26 @@ bnorm_fused_kernel(float* __restrict__ out,            // y or dx
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float part[4];
   __shared__ float coef[4];
-  __shared__ float warpRed[kThreads / 32][4];
+  __shared__ float warpRed[kFusedThreads / 32][4];
   int const c = blockIdx.x;
   int const rank = (int)cluster.block_rank();   // the cluster spans grid y
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  int const WH4 = WH >> 2;
-  long long const items = kVec ? (long long)N * WH4 : (long long)N * WH;
-  long long const first = (long long)rank * kThreads + threadIdx.x, step = (long long)kCluster * kThreads;
+  using Item = std::conditional_t<kVec, float4, float>;
+  int const per = kVec ? WH >> 2 : WH;                                  // items of a plane
+  int const step = kCl * kFusedThreads, first = rank * kFusedThreads + (int)threadIdx.x;
+  long long const items = (long long)N * per;
+  auto xAt = [&](size_t off) { return *reinterpret_cast<Item const*>(x + off); };
+  auto dyAt = [&](size_t off) { return *reinterpret_cast<Item const*>(dy + off); };
 
+  int const mine = first < items ? (int)((items - first + step - 1) / step) : 0;
+
+  Walk w(first, step, per, kVec ? 4 : 1, c, C, WH);
+  Walk const w0 = w;
 #pragma unroll 8
-  for (long long i = first; i < items; i += step) {
-    if (kVec) {
-      int n = (int)(i / WH4);
-      int q = (int)(i - (long long)n * WH4);
-      size_t off = ((size_t)n * C + c) * (size_t)WH + 4 * (size_t)q;
-      float4 xv = *reinterpret_cast<float4 const*>(x + off);
-      float4 dv = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (kMode != 0) dv = *reinterpret_cast<float4 const*>(dy + off);
-      if (kMode == 2) {
-        acc[2] = fmaf(dv.x, xv.x, acc[2]); acc[2] = fmaf(dv.y, xv.y, acc[2]);
-        acc[2] = fmaf(dv.z, xv.z, acc[2]); acc[2] = fmaf(dv.w, xv.w, acc[2]);
-        acc[3] += (dv.x + dv.y) + (dv.z + dv.w);
-      } else {
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.x, dv.x);
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.y, dv.y);
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.z, dv.z);
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.w, dv.w);
-      }
-    } else {
-      int n = (int)(i / WH);
-      int q = (int)(i - (long long)n * WH);
-      size_t off = ((size_t)n * C + c) * (size_t)WH + q;
-      float xv = x[off];
-      float dv = (kMode != 0) ? dy[off] : 0.f;
-      if (kMode == 2) { acc[2] = fmaf(dv, xv, acc[2]); acc[3] += dv; }
-      else accumulate<kMode == 0 ? 2 : 4>(acc, xv, dv);
-    }
+  for (int u = 0; u < mine; ++u) {
+    Item const d = kMode != 0 ? dyAt(w.off) : Item{};
+    add_item<kMode>(acc, xAt(w.off), d);
+    w.move();
   }
 
 #pragma unroll
@@ -191,21 +235,21 @@ bnorm_fused_kernel(float* __restrict__ out,            // y or dx
   __syncthreads();
   if (threadIdx.x < 4) {
     float s = 0.f;
-    for (int w = 0; w < kThreads / 32; ++w) s += warpRed[w][threadIdx.x];
+    for (int w = 0; w < kFusedThreads / 32; ++w) s += warpRed[w][threadIdx.x];
     part[threadIdx.x] = s;
   }
   cluster.sync();
   // rank 0 gathers the partial sums of all ranks through distributed shared memory -- 32 threads fetch one value each, so that
   // the remote reads are one round trip instead of 32 -- and thread 0 adds them in rank order
-  __shared__ float gath[kCluster][4];
-  if (rank == 0 && threadIdx.x < kCluster * 4) {
+  __shared__ float gath[kCl][4];
+  if (rank == 0 && threadIdx.x < kCl * 4) {
     int const r = threadIdx.x >> 2, j = threadIdx.x & 3;
     gath[r][j] = cluster.map_shared_rank(part, r)[j];
   }
   if (rank == 0) __syncwarp();
   if (rank == 0 && threadIdx.x == 0) {
     float tot[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int r = 0; r < kCluster; ++r)
+    for (int r = 0; r < kCl; ++r)
       for (int j = 0; j < 4; ++j) tot[j] += gath[r][j];
     float const mass = (float)((long long)WH * N);
     float mean, sigma;
@@ -240,46 +284,35 @@ bnorm_fused_kernel(float* __restrict__ out,            // y or dx
   }
   // (rank 0's shared memory has to outlive these reads: the cluster meets once more at the very end, where nobody waits long)
 
+  float4 const k = make_float4(k0, k1, k2, k3);
+  w = w0;
 #pragma unroll 8
-  for (long long i = first; i < items; i += step) {
-    if (kVec) {
-      int n = (int)(i / WH4);
-      int q = (int)(i - (long long)n * WH4);
-      size_t off = ((size_t)n * C + c) * (size_t)WH + 4 * (size_t)q;
-      float4 xv = *reinterpret_cast<float4 const*>(x + off);
-      float4 o;
-      if (kMode == 0) {
-        o.x = __fadd_rn(__fmul_rn(k1, __fadd_rn(xv.x, -k0)), k2);
-        o.y = __fadd_rn(__fmul_rn(k1, __fadd_rn(xv.y, -k0)), k2);
-        o.z = __fadd_rn(__fmul_rn(k1, __fadd_rn(xv.z, -k0)), k2);
-        o.w = __fadd_rn(__fmul_rn(k1, __fadd_rn(xv.w, -k0)), k2);
-        if (relu) { o.x = o.x > 0.f ? o.x : 0.f; o.y = o.y > 0.f ? o.y : 0.f; o.z = o.z > 0.f ? o.z : 0.f; o.w = o.w > 0.f ? o.w : 0.f; }
-      } else {
-        float4 dv = *reinterpret_cast<float4 const*>(dy + off);
-        o.x = __fadd_rn(__fmul_rn(k2, __fadd_rn(dv.x, -k1)), -__fmul_rn(k3, __fadd_rn(xv.x, -k0)));
-        o.y = __fadd_rn(__fmul_rn(k2, __fadd_rn(dv.y, -k1)), -__fmul_rn(k3, __fadd_rn(xv.y, -k0)));
-        o.z = __fadd_rn(__fmul_rn(k2, __fadd_rn(dv.z, -k1)), -__fmul_rn(k3, __fadd_rn(xv.z, -k0)));
-        o.w = __fadd_rn(__fmul_rn(k2, __fadd_rn(dv.w, -k1)), -__fmul_rn(k3, __fadd_rn(xv.w, -k0)));
-      }
-      *reinterpret_cast<float4*>(out + off) = o;
-    } else {
-      int n = (int)(i / WH);
-      int q = (int)(i - (long long)n * WH);
-      size_t off = ((size_t)n * C + c) * (size_t)WH + q;
-      if (kMode == 0) { float o = __fadd_rn(__fmul_rn(k1, __fadd_rn(x[off], -k0)), k2); out[off] = (relu && !(o > 0.f)) ? 0.f : o; }
-      else out[off] = __fadd_rn(__fmul_rn(k2, __fadd_rn(dy[off], -k1)), -__fmul_rn(k3, __fadd_rn(x[off], -k0)));
-    }
+  for (int u = 0; u < mine; ++u) {
+    Item const d = kMode != 0 ? dyAt(w.off) : Item{};
+    *reinterpret_cast<Item*>(out + w.off) = apply_item<kMode>(xAt(w.off), d, k, relu);
+    w.move();
   }
   cluster.sync();   // every CTA has read rank 0's coefficients long ago; rank 0 may exit
 }
 
+// Blocks per channel: as few as give every SM three (of the eight that fit), for every block then has the most to do between the meetings.
 template <int kMode>
 void launch_fused(vlb_ctx* ctx, bool vec, float* out, float* momOut, float* dg, float* db, float const* momIn,
-                  float const* x, float const* dy, float const* g, float const* b, int WH, int C, int N, float eps, int relu = 0)
+                 float const* x, float const* dy, float const* g, float const* b, int WH, int C, int N, float eps, int relu = 0)
 {
-  dim3 grid(C, kCluster);
-  if (vec) vlb::launch(ctx->stream, bnorm_fused_kernel<kMode, true>, grid, kThreads, 0, out, momOut, dg, db, momIn, x, dy, g, b, WH, C, N, eps, relu);
-  else     vlb::launch(ctx->stream, bnorm_fused_kernel<kMode, false>, grid, kThreads, 0, out, momOut, dg, db, momIn, x, dy, g, b, WH, C, N, eps, relu);
+  int cl = 1;
+  while (cl < 8 && (long long)C * cl < 3LL * ctx->smCount) cl *= 2;
+  auto go = [&](auto v, auto n) {
+    vlb::launch(ctx->stream, bnorm_fused_kernel<kMode, decltype(v)::value, decltype(n)::value>, dim3(C, decltype(n)::value), kFusedThreads, 0, out, momOut, dg, db,
+                momIn, x, dy, g, b, WH, C, N, eps, relu);
+  };
+  auto pick = [&](auto v) {
+    if (cl == 1) return go(v, std::integral_constant<int, 1>{});
+    if (cl == 2) return go(v, std::integral_constant<int, 2>{});
+    if (cl == 4) return go(v, std::integral_constant<int, 4>{});
+    return go(v, std::integral_constant<int, 8>{});
+  };
+  if (vec) pick(std::true_type{}); else pick(std::false_type{});
   VLB_LAUNCHED(ctx, 1);
 }
 
