@@ -175,6 +175,25 @@ __device__ inline void block_exclusive_scan(int* v, int n, int* warpSums)
   for (int i = beg; i < end; ++i) { int c = v[i]; v[i] = run; run += c; }
   __syncthreads();
 }
+
+// nc <= 4 planes of HW pixels into shared memory, a pixel's values side by side (planes that do not exist repeat the first); by the whole block, every
+// thread with up to sixteen loads on the way
+__device__ __forceinline__ void stage_planes(float4* xs, float const* x, int HW, int nc)
+{
+  int const T = blockDim.x;
+  int const o1 = nc > 1 ? HW : 0, o2 = nc > 2 ? 2 * HW : 0, o3 = nc > 3 ? 3 * HW : 0;
+  for (int i = threadIdx.x; i < HW; i += 4 * T) {
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float const* const q = x + min(i + k * T, HW - 1);
+      v[k] = make_float4(__ldg(q), __ldg(q + o1), __ldg(q + o2), __ldg(q + o3));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * T < HW) xs[i + k * T] = v[k];
+  }
+}
 }  // namespace vlb
 #endif
 

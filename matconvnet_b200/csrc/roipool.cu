@@ -6,17 +6,16 @@
 // float, float products with floor/ceil (bits/nnroipooling.cu:129-165) -- using the
 // _rn intrinsics so that no multiply-add is contracted; the reference's own GPU code
 // does the same maths in float throughout and can differ in the last place.
-// Forward: one thread per output bin; adjacent threads take adjacent ph, so reads of a bin
-// column are contiguous.  The scan order for the arg-max is the CPU's (w outer, h inner,
-// first strictly greater).
+// Forward: one thread per output bin and four channels, whose planes lie side by side in shared memory; maps too large for that
+// are read from global memory, one thread per output bin and channel.  The scan order for the arg-max is
+// the CPU's (w outer, h inner, first strictly greater).
 //
 // Backward (max) does not scatter with atomics as the reference GPU code does
 // (bits/impl/nnroipooling_gpu.cu:114-246).  One CTA takes one image and a few channels.  All its
 // threads first find, from the input plane in shared memory, the arg-max pixel of every bin of every
 // ROI of the image; then one warp per channel walks the bins in the order of the CPU loop (ROI, bin
 // column, bin row; bits/nnroipooling.cu:239-300), 32 at a time, and adds their derivatives to a copy
-// of the channel's dX plane in shared memory -- lanes whose bins routed to the same pixel one after
-// the other in lane order (__match_any_sync), all others at once.  The work is proportional to the
+// of the channel's dX plane in shared memory, the additions of one step to one pixel in lane order.  The work is proportional to the
 // number of bins, the sums are the CPU's bit for bit and identical from run to run, dX is written
 // exactly once (no zero fill), and nothing but x, dY and dX crosses HBM.  Backward (avg), where every
 // pixel of a bin receives a share, is a gather: every pixel of a channel slab walks the ROIs that
@@ -24,6 +23,7 @@
 // scatter.
 #include "common.cuh"
 #include <math.h>
+#include <algorithm>
 
 namespace {
 
@@ -141,6 +141,88 @@ __global__ void roipool_kernel(float* __restrict__ out, float const* __restrict_
   }
 }
 
+// ---- forward with the planes of four channels in shared memory ----
+// The direct kernel above computes the bin geometry, in double precision, for every channel, and its scans wait for L1 at every pixel.  Here a
+// block takes one image, four channels and up to RB ROIs: the geometry once per ROI into tables, the four planes side by side, and
+// a bin is scanned for four channels at once.  B200, 38 x 50 x 512 x 2, 256 ROIs, 7 x 7 bins: 117 -> 35 us.
+constexpr int kFwdThreads = 256;
+
+__host__ __device__ inline size_t fwd_smem(int RB, long long HW, int S0, int S1)
+{ return sizeof(float4) * (size_t)HW + sizeof(uint32_t) * (size_t)RB * (S0 + S1) + sizeof(int) * (size_t)RB; }
+
+// start | end << 16 of every bin row and bin column of nb ROIs (the double-precision part of the arithmetic, once per ROI)
+__device__ __forceinline__ void bin_tables(uint32_t* binRow, uint32_t* binCol, int const* roiIdx, int nb, float const* rois, RoiParams const& p)
+{
+  for (int i = threadIdx.x; i < nb * (p.S0 + p.S1); i += blockDim.x) {
+    bool const isRow = i < nb * p.S0;
+    int const k = isRow ? i : i - nb * p.S0;
+    int const S = isRow ? p.S0 : p.S1;
+    int const j = k / S, b = k - j * S;
+    RoiGeom g = roi_geom(rois + 5 * (size_t)roiIdx[j], p);
+    int s, e;
+    roi_bin(b, isRow ? g.bin_h : g.bin_w, isRow ? g.start_h : g.start_w, isRow ? p.H : p.W, s, e);
+    (isRow ? binRow : binCol)[k] = (uint32_t)s | ((uint32_t)e << 16);
+  }
+}
+
+template <bool kMax>
+__global__ void __launch_bounds__(kFwdThreads)
+roipool_fwd_planes_kernel(float* __restrict__ y, float const* __restrict__ x, float const* __restrict__ rois, RoiParams p, int RB, int parts, int quads)
+{
+  vlb::pdl_wait();
+  extern __shared__ __align__(16) uint8_t sm[];
+  __shared__ int sCount;
+  int const HW = p.H * p.W, bins = p.S0 * p.S1, tid = threadIdx.x;
+  int const plane = blockIdx.x / parts, part = blockIdx.x - plane * parts;
+  int const img = plane / quads, c0 = (plane - img * quads) * 4, nc = min(4, p.C - c0);
+  float4* const xs = reinterpret_cast<float4*>(sm);
+  uint32_t* const binRow = reinterpret_cast<uint32_t*>(xs + HW);
+  uint32_t* const binCol = binRow + (size_t)RB * p.S0;
+  int* const roiIdx = reinterpret_cast<int*>(binCol + (size_t)RB * p.S1);
+  if (tid == 0) sCount = 0;
+  __syncthreads();
+  // the ROIs of this part that lie on this image, in any order
+  for (int r = part * RB + tid; r < min(p.numROIs, (part + 1) * RB); r += kFwdThreads)
+    if (min(max((int)rois[5 * (size_t)r] - 1, 0), p.N - 1) == img) roiIdx[atomicAdd(&sCount, 1)] = r;
+  __syncthreads();
+  int const nb = sCount;
+  if (nb == 0) return;
+  vlb::stage_planes(xs, x + (size_t)HW * ((size_t)c0 + (size_t)p.C * img), HW, nc);
+  bin_tables(binRow, binCol, roiIdx, nb, rois, p);
+  __syncthreads();
+  float const invBins = 1.f / (float)bins, invS0 = 1.f / (float)p.S0;
+  for (int b = tid; b < nb * bins; b += kFwdThreads) {
+    int const j = (int)(((float)b + 0.5f) * invBins), t = b - j * bins;      // (exact: see the rule in vlb_roipool_forward)
+    int const pw = (int)(((float)t + 0.5f) * invS0), ph = t - pw * p.S0;
+    uint32_t const rs = binRow[j * p.S0 + ph], cs = binCol[j * p.S1 + pw];
+    int const hs = (int)(rs & 0xFFFFu), he = (int)(rs >> 16), ws = (int)(cs & 0xFFFFu), we = (int)(cs >> 16);
+    bool const empty = he <= hs || we <= ws;
+    float const v0 = kMax && !empty ? -INFINITY : 0.f;
+    float4 o = make_float4(v0, v0, v0, v0);
+    for (int w = ws; w < we; ++w) {
+      float4 const* const col = xs + w * p.H;
+#pragma unroll 2
+      for (int h = hs; h < he; ++h) {
+        float4 const a = col[h];
+        if (kMax) {
+          o.x = o.x < a.x ? a.x : o.x; o.y = o.y < a.y ? a.y : o.y; o.z = o.z < a.z ? a.z : o.z; o.w = o.w < a.w ? a.w : o.w;
+        } else {
+          o.x = __fadd_rn(o.x, a.x); o.y = __fadd_rn(o.y, a.y); o.z = __fadd_rn(o.z, a.z); o.w = __fadd_rn(o.w, a.w);
+        }
+      }
+    }
+    if (!kMax && !empty) {
+      float const inv = __fdiv_rn(1.f, (float)((he - hs) * (we - ws)));
+      o.x = __fmul_rn(o.x, inv); o.y = __fmul_rn(o.y, inv); o.z = __fmul_rn(o.z, inv); o.w = __fmul_rn(o.w, inv);
+    }
+    float* const q = y + (size_t)bins * ((size_t)c0 + (size_t)p.C * roiIdx[j]) + t;
+    q[0] = o.x;
+    if (nc > 1) q[bins] = o.y;
+    if (nc > 2) q[2 * bins] = o.z;
+    if (nc > 3) q[3 * bins] = o.w;
+  }
+}
+
 // ---- backward as a gather (see the header comment) ----
 constexpr int kGatherThreads = 1024;
 constexpr uint32_t kNoBin = 0xFFFFu;
@@ -222,17 +304,7 @@ roipool_bwd_gather_kernel(float* __restrict__ dx, float const* __restrict__ x, f
     int const nb = sCount;
     base = sNext;
     if (nb == 0) break;
-    // bin geometry of every ROI of the batch, once (the double-precision part of the arithmetic)
-    for (int i = tid; i < nb * (p.S0 + p.S1); i += kGatherThreads) {
-      bool const isRow = i < nb * p.S0;
-      int const k = isRow ? i : i - nb * p.S0;
-      int const S = isRow ? p.S0 : p.S1;
-      int const j = k / S, b = k - j * S;
-      RoiGeom g = roi_geom(rois + 5 * (size_t)roiIdx[j], p);
-      int s, e;
-      roi_bin(b, isRow ? g.bin_h : g.bin_w, isRow ? g.start_h : g.start_w, isRow ? p.H : p.W, s, e);
-      (isRow ? binRow : binCol)[k] = (uint32_t)s | ((uint32_t)e << 16);
-    }
+    bin_tables(binRow, binCol, roiIdx, nb, rois, p);
     __syncthreads();
     // which bin rows cover map row h, which bin columns cover map column w
     for (int i = tid; i < nb * (p.H + p.W); i += kGatherThreads) {
@@ -325,34 +397,35 @@ roipool_bwd_gather_kernel(float* __restrict__ dx, float const* __restrict__ x, f
   }
 }
 
-// ---- backward (max): arg-max of every bin in parallel, then one warp per channel adds the bins' derivatives to their
-// pixels in bin order (see the header comment) ----
-constexpr int kOrdThreads = 256;
+// ---- backward (max): arg-max of every bin in parallel, four channels at a time, then one warp per channel adds the bins' derivatives to
+// their pixels in bin order (see the header comment) ----
+constexpr int kOrdThreads = 512;
 
-// Shared memory (bytes): plane float[HW] | dxs float[G*HW] | binRow uint32[RB*S0] | binCol uint32[RB*S1] | roiIdx int[RB] |
-// am uint16[G*RB*bins]
-__host__ __device__ inline size_t ordered_smem(int G, int RB, int HW, int S0, int S1)
-{
-  return 4 * (size_t)HW * (1 + G) + 4 * (size_t)RB * (S0 + S1) + 4 * (size_t)RB + 2 * (size_t)G * RB * S0 * S1 + 64;
-}
+// Shared memory (bytes): plane float4[HW] | dxs float[4*HW] | binRow uint32[RB*S0] | binCol uint32[RB*S1] | roiIdx int[RB] |
+// am uint16[4*RB*bins]
+__host__ __device__ inline size_t ordered_smem(int RB, int HW, int S0, int S1)
+{ return 32 * (size_t)HW + 4 * (size_t)RB * (S0 + S1) + 4 * (size_t)RB + 8 * (size_t)RB * S0 * S1 + 64; }
 
+// Bound by latency: the scans of the bins, then the chain of additions.  With one channel at a time and one warp per channel for the additions
+// (38 x 50 x 512 x 2, 256 ROIs, 7 x 7 bins) 190 us; four channels per scan, and a step's additions without
+// a pass through memory for every lane: 124 us.  Two or four warps per channel, each for a part of the pixels, were no faster.
 __global__ void __launch_bounds__(kOrdThreads)
 roipool_bwd_ordered_kernel(float* __restrict__ dx, float const* __restrict__ x, float const* __restrict__ rois,
-                           float const* __restrict__ dy, RoiParams p, int G, int RB, int groups)
+                           float const* __restrict__ dy, RoiParams p, int RB, int quads)
 {
   vlb::pdl_wait();
   extern __shared__ __align__(16) uint8_t sm[];
   __shared__ int sCount, sNext;
   int const HW = p.H * p.W, bins = p.S0 * p.S1;
-  int const img = blockIdx.x / groups, c0 = (blockIdx.x % groups) * G;
-  int const nch = min(G, p.C - c0);
+  int const img = blockIdx.x / quads, c0 = (blockIdx.x % quads) * 4;
+  int const nch = min(4, p.C - c0);
   int const tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float* plane = reinterpret_cast<float*>(sm);
-  float* dxs = plane + HW;
-  uint32_t* binRow = reinterpret_cast<uint32_t*>(dxs + (size_t)G * HW);
-  uint32_t* binCol = binRow + (size_t)RB * p.S0;
-  int* roiIdx = reinterpret_cast<int*>(binCol + (size_t)RB * p.S1);
-  uint16_t* am = reinterpret_cast<uint16_t*>(roiIdx + RB);
+  float4* const plane = reinterpret_cast<float4*>(sm);
+  float* const dxs = reinterpret_cast<float*>(plane + HW);
+  uint32_t* const binRow = reinterpret_cast<uint32_t*>(dxs + 4 * (size_t)HW);
+  uint32_t* const binCol = binRow + (size_t)RB * p.S0;
+  int* const roiIdx = reinterpret_cast<int*>(binCol + (size_t)RB * p.S1);
+  uint16_t* const am = reinterpret_cast<uint16_t*>(roiIdx + RB);
   float const invBins = 1.f / (float)bins, invS0 = 1.f / (float)p.S0;
 
   for (int i = tid; i < nch * HW; i += kOrdThreads) dxs[i] = 0.f;
@@ -386,48 +459,44 @@ roipool_bwd_ordered_kernel(float* __restrict__ dx, float const* __restrict__ x, 
     int const nb = sCount;
     base = sNext;
     if (nb == 0) break;
-    // bin geometry of every ROI of the batch, once (the double-precision part of the arithmetic)
-    for (int i = tid; i < nb * (p.S0 + p.S1); i += kOrdThreads) {
-      bool const isRow = i < nb * p.S0;
-      int const k = isRow ? i : i - nb * p.S0;
-      int const S = isRow ? p.S0 : p.S1;
-      int const j = k / S, b = k - j * S;
-      RoiGeom g = roi_geom(rois + 5 * (size_t)roiIdx[j], p);
-      int s, e;
-      roi_bin(b, isRow ? g.bin_h : g.bin_w, isRow ? g.start_h : g.start_w, isRow ? p.H : p.W, s, e);
-      (isRow ? binRow : binCol)[k] = (uint32_t)s | ((uint32_t)e << 16);
-    }
+    bin_tables(binRow, binCol, roiIdx, nb, rois, p);
+    vlb::stage_planes(plane, x + (size_t)HW * ((size_t)c0 + (size_t)p.C * img), HW, nch);
+    __syncthreads();
     int const total = nb * bins;
-    // arg-max of every bin of every channel of the group, all threads: CPU scan order, first strictly greater, none for
-    // an empty or all -inf / NaN bin
-    for (int cc = 0; cc < nch; ++cc) {
-      __syncthreads();                                 // geometry written; the plane is no longer read
-      float const* const src = x + (size_t)HW * ((size_t)(c0 + cc) + (size_t)p.C * img);
-      for (int i = tid; i < HW; i += kOrdThreads) plane[i] = src[i];
-      __syncthreads();
-      uint16_t* const amc = am + (size_t)cc * RB * bins;
-      for (int b = tid; b < total; b += kOrdThreads) {
-        // quotients by way of a float reciprocal: exact for these small operands, a fraction of the cost of integer division
-        int const j = (int)(((float)b + 0.5f) * invBins), t = b - j * bins;
-        int const pw = (int)(((float)t + 0.5f) * invS0), ph = t - pw * p.S0;
-        uint32_t const rs = binRow[j * p.S0 + ph], cs = binCol[j * p.S1 + pw];
-        int const hs = (int)(rs & 0xFFFFu), he = (int)(rs >> 16), ws = (int)(cs & 0xFFFFu), we = (int)(cs >> 16);
-        float best = -INFINITY;
-        uint32_t where = kNoBin;
-        for (int w = ws; w < we; ++w)
-          for (int h = hs; h < he; ++h) {
-            float a = plane[w * p.H + h];
-            if (a > best) { best = a; where = (uint32_t)(w * p.H + h); }
-          }
-        amc[b] = (uint16_t)where;
-      }
+    // arg-max of every bin, all threads: CPU scan order, first strictly greater, none for an empty or all -inf / NaN bin
+    for (int b = tid; b < total; b += kOrdThreads) {
+      // quotients by way of a float reciprocal: exact for these small operands, a fraction of the cost of integer division
+      int const j = (int)(((float)b + 0.5f) * invBins), t = b - j * bins;
+      int const pw = (int)(((float)t + 0.5f) * invS0), ph = t - pw * p.S0;
+      uint32_t const rs = binRow[j * p.S0 + ph], cs = binCol[j * p.S1 + pw];
+      int const hs = (int)(rs & 0xFFFFu), he = (int)(rs >> 16), ws = (int)(cs & 0xFFFFu), we = (int)(cs >> 16);
+      float4 best = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      uint32_t wx = kNoBin, wy = kNoBin, wz = kNoBin, ww = kNoBin;
+      for (int w = ws; w < we; ++w)
+#pragma unroll 2
+        for (int h = hs; h < he; ++h) {
+          uint32_t const at = (uint32_t)(w * p.H + h);
+          float4 const a = plane[at];
+          if (a.x > best.x) { best.x = a.x; wx = at; }
+          if (a.y > best.y) { best.y = a.y; wy = at; }
+          if (a.z > best.z) { best.z = a.z; wz = at; }
+          if (a.w > best.w) { best.w = a.w; ww = at; }
+        }
+      uint16_t* const o = am + b;
+      size_t const perCh = (size_t)RB * bins;
+      o[0] = (uint16_t)wx; o[perCh] = (uint16_t)wy; o[2 * perCh] = (uint16_t)wz; o[3 * perCh] = (uint16_t)ww;
     }
     __syncthreads();
-    // One warp per channel walks the bins in order -- ROI, bin column, bin row: the order of the CPU loop -- 32 at a time.
-    // Lanes whose bins routed to the same pixel add one after the other, in lane order; all others add at once.
-    for (int cc = warp; cc < nch; cc += kOrdThreads / 32) {
+    // the planes have served: their room holds a word per pixel and channel, in which the lanes of a step meet
+    for (int i = tid; i < HW; i += kOrdThreads) plane[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    // One warp per channel walks the bins in order -- ROI, bin column, bin row: the order of the CPU loop -- 32 at a time.  Among lanes whose
+    // bins routed to the same pixel the first adds up for all, in lane order, and the pixel is read and written once a step.
+    int const cc = warp;
+    if (cc < nch) {
       uint16_t const* const amc = am + (size_t)cc * RB * bins;
       float* const acc = dxs + (size_t)cc * HW;
+      unsigned* const mask = reinterpret_cast<unsigned*>(plane) + (size_t)cc * HW;
       // eight steps' derivatives are fetched together, so that their latency passes once per eight steps
       for (int b0 = 0; b0 < total; b0 += 32 * 8) {
         uint32_t wh[8];
@@ -444,15 +513,26 @@ roipool_bwd_ordered_kernel(float* __restrict__ dx, float const* __restrict__ x, 
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          if (b0 + 32 * u >= total) break;
           uint32_t const where = wh[u];
-          unsigned const peers = __match_any_sync(0xffffffffu, where);
-          int const rank = where != kNoBin ? __popc(peers & ((1u << lane) - 1u)) : -1;
-          int const rounds = __reduce_max_sync(0xffffffffu, rank);
-          for (int r = 0; r <= rounds; ++r) {
-            if (rank == r) acc[where] = __fadd_rn(acc[where], vv[u]);
-            __syncwarp();
+          // the lanes of this step with the same pixel, for the first of them; 0 for the others
+          unsigned m = 0;
+          if (where != kNoBin) atomicOr(mask + where, 1u << lane);
+          __syncwarp();
+          if (where != kNoBin) m = mask[where];
+          if ((m & ((1u << lane) - 1u)) != 0) m = 0;
+          __syncwarp();
+          if (m) mask[where] = 0;
+          int const rounds = __reduce_max_sync(0xffffffffu, __popc(m));
+          if (rounds == 0) continue;
+          bool const first = m != 0;
+          float sum = first ? acc[where] : 0.f;
+          for (int r = 0; r < rounds; ++r) {
+            float const v = __shfl_sync(0xffffffffu, vv[u], m ? __ffs(m) - 1 : 0);
+            if (m) sum = __fadd_rn(sum, v);
+            m &= m - 1;
           }
+          if (first) acc[where] = sum;
+          __syncwarp();
         }
       }
     }
@@ -503,6 +583,30 @@ int vlb_roipool_forward(vlb_ctx* ctx, float* Y, float const* X, float const* roi
   if (rc) return rc;
   VLB_REQUIRE(ctx, Y && X && rois, "roipool_forward: null tensor");
   if (numROIs == 0) return VLB_Success;
+  {
+    // planes in shared memory, where they fit (with room for three blocks per SM, or at least one for large maps) and the quotients by way of a float
+    // reciprocal are exact (fewer than 2^18 bins a block, 2^12 a ROI).  64 ROIs per block pay for the staging of the planes; fewer
+    // where that leaves the chip short of blocks.
+    int const quads = vlb::ceil_div(C, 4);
+    int RB = 64;
+    while (RB > 8 && (long long)N * quads * vlb::ceil_div(numROIs, RB) < 4LL * ctx->smCount) RB /= 2;
+    long long const HW = (long long)H * W, blocks = (long long)N * quads * vlb::ceil_div(numROIs, RB);
+    if (H < 65535 && W < 65535 && HW < (1 << 20) && S0 <= 4096 && S1 <= 4096 && S0 * S1 <= 4096 && fwd_smem(RB, HW, S0, S1) <= 220 * 1024 && blocks < (1LL << 31)) {
+      static bool attrDone[64] = {};
+      if (!(ctx->device < 64 && attrDone[ctx->device])) {
+        cudaError_t ea = vlb::allow_max_dynamic_smem(roipool_fwd_planes_kernel<true>);
+        if (ea == cudaSuccess) ea = vlb::allow_max_dynamic_smem(roipool_fwd_planes_kernel<false>);
+        if (ea != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(ea)); }
+        if (ctx->device < 64) attrDone[ctx->device] = true;
+      }
+      size_t const smem = fwd_smem(RB, HW, S0, S1);
+      int const parts = vlb::ceil_div(numROIs, RB);
+      if (method == VLB_POOL_MAX) vlb::launch(ctx->stream, roipool_fwd_planes_kernel<true>, (unsigned)blocks, kFwdThreads, smem, Y, X, rois, p, RB, parts, quads);
+      else                        vlb::launch(ctx->stream, roipool_fwd_planes_kernel<false>, (unsigned)blocks, kFwdThreads, smem, Y, X, rois, p, RB, parts, quads);
+      VLB_LAUNCHED(ctx, 1);
+      return vlb::check_launch(ctx, "vlb_roipool_forward");
+    }
+  }
   size_t total = (size_t)S0 * S1 * C * numROIs;
   unsigned grid = vlb::grid_for(total, kThreads, ctx->smCount * 16);
   if (method == VLB_POOL_MAX) vlb::launch(ctx->stream, roipool_kernel<true, false>, grid, kThreads, 0, Y, X, rois, nullptr, p);
@@ -526,27 +630,21 @@ int vlb_roipool_backward(vlb_ctx* ctx, float* dX, float const* X, float const* r
     long long const HW = (long long)H * W;
     size_t const budget = 200 * 1024;
     if (isMax && HW < 65535 && S0 <= 255 && S1 <= 255 && numROIs > 0) {
-      // channel groups so that about four CTAs come to every SM; as many ROIs per batch as the rest of 56 KB of shared
-      // memory per CTA holds (four CTAs resident per SM)
-      long long const planes = (long long)N * C;
-      int G = (int)((planes + 4LL * ctx->smCount - 1) / (4LL * ctx->smCount));
-      if (G < 1) G = 1;
-      if (G > kOrdThreads / 32) G = kOrdThreads / 32;
-      if (G > C) G = C;
-      size_t const budget = 56 * 1024;
-      size_t const fixed = ordered_smem(G, 0, (int)HW, S0, S1), perRoi = ordered_smem(G, 1, (int)HW, S0, S1) - fixed;
-      long long RB = fixed < budget ? (long long)((budget - fixed) / perRoi) : 0;
-      if (RB > numROIs) RB = numROIs;
-      if (RB >= 8 || RB == numROIs) {
-        int const groups = vlb::ceil_div(C, G);
-        size_t const smem = ordered_smem(G, (int)RB, (int)HW, S0, S1);
+      // as many ROIs per batch as shared memory holds: two blocks per SM where that leaves room for 64 or for all, else one
+      int const quads = vlb::ceil_div(C, 4);
+      size_t const fixed = ordered_smem(0, (int)HW, S0, S1), perRoi = ordered_smem(1, (int)HW, S0, S1) - fixed;
+      auto fit = [&](size_t budget) { return fixed < budget ? std::min<long long>((long long)((budget - fixed) / perRoi), numROIs) : 0LL; };
+      long long RB = fit(112 * 1024);
+      if (RB < 64 && RB < numROIs) RB = fit(224 * 1024);
+      if ((RB >= 8 || RB == numROIs) && (long long)S0 * S1 <= 4096) {
+        size_t const smem = ordered_smem((int)RB, (int)HW, S0, S1);
         static bool attrDone[64] = {};
         if (!(ctx->device < 64 && attrDone[ctx->device])) {
           cudaError_t ea = vlb::allow_max_dynamic_smem(roipool_bwd_ordered_kernel);
           if (ea != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(ea)); }
           if (ctx->device < 64) attrDone[ctx->device] = true;
         }
-        vlb::launch(ctx->stream, roipool_bwd_ordered_kernel, (unsigned)(N * groups), kOrdThreads, smem, dX, X, rois, dY, p, G, (int)RB, groups);
+        vlb::launch(ctx->stream, roipool_bwd_ordered_kernel, (unsigned)(N * quads), kOrdThreads, smem, dX, X, rois, dY, p, (int)RB, quads);
         VLB_LAUNCHED(ctx, 1);
         return vlb::check_launch(ctx, "vlb_roipool_backward");
       }

@@ -196,24 +196,6 @@ __device__ __forceinline__ void stage_plane(float* dst, float const* src, int n)
   }
 }
 
-// n pixels of nc <= 4 planes (HW apart) into xs; every thread has up to sixteen loads on the way
-__device__ __forceinline__ void stage_planes(float4* xs, float const* x, int HW, int nc)
-{
-  int const T = blockDim.x;
-  int const o1 = nc > 1 ? HW : 0, o2 = nc > 2 ? 2 * HW : 0, o3 = nc > 3 ? 3 * HW : 0;
-  for (int i = threadIdx.x; i < HW; i += 4 * T) {
-    float4 v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float const* const q = x + min(i + k * T, HW - 1);
-      v[k] = make_float4(__ldg(q), __ldg(q + o1), __ldg(q + o2), __ldg(q + o3));
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (i + k * T < HW) xs[i + k * T] = v[k];
-  }
-}
-
 __device__ __forceinline__ void add_tap(float4& a, float w, float4 v)
 {
   a.x = __fadd_rn(a.x, __fmul_rn(w, v.x)); a.y = __fadd_rn(a.y, __fmul_rn(w, v.y));
@@ -228,7 +210,7 @@ sampler_fwd_planes_kernel(float* __restrict__ y, float const* __restrict__ x, fl
   vlb::pdl_wait();
   extern __shared__ float4 xs[];
   int const img = blockIdx.x / quads, c0 = (blockIdx.x - img * quads) * 4, nc = min(4, C - c0), HW = H * W;
-  stage_planes(xs, x + (size_t)HW * ((size_t)C * img + c0), HW, nc);
+  vlb::stage_planes(xs, x + (size_t)HW * ((size_t)C * img + c0), HW, nc);
   __syncthreads();
   for (int gi = 0; gi < group; ++gi) {
     int const n = img * group + gi;
