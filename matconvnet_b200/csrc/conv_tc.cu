@@ -2711,11 +2711,13 @@ ConvGeom plane_geom(int pixels, int channels, int filters)
 //   forward   Y(K x N) = F'(K x V) X(V x N): rows = filters, the reduction index v is contiguous in a row -> row mode, X as tile images;
 //   data      dX(V x N) = F(V x K) dY(K x N): a 1 x 1 convolution over the "plane" of V elements with K channels, dY as its N filters;
 //   weights   dF(V x K) = X(V x N) dY'(N x K): a 1 x 1 convolution over the plane X (N channels) with the K rows of dY as filters.
-// Each returns -1 when the shape is not eligible (the caller then takes tc_gemm_kernel).
+// Each returns -1 when the shape is not eligible (the caller then takes tc_gemm_kernel): rows that are not whole 16-byte pieces, or so little work
+// that the tiles of the second operand are not worth laying out.  V = K = 4096, layout included: forward 107 -> 56 us with 256 images, 56 -> 53 with
+// 128, 50 -> 54 with 64; weights 121 -> 70, 72 -> 45 and 54 -> 41, but K = 1000 with 64 images 17 -> 19.
 int fc_fprop_ts(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float const* F, float const* b)
 {
   int const V = g.FH * g.FW * g.FC;
-  if ((ctx->testSwitch & 4) || V % 32 != 0 || V < 128 * 64 || g.K % 128 != 0 || g.N > 4096 || !aligned16(X) || !aligned16(F)) return -1;
+  if ((ctx->testSwitch & 4) || V % 32 != 0 || V < (g.N > 128 ? 128 * 16 : 128 * 64) || g.K % 128 != 0 || g.N > 4096 || !aligned16(X) || !aligned16(F)) return -1;
   Params p = {};
   p.cPer = 128; p.tapsPerTile = 1; p.tapGroups = 1;
   p.M = g.K; p.N = g.N; p.R = V;
@@ -2777,7 +2779,8 @@ int fc_dgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, floa
 int fc_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, float const* dY)
 {
   int const V = g.FH * g.FW * g.FC;
-  if ((ctx->testSwitch & 4) || V % 4 != 0 || g.N % 32 != 0 || !aligned16(X) || !aligned16(dY) || V < 128 * 64) return -1;
+  if ((ctx->testSwitch & 4) || V % 4 != 0 || g.N % 32 != 0 || !aligned16(X) || !aligned16(dY) || V < 128 * 16) return -1;
+  if (V < 128 * 64 && (long long)V * g.K < (1 << 23)) return -1;
   Params p = {};
   p.M = V; p.N = g.K; p.R = g.N;
   ConvGeom const t = plane_geom(V, g.N, g.K);
@@ -3163,9 +3166,23 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     p.a = Operand{}; p.a.ptr = F; p.a.ld = V; p.a.rows = V; p.a.vec = (V % 4 == 0) && aligned16(F);
     p.b = Operand{}; p.b.ptr = dY; p.b.ld = g.K; p.b.rows = g.N; p.b.vec = (g.K % 4 == 0) && aligned16(dY);
     p.BN = pick_bn(p.N);
-    p.numKb = ceil_div(p.R, BK); p.kbPerSplit = p.numKb;
+    // few output tiles: the reduction in parts, as in the forward pass (V = 4096, K = 1000, N = 128: 49 -> 22 us)
+    p.numKb = ceil_div(p.R, BK);
+    int const tiles = ceil_div(p.M, BM) * ceil_div(p.N, p.BN);
+    int splits = pick_splits(ctx, tiles, p.numKb, 8);
+    p.kbPerSplit = ceil_div(p.numKb, splits);
+    splits = ceil_div(p.numKb, p.kbPerSplit);
     p.e = Epilogue{}; p.e.out = dX; p.e.ldd = V;
-    return launch_gemm<OP_DENSE_MN, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "fc_dgrad_tc");
+    if (splits == 1) return launch_gemm<OP_DENSE_MN, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "fc_dgrad_tc");
+    size_t const nOut = (size_t)V * g.N;
+    float* const part = (float*)workspace(ctx, sizeof(float) * nOut * splits);
+    if (!part) return ctx->lastError;
+    p.e.out = part; p.e.splitStride = (long long)nOut;
+    int const rc = launch_gemm<OP_DENSE_MN, OP_DENSE_K, EPI_PLAIN>(ctx, p, splits, "fc_dgrad_tc");
+    if (rc) return rc;
+    SumEpilogue epi;
+    epi.mask = ctx->reluMask; ctx->maskDone = ctx->reluMask != nullptr;
+    return sum_parts(ctx, dX, part, nOut, nOut, splits, epi);
   }
   if (g.G != 1 || g.sy != 1 || g.sx != 1 || g.K % 32 != 0 || g.FH * g.FW > 64) {
     ProfScope prof(ctx, kProfDgrad);

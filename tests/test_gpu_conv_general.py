@@ -66,6 +66,8 @@ FEW = {
     "fc_n1": ((7, 7, 64, 1), (7, 7, 64, 130), 0), "fc_n3_ragged": ((5, 3, 23, 3), (5, 3, 23, 1201), 0), "fc_n8": ((1, 1, 512, 8), (1, 1, 512, 67), 0),
     "few_tiles_plain": ((14, 14, 256, 1), (3, 3, 256, 160), 1), "few_tiles_windows": ((32, 16, 64, 1), (5, 5, 64, 48), 2),
     "few_tiles_general": ((8, 8, 50, 5), (5, 5, 50, 70), 0),
+    "fc_n130_16_row_tiles": ((4, 4, 128, 130), (4, 4, 128, 4096), 0), "fc_below_the_line": ((4, 4, 128, 128), (4, 4, 128, 128), 0),
+    "fc_dgrad_parts": ((1, 1, 300, 33), (1, 1, 300, 1000), 0),
 }
 
 
