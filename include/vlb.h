@@ -285,6 +285,10 @@ int vlb_lrn_forward(vlb_ctx* ctx, float* Y, float const* X, int H, int W, int C,
                     double alpha, double beta);
 int vlb_lrn_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, int H, int W, int C, int N, int normDepth,
                      double kappa, double alpha, double beta);
+/* The same and the ReLU before it in one call, for an X that is the output of a ReLU: bit-identical to vlb_lrn_backward followed by
+ * vlb_relu_backward(dX, X, dX). */
+int vlb_relu_lrn_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, int H, int W, int C, int N, int normDepth,
+                          double kappa, double alpha, double beta);
 /* matlab/vl_nnsoftmax.m: softmax over the channels; backward takes X (not Y), as the MATLAB function does. */
 int vlb_softmax_forward(vlb_ctx* ctx, float* Y, float const* X, int H, int W, int C, int N);
 int vlb_softmax_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, int H, int W, int C, int N);

@@ -115,6 +115,7 @@ SIGNATURES = {
     "vlb_sgd_update": (_I, [_P, _P, _P, _P, _Z, _D, _D, _D, _D, _I]),
     "vlb_lrn_forward": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _D, _D, _D]),
     "vlb_lrn_backward": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _D, _D, _D]),
+    "vlb_relu_lrn_backward": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _D, _D, _D]),
     "vlb_softmax_forward": (_I, [_P, _P, _P, _I, _I, _I, _I]),
     "vlb_softmax_backward": (_I, [_P, _P, _P, _P, _I, _I, _I, _I]),
     "vlb_dropout_mask": (_I, [_P, _P, _Z, _D, C.c_ulonglong]),

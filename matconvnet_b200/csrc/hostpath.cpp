@@ -439,10 +439,10 @@ PyObject* relu(PyObject*, Args a, Py_ssize_t n)
   });
 }
 
-// ---------------------------------------------------------------- vl_nnnormalize: ctx, x, dzdy, depth, kappa, alpha, beta
+// ---------------------------------------------------------------- vl_nnnormalize: ctx, x, dzdy, depth, kappa, alpha, beta, through_relu
 PyObject* normalize(PyObject*, Args a, Py_ssize_t n)
 {
-  return guarded(n, 7, [&]() -> PyObject* {
+  return guarded(n, 8, [&]() -> PyObject* {
     Ctx ctx(a[0]);
     at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy");
     Shape const s = shape4(x);
@@ -451,7 +451,7 @@ PyObject* normalize(PyObject*, Args a, Py_ssize_t n)
     if (dzdy.defined() && !same4(shape4(dzdy), H, W, C, N)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X.");
     at::Tensor out = empty4(s, x.device());
     if (!dzdy.defined()) ctx.check(vlb_lrn_forward(ctx.h, ptr(out), ptr(x), H, W, C, N, depth, kappa, alpha, beta));
-    else                 ctx.check(vlb_lrn_backward(ctx.h, ptr(out), ptr(x), ptr(dzdy), H, W, C, N, depth, kappa, alpha, beta));
+    else                 ctx.check((as_bool(a[7]) ? vlb_relu_lrn_backward : vlb_lrn_backward)(ctx.h, ptr(out), ptr(x), ptr(dzdy), H, W, C, N, depth, kappa, alpha, beta));
     return wrap(out);
   });
 }

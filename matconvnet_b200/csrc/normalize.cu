@@ -17,7 +17,11 @@ namespace {
 
 constexpr int kThreads = 256;
 
-struct LrnParams { int P, C, N, m1, m2; float kappa, alpha, beta; };
+struct LrnParams {
+  int P, C, N, m1, m2;
+  float kappa, alpha, beta;
+  int relu;            // backward: X is the output of a ReLU, dX is zero where it is not positive
+};
 
 __global__ void lrn_forward_kernel(float* __restrict__ y, float const* __restrict__ x, LrnParams p)
 {
@@ -68,7 +72,8 @@ __global__ void lrn_backward_kernel(float* __restrict__ dx, float* __restrict__ 
       int const q1 = t - p.m2 - 1, q2 = min(t + p.m1, p.C - 1);
       float s = ip[(size_t)p.P * q2];
       if (q1 >= 0) s -= ip[(size_t)p.P * q1];
-      dp[(size_t)p.P * t] -= s * xp[(size_t)p.P * t];
+      float const xt = xp[(size_t)p.P * t], d = dp[(size_t)p.P * t] - s * xt;
+      dp[(size_t)p.P * t] = p.relu && !(xt > 0.f) ? 0.f : d;
     }
   }
 }
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(128) lrn_backward_window_kernel(float* __restr
       float s = 0.f;
 #pragma unroll
       for (int k = 0; k < kD; ++k) s += b[k];
-      dp[(size_t)p.P * o] = a[0] - s * r[0];
+      dp[(size_t)p.P * o] = p.relu && !(r[0] > 0.f) ? 0.f : a[0] - s * r[0];
     }
   }
 }
@@ -285,6 +290,7 @@ int lrn_params(vlb_ctx* ctx, LrnParams* p, int H, int W, int C, int N, int normD
   VLB_REQUIRE(ctx, normDepth >= 1, "normalize: the normalisation depth is smaller than 1");       // matlab/src/vl_nnnormalize.cu:128-130
   p->P = H * W; p->C = C; p->N = N;
   p->m1 = (normDepth - 1) / 2; p->m2 = normDepth - p->m1 - 1;
+  p->relu = 0;
   p->kappa = (float)kappa; p->alpha = (float)alpha; p->beta = (float)beta;
   return VLB_Success;
 }
@@ -307,21 +313,30 @@ int vlb_lrn_forward(vlb_ctx* ctx, float* Y, float const* X, int H, int W, int C,
   return vlb::check_launch(ctx, "vlb_lrn_forward");
 }
 
-int vlb_lrn_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, int H, int W, int C, int N, int normDepth,
-                     double kappa, double alpha, double beta)
+static int lrn_backward_common(vlb_ctx* ctx, float* dX, float const* X, float const* dY, int H, int W, int C, int N, int normDepth,
+                               double kappa, double alpha, double beta, int relu, char const* where)
 {
   if (!ctx) return VLB_IllegalArgument;
   LrnParams p;
   int rc = lrn_params(ctx, &p, H, W, C, N, normDepth, kappa, alpha, beta);
   if (rc) return rc;
+  p.relu = relu;
   VLB_REQUIRE(ctx, dX && X && dY, "lrn_backward: null tensor");
-  if (launch_lrn_window<true>(ctx, dX, X, dY, p, normDepth)) return vlb::check_launch(ctx, "vlb_lrn_backward");
+  if (launch_lrn_window<true>(ctx, dX, X, dY, p, normDepth)) return vlb::check_launch(ctx, where);
   float* integral = (float*)vlb::workspace(ctx, sizeof(float) * (size_t)p.P * C * N);
-  if (!integral) return vlb::pass_error(ctx, ctx->lastError, "vlb_lrn_backward");
+  if (!integral) return vlb::pass_error(ctx, ctx->lastError, where);
   vlb::launch(ctx->stream, lrn_backward_kernel, vlb::grid_for((size_t)p.P * N, kThreads, ctx->smCount * 8), kThreads, 0, dX, integral, X, dY, p);
   VLB_LAUNCHED(ctx, 1);
-  return vlb::check_launch(ctx, "vlb_lrn_backward");
+  return vlb::check_launch(ctx, where);
 }
+
+int vlb_lrn_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, int H, int W, int C, int N, int normDepth,
+                     double kappa, double alpha, double beta)
+{ return lrn_backward_common(ctx, dX, X, dY, H, W, C, N, normDepth, kappa, alpha, beta, 0, "vlb_lrn_backward"); }
+
+int vlb_relu_lrn_backward(vlb_ctx* ctx, float* dX, float const* X, float const* dY, int H, int W, int C, int N, int normDepth,
+                          double kappa, double alpha, double beta)
+{ return lrn_backward_common(ctx, dX, X, dY, H, W, C, N, normDepth, kappa, alpha, beta, 1, "vlb_relu_lrn_backward"); }
 
 int vlb_softmax_forward(vlb_ctx* ctx, float* Y, float const* X, int H, int W, int C, int N)
 {

@@ -220,9 +220,10 @@ def vl_nnrelu(x, dzdy=None, ctx=None):
     return _hostpath.relu(ctx or default_context(), x, dzdy)
 
 
-def vl_nnnormalize(x, param, dzdy=None, ctx=None):
+def vl_nnnormalize(x, param, dzdy=None, ctx=None, through_relu=False):
     """Y = VL_NNNORMALIZE(X, PARAM) / DZDX = VL_NNNORMALIZE(X, PARAM, DZDY), PARAM = [N KAPPA ALPHA BETA]
-    (matlab/vl_nnnormalize.m; gateway matlab/src/vl_nnnormalize.cu:117-162)."""
+    (matlab/vl_nnnormalize.m; gateway matlab/src/vl_nnnormalize.cu:117-162).  through_relu=True (backward only) is for an X that
+    is the output of a ReLU: DZDX is then the derivative with respect to that ReLU's input."""
     if not (isinstance(param, (list, tuple)) and len(param) == 4):
         param = np.asarray(param, dtype=np.float64).ravel()
         if len(param) != 4:
@@ -230,7 +231,7 @@ def vl_nnnormalize(x, param, dzdy=None, ctx=None):
     depth = int(param[0])
     if depth < 1:
         raise ValueError("The normalization depth is smaller than 1.")
-    return _hostpath.normalize(ctx or default_context(), x, dzdy, depth, float(param[1]), float(param[2]), float(param[3]))
+    return _hostpath.normalize(ctx or default_context(), x, dzdy, depth, float(param[1]), float(param[2]), float(param[3]), through_relu)
 
 
 def vl_nnsoftmax(x, dzdy=None, ctx=None):

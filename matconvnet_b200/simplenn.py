@@ -103,10 +103,10 @@ def vl_simplenn(net, x, dzdy=None, res=None, on_dzdw=None, ctx=None, skip_forwar
         l = layers[i]
         t = l["type"]
         xi, d = res[i]["x"], res[i + 1]["dzdx"]
-        # fuse_relu: the backward pass of a ReLU directly before a convolution or pooling layer is done by that layer's
+        # fuse_relu: the backward pass of a ReLU directly before a convolution, pooling or normalisation layer is done by that layer's
         # own data-gradient kernel, which zeroes the derivative where its input (the ReLU's output) is not positive; the
         # derivative between the two layers is never stored, as when the reference conserves memory (vl_simplenn.m:512-514)
-        through = fuse_relu and t in ("conv", "pool") and i - 1 >= first and layers[i - 1]["type"] == "relu"
+        through = fuse_relu and t in ("conv", "pool", "normalize") and i - 1 >= first and layers[i - 1]["type"] == "relu"
         if t == "conv":
             dx, df, db = nn.vl_nnconv(xi, l["weights"][0], l["weights"][1], d, stride=_get(l, "stride", 1),
                                       pad=_get(l, "pad", 0), dilate=_get(l, "dilate", 1), through_relu=through,
@@ -131,7 +131,8 @@ def vl_simplenn(net, x, dzdy=None, res=None, on_dzdw=None, ctx=None, skip_forwar
         elif t == "softmaxloss":
             res[i]["dzdx"] = nn.vl_nnsoftmaxloss(xi, l["class"], d, ctx=ctx)
         elif t == "normalize":
-            res[i]["dzdx"] = nn.vl_nnnormalize(xi, l["param"], d, ctx=ctx)
+            dx = nn.vl_nnnormalize(xi, l["param"], d, ctx=ctx, through_relu=through)
+            res[i]["dzdx"], res[i - 1 if through else i]["dzdx"] = None, dx
         elif t == "softmax":
             res[i]["dzdx"] = nn.vl_nnsoftmax(xi, d, ctx=ctx)
         elif t == "dropout":

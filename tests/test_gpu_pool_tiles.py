@@ -49,4 +49,6 @@ def test_lrn_windows_vs_oracle(gpu, oracle, shape, prm):
     dx = oracle.lrn_backward(x.astype(np.float64), prm, dy.astype(np.float64))
     xd = mat.from_numpy(x)
     assert rel_l2(mat.to_numpy(nn.vl_nnnormalize(xd, prm)), y) < 1e-6
-    assert rel_l2(mat.to_numpy(nn.vl_nnnormalize(xd, prm, mat.from_numpy(dy))), dx) < 1e-6
+    got = mat.to_numpy(nn.vl_nnnormalize(xd, prm, mat.from_numpy(dy)))
+    assert rel_l2(got, dx) < 1e-6
+    assert bit_equal(mat.to_numpy(nn.vl_nnnormalize(xd, prm, mat.from_numpy(dy), through_relu=True)), np.where(x > 0, got, np.float32(0)))
