@@ -1,6 +1,6 @@
-// CUDA-core implicit-GEMM convolution: the exact-fp32 path (VLB_PRECISION_FP32) and the path
-// for every stride / dilation / padding / group configuration of vl::nn::Convolution
-// (reference bits/nnconv.cu:71-317) that the tensor-core kernels do not cover.
+// CUDA-core implicit-GEMM convolution: the exact-fp32 path (VLB_PRECISION_FP32), and what little of
+// vl::nn::Convolution (reference bits/nnconv.cu:71-317) the tensor-core kernels leave: filter groups of fewer than
+// four channels, strided filters of more than 128 taps, more than 16 residue classes of a strided data gradient.
 //
 // No patch matrix is ever written (the reference builds one per image, bits/nnconv.cu:
 // 109-117,283-291): operands are gathered straight from the tensors with the index algebra

@@ -4,10 +4,12 @@
 // Every contraction on the path is D[m][n] = sum_r A(m,r) * B(n,r) with fp32 accumulation
 // in tensor memory, 128 x BN output tile, reduction in blocks of 32.  Two kernels:
 //
-//   conv_ts_kernel   convolution forward and stride-1 data gradient: the gathered operand goes to
-//                    tensor memory, only the filter tiles to shared memory (further down).
-//   tc_gemm_kernel   filter gradient, fully connected layers, and convolutions whose filter support
-//                    exceeds the tap table: both operands in shared memory, warp-specialised:
+//   conv_ts_kernel   convolution forward and data gradient, the filter gradient and fully connected layers where the
+//                    reduction runs along memory: the gathered operand goes to tensor memory, only the filter tiles to
+//                    shared memory (further down).  conv_ts_gen_kernel is the same body for any stride, dilation,
+//                    channel count and filter groups.
+//   tc_gemm_kernel   the other filter gradients and fully connected layers, and convolutions whose filter support
+//                    exceeds the tap tables: both operands in shared memory, warp-specialised:
 //     warps 0-3   fp32 drain of the accumulation chains, then epilogue: tcgen05.ld the accumulator
 //                 (one TMEM lane = one output row per thread), store to global memory, coalesced along m;
 //     warp  4     allocates TMEM and issues tcgen05.mma (kind::tf32, cta_group::1) from one
@@ -77,7 +79,7 @@ struct Operand {
   int P;               // run length of contiguous reduction indices (DENSE_K, batched); 0 = unbatched
   int rows;            // valid extent of the row (M or N) index
   int vec;             // 1 when 16-byte loads are legal for this operand
-  int fast;            // pipelined gather: 1 aligned windows, 2 element-wise (any geometry), 0 none (IM2COL, WGATHER)
+  int fast;            // gather by tap tables: 1 aligned windows, 2 element-wise (any geometry), 0 filter too large for the tables (IM2COL, WGATHER)
   // convolution geometry (IM2COL, WGATHER)
   int H, W, C, FH, FW, Ho, Wo, sy, sx, pt, pl, dy, dx;
   long long imgStride;   // H*W*Ctotal
@@ -104,7 +106,6 @@ struct Params {
   int drainEvery;         // 3xTF32: k-blocks per tensor-core accumulation chain
   int tilesM, tilesN;     // conv_ts_kernel: the grid of output tiles its persistent CTAs walk
   int chanFast;           // conv_ts_kernel: reduction in blocks of 32 channels, r = c%32 + 32*(tap + taps*(c/32)); needs C % 32 == 0
-  int pipelined;          // 1: producers prefetch one stage ahead in registers (aligned gathers only)
   float const* bTiles;    // when non-null: B pre-split into shared-memory tile images, fetched with bulk copies
   int* status;
   int testSwitch;         // vlb_ctx_set_test_switch: bit 0 = conv_ts_kernel's filter-tile loader stays idle
@@ -165,24 +166,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
   }
 }
 
-// One try_wait: true when the phase has completed; otherwise the thread was suspended for about `ns` nanoseconds at most.
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity, uint32_t ns)
-{
-  uint32_t ok;
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-               : "=r"(ok) : "r"(bar), "r"(parity), "r"(ns) : "memory");
-  return ok != 0;
-}
-
-// Has the phase completed?  No waiting.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity)
-{
-  uint32_t ok;
-  asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return ok != 0;
-}
-
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
 { asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
 
@@ -230,15 +213,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, uint32_t const (&r)[16
                  "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
-{
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 // Shared-memory matrix descriptor (sm_100 format): start address, LBO, SBO in 16-byte
 // units, version 1 at bit 46, layout type at bits 61-63: 2 = 128-byte swizzle (K-major tiles),
@@ -353,7 +327,7 @@ __device__ __forceinline__ void load_im2col(Operand const& o, PixCtx const (&px)
   }
 }
 
-// Filter-tap context of one row (fh,fw,c), fixed for a producer thread in WGATHER mode.
+// Filter tap and channel of one row (fh,fw,c) in WGATHER mode.
 struct TapCtx { int dh, dw; long long coff; bool valid; };
 
 __device__ __forceinline__ TapCtx tap_ctx(Operand const& o, int i)
@@ -366,25 +340,10 @@ __device__ __forceinline__ TapCtx tap_ctx(Operand const& o, int i)
   return c;
 }
 
-__device__ __forceinline__ void load_wgather(Operand const& o, TapCtx const& tc, int r, int R, float (&v)[4])
-{
-  v[0] = v[1] = v[2] = v[3] = 0.f;
-  if (!tc.valid || r >= R) return;
-  int ho = r % o.Ho, t = r / o.Ho, wo = t % o.Wo, n = t / o.Wo;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    if (r + e < R) {
-      int h = ho * o.sy + tc.dh, w = wo * o.sx + tc.dw;
-      if (h >= 0 && h < o.H && w >= 0 && w < o.W) v[e] = o.ptr[(long long)n * o.imgStride + tc.coff + (long long)w * o.H + h];
-    }
-    if (++ho == o.Ho) { ho = 0; if (++wo == o.Wo) { wo = 0; ++n; } }
-  }
-}
-
 // ---- fast gathers.  Preconditions (Operand::fast): stride 1, H % 4 == 0, Ho % 4 == 0, base 16-byte
 // aligned, fewer than 2^31 elements.  Then four consecutive output pixels lie in one column, and
-// every 16-byte-aligned group of four input rows is wholly inside the image or wholly padding, so a
-// shifted window of four rows is two aligned 128-bit loads and a funnel shift.
+// every 16-byte-aligned group of four input rows is wholly inside the image or wholly padding, so that
+// two tests serve a shifted window of four rows.
 struct FastPix { int base, ho0, wo; bool valid; };   // base = image*imgStride + wo*H + ho0, in elements
 
 __device__ __forceinline__ FastPix fast_pix(Operand const& o, int m, int limit)
@@ -396,23 +355,6 @@ __device__ __forceinline__ FastPix fast_pix(Operand const& o, int m, int limit)
   c.ho0 = ho;
   c.base = (t / o.Wo) * (int)o.imgStride + c.wo * o.H + ho;
   return c;
-}
-
-// v[e] = x[row ho0 + s + e, column wo + dw, plane offset coff] (zero outside the image), e = 0..3
-__device__ __forceinline__ void load_shifted(float const* __restrict__ ptr, int H, int W, FastPix const& px, int s, int dw,
-                                             int coff, bool on, float (&v)[4])
-{
-  int const o = s & 3;
-  int const h0 = px.ho0 + s - o;
-  int const w = px.wo + dw;
-  bool const wok = on && px.valid && w >= 0 && w < W;
-  float const* a0 = ptr + (px.base + coff + dw * H + (s - o));
-  float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
-  if (wok && h0 >= 0 && h0 < H) c0 = *reinterpret_cast<float4 const*>(a0);
-  if (wok && o != 0 && h0 + 4 >= 0 && h0 + 4 < H) c1 = *reinterpret_cast<float4 const*>(a0 + 4);
-  bool const s2 = (o & 2) != 0, s1 = (o & 1) != 0;
-  float t0 = s2 ? c0.z : c0.x, t1 = s2 ? c0.w : c0.y, t2 = s2 ? c1.x : c0.z, t3 = s2 ? c1.y : c0.w, t4 = s2 ? c1.z : c1.x;
-  v[0] = s1 ? t1 : t0; v[1] = s1 ? t2 : t1; v[2] = s1 ? t3 : t2; v[3] = s1 ? t4 : t3;
 }
 
 // One row of a reduction-contiguous operand whose 16-byte loads are legal: p points at (row, batch) start.
@@ -430,8 +372,8 @@ __device__ __forceinline__ void load_row4(float const* __restrict__ p, int r, in
   }
 }
 
-// ------------------------------------------------------------------ pipelined producer
-// Pipelined producers work in kGroups independent groups of warps; group g fills the stages
+// ------------------------------------------------------------------ producers of the filter gradient (WGATHER)
+// They work in kGroups independent groups of warps; group g fills the stages
 // it = g, g + kGroups, ...  A warp stalls for the full latency of its own stage's global loads, but
 // the other groups are then busy with other stages, so kGroups stages of loads are in flight per SM
 // without relying on how the compiler tracks outstanding loads inside one thread.
@@ -440,41 +382,9 @@ __device__ __forceinline__ void load_row4(float const* __restrict__ p, int r, in
 constexpr int kGroups = 3;
 constexpr int kGroupThreads = kProducerThreads / kGroups;       // 128
 constexpr int CHG = (BM * 8) / kGroupThreads;                    // chunks per thread per stage (8)
-constexpr int KSTEPG = 32 / CHG;                                 // MN-major: k rows between a thread's chunks (4)
 constexpr int RSTEPG = BM / CHG;                                 // K-major: rows between a thread's chunks (16)
 
-// Four consecutive rows ho0+s .. ho0+s+3 of one input column, loaded straight into their final
-// registers.  The window straddles at most two aligned groups of four rows, each wholly inside the
-// image or wholly padding, so every load has a single predicate; the load widths follow the
-// alignment of the window start (s & 3): 128 | 32+64+32 | 64+64 | 32+64+32 bits.
-__device__ __forceinline__ void issue_window(float const* __restrict__ ptr, int H, int W, FastPix const& px, int s, int dw,
-                                             int coff, bool on, float4& v)
-{
-  int const o = s & 3;
-  int const h0 = px.ho0 + s - o;            // first row of the aligned group that holds the window start
-  int const w = px.wo + dw;
-  bool const wok = on && px.valid && w >= 0 && w < W;
-  bool const g0 = wok && h0 >= 0 && h0 < H;
-  bool const g1 = wok && h0 + 4 >= 0 && h0 + 4 < H;
-  float const* a = ptr + (px.base + coff + dw * H + s);
-  v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (o == 0) {
-    if (g0) v = *reinterpret_cast<float4 const*>(a);
-  } else if (o == 2) {
-    if (g0) { float2 t = *reinterpret_cast<float2 const*>(a); v.x = t.x; v.y = t.y; }
-    if (g1) { float2 t = *reinterpret_cast<float2 const*>(a + 2); v.z = t.x; v.w = t.y; }
-  } else {
-    // o == 1: rows 0..2 lie in the first group, row 3 in the second; o == 3: row 0 | rows 1..3
-    bool const gm = (o == 1) ? g0 : g1;
-    if (g0) v.x = a[0];
-    if (gm) { float2 t = *reinterpret_cast<float2 const*>(a + 1); v.y = t.x; v.z = t.y; }
-    if (g1) v.w = a[3];
-  }
-}
-
-// The same window load with everything precomputed: a = address of the window start, o = its
-// alignment (s & 3), g0 / g1 = whether the first / second aligned group of rows is inside the image.
-// The window start is aligned to o = s & 3 elements only, so the four rows are fetched as four
+// Four consecutive rows ho0+s .. ho0+s+3 of one input column.  The window start is aligned to o = s & 3 elements only, so the four rows are fetched as four
 // independent predicated 32-bit loads: straight-line code (a load inside a branch makes the compiler
 // wait for it before the paths rejoin) and one destination register per load (two loads that may
 // write the same register are serialised by the scoreboard even when one is predicated off).  Both
@@ -506,8 +416,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
   __shared__ __align__(8) uint64_t accumBar;
   __shared__ __align__(8) uint64_t drainFull[2], drainEmpty[2], sumBar;   // T0/T1 hand-over; P complete
   __shared__ uint32_t tmemBase;
-  __shared__ int2 tapLut[64];       // IM2COL, pipelined: per filter tap fh + FH*fw {element offset of the tap, fh | fw<<5 | (s&3)<<10}
-  __shared__ int4 tapTab[BM];       // WGATHER, pipelined: per tile row (fh,fw,c) {element offset, row shift s, column shift dw, valid}
+  __shared__ int4 tapTab[BM];       // WGATHER: per tile row (fh,fw,c) {element offset, row shift s, column shift dw, valid}
 
   constexpr bool kAMN = (kAMode == OP_DENSE_MN || kAMode == OP_IM2COL);
   constexpr bool kBMN = (kBMode == OP_DENSE_MN);
@@ -538,19 +447,14 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
   int const numChunks = kSplit ? (numIter + p.drainEvery - 1) / p.drainEvery : 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(smem_u32(&fullBar[s]), p.pipelined ? kProducerWarps / kGroups : kGenericWarps); mbar_init(smem_u32(&emptyBar[s]), 1); }
+    for (int s = 0; s < p.stages; ++s) { mbar_init(smem_u32(&fullBar[s]), kAMode == OP_WGATHER ? kProducerWarps / kGroups : kGenericWarps); mbar_init(smem_u32(&emptyBar[s]), 1); }
     mbar_init(smem_u32(&accumBar), 1);
     for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(&drainFull[b]), 1); mbar_init(smem_u32(&drainEmpty[b]), kEpilogueWarps); }
     mbar_init(smem_u32(&sumBar), kEpilogueWarps);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kEpilogueWarps) tmem_alloc(smem_u32(&tmemBase), tmemCols);
-  if (kAMode == OP_IM2COL && p.pipelined && (int)threadIdx.x < p.a.FH * p.a.FW) {
-    int const fh = (int)threadIdx.x % p.a.FH, fw = (int)threadIdx.x / p.a.FH;
-    int const sft = fh * p.a.dy - p.a.pt;
-    tapLut[threadIdx.x] = make_int2((fw * p.a.dx - p.a.pl) * p.a.H + sft, fh | (fw << 5) | ((sft & 3) << 10));
-  }
-  if (kAMode == OP_WGATHER && p.pipelined && threadIdx.x < BM) {
+  if (kAMode == OP_WGATHER && threadIdx.x < BM) {
     TapCtx tc = tap_ctx(p.a, m0 + (int)threadIdx.x);
     tapTab[threadIdx.x] = make_int4((int)(tc.coff + fgrp * p.aGroup) + tc.dw * p.a.H + tc.dh, tc.dh, tc.dw, tc.valid ? 1 : 0);
   }
@@ -657,45 +561,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
     int const t = threadIdx.x - (kEpilogueWarps + 1) * 32;      // 0..kProducerThreads-1
     // MN-major tiles: chunk column t % 32, k rows t / 32 + KSTEP j.  K-major tiles: chunk t % 8, rows t / 8 + RSTEP j.
     int const mnChunk = t & 31, mnK = t >> 5, kmChunk = t & 7, kmRow = t >> 3;
-    bool const aFast = p.a.fast == 1;
     PixCtx px[4];
-    TapCtx tap[CH];
-    // fast IM2COL: this thread's four pixels, and its reduction index (fh,fw,c), which advances by KSTEP per step
-    FastPix fpx = {0, 0, 0, false};
-    int fFh = 0, fFw = 0, fC = 0, fR = 0, d8fh = 0, d8fw = 0, d8c = 0;
-    uint32_t g0mask = 0, g1mask = 0, wmask = 0;    // per tap row fh / column fw: is the aligned row group / the column inside the image
-    // fast WGATHER: this thread's four filter taps
-    int tapS[CH], tapDw[CH], tapCoff[CH];
-    bool tapOk[CH];
-    int const HW = p.a.H * p.a.W;
     if (kAMode == OP_IM2COL) {
-      if (aFast) {
-        fpx = fast_pix(p.a, m0 + 4 * mnChunk, p.a.rows);
-        fR = kbBeg * BK + mnK;
-        fFh = fR % p.a.FH; int q = fR / p.a.FH; fFw = q % p.a.FW; fC = q / p.a.FW;
-        d8fh = KSTEP % p.a.FH; q = KSTEP / p.a.FH; d8fw = q % p.a.FW; d8c = q / p.a.FW;
-        if (fpx.valid) {
-          for (int fh = 0; fh < p.a.FH; ++fh) {
-            int sft = fh * p.a.dy - p.a.pt, h0 = fpx.ho0 + sft - (sft & 3);
-            if (h0 >= 0 && h0 < p.a.H) g0mask |= 1u << fh;
-            if (h0 + 4 >= 0 && h0 + 4 < p.a.H) g1mask |= 1u << fh;
-          }
-          for (int fw = 0; fw < p.a.FW; ++fw) {
-            int w = fpx.wo + fw * p.a.dx - p.a.pl;
-            if (w >= 0 && w < p.a.W) wmask |= 1u << fw;
-          }
-        }
-      } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) px[e] = pix_ctx(p.a, m0 + 4 * mnChunk + e);
-      }
-    }
-    if (kAMode == OP_WGATHER) {
-#pragma unroll
-      for (int j = 0; j < CH; ++j) {
-        tap[j] = tap_ctx(p.a, m0 + kmRow + RSTEP * j);
-        tapS[j] = tap[j].dh; tapDw[j] = tap[j].dw; tapCoff[j] = (int)tap[j].coff; tapOk[j] = tap[j].valid;
-      }
+      for (int e = 0; e < 4; ++e) px[e] = pix_ctx(p.a, m0 + 4 * mnChunk + e);
     }
     // reduction-contiguous dense operands: row pointers are fixed for the thread
     float const* aRow[CH];
@@ -709,84 +578,17 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
       bRowOk[j] = (kBMode == OP_DENSE_K) && ib < p.b.rows && kmRow + RSTEP * j < BN;
       bRow[j] = p.b.ptr + (bRowOk[j] ? (long long)ib * p.b.ld : 0);
     }
-    if (p.pipelined && p.bTiles != nullptr && (kAMode == OP_IM2COL || kAMode == OP_WGATHER)) {
-      // ---- pipelined: group-per-stage producers; B arrives as a ready-made tile image through one
-      // bulk copy per stage.
+    if constexpr (kAMode == OP_WGATHER) {
+      // ---- group-per-stage producers; B arrives as a ready-made tile image through one bulk copy per stage.
       int const grp = t / kGroupThreads, tg = t % kGroupThreads;
-      int const gChunk = tg & 31, gK = tg >> 5;          // MN-major: chunk column, first k row
       int const gKc = tg & 7, gRow = tg >> 3;            // K-major: 16-byte chunk within the row, first row
       uint32_t const bBytes = (kSplit ? 2u : 1u) * bTileBytes;
-      FastPix gpx = {0, 0, 0, false};
-      uint32_t g0m = 0, g1m = 0, wm = 0;
-      if (kAMode == OP_IM2COL) {
-        if (p.a.fast == 1) gpx = fast_pix(p.a, m0 + 4 * gChunk, p.a.rows);
-        if (gpx.valid) {
-          for (int fh = 0; fh < p.a.FH; ++fh) {
-            int sft = fh * p.a.dy - p.a.pt, h0 = gpx.ho0 + sft - (sft & 3);
-            if (h0 >= 0 && h0 < p.a.H) g0m |= 1u << fh;
-            if (h0 + 4 >= 0 && h0 + 4 < p.a.H) g1m |= 1u << fh;
-          }
-          for (int fw = 0; fw < p.a.FW; ++fw) {
-            int w = gpx.wo + fw * p.a.dx - p.a.pl;
-            if (w >= 0 && w < p.a.W) wm |= 1u << fw;
-          }
-        }
-      }
-      // general gather (p.a.fast == 2: any extent, stride or dilation): the four pixels of a chunk are
-      // tracked one by one -- element offset of the pixel's window origin, and which tap rows / columns
-      // fall inside the image
       bool const aligned = p.a.fast == 1;
-      int eBase[4] = {0, 0, 0, 0};
-      uint32_t eHm[4] = {0, 0, 0, 0}, eWm[4] = {0, 0, 0, 0};
-      if (kAMode == OP_IM2COL && !aligned) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          int const m = m0 + 4 * gChunk + e;
-          if (m < p.a.rows) {
-            int ho = m % p.a.Ho, q = m / p.a.Ho, wo = q % p.a.Wo, n = q / p.a.Wo;
-            eBase[e] = n * (int)p.a.imgStride + wo * p.a.sx * p.a.H + ho * p.a.sy;
-            for (int fh = 0; fh < p.a.FH; ++fh) { int h = ho * p.a.sy + fh * p.a.dy - p.a.pt; if (h >= 0 && h < p.a.H) eHm[e] |= 1u << fh; }
-            for (int fw = 0; fw < p.a.FW; ++fw) { int w = wo * p.a.sx + fw * p.a.dx - p.a.pl; if (w >= 0 && w < p.a.W) eWm[e] |= 1u << fw; }
-          }
-        }
-      }
-      float const* const xb = p.a.ptr + gpx.base;
-      // reduction index of this thread's first chunk in its group's current stage, as (tap, channel);
-      // it advances by KSTEPG per chunk and by kGroups * BK per stage, with carries instead of divisions
-      int const taps = p.a.FH * p.a.FW;
-      int tap0 = 0, ch0 = 0;
-      if (kAMode == OP_IM2COL) { int r = (kbBeg + grp) * BK + gK; tap0 = r % taps; ch0 = r / taps; }
-      int const dTapJ = KSTEPG % taps, dChJ = KSTEPG / taps, dTapIt = (kGroups * BK) % taps, dChIt = (kGroups * BK) / taps;
       uint32_t aOff[CHG];
 #pragma unroll
-      for (int j = 0; j < CHG; ++j) aOff[j] = kAMN ? mnmajor_off(gChunk, gK + KSTEPG * j, BM / 32) : kmajor_off(gRow + RSTEPG * j, gKc);
+      for (int j = 0; j < CHG; ++j) aOff[j] = kmajor_off(gRow + RSTEPG * j, gKc);
       for (int it = grp; it < numIter; it += kGroups) {
         float4 R[CHG];
-        if (kAMode == OP_IM2COL) {
-          int tap = tap0, ch = ch0, r = (kbBeg + it) * BK + gK;
-#pragma unroll
-          for (int j = 0; j < CHG; ++j) {
-            int2 const te = tapLut[tap];
-            uint32_t const e = (uint32_t)te.y;
-            uint32_t const wv = (r < p.R ? 1u : 0u) & (wm >> ((e >> 5) & 31u));
-            if (aligned) {
-              bool const g0 = (wv & (g0m >> (e & 31u)) & 1u) != 0, g1 = (wv & (g1m >> (e & 31u)) & 1u) != 0;
-              issue_window2(xb + (ch * HW + te.x), (int)((e >> 10) & 3u), g0, g1, R[j]);
-            } else {
-              uint32_t const rv = r < p.R ? 1u : 0u, fh = e & 31u, fw = (e >> 5) & 31u;
-              float const* const q = p.a.ptr + (ch * HW + te.x);
-              R[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-              ldg32_if(R[j].x, q + eBase[0], (rv & (eHm[0] >> fh) & (eWm[0] >> fw) & 1u) != 0);
-              ldg32_if(R[j].y, q + eBase[1], (rv & (eHm[1] >> fh) & (eWm[1] >> fw) & 1u) != 0);
-              ldg32_if(R[j].z, q + eBase[2], (rv & (eHm[2] >> fh) & (eWm[2] >> fw) & 1u) != 0);
-              ldg32_if(R[j].w, q + eBase[3], (rv & (eHm[3] >> fh) & (eWm[3] >> fw) & 1u) != 0);
-            }
-            r += KSTEPG; tap += dTapJ; ch += dChJ;
-            if (tap >= taps) { tap -= taps; ++ch; }
-          }
-          tap0 += dTapIt; ch0 += dChIt;
-          if (tap0 >= taps) { tap0 -= taps; ++ch0; }
-        } else {
           if (aligned) {
             FastPix rp = fast_pix(p.a, (kbBeg + it) * BK + 4 * gKc, p.R);
             float const* const rb = p.a.ptr + rp.base;
@@ -822,7 +624,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
               ldg32_if(R[j].w, qp + pb[3], on && (unsigned)(ph[3] + e.y) < (unsigned)p.a.H && (unsigned)(pw[3] + e.z) < (unsigned)p.a.W);
             }
           }
-        }
         int const s = it % p.stages;
         if (!mbar_wait(smem_u32(&emptyBar[s]), (uint32_t)(((it / p.stages) & 1) ^ 1))) { atomicExch(p.status, 1); break; }
         uint8_t* base = smem + (size_t)s * stageBytes;
@@ -849,19 +650,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
       int const r0 = (kbBeg + it) * BK;
       float va[CH][4], vb[CH][4];
       // global loads first, so that all of them are in flight before the first use
-      if (kAMode == OP_IM2COL && aFast) {
-#pragma unroll
-        for (int j = 0; j < CH; ++j) {
-          load_shifted(p.a.ptr, p.a.H, p.a.W, fpx, fFh * p.a.dy - p.a.pt, fFw * p.a.dx - p.a.pl, fC * HW, fR < p.R, va[j]);
-          fR += KSTEP; fFh += d8fh; fFw += d8fw; fC += d8c;
-          if (fFh >= p.a.FH) { fFh -= p.a.FH; ++fFw; }
-          if (fFw >= p.a.FW) { fFw -= p.a.FW; ++fC; }
-        }
-      } else if (kAMode == OP_WGATHER && aFast) {
-        FastPix rp = fast_pix(p.a, r0 + 4 * kmChunk, p.R);
-#pragma unroll
-        for (int j = 0; j < CH; ++j) load_shifted(p.a.ptr, p.a.H, p.a.W, rp, tapS[j], tapDw[j], tapCoff[j], tapOk[j], va[j]);
-      } else if (kAMode == OP_DENSE_K && p.a.vec) {
+      if (kAMode == OP_DENSE_K && p.a.vec) {
         int const r = r0 + 4 * kmChunk;
         long long boff = 0;
         if (p.a.P) { int nb = r / p.a.P; boff = (long long)nb * p.a.bs - (long long)nb * p.a.P; }
@@ -872,7 +661,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
         for (int j = 0; j < CH; ++j) {
           if (kAMode == OP_IM2COL) load_im2col(p.a, px, r0 + mnK + KSTEP * j, p.R, va[j]);
           else if (kAMode == OP_DENSE_MN) load_dense_mn(p.a, m0 + 4 * mnChunk, r0 + mnK + KSTEP * j, p.R, va[j]);
-          else if (kAMode == OP_WGATHER) load_wgather(p.a, tap[j], r0 + 4 * kmChunk, p.R, va[j]);
           else load_dense_k(p.a, m0 + kmRow + RSTEP * j, r0 + 4 * kmChunk, p.R, va[j]);
         }
       }
@@ -1301,7 +1089,6 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
 
   int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int const numIter = p.kbPerSplit;                      // k-blocks per tile (work item: one range of the reduction of one output tile)
-  int const chunksPerTile = kSplit ? (numIter + kTsDrainEvery - 1) / kTsDrainEvery : 1;
   int const numTiles = p.tilesM * p.tilesN * p.splits;
   // this CTA's tiles: cta, cta + ctas, ...; tile t = (row tile t / tilesN, column tile t % tilesN)
   int const myTiles = cta < numTiles ? (numTiles - 1 - cta) / ctas + 1 : 0;
@@ -2583,7 +2370,7 @@ void conv_operand(Operand& o, ConvGeom const& g, float const* ptr, int channels)
   o.sy = g.sy; o.sx = g.sx; o.pt = g.pt; o.pl = g.pl; o.dy = g.dy; o.dx = g.dx;
   o.imgStride = (long long)g.H * g.W * channels;
   o.ld = 0; o.bs = 0; o.P = 0; o.vec = 0;
-  // 1: aligned windows (stride 1, extents multiples of 4); 2: element-wise gather, any geometry; 0: no pipelined path
+  // 1: aligned windows (stride 1, extents multiples of 4); 2: element-wise gather, any geometry; 0: the filter does not fit the tap tables
   bool const lut = g.FH <= 32 && g.FW <= 32 && g.FH * g.FW <= 64;
   o.fast = !lut ? 0 : ((g.sy == 1 && g.sx == 1 && g.H % 4 == 0 && g.Ho % 4 == 0 && aligned16(ptr)) ? 1 : 2);
 }
@@ -2760,7 +2547,7 @@ int fc_dgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, floa
   int const numKb = vlb::ceil_div(g.K, BK);
   p.splits = pick_wg_splits(ctx->smCount, vlb::ceil_div(V, BM) * vlb::ceil_div(p.N, p.BN), numKb, &p.kbPerSplit, 16);
   p.numKb = p.splits * p.kbPerSplit;
-  p.chanFast = 1; p.pipelined = 1;
+  p.chanFast = 1;
   size_t const nOut = (size_t)V * g.N;
   size_t const partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
   ProfScope prof(ctx, kProfFc);
@@ -2788,7 +2575,7 @@ int fc_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, floa
   p.a.rows = V;
   p.BN = pick_bn(p.N);
   p.numKb = vlb::ceil_div(g.N, BK); p.kbPerSplit = p.numKb; p.splits = 1;
-  p.chanFast = 1; p.pipelined = 1;
+  p.chanFast = 1;
   ProfScope prof(ctx, kProfFc);
   prof.rec.flops = 2.0 * (double)V * (double)g.K * (double)g.N;
   p.bTiles = prep_dense_tiles(ctx, dY, g.K, g.N, p.BN, p.numKb, false);                       // B(k, n) = dY[k + K n]
@@ -3137,7 +2924,6 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
     size_t const nOut = (size_t)p.M * g.K, partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
     p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, false, partBytes);
     if (!p.bTiles) return ctx->lastError;
-    p.pipelined = 1;
     if (p.splits == 1) return launch_ts(ctx, p, "conv_fprop_ts");
     SumEpilogue epi;
     epi.bias = b; epi.P = p.e.P; epi.K = g.K; epi.inMult = inMult; epi.outMult = outMult; epi.relu = ctx->fuseRelu;
@@ -3212,8 +2998,6 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     p.numKb = p.splits * p.kbPerSplit;
     p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, true, p.splits > 1 ? sizeof(float) * (size_t)p.M * g.C * p.splits : 0);
     if (!p.bTiles) return ctx->lastError;
-    p.b.ptr = p.bTiles;          // not read by the pipelined producers
-    p.pipelined = 1;
   } else {
     size_t nF = (size_t)g.FH * g.FW * g.FC * g.K;
     float* ft = (float*)workspace(ctx, sizeof(float) * nF);
@@ -3223,7 +3007,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     p.b.ptr = ft; p.b.vec = (V % 4 == 0);
   }
   p.e = Epilogue{}; p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
-  if (p.pipelined) {
+  if (p.bTiles) {
     ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true;
     if (p.splits == 1) { p.e.mask = ctx->reluMask; p.e.bias = ctx->dgradBias; return launch_ts(ctx, p, "conv_dgrad_ts"); }
     SumEpilogue epi;
@@ -3287,7 +3071,6 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
   p.bTiles = prep_dy_tiles(ctx, dY, g.K, p.R, P, p.BN, p.numKb, partBytes, dbHere, 0, g.G);
   if (!p.bTiles) return ctx->lastError;
   *dbDone = dbHere != nullptr;
-  p.pipelined = 1;
   if (splits == 1) {
     p.e.out = dF;
     return launch_gemm<OP_WGATHER, OP_DENSE_K, EPI_PLAIN>(ctx, p, 1, "conv_wgrad_tc");
