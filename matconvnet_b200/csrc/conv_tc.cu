@@ -831,13 +831,13 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 { asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(bar), "r"(bytes) : "memory"); }
 
 // Chains of one issuer in a tile of numIter k-blocks: the issuer that owns the tile's first k-block (second = 0) takes
-// the k-blocks 0, 2, ..., the other one (second = 1) the k-blocks 1, 3, ...; a chain is kTsDrainEvery own k-blocks (3xTF32)
+// the k-blocks 0, 2, ..., the other one (second = 1) the k-blocks 1, 3, ...; a chain is kChain own k-blocks (3xTF32)
 // or all of them (plain TF32).
-template <bool kSplit>
+template <bool kSplit, int kChain>
 __device__ __forceinline__ int ts_chains(int numIter, int second)
 {
   int const nOwn = numIter > second ? (numIter - second + 1) / 2 : 0;
-  return kSplit ? (nOwn + kTsDrainEvery - 1) / kTsDrainEvery : (nOwn > 0 ? 1 : 0);
+  return kSplit ? (nOwn + kChain - 1) / kChain : (nOwn > 0 ? 1 : 0);
 }
 
 // 4-D tensor-map copy global -> shared (tile mode, one destination CTA; the map covers this GPU's own memory only); completion
@@ -1053,6 +1053,10 @@ static_assert(kTsBStages < kTsDoneRing, "the loader must not be able to fall a w
 template <bool kSplit, int kMode, bool kNarrow, bool kGen>
 __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const* xmap, int const cta, int const ctas)
 {
+  // Chains half as long in the general gather: what it computes came from CUDA cores or from chains of large terms alone, and was nearer to the
+  // exact sum than chains of four own k-blocks are (AlexNet's first layer: 4.7e-7 of the output's spread beside a common factor, 3.2e-7 before,
+  // 2.8e-7 with two).  AlexNet batch 128 5.21 -> 5.34 ms, others level.
+  constexpr int kChain = kGen ? 2 : kTsDrainEvery;
   constexpr bool kTma = kMode == 1, kWg = kMode == 2;
   extern __shared__ uint8_t smemRaw[];
   __shared__ __align__(8) uint64_t fullA[4], doneK[kTsDoneRing], fullB[kTsBStages], emptyB[kTsBStages];
@@ -1142,7 +1146,7 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
         int const tm = p.dTilesN(tile);
         TileCols const tc = tile_cols<kGen>(p, tile - tm * p.tilesN);
         int const n0 = tc.n0;
-        int const chainsF = ts_chains<kSplit>(numIter, 0), chainsS = ts_chains<kSplit>(numIter, 1);   // of the issuer that owns the tile's first k-block, of the other
+        int const chainsF = ts_chains<kSplit, kChain>(numIter, 0), chainsS = ts_chains<kSplit, kChain>(numIter, 1);   // of the issuer that owns the tile's first k-block, of the other
         bool fresh = true;                              // P holds nothing of this tile yet
         if (kRegs > 0) {
 #pragma unroll
@@ -1301,7 +1305,7 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
     // Two issuing threads (in two warps, on two schedulers).  The tensor core's queue is about one MMA deep, so
     // while a thread waits on a barrier or commits, nothing of its own is in flight; with two threads the other
     // one's MMAs fill the gap.  Issuer q takes the k-blocks gi = q, q+2, ... (numbered over the CTA's life), which
-    // live in A stage q.  Chains (kTsDrainEvery own k-blocks) take the three T buffers in turn, in the order the
+    // live in A stage q.  Chains (kChain own k-blocks) take the three T buffers in turn, in the order the
     // drain warps will add them to P, so two chains are being accumulated while the third is drained; the two
     // issuers never touch the same tensor-memory columns, so no ordering between the two streams is needed.
     // Per k-block: one barrier wait (A written and B landed), twelve MMAs, one commit; per chain: a wait for the T
@@ -1322,14 +1326,14 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
       bool const takeTurns = BN > 64 && !kWg;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
         int const first = (int)((((long long)ts * numIter) ^ q) & 1);      // 0: this issuer owns the tile's first k-block
-        int const chainsF = ts_chains<kSplit>(numIter, 0), chainsS = ts_chains<kSplit>(numIter, 1);
+        int const chainsF = ts_chains<kSplit, kChain>(numIter, 0), chainsS = ts_chains<kSplit, kChain>(numIter, 1);
         for (int it = first, j = 0; it < numIter; it += 2, ++j) {
-          int const inChunk = kSplit ? j % kTsDrainEvery : j;
+          int const inChunk = kSplit ? j % kChain : j;
           bool const chunkStart = inChunk == 0;
-          bool const chunkEnd = it + 2 >= numIter || (kSplit && inChunk + 1 == kTsDrainEvery);
+          bool const chunkEnd = it + 2 >= numIter || (kSplit && inChunk + 1 == kChain);
           if (chunkStart) {
             // this chain's place in the drain order (first issuer's chain c, second issuer's chain c, first's c+1, ...)
-            int const c = kSplit ? j / kTsDrainEvery : 0;
+            int const c = kSplit ? j / kChain : 0;
             g = gBase + min(c, chainsF) + min(c, chainsS) + (first == 1 && c < chainsF ? 1 : 0);
             tAcc = tmemAcc + (uint32_t)((g % kNT) * BN);
             if (g >= kNT) {                           // the chain that sat in this T before must have been added to P
