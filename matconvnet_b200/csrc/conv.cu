@@ -184,7 +184,10 @@ int vlb_conv_backward(vlb_ctx* ctx, float* dX, float* dF, float* db, float const
   if (dX) {
     rc = vlb::conv_dgrad_small(ctx, g, dX, F, dY);
     if (rc == VLB_Unsupported) rc = tc ? vlb::conv_dgrad_tc(ctx, g, dX, F, dY) : VLB_Unsupported;
-    if (rc == VLB_Unsupported) rc = vlb::conv_dgrad_simt(ctx, g, dX, F, dY);
+    if (rc == VLB_Unsupported) {
+      ctx->maskDone = ctx->biasDone = false;      // the CUDA-core kernel below has neither the fused mask nor the fused bias
+      rc = vlb::conv_dgrad_simt(ctx, g, dX, F, dY);
+    }
     if (rc) return vlb::pass_error(ctx, rc, "vlb_conv_backward");
   }
   return VLB_Success;

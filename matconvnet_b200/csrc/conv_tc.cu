@@ -2817,11 +2817,12 @@ int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, f
       p.oys = g.sy; p.oxs = g.sx; p.oy = g.sy * iy - g.pt; p.ox = g.sx * ix - g.pl; p.outH = g.H; p.outW = g.W;
       p.shufY = g.sy; p.shufX = g.sx; p.outC = C;
       p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
-      ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true;
       PrepFilters& q = prep.p[0] = gen_prep(p, g, F);
       q.bh = g.sy * (FHm - 1); q.ah = -g.sy; q.bw = g.sx * (FWm - 1); q.aw = -g.sx;
       q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
-      return launch_ts_gen(ctx, ts, prep, dX, nOut, fin, true, "conv_dgrad_gen");
+      int const rc = launch_ts_gen(ctx, ts, prep, dX, nOut, fin, true, "conv_dgrad_gen");
+      if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true; }      // (a refused launch applies neither)
+      return rc;
     }
   }
   if (!classesOk) return VLB_Unsupported;
@@ -2847,9 +2848,10 @@ int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, f
       ++ts.n;
     }
   if (holes) fin.bias = nullptr;                    // (the zeros of the classes without a tap would miss it)
-  ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = !holes;
-  if (ts.n == 0) return VLB_Success;                // no tap reaches any pixel: all zeros, written above
-  return launch_ts_gen(ctx, ts, prep, dX, nOut, fin, !holes, "conv_dgrad_gen");
+  // (ts.n == 0: no tap reaches any pixel; all zeros, written above)
+  int const rc = ts.n == 0 ? VLB_Success : launch_ts_gen(ctx, ts, prep, dX, nOut, fin, !holes, "conv_dgrad_gen");
+  if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = !holes; }
+  return rc;
 }
 
 bool is_fc(ConvGeom const& g)

@@ -98,3 +98,28 @@ def test_few_images_and_few_tiles_vs_oracle(gpu, oracle, case, precision, tol):
         assert rel_l2(mat.to_numpy(dxm), np.where(x > 0, dx_ref, 0)) < tol
     finally:
         ctx.set_precision(0)
+
+
+@pytest.mark.parametrize("stride,k", [(2, 524321)])
+def test_mask_and_bias_survive_a_refused_launch(gpu, stride, k):
+    """A reduction of more than 65535 k-blocks (4 taps of k filters) is refused by the general gather and taken by the next kernel, which
+    fuses neither the ReLU mask nor the bias of a transposed convolution: both are then applied by passes of their own, so the results
+    equal the unfused ones bit for bit."""
+    import torch
+    nn, mat, ctx = gpu
+    ctx.set_precision(0)
+    g = torch.Generator(device="cuda").manual_seed(k)
+    normal = lambda *s: mat.empty(s).normal_(generator=g)       # noqa: E731
+    x, f = normal(4, 4, 8, 1), normal(3, 3, 8, k)
+    side = 2 if stride == 2 else 4
+    dy = normal(side, side, k, 1)
+    kw = dict(stride=stride, pad=1, no_der_filters=True, no_der_biases=True, ctx=ctx)
+    dx = nn.vl_nnconv(x, f, None, dy, **kw)[0]
+    dxm = nn.vl_nnconv(x, f, None, dy, through_relu=True, **kw)[0]
+    assert bool((dx != 0).all()) and torch.equal(dxm, torch.where(x > 0, dx, torch.zeros_like(dx)))
+    b = normal(1, 8)
+    crop = (1, 0, 1, 0) if stride == 2 else 1
+    y = nn.vl_nnconvt(dy, f, None, upsample=stride, crop=crop, ctx=ctx)
+    yb = nn.vl_nnconvt(dy, f, b, upsample=stride, crop=crop, ctx=ctx)
+    assert torch.equal(yb, y + b.reshape(1, 1, 8, 1))
+    assert ctx.device_status() == 0
