@@ -148,8 +148,8 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 { asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(bar) : "memory"); }
 
-// Bounded wait: false when the phase did not complete within gWaitCycles.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
+// Bounded wait: false when the phase did not complete within gWaitCycles + extra.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long extra = 0)
 {
   long long t0 = 0;
   for (uint32_t it = 0;; ++it) {
@@ -161,7 +161,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     if ((it & 15u) == 15u) {
       long long now = clock64();
       if (t0 == 0) t0 = now;
-      else if (now - t0 > gWaitCycles) return false;
+      else if (now - t0 > gWaitCycles + extra) return false;
     }
   }
 }
@@ -713,7 +713,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
   // quarter (warp % 4), so the five warps of a quarter (one of warps 0-3 and four producers, which
   // have finished by now) share that quarter's 32 output rows and split the columns in chunks of 16.
   if (warp != kEpilogueWarps) {
-    bool ok = mbar_wait(smem_u32(&accumBar), 0);
+    // The producer warps that have nothing to gather wait here for the whole reduction, so the bound grows with it: a k-block takes about 3000
+    // cycles at worst (element-wise gathers), a reduction of 65565 of them ran past the fixed bound.
+    bool ok = mbar_wait(smem_u32(&accumBar), 0, (long long)numIter * 16384);
     if (kSplit && ok) ok = mbar_wait(smem_u32(&sumBar), 0);
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();

@@ -123,3 +123,28 @@ def test_mask_and_bias_survive_a_refused_launch(gpu, stride, k):
     yb = nn.vl_nnconvt(dy, f, b, upsample=stride, crop=crop, ctx=ctx)
     assert torch.equal(yb, y + b.reshape(1, 1, 8, 1))
     assert ctx.device_status() == 0
+
+
+def test_data_gradient_of_a_very_long_reduction(gpu):
+    """65565 k-blocks in one output tile (9 taps of 233101 filters): longer than the bound of a single pipeline wait, which the warps without a
+    share of the gather spend in one wait for the whole reduction.  Against 64-bit sums; the bound: the small terms of the split (2^-11 of the
+    result) are added with truncation 2 * 4 * 65565 times, 2^-11 * 2^-24 * 524520 = 1.5e-5, the sums of chains far less."""
+    import torch
+    nn, mat, ctx = gpu
+    ctx.set_precision(0)
+    k = 233101
+    g = torch.Generator(device="cuda").manual_seed(k)
+    f = mat.empty((3, 3, 8, k)).normal_(generator=g)
+    dy = mat.empty((4, 4, k, 1)).normal_(generator=g)
+    x = mat.empty((4, 4, 8, 1)).normal_(generator=g)
+    dx = nn.vl_nnconv(x, f, None, dy, pad=1, no_der_filters=True, no_der_biases=True, ctx=ctx)[0]
+    dxm = nn.vl_nnconv(x, f, None, dy, pad=1, no_der_filters=True, no_der_biases=True, through_relu=True, ctx=ctx)[0]
+    assert ctx.device_status() == 0
+    want = torch.zeros(6, 6, 8, dtype=torch.float64, device="cuda")             # the padded plane
+    f64, dy64 = f.double(), dy[..., 0].double()
+    for a in range(3):
+        for b in range(3):
+            want[a:a + 4, b:b + 4] += dy64.reshape(16, k).matmul(f64[a, b].T).reshape(4, 4, 8)
+    want = want[1:5, 1:5]
+    assert float((dx[..., 0].double() - want).norm() / want.norm()) < 2e-5
+    assert torch.equal(dxm, torch.where(x > 0, dx, torch.zeros_like(dx)))
