@@ -312,8 +312,8 @@ int vlb_solver_update(vlb_ctx* ctx, int solver, float* W, float* S1, float* S2, 
                       double decay, double lr, vlb_solver_opts const* opts, long long t);
 
 /* The trainer's update of several parameter tensors in one launch (the loop over layers and parameters of
- * examples/cnn_train.m:451-507), each element as vlb_sgd_update / vlb_solver_update computes it.  The tensors of a list must not
- * overlap.  S2 is used by adadelta and adam only, t (the step count after this step) by adam only; S1 is the momentum state of
+ * examples/cnn_train.m:451-507), each element as vlb_sgd_update / vlb_solver_update computes it.  The result is that of the items
+ * one after the other: an item whose tensors overlap an earlier one's (weights shared by two layers) starts a launch of its own.  S2 is used by adadelta and adam only, t (the step count after this step) by adam only; S1 is the momentum state of
  * vlb_sgd_update_many. */
 typedef struct { float *W, *S1, *S2; float const* G; size_t n; double decay, lr; long long t; } vlb_param_update;
 int vlb_sgd_update_many(vlb_ctx* ctx, int count, vlb_param_update const* u, double gradMult, double momentum, int nesterov);

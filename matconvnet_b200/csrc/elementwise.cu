@@ -3,6 +3,7 @@
 // sized from the SM count.
 #include "common.cuh"
 #include <math.h>
+#include <algorithm>
 
 namespace {
 
@@ -173,31 +174,72 @@ __global__ void __launch_bounds__(kThreads) update_kernel(const __grid_constant_
   }
 }
 
-// Fills batches of kMaxUpdates and launches them; `lrOf` gives a tensor's learning rate as the kernel takes it.
+// How many of the n items of u, at most kMaxUpdates, may share a launch: no item writes what an earlier one of them reads or writes, or reads
+// what an earlier one writes (weights that two layers share; views into one buffer).  Such an item starts the next launch, which waits
+// for this one.  Sorted by address, the spans of a list without overlaps are checked in one pass; only a list with one is compared pair by pair.
+struct Span { uintptr_t beg, end; bool written; };
+
+int spans_of(vlb_param_update const& q, bool two, Span* s)
+{
+  size_t const bytes = sizeof(float) * q.n;
+  auto span = [&](float const* p, bool written) { return Span{(uintptr_t)p, (uintptr_t)p + bytes, written}; };
+  if (bytes == 0) return 0;
+  s[0] = span(q.W, true); s[1] = span(q.S1, true); s[2] = span(q.G, false);
+  if (two) s[3] = span(q.S2, true);
+  return two ? 4 : 3;
+}
+
+int batch_length(vlb_param_update const* u, int n, bool two)
+{
+  Span all[4 * kMaxUpdates];
+  int count = 0;
+  for (int i = 0; i < n; ++i) count += spans_of(u[i], two, all + count);
+  std::sort(all, all + count, [](Span const& a, Span const& b) { return a.beg < b.beg; });
+  uintptr_t endAll = 0, endWritten = 0;
+  bool overlap = false;
+  for (int k = 0; k < count; ++k) {
+    overlap = overlap || all[k].beg < (all[k].written ? endAll : endWritten);
+    endAll = std::max(endAll, all[k].end);
+    if (all[k].written) endWritten = std::max(endWritten, all[k].end);
+  }
+  if (!overlap) return n;
+  for (int i = 1; i < n; ++i) {
+    Span mine[4], other[4];
+    int const m = spans_of(u[i], two, mine);
+    for (int j = 0; j < i; ++j) {
+      int const o = spans_of(u[j], two, other);
+      for (int a = 0; a < m; ++a)
+        for (int b = 0; b < o; ++b)
+          if ((mine[a].written || other[b].written) && mine[a].beg < other[b].end && other[b].beg < mine[a].end) return i;
+    }
+  }
+  return n;
+}
+
+// Fills batches and launches them; `lrOf` gives a tensor's learning rate as the kernel takes it.
 template <bool kSgd, class LrOf>
 int launch_updates(vlb_ctx* ctx, UpdateBatch& b, bool two, int count, vlb_param_update const* u, LrOf lrOf, char const* where)
 {
-  unsigned blocks = 0;
-  b.count = 0;
-  auto flush = [&] {
-    if (b.count == 0) return;
+  for (int i = 0; i < count; ++i) VLB_REQUIRE(ctx, u[i].n / kUpdateChunk < (1u << 30) - 1, "update: tensor too large");
+  for (int first = 0; first < count;) {
+    int const end = first + batch_length(u + first, std::min(count - first, kMaxUpdates), two);
+    unsigned blocks = 0;
+    b.count = 0;
+    for (; first < end; ++first) {
+      vlb_param_update const& q = u[first];
+      unsigned const need = (unsigned)((q.n + kUpdateChunk - 1) / kUpdateChunk);
+      if (need == 0) continue;
+      if (blocks + need >= (1u << 31)) break;
+      UpdateItem& t = b.it[b.count++];
+      t.w = q.W; t.s1 = q.S1; t.s2 = two ? q.S2 : nullptr; t.g = q.G; t.n = q.n; t.decay = (float)q.decay; t.lr = lrOf(q); t.firstBlock = blocks;
+      t.vec = aligned16(q.W) && aligned16(q.S1) && aligned16(q.G) && (!two || aligned16(q.S2));
+      blocks += need;
+    }
+    if (b.count == 0) continue;
     if (two) vlb::launch(ctx->stream, update_kernel<kSgd, true>, blocks, kThreads, 0, b);
     else     vlb::launch(ctx->stream, update_kernel<kSgd, false>, blocks, kThreads, 0, b);
     VLB_LAUNCHED(ctx, 1);
-    b.count = 0; blocks = 0;
-  };
-  for (int i = 0; i < count; ++i) {
-    vlb_param_update const& q = u[i];
-    if (q.n == 0) continue;
-    size_t const need = (q.n + kUpdateChunk - 1) / kUpdateChunk;
-    VLB_REQUIRE(ctx, need < (1u << 30), "update: tensor too large");
-    if (b.count == kMaxUpdates || blocks + need >= (1u << 31)) flush();
-    UpdateItem& t = b.it[b.count++];
-    t.w = q.W; t.s1 = q.S1; t.s2 = two ? q.S2 : nullptr; t.g = q.G; t.n = q.n; t.decay = (float)q.decay; t.lr = lrOf(q); t.firstBlock = blocks;
-    t.vec = aligned16(q.W) && aligned16(q.S1) && aligned16(q.G) && (!two || aligned16(q.S2));
-    blocks += (unsigned)need;
   }
-  flush();
   return vlb::check_launch(ctx, where);
 }
 

@@ -262,3 +262,101 @@ def test_accumulate_gradients_with_a_solver(gpu):
                                num_workers=2, ctx=ctx)
     for (l, j), w in want.items():
         assert torch.equal(layers[l]["weights"][j], w) and state[(l, j)]["t"] == 1
+
+
+def _one_by_one(nn, solver, updates, args):
+    for u in updates:
+        if solver == "sgd":
+            nn.sgd_update_many_([u], *args)
+        else:
+            nn.solver_update_many_(solver, [u], args[0])
+
+
+@pytest.mark.parametrize("solver", ["sgd", "adam"])
+@pytest.mark.parametrize("shared", ["same", "view", "gradient"])
+def test_update_of_tensors_that_overlap_keeps_the_lists_order(gpu, solver, shared):
+    """Weights that two layers hold, views into one buffer and a gradient that is another item's weight: bit for bit the updates one after the
+    other.  The tensors are long enough that two items of one launch would run at the same time."""
+    import torch
+    nn, mat, ctx = gpu
+    n = 3_000_001
+
+    def make():
+        g = torch.Generator(device="cuda").manual_seed(7)
+        normal = lambda: torch.randn(n, device="cuda", generator=g)       # noqa: E731
+        buf = normal()
+        if shared == "same":
+            ws = [buf, normal(), buf, buf]
+        elif shared == "view":
+            ws = [buf[:2_000_000], normal()[:2_000_000], buf[500_000:2_500_000], buf[1_000_001:3_000_001]]
+        else:
+            ws = [buf, normal(), normal(), normal()]
+        m = ws[0].numel()
+        gs = [normal()[:m] for _ in ws]
+        if shared == "gradient":
+            gs[2] = ws[0]
+        st = [torch.zeros(m, device="cuda") if solver == "sgd" else {} for _ in ws]
+        return [(w, s, d, 0.0005, 0.1 * (i + 1)) for i, (w, s, d) in enumerate(zip(ws, st, gs))]
+
+    together, single = make(), make()
+    args = (0.5, 0.9, True)
+    for _ in range(3):
+        if solver == "sgd":
+            nn.sgd_update_many_(together, *args)
+        else:
+            nn.solver_update_many_(solver, together, args[0])
+        _one_by_one(nn, solver, single, args)
+    for a, b in zip(together, single):
+        assert torch.equal(a[0], b[0])
+        assert torch.equal(a[1], b[1]) if solver == "sgd" else torch.equal(a[1]["s2"], b[1]["s2"])
+
+
+def test_layers_that_share_their_weights(gpu):
+    """train.accumulate_gradients on two layers holding one tensor: the last layer's update, then the first one's (the order of
+    examples/cnn_train.m:452), each with a momentum of its own."""
+    import torch
+    from matconvnet_b200 import train
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(8)
+    w, d0, d1 = (mat.as_mat(torch.randn(64, 64, 64, 4, device="cuda", generator=g)) for _ in range(3))
+    want, m0, m1 = w.clone(), torch.zeros_like(w), torch.zeros_like(w)
+    net = {"layers": [dict(type="conv", weights=[w, None]), dict(type="conv", weights=[w, None])]}
+    params, state = train.default_params(), {}
+    for _ in range(3):
+        train.accumulate_gradients(net, [dict(dzdw=[d0, None]), dict(dzdw=[d1, None])], state, params, ctx=ctx)
+        nn.sgd_update_(want, m1, d1, 1.0, 0.0005, 0.9, 0.001, ctx=ctx)
+        nn.sgd_update_(want, m0, d0, 1.0, 0.0005, 0.9, 0.001, ctx=ctx)
+    assert torch.equal(w, want) and torch.equal(state[(1, 0)], m1) and torch.equal(state[(0, 0)], m0)
+
+
+@pytest.mark.parametrize("solver", ["sgd", "adagrad", "adadelta", "adam", "rmsprop"])
+def test_update_of_many_tensors(gpu, solver):
+    """150 tensors (three launches) of 1 to 9000 elements, some at unaligned addresses, with step counts that differ: bit for bit the updates
+    one by one."""
+    import torch
+    nn, mat, ctx = gpu
+    sizes = [2, 1, 3, 4, 5, 4095, 4096, 4097, 8192, 9000] * 15
+
+    def make():
+        g = torch.Generator(device="cuda").manual_seed(9)
+        out = []
+        for i, n in enumerate(sizes):
+            w, m, d = (torch.randn(n + 4, device="cuda", generator=g)[(i % 7 == k):][:n] for k in (1, 2, 3))
+            out.append((w, m if solver == "sgd" else {}, d, 0.001 * (i % 3), 0.01 + 0.001 * i))
+        return out
+
+    together, single = make(), make()
+    args = (0.25, 0.9, False)
+    for some in (together[::3], together, together[1::2]):          # (the step counts of the tensors drift apart)
+        if solver == "sgd":
+            nn.sgd_update_many_(some, *args)
+        else:
+            nn.solver_update_many_(solver, some, args[0])
+    for some in (single[::3], single, single[1::2]):
+        _one_by_one(nn, solver, some, args)
+    for a, b in zip(together, single):
+        assert torch.equal(a[0], b[0])
+        if solver == "sgd":
+            assert torch.equal(a[1], b[1])
+        else:
+            assert a[1]["t"] == b[1]["t"] and torch.equal(a[1]["s1"], b[1]["s1"])
