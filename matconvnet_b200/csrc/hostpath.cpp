@@ -83,6 +83,29 @@ at::Tensor flat32(PyObject* o, char const* name)
   return t;
 }
 
+// A new reference, let go of at the end of the scope.
+struct PyRef {
+  PyObject* p = nullptr;
+  PyRef() = default;
+  PyRef(PyRef const&) = delete;
+  PyRef& operator=(PyRef const&) = delete;
+  ~PyRef() { Py_XDECREF(p); }
+};
+
+// The two items of der_out = (first, second); `held` keeps them: the caller's sequence may make its items on access.
+struct Pair { PyObject *first = nullptr, *second = nullptr; };
+
+Pair two_items(PyObject* seq, PyRef& held)
+{
+  Pair r;
+  if (seq == Py_None) return r;
+  held.p = PySequence_Tuple(seq);
+  if (!held.p) throw PyFail();
+  if (PyTuple_GET_SIZE(held.p) != 2) fail(PyExc_ValueError, "der_out must have two items.");
+  r.first = PyTuple_GET_ITEM(held.p, 0); r.second = PyTuple_GET_ITEM(held.p, 1);
+  return r;
+}
+
 float* ptr(at::Tensor const& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 
 // A caller-supplied output for a parameter derivative (e.g. a view into a gradient bucket), checked, else a new tensor.
@@ -244,17 +267,12 @@ PyObject* conv(PyObject*, Args a, Py_ssize_t n)
     Shape const sd = shape4(dzdy);
     if (sd.d[0] != Ho || sd.d[1] != Wo || sd.d[2] != d.K || sd.d[3] != d.N)
       fail(PyExc_ValueError, "DEROUTPUT dimensions are incompatible with X and FILTERS.");
-    PyObject *gf = nullptr, *gb = nullptr;
-    if (a[13] != Py_None) {
-      gf = PySequence_GetItem(a[13], 0);
-      gb = gf ? PySequence_GetItem(a[13], 1) : nullptr;
-      Py_XDECREF(gf); Py_XDECREF(gb);              // (the caller's sequence keeps them)
-      if (!gb) throw PyFail();
-    }
+    PyRef held;
+    Pair const given = two_items(a[13], held);
     at::Tensor dx, df, db;
     if (!as_bool(a[8])) dx = empty_cm(d.H, d.W, d.C, d.N, x.device());
-    if (!as_bool(a[9])) df = der_out(gf, at::IntArrayRef(sf.d, 4), x.device(), "DF");
-    if (!as_bool(a[10]) && b.defined()) { int64_t const s[2] = {1, d.K}; db = der_out(gb, at::IntArrayRef(s, 2), x.device(), "DB"); }
+    if (!as_bool(a[9])) df = der_out(given.first, at::IntArrayRef(sf.d, 4), x.device(), "DF");
+    if (!as_bool(a[10]) && b.defined()) { int64_t const s[2] = {1, d.K}; db = der_out(given.second, at::IntArrayRef(s, 2), x.device(), "DB"); }
     auto const fn = as_bool(a[12]) ? vlb_relu_conv_backward : (fc ? vlb_fc_backward : vlb_conv_backward);
     ctx.check(fn(ctx.h, ptr(dx), ptr(df), ptr(db), ptr(x), ptr(f), ptr(dzdy), &d));
     return tuple_of({dx, df, db});
@@ -333,15 +351,10 @@ PyObject* bnorm(PyObject*, Args a, Py_ssize_t n)
       return tuple_of({y, mom});
     }
     if (!same4(shape4(dzdy), H, W, C, N)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X.");
-    PyObject *gg = nullptr, *gb = nullptr;
-    if (a[7] != Py_None) {
-      gg = PySequence_GetItem(a[7], 0);
-      gb = gg ? PySequence_GetItem(a[7], 1) : nullptr;
-      Py_XDECREF(gg); Py_XDECREF(gb);
-      if (!gb) throw PyFail();
-    }
+    PyRef held;
+    Pair const own = two_items(a[7], held);
     int64_t const sc[2] = {C, 1};
-    at::Tensor dx = empty4(s, x.device()), dg = der_out(gg, at::IntArrayRef(sc, 2), x.device(), "DG"), db = der_out(gb, at::IntArrayRef(sc, 2), x.device(), "DB");
+    at::Tensor dx = empty4(s, x.device()), dg = der_out(own.first, at::IntArrayRef(sc, 2), x.device(), "DG"), db = der_out(own.second, at::IntArrayRef(sc, 2), x.device(), "DB");
     if (given) ctx.check(vlb_bnorm_backward_moment(ctx.h, ptr(dx), ptr(dg), ptr(db), ptr(mom), ptr(x), ptr(g), ptr(b), ptr(dzdy), H, W, C, N, eps));
     else       ctx.check(vlb_bnorm_backward(ctx.h, ptr(dx), ptr(dg), ptr(db), ptr(mom), ptr(x), ptr(g), ptr(b), ptr(dzdy), H, W, C, N, eps));
     return tuple_of({dx, dg, db, mom});

@@ -473,3 +473,44 @@ def test_bnorm_relu_fused_forward_is_bit_identical(gpu):
     for a, c in zip(plain, fused):
         for u, v in zip(a["dzdw"] or [], c["dzdw"] or []):
             assert (u is None and v is None) or torch.equal(u, v)
+
+
+@pytest.mark.parametrize("block", ["conv", "bnorm"])
+def test_der_out_of_a_sequence_that_makes_its_items_on_access(gpu, block):
+    """der_out may be any sequence; one whose items exist only while they are asked for (views cut from a bucket) must keep them alive
+    through the call.  The garbage made between the two look-ups would take the place of an item that was let go of."""
+    import torch
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = mat.as_mat(torch.randn(8, 8, 16, 2, device="cuda", generator=g))
+    f = mat.as_mat(torch.randn(3, 3, 16, 16, device="cuda", generator=g))
+    v = mat.as_mat(torch.randn(16, 1, device="cuda", generator=g))
+    dy = mat.as_mat(torch.randn(8, 8, 16, 2, device="cuda", generator=g))
+    bucket = torch.zeros(f.numel() + 16, device="cuda")
+
+    class Views:
+        def __getitem__(self, i):
+            if i > 1:
+                raise IndexError(i)
+            junk = [torch.zeros(1, device="cuda") for _ in range(64)]       # noqa: F841
+            if block == "bnorm":
+                return bucket[16 * i:][:16].reshape(1, 16).permute(1, 0)
+            return bucket[:f.numel()].reshape(16, 16, 3, 3).permute(3, 2, 1, 0) if i == 0 else bucket[f.numel():].reshape(16, 1).permute(1, 0)
+
+        def __len__(self):
+            return 2
+
+    if block == "conv":
+        call = lambda **kw: nn.vl_nnconv(x, f, v, dy, pad=1, **kw)[1:3]       # noqa: E731
+    else:
+        call = lambda **kw: nn.vl_nnbnorm(x, v, v, dy, **kw)[1:3]       # noqa: E731
+    want = call()
+    for _ in range(20):
+        bucket.zero_()
+        got = call(der_out=Views())
+        assert got[0].data_ptr() == bucket.data_ptr()
+        assert all(torch.equal(a.reshape(b.shape), b) for a, b in zip(got, want))
+    assert all(torch.equal(a.reshape(b.shape), b) for a, b in zip(call(der_out=(None for _ in range(2))), want))
+    for items in ((None,), (None,) * 3):
+        with pytest.raises(ValueError):
+            call(der_out=items)
