@@ -383,7 +383,7 @@ PyObject* pool(PyObject*, Args a, Py_ssize_t n)
       ctx.check(vlb_pool_forward(ctx.h, ptr(y), ptr(x), &d));
       return wrap(y);
     }
-    if (!same4(shape4(dzdy), Ho, Wo, d.C, d.N)) fail(PyExc_ValueError, "DEROUTPUT dimensions are incompatible with X and POOL.");
+    if (!same4(shape4(dzdy), Ho, Wo, d.C, d.N)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X and POOL.");
     at::Tensor dx = empty4(s, x.device());
     auto const fn = as_bool(a[7]) ? vlb_relu_pool_backward : vlb_pool_backward;
     ctx.check(fn(ctx.h, ptr(dx), ptr(x), ptr(dzdy), &d));
@@ -411,7 +411,7 @@ PyObject* roipool(PyObject*, Args a, Py_ssize_t n)
       ctx.check(vlb_roipool_forward(ctx.h, ptr(y), ptr(x), ptr(rois), H, W, C, N, K, S[0], S[1], tf, method));
       return wrap(y);
     }
-    if (!same4(shape4(dzdy), S[0], S[1], C, K)) fail(PyExc_ValueError, "DEROUTPUT dimensions are incompatible with X and ROIS.");
+    if (!same4(shape4(dzdy), S[0], S[1], C, K)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X and ROIS.");
     at::Tensor dx = empty4(s, x.device());
     ctx.check(vlb_roipool_backward(ctx.h, ptr(dx), ptr(x), ptr(rois), ptr(dzdy), H, W, C, N, K, S[0], S[1], tf, method));
     return wrap(dx);
@@ -433,7 +433,7 @@ PyObject* sampler(PyObject*, Args a, Py_ssize_t n)
       ctx.check(vlb_sampler_forward(ctx.h, ptr(y), ptr(x), ptr(grid), H, W, C, N, Ho, Wo, Ng));
       return wrap(y);
     }
-    if (!same4(shape4(dzdy), Ho, Wo, C, Ng)) fail(PyExc_ValueError, "DEROUTPUT dimensions are incompatible with X and GRID.");
+    if (!same4(shape4(dzdy), Ho, Wo, C, Ng)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X and GRID.");
     at::Tensor dx = empty4(s, x.device()), dgrid = empty_cm(2, Ho, Wo, Ng, x.device());
     ctx.check(vlb_sampler_backward(ctx.h, ptr(dx), ptr(dgrid), ptr(x), ptr(grid), ptr(dzdy), H, W, C, N, Ho, Wo, Ng));
     return tuple_of({dx, dgrid});

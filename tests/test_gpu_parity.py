@@ -514,3 +514,21 @@ def test_der_out_of_a_sequence_that_makes_its_items_on_access(gpu, block):
     for items in ((None,), (None,) * 3):
         with pytest.raises(ValueError):
             call(der_out=items)
+
+
+def test_texts_of_refused_derivatives(gpu):
+    """Every operator names the argument it refuses as it did when the checks were in Python."""
+    import torch
+    nn, mat, ctx = gpu
+    x, bad = mat.as_mat(torch.zeros(8, 8, 4, 2, device="cuda")), mat.as_mat(torch.zeros(3, 3, 4, 2, device="cuda"))
+    f, v = mat.as_mat(torch.zeros(3, 3, 4, 5, device="cuda")), mat.as_mat(torch.zeros(4, 1, device="cuda"))
+    rois, grid = mat.as_mat(torch.ones(5, 2, device="cuda")), mat.as_mat(torch.zeros(2, 6, 6, 2, device="cuda"))
+    for call, text in ((lambda: nn.vl_nnconv(x, f, None, bad), "DEROUTPUT dimensions are incompatible with X and FILTERS."),
+                       (lambda: nn.vl_nnpool(x, 2, bad, stride=2), "DZDY dimensions are incompatible with X and POOL."),
+                       (lambda: nn.vl_nnroipool(x, rois, bad, subdivisions=(2, 2)), "DZDY dimensions are incompatible with X and ROIS."),
+                       (lambda: nn.vl_nnbilinearsampler(x, grid, bad), "DZDY dimensions are incompatible with X and GRID."),
+                       (lambda: nn.vl_nnbnorm(x, v, v, bad), "DZDY dimensions are incompatible with X."),
+                       (lambda: nn.vl_nnnormalize(x, [3, 1, 1, 0.75], bad), "DZDY dimensions are incompatible with X.")):
+        with pytest.raises(ValueError) as e:
+            call()
+        assert str(e.value) == text
