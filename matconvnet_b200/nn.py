@@ -201,6 +201,11 @@ def solver_update_many_(solver, updates, grad_mult, opts=None, ctx=None):
     o = dict(capi.SOLVER_DEFAULTS[solver])
     o.update(opts or {})
     two = solver in ("adadelta", "adam")
+    for w, _, g, _, _ in updates:             # a refused list leaves every state and step count as it was
+        if not all(isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 for t in (w, g)):
+            raise TypeError("w and grad must be CUDA float32 tensors")
+        if w.numel() != g.numel():
+            raise ValueError("parameter and gradient do not have the same number of elements.")
     items = []
     for w, state, g, decay, lr in updates:
         if "s1" not in state:

@@ -360,3 +360,16 @@ def test_update_of_many_tensors(gpu, solver):
             assert torch.equal(a[1], b[1])
         else:
             assert a[1]["t"] == b[1]["t"] and torch.equal(a[1]["s1"], b[1]["s1"])
+
+
+def test_a_refused_solver_step_leaves_the_state_as_it_was(gpu):
+    import torch
+    nn, mat, ctx = gpu
+    w, d = torch.ones(10, device="cuda"), torch.ones(10, device="cuda")
+    state, fresh = {}, {}
+    nn.solver_update_("adam", w, state, d, 1.0, 0.0, 0.1, ctx=ctx)
+    before = state["s1"].clone()
+    for bad, error in ((d[:9], ValueError), (d.double(), TypeError)):
+        with pytest.raises(error):
+            nn.solver_update_many_("adam", [(w, state, d, 0.0, 0.1), (w, fresh, bad, 0.0, 0.1)], 1.0, ctx=ctx)
+    assert state["t"] == 1 and torch.equal(state["s1"], before) and fresh == {}
