@@ -4,7 +4,7 @@
 // networks; here it is 2 to 4 us.  Nothing is kept from one call to the next.
 //
 // Tensors are column-major CUDA float32 torch tensors (matconvnet_b200/mat.py); memory comes from torch's allocator, work goes
-// to torch's current stream.  Errors of the engine are raised by the Python context (Context.check).
+// to torch's current stream.  Arguments are read under the interpreter lock; outputs are allocated and the engine is called without it.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <ATen/ATen.h>
@@ -12,6 +12,8 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <array>
+#include <mutex>
+#include <string>
 #include <vector>
 #include "../../include/vlb.h"
 
@@ -23,8 +25,17 @@ struct PyFail {};        // a Python exception is set
 [[noreturn]] void fail(PyObject* type, char const* fmt, char const* a) { PyErr_Format(type, fmt, a); throw PyFail(); }
 
 PyObject* gHandleName;                // "_h": the context's vlb_ctx pointer as a Python int
-PyObject* gCheckName;                 // "check"
 PyObject *gPair, *gQuad;              // nn._pair, nn._quad: any sequence numpy understands, and the error messages
+PyObject* gError;                     // capi.VlbError
+
+// The interpreter lock let go of for a scope.
+struct Unlocked {
+  PyThreadState* const state = PyEval_SaveThread();
+  Unlocked() = default;
+  Unlocked(Unlocked const&) = delete;
+  Unlocked& operator=(Unlocked const&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
 
 // ---------------------------------------------------------------- tensors
 struct Shape { int64_t d[4]; };
@@ -70,6 +81,7 @@ at::Tensor need(PyObject* o, char const* name)
   at::Tensor const& t = THPVariable_Unpack(o);
   if (!t.is_cuda() || t.scalar_type() != at::kFloat) fail(PyExc_TypeError, "%s must be a CUDA float32 tensor (this engine has no CPU path)", name);
   if (column_major(t)) return t;
+  Unlocked u;
   at::Tensor c = empty_cm(t.sizes(), t.device());
   c.copy_(t);
   return c;
@@ -108,10 +120,10 @@ Pair two_items(PyObject* seq, PyRef& held)
 
 float* ptr(at::Tensor const& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 
-// A caller-supplied output for a parameter derivative (e.g. a view into a gradient bucket), checked, else a new tensor.
-at::Tensor der_out(PyObject* given, at::IntArrayRef shape, at::Device dev, char const* name)
+// A caller-supplied output for a parameter derivative of `shape` (e.g. a view into a gradient bucket), checked; undefined without one.
+at::Tensor der_out(PyObject* given, at::IntArrayRef shape, char const* name)
 {
-  if (given == nullptr || given == Py_None) return empty_cm(shape, dev);
+  if (given == nullptr || given == Py_None) return at::Tensor();
   int64_t n = 1;
   for (int64_t s : shape) n *= s;
   if (THPVariable_Check(given)) {
@@ -180,27 +192,45 @@ void ints(PyObject* o, int n, int* out, char const* name)
   if (PyErr_Occurred()) throw PyFail();
 }
 
+// The calls of one context come one at a time, whatever threads they come from: its stream, scratch and error message belong to the call.
+// The locks stand in a fixed table; two contexts that share a place wait for one another's launches, nothing more.
+std::mutex& lock_of(vlb_ctx* h)
+{
+  static std::mutex locks[61];
+  return locks[((uintptr_t)h >> 4) % 61];
+}
+
 // The engine context behind a capi.Context, on torch's current stream.
 struct Ctx {
-  PyObject* obj;
   vlb_ctx* h;
-  explicit Ctx(PyObject* o) : obj(o)
+  void* stream;
+  explicit Ctx(PyObject* o)
   {
     PyObject* p = PyObject_GetAttr(o, gHandleName);
     if (!p) throw PyFail();
     h = static_cast<vlb_ctx*>(PyLong_AsVoidPtr(p));
     Py_DECREF(p);
     if (PyErr_Occurred()) throw PyFail();
-    vlb_ctx_set_stream(h, c10::cuda::getCurrentCUDAStream().stream());
+    stream = c10::cuda::getCurrentCUDAStream().stream();
   }
-  void check(int rc) const
+  // f: allocates the outputs, calls the engine and returns its error code, which becomes capi.VlbError.  Without the interpreter lock, since it may wait: in the
+  // allocator, for a place in the launch queue, for the stream when scratch grows.
+  template <class F>
+  void run(F f) const
   {
+    int rc;
+    std::string message;
+    {
+      Unlocked u;                                                  // (before the context's lock: a thread that waits for that one holds no other)
+      std::lock_guard<std::mutex> one(lock_of(h));
+      vlb_ctx_set_stream(h, stream);
+      rc = f();
+      if (rc) { message = vlb_ctx_last_error(h); vlb_ctx_reset_error(h); }
+    }
     if (rc == 0) return;
-    PyObject* code = PyLong_FromLong(rc);
-    PyObject* r = code ? PyObject_CallMethodOneArg(obj, gCheckName, code) : nullptr;
-    Py_XDECREF(code);
-    Py_XDECREF(r);
-    if (r) PyErr_SetString(PyExc_RuntimeError, "the engine reported an error");
+    PyObject* e = PyObject_CallFunction(gError, "is", rc, message.c_str());
+    if (e) PyErr_SetObject((PyObject*)Py_TYPE(e), e);
+    Py_XDECREF(e);
     throw PyFail();
   }
 };
@@ -258,10 +288,14 @@ PyObject* conv(PyObject*, Args a, Py_ssize_t n)
     bool const fc = Ho == 1 && Wo == 1 && d.strideY == 1 && d.strideX == 1 && d.padTop == 0 && d.padBottom == 0 && d.padLeft == 0 && d.padRight == 0 &&
                     d.dilateY == 1 && d.dilateX == 1 && d.FC == d.C && d.FH == d.H && d.FW == d.W;
     if (!dzdy.defined()) {
-      at::Tensor y = empty_cm(Ho, Wo, d.K, d.N, x.device());
-      if (as_bool(a[11])) ctx.check(vlb_conv_relu_forward(ctx.h, ptr(y), ptr(x), ptr(f), ptr(b), &d));
-      else if (fc)        ctx.check(vlb_fc_forward(ctx.h, ptr(y), ptr(x), ptr(f), ptr(b), &d));
-      else                ctx.check(vlb_conv_forward(ctx.h, ptr(y), 0.0, ptr(x), 1.0, ptr(f), ptr(b), &d));
+      at::Tensor y;
+      bool const relu = as_bool(a[11]);
+      ctx.run([&] {
+        y = empty_cm(Ho, Wo, d.K, d.N, x.device());
+        if (relu) return vlb_conv_relu_forward(ctx.h, ptr(y), ptr(x), ptr(f), ptr(b), &d);
+        if (fc)   return vlb_fc_forward(ctx.h, ptr(y), ptr(x), ptr(f), ptr(b), &d);
+        return vlb_conv_forward(ctx.h, ptr(y), 0.0, ptr(x), 1.0, ptr(f), ptr(b), &d);
+      });
       return wrap(y);
     }
     Shape const sd = shape4(dzdy);
@@ -269,12 +303,18 @@ PyObject* conv(PyObject*, Args a, Py_ssize_t n)
       fail(PyExc_ValueError, "DEROUTPUT dimensions are incompatible with X and FILTERS.");
     PyRef held;
     Pair const given = two_items(a[13], held);
+    bool const wantX = !as_bool(a[8]), wantF = !as_bool(a[9]), wantB = !as_bool(a[10]) && b.defined();
+    int64_t const sb[2] = {1, d.K};
     at::Tensor dx, df, db;
-    if (!as_bool(a[8])) dx = empty_cm(d.H, d.W, d.C, d.N, x.device());
-    if (!as_bool(a[9])) df = der_out(given.first, at::IntArrayRef(sf.d, 4), x.device(), "DF");
-    if (!as_bool(a[10]) && b.defined()) { int64_t const s[2] = {1, d.K}; db = der_out(given.second, at::IntArrayRef(s, 2), x.device(), "DB"); }
+    if (wantF) df = der_out(given.first, at::IntArrayRef(sf.d, 4), "DF");
+    if (wantB) db = der_out(given.second, at::IntArrayRef(sb, 2), "DB");
     auto const fn = as_bool(a[12]) ? vlb_relu_conv_backward : (fc ? vlb_fc_backward : vlb_conv_backward);
-    ctx.check(fn(ctx.h, ptr(dx), ptr(df), ptr(db), ptr(x), ptr(f), ptr(dzdy), &d));
+    ctx.run([&] {
+      if (wantX) dx = empty_cm(d.H, d.W, d.C, d.N, x.device());
+      if (wantF && !df.defined()) df = empty_cm(at::IntArrayRef(sf.d, 4), x.device());
+      if (wantB && !db.defined()) db = empty_cm(at::IntArrayRef(sb, 2), x.device());
+      return fn(ctx.h, ptr(dx), ptr(df), ptr(db), ptr(x), ptr(f), ptr(dzdy), &d);
+    });
     return tuple_of({dx, df, db});
   });
 }
@@ -299,18 +339,24 @@ PyObject* convt(PyObject*, Args a, Py_ssize_t n)
     int Ho = 0, Wo = 0;
     vlb_convt_output_shape(&d, &Ho, &Wo);
     if (!dzdy.defined()) {
-      at::Tensor y = empty_cm(Ho > 0 ? Ho : 0, Wo > 0 ? Wo : 0, K > 0 ? K : 0, d.N, x.device());
-      ctx.check(vlb_convt_forward(ctx.h, ptr(y), ptr(x), ptr(f), ptr(b), &d));
+      at::Tensor y;
+      ctx.run([&] {
+        y = empty_cm(Ho > 0 ? Ho : 0, Wo > 0 ? Wo : 0, K > 0 ? K : 0, d.N, x.device());
+        return vlb_convt_forward(ctx.h, ptr(y), ptr(x), ptr(f), ptr(b), &d);
+      });
       return wrap(y);
     }
     Shape const sd = shape4(dzdy);
     if (sd.d[0] != Ho || sd.d[1] != Wo || sd.d[2] != K || sd.d[3] != d.N)
       fail(PyExc_ValueError, "DEROUTPUT dimensions are incompatible with X and FILTERS.");
+    bool const wantX = !as_bool(a[8]), wantF = !as_bool(a[9]), wantB = !as_bool(a[10]) && b.defined();
     at::Tensor dx, df, db;
-    if (!as_bool(a[8])) dx = empty_cm(d.H, d.W, d.C, d.N, x.device());
-    if (!as_bool(a[9])) df = empty_cm(at::IntArrayRef(sf.d, 4), x.device());
-    if (!as_bool(a[10]) && b.defined()) db = empty_cm(1, K, x.device());
-    ctx.check(vlb_convt_backward(ctx.h, ptr(dx), ptr(df), ptr(db), ptr(x), ptr(f), ptr(dzdy), &d));
+    ctx.run([&] {
+      if (wantX) dx = empty_cm(d.H, d.W, d.C, d.N, x.device());
+      if (wantF) df = empty_cm(at::IntArrayRef(sf.d, 4), x.device());
+      if (wantB) db = empty_cm(1, K, x.device());
+      return vlb_convt_backward(ctx.h, ptr(dx), ptr(df), ptr(db), ptr(x), ptr(f), ptr(dzdy), &d);
+    });
     return tuple_of({dx, df, db});
   });
 }
@@ -338,25 +384,32 @@ PyObject* bnorm(PyObject*, Args a, Py_ssize_t n)
     if (g.numel() != C || b.numel() != C) fail(PyExc_ValueError, "The number of elements of MULTIPLIERS / BIASES is not the number of channels.");
     bool const given = mom.defined(), relu = as_bool(a[8]);
     if (given && mom.numel() != 2 * (int64_t)C) fail(PyExc_ValueError, "MOMENTS must have 2*C elements.");
-    if (!given) mom = empty_cm(C, 2, x.device());
     if (!dzdy.defined()) {
-      at::Tensor y = empty4(s, x.device());
-      if (given) {
-        ctx.check(vlb_bnorm_forward_moment(ctx.h, ptr(y), ptr(mom), ptr(x), ptr(g), ptr(b), H, W, C, N, eps));
-        if (relu) ctx.check(vlb_relu_forward(ctx.h, ptr(y), ptr(y), (size_t)y.numel()));
-      } else {
-        auto const fn = relu ? vlb_bnorm_relu_forward : vlb_bnorm_forward;
-        ctx.check(fn(ctx.h, ptr(y), ptr(mom), ptr(x), ptr(g), ptr(b), H, W, C, N, eps));
-      }
+      at::Tensor y;
+      ctx.run([&] {
+        y = empty4(s, x.device());
+        if (given) {
+          int const rc = vlb_bnorm_forward_moment(ctx.h, ptr(y), ptr(mom), ptr(x), ptr(g), ptr(b), H, W, C, N, eps);
+          return rc || !relu ? rc : vlb_relu_forward(ctx.h, ptr(y), ptr(y), (size_t)y.numel());
+        }
+        mom = empty_cm(C, 2, x.device());
+        return (relu ? vlb_bnorm_relu_forward : vlb_bnorm_forward)(ctx.h, ptr(y), ptr(mom), ptr(x), ptr(g), ptr(b), H, W, C, N, eps);
+      });
       return tuple_of({y, mom});
     }
     if (!same4(shape4(dzdy), H, W, C, N)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X.");
     PyRef held;
     Pair const own = two_items(a[7], held);
     int64_t const sc[2] = {C, 1};
-    at::Tensor dx = empty4(s, x.device()), dg = der_out(own.first, at::IntArrayRef(sc, 2), x.device(), "DG"), db = der_out(own.second, at::IntArrayRef(sc, 2), x.device(), "DB");
-    if (given) ctx.check(vlb_bnorm_backward_moment(ctx.h, ptr(dx), ptr(dg), ptr(db), ptr(mom), ptr(x), ptr(g), ptr(b), ptr(dzdy), H, W, C, N, eps));
-    else       ctx.check(vlb_bnorm_backward(ctx.h, ptr(dx), ptr(dg), ptr(db), ptr(mom), ptr(x), ptr(g), ptr(b), ptr(dzdy), H, W, C, N, eps));
+    at::Tensor dx, dg = der_out(own.first, at::IntArrayRef(sc, 2), "DG"), db = der_out(own.second, at::IntArrayRef(sc, 2), "DB");
+    ctx.run([&] {
+      dx = empty4(s, x.device());
+      if (!dg.defined()) dg = empty_cm(at::IntArrayRef(sc, 2), x.device());
+      if (!db.defined()) db = empty_cm(at::IntArrayRef(sc, 2), x.device());
+      if (given) return vlb_bnorm_backward_moment(ctx.h, ptr(dx), ptr(dg), ptr(db), ptr(mom), ptr(x), ptr(g), ptr(b), ptr(dzdy), H, W, C, N, eps);
+      mom = empty_cm(C, 2, x.device());
+      return vlb_bnorm_backward(ctx.h, ptr(dx), ptr(dg), ptr(db), ptr(mom), ptr(x), ptr(g), ptr(b), ptr(dzdy), H, W, C, N, eps);
+    });
     return tuple_of({dx, dg, db, mom});
   });
 }
@@ -379,14 +432,20 @@ PyObject* pool(PyObject*, Args a, Py_ssize_t n)
     int Ho = 0, Wo = 0;
     vlb_pool_output_shape(&d, &Ho, &Wo);
     if (!dzdy.defined()) {
-      at::Tensor y = empty_cm(Ho > 0 ? Ho : 0, Wo > 0 ? Wo : 0, d.C, d.N, x.device());
-      ctx.check(vlb_pool_forward(ctx.h, ptr(y), ptr(x), &d));
+      at::Tensor y;
+      ctx.run([&] {
+        y = empty_cm(Ho > 0 ? Ho : 0, Wo > 0 ? Wo : 0, d.C, d.N, x.device());
+        return vlb_pool_forward(ctx.h, ptr(y), ptr(x), &d);
+      });
       return wrap(y);
     }
     if (!same4(shape4(dzdy), Ho, Wo, d.C, d.N)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X and POOL.");
-    at::Tensor dx = empty4(s, x.device());
+    at::Tensor dx;
     auto const fn = as_bool(a[7]) ? vlb_relu_pool_backward : vlb_pool_backward;
-    ctx.check(fn(ctx.h, ptr(dx), ptr(x), ptr(dzdy), &d));
+    ctx.run([&] {
+      dx = empty4(s, x.device());
+      return fn(ctx.h, ptr(dx), ptr(x), ptr(dzdy), &d);
+    });
     return wrap(dx);
   });
 }
@@ -407,13 +466,19 @@ PyObject* roipool(PyObject*, Args a, Py_ssize_t n)
     double tf[6];
     for (int i = 0; i < 6; ++i) tf[i] = as_double(PyTuple_GET_ITEM(a[5], i));
     if (!dzdy.defined()) {
-      at::Tensor y = empty_cm(S[0], S[1], C, K, x.device());
-      ctx.check(vlb_roipool_forward(ctx.h, ptr(y), ptr(x), ptr(rois), H, W, C, N, K, S[0], S[1], tf, method));
+      at::Tensor y;
+      ctx.run([&] {
+        y = empty_cm(S[0], S[1], C, K, x.device());
+        return vlb_roipool_forward(ctx.h, ptr(y), ptr(x), ptr(rois), H, W, C, N, K, S[0], S[1], tf, method);
+      });
       return wrap(y);
     }
     if (!same4(shape4(dzdy), S[0], S[1], C, K)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X and ROIS.");
-    at::Tensor dx = empty4(s, x.device());
-    ctx.check(vlb_roipool_backward(ctx.h, ptr(dx), ptr(x), ptr(rois), ptr(dzdy), H, W, C, N, K, S[0], S[1], tf, method));
+    at::Tensor dx;
+    ctx.run([&] {
+      dx = empty4(s, x.device());
+      return vlb_roipool_backward(ctx.h, ptr(dx), ptr(x), ptr(rois), ptr(dzdy), H, W, C, N, K, S[0], S[1], tf, method);
+    });
     return wrap(dx);
   });
 }
@@ -429,13 +494,19 @@ PyObject* sampler(PyObject*, Args a, Py_ssize_t n)
     if (g.d[0] != 2) fail(PyExc_ValueError, "GRID has more than 2 channels.");
     if (N == 0 || Ng % N != 0) fail(PyExc_ValueError, "The number of GRIDs is not a multiple of the number of images.");
     if (!dzdy.defined()) {
-      at::Tensor y = empty_cm(Ho, Wo, C, Ng, x.device());
-      ctx.check(vlb_sampler_forward(ctx.h, ptr(y), ptr(x), ptr(grid), H, W, C, N, Ho, Wo, Ng));
+      at::Tensor y;
+      ctx.run([&] {
+        y = empty_cm(Ho, Wo, C, Ng, x.device());
+        return vlb_sampler_forward(ctx.h, ptr(y), ptr(x), ptr(grid), H, W, C, N, Ho, Wo, Ng);
+      });
       return wrap(y);
     }
     if (!same4(shape4(dzdy), Ho, Wo, C, Ng)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X and GRID.");
-    at::Tensor dx = empty4(s, x.device()), dgrid = empty_cm(2, Ho, Wo, Ng, x.device());
-    ctx.check(vlb_sampler_backward(ctx.h, ptr(dx), ptr(dgrid), ptr(x), ptr(grid), ptr(dzdy), H, W, C, N, Ho, Wo, Ng));
+    at::Tensor dx, dgrid;
+    ctx.run([&] {
+      dx = empty4(s, x.device()); dgrid = empty_cm(2, Ho, Wo, Ng, x.device());
+      return vlb_sampler_backward(ctx.h, ptr(dx), ptr(dgrid), ptr(x), ptr(grid), ptr(dzdy), H, W, C, N, Ho, Wo, Ng);
+    });
     return tuple_of({dx, dgrid});
   });
 }
@@ -445,9 +516,11 @@ PyObject* relu(PyObject*, Args a, Py_ssize_t n)
 {
   return guarded(n, 3, [&]() -> PyObject* {
     Ctx ctx(a[0]);
-    at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy"), out = empty_cm(x.sizes(), x.device());
-    if (!dzdy.defined()) ctx.check(vlb_relu_forward(ctx.h, ptr(out), ptr(x), (size_t)x.numel()));
-    else                 ctx.check(vlb_relu_backward(ctx.h, ptr(out), ptr(x), ptr(dzdy), (size_t)x.numel()));
+    at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy"), out;
+    ctx.run([&] {
+      out = empty_cm(x.sizes(), x.device());
+      return dzdy.defined() ? vlb_relu_backward(ctx.h, ptr(out), ptr(x), ptr(dzdy), (size_t)x.numel()) : vlb_relu_forward(ctx.h, ptr(out), ptr(x), (size_t)x.numel());
+    });
     return wrap(out);
   });
 }
@@ -462,9 +535,13 @@ PyObject* normalize(PyObject*, Args a, Py_ssize_t n)
     int const H = (int)s.d[0], W = (int)s.d[1], C = (int)s.d[2], N = (int)s.d[3], depth = as_int(a[3]);
     double const kappa = as_double(a[4]), alpha = as_double(a[5]), beta = as_double(a[6]);
     if (dzdy.defined() && !same4(shape4(dzdy), H, W, C, N)) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X.");
-    at::Tensor out = empty4(s, x.device());
-    if (!dzdy.defined()) ctx.check(vlb_lrn_forward(ctx.h, ptr(out), ptr(x), H, W, C, N, depth, kappa, alpha, beta));
-    else                 ctx.check((as_bool(a[7]) ? vlb_relu_lrn_backward : vlb_lrn_backward)(ctx.h, ptr(out), ptr(x), ptr(dzdy), H, W, C, N, depth, kappa, alpha, beta));
+    auto const back = as_bool(a[7]) ? vlb_relu_lrn_backward : vlb_lrn_backward;
+    at::Tensor out;
+    ctx.run([&] {
+      out = empty4(s, x.device());
+      if (dzdy.defined()) return back(ctx.h, ptr(out), ptr(x), ptr(dzdy), H, W, C, N, depth, kappa, alpha, beta);
+      return vlb_lrn_forward(ctx.h, ptr(out), ptr(x), H, W, C, N, depth, kappa, alpha, beta);
+    });
     return wrap(out);
   });
 }
@@ -477,9 +554,11 @@ PyObject* softmax(PyObject*, Args a, Py_ssize_t n)
     at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy");
     Shape const s = shape4(x);
     int const H = (int)s.d[0], W = (int)s.d[1], C = (int)s.d[2], N = (int)s.d[3];
-    at::Tensor out = empty4(s, x.device());
-    if (!dzdy.defined()) ctx.check(vlb_softmax_forward(ctx.h, ptr(out), ptr(x), H, W, C, N));
-    else                 ctx.check(vlb_softmax_backward(ctx.h, ptr(out), ptr(x), ptr(dzdy), H, W, C, N));
+    at::Tensor out;
+    ctx.run([&] {
+      out = empty4(s, x.device());
+      return dzdy.defined() ? vlb_softmax_backward(ctx.h, ptr(out), ptr(x), ptr(dzdy), H, W, C, N) : vlb_softmax_forward(ctx.h, ptr(out), ptr(x), H, W, C, N);
+    });
     return wrap(out);
   });
 }
@@ -490,16 +569,26 @@ PyObject* dropout(PyObject*, Args a, Py_ssize_t n)
   return guarded(n, 6, [&]() -> PyObject* {
     Ctx ctx(a[0]);
     at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy"), mask = need(a[4], "mask");
-    if (!mask.defined()) {
-      unsigned long long const seed = PyLong_AsUnsignedLongLongMask(a[5]);
+    bool const drawn = !mask.defined();
+    unsigned long long seed = 0;
+    double rate = 0;
+    if (drawn) {
+      seed = PyLong_AsUnsignedLongLongMask(a[5]);
       if (PyErr_Occurred()) throw PyFail();
-      mask = empty_cm(x.sizes(), x.device());
-      ctx.check(vlb_dropout_mask(ctx.h, ptr(mask), (size_t)x.numel(), as_double(a[3]), seed));
+      rate = as_double(a[3]);
     } else if (mask.numel() != x.numel()) {
       fail(PyExc_ValueError, "MASK and X do not have the same number of elements.");
     }
-    at::Tensor out = empty_cm(x.sizes(), x.device());
-    ctx.check(vlb_mul(ctx.h, ptr(out), ptr(mask), ptr(dzdy.defined() ? dzdy : x), (size_t)x.numel()));
+    at::Tensor out;
+    ctx.run([&] {
+      if (drawn) {
+        mask = empty_cm(x.sizes(), x.device());
+        int const rc = vlb_dropout_mask(ctx.h, ptr(mask), (size_t)x.numel(), rate, seed);
+        if (rc) return rc;
+      }
+      out = empty_cm(x.sizes(), x.device());
+      return vlb_mul(ctx.h, ptr(out), ptr(mask), ptr(dzdy.defined() ? dzdy : x), (size_t)x.numel());
+    });
     return tuple_of({out, mask});
   });
 }
@@ -514,13 +603,19 @@ PyObject* softmaxloss(PyObject*, Args a, Py_ssize_t n)
     int const H = (int)s.d[0], W = (int)s.d[1], C = (int)s.d[2], N = (int)s.d[3];
     if (c.numel() != N) fail(PyExc_ValueError, "one label per image expected");
     if (a[3] == Py_None) {
-      at::Tensor loss = at::empty({1}, x.options());
-      ctx.check(vlb_softmaxloss_forward(ctx.h, ptr(loss), ptr(x), ptr(c), H, W, C, N));
+      at::Tensor loss;
+      ctx.run([&] {
+        loss = at::empty({1}, x.options());
+        return vlb_softmaxloss_forward(ctx.h, ptr(loss), ptr(x), ptr(c), H, W, C, N);
+      });
       return wrap(loss);
     }
     double const dzdy = as_double(a[3]);
-    at::Tensor dx = empty4(s, x.device());
-    ctx.check(vlb_softmaxloss_backward(ctx.h, ptr(dx), ptr(x), ptr(c), dzdy, H, W, C, N));
+    at::Tensor dx;
+    ctx.run([&] {
+      dx = empty4(s, x.device());
+      return vlb_softmaxloss_backward(ctx.h, ptr(dx), ptr(x), ptr(c), dzdy, H, W, C, N);
+    });
     return wrap(dx);
   });
 }
@@ -532,8 +627,13 @@ PyObject* taccum(PyObject*, Args a, Py_ssize_t n)
     Ctx ctx(a[0]);
     at::Tensor u = flat32(a[2], "a"), v = flat32(a[4], "b");
     if (u.numel() != v.numel()) fail(PyExc_ValueError, "A and B do not have the same number of elements.");
-    at::Tensor y = a[5] == Py_None ? at::empty_like(u) : flat32(a[5], "out");
-    ctx.check(vlb_taccum(ctx.h, ptr(y), as_double(a[1]), ptr(u), as_double(a[3]), ptr(v), (size_t)u.numel()));
+    at::Tensor y;
+    if (a[5] != Py_None) y = flat32(a[5], "out");
+    double const alpha = as_double(a[1]), beta = as_double(a[3]);
+    ctx.run([&] {
+      if (!y.defined()) y = at::empty_like(u);
+      return vlb_taccum(ctx.h, ptr(y), alpha, ptr(u), beta, ptr(v), (size_t)u.numel());
+    });
     return wrap(y);
   });
 }
@@ -548,6 +648,8 @@ PyObject* update(PyObject*, Args a, Py_ssize_t n)
     if (!PyList_CheckExact(a[2]) || !PyTuple_CheckExact(a[6]) || PyTuple_GET_SIZE(a[6]) != 4) fail(PyExc_TypeError, "a list of updates and four options expected");
     Py_ssize_t const count = PyList_GET_SIZE(a[2]);
     std::vector<vlb_param_update> u((size_t)count);
+    std::vector<at::Tensor> held;                        // (another thread may change the list's tuples meanwhile)
+    held.reserve(4 * (size_t)count);
     for (Py_ssize_t i = 0; i < count; ++i) {
       PyObject* t = PyList_GET_ITEM(a[2], i);
       if (!PyTuple_CheckExact(t) || PyTuple_GET_SIZE(t) != 7) fail(PyExc_TypeError, "an update is a tuple of seven");
@@ -559,6 +661,7 @@ PyObject* update(PyObject*, Args a, Py_ssize_t n)
                                           : "parameter and gradient do not have the same number of elements.");
       vlb_param_update& p = u[(size_t)i];
       p.W = ptr(w); p.S1 = ptr(s1); p.S2 = ptr(s2); p.G = ptr(g); p.n = (size_t)w.numel();
+      held.insert(held.end(), {w, s1, s2, g});
       p.decay = as_double(PyTuple_GET_ITEM(t, 4)); p.lr = as_double(PyTuple_GET_ITEM(t, 5));
       p.t = PyLong_AsLongLong(PyTuple_GET_ITEM(t, 6));
       if (PyErr_Occurred()) throw PyFail();
@@ -567,18 +670,20 @@ PyObject* update(PyObject*, Args a, Py_ssize_t n)
     vlb_solver_opts so = {};
     so.rho = as_double(PyTuple_GET_ITEM(a[6], 0)); so.epsilon = as_double(PyTuple_GET_ITEM(a[6], 1));
     so.beta1 = as_double(PyTuple_GET_ITEM(a[6], 2)); so.beta2 = as_double(PyTuple_GET_ITEM(a[6], 3));
-    if (solver < 0) ctx.check(vlb_sgd_update_many(ctx.h, (int)count, u.data(), gm, momentum, as_bool(a[5]) ? 1 : 0));
-    else            ctx.check(vlb_solver_update_many(ctx.h, solver, (int)count, u.data(), gm, &so));
+    int const nesterov = as_bool(a[5]) ? 1 : 0;
+    ctx.run([&] {
+      return solver < 0 ? vlb_sgd_update_many(ctx.h, (int)count, u.data(), gm, momentum, nesterov) : vlb_solver_update_many(ctx.h, solver, (int)count, u.data(), gm, &so);
+    });
     Py_RETURN_NONE;
   });
 }
 
 // ---------------------------------------------------------------- the module
-PyObject* setup(PyObject*, Args a, Py_ssize_t n)      // nn._pair, nn._quad
+PyObject* setup(PyObject*, Args a, Py_ssize_t n)      // nn._pair, nn._quad, capi.VlbError
 {
-  if (n != 2) { PyErr_SetString(PyExc_TypeError, "two callables expected"); return nullptr; }
-  Py_INCREF(a[0]); Py_INCREF(a[1]);
-  Py_XSETREF(gPair, a[0]); Py_XSETREF(gQuad, a[1]);
+  if (n != 3) { PyErr_SetString(PyExc_TypeError, "three callables expected"); return nullptr; }
+  Py_INCREF(a[0]); Py_INCREF(a[1]); Py_INCREF(a[2]);
+  Py_XSETREF(gPair, a[0]); Py_XSETREF(gQuad, a[1]); Py_XSETREF(gError, a[2]);
   Py_RETURN_NONE;
 }
 
@@ -593,6 +698,5 @@ PyModuleDef gModule = {PyModuleDef_HEAD_INIT, "_hostpath", "Native host side of 
 PyMODINIT_FUNC PyInit__hostpath(void)
 {
   gHandleName = PyUnicode_InternFromString("_h");
-  gCheckName = PyUnicode_InternFromString("check");
   return PyModule_Create(&gModule);
 }

@@ -62,7 +62,7 @@ def _quad(v, name):
     raise ValueError("%s must have one or four elements" % name)
 
 
-_hostpath.setup(_pair, _quad)
+_hostpath.setup(_pair, _quad, capi.VlbError)
 
 
 # --------------------------------------------------------------------- vl_nnconv
