@@ -517,6 +517,7 @@ PyObject* relu(PyObject*, Args a, Py_ssize_t n)
   return guarded(n, 3, [&]() -> PyObject* {
     Ctx ctx(a[0]);
     at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy"), out;
+    if (dzdy.defined() && dzdy.numel() != x.numel()) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X.");
     ctx.run([&] {
       out = empty_cm(x.sizes(), x.device());
       return dzdy.defined() ? vlb_relu_backward(ctx.h, ptr(out), ptr(x), ptr(dzdy), (size_t)x.numel()) : vlb_relu_forward(ctx.h, ptr(out), ptr(x), (size_t)x.numel());
@@ -554,6 +555,7 @@ PyObject* softmax(PyObject*, Args a, Py_ssize_t n)
     at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy");
     Shape const s = shape4(x);
     int const H = (int)s.d[0], W = (int)s.d[1], C = (int)s.d[2], N = (int)s.d[3];
+    if (dzdy.defined() && dzdy.numel() != x.numel()) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X.");
     at::Tensor out;
     ctx.run([&] {
       out = empty4(s, x.device());
@@ -569,6 +571,7 @@ PyObject* dropout(PyObject*, Args a, Py_ssize_t n)
   return guarded(n, 6, [&]() -> PyObject* {
     Ctx ctx(a[0]);
     at::Tensor x = need_one(a[1], "x"), dzdy = need(a[2], "dzdy"), mask = need(a[4], "mask");
+    if (dzdy.defined() && dzdy.numel() != x.numel()) fail(PyExc_ValueError, "DZDY dimensions are incompatible with X.");
     bool const drawn = !mask.defined();
     unsigned long long seed = 0;
     double rate = 0;
@@ -629,6 +632,7 @@ PyObject* taccum(PyObject*, Args a, Py_ssize_t n)
     if (u.numel() != v.numel()) fail(PyExc_ValueError, "A and B do not have the same number of elements.");
     at::Tensor y;
     if (a[5] != Py_None) y = flat32(a[5], "out");
+    if (y.defined() && y.numel() != u.numel()) fail(PyExc_ValueError, "OUT and A do not have the same number of elements.");
     double const alpha = as_double(a[1]), beta = as_double(a[3]);
     ctx.run([&] {
       if (!y.defined()) y = at::empty_like(u);

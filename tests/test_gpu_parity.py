@@ -532,3 +532,15 @@ def test_texts_of_refused_derivatives(gpu):
         with pytest.raises(ValueError) as e:
             call()
         assert str(e.value) == text
+
+
+def test_element_wise_operators_refuse_derivatives_of_another_size(gpu):
+    import torch
+    nn, mat, ctx = gpu
+    x = mat.as_mat(torch.ones(8, 8, 4, 2, device="cuda"))
+    for bad in (mat.as_mat(torch.ones(8, 8, 4, 1, device="cuda")), mat.as_mat(torch.ones(9, 8, 4, 2, device="cuda"))):
+        for call in (lambda: nn.vl_nnrelu(x, bad), lambda: nn.vl_nnsoftmax(x, bad), lambda: nn.vl_nndropout(x, bad),
+                     lambda: nn.vl_nndropout(x, bad, mask=x), lambda: nn.vl_taccum(1.0, x, 1.0, x, out=bad)):
+            with pytest.raises(ValueError):
+                call()
+    assert torch.equal(nn.vl_nnrelu(x, x.reshape(8, 8, 8).permute(0, 1, 2)).reshape(-1), x.reshape(-1))       # (another shape of the same size is taken, as before)
