@@ -505,9 +505,12 @@ sampler_bwd_gather_kernel(float* __restrict__ dx, float const* __restrict__ grid
 }
 
 // The planes of four channels in shared memory (pixels: of the plane or planes that a block holds at a time), where an image fills a good part of
-// the chip with blocks, a stage of x is not mostly unread (Q at least half of a plane), and the planes fit.
-bool planes_apply(vlb_ctx* ctx, long long pixels, bool readsMost, int C, long long blocks)
-{ return C >= 3 && (long long)sizeof(float4) * pixels <= 220 * 1024 && readsMost && blocks >= ctx->smCount; }
+// the chip with blocks, a stage of x is not mostly unread (Q at least half of a plane), and the planes fit.  These kernels count output pixels, and
+// four planes of them, in 32 bits: grids of 2^29 pixels and more, and more blocks than a launch has, take the thread-per-pixel kernel.
+bool planes_apply(vlb_ctx* ctx, long long pixels, bool readsMost, int C, int Q, long long blocks)
+{
+  return C >= 3 && (long long)sizeof(float4) * pixels <= 220 * 1024 && readsMost && Q < (1 << 29) && blocks >= ctx->smCount && blocks < (1LL << 31);
+}
 
 // the three kernels above take as much shared memory as an SM has; false with a CUDA error pending
 bool allow_smem(vlb_ctx* ctx)
@@ -542,7 +545,7 @@ int vlb_sampler_forward(vlb_ctx* ctx, float* Y, float const* X, float const* gri
   VLB_REQUIRE(ctx, Y && X && grid, "sampler_forward: null tensor");
   VLB_REQUIRE(ctx, (((uintptr_t)grid) & 7) == 0, "sampler_forward: grid must be 8-byte aligned");
   int const Q = Ho * Wo, quads = vlb::ceil_div(C, 4);
-  if (planes_apply(ctx, (long long)H * W, 2LL * Q >= (long long)H * W, C, (long long)N * quads)) {
+  if (planes_apply(ctx, (long long)H * W, 2LL * Q >= (long long)H * W, C, Q, (long long)N * quads)) {
     if (!allow_smem(ctx)) return vlb::check_launch(ctx, "vlb_sampler_forward");
     vlb::launch(ctx->stream, sampler_fwd_planes_kernel, (unsigned)(N * quads), kPlaneThreads, sizeof(float4) * (size_t)H * W, Y, X, grid, H, W, C, Q, Ng / N, quads);
     VLB_LAUNCHED(ctx, 1);
@@ -583,7 +586,7 @@ int vlb_sampler_backward(vlb_ctx* ctx, float* dX, float* dGrid, float const* X, 
   if (!dX) {
     // the grid derivative alone: blocks of at most kGridThreads * kPlaneQ output pixels (each reads the whole image, from L2 all but once)
     int const parts = vlb::ceil_div(Qo, kGridThreads * kPlaneQ);
-    if (planes_apply(ctx, 2LL * HWi * kGridCh / 4, 2LL * Qo >= HWi, C, (long long)Ng * parts)) {
+    if (planes_apply(ctx, 2LL * HWi * kGridCh / 4, 2LL * Qo >= HWi, C, Qo, (long long)Ng * parts)) {
       int const QP = vlb::ceil_div(Qo, parts);
       if (!allow_smem(ctx)) return vlb::check_launch(ctx, "vlb_sampler_backward");
       vlb::launch(ctx->stream, sampler_grid_planes_kernel, (unsigned)(Ng * parts), kGridThreads, 2 * kGridCh * sizeof(float) * (size_t)HWi, dGrid, X, grid, dY, H, W, C, Qo,

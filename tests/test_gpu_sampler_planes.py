@@ -27,3 +27,33 @@ def test_sampler_planes(gpu, oracle, h, w, c, n, group, ho, wo):
     dxr, dgr = oracle.sampler_backward(x, grid, dy)
     assert np.array_equal(mat.to_numpy(dx), dxr)
     assert np.array_equal(mat.to_numpy(dgrid), dgr)
+
+
+def test_grid_derivative_of_the_largest_grid(gpu):
+    """2^31 - 1 output pixels, more than the kernel with the planes in shared memory can count: the first and the last pixels equal those of a
+    small call bit for bit (a pixel's derivative depends on no other pixel)."""
+    import ctypes
+    import torch
+    nn, mat, ctx = gpu
+    H = W = 8
+    C, Q, few = 3, (1 << 31) - 1, 5000
+    torch.cuda.empty_cache()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = mat.empty((H, W, C, 1)).normal_(generator=g)
+    ends = torch.rand(2 * few, 2, device="cuda", generator=g) * 2.4 - 1.2
+    dends = torch.randn(C, 2 * few, device="cuda", generator=g)
+
+    def run(grid, dy, q):
+        out = torch.empty(q, 2, device="cuda")
+        ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+        ctx.check(ctx.lib.vlb_sampler_backward(ctx.handle, None, *(ctypes.c_void_p(t.data_ptr()) for t in (out, x, grid, dy)), H, W, C, 1, 1, q, 1))
+        return out
+
+    want = run(ends, dends, 2 * few)
+    grid, dy = torch.zeros(Q, 2, device="cuda"), torch.zeros(C, Q, device="cuda")
+    for t, e in ((grid.T, ends.T), (dy, dends)):
+        t[:, :few], t[:, Q - few:] = e[:, :few], e[:, few:]
+    got = run(grid, dy, Q)
+    assert torch.equal(got[:few], want[:few]) and torch.equal(got[Q - few:], want[few:])
+    del grid, dy, got
+    torch.cuda.empty_cache()
