@@ -28,104 +28,6 @@ constexpr int kThreads = 256;
 // stats layout handed from pass 1 to pass 2 (device memory, 4*C floats):
 // [0,C) mean, [C,2C) sigma, [2C,3C) dgamma, [3C,4C) dbeta
 
-template <int kSums>
-__device__ __forceinline__ void accumulate(float (&acc)[4], float x, float dy)
-{
-  acc[0] += x;
-  acc[1] = fmaf(x, x, acc[1]);
-  if (kSums == 4) { acc[2] = fmaf(dy, x, acc[2]); acc[3] += dy; }
-}
-
-// kMode 0: moments only (forward).  1: moments + ders (backward).  2: ders only, moments given.
-template <int kMode, bool kVec>
-__global__ void __cluster_dims__(1, kCluster, 1) __launch_bounds__(kThreads)
-bnorm_reduce_kernel(float* __restrict__ momentsOut,   // 2*C or nullptr
-                    float* __restrict__ dgOut, float* __restrict__ dbOut,
-                    float const* __restrict__ momentsIn,  // mode 2
-                    float const* __restrict__ x, float const* __restrict__ dy,
-                    int WH, int C, int N, float eps)
-{
-  vlb::pdl_wait();
-  cg::cluster_group cluster = cg::this_cluster();
-  __shared__ float part[4];
-  __shared__ float warpRed[kThreads / 32][4];
-  int c = blockIdx.x;
-  int rank = (int)cluster.block_rank();   // the cluster spans grid y
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-
-  // Work items: (image n, chunk of the plane).  Item i of this channel goes to CTA i % kCluster.
-  if (kVec) {
-    int WH4 = WH >> 2;
-    long long items = (long long)N * WH4;
-    for (long long i = (long long)rank * kThreads + threadIdx.x; i < items; i += (long long)kCluster * kThreads) {
-      int n = (int)(i / WH4);
-      int q = (int)(i - (long long)n * WH4);
-      size_t off = ((size_t)n * C + c) * (size_t)WH + 4 * (size_t)q;
-      float4 xv = *reinterpret_cast<float4 const*>(x + off);
-      float4 dv = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (kMode != 0) dv = *reinterpret_cast<float4 const*>(dy + off);
-      if (kMode == 2) {
-        acc[2] = fmaf(dv.x, xv.x, acc[2]); acc[2] = fmaf(dv.y, xv.y, acc[2]);
-        acc[2] = fmaf(dv.z, xv.z, acc[2]); acc[2] = fmaf(dv.w, xv.w, acc[2]);
-        acc[3] += (dv.x + dv.y) + (dv.z + dv.w);
-      } else {
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.x, dv.x);
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.y, dv.y);
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.z, dv.z);
-        accumulate<kMode == 0 ? 2 : 4>(acc, xv.w, dv.w);
-      }
-    }
-  } else {
-    long long items = (long long)N * WH;
-    for (long long i = (long long)rank * kThreads + threadIdx.x; i < items; i += (long long)kCluster * kThreads) {
-      int n = (int)(i / WH);
-      int q = (int)(i - (long long)n * WH);
-      size_t off = ((size_t)n * C + c) * (size_t)WH + q;
-      float xv = x[off];
-      float dv = (kMode != 0) ? dy[off] : 0.f;
-      if (kMode == 2) { acc[2] = fmaf(dv, xv, acc[2]); acc[3] += dv; }
-      else accumulate<kMode == 0 ? 2 : 4>(acc, xv, dv);
-    }
-  }
-
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { for (int j = 0; j < 4; ++j) warpRed[warp][j] = acc[j]; }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    float s = 0.f;
-    for (int w = 0; w < kThreads / 32; ++w) s += warpRed[w][threadIdx.x];
-    part[threadIdx.x] = s;
-  }
-  cluster.sync();
-  if (rank == 0 && threadIdx.x == 0) {
-    float tot[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int r = 0; r < kCluster; ++r) {
-      float const* remote = cluster.map_shared_rank(part, r);
-      for (int j = 0; j < 4; ++j) tot[j] += remote[j];
-    }
-    float mass = (float)((long long)WH * N);
-    float mean, sigma;
-    if (kMode == 2) { mean = momentsIn[c]; sigma = momentsIn[c + C]; }
-    else {
-      // reference bits/nnbnorm.cu:65-70
-      mean = __fdiv_rn(tot[0], mass);
-      float s2 = __fadd_rn(__fdiv_rn(tot[1], mass), -__fmul_rn(mean, mean));
-      s2 = fmaxf(s2, 0.f);
-      sigma = __fsqrt_rn(__fadd_rn(s2, eps));
-      if (momentsOut) { momentsOut[c] = mean; momentsOut[c + C] = sigma; }
-    }
-    if (kMode != 0) {
-      // reference bits/nnbnorm.cu:94-98
-      dbOut[c] = tot[3];
-      dgOut[c] = __fdiv_rn(__fadd_rn(tot[2], -__fmul_rn(mean, tot[3])), sigma);
-    }
-  }
-  cluster.sync();   // keep every CTA's shared memory alive until rank 0 has read it
-}
-
 // Position of a thread in its channel's items (float4s or floats: item i is element i % per of image i / per), moved by a fixed stride without
 // dividing.
 struct Walk {
@@ -149,24 +51,111 @@ struct Walk {
   }
 };
 
-template <int kMode> __device__ __forceinline__ void add_item(float (&acc)[4], float x, float dy)
+// kMode 0: sums of x, x^2.  1: and of dy*x, dy.  2: the latter two alone.  Four values among themselves first.
+__device__ __forceinline__ float sum4(float4 a) { return (a.x + a.y) + (a.z + a.w); }
+__device__ __forceinline__ float dot4(float4 a, float4 b) { return fmaf(a.x, b.x, a.y * b.y) + fmaf(a.z, b.z, a.w * b.w); }
+template <int kMode> __device__ __forceinline__ void add4(float (&acc)[4], float4 x, float4 dy)
 {
-  if (kMode == 2) { acc[2] = fmaf(dy, x, acc[2]); acc[3] += dy; }
-  else accumulate<kMode == 0 ? 2 : 4>(acc, x, dy);
+  if (kMode != 2) { acc[0] += sum4(x); acc[1] += dot4(x, x); }
+  if (kMode != 0) { acc[2] += dot4(dy, x); acc[3] += sum4(dy); }
 }
-template <int kMode> __device__ __forceinline__ void add_item(float (&acc)[4], float4 x, float4 dy)
+
+// The sums over a thread's `mine` items from w on (kVec: float4s).  In steps -- four values, eight items, all -- for with one block per channel a
+// thread has eight times the terms it has with eight, and one running sum over all of them loses the digits that eight blocks keep
+// (28 x 28 x 512 x 64, the mean of inputs around zero: 2.7e-7 off in one sum, 1.4e-7 with eight blocks, 1.3e-7 in steps; the groups of
+// loads that this makes: 60 -> 53 us forward, 82 as before backward).
+template <int kMode, bool kVec>
+__device__ __forceinline__ void sum_items(float (&acc)[4], Walk w, int mine, float const* x, float const* dy)
 {
-  if (kMode == 2) {
-    acc[2] = fmaf(dy.x, x.x, acc[2]); acc[2] = fmaf(dy.y, x.y, acc[2]);
-    acc[2] = fmaf(dy.z, x.z, acc[2]); acc[2] = fmaf(dy.w, x.w, acc[2]);
-    acc[3] += (dy.x + dy.y) + (dy.z + dy.w);
-  } else {
-    accumulate<kMode == 0 ? 2 : 4>(acc, x.x, dy.x);
-    accumulate<kMode == 0 ? 2 : 4>(acc, x.y, dy.y);
-    accumulate<kMode == 0 ? 2 : 4>(acc, x.z, dy.z);
-    accumulate<kMode == 0 ? 2 : 4>(acc, x.w, dy.w);
+  auto eight = [&](auto whole, int left) {
+    float run[4] = {0.f, 0.f, 0.f, 0.f};
+    int k = 0;
+    auto next = [&](auto item, float const* p) {
+      using Item = decltype(item);
+      return decltype(whole)::value || k < left ? *reinterpret_cast<Item const*>(p + w.off) : Item{};
+    };
+    if (kVec) {
+#pragma unroll
+      for (k = 0; k < 8; ++k) {
+        float4 const d = kMode != 0 ? next(float4{}, dy) : float4{};
+        add4<kMode>(run, next(float4{}, x), d);
+        w.move();
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v[4], d[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          k = 4 * h + j;
+          d[j] = kMode != 0 ? next(0.f, dy) : 0.f; v[j] = next(0.f, x);
+          w.move();
+        }
+        add4<kMode>(run, make_float4(v[0], v[1], v[2], v[3]), make_float4(d[0], d[1], d[2], d[3]));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] += run[j];
+  };
+  int left = mine;
+  for (; left >= 8; left -= 8) eight(std::true_type{}, 8);
+  if (left > 0) eight(std::false_type{}, left);
+}
+
+// Moments and derivatives of the parameters (backward pass of the entry point that may not allocate).
+template <bool kVec>
+__global__ void __cluster_dims__(1, kCluster, 1) __launch_bounds__(kThreads)
+bnorm_reduce_kernel(float* __restrict__ momentsOut,   // 2*C
+                    float* __restrict__ dgOut, float* __restrict__ dbOut,
+                    float const* __restrict__ x, float const* __restrict__ dy,
+                    int WH, int C, int N, float eps)
+{
+  vlb::pdl_wait();
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ float part[4];
+  __shared__ float warpRed[kThreads / 32][4];
+  int c = blockIdx.x;
+  int rank = (int)cluster.block_rank();   // the cluster spans grid y
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+
+  // Work items: (image n, chunk of the plane).  Item i of this channel goes to CTA (i / kThreads) % kCluster.
+  int const per = kVec ? WH >> 2 : WH, step = kCluster * kThreads, first = rank * kThreads + (int)threadIdx.x;
+  long long const items = (long long)N * per;
+  int const mine = first < items ? (int)((items - first + step - 1) / step) : 0;
+  sum_items<1, kVec>(acc, Walk(first, step, per, kVec ? 4 : 1, c, C, WH), mine, x, dy);
+
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) { for (int j = 0; j < 4; ++j) warpRed[warp][j] = acc[j]; }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    float s = 0.f;
+    for (int w = 0; w < kThreads / 32; ++w) s += warpRed[w][threadIdx.x];
+    part[threadIdx.x] = s;
   }
+  cluster.sync();
+  if (rank == 0 && threadIdx.x == 0) {
+    float tot[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int r = 0; r < kCluster; ++r) {
+      float const* remote = cluster.map_shared_rank(part, r);
+      for (int j = 0; j < 4; ++j) tot[j] += remote[j];
+    }
+    float mass = (float)((long long)WH * N);
+    // reference bits/nnbnorm.cu:65-70
+    float mean = __fdiv_rn(tot[0], mass);
+    float s2 = __fadd_rn(__fdiv_rn(tot[1], mass), -__fmul_rn(mean, mean));
+    s2 = fmaxf(s2, 0.f);
+    float sigma = __fsqrt_rn(__fadd_rn(s2, eps));
+    momentsOut[c] = mean; momentsOut[c + C] = sigma;
+    // reference bits/nnbnorm.cu:94-98
+    dbOut[c] = tot[3];
+    dgOut[c] = __fdiv_rn(__fadd_rn(tot[2], -__fmul_rn(mean, tot[3])), sigma);
+  }
+  cluster.sync();   // keep every CTA's shared memory alive until rank 0 has read it
 }
+
 // kMode 0: k = {mean, G1, b, -}; else {mean, db/m, G1, G2}
 template <int kMode> __device__ __forceinline__ float apply_item(float x, float dy, float4 k, int relu)
 {
@@ -187,12 +176,14 @@ template <int kMode> __device__ __forceinline__ float4 apply_item(float4 x, floa
 // x and dy once and the result once: 12*m*C bytes backward, 8*m*C forward.  What binds beside the traffic is the two
 // meetings of a cluster, and the issue of instructions: a block must have enough to do between the meetings, and no item divides.
 // Clusters of eight with a 64-bit division per item: 28 x 28 x 512 x 64 took 70 us forward and 89 us backward, x 32 images 43 and 66, 28 x 28 x 128 x 64
-// 21 and 26; now 60 and 83, 22 and 44, 12 and 18 (at copy speed 31 and 47, 16 and 24, 8 and 12).  Holding the items in registers or shared memory between
+// 21 and 26; now 53 and 82, 26 and 43, 14 and 20 (at copy speed 32 and 48, 16 and 24, 8 and 12).  Holding the items in registers or shared memory between
 // the two sweeps was slower: it costs the blocks that hide one another's meetings.
 constexpr int kFusedThreads = 256;
+// Six blocks per SM are asked for where planes are read float by float in the backward pass (48 registers otherwise, five blocks: 55 x 55 x 96 x 16 24.5 us, with
+// six and a few spills 19.3; forward and float4 reads lose 10 to 40% by it).
 // kMode 0: forward, moments computed.  1: backward, moments computed.  2: backward, moments given.
 template <int kMode, bool kVec, int kCl>
-__global__ void __cluster_dims__(1, kCl, 1) __launch_bounds__(kFusedThreads)
+__global__ void __cluster_dims__(1, kCl, 1) __launch_bounds__(kFusedThreads, !kVec && kMode != 0 ? 6 : 0)
 bnorm_fused_kernel(float* __restrict__ out,            // y or dx
                    float* __restrict__ momentsOut,     // 2*C or nullptr
                    float* __restrict__ dgOut, float* __restrict__ dbOut,
@@ -217,15 +208,8 @@ bnorm_fused_kernel(float* __restrict__ out,            // y or dx
   auto dyAt = [&](size_t off) { return *reinterpret_cast<Item const*>(dy + off); };
 
   int const mine = first < items ? (int)((items - first + step - 1) / step) : 0;
-
-  Walk w(first, step, per, kVec ? 4 : 1, c, C, WH);
-  Walk const w0 = w;
-#pragma unroll 8
-  for (int u = 0; u < mine; ++u) {
-    Item const d = kMode != 0 ? dyAt(w.off) : Item{};
-    add_item<kMode>(acc, xAt(w.off), d);
-    w.move();
-  }
+  Walk const w0(first, step, per, kVec ? 4 : 1, c, C, WH);
+  sum_items<kMode, kVec>(acc, w0, mine, x, dy);
 
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -285,9 +269,9 @@ bnorm_fused_kernel(float* __restrict__ out,            // y or dx
   // (rank 0's shared memory has to outlive these reads: the cluster meets once more at the very end, where nobody waits long)
 
   float4 const k = make_float4(k0, k1, k2, k3);
-  w = w0;
+  Walk w = w0;
 #pragma unroll 8
-  for (int u = 0; u < mine; ++u) {
+  for (int i = 0; i < mine; ++i) {
     Item const d = kMode != 0 ? dyAt(w.off) : Item{};
     *reinterpret_cast<Item*>(out + w.off) = apply_item<kMode>(xAt(w.off), d, k, relu);
     w.move();
@@ -409,16 +393,6 @@ int validate(vlb_ctx* ctx, int H, int W, int C, int N)
   VLB_REQUIRE(ctx, H > 0 && W > 0 && C > 0 && N > 0, "bnorm: empty input");
   VLB_REQUIRE(ctx, (long long)H * W * N < (1LL << 31), "bnorm: H*W*N too large");
   return VLB_Success;
-}
-
-template <int kMode>
-void launch_reduce(vlb_ctx* ctx, bool vec, float* momOut, float* dg, float* db, float const* momIn,
-                   float const* x, float const* dy, int WH, int C, int N, float eps)
-{
-  dim3 grid(C, kCluster);
-  if (vec) vlb::launch(ctx->stream, bnorm_reduce_kernel<kMode, true>, grid, kThreads, 0, momOut, dg, db, momIn, x, dy, WH, C, N, eps);
-  else     vlb::launch(ctx->stream, bnorm_reduce_kernel<kMode, false>, grid, kThreads, 0, momOut, dg, db, momIn, x, dy, WH, C, N, eps);
-  VLB_LAUNCHED(ctx, 1);
 }
 
 // Scratch layout (context workspace): [0, 2C) moments when the caller passes none,
@@ -590,8 +564,8 @@ extern "C" int vlb_bnorm_backward_noalloc(void* cudaStream, float* dX, float* dG
   int WH = H * W;
   bool vec = vec_ok(WH, X, dY, dX);
   dim3 grid(C, kCluster);
-  if (vec) vlb::launch(stream, bnorm_reduce_kernel<1, true>, grid, kThreads, 0, mom, dG, dB, nullptr, X, dY, WH, C, N, (float)eps);
-  else     vlb::launch(stream, bnorm_reduce_kernel<1, false>, grid, kThreads, 0, mom, dG, dB, nullptr, X, dY, WH, C, N, (float)eps);
+  if (vec) vlb::launch(stream, bnorm_reduce_kernel<true>, grid, kThreads, 0, mom, dG, dB, X, dY, WH, C, N, (float)eps);
+  else     vlb::launch(stream, bnorm_reduce_kernel<false>, grid, kThreads, 0, mom, dG, dB, X, dY, WH, C, N, (float)eps);
   float mass = (float)((long long)WH * N);
   vlb::launch(stream, bnorm_coef_kernel, vlb::ceil_div(C, 256), 256, 0, cf, mom, g, nullptr, dG, dB, C, mass);
   size_t total = (size_t)WH * C * N;

@@ -30,3 +30,26 @@ def test_bnorm_split(gpu, oracle, plane, c, n):
         assert np.abs(mat.to_numpy(got[i]).ravel() - want[i].ravel()).max() < 1e-4 * np.sqrt(plane[0] * plane[1] * n) * 4
     moments = nn.vl_nnbnorm(xd, gd, bd, dyd, epsilon=eps, moments=mom)
     assert np.abs(mat.to_numpy(moments[0]) - want[0]).max() < 1e-5 * scale
+
+
+@pytest.mark.parametrize("shape", [(28, 28, 512, 64), (27, 27, 512, 48), (112, 112, 64, 32)])
+def test_bnorm_sums_keep_their_digits_however_few_the_blocks(gpu, shape):
+    """The sums of a channel in which one block has 35000 to 50000 terms, or eight have 400000, of inputs around zero, against 64 bits.  A sum of n terms in
+    steps of sizes m_i errs by about 2^-24 / sqrt(3) of the partial sums' own spread per addition: 1.3e-7 of the result in the steps taken
+    (four values, eight items, a thread's items, a warp, a block), and as measured; one running sum per thread errs by 2.2e-7 to 2.9e-7."""
+    import torch
+    nn, mat, _ = gpu
+    c = shape[2]
+    errors = {"mean": [], "dg": [], "dg_given": []}
+    for seed in range(3):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        x, dy = (mat.empty(shape).normal_(generator=g) for _ in range(2))
+        one = mat.zeros((c, 1)) + 1.0
+        _, dg, _, mom = nn.vl_nnbnorm(x, one, one, dy, epsilon=1e-5)
+        dg_given = nn.vl_nnbnorm(x, one, one, dy, epsilon=1e-5, moments=mom)[1]
+        mean, var = x.double().mean(dim=(0, 1, 3)), (x.double() ** 2).mean(dim=(0, 1, 3))
+        want = ((dy.double() * x.double()).sum(dim=(0, 1, 3)) - mean * dy.double().sum(dim=(0, 1, 3))) / (var - mean ** 2 + 1e-5).sqrt()
+        for name, got, ref in (("mean", mom[:, 0], mean), ("dg", dg, want), ("dg_given", dg_given, want)):
+            errors[name].append(float((got.double().reshape(-1) - ref).norm() / ref.norm()))
+    for name, e in errors.items():
+        assert np.mean(e) < 1.8e-7, (name, e)
