@@ -78,10 +78,10 @@ __global__ void lrn_backward_kernel(float* __restrict__ dx, float* __restrict__ 
   }
 }
 
-// L^-beta and 1 / L.  kThreeQuarters: beta = 0.75 (every LRN layer of the reference's model builders), r * sqrt(r) with r = L^-1/2
-// from the hardware's approximation and one Newton step (half a unit in the last place), the square root from the hardware's (relative
-// error 2^-23 by its documentation): two units in the last place together, where powf is documented to keep four, at a fifth of its
-// instructions; 1 / L = r * r.
+// L^-beta and 1 / L.  kThreeQuarters: beta = 0.75 (every LRN layer of the reference's model builders), from the hardware's approximations r of
+// L^-1/2 and s of r^1/2 and their residuals, which fused multiply-adds give exactly: with e = 1 - L r^2 and f = r - s^2 (both of the order of 2^-22)
+// L^-3/4 = r s (1 + 3/4 e) + f s / 2 and 1 / L = r^2 (1 + e) to the order of e^2.  What is left of the power is the rounding of its last addition, nearer
+// than powf (y against 64 bits: 4.1e-8 with powf, 5.9e-8 with one Newton step for r and s as it comes, 3.5e-8 here) at a third of its time.
 struct Powers { float negBeta, inv; };
 
 template <bool kThreeQuarters>
@@ -89,12 +89,15 @@ __device__ __forceinline__ Powers powers_of(float L, float beta)
 {
   Powers w;
   if (!kThreeQuarters) { w.negBeta = powf(L, -beta); w.inv = __fdiv_rn(1.f, L); return w; }
-  float r = rsqrtf(L);
-  float const h = __fmul_rn(L, r), n = fmaf(__fmul_rn(0.5f, r), fmaf(-h, r, 1.f), r);
-  if (h == h) r = n;                       // (L = 0 or infinite: nothing to refine)
-  float q;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(q) : "f"(r));
-  w.negBeta = __fmul_rn(r, q); w.inv = __fmul_rn(r, r);
+  float const r = rsqrtf(L);
+  float s;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(s) : "f"(r));
+  float const u = __fmul_rn(L, r), e = fmaf(-fmaf(L, r, -u), r, fmaf(-u, r, 1.f)), f = fmaf(-s, s, r);
+  float const p = __fmul_rn(r, s), q = __fmul_rn(r, r);
+  float const dp = fmaf(__fmul_rn(0.5f, f), s, fmaf(__fmul_rn(0.75f, e), p, fmaf(r, s, -p)));
+  bool const fine = dp == dp;          // (L = 0 or infinite: nothing to refine)
+  w.negBeta = __fadd_rn(p, fine ? dp : 0.f);
+  w.inv = fmaf(q, fine ? e : 0.f, q);
   return w;
 }
 
@@ -153,28 +156,33 @@ __global__ void __launch_bounds__(128) lrn_backward_window_kernel(float* __restr
   for (int k = 0; k < kD; ++k) { int const c = t0 - m1 - 1 + k; r[k] = c >= 0 && c < p.C ? xp[(size_t)p.P * c] : 0.f; b[k] = 0.f; }
 #pragma unroll
   for (int k = 0; k <= m1; ++k) a[k] = 0.f;
-#pragma unroll 4
-  for (int t = t0; t < c1 + m1; ++t) {
+  auto xAt = [&](int c) { return c < p.C && c >= 0 ? __ldg(xp + (size_t)p.P * c) : 0.f; };
+  auto zAt = [&](int c) { return c < p.C && c >= 0 ? __ldg(zp + (size_t)p.P * c) : 0.f; };
+  // four channels at a time, their loads on the way together (left to the compiler, the power's correction terms cost 30 to 50%: 55x55x96x128 133 us
+  // against 184, 27x27x256x128 93 against 123; with the shorter power of 5.9e-8 the compiler's order took 141 and 81)
+  for (int t4 = t0; t4 < c1 + m1; t4 += 4) {
+    float xn[4], zn[4];
 #pragma unroll
-    for (int k = 0; k + 1 < kD; ++k) { r[k] = r[k + 1]; b[k] = b[k + 1]; }
+    for (int u = 0; u < 4; ++u) { xn[u] = xAt(t4 + u + m2); zn[u] = zAt(t4 + u); }
 #pragma unroll
-    for (int k = 0; k < m1; ++k) a[k] = a[k + 1];
-    r[kD - 1] = t + m2 < p.C && t + m2 >= 0 ? __ldg(xp + (size_t)p.P * (t + m2)) : 0.f;
-    bool const on = t >= 0 && t < p.C;
-    float const z = on ? __ldg(zp + (size_t)p.P * t) : 0.f;
-    float acc = 0.f;
+    for (int u = 0; u < 4; ++u) {
+      int const t = t4 + u, o = t - m1;
 #pragma unroll
-    for (int k = 0; k < kD; ++k) acc = fmaf(r[k], r[k], acc);
-    float const L = p.kappa + p.alpha * acc;
-    Powers const w = powers_of<kThreeQuarters>(L, p.beta);
-    a[m1] = z * w.negBeta;
-    b[kD - 1] = on ? r[m1] * ab2 * a[m1] * w.inv : 0.f;
-    int const o = t - m1;
-    if (o >= c0) {
-      float s = 0.f;
+      for (int k = 0; k + 1 < kD; ++k) { r[k] = r[k + 1]; b[k] = b[k + 1]; }
 #pragma unroll
-      for (int k = 0; k < kD; ++k) s += b[k];
-      dp[(size_t)p.P * o] = p.relu && !(r[0] > 0.f) ? 0.f : a[0] - s * r[0];
+      for (int k = 0; k < m1; ++k) a[k] = a[k + 1];
+      r[kD - 1] = xn[u];
+      float acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < kD; ++k) acc = fmaf(r[k], r[k], acc);
+      float const L = p.kappa + p.alpha * acc;
+      Powers const w = powers_of<kThreeQuarters>(L, p.beta);
+      a[m1] = zn[u] * w.negBeta;
+      b[kD - 1] = t >= 0 && t < p.C ? r[m1] * ab2 * a[m1] * w.inv : 0.f;
+      float sum = 0.f;
+#pragma unroll
+      for (int k = 0; k < kD; ++k) sum += b[k];
+      if (o >= c0 && o < c1) dp[(size_t)p.P * o] = p.relu && !(r[0] > 0.f) ? 0.f : a[0] - sum * r[0];
     }
   }
 }

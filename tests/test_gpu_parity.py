@@ -544,3 +544,38 @@ def test_element_wise_operators_refuse_derivatives_of_another_size(gpu):
             with pytest.raises(ValueError):
                 call()
     assert torch.equal(nn.vl_nnrelu(x, x.reshape(8, 8, 8).permute(0, 1, 2)).reshape(-1), x.reshape(-1))       # (another shape of the same size is taken, as before)
+
+
+@pytest.mark.parametrize("depth", [3, 5, 7, 9])
+def test_lrn_power_is_as_near_as_powf(gpu, depth):
+    """beta = 0.75 against 64 bits, the depths whose windows are summed afresh for every channel (the others slide their sum, whose error grows with the channels).  The power and its product with x, each rounded once: 2^-24 / sqrt(3) / 1.44 (the mean significand) each, 3.4e-8 together,
+    and the window's sum of up to nine squares before them, damped by 0.75: below 4.5e-8 as with powf (4.1e-8), where the approximations without their
+    residuals give 5.9e-8; the derivative has two more factors and a sum.  Zero, infinite and not-a-number windows come out as the formula has them."""
+    import torch
+    import torch.nn.functional as F
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(depth)
+    x, dy = (mat.empty((13, 14, 45, 6)).normal_(generator=g) for _ in range(2))
+    m1 = (depth - 1) // 2
+
+    def exact(x, kappa, alpha):
+        x = x.permute(3, 2, 1, 0).double().requires_grad_()
+        sq = F.pad(x * x, (0, 0, 0, 0, m1, depth - m1 - 1))
+        y = x * (kappa + alpha * sum(sq[:, i:i + 45] for i in range(depth))).pow(-0.75)
+        return x, y
+
+    for kappa, alpha in ((1.0, 0.1), (2.0, 1e-4), (1e-6, 1.0), (1e12, 1e3)):
+        par = [depth, kappa, alpha, 0.75]
+        kappa, alpha = float(torch.tensor(kappa)), float(torch.tensor(alpha))       # as the kernel has them
+        X, Y = exact(x, kappa, alpha)
+        Y.backward(dy.permute(3, 2, 1, 0).double())
+        for got, want, bound in ((nn.vl_nnnormalize(x, par, ctx=ctx), Y.detach(), 6e-8), (nn.vl_nnnormalize(x, par, dy, ctx=ctx), X.grad, 1e-7)):
+            err = float((got.permute(3, 2, 1, 0).double() - want).norm() / want.norm())
+            assert err < (4.5e-8 if kappa == 1.0 and bound == 6e-8 else bound), (kappa, alpha, err)
+    x[2:5, :, 20, :] = float("inf")
+    x[6, :, 11, :] = float("nan")
+    x[8:10] = 0.0
+    for kappa in (0.0, 1.0):
+        want = exact(x, kappa, 0.25)[1].detach()
+        got = nn.vl_nnnormalize(x, [depth, kappa, 0.25, 0.75], ctx=ctx).permute(3, 2, 1, 0).double()
+        assert torch.allclose(got, want, rtol=1e-6, atol=0, equal_nan=True)
