@@ -119,6 +119,8 @@ struct Params {
   // reduction (output pixels of the whole batch, kbTot k-blocks in the dY tile images) is cut into `splits` ranges of kbPerSplit
   // k-blocks, one work item per (range, row tile, column tile); the x runs arrive by tensor-map copies, xStages buffers.
   int wg, cPer, tapsPerTile, tapGroups, kbTot, splits, xStages;
+  int chainShift;         // conv_ts_gen_kernel: 1 << chainShift own k-blocks per accumulation chain
+  int fine;               // conv_ts_kernel, 128-column tiles: chains half as long, small terms first (kFine)
   int biasFirst;          // conv_ts_kernel: a tile's running sum starts at the bias (16-byte loads of it legal, no multiplier, columns in order)
   int smemSum;            // conv_ts_kernel, kMode 0 / 1: keep the running sum of a tile in shared memory even for the tile widths that fit the
                           // drain warps' registers (one short tile per CTA, whose stores all warps share; test switch bit 3)
@@ -809,7 +811,7 @@ constexpr int kTsThreads = (kTsFirstProducer + 4 * kTsGroups) * 32;      // 512:
 constexpr int kTsRunWarp = kTsFirstProducer + 4 * kTsGroups;             // row mode only: warp 16 issues the runs (tensor-map copies)
 constexpr int kTsThreadsRows = (kTsRunWarp + 4) * 32;                    // 640: warp 16's warpgroup is launched whole (warps 17-19 idle), so that it can hand its registers over
 constexpr int kTsBStages = 6;           // at most; Params::bStages are in use
-constexpr int kTsDrainEvery = 4;        // own k-blocks per accumulation chain: 4 x 4 k-steps x 3 MMAs.  Measured relative error of one layer
+constexpr int kTsChainShift = 2;        // 4 own k-blocks per accumulation chain: 4 x 4 k-steps x 3 MMAs.  Measured relative error of one layer
                                         // at the full VGG sizes: 4 -> 9e-7, 8 -> 1.7e-6, 16 -> 3.3e-6 (8 is 5-8% faster, 16 another 0-7%), but with 8
                                         // the end-to-end gradients of the LeNet and ResNet configurations no longer stay within 1e-5
 
@@ -833,13 +835,13 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 { asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(bar), "r"(bytes) : "memory"); }
 
 // Chains of one issuer in a tile of numIter k-blocks: the issuer that owns the tile's first k-block (second = 0) takes
-// the k-blocks 0, 2, ..., the other one (second = 1) the k-blocks 1, 3, ...; a chain is kChain own k-blocks (3xTF32)
+// the k-blocks 0, 2, ..., the other one (second = 1) the k-blocks 1, 3, ...; a chain is 1 << chainShift own k-blocks (3xTF32)
 // or all of them (plain TF32).
-template <bool kSplit, int kChain>
-__device__ __forceinline__ int ts_chains(int numIter, int second)
+template <bool kSplit>
+__device__ __forceinline__ int ts_chains(int numIter, int second, int chainShift)
 {
   int const nOwn = numIter > second ? (numIter - second + 1) / 2 : 0;
-  return kSplit ? (nOwn + kChain - 1) / kChain : (nOwn > 0 ? 1 : 0);
+  return kSplit ? (nOwn + (1 << chainShift) - 1) >> chainShift : (nOwn > 0 ? 1 : 0);
 }
 
 // 4-D tensor-map copy global -> shared (tile mode, one destination CTA; the map covers this GPU's own memory only); completion
@@ -1052,13 +1054,13 @@ static_assert(kTsBStages < kTsDoneRing, "the loader must not be able to fall a w
 // kNarrow: tiles of 64 columns or fewer (kMode 0, 1), which get more accumulators and A stages (below).
 // kGen: the general gather (below) instead of the one that needs whole blocks of 32 channels.  cta, ctas: this CTA's place among
 // those that walk the problem's tiles.
-template <bool kSplit, int kMode, bool kNarrow, bool kGen>
+template <bool kSplit, int kMode, bool kNarrow, bool kGen, bool kFine>
 __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const* xmap, int const cta, int const ctas)
 {
-  // Chains half as long in the general gather: what it computes came from CUDA cores or from chains of large terms alone, and was nearer to the
-  // exact sum than chains of four own k-blocks are (AlexNet's first layer: 4.7e-7 of the output's spread beside a common factor, 3.2e-7 before,
-  // 2.8e-7 with two).  AlexNet batch 128 5.21 -> 5.34 ms, others level.
-  constexpr int kChain = kGen ? 2 : kTsDrainEvery;
+  // kFine: chains half as long (or shorter still), and a k-block's small terms (lo*hi, hi*lo) before its large ones, so that the first of a chain meet an
+  // accumulator that is still small.  For what came from CUDA cores or from chains of large terms alone, which were nearer to the exact sum
+  // than chains of four own k-blocks are.
+  int const chainShift = kGen ? p.chainShift : (kFine ? kTsChainShift - 1 : kTsChainShift);
   constexpr bool kTma = kMode == 1, kWg = kMode == 2;
   extern __shared__ uint8_t smemRaw[];
   __shared__ __align__(8) uint64_t fullA[4], doneK[kTsDoneRing], fullB[kTsBStages], emptyB[kTsBStages];
@@ -1148,7 +1150,7 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
         int const tm = p.dTilesN(tile);
         TileCols const tc = tile_cols<kGen>(p, tile - tm * p.tilesN);
         int const n0 = tc.n0;
-        int const chainsF = ts_chains<kSplit, kChain>(numIter, 0), chainsS = ts_chains<kSplit, kChain>(numIter, 1);   // of the issuer that owns the tile's first k-block, of the other
+        int const chainsF = ts_chains<kSplit>(numIter, 0, chainShift), chainsS = ts_chains<kSplit>(numIter, 1, chainShift);   // of the issuer that owns the tile's first k-block, of the other
         bool fresh = true;                              // P holds nothing of this tile yet
         if (kRegs > 0) {
 #pragma unroll
@@ -1307,7 +1309,7 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
     // Two issuing threads (in two warps, on two schedulers).  The tensor core's queue is about one MMA deep, so
     // while a thread waits on a barrier or commits, nothing of its own is in flight; with two threads the other
     // one's MMAs fill the gap.  Issuer q takes the k-blocks gi = q, q+2, ... (numbered over the CTA's life), which
-    // live in A stage q.  Chains (kChain own k-blocks) take the three T buffers in turn, in the order the
+    // live in A stage q.  Chains (1 << chainShift own k-blocks) take the three T buffers in turn, in the order the
     // drain warps will add them to P, so two chains are being accumulated while the third is drained; the two
     // issuers never touch the same tensor-memory columns, so no ordering between the two streams is needed.
     // Per k-block: one barrier wait (A written and B landed), twelve MMAs, one commit; per chain: a wait for the T
@@ -1328,14 +1330,14 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
       bool const takeTurns = BN > 64 && !kWg;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
         int const first = (int)((((long long)ts * numIter) ^ q) & 1);      // 0: this issuer owns the tile's first k-block
-        int const chainsF = ts_chains<kSplit, kChain>(numIter, 0), chainsS = ts_chains<kSplit, kChain>(numIter, 1);
+        int const chainsF = ts_chains<kSplit>(numIter, 0, chainShift), chainsS = ts_chains<kSplit>(numIter, 1, chainShift);
         for (int it = first, j = 0; it < numIter; it += 2, ++j) {
-          int const inChunk = kSplit ? j % kChain : j;
+          int const inChunk = kSplit ? j & ((1 << chainShift) - 1) : j;
           bool const chunkStart = inChunk == 0;
-          bool const chunkEnd = it + 2 >= numIter || (kSplit && inChunk + 1 == kChain);
+          bool const chunkEnd = it + 2 >= numIter || (kSplit && inChunk + 1 == 1 << chainShift);
           if (chunkStart) {
             // this chain's place in the drain order (first issuer's chain c, second issuer's chain c, first's c+1, ...)
-            int const c = kSplit ? j / kChain : 0;
+            int const c = kSplit ? j >> chainShift : 0;
             g = gBase + min(c, chainsF) + min(c, chainsS) + (first == 1 && c < chainsF ? 1 : 0);
             tAcc = tmemAcc + (uint32_t)((g % kNT) * BN);
             if (g >= kNT) {                           // the chain that sat in this T before must have been added to P
@@ -1361,7 +1363,10 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
 #pragma unroll
           for (int k8 = 0; k8 < BK / 8; ++k8) {
             uint32_t const acc = (chunkStart && k8 == 0) ? 0u : 1u;      // 0 = overwrite: first MMA of a chain
-            if (kSplit) {
+            if (kSplit && kFine) {
+              umma_tf32_ts(tAcc, aLo + 8u * k8, dBh + 2u * k8, idesc, acc);
+              umma_tf32_ts(tAcc, aHi + 8u * k8, dBl + 2u * k8, idesc, 1u);
+            } else if (kSplit) {
               asm volatile(
                   "{\n .reg .pred p0, p1;\n setp.ne.b32 p0, %6, 0;\n setp.eq.b32 p1, %6, %6;\n"
                   " tcgen05.mma.cta_group::1.kind::tf32 [%0], [%2], %3, %5, p0;\n"
@@ -1374,7 +1379,14 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
             // The turn goes to the other issuer before the last MMAs of this k-block are queued: it needs about 200 cycles
             // (three MMAs) to wake up from its wait, and its MMAs, which use another A stage and another accumulator, may
             // queue up behind or between the remaining ones in any order.
-            if (takeTurns && k8 == BK / 8 - 2) mbar_arrive(smem_u32(&turn[q ^ 1]));
+            if (!(kSplit && kFine) && takeTurns && k8 == BK / 8 - 2) mbar_arrive(smem_u32(&turn[q ^ 1]));
+          }
+          if (kSplit && kFine) {
+#pragma unroll
+            for (int k8 = 0; k8 < BK / 8; ++k8) {
+              umma_tf32_ts(tAcc, aHi + 8u * k8, dBh + 2u * k8, idesc, 1u);
+              if (takeTurns && k8 == 0) mbar_arrive(smem_u32(&turn[q ^ 1]));
+            }
           }
           if (!ok) break;
           umma_commit(smem_u32(&doneK[(2u * own + (uint32_t)q) & (uint32_t)(kRing - 1)]));     // when these MMAs are through: the A stage goes back to its producers and (forward, data gradient) the filter stage to the loader
@@ -1727,11 +1739,11 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
   if (warp == kEpilogueWarps) tmem_dealloc(tmemAcc, tmemCols);
 }
 
-template <bool kSplit, int kMode, bool kNarrow>
+template <bool kSplit, int kMode, bool kNarrow, bool kFine = false>
 __global__ void __launch_bounds__(kMode == 2 ? kTsThreadsRows : kTsThreads, 1)
 conv_ts_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap xmap)
 {
-  conv_ts_body<kSplit, kMode, kNarrow, false>(p, &xmap, (int)blockIdx.x, (int)gridDim.x);
+  conv_ts_body<kSplit, kMode, kNarrow, false, kFine>(p, &xmap, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // The same for what the plain kernel's gather does not cover: channels that are no multiple of 32, filter groups, and the residue
@@ -1741,7 +1753,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) conv_ts_gen_kernel(const __grid
 {
   int i = 0;
   while (i + 1 < b.n && (int)blockIdx.x >= b.p[i + 1].ctaBeg) ++i;
-  conv_ts_body<kSplit, 0, kNarrow, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
+  conv_ts_body<kSplit, 0, kNarrow, true, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
 }
 
 // Ft[fh', fw', k, c] = F[FH-1-fh', FW-1-fw', c, k]: the filter bank whose forward convolution
@@ -2129,7 +2141,10 @@ template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<true, true>>() { retu
 template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<true, false>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<false, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<false, false>>() { return 128; }
+template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 0, false, true>>() { return 128; }
+template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 1, false, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 2, false>>() { return 96; }
 
 // The opt-in to more than 48 KB of dynamic shared memory, once per kernel and device instead of before every launch.
@@ -2160,7 +2175,7 @@ int launch_gemm(vlb_ctx* ctx, Params& p, int splits, char const* where)
   if (stages > 6) stages = 6;
   p.stages = stages;
   p.status = ctx->deviceStatus;
-  p.drainEvery = kDrainEvery;
+  if (!p.drainEvery) p.drainEvery = kDrainEvery;
   size_t smemBytes = (size_t)stages * stageBytes + 1024;
   p.tilesM = vlb::ceil_div(p.M, BM);
   dim3 grid(p.tilesM * std::max(p.groups, 1), vlb::ceil_div(p.N, p.BN), splits);
@@ -2312,13 +2327,15 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
     e = allow_large_smem<decltype(kernel)::value>(ctx->device);
     if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, grid, kTsThreads, smemBytes, p, map);
   };
-#define VLB_TS(split, mode, nar) go(std::integral_constant<decltype(&conv_ts_kernel<split, mode, nar>), &conv_ts_kernel<split, mode, nar>>{})
-  if (split3) {
-    if (windows) { if (narrow) VLB_TS(true, 1, true); else VLB_TS(true, 1, false); }
-    else         { if (narrow) VLB_TS(true, 0, true); else VLB_TS(true, 0, false); }
+#define VLB_TS(split, mode, nar, fine) go(std::integral_constant<decltype(&conv_ts_kernel<split, mode, nar, fine>), &conv_ts_kernel<split, mode, nar, fine>>{})
+  if (split3 && p.fine && !narrow) {
+    if (windows) VLB_TS(true, 1, false, true); else VLB_TS(true, 0, false, true);
+  } else if (split3) {
+    if (windows) { if (narrow) VLB_TS(true, 1, true, false); else VLB_TS(true, 1, false, false); }
+    else         { if (narrow) VLB_TS(true, 0, true, false); else VLB_TS(true, 0, false, false); }
   } else {
-    if (windows) { if (narrow) VLB_TS(false, 1, true); else VLB_TS(false, 1, false); }
-    else         { if (narrow) VLB_TS(false, 0, true); else VLB_TS(false, 0, false); }
+    if (windows) { if (narrow) VLB_TS(false, 1, true, false); else VLB_TS(false, 1, false, false); }
+    else         { if (narrow) VLB_TS(false, 0, true, false); else VLB_TS(false, 0, false, false); }
   }
 #undef VLB_TS
   if (record) { cudaEventRecord(rec.stop, ctx->stream); ctx->prof.push_back(rec); }
@@ -2413,13 +2430,13 @@ int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* whe
   if (numTiles >= (1LL << 31)) return VLB_Unsupported;
   dim3 grid((unsigned)std::min<long long>(numTiles, ctx->smCount), 1, 1);
   cudaError_t e;
-  if (split3) {
-    e = allow_large_smem<conv_ts_kernel<true, 2, false>>(ctx->device);
-    if (e == cudaSuccess) vlb::launch(ctx->stream, conv_ts_kernel<true, 2, false>, grid, kTsThreadsRows, smemBytes, p, map);
-  } else {
-    e = allow_large_smem<conv_ts_kernel<false, 2, false>>(ctx->device);
-    if (e == cudaSuccess) vlb::launch(ctx->stream, conv_ts_kernel<false, 2, false>, grid, kTsThreadsRows, smemBytes, p, map);
-  }
+  auto go = [&](auto kernel) {
+    e = allow_large_smem<decltype(kernel)::value>(ctx->device);
+    if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, grid, kTsThreadsRows, smemBytes, p, map);
+  };
+#define VLB_TSR(split, fine) go(std::integral_constant<decltype(&conv_ts_kernel<split, 2, false, fine>), &conv_ts_kernel<split, 2, false, fine>>{})
+  if (!split3) VLB_TSR(false, false); else if (p.fine) VLB_TSR(true, true); else VLB_TSR(true, false);
+#undef VLB_TSR
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, where);
@@ -2507,11 +2524,17 @@ ConvGeom plane_geom(int pixels, int channels, int filters)
 // Each returns -1 when the shape is not eligible (the caller then takes tc_gemm_kernel): rows that are not whole 16-byte pieces, or so little work
 // that the tiles of the second operand are not worth laying out.  V = K = 4096, layout included: forward 107 -> 56 us with 256 images, 56 -> 53 with
 // 128, 50 -> 54 with 64; weights 121 -> 70, 72 -> 45 and 54 -> 41, but K = 1000 with 64 images 17 -> 19.
+// Below kFineV positions the other kernel was the rule, whose chains hold large terms alone; conv_ts_kernel takes such a layer in its fine form,
+// which is no further from the exact sums than that (256 images, forward / weights: 6.4e-7 there, 9.2e-7 in long chains, 3.9e-7 / 3.7e-7 in
+// fine ones, which take 1 to 2% longer).
+constexpr int kFineV = 128 * 64;
+
 int fc_fprop_ts(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float const* F, float const* b)
 {
   int const V = g.FH * g.FW * g.FC;
-  if ((ctx->testSwitch & 4) || V % 32 != 0 || V < (g.N > 128 ? 128 * 16 : 128 * 64) || g.K % 128 != 0 || g.N > 4096 || !aligned16(X) || !aligned16(F)) return -1;
+  if ((ctx->testSwitch & 4) || V % 32 != 0 || V < (g.N > 128 ? 128 * 16 : kFineV) || g.K % 128 != 0 || g.N > 4096 || !aligned16(X) || !aligned16(F)) return -1;
   Params p = {};
+  p.fine = V < kFineV;
   p.cPer = 128; p.tapsPerTile = 1; p.tapGroups = 1;
   p.M = g.K; p.N = g.N; p.R = V;
   p.BN = pick_bn(p.N);
@@ -2573,12 +2596,13 @@ int fc_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, floa
 {
   int const V = g.FH * g.FW * g.FC;
   if ((ctx->testSwitch & 4) || V % 4 != 0 || g.N % 32 != 0 || !aligned16(X) || !aligned16(dY) || V < 128 * 16) return -1;
-  if (V < 128 * 64 && (long long)V * g.K < (1 << 23)) return -1;
+  if (V < kFineV && (long long)V * g.K < (1 << 23)) return -1;
   Params p = {};
   p.M = V; p.N = g.K; p.R = g.N;
   ConvGeom const t = plane_geom(V, g.N, g.K);
   conv_operand(p.a, t, X, g.N);
   p.a.rows = V;
+  p.fine = V < kFineV;
   p.BN = pick_bn(p.N);
   p.numKb = vlb::ceil_div(g.N, BK); p.kbPerSplit = p.numKb; p.splits = 1;
   p.chanFast = 1;
@@ -2609,6 +2633,11 @@ int gen_unit(int C)
 // Filter groups narrower than this (depthwise convolutions) leave a tensor-core tile nearly empty: CUDA cores.
 constexpr int kMinGroupCols = 4;
 
+// Up to this many products an output sums up, the general gather accumulates single k-blocks: the sums of the CUDA-core kernel whose strided and grouped layers
+// it took are off by about 1.7e-8 * sqrt(products), chains of one k-block by 1.4e-7, of two by 3.1 to 3.9e-7.  (Single ones for all: AlexNet's second layer
+// forward 137 -> 146 us, data gradients of its first two layers 239 -> 259 and 271 -> 285; layers with short reductions level to 5% slower.)
+constexpr int kShortReduction = 512;
+
 bool gen_taps_ok(int FH, int FW) { return FH <= 32 && FW <= 32 && FH * FW <= kMaxGenTaps; }
 
 // One contraction of conv_ts_gen_kernel: the stride / pad / dilation geometry t over src, `groups` groups of chPerGroup channels
@@ -2622,6 +2651,7 @@ void gen_problem(Params& p, ConvGeom const& t, float const* src, int chPerGroup,
   p.numKb = vlb::ceil_div(t.FH * t.FW * vlb::ceil_div(chPerGroup, p.unit), p.upk);
   p.BN = BN; p.cols = cols; p.tilesPerGroup = vlb::ceil_div(cols, BN); p.tilesN = groups * p.tilesPerGroup; p.tilesM = vlb::ceil_div(p.M, BM);
   p.splits = 1; p.kbPerSplit = p.kbTot = p.numKb;
+  p.chainShift = p.R < kShortReduction ? 0 : 1;
   p.oy = p.ox = 0; p.oys = p.oxs = 1; p.outH = t.Ho; p.outW = t.Wo; p.shufY = p.shufX = 0; p.outC = cols;
 }
 
@@ -3070,6 +3100,13 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
   int splits = pick_splits(ctx, tiles, p.numKb, 8);
   p.kbPerSplit = ceil_div(p.numKb, splits);
   splits = ceil_div(p.numKb, p.kbPerSplit);
+  if (g.G > 1) {
+    // Chains as short as it takes to be no further from the exact sums than the CUDA-core kernel that had the grouped gradients: that one sums
+    // ranges of `range` pixels, 1.7e-8 * sqrt(range) off; chains of 1, 2, 4 and 8 k-blocks are 1.4, 2.0, 3.2 and 5.8e-7 off.
+    int const simtTiles = ceil_div(V, 64) * ceil_div(g.Kg, 64) * g.G;
+    long long const range = R / std::max(1, ceil_div(2 * ctx->smCount, simtTiles));
+    p.drainEvery = range < 140 ? 1 : range < 400 ? 2 : range < 1250 ? 4 : kDrainEvery;
+  }
   p.e = Epilogue{}; p.e.ldd = V;
   size_t nF = (size_t)V * g.K;
   size_t const partBytes = splits > 1 ? (sizeof(float) * nF * splits + 255) & ~(size_t)255 : 0;

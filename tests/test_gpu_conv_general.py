@@ -148,3 +148,41 @@ def test_data_gradient_of_a_very_long_reduction(gpu):
     want = want[1:5, 1:5]
     assert float((dx[..., 0].double() - want).norm() / want.norm()) < 2e-5
     assert torch.equal(dxm, torch.where(x > 0, dx, torch.zeros_like(dx)))
+
+
+# x, filters, stride, pad, groups, bounds of (y, dx, df), None: not this test's
+NEAR = {
+    "groups_short": ((30, 31, 48, 6), (3, 3, 12, 64), 1, 1, (1.6e-7, 1.6e-7, 2.4e-7)),           # 108 and 144 products
+    "groups_512_products": ((9, 9, 96, 3), (1, 1, 48, 1024), 1, 0, (1.6e-7, 4.2e-7, None)),         # 48; 512: the first two-block chains
+    "groups_511_products": ((9, 9, 14, 3), (1, 1, 7, 1022), 1, 0, (1.6e-7, 1.7e-7, None)),         # 7; 511: the last one-block chains
+    "groups_small_batch": ((13, 13, 384, 1), (3, 3, 192, 384), 1, 1, (4.2e-7, 4.2e-7, 1.6e-7)),       # ranges of 85 pixels
+    "groups_batch_8": ((13, 13, 384, 8), (3, 3, 192, 256), 1, 1, (4.2e-7, 4.2e-7, 3.6e-7)),       # of 451
+    "strided": ((40, 41, 33, 5), (5, 5, 33, 70), 3, 2, (4.2e-7, 1.6e-7, None)),              # 280 and fewer products per class
+    "fc_256_images": ((1, 1, 4096, 256), (1, 1, 4096, 4096), 1, 0, (4.3e-7, None, 4.2e-7)),        # the fine form of the tensor-memory kernel
+    "fc_64_images": ((1, 1, 4096, 64), (1, 1, 4096, 4096), 1, 0, (None, None, 1.6e-7)),
+}
+
+
+@pytest.mark.parametrize("case", sorted(NEAR))
+def test_default_arithmetic_is_as_near_as_the_kernels_before(gpu, case):
+    """Strided and grouped layers came from the CUDA-core kernel (exact products, about 1.7e-8 * sqrt(products) off the exact sums), the fully connected ones from
+    chains of large terms alone (6.4e-7): what took their place is no further off.  Chains of 1, 2 and 4 k-blocks measured 1.4e-7, 3.1 to 3.9e-7
+    (gathered operand in tensor memory) or 2.0 and 3.2e-7 (both in shared memory); the bounds leave a tenth."""
+    import torch
+    import torch.nn.functional as F
+    nn, mat, ctx = gpu
+    ctx.set_precision(0)
+    xs, fs, stride, pad, bounds = NEAR[case]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, f = mat.empty(xs).normal_(generator=g), mat.empty(fs).normal_(0.0, float(np.sqrt(2.0 / np.prod(fs[:3]))), generator=g)
+    X, W = (t.permute(3, 2, 1, 0).double().requires_grad_() for t in (x, f))
+    Y = F.conv2d(X, W, stride=stride, padding=pad, groups=xs[2] // fs[2])
+    y = nn.vl_nnconv(x, f, None, stride=stride, pad=pad, ctx=ctx)
+    dy = mat.empty(tuple(y.shape)).normal_(generator=g)
+    dx, df, _ = nn.vl_nnconv(x, f, None, dy, stride=stride, pad=pad, ctx=ctx)
+    Y.backward(dy.permute(3, 2, 1, 0).double())
+    for got, want, bound, name in zip((y, dx, df), (Y.detach(), X.grad, W.grad), bounds, ("y", "dx", "df")):
+        if bound is not None:
+            err = float((got.permute(3, 2, 1, 0).double() - want).norm() / want.norm())
+            assert err < bound, (name, err)
+    assert ctx.device_status() == 0
