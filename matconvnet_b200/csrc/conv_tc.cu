@@ -2378,12 +2378,16 @@ int pick_wg_splits(int smCount, int tiles, int numKb, int* kbPerSplit, int minKb
 
 // A forward or data-gradient contraction with fewer output tiles than SMs leaves most of the chip idle for the length of its whole reduction
 // (one image through VGG-16's 28 x 28 layers: 28 tiles of 144 k-blocks): its reduction is cut into ranges as the filter gradients' are,
-// and sum_parts adds them and applies the epilogue.  Returns the number of ranges; 1: left alone.
+// and sum_parts adds them and applies the epilogue.  Returns the number of ranges; 1: left alone.  The lines, whole calls on 148 SMs:
+//   tiles       8 of 144 k-blocks 90 -> 26 us, 100 93 -> 88, 124 and 148 level, 172 182 -> 147; of 36 k-blocks 172 53 -> 56.  Above the line
+//               196 of 144 would gain (178 -> 150), of 36 lose (52 -> 55), 224 and more are level.
+//   k-blocks    ranges of fewer than eight keep their sum in shared memory, and two of them cost more than one long reduction: 12 k-blocks in two
+//               ranges 23.1 us, in one 14.1; 18 in three 19.2, in two 14.9, in one 15.3; 16 in two 18.0, in one 19.5.
 int split_few_tiles(int smCount, int tiles, int numKb, int* kbPerSplit)
 {
   *kbPerSplit = numKb;
-  if (tiles * 4 > smCount * 5 || numKb < 12) return 1;
-  return pick_wg_splits(smCount, tiles, numKb, kbPerSplit, 6);
+  if (tiles * 4 > smCount * 5 || numKb < 16) return 1;
+  return pick_wg_splits(smCount, tiles, numKb, kbPerSplit, 8);
 }
 
 void conv_operand(Operand& o, ConvGeom const& g, float const* ptr, int channels)
