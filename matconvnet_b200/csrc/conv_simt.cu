@@ -205,18 +205,6 @@ __global__ void __launch_bounds__(kThreads) igemm_simt_kernel(Op op)
     for (int q = 0; q < 4; ++q) op.store(i0 + tx + 16 * p, j0 + ty + 16 * q, grp, split, acc[p][q]);
 }
 
-// dF[e] = sum over splits (ascending) of partial[s][e]
-__global__ void splitk_reduce_kernel(float* __restrict__ out, float const* __restrict__ part, size_t n, int splits)
-{
-  vlb::pdl_wait();
-  size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    float s = part[e];
-    for (int k = 1; k < splits; ++k) s += part[(size_t)k * n + e];
-    out[e] = s;
-  }
-}
-
 }  // namespace
 
 namespace vlb {
@@ -279,11 +267,8 @@ int conv_wgrad_simt(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, 
   VLB_REQUIRE(ctx, grid.y <= 65535 && grid.z <= 65535, "conv: too many filters or groups");
   vlb::launch(ctx->stream, igemm_simt_kernel<WgradOp>, grid, kThreads, 0, op);
   VLB_LAUNCHED(ctx, 1);
-  if (splits > 1) {
-    vlb::launch(ctx->stream, splitk_reduce_kernel, grid_for(nF, 256, ctx->smCount * 8), 256, 0, dF, op.out, nF, splits);
-    VLB_LAUNCHED(ctx, 1);
-  }
-  return check_launch(ctx, "conv_wgrad_simt");
+  int const rc = check_launch(ctx, "conv_wgrad_simt");
+  return rc || splits == 1 ? rc : sum_parts(ctx, dF, op.out, nF, nF, splits);
 }
 
 }  // namespace vlb

@@ -2312,8 +2312,7 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
   if (numTiles >= (1LL << 31)) return VLB_Unsupported;
   // Persistent: one CTA per SM walks the tiles, so that the pipeline never drains between tiles and a tile is stored
   // while the next one is computed.  With fewer tiles than SMs every CTA has one tile and all its warps share the stores.
-  bool const persistent = true;
-  dim3 grid((unsigned)(persistent && numTiles > ctx->smCount ? ctx->smCount : numTiles), 1, 1);
+  dim3 grid((unsigned)std::min<long long>(numTiles, ctx->smCount), 1, 1);
   cudaError_t e;
   vlb_ctx::ProfRec rec;
   bool const record = ctx->profiling && ctx->profDepth == 0;

@@ -94,8 +94,14 @@ void run(vlb_ctx* ctx, float* Y, float const* X, float const* F, float const* b,
 
 namespace vlb {
 
-// At most 8 images, and enough weights (256 positions per filter) that the passes over them are what counts; two rows per block instead
-// of four where there are too few filters for the chip.
+// At most 8 images and at least 256 positions per filter; two rows per block instead of four where there are too few filters for the chip.  Both sides of
+// the lines, us here / on the tensor cores (K filters of V positions):
+//   V = 25088, K = 4096   one image 64 / 125, two 64 / 125, three 92 / 125, four 95 / 125, five 144 / 125, eight 201 / 125
+//   V = 9216, K = 4096    one 25 / 65, four 35 / 65, five 47 / 65, eight 77 / 65
+//   V = 4096, K = 4096    one 13 / 48, eight 30 / 49;  K = 1000: one 4.8 / 16.6, eight 9.9 / 17.1
+//   V = 256, K = 256      one 1.5 / 12.1, eight 2.0 / 12.2
+//   V = 128, K = 64       one 1.4 / 7.9, eight 1.9 / 8.1 (left to the tensor cores)
+// Five to eight images of the longest rows are slower than they could be, with exact products.
 int fc_fprop_small(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float const* F, float const* b)
 {
   int const V = g.FH * g.FW * g.FC, N = g.N;

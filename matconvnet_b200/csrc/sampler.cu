@@ -119,34 +119,24 @@ __global__ void sampler_kernel(float* __restrict__ y, float* __restrict__ dx, fl
       continue;
     }
     for (int c = 0; c < C; ++c) {
-      if (kMode == 0) {
-        float acc = 0.f;
+      float d = dy[outOff];
+      float dgx = 0.f, dgy = 0.f;
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int ii = 0; ii < 2; ++ii)
-            if (ok[j][ii]) acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(wwx[j], wwy[ii]), xz[idx[j][ii]]));
-        y[outOff] = acc;
-      } else {
-        float d = dy[outOff];
-        float dgx = 0.f, dgy = 0.f;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int ii = 0; ii < 2; ++ii)
-            if (ok[j][ii]) {
-              if (dxz) atomicAdd(dxz + idx[j][ii], __fmul_rn(__fmul_rn(wwx[j], wwy[ii]), d));
-              if (dgrid) {
-                float xv = xz[idx[j][ii]];
-                float sj = j ? 1.f : -1.f, si = ii ? 1.f : -1.f;
-                dgx = __fadd_rn(dgx, __fmul_rn(__fmul_rn(__fmul_rn(sj, wwy[ii]), d), xv));
-                dgy = __fadd_rn(dgy, __fmul_rn(__fmul_rn(__fmul_rn(si, wwx[j]), d), xv));
-              }
+        for (int ii = 0; ii < 2; ++ii)
+          if (ok[j][ii]) {
+            if (dxz) atomicAdd(dxz + idx[j][ii], __fmul_rn(__fmul_rn(wwx[j], wwy[ii]), d));
+            if (dgrid) {
+              float xv = xz[idx[j][ii]];
+              float sj = j ? 1.f : -1.f, si = ii ? 1.f : -1.f;
+              dgx = __fadd_rn(dgx, __fmul_rn(__fmul_rn(__fmul_rn(sj, wwy[ii]), d), xv));
+              dgy = __fadd_rn(dgy, __fmul_rn(__fmul_rn(__fmul_rn(si, wwx[j]), d), xv));
             }
-        if (dgrid) {
-          accGy = __fadd_rn(accGy, __fmul_rn(__fmul_rn(0.5f, (float)(H - 1)), dgy));
-          accGx = __fadd_rn(accGx, __fmul_rn(__fmul_rn(0.5f, (float)(W - 1)), dgx));
-        }
+          }
+      if (dgrid) {
+        accGy = __fadd_rn(accGy, __fmul_rn(__fmul_rn(0.5f, (float)(H - 1)), dgy));
+        accGx = __fadd_rn(accGx, __fmul_rn(__fmul_rn(0.5f, (float)(W - 1)), dgx));
       }
       xz += (size_t)H * W;
       if (dxz) dxz += (size_t)H * W;
