@@ -35,9 +35,15 @@ enum {
 /* Arithmetic of the convolution / fully-connected contractions. */
 enum {
   VLB_PRECISION_3XTF32 = 0, /* tcgen05 kind::tf32, hi/lo split, 3 MMAs per product: fp32-faithful (default) */
-  VLB_PRECISION_TF32 = 1,   /* tcgen05 kind::tf32, single pass: fast path, about 1e-3 relative error */
-  VLB_PRECISION_FP32 = 2    /* CUDA-core FMA implicit GEMM: exact fp32 products, slow; also the path for
-                               strides / dilations / groups the tensor-core kernels do not cover */
+  VLB_PRECISION_TF32 = 1,   /* tcgen05 kind::tf32, single pass: fast path, the operands of every contraction on the tensor
+                               cores rounded to TF32, about 5e-4 relative error -- strided, dilated and grouped layers
+                               and all their gradients included.  Exact products as in the other modes: the direct kernels of a
+                               network's image end (at most 64 inputs per output pixel forward, 27 for the filter gradient,
+                               4 input channels for the data gradient), fully connected forward passes of up to 8 images, and
+                               what FP32 below lists */
+  VLB_PRECISION_FP32 = 2    /* CUDA-core FMA implicit GEMM: exact fp32 products, slow; in every mode also the path for filter
+                               groups of fewer than four channels, strided filters of more than 128 taps, more than 16
+                               residue classes of a strided data gradient and reductions of more than 65535 x 32 */
 };
 
 /* ---- context: replaces vl::Context (bits/data.hpp:150-179) and the stream part of

@@ -123,7 +123,7 @@ __device__ __forceinline__ void solver1(float& w, float& s1, float& s2, float g0
 }
 
 // The update of up to kMaxUpdates parameter tensors in one launch: a network's biases and small filter banks take as long as their
-// launches when each has its own (VGG-16: 32 launches, 565 us; one: 450 us = 6.1 TB/s of the 20 bytes per parameter).  A block takes
+// launches when each has its own (VGG-16: 32 launches, 565 us; one: 404 us = 6.8 TB/s of the 20 bytes per parameter).  A block takes
 // kUpdateChunk consecutive elements of one tensor; a thread loads everything of its four float4s before it stores the first.
 constexpr int kMaxUpdates = 64, kUpdateVecs = 4, kUpdateChunk = kThreads * 4 * kUpdateVecs;
 struct UpdateItem { float *w, *s1, *s2; float const* g; unsigned long long n; float decay, lr; unsigned firstBlock; int vec; };

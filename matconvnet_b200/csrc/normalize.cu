@@ -106,6 +106,7 @@ __device__ __forceinline__ Powers powers_of(float L, float beta)
 // backward passes of AlexNet's two layers at batch 128, 55x55x96 and 27x27x256, 733 MB, went from 912 to 226 us, the forward passes,
 // 489 MB, from 368 to 171 us).  A thread takes `per` consecutive channels of one
 // (pixel, image), kD - 1 more at either end for the windows that reach in: channels are split where there are too few pixels for the chip.
+// (A window is summed afresh, so an infinite or not-a-number value spoils the windows that hold it and not, as in a sliding sum, all channels behind.)
 // At step s the ring x[] holds the channels s - kD + 1 .. s: the window of channel t = s - m2.
 template <int kD, bool kThreeQuarters>
 __global__ void __launch_bounds__(128) lrn_forward_window_kernel(float* __restrict__ y, float const* __restrict__ x, LrnParams p, int per, int segments)
