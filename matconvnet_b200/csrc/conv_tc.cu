@@ -2525,8 +2525,8 @@ ConvGeom plane_geom(int pixels, int channels, int filters)
 //   data      dX(V x N) = F(V x K) dY(K x N): a 1 x 1 convolution over the "plane" of V elements with K channels, dY as its N filters;
 //   weights   dF(V x K) = X(V x N) dY'(N x K): a 1 x 1 convolution over the plane X (N channels) with the K rows of dY as filters.
 // Each returns -1 when the shape is not eligible (the caller then takes tc_gemm_kernel): rows that are not whole 16-byte pieces, or so little work
-// that the tiles of the second operand are not worth laying out.  V = K = 4096, layout included: forward 107 -> 56 us with 256 images, 56 -> 53 with
-// 128, 50 -> 54 with 64; weights 121 -> 70, 72 -> 45 and 54 -> 41, but K = 1000 with 64 images 17 -> 19.
+// that the tiles of the second operand are not worth laying out.  V = K = 4096, layout included: forward 107 -> 57 us with 256 images, 56 -> 53 with
+// 128, 50 -> 54 with 64; weights 121 -> 71, 72 -> 45 and 54 -> 41, but K = 1000 with 64 images 17 -> 19.
 // Below kFineV positions the other kernel was the rule, whose chains hold large terms alone; conv_ts_kernel takes such a layer in its fine form,
 // which is no further from the exact sums than that (256 images, forward / weights: 6.4e-7 there, 9.2e-7 in long chains, 3.9e-7 / 3.7e-7 in
 // fine ones, which take 1 to 2% longer).

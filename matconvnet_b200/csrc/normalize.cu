@@ -103,8 +103,8 @@ __device__ __forceinline__ Powers powers_of(float L, float beta)
 
 // Windows of kD channels, kD small: everything a channel needs is in registers while the thread walks its channels, so x, dz and
 // the result cross memory once and no integral is kept (the form with the integral in scratch moved 2.7 times the bytes: the
-// backward passes of AlexNet's two layers at batch 128, 55x55x96 and 27x27x256, 733 MB, went from 912 to 226 us, the forward passes,
-// 489 MB, from 368 to 171 us).  A thread takes `per` consecutive channels of one
+// backward passes of AlexNet's two layers at batch 128, 55x55x96 and 27x27x256, 733 MB, went from 912 to 227 us, the forward passes,
+// 489 MB, from 368 to 174 us).  A thread takes `per` consecutive channels of one
 // (pixel, image), kD - 1 more at either end for the windows that reach in: channels are split where there are too few pixels for the chip.
 // (A window is summed afresh, so an infinite or not-a-number value spoils the windows that hold it and not, as in a sliding sum, all channels behind.)
 // At step s the ring x[] holds the channels s - kD + 1 .. s: the window of channel t = s - m2.
