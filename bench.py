@@ -153,17 +153,19 @@ def _peaks():
 def contraction_kernels(ctx, passes, peak_tf32):
     """The per-kind sums of the last profile as entries of the bench line's `kernels` list."""
     names = ["conv fprop (conv_ts_kernel; conv1_1 runs on CUDA cores and is not in this sum)",
-             "conv dgrad (conv_ts_kernel, ReLU mask fused)",
-             "conv wgrad + dbias (dY tile images + conv_ts_kernel in its row mode + sum of the reduction ranges; conv1_1 on CUDA cores)",
-             "fully connected fprop/dgrad/wgrad (fc6 on conv_ts_kernel: weights read or written once; fc7, fc8 on tc_gemm_kernel)"]
+             "conv dgrad (dY split into chunks + conv_half_kernel, ReLU mask fused)",
+             "conv wgrad + dbias (x split into chunks, dY tile images, conv_half_kernel, sum of the reduction ranges; conv1_1 on CUDA cores)",
+             "fully connected fprop/dgrad/wgrad (fc6 on conv_ts_kernel and conv_half_kernel: weights read or written once; fc7, fc8 on tc_gemm_kernel)"]
     out = []
     for kind, name in enumerate(names):
         ms, fl, n = ctx.profile_kind(kind)
         if n == 0:
             continue
         tf = fl / (ms * 1e-3) / 1e12 if ms > 0 else 0.0
+        # the backward passes of the convolutions multiply halves (kind::f16, twice kind::tf32's rate); the fully connected layers use both
+        top = 2 * peak_tf32 if kind in (1, 2) else peak_tf32
         out.append({"name": name, "bound": "tensor", "ms_per_step": ms, "contractions": n, "gflop": fl / 1e9, "tflops": tf,
-                    "frac": tf / peak_tf32, "tensor_work_frac": passes * tf / peak_tf32})
+                    "peak": top, "frac": tf / top, "tensor_work_frac": passes * tf / top})
     return out
 
 
@@ -354,11 +356,12 @@ def main():
                 "traffic": None,
                 "traffic_note": "DRAM bytes are captured per kernel on single layers (one kernel, a few launches) and kept under "
                                 "profiles/; no whole-step counter capture is made",
-                "kernel": "conv_ts_kernel (conv fprop / dgrad / wgrad, fc6) + tc_gemm_kernel (fc7, fc8), operand "
+                "kernel": "conv_ts_kernel (conv fprop, fc6), conv_half_kernel (conv dgrad / wgrad, fc6) + tc_gemm_kernel (fc7, fc8), operand "
                           "preparation and the sums over reduction ranges included",
                 "contractions_per_step": tc_count, "ms_per_step": tc_ms, "mma_passes": passes,
                 "tensor_work_frac": passes * achieved / peak, "peak_source": peak_src,
-                "note": "achieved counts each contraction's 2*M*N*K once; the 3xTF32 arithmetic issues 3 MMAs per product"}
+                "note": "achieved counts each contraction's 2*M*N*K once; three MMAs per product, kind::tf32 forward and kind::f16 (twice "
+                        "the rate) in the backward passes of the convolutions; peak is kind::tf32's"}
     kernels = contraction_kernels(ctx, passes, peak)
 
     # ---- the plain-TF32 fast path, reported separately (one MMA per product, about 1e-3 relative error) ----

@@ -77,6 +77,7 @@ int vlb_ctx_set_wait_limit(vlb_ctx* ctx, long long cycles);
  * them delivered by tensor-map copies; the two routes give the same result bit for bit, which is what a test compares.
  * Bit 2: the filter gradient of a convolution takes the kernel with both operands in shared memory even where the
  * tensor-memory kernel applies (the two differ in the order of the sums; a test checks both against the CPU checker).
+ * Bit 4: the filter gradient takes the form with the images along the reduction wherever that is possible, not only where it pays.
  * Bit 3: the tensor-memory convolution kernel keeps the running sum of an output tile in shared memory even for the tile
  * widths (64 and 128 columns) whose sum fits the registers of its drain warps; same additions in the same order, so the
  * results are equal, which is what a test compares. */

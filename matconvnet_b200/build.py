@@ -16,7 +16,7 @@ LIB = os.path.join(HERE, "libvlb.so")
 HOST = os.path.join(HERE, "_hostpath.so")
 
 SOURCES = ["ctx.cu", "elementwise.cu", "normalize.cu", "pool.cu", "bnorm.cu", "roipool.cu", "sampler.cu", "reduce.cu", "fc_small.cu",
-           "conv.cu", "conv_simt.cu", "conv_small.cu", "conv_tc.cu"]
+           "conv.cu", "conv_simt.cu", "conv_small.cu", "conv_tc.cu", "conv_half.cu"]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v"]

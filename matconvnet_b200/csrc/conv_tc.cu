@@ -32,20 +32,10 @@
 //            row k & 3 at 128 bytes, 32-byte chunk q of a row stored at chunk q ^ (k & 3); atom
 //            (ci, kq) at (kq * cols/32 + ci) * 512; LBO = 512 between column atoms, SBO =
 //            cols/32 * 512 between k quads, advance 2 * SBO per MMA.
-#include "conv_internal.cuh"
-#include <cuda.h>
-#include <stdlib.h>
-#include <string.h>
-#include <algorithm>
-#include <type_traits>
+#include "tc_common.cuh"
 
 namespace {
 
-using vlb::ConvGeom;
-using vlb::ProfScope;
-using vlb::kProfFprop; using vlb::kProfDgrad; using vlb::kProfWgrad; using vlb::kProfFc;
-
-constexpr int BM = 128;          // output rows per CTA (TMEM lanes)
 constexpr int BK = 32;           // reduction elements per stage (one 128-byte swizzle row)
 constexpr int kEpilogueWarps = 4;
 constexpr int kProducerWarps = 12;
@@ -58,8 +48,6 @@ constexpr int KSTEP = 32 / CH;                    // MN-major tiles: k rows betw
 constexpr int RSTEP = BM / CH;                    // K-major tiles: rows between a thread's consecutive chunks
 constexpr int kMaxStages = 8;
 constexpr int kDrainEvery = 8;                    // 3xTF32: k-blocks (of 32) accumulated by the tensor core before the fp32 drain
-constexpr long long kWaitCycles = 200000000LL;    // default bound on any single barrier wait (about 0.1 s)
-__constant__ long long gWaitCycles = kWaitCycles; // the bound in force on this device (vlb_ctx_set_wait_limit)
 
 enum OperandMode {
   OP_DENSE_K = 0,    // addr(i, r) = (r / P) * bs + i * ld + (r % P)      (reduction contiguous)
@@ -72,158 +60,6 @@ enum EpilogueMode {
   EPI_PLAIN = 0,     // out[m + n*ldd] (+ bias[m]); with splits: out + split*splitStride
   EPI_CONV = 1       // m = (pixel, image): out[(image*Ktot + n)*P + pixel] = inMult*acc + bias[n] + outMult*old
 };
-
-struct Operand {
-  float const* ptr;
-  long long ld, bs;
-  int P;               // run length of contiguous reduction indices (DENSE_K, batched); 0 = unbatched
-  int rows;            // valid extent of the row (M or N) index
-  int vec;             // 1 when 16-byte loads are legal for this operand
-  int fast;            // gather by tap tables: 1 aligned windows, 2 element-wise (any geometry), 0 filter too large for the tables (IM2COL, WGATHER)
-  // convolution geometry (IM2COL, WGATHER)
-  int H, W, C, FH, FW, Ho, Wo, sy, sx, pt, pl, dy, dx;
-  long long imgStride;   // H*W*Ctotal
-};
-
-struct Epilogue {
-  float* out;
-  float const* bias;
-  long long ldd;
-  long long splitStride;
-  float inMult, outMult;
-  int P, Ktot;
-  int relu;            // apply max(., 0) to the stored value (forward convolution followed by a ReLU layer)
-  float const* mask;   // conv_ts_kernel, when non-null: laid out like out; the stored value is zeroed where mask is not positive
-};
-
-struct Params {
-  Operand a, b;
-  Epilogue e;
-  int M, N, R;
-  int BN;                 // tile columns: 16, 32, 64 or 128
-  int numKb, kbPerSplit;
-  int stages;
-  int drainEvery;         // 3xTF32: k-blocks per tensor-core accumulation chain
-  int tilesM, tilesN;     // conv_ts_kernel: the grid of output tiles its persistent CTAs walk
-  int chanFast;           // conv_ts_kernel: reduction in blocks of 32 channels, r = c%32 + 32*(tap + taps*(c/32)); needs C % 32 == 0
-  float const* bTiles;    // when non-null: B pre-split into shared-memory tile images, fetched with bulk copies
-  int* status;
-  int testSwitch;         // vlb_ctx_set_test_switch: bit 0 = conv_ts_kernel's filter-tile loader stays idle
-  // conv_ts_kernel fed by tensor-map copies (tma != 0): an output tile is a box of bh x bw pixels of one image (tilesH x
-  // tilesW boxes per image); its input window -- boxH rows (rowOff spare rows in front, so that the copy starts on a
-  // 16-byte boundary) x boxW columns x 32 channels -- arrives in shared memory by one cp.async.bulk.tensor per channel block
-  int tma, bh, bw, tilesH, tilesW, boxH, boxW, rowOff;
-  int bStages;            // conv_ts_kernel: filter-tile stages in shared memory (4, or 3 where the input windows need the room)
-  // conv_ts_kernel computing a filter gradient (wg != 0): D[(tap, c)][k] = sum over output pixels of x(pixel + tap, c) * dY(pixel, k).
-  // A tile row is one channel of one filter tap: tapsPerTile taps x cPer channels = 128 rows, tapGroups x C/cPer row tiles; the
-  // reduction (output pixels of the whole batch, kbTot k-blocks in the dY tile images) is cut into `splits` ranges of kbPerSplit
-  // k-blocks, one work item per (range, row tile, column tile); the x runs arrive by tensor-map copies, xStages buffers.
-  int wg, cPer, tapsPerTile, tapGroups, kbTot, splits, xStages;
-  int chainShift;         // conv_ts_gen_kernel: 1 << chainShift own k-blocks per accumulation chain
-  int fine;               // conv_ts_kernel, 128-column tiles: chains half as long, small terms first (kFine)
-  int biasFirst;          // conv_ts_kernel: a tile's running sum starts at the bias (16-byte loads of it legal, no multiplier, columns in order)
-  int smemSum;            // conv_ts_kernel, kMode 0 / 1: keep the running sum of a tile in shared memory even for the tile widths that fit the
-                          // drain warps' registers (one short tile per CTA, whose stores all warps share; test switch bit 3)
-  vlb::FastDiv31 dHo, dWo, dTilesN, dTilesM;      // conv_ts_kernel: by a.Ho, a.Wo, tilesN, tilesM (set by ts_divisors)
-  int plane;              // row mode: reduction indices per image in the tile images -- the plane's pixels rounded up to whole k-blocks
-  // conv_ts_gen_kernel (general gather).  The reduction runs over units of `unit` channels of one filter tap, upk = 32 / unit of
-  // them per k-block: unit number = tap + taps * (channel / unit).  Column tile nt belongs to filter group nt / tilesPerGroup;
-  // a group has `cols` columns and reads a.C channels, aGroup elements further on.  Row (i, j) of an image is the output pixel
-  // (oy + oys * i, ox + oxs * j) of a plane of outH x outW.  shufY > 0: column n of a group is channel n / (shufY * shufX) at the
-  // output pixel moved by (n % shufY, n / shufY % shufX), outC channels per group.  ctaBeg, ctas: the CTAs that walk this problem.
-  int unit, upk, tilesPerGroup, cols;
-  int groups;             // tc_gemm_kernel, filter gradient: filter groups (0 counts as one), M rows and N columns each
-  long long aGroup;
-  int oy, ox, oys, oxs, outH, outW, shufY, shufX, outC, ctaBeg, ctas;
-};
-
-// Several contractions in one launch of conv_ts_gen_kernel (the residue classes of a strided data gradient), each with CTAs of its own.
-constexpr int kMaxTsProblems = 16;
-struct TsProblems { int n; Params p[kMaxTsProblems]; };
-
-// ------------------------------------------------------------------ PTX wrappers
-__device__ __forceinline__ uint32_t smem_u32(void const* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
-{ asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{ asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}" ::"r"(bar) : "memory"); }
-
-// Bounded wait: false when the phase did not complete within gWaitCycles + extra.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long extra = 0)
-{
-  long long t0 = 0;
-  for (uint32_t it = 0;; ++it) {
-    uint32_t ok;
-    // the thread is suspended by the hardware until the phase completes or the time hint (ns) runs out
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(100000u) : "memory");
-    if (ok) return true;
-    if ((it & 15u) == 15u) {
-      long long now = clock64();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > gWaitCycles + extra) return false;
-    }
-  }
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
-{ asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
-
-// Bulk asynchronous copy global -> shared (both 16-byte aligned, size a multiple of 16); completion is
-// signalled on the mbarrier as transaction bytes.  Source is always this GPU's own memory.
-__device__ __forceinline__ void bulk_copy_g2s(uint32_t dstSmem, void const* src, uint32_t bytes, uint32_t bar)
-{
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dstSmem), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc(uint32_t dstSmem, uint32_t cols)
-{
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dstSmem), "r"(cols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols)
-{ asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory"); }
-
-__device__ __forceinline__ void umma_tf32(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t iDesc, uint32_t accumulate)
-{
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}"
-               ::"r"(dTmem), "l"(aDesc), "l"(bDesc), "r"(iDesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar)
-{ asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory"); }
-
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16])
-{
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, uint32_t const (&r)[16])
-{
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                 "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptor (sm_100 format): start address, LBO, SBO in 16-byte
-// units, version 1 at bit 46, layout type at bits 61-63: 2 = 128-byte swizzle (K-major tiles),
-// 1 = 128-byte swizzle with 32-byte base (MN-major tiles of 32-bit elements).
-__device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lboBytes, uint32_t sboBytes, uint32_t layoutType = 2)
-{
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lboBytes >> 4) << 16) | ((uint64_t)(sboBytes >> 4) << 32) |
-         (1ull << 46) | ((uint64_t)layoutType << 61);
-}
 
 // kind::tf32 instruction descriptor: D = F32 (bits 4-5 = 1), A and B = TF32 (bits 7-9, 10-12 = 2),
 // major-ness bits 15 / 16 (1 = MN-major), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
@@ -391,10 +227,6 @@ constexpr int RSTEPG = BM / CHG;                                 // K-major: row
 // wait for it before the paths rejoin) and one destination register per load (two loads that may
 // write the same register are serialised by the scoreboard even when one is predicated off).  Both
 // effects were measured at about 5000 cycles per stage; this form keeps a stage's 32 loads in flight.
-__device__ __forceinline__ void ldg32_if(float& x, float const* a, bool pred)
-{
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p ld.global.nc.f32 %0, [%1];\n}" : "+f"(x) : "l"(a), "r"((int)pred));
-}
 
 // a = address of the window start, o = its alignment (s & 3), g0 / g1 = whether the first / second
 // aligned group of four rows is inside the image; row e of the window lies in the first group iff e < 4 - o.
@@ -831,9 +663,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, uint32_t const (&r)[32
                  "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes)
-{ asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(bar), "r"(bytes) : "memory"); }
-
 // Chains of one issuer in a tile of numIter k-blocks: the issuer that owns the tile's first k-block (second = 0) takes
 // the k-blocks 0, 2, ..., the other one (second = 1) the k-blocks 1, 3, ...; a chain is 1 << chainShift own k-blocks (3xTF32)
 // or all of them (plain TF32).
@@ -842,181 +671,6 @@ __device__ __forceinline__ int ts_chains(int numIter, int second, int chainShift
 {
   int const nOwn = numIter > second ? (numIter - second + 1) / 2 : 0;
   return kSplit ? (nOwn + (1 << chainShift) - 1) >> chainShift : (nOwn > 0 ? 1 : 0);
-}
-
-// 4-D tensor-map copy global -> shared (tile mode, one destination CTA; the map covers this GPU's own memory only); completion
-// is signalled on the mbarrier as transaction bytes.  The innermost coordinate c0 must be a multiple of four elements.
-__device__ __forceinline__ void tma_load_4d(uint32_t dstSmem, void const* map, int c0, int c1, int c2, int c3, uint32_t bar)
-{
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-               ::"r"(dstSmem), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(uint32_t dstSmem, void const* map, int c0, int c1, int c2, uint32_t bar)
-{
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-               ::"r"(dstSmem), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void lds128(uint32_t addr, float (&v)[4])
-{
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(addr));
-}
-
-__device__ __forceinline__ float lds32(uint32_t addr)
-{
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-
-// Bit f is set when position at + f * dilate lies inside [0, extent), f < taps (at most 32).
-__device__ __forceinline__ uint32_t taps_inside(int at, int taps, int dilate, int extent)
-{
-  if (dilate == 1) {
-    int const lo = max(-at, 0), hi = min(extent - at, taps);          // f in [lo, hi)
-    return hi <= lo ? 0u : (0xffffffffu >> (32 - hi)) & (0xffffffffu << lo);
-  }
-  uint32_t m = 0;
-  for (int f = 0; f < taps; ++f) if ((unsigned)(at + f * dilate) < (unsigned)extent) m |= 1u << f;
-  return m;
-}
-
-// Where row `row` (0..127, = TMEM lane) of row tile `tm` lies in the output: image, pixel ho + Ho*wo, and whether it exists.
-// Linear mode: the tile is 128 consecutive output pixels (ho fastest, images following one another).  Box mode (p.tma):
-// the tile is a box of bh x bw pixels of one image, row = dh + bh*dw.
-struct RowPos { int img, pix, split; bool valid; int h, w; };
-
-template <bool kGen>
-__device__ __forceinline__ RowPos row_pos(Params const& p, int tm, int row)
-{
-  RowPos r;
-  r.h = r.w = 0;
-  if (kGen) {
-    r.split = p.dTilesM(tm); tm -= r.split * p.tilesM;
-    int const m = tm * BM + row;
-    r.valid = m < p.M;
-    int const mm = min(m, p.M - 1), t = p.dHo(mm);
-    r.img = p.dWo(t);
-    r.h = p.oy + p.oys * (mm - t * p.a.Ho); r.w = p.ox + p.oxs * (t - r.img * p.a.Wo);
-    r.pix = r.h + p.outH * r.w;
-    return r;
-  }
-  if (p.wg) {
-    // tm = row tile + tilesM * reduction range; row tile = tap group + tapGroups * channel block; row = local tap * cPer + channel.
-    // The "pixel" is the element of dF the row belongs to, fh + FH*(fw + FW*c), plus the offset of the range's partial result.
-    int const split = tm / p.tilesM, t = tm - split * p.tilesM, cb = t / p.tapGroups, tg = t - cb * p.tapGroups;
-    int const tl = row / p.cPer, c = cb * p.cPer + (row - tl * p.cPer), tap = tg * p.tapsPerTile + tl, taps = p.a.FH * p.a.FW;
-    r.valid = tap < taps && c < p.a.C;
-    r.img = 0; r.pix = r.valid ? tap + taps * c : 0; r.split = split;
-    return r;
-  }
-  // tm = row tile + tilesM * reduction range (one range unless the caller cut the reduction)
-  r.split = p.dTilesM(tm); tm -= r.split * p.tilesM;
-  if (!p.tma) {
-    int const m = tm * BM + row;
-    r.valid = m < p.M;
-    int const mm = min(m, p.M - 1);
-    r.img = p.dWo(p.dHo(mm)); r.pix = mm - r.img * p.e.P;          // (a plane is a.Ho x a.Wo pixels)
-  } else {
-    int const per = p.tilesH * p.tilesW;
-    int const n = tm / per, t = tm - n * per, wb = t / p.tilesH, hb = t - wb * p.tilesH;
-    int const dw = row / p.bh, dh = row - dw * p.bh;
-    int const h = hb * p.bh + dh, w = wb * p.bw + dw;
-    r.valid = dw < p.bw && h < p.a.Ho && w < p.a.Wo;
-    r.img = n; r.pix = r.valid ? h + p.a.Ho * w : 0;
-  }
-  return r;
-}
-
-// The columns of column tile nt: the first one among the output's columns, and how many of the tile's columns exist.
-struct TileCols { int n0, cnt, grp; };
-
-template <bool kGen>
-__device__ __forceinline__ TileCols tile_cols(Params const& p, int nt)
-{
-  TileCols c;
-  if (kGen) {
-    c.grp = nt / p.tilesPerGroup;
-    int const local = (nt - c.grp * p.tilesPerGroup) * p.BN;
-    c.n0 = c.grp * p.cols + local; c.cnt = min(p.BN, p.cols - local);
-  } else {
-    c.grp = 0; c.n0 = nt * p.BN; c.cnt = min(p.BN, p.N - c.n0);
-  }
-  return c;
-}
-
-// Where the row of a tile that a thread stores goes.
-struct TsDst { long long at; int row; bool valid; int h, w, img, split; };
-
-template <bool kGen>
-__device__ __forceinline__ TsDst ts_dst(Params const& p, int tm, int row)
-{
-  TsDst d;
-  d.row = row;
-  RowPos const rp = row_pos<kGen>(p, tm, row);
-  d.valid = rp.valid; d.h = rp.h; d.w = rp.w; d.img = rp.img; d.split = rp.split;
-  d.at = (long long)rp.split * p.e.splitStride + (long long)rp.img * p.e.Ktot * p.e.P + rp.pix;
-  return d;
-}
-
-// Epilogue of conv_ts_kernel for what the direct store of the registers does not cover: the columns cBeg .. cBeg + cCnt - 1 of a tile from
-// shared memory, P[column][row]: out[(image*Ktot + n)*P + pixel] = inMult*acc + bias[n] + outMult*old, then ReLU / mask.  Eight columns in flight.
-// masked: the mask has been applied to P already.
-template <bool kGen>
-__device__ __forceinline__ void ts_store_cols(Params const& p, float const* P, TsDst const& d, TileCols const& tc, int cBeg, int cCnt, bool masked)
-{
-  int const nEnd = min(cCnt, tc.cnt - cBeg), n0 = tc.n0 + cBeg;
-  if (!d.valid) return;
-  float* const out = p.e.out + d.at;
-  float const* const mask = masked ? nullptr : p.e.mask;
-  P += d.row;
-  if (kGen && p.shufY > 0) {
-    // column n = moved by (ry, rx), channel c: the pixel is (h + ry, w + rx) where that lies inside the plane
-    int const first = n0 - tc.grp * p.cols, per = p.shufY * p.shufX;
-    int c = first / per, ry = (first - c * per) % p.shufY, rx = (first - c * per) / p.shufY;
-    long long const plane = ((long long)d.img * p.e.Ktot + tc.grp * p.outC) * p.e.P;
-    float* const base = p.e.out + (long long)d.split * p.e.splitStride;
-#pragma unroll 4
-    for (int k = 0; k < nEnd; ++k) {
-      int const h = d.h + ry, w = d.w + rx;
-      if ((unsigned)h < (unsigned)p.outH && (unsigned)w < (unsigned)p.outW) {
-        long long const at = plane + (long long)c * p.e.P + (h + (long long)p.outH * w);
-        float o = P[k * BM] + (p.e.bias ? p.e.bias[tc.grp * p.outC + c] : 0.f);
-        if (mask && !(__ldg(mask + at) > 0.f)) o = 0.f;
-        base[at] = o;
-      }
-      if (++ry == p.shufY) { ry = 0; if (++rx == p.shufX) { rx = 0; ++c; } }
-    }
-    return;
-  }
-  bool const hasBias = p.e.bias != nullptr && !p.biasFirst, hasOld = p.e.outMult != 0.f;
-  float* o0 = out + (long long)n0 * p.e.P;
-  for (int c0 = 0; c0 < nEnd; c0 += 8, o0 += 8LL * p.e.P) {
-    float v[8], b[8], old[8], mk[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { v[i] = P[min(c0 + i, nEnd - 1) * BM] * p.e.inMult; b[i] = 0.f; old[i] = 0.f; mk[i] = 1.f; }
-    if (hasBias) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) b[i] = __ldg(p.e.bias + n0 + min(c0 + i, nEnd - 1));
-    }
-    if (hasOld) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) if (c0 + i < nEnd) old[i] = o0[(long long)i * p.e.P];
-    }
-    if (mask) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) if (c0 + i < nEnd) mk[i] = __ldg(mask + d.at + (long long)(n0 + c0 + i) * p.e.P);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float o = v[i];
-      if (hasBias) o += b[i];
-      if (hasOld) o += p.e.outMult * old[i];
-      if (p.e.relu) o = o > 0.f ? o : 0.f;
-      if (c0 + i < nEnd) o0[(long long)i * p.e.P] = mk[i] > 0.f ? o : 0.f;
-    }
-  }
 }
 
 // kTma: the producers take the input windows from shared memory, where the loader thread has them delivered by tensor-map copies
@@ -1038,7 +692,6 @@ constexpr int kTsXStages = 6;                           // at most
 // was tried first: with six filter stages and four A stages the loader fell a whole phase behind on conv1_2 at batch 64 and then
 // waited for a completion that needed its own copies -- the bounded wait ran out.)
 constexpr int kTsDoneRing = 8;
-constexpr int kMaxGenTaps = 128;                        // of the general gather (11 x 11 filters)
 static_assert(kTsBStages < kTsDoneRing, "the loader must not be able to fall a whole ring behind");
 
 // Registers (kMode 0, 1): 128 per thread at launch (512 threads: the whole register file, one CTA per SM); then the warps 4-7
@@ -1775,29 +1428,6 @@ __global__ void flip_filters_kernel(float* __restrict__ ft, float const* __restr
 // shared-memory tile images -- for n-tile t and k-block kb: [hi tile BN x 32][lo tile BN x 32], K-major with the 128-byte swizzle --
 // so that a stage of B is one bulk copy.  Dense operands here, filter banks below:
 // kRows: B(n, r) = f[n*R + r]; else B(n, r) = f[n + N*r].
-template <bool kSplit, bool kRows>
-__global__ void prep_dense_tiles_kernel(float* __restrict__ out, float const* __restrict__ f, int N, int R, int BN, int numKb)
-{
-  vlb::pdl_wait();
-  size_t const Rp = (size_t)numKb * 32;
-  size_t const total = (size_t)((N + BN - 1) / BN) * BN * Rp;
-  size_t const step = (size_t)gridDim.x * blockDim.x;
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += step) {
-    int const r = (int)(idx % Rp), n = (int)(idx / Rp);
-    float const val = n < N && r < R ? f[kRows ? (size_t)n * R + r : (size_t)r * N + n] : 0.f;
-    int const tile = n / BN, row = n % BN, kb = r >> 5, kk = r & 31;
-    size_t const base = ((size_t)tile * numKb + kb) * (kSplit ? 2 : 1) * (size_t)BN * 32;
-    size_t const off = (size_t)row * 32 + ((((kk >> 2) ^ (row & 7)) << 2) | (kk & 3));
-    if (kSplit) {
-      float hi = tf32_hi(val);
-      out[base + off] = hi;
-      out[base + (size_t)BN * 32 + off] = val - hi;
-    } else {
-      out[base + off] = val;
-    }
-  }
-}
-
 // Filter tile images for conv_ts_kernel and conv_ts_gen_kernel, for the units of channels, filter groups, tap subsets
 // (residue classes of a strided data gradient) and shuffled columns of the general gather.  Row n of a tile is column n of its
 // group; tap (fh', fw') of the problem is tap (bh + ah*fh', bw + aw*fw') of the filter bank, zero where that does not exist; the
@@ -2061,22 +1691,6 @@ size_t b_tiles_bytes(vlb_ctx* ctx, int N, int BN, int numKb)
   return (bytes + 255) & ~(size_t)255;
 }
 
-// `extraBytes` of scratch are reserved behind the tiles for the caller (split-K partials).
-float const* prep_dense_tiles(vlb_ctx* ctx, float const* f, int N, int R, int BN, int numKb, bool rows, size_t extraBytes = 0)
-{
-  bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
-  size_t const total = (size_t)vlb::ceil_div(N, BN) * BN * (size_t)numKb * 32;
-  float* tiles = (float*)vlb::workspace(ctx, b_tiles_bytes(ctx, N, BN, numKb) + extraBytes);
-  if (!tiles) return nullptr;
-  unsigned const grid = vlb::grid_for(total, 256, ctx->smCount * 8);
-#define VLB_PD(split, r) vlb::launch(ctx->stream, prep_dense_tiles_kernel<split, r>, grid, 256, 0, tiles, f, N, R, BN, numKb)
-  if (split3) { if (rows) VLB_PD(true, true); else VLB_PD(true, false); }
-  else        { if (rows) VLB_PD(false, true); else VLB_PD(false, false); }
-#undef VLB_PD
-  VLB_LAUNCHED(ctx, 1);
-  return tiles;
-}
-
 // The filter bank of one group, reduction in blocks of 32 channels (conv_ts_kernel): forward, or flipped and transposed for the data gradient
 // of a stride-1 convolution.
 float const* prep_conv_tiles(vlb_ctx* ctx, float const* f, vlb::ConvGeom const& g, int BN, int numKb, bool dgrad, size_t extraBytes)
@@ -2122,13 +1736,6 @@ float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, i
   return tiles;
 }
 
-// ------------------------------------------------------------------ host side
-int pick_bn(int N) { return N > 64 ? 128 : (N > 32 ? 64 : (N > 16 ? 32 : 16)); }
-
-bool aligned16(void const* p) { return (((uintptr_t)p) & 15) == 0; }
-
-// Registers per thread a kernel must have been compiled with (0: no requirement).
-template <auto kKernel> constexpr int kRegsAtLaunch() { return 0; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 0, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 0, false>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 1, true>>() { return 128; }
@@ -2146,24 +1753,6 @@ template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 1, false, true>>() 
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 2, false>>() { return 96; }
-
-// The opt-in to more than 48 KB of dynamic shared memory, once per kernel and device instead of before every launch.
-template <auto kKernel>
-cudaError_t allow_large_smem(int device)
-{
-  static bool done[64] = {};
-  if (device >= 0 && device < 64 && done[device]) return cudaSuccess;
-  cudaError_t e = vlb::allow_max_dynamic_smem(kKernel);
-  if (e == cudaSuccess && kRegsAtLaunch<kKernel>() > 0) {
-    // conv_ts_kernel redistributes registers between its warps (setmaxnreg) on the premise that every thread starts with
-    // exactly this many; a build that gave it another count must not run (the hand-over would wait for registers for ever)
-    cudaFuncAttributes attr;
-    e = cudaFuncGetAttributes(&attr, kKernel);
-    if (e == cudaSuccess && attr.numRegs != kRegsAtLaunch<kKernel>()) e = cudaErrorInvalidDeviceFunction;
-  }
-  if (e == cudaSuccess && device >= 0 && device < 64) done[device] = true;
-  return e;
-}
 
 template <int kAMode, int kBMode, int kEpi>
 int launch_gemm(vlb_ctx* ctx, Params& p, int splits, char const* where)
@@ -2199,27 +1788,6 @@ int launch_gemm(vlb_ctx* ctx, Params& p, int splits, char const* where)
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, where);
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point query (the library does not link libcuda).
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, cuuint64_t const*, cuuint64_t const*,
-                                  cuuint32_t const*, cuuint32_t const*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled()
-{
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)f;
-    else
-      cudaGetLastError();
-  }
-  return fn;
 }
 
 // Decides whether conv_ts_kernel can take its input windows from tensor-map copies and, if so, fills the box geometry in p,
@@ -2277,14 +1845,6 @@ bool plan_windows(vlb_ctx* ctx, Params& p, CUtensorMap* map, size_t* smemBytes, 
   p.tilesM = (int)(images * p.tilesH * p.tilesW);
   *smemBytes = (size_t)nB * bBytes + pBytes + nX * xTileBytes + 1024;
   return true;
-}
-
-// The multiply-for-division constants of a launch, once its tiling is known: a thread's tile set-up (four divisions, a test per filter row and
-// column) otherwise took the producers 2800 cycles per tile, in which the tensor core runs dry.
-void ts_divisors(Params& p)
-{
-  p.dHo = vlb::FastDiv31(std::max(p.a.Ho, 1)); p.dWo = vlb::FastDiv31(std::max(p.a.Wo, 1));
-  p.dTilesN = vlb::FastDiv31(p.tilesN); p.dTilesM = vlb::FastDiv31(p.tilesM);
 }
 
 // fprop / stride-1 dgrad with the gathered operand in tensor memory (p.bTiles set, p.a a convolution operand).
@@ -2355,58 +1915,6 @@ int pick_splits(vlb_ctx* ctx, int tiles, int numKb, int minKbPerSplit)
   return s < 1 ? 1 : s;
 }
 
-// The cut of a filter gradient's reduction (numKb k-blocks, `tiles` output tiles) into ranges: the work items -- tiles x
-// ranges -- should fill whole waves of the persistent CTAs, with ranges long enough that a tile's fixed cost stays small.
-int pick_wg_splits(int smCount, int tiles, int numKb, int* kbPerSplit, int minKb = 48)
-{
-  int best = 1; double bestEff = 0.0;
-  for (int w = 1; w <= 6; ++w) {
-    int s = std::max(1, (w * smCount) / tiles);
-    s = std::min(s, std::max(1, numKb / minKb));
-    int const per = vlb::ceil_div(numKb, s);
-    s = vlb::ceil_div(numKb, per);
-    long long const items = (long long)tiles * s;
-    long long const perCta = (items + smCount - 1) / smCount;          // items of the busiest CTA
-    // useful k-blocks per SM over the k-block slots the busiest CTA spends, a dozen k-blocks' worth of fixed cost per item
-    double const eff = ((double)tiles * numKb / smCount) / ((double)perCta * (per + 12));
-    if (eff > bestEff * 1.01) { bestEff = eff; best = s; }
-  }
-  *kbPerSplit = vlb::ceil_div(numKb, best);
-  return vlb::ceil_div(numKb, *kbPerSplit);
-}
-
-// A forward or data-gradient contraction with fewer output tiles than SMs leaves most of the chip idle for the length of its whole reduction
-// (one image through VGG-16's 28 x 28 layers: 28 tiles of 144 k-blocks): its reduction is cut into ranges as the filter gradients' are,
-// and sum_parts adds them and applies the epilogue.  Returns the number of ranges; 1: left alone.  The lines, whole calls on 148 SMs:
-//   tiles       8 of 144 k-blocks 90 -> 26 us, 100 93 -> 88, 124 and 148 level, 172 182 -> 147; of 36 k-blocks 172 53 -> 56.  Above the line
-//               196 of 144 would gain (178 -> 150), of 36 lose (52 -> 55), 224 and more are level.
-//   k-blocks    ranges of fewer than eight keep their sum in shared memory, and two of them cost more than one long reduction: 12 k-blocks in two
-//               ranges 23.1 us, in one 14.1; 18 in three 19.2, in two 14.9, in one 15.3; 16 in two 18.0, in one 19.5.
-int split_few_tiles(int smCount, int tiles, int numKb, int* kbPerSplit)
-{
-  *kbPerSplit = numKb;
-  if (tiles * 4 > smCount * 5 || numKb < 16) return 1;
-  return pick_wg_splits(smCount, tiles, numKb, kbPerSplit, 8);
-}
-
-void conv_operand(Operand& o, ConvGeom const& g, float const* ptr, int channels)
-{
-  o.ptr = ptr;
-  o.H = g.H; o.W = g.W; o.C = channels; o.FH = g.FH; o.FW = g.FW; o.Ho = g.Ho; o.Wo = g.Wo;
-  o.sy = g.sy; o.sx = g.sx; o.pt = g.pt; o.pl = g.pl; o.dy = g.dy; o.dx = g.dx;
-  o.imgStride = (long long)g.H * g.W * channels;
-  o.ld = 0; o.bs = 0; o.P = 0; o.vec = 0;
-  // 1: aligned windows (stride 1, extents multiples of 4); 2: element-wise gather, any geometry; 0: the filter does not fit the tap tables
-  bool const lut = g.FH <= 32 && g.FW <= 32 && g.FH * g.FW <= 64;
-  o.fast = !lut ? 0 : ((g.sy == 1 && g.sx == 1 && g.H % 4 == 0 && g.Ho % 4 == 0 && aligned16(ptr)) ? 1 : 2);
-}
-
-bool fits32(ConvGeom const& g)
-{
-  long long in = (long long)g.H * g.W * g.C * g.N, out = (long long)g.Ho * g.Wo * g.K * g.N;
-  return in < (1LL << 31) - 256 && out < (1LL << 31) - 256 && (long long)g.FH * g.FW * g.FC * g.K < (1LL << 31);
-}
-
 // conv_ts_kernel in its row mode (kMode 2): rows whose reduction index is contiguous in memory, delivered by the 3-D tensor map `map`
 // (run of 36 elements x cPer rows x 1).  p holds the tiling (cPer, tapsPerTile, tapGroups, tilesM, tilesN, splits, kbPerSplit,
 // kbTot), the operand geometry, the tile images and the epilogue.
@@ -2445,79 +1953,6 @@ int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* whe
   return vlb::check_launch(ctx, where);
 }
 
-// The 3-D tensor map (run, rows, planes) of launch_rows; false when the driver refuses it.
-bool rows_map(CUtensorMap* map, float const* ptr, long long run, long long rows, long long planes, int cPer)
-{
-  EncodeTiledFn const encode = encode_tiled();
-  if (!encode) return false;
-  memset(map, 0, sizeof(*map));
-  cuuint64_t const dims[3] = {(cuuint64_t)run, (cuuint64_t)rows, (cuuint64_t)planes};
-  cuuint64_t const strides[2] = {(cuuint64_t)run * 4, (cuuint64_t)run * rows * 4};
-  cuuint32_t const box[3] = {(cuuint32_t)kWgRowWords, (cuuint32_t)cPer, 1u};
-  cuuint32_t const estr[3] = {1u, 1u, 1u};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// Filter gradient of a stride-1 convolution whose output has the input's height (every VGG / ResNet 3x3 layer), through
-// conv_ts_kernel: rows (tap, channel) in tensor memory, dY as tile images.  Returns -1 when the layer is not eligible (the
-// caller then takes tc_gemm_kernel), else an error code.
-//   needs: Ho == H (a tap is then a constant shift of the flattened plane), planes of a multiple of four pixels (the 16-byte
-//   strides the tensor map wants) that whole k-blocks cover with at most 1/8 to spare, channels in blocks of 32.
-int conv_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float const* X, float const* dY, bool* dbDone)
-{
-  int const taps = g.FH * g.FW, P = g.Ho * g.Wo, HW = g.H * g.W;
-  if (ctx->testSwitch & 4) return -1;
-  int const Pp = (P + BK - 1) / BK * BK;             // planes are padded to whole k-blocks (at most 1/8 more work: 14 x 14 planes still gain 3% over the other kernel), so that no k-block straddles two images
-  if (g.sy != 1 || g.sx != 1 || g.Ho != g.H || P % 4 != 0 || (Pp - P) * 8 > Pp || HW % 4 != 0 || taps > 64 || g.FH > 32 || g.FW > 32) return -1;
-  if (g.C % 32 != 0 || (g.C > 128 && g.C % 128 != 0) || (g.C < 128 && 128 % g.C != 0)) return -1;
-  if (g.K > 4096 || !aligned16(X) || !aligned16(dY)) return -1;
-  if ((g.FH - 1) * g.dy - g.pt >= g.H || g.pt >= g.H) return -1;
-  int const V = taps * g.C;
-  long long const R = (long long)P * g.N;
-  Params p = {};
-  p.cPer = std::min(g.C, 128); p.tapsPerTile = 128 / p.cPer; p.tapGroups = vlb::ceil_div(taps, p.tapsPerTile);
-  p.M = V; p.N = g.K; p.R = (int)R;
-  p.BN = pick_bn(p.N);
-  p.tilesM = p.tapGroups * (g.C / p.cPer); p.tilesN = vlb::ceil_div(p.N, p.BN);
-  if (vlb::ceil_div(g.K, p.BN) * p.BN > 65535) return -1;
-  if ((long long)Pp * g.N >= (1LL << 31) - 4096) return -1;
-  int const numKb = (int)((long long)Pp * g.N / BK);
-  p.plane = Pp;
-  p.splits = pick_wg_splits(ctx->smCount, p.tilesM * p.tilesN, numKb, &p.kbPerSplit);
-  p.kbTot = p.splits * p.kbPerSplit;               // the tile images are padded with zeros to whole ranges
-  p.numKb = p.kbTot;
-  conv_operand(p.a, g, X, g.C);
-  p.a.rows = V;
-  size_t const nF = (size_t)V * g.K;
-  if ((long long)nF * p.splits >= (1LL << 31)) return -1;
-  size_t const partBytes = p.splits > 1 ? ((sizeof(float) * nF * p.splits + 255) & ~(size_t)255) : 0;
-  size_t const tileBytes = b_tiles_bytes(ctx, g.K, p.BN, p.kbTot);
-  CUtensorMap map;
-  if (!rows_map(&map, X, HW, g.C, g.N, p.cPer)) return -1;
-
-  ProfScope prof(ctx, kProfWgrad);      // includes the dY tile images (with the bias gradient) and the sum of the partial results
-  prof.rec.flops = 2.0 * (double)V * (double)g.K * (double)R;
-  p.bTiles = prep_dy_tiles(ctx, dY, g.K, (int)R, P, p.BN, p.kbTot, partBytes, db, Pp);
-  if (!p.bTiles) return ctx->lastError;
-  *dbDone = db != nullptr;
-  float* const part = p.splits > 1 ? (float*)((char*)p.bTiles + tileBytes) : nullptr;
-  p.e = Epilogue{};
-  p.e.out = part ? part : dF; p.e.splitStride = part ? (long long)nF : 0; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.K;
-  int const rc = launch_rows(ctx, p, map, "conv_wgrad_ts");
-  if (rc) return rc;
-  return part ? vlb::sum_parts(ctx, dF, part, nF, nF, p.splits) : VLB_Success;
-}
-
-// The geometry of a 1 x 1 convolution over a "plane" of `pixels` elements with `channels` channels (channel stride = pixels).
-ConvGeom plane_geom(int pixels, int channels, int filters)
-{
-  ConvGeom t = {};
-  t.H = pixels; t.W = 1; t.C = channels; t.N = 1; t.FH = 1; t.FW = 1; t.FC = channels; t.K = filters; t.Ho = pixels; t.Wo = 1;
-  t.sy = 1; t.sx = 1; t.dy = 1; t.dx = 1; t.G = 1;
-  return t;
-}
-
 // Fully connected layers at small batch are bound by the one pass over the weights (fc6 of VGG-16: 411 MB against 13 GFLOP at
 // batch 64).  All three passes run through conv_ts_kernel, whose A operand goes from global memory to tensor memory without a
 // shared-memory tile of its own, each with the weights (or their gradient) as the operand that is read or written exactly once:
@@ -2527,11 +1962,6 @@ ConvGeom plane_geom(int pixels, int channels, int filters)
 // Each returns -1 when the shape is not eligible (the caller then takes tc_gemm_kernel): rows that are not whole 16-byte pieces, or so little work
 // that the tiles of the second operand are not worth laying out.  V = K = 4096, layout included: forward 107 -> 57 us with 256 images, 56 -> 53 with
 // 128, 50 -> 54 with 64; weights 121 -> 71, 72 -> 45 and 54 -> 41, but K = 1000 with 64 images 17 -> 19.
-// Below kFineV positions the other kernel was the rule, whose chains hold large terms alone; conv_ts_kernel takes such a layer in its fine form,
-// which is no further from the exact sums than that (256 images, forward / weights: 6.4e-7 there, 9.2e-7 in long chains, 3.9e-7 / 3.7e-7 in
-// fine ones, which take 1 to 2% longer).
-constexpr int kFineV = 128 * 64;
-
 int fc_fprop_ts(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float const* F, float const* b)
 {
   int const V = g.FH * g.FW * g.FC;
@@ -2542,7 +1972,7 @@ int fc_fprop_ts(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float
   p.M = g.K; p.N = g.N; p.R = V;
   p.BN = pick_bn(p.N);
   p.tilesM = g.K / 128; p.tilesN = vlb::ceil_div(p.N, p.BN);
-  p.splits = pick_wg_splits(ctx->smCount, p.tilesM * p.tilesN, V / BK, &p.kbPerSplit);
+  p.splits = pick_wg_splits(ctx->smCount, p.tilesM * p.tilesN, V / BK, &p.kbPerSplit, 48);
   p.kbTot = p.splits * p.kbPerSplit; p.numKb = p.kbTot;
   p.plane = V;
   conv_operand(p.a, plane_geom(V, g.K, g.N), F, g.K);
@@ -2550,7 +1980,7 @@ int fc_fprop_ts(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float
   size_t const nOut = (size_t)g.K * g.N;
   size_t const partBytes = p.splits > 1 ? ((sizeof(float) * nOut * p.splits + 255) & ~(size_t)255) : 0;
   CUtensorMap map;
-  if (!rows_map(&map, F, V, g.K, 1, 128)) return -1;
+  if (!rows_map(&map, F, V, g.K, 1, kWgRowWords, 128)) return -1;
   ProfScope prof(ctx, kProfFc);
   prof.rec.flops = 2.0 * (double)g.K * (double)g.N * (double)V;
   p.bTiles = prep_dy_tiles(ctx, X, g.N, V, V, p.BN, p.kbTot, partBytes, nullptr);      // B(n, v) = X[v + V n]
@@ -2566,82 +1996,11 @@ int fc_fprop_ts(vlb_ctx* ctx, ConvGeom const& g, float* Y, float const* X, float
   return vlb::sum_parts(ctx, Y, part, nOut, nOut, p.splits, epi);
 }
 
-int fc_dgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
-{
-  int const V = g.FH * g.FW * g.FC;
-  if ((ctx->testSwitch & 4) || V % 4 != 0 || g.K % 32 != 0 || !aligned16(F) || !aligned16(dY) || V < 128 * 16) return -1;
-  Params p = {};
-  p.M = V; p.N = g.N; p.R = g.K;
-  ConvGeom const t = plane_geom(V, g.K, g.N);
-  conv_operand(p.a, t, F, g.K);
-  p.a.rows = V;
-  p.BN = pick_bn(p.N);
-  int const numKb = vlb::ceil_div(g.K, BK);
-  p.splits = pick_wg_splits(ctx->smCount, vlb::ceil_div(V, BM) * vlb::ceil_div(p.N, p.BN), numKb, &p.kbPerSplit, 16);
-  p.numKb = p.splits * p.kbPerSplit;
-  p.chanFast = 1;
-  size_t const nOut = (size_t)V * g.N;
-  size_t const partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
-  ProfScope prof(ctx, kProfFc);
-  prof.rec.flops = 2.0 * (double)V * (double)g.N * (double)g.K;
-  p.bTiles = prep_dense_tiles(ctx, dY, g.N, g.K, p.BN, p.numKb, true, partBytes);            // B(n, k) = dY[k + K n]
-  if (!p.bTiles) return ctx->lastError;
-  float* const part = p.splits > 1 ? (float*)((char*)p.bTiles + b_tiles_bytes(ctx, g.N, p.BN, p.numKb)) : nullptr;
-  p.e = Epilogue{};
-  p.e.out = part ? part : dX; p.e.splitStride = part ? (long long)nOut : 0; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.N;
-  vlb::SumEpilogue epi;
-  (part ? epi.mask : p.e.mask) = ctx->reluMask; ctx->maskDone = ctx->reluMask != nullptr;
-  int rc = launch_ts(ctx, p, "fc_dgrad_ts");
-  return rc || !part ? rc : vlb::sum_parts(ctx, dX, part, nOut, nOut, p.splits, epi);
-}
-
-int fc_wgrad_ts(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, float const* dY)
-{
-  int const V = g.FH * g.FW * g.FC;
-  if ((ctx->testSwitch & 4) || V % 4 != 0 || g.N % 32 != 0 || !aligned16(X) || !aligned16(dY) || V < 128 * 16) return -1;
-  if (V < kFineV && (long long)V * g.K < (1 << 23)) return -1;
-  Params p = {};
-  p.M = V; p.N = g.K; p.R = g.N;
-  ConvGeom const t = plane_geom(V, g.N, g.K);
-  conv_operand(p.a, t, X, g.N);
-  p.a.rows = V;
-  p.fine = V < kFineV;
-  p.BN = pick_bn(p.N);
-  p.numKb = vlb::ceil_div(g.N, BK); p.kbPerSplit = p.numKb; p.splits = 1;
-  p.chanFast = 1;
-  ProfScope prof(ctx, kProfFc);
-  prof.rec.flops = 2.0 * (double)V * (double)g.K * (double)g.N;
-  p.bTiles = prep_dense_tiles(ctx, dY, g.K, g.N, p.BN, p.numKb, false);                       // B(k, n) = dY[k + K n]
-  if (!p.bTiles) return ctx->lastError;
-  p.e = Epilogue{};
-  p.e.out = dF; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.K;
-  return launch_ts(ctx, p, "fc_wgrad_ts");
-}
-
 // ------------------------------------------------------------------ general gather: host side
-// Channels per unit of the general gather: the least work, counting the gathered zeros (channels rounded up to units; kU = 3 leaves two of
-// a k-block's 32 places empty) and the look-ups of small units (relative cost of a k-block, measured on 56 x 56 maps).
-int gen_unit(int C)
-{
-  static int const unit[] = {32, 16, 8, 4, 3, 1};
-  static double const cost[] = {1.0, 1.03, 1.1, 1.25, 1.35, 2.0};
-  int best = 1; double bestCost = 1e30;
-  for (int i = 0; i < 6; ++i) {
-    double const c = cost[i] * (vlb::ceil_div(C, unit[i]) * unit[i]) * (32.0 / (32 / unit[i] * unit[i])) / C;
-    if (c < bestCost) { bestCost = c; best = unit[i]; }
-  }
-  return best;
-}
-
-// Filter groups narrower than this (depthwise convolutions) leave a tensor-core tile nearly empty: CUDA cores.
-constexpr int kMinGroupCols = 4;
-
 // Up to this many products an output sums up, the general gather accumulates single k-blocks: the sums of the CUDA-core kernel whose strided and grouped layers
 // it took are off by about 1.7e-8 * sqrt(products), chains of one k-block by 1.4e-7, of two by 3.1 to 3.9e-7.  (Single ones for all: AlexNet's second layer
 // forward 137 -> 146 us, data gradients of its first two layers 239 -> 259 and 271 -> 285; layers with short reductions level to 5% slower.)
 constexpr int kShortReduction = 512;
-
-bool gen_taps_ok(int FH, int FW) { return FH <= 32 && FW <= 32 && FH * FW <= kMaxGenTaps; }
 
 // One contraction of conv_ts_gen_kernel: the stride / pad / dilation geometry t over src, `groups` groups of chPerGroup channels
 // and `cols` output columns each.
@@ -2669,13 +2028,6 @@ PrepFilters gen_prep(Params const& p, ConvGeom const& g, float const* f)
   return q;
 }
 
-// Time of a problem's k-blocks in units of a 128-column k-block, for comparing routes: narrower tiles save less than they drop columns.
-double gen_cost(int tiles, int numKb, int BN)
-{
-  double const kb = BN == 128 ? 1.0 : (BN == 64 ? 0.62 : 0.5);
-  return (double)tiles * (numKb + 6) * kb;
-}
-
 // Builds the tile images of all problems (one launch) and runs them (one launch).  The problems share the tile width.
 // Where the problems' tiles are too few for the chip the reductions are cut, all into the same number of ranges, and `fin` (the epilogue,
 // which the problems then do not apply themselves) goes to the sum over the ranges; they cover every element of the output then
@@ -2693,7 +2045,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     long long t = 0, kb = 0;
     for (int i = 0; i < b.n; ++i) { long long const ti = (long long)b.p[i].tilesM * b.p[i].tilesN; t += ti; kb += ti * b.p[i].numKb; }
     int per;
-    if (covered && t < (1 << 20)) splits = split_few_tiles(ctx->smCount, (int)t, (int)(kb / t), &per);
+    if (covered && t < (1 << 20)) splits = split_few_tiles(ctx->smCount, (int)t, (int)(kb / t), &per, 8);
   }
   for (int i = 0; i < b.n; ++i) {
     Params& p = b.p[i];
@@ -2780,121 +2132,6 @@ int conv_fprop_gen(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, flo
   return launch_ts_gen(ctx, ts, prep, Y, (size_t)p.M * g.K, fin, true, "conv_fprop_gen");
 }
 
-// One dimension of a data gradient's residue class: the input positions h with (h + pad) % stride == r, and the filter taps that reach
-// them.  Positions are h0 + stride * i, i < count; tap f0 + step * (taps - 1 - f') of the filter meets position i at output
-// position i + f' * dil - pad: a stride-1 convolution of the output derivative with `taps` taps.
-struct ClassDim { int h0, count, taps, f0, step, dil, pad; };
-
-ClassDim class_dim(int r, int H, int FH, int stride, int pad, int dilate)
-{
-  ClassDim c = {};
-  c.h0 = ((r - pad) % stride + stride) % stride;
-  c.count = c.h0 < H ? (H - 1 - c.h0) / stride + 1 : 0;
-  int a = stride, d = dilate;
-  while (d) { int const t = a % d; a = d; d = t; }                   // a = gcd(stride, dilate)
-  c.step = stride / a; c.dil = dilate / a;
-  c.f0 = -1;
-  for (int f = 0; f < c.step && f < FH; ++f) if ((f * dilate) % stride == r) c.f0 = f;
-  c.taps = c.f0 < 0 ? 0 : (FH - 1 - c.f0) / c.step + 1;
-  // output position of tap f0 + step*j at position h: (h + pad - (f0 + step*j)*dilate) / stride = i + first - j*dil
-  int const first = c.f0 < 0 ? 0 : (c.h0 + pad - c.f0 * dilate) / stride;          // exact: the numerator is a multiple of the stride
-  c.pad = (c.taps - 1) * c.dil - first;
-  return c;
-}
-
-// Data gradient of a strided or grouped convolution, or one whose filters are no multiple of 32, through the general gather.  Two forms:
-//   classes   one problem per residue class of the input pixel modulo the stride, each a stride-1 convolution of dY with the taps that
-//             reach the class: no product with a structural zero, but C columns each;
-//   shuffled  (dilation 1) one problem over the stride-sized blocks of input pixels whose columns are (pixel of the block, channel):
-//             the classes' taps padded to the largest class, C * strideY * strideX columns -- for few channels, whose class
-//             tiles would be mostly empty columns (11 x 11 stride 4 onto 3 channels: one 48-column problem instead of 16 with 3).
-int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
-{
-  int const C = g.FC, nc = g.sy * g.sx;
-  ConvGeom t = g;
-  t.H = g.Ho; t.W = g.Wo; t.N = g.N; t.sy = t.sx = 1;
-  ClassDim ch[kMaxTsProblems], cw[kMaxTsProblems];
-  bool const classesOk = g.sy <= kMaxTsProblems && g.sx <= kMaxTsProblems && nc <= kMaxTsProblems;
-  double classCost = 1e30;
-  bool holes = false;               // classes that no tap reaches: zeros
-  int const unit = gen_unit(g.Kg), upk = 32 / unit;
-  auto kblocks = [&](int taps) { return vlb::ceil_div(taps * vlb::ceil_div(g.Kg, unit), upk); };
-  if (classesOk) {
-    classCost = 0;
-    for (int r = 0; r < g.sy; ++r) ch[r] = class_dim(r, g.H, g.FH, g.sy, g.pt, g.dy);
-    for (int r = 0; r < g.sx; ++r) cw[r] = class_dim(r, g.W, g.FW, g.sx, g.pl, g.dx);
-    int const BN = pick_bn(C);
-    for (int y = 0; y < g.sy; ++y)
-      for (int x = 0; x < g.sx; ++x) {
-        int const taps = ch[y].taps * cw[x].taps, pix = ch[y].count * cw[x].count;
-        if (pix == 0) continue;
-        if (taps == 0) { holes = true; continue; }
-        classCost += gen_cost(vlb::ceil_div((long long)pix * g.N, BM) * g.G * vlb::ceil_div(C, BN), kblocks(taps), BN);
-      }
-  }
-  TsProblems ts = {};
-  PrepBatch prep = {};
-  size_t const nOut = (size_t)g.H * g.W * g.C * g.N;
-  vlb::SumEpilogue fin;
-  fin.mask = ctx->reluMask;
-  fin.bias = ctx->dgradBias; fin.P = g.H * g.W; fin.K = g.C;
-  // shuffled form
-  int const FHm = vlb::ceil_div(g.FH, g.sy), FWm = vlb::ceil_div(g.FW, g.sx);
-  int const iy = g.pt / g.sy, ix = g.pl / g.sx, Hm = (g.H - 1 + g.pt) / g.sy - iy + 1, Wm = (g.W - 1 + g.pl) / g.sx - ix + 1;
-  if (nc > 1 && g.dy == 1 && g.dx == 1 && gen_taps_ok(FHm, FWm)) {
-    int const cols = C * nc, BN = pick_bn(cols);
-    double const cost = gen_cost(vlb::ceil_div((long long)Hm * Wm * g.N, BM) * g.G * vlb::ceil_div(cols, BN), kblocks(FHm * FWm), BN);
-    if (cost < classCost) {
-      t.FH = FHm; t.FW = FWm; t.Ho = Hm; t.Wo = Wm; t.pt = FHm - 1 - iy; t.pl = FWm - 1 - ix;
-      ts.n = 1;
-      Params& p = ts.p[0];
-      gen_problem(p, t, dY, g.Kg, g.G, cols, BN);
-      p.oys = g.sy; p.oxs = g.sx; p.oy = g.sy * iy - g.pt; p.ox = g.sx * ix - g.pl; p.outH = g.H; p.outW = g.W;
-      p.shufY = g.sy; p.shufX = g.sx; p.outC = C;
-      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
-      PrepFilters& q = prep.p[0] = gen_prep(p, g, F);
-      q.bh = g.sy * (FHm - 1); q.ah = -g.sy; q.bw = g.sx * (FWm - 1); q.aw = -g.sx;
-      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
-      int const rc = launch_ts_gen(ctx, ts, prep, dX, nOut, fin, true, "conv_dgrad_gen");
-      if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true; }      // (a refused launch applies neither)
-      return rc;
-    }
-  }
-  if (!classesOk) return VLB_Unsupported;
-  for (int y = 0; y < g.sy; ++y) for (int x = 0; x < g.sx; ++x) if (ch[y].taps * cw[x].taps > 0 && !gen_taps_ok(ch[y].taps, cw[x].taps)) return VLB_Unsupported;
-  if (holes) {
-    cudaError_t const e = cudaMemsetAsync(dX, 0, sizeof(float) * (size_t)g.H * g.W * g.C * g.N, ctx->stream);
-    if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
-  }
-  ts.n = 0;
-  for (int y = 0; y < g.sy; ++y)
-    for (int x = 0; x < g.sx; ++x) {
-      ClassDim const& h = ch[y];
-      ClassDim const& w = cw[x];
-      if (h.taps * w.taps == 0 || h.count * w.count == 0) continue;
-      t.FH = h.taps; t.FW = w.taps; t.Ho = h.count; t.Wo = w.count; t.pt = h.pad; t.pl = w.pad; t.dy = h.dil; t.dx = w.dil;
-      Params& p = ts.p[ts.n];
-      gen_problem(p, t, dY, g.Kg, g.G, C, pick_bn(C));
-      p.oys = g.sy; p.oxs = g.sx; p.oy = h.h0; p.ox = w.h0; p.outH = g.H; p.outW = g.W;
-      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
-      PrepFilters& q = prep.p[ts.n] = gen_prep(p, g, F);
-      q.bh = h.f0 + h.step * (h.taps - 1); q.ah = -h.step; q.bw = w.f0 + w.step * (w.taps - 1); q.aw = -w.step;
-      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
-      ++ts.n;
-    }
-  if (holes) fin.bias = nullptr;                    // (the zeros of the classes without a tap would miss it)
-  // (ts.n == 0: no tap reaches any pixel; all zeros, written above)
-  int const rc = ts.n == 0 ? VLB_Success : launch_ts_gen(ctx, ts, prep, dX, nOut, fin, !holes, "conv_dgrad_gen");
-  if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = !holes; }
-  return rc;
-}
-
-bool is_fc(ConvGeom const& g)
-{
-  return g.Ho == 1 && g.Wo == 1 && g.FH == g.H && g.FW == g.W && g.FC == g.C && g.sy == 1 && g.sx == 1 && g.pt == 0 &&
-         g.pb == 0 && g.pl == 0 && g.pr == 0 && g.dy == 1 && g.dx == 1;
-}
-
 }  // namespace
 
 namespace vlb {
@@ -2960,7 +2197,7 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
   p.e.relu = ctx->fuseRelu; ctx->reluDone = ctx->fuseRelu;
   if (p.a.fast && g.C % 32 == 0) {
     p.chanFast = 1;
-    p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit);
+    p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit, 8);
     p.numKb = p.splits * p.kbPerSplit;
     size_t const nOut = (size_t)p.M * g.K, partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
     p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, false, partBytes);
@@ -2984,7 +2221,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     // dX(V x N) = F(V x K) dY(K x N)  (reference bits/nnfullyconnected.cu:139-151): rows = input elements
     int const V = g.FH * g.FW * g.FC;
     {
-      int const rc = fc_dgrad_ts(ctx, g, dX, F, dY);
+      int const rc = fc_dgrad_half(ctx, g, dX, F, dY);
       if (rc >= 0) return rc;
     }
     ProfScope prof(ctx, kProfFc);
@@ -3019,6 +2256,10 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     prof.rec.flops = 0;
   }
   if (g.G != 1 || g.sy != 1 || g.sx != 1) return VLB_Unsupported;
+  {
+    int const rc = conv_dgrad_half(ctx, g, dX, F, dY);
+    if (rc >= 0) return rc;
+  }
   // dX = conv(dY, flipped and transposed filters) with padding (F-1)*dilate - pad
   ConvGeom t = g;
   t.H = g.Ho; t.W = g.Wo; t.C = g.K; t.FC = g.K; t.K = g.C; t.Ho = g.H; t.Wo = g.W;
@@ -3033,13 +2274,7 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
   p.BN = pick_bn(p.N);
   p.numKb = ceil_div(p.R, BK); p.kbPerSplit = p.numKb;
   p.b = Operand{}; p.b.ld = V; p.b.rows = g.C;
-  if (p.a.fast && g.K % 32 == 0) {
-    p.chanFast = 1;
-    p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit);
-    p.numKb = p.splits * p.kbPerSplit;
-    p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, true, p.splits > 1 ? sizeof(float) * (size_t)p.M * g.C * p.splits : 0);
-    if (!p.bTiles) return ctx->lastError;
-  } else {
+  {
     size_t nF = (size_t)g.FH * g.FW * g.FC * g.K;
     float* ft = (float*)workspace(ctx, sizeof(float) * nF);
     if (!ft) return ctx->lastError;
@@ -3048,17 +2283,6 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
     p.b.ptr = ft; p.b.vec = (V % 4 == 0);
   }
   p.e = Epilogue{}; p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
-  if (p.bTiles) {
-    ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true;
-    if (p.splits == 1) { p.e.mask = ctx->reluMask; p.e.bias = ctx->dgradBias; return launch_ts(ctx, p, "conv_dgrad_ts"); }
-    SumEpilogue epi;
-    epi.mask = ctx->reluMask; epi.bias = ctx->dgradBias; epi.P = p.e.P; epi.K = g.C;
-    size_t const nOut = (size_t)p.M * g.C;
-    float* const part = (float*)((char*)p.bTiles + b_tiles_bytes(ctx, g.C, p.BN, p.numKb));
-    p.e.out = part; p.e.splitStride = (long long)nOut;
-    int const rc = launch_ts(ctx, p, "conv_dgrad_ts");
-    return rc ? rc : sum_parts(ctx, dX, part, nOut, nOut, p.splits, epi);
-  }
   return launch_gemm<OP_IM2COL, OP_DENSE_K, EPI_CONV>(ctx, p, 1, "conv_dgrad_tc");
 }
 
@@ -3071,7 +2295,7 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
   if (is_fc(g)) {
     // dF(V x K) = X(V x N) dY'(N x K)  (reference bits/nnfullyconnected.cu:126-137): reduction over the batch
     {
-      int const rc = fc_wgrad_ts(ctx, g, dF, X, dY);
+      int const rc = fc_wgrad_half(ctx, g, dF, X, dY);
       if (rc >= 0) return rc;
     }
     ProfScope prof(ctx, kProfFc);
@@ -3084,8 +2308,8 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
     p.e = Epilogue{}; p.e.out = dF; p.e.ldd = V;
     return launch_gemm<OP_DENSE_MN, OP_DENSE_MN, EPI_PLAIN>(ctx, p, 1, "fc_wgrad_tc");
   }
-  if (g.G == 1) {
-    int const rc = conv_wgrad_ts(ctx, g, dF, db, X, dY, dbDone);
+  {
+    int const rc = conv_wgrad_half(ctx, g, dF, db, X, dY, dbDone);
     if (rc >= 0) return rc;
   }
   long long R = (long long)g.Ho * g.Wo * g.N;
@@ -3138,6 +2362,7 @@ extern "C" int vlb_ctx_set_wait_limit(vlb_ctx* ctx, long long cycles)
   long long const v = cycles == 0 ? kWaitCycles : cycles;
   // ordered behind the kernels already enqueued on the context's stream, which keep the limit they were launched under
   cudaError_t e = cudaMemcpyToSymbolAsync(gWaitCycles, &v, sizeof(v), 0, cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = vlb::half_set_wait_limit(cycles, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   return VLB_Success;

@@ -1,0 +1,145 @@
+"""Backward contractions on scaled half-precision operands (conv_half.cu): data gradients of split chunks, filter gradients with the images
+along the reduction, both against float64, and what the powers of two have to keep: any magnitude, infinities in their own column or pixel.
+
+Bound: an operand is off by 2^-22 of itself at most, a product by 2^-21, an fp32 sum of a k-block's 12 MMAs by about 2^-21 of itself; random signs leave
+1.2e-7 to 6e-7 of the result's norm at every size measured, 1e-6 is asked for.  VLB_PRECISION_TF32 rounds the operands to 11 bits (2^-12 each on average
+half of that): 2.4e-4, 5e-4 is asked for.  A filter gradient too small for these kernels comes from tc_gemm_kernel, whose plain TF32 operands are cut off
+instead of rounded: each is 0 to 2^-10 of itself too small, 3.6e-4 on average (the mean of 2^-11 / mantissa), the product twice that, all in one direction; 1e-3
+is asked for there."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (H, W, C, N), (FH, FW, C/G, K), stride, pad, dilate
+CASES = [((16, 16, 64, 8), (3, 3, 64, 64), 1, 1, 1),           # one block of 64 channels, 64 columns
+         ((16, 16, 64, 8), (3, 3, 64, 16), 1, 1, 1),           # 16 filters: 16 of 64 places of a k-block
+         ((9, 11, 65, 16), (3, 3, 65, 129), 1, 1, 1),          # one more than a block of channels, than a column tile
+         ((8, 7, 128, 64), (3, 3, 128, 128), 1, 1, 1),         # whole tiles; 64 images: one pixel per k-block
+         ((13, 13, 48, 70), (5, 5, 24, 96), 1, 2, 1),          # two filter groups, six images more than a group of 64
+         ((14, 10, 96, 33), (3, 3, 96, 43), 2, 1, 1),          # stride 2; 43 channels filled up to 64
+         ((12, 9, 32, 13), (3, 3, 32, 200), 1, 2, 2),          # dilation; 13 images: groups of eight
+         ((7, 5, 70, 5), (1, 1, 70, 300), 1, 0, 1),            # 1x1, three column tiles
+         ((6, 31, 40, 24), (3, 2, 40, 80), (1, 3), (0, 1, 1, 0), 1),
+         ((4, 4, 512, 3), (3, 3, 512, 512), 1, 1, 1)]          # few tiles, long reduction: cut into ranges
+
+
+def reference(x, f, dy, stride, pad, dilate):
+    import torch
+    import torch.nn.functional as F
+    st = (stride, stride) if np.isscalar(stride) else stride
+    p = (pad,) * 4 if np.isscalar(pad) else pad
+    groups = x.shape[2] // f.shape[2]
+    X, W = (t.permute(3, 2, 1, 0).double().requires_grad_() for t in (x, f))
+    # (image, channel, column, row): torch's last dimension is the row here
+    Y = F.conv2d(F.pad(X, p), W, stride=(st[1], st[0]), dilation=dilate, groups=groups)
+    if dy is None:
+        return tuple(Y.permute(3, 2, 1, 0).shape)
+    Y.backward(dy.permute(3, 2, 1, 0).double())
+    return X.grad.permute(3, 2, 1, 0), W.grad.permute(3, 2, 1, 0), dy.double().sum((0, 1, 3))
+
+
+def inputs(mat, case):
+    import torch
+    xs, fs, stride, pad, dilate = CASES[case]
+    g = torch.Generator(device="cuda").manual_seed(500 + case)
+    x, f = mat.empty(xs).normal_(generator=g), mat.empty(fs).normal_(0.0, float((2.0 / np.prod(fs[:3])) ** 0.5), generator=g)
+    dy = mat.empty(reference(x, f, None, stride, pad, dilate)).normal_(generator=g)
+    return x, f, dy, dict(stride=stride, pad=pad, dilate=dilate)
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("precision,bound", [(0, 1e-6), (1, 5e-4)])
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_gradients_against_float64(gpu, case, precision, bound):
+    import torch
+    nn, mat, ctx = gpu
+    x, f, dy, kw = inputs(mat, case)
+    b = mat.zeros((1, f.shape[3]))
+    dxr, dfr, dbr = reference(x, f, dy, **kw)
+    ctx.set_precision(precision)
+    lib = ctx.lib
+    try:
+        for switch in (0, 16):              # 16: the images along the reduction wherever they can be
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            dx, df, db = nn.vl_nnconv(x, f, b, dy, ctx=ctx, **kw)
+            again = nn.vl_nnconv(x, f, b, dy, ctx=ctx, **kw)
+            assert ctx.device_status() == 0
+            assert rel(dx, dxr) < bound and rel(db.reshape(-1), dbr) < 1e-6, switch
+            assert rel(df, dfr) < (1e-3 if precision == 1 and switch == 0 else bound), switch
+            assert all(torch.equal(a, c) for a, c in zip((dx, df, db), again))          # run to run identical
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+        ctx.set_precision(0)
+
+
+@pytest.mark.parametrize("case", [0, 2, 3, 5])
+@pytest.mark.parametrize("ex,ef,ed", [(40, -30, 20), (-60, 0, 50), (0, -20, -80), (70, 10, 30)])
+def test_powers_of_two_change_nothing_but_the_scale(gpu, case, ex, ef, ed):
+    """Operands times powers of two: the result times their product, bit for bit (as long as it has a normal exponent) -- also where the factor of a k-block has not."""
+    import torch
+    nn, mat, ctx = gpu
+    x, f, dy, kw = inputs(mat, case)
+    lib = ctx.lib
+    try:
+        for switch in (0, 16):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            dx, df, _ = nn.vl_nnconv(x, f, None, dy, ctx=ctx, **kw)
+            dx2, df2, _ = nn.vl_nnconv(mat.as_mat(x * 2.0 ** ex), mat.as_mat(f * 2.0 ** ef), None, mat.as_mat(dy * 2.0 ** ed), ctx=ctx, **kw)
+            small = 2.0 ** -10                # (what is left where a sum almost cancels may be subnormal on the way when scaled)
+            for a, c, e in ((dx, dx2, ef + ed), (df, df2, ex + ed)):
+                keep = a.abs() > small
+                assert torch.equal((a.double() * 2.0 ** e)[keep], c.double()[keep]), (switch, e)
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+
+
+@pytest.mark.parametrize("case", [0, 3, 6])
+def test_values_that_are_not_finite_stay_where_they_are(gpu, case):
+    import torch
+    nn, mat, ctx = gpu
+    x, f, dy, kw = inputs(mat, case)
+    lib = ctx.lib
+    try:
+        for switch in (0, 16):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            dx, df, _ = nn.vl_nnconv(x, f, None, dy, ctx=ctx, **kw)
+            # a filter bank with an infinity in one channel: that channel's derivative only
+            f2 = f.clone()
+            f2[0, 0, 3, 1] = float("inf")
+            dxf, _, _ = nn.vl_nnconv(x, mat.as_mat(f2), None, dy, no_der_filters=True, ctx=ctx, **kw)
+            assert not torch.isfinite(dxf[:, :, 3]).all()
+            other = [c for c in range(x.shape[2]) if c != 3]
+            assert torch.equal(dxf[:, :, other], dx[:, :, other])
+            # a derivative that is not a number: its filter's gradient only; the pixels it reaches only
+            dy2 = dy.clone()
+            dy2[2, 2, 5, 1] = float("nan")
+            dxd, dfd, _ = nn.vl_nnconv(x, f, None, mat.as_mat(dy2), ctx=ctx, **kw)
+            other = [k for k in range(f.shape[3]) if k != 5]
+            assert torch.isnan(dfd[:, :, :, 5]).any() and torch.equal(dfd[:, :, :, other], df[:, :, :, other])
+            assert torch.isnan(dxd[:, :, :, 1]).any() and torch.equal(dxd[:, :, :, 0], dx[:, :, :, 0])
+            # an input that is infinite: its channel's rows only
+            x2 = x.clone()
+            x2[1, 1, 7, 0] = float("inf")
+            _, dfx, _ = nn.vl_nnconv(mat.as_mat(x2), f, None, dy, no_der_data=True, ctx=ctx, **kw)
+            other = [c for c in range(x.shape[2]) if c != 7]
+            assert not torch.isfinite(dfx[:, :, 7]).all() and torch.equal(dfx[:, :, other], df[:, :, other])
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+
+
+def test_an_odd_number_of_run_buffers_keeps_the_groups_apart(gpu):
+    """128-column tiles of the row mode have three run buffers for two groups of producers: a buffer's previous run belongs to the other group.  A group that
+    did not wait for it to be let go of took a run of three k-blocks before for its own, once in some thousand launches."""
+    import torch
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(77)
+    x, f, dy = mat.empty((28, 28, 512, 16)).normal_(generator=g), mat.empty((1, 1, 512, 128)).normal_(generator=g), mat.empty((28, 28, 128, 16)).normal_(generator=g)
+    _, first, _ = nn.vl_nnconv(x, f, None, dy, no_der_data=True, ctx=ctx)
+    for _ in range(500):
+        _, df, _ = nn.vl_nnconv(x, f, None, dy, no_der_data=True, ctx=ctx)
+        assert torch.equal(df, first)
+    assert ctx.device_status() == 0
