@@ -992,8 +992,14 @@ split_images_kernel(uint4* __restrict__ hi, long long loOff, int8_t* __restrict_
     if (c >= C || pix >= HW) return;
     float const* const src = x + ((long long)ng * 64 * C + c) * HW + pix;
     float v[64];
+    long long const step = (long long)C * HW;
+    if (ng * 64 + 64 <= N) {
 #pragma unroll
-    for (int k = 0; k < 64; ++k) v[k] = ng * 64 + k < N ? __ldg(src + (long long)k * C * HW) : 0.f;
+      for (int k = 0; k < 64; ++k) v[k] = __ldg(src + k * step);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 64; ++k) v[k] = ng * 64 + k < N ? __ldg(src + k * step) : 0.f;
+    }
     float m0 = 0.f, m1 = 0.f;
 #pragma unroll
     for (int k = 0; k < 64; k += 4) { m0 = max3(m0, fabsf(v[k]), fabsf(v[k + 1])); m1 = max3(m1, fabsf(v[k + 2]), fabsf(v[k + 3])); }
@@ -1057,13 +1063,14 @@ split_images_kernel(uint4* __restrict__ hi, long long loOff, int8_t* __restrict_
 // dY of such a filter gradient as tile images, and the bias gradient from the same sweep.  A block takes 32 filters of a column tile and octets -- eight
 // consecutive rows of an output column, the 8 * kG images of a group: kG k-blocks -- one after the other; a thread has one row and filter of it in registers
 // (64 values with kG = 8), so that dY is read once.  32 columns of a k-block therefore share an exponent here, not all of the tile's; the drain warps, who
-// take 32 columns at a time, have one for each.  (A block of all 128 columns, reading an octet a second time from L2: 196 us for 103 MB, now 44.)
+// take 32 columns at a time, have one for each.  (A block of all 128 columns, reading an octet a second time from L2: 196 us for 103 MB, now 55; a range of
+// octets of its own per block 61; every octet inside one column 76; every place's image number and magnitude tested by itself 93.)
 // A filter's sum: in double over a thread's octets, then over the rows, then (last ticket) over the blocks in block order.
-// grid (ranges of octets, blocks of 32 filters of the column tiles of all filter groups)
+// grid (octets dealt out in turn, blocks of 32 filters of the column tiles of all filter groups)
 template <bool kSplit, int kG>
 __global__ void __launch_bounds__(256, kG == 8 ? 2 : 3)
 prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int Wo, int N, int K, int Kg, int tilesPerGroup, int BN, int nGroups, int rowBlocks, int kbTot,
-                        int octets, int per, float* __restrict__ db, float* __restrict__ dbPart, unsigned* __restrict__ tickets)
+                        int octets, float* __restrict__ db, float* __restrict__ dbPart, unsigned* __restrict__ tickets)
 {
   vlb::pdl_wait();
   constexpr int kRows = 8 / kG;                         // rows of a k-block
@@ -1078,27 +1085,42 @@ prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int W
   long long const imgStep = (long long)K * P;
   float const* const mine = dy + (long long)(real ? fg * Kg + local : 0) * P;
   double acc = 0.0;
-  int const oBeg = (int)blockIdx.x * per, oEnd = min(octets, oBeg + per);
-  for (int o = oBeg; o < oEnd; ++o) {
+  // (blocks that run at the same time take neighbouring octets: with a range of its own for each, 64 images far apart times hundreds of places are more
+  // pages than the address translation holds)
+  int turn = 0;
+  for (int o = (int)blockIdx.x; o < octets; o += (int)gridDim.x, turn ^= 1) {
     int const col = o / perCol, h8 = o - col * perCol, ng = col / Wo, w = col - ng * Wo, h = h8 * 8 + px;
     int const kbAt = h8 * kG + px / kRows, kb = col * rowBlocks + kbAt;
     bool const on = real && ng < nGroups && h < Ho;
     float const* const src = mine + (long long)ng * 8 * kG * imgStep + w * Ho + h;
     float v[8 * kG];
+    if (!on) {
 #pragma unroll
-    for (int n = 0; n < 8 * kG; ++n) v[n] = on && ng * 8 * kG + n < N ? __ldg(src + n * imgStep) : 0.f;
-    uint32_t m = 0;
-    float sum = 0.f;
+      for (int n = 0; n < 8 * kG; ++n) v[n] = 0.f;
+    } else if (ng * 8 * kG + 8 * kG <= N) {
+#pragma unroll
+      for (int n = 0; n < 8 * kG; ++n) v[n] = __ldg(src + n * imgStep);
+    } else {
+#pragma unroll
+      for (int n = 0; n < 8 * kG; ++n) v[n] = ng * 8 * kG + n < N ? __ldg(src + n * imgStep) : 0.f;
+    }
+    float m0 = 0.f, m1 = 0.f, sum = 0.f;
 #pragma unroll
     for (int n = 0; n < 8 * kG; n += 8) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) max_finite(m, v[n + e]);
+      m0 = max3(m0, fabsf(v[n]), fabsf(v[n + 1])); m1 = max3(m1, fabsf(v[n + 2]), fabsf(v[n + 3]));
+      m0 = max3(m0, fabsf(v[n + 4]), fabsf(v[n + 5])); m1 = max3(m1, fabsf(v[n + 6]), fabsf(v[n + 7]));
       sum += ((v[n] + v[n + 1]) + (v[n + 2] + v[n + 3])) + ((v[n + 4] + v[n + 5]) + (v[n + 6] + v[n + 7]));
     }
     acc += (double)sum;
+    uint32_t m = __float_as_uint(fmaxf(m0, m1));
+    if (m >= 0x7f800000u) {                             // an infinity among them (a not-a-number counts as nothing in the maximum): the largest finite one
+      m = 0;
+#pragma unroll
+      for (int n = 0; n < 8 * kG; ++n) max_finite(m, v[n]);
+    }
 #pragma unroll
     for (int q = 1; q < 32; q <<= 1) if (q < kRows || q >= 8) m = max(m, __shfl_xor_sync(0xffffffffu, m, q));
-    uint32_t (&r)[8][8] = red[(o - oBeg) & 1];          // (read again two octets on, with a barrier in between)
+    uint32_t (&r)[8][8] = red[turn];                    // (written again two octets on, with a barrier in between)
     if (lane < 8) r[warp][px] = m;
     __syncthreads();
 #pragma unroll
@@ -1111,11 +1133,14 @@ prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int W
     bool const kbOn = rowOn && kbAt < rowBlocks && kb < kbTot;
     // Neighbouring chunks of an image row belong to one thread (two groups of images) where kG > 1.  Rows of pixels change hands in pairs, so that two threads
     // write them together, a whole 32-byte sector: the even thread takes the even chunks of both, the odd one the odd ones.
+    bool const oddPx = (px & 1) != 0;
     int const kbO = __shfl_xor_sync(0xffffffffu, kb, 1);
     bool const kbOnO = __shfl_xor_sync(0xffffffffu, kbOn ? 1 : 0, 1) != 0;
-    bool const oddPx = (px & 1) != 0;
-    auto put = [&](int kbT, int rowT, int i, uint4 const& h4, uint4 const& l4) {
-      uint8_t* const c = rowAt + (size_t)kbT * imgBytes + (((rowT * kG + i) ^ (row & 7)) << 4);
+    uint8_t* const at0 = rowAt + (size_t)(oddPx ? kbO : kb) * imgBytes;      // image row of the even pixel of the pair, of the odd one
+    uint8_t* const at1 = rowAt + (size_t)(oddPx ? kb : kbO) * imgBytes;
+    bool const on0 = oddPx ? kbOnO : kbOn, on1 = oddPx ? kbOn : kbOnO;
+    auto put = [&](uint8_t* at, int chunk, uint4 const& h4, uint4 const& l4) {
+      uint8_t* const c = at + ((chunk ^ (row & 7)) << 4);
       *reinterpret_cast<uint4*>(c) = h4;
       if (kSplit) *reinterpret_cast<uint4*>(c + (size_t)BN * kTsRowBytes) = l4;
     };
@@ -1129,7 +1154,7 @@ prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int W
     if constexpr (kG == 1) {
       uint4 h4, l4;
       halves(0, h4, l4);
-      if (kbOn) put(kb, px, 0, h4, l4);
+      if (kbOn) put(rowAt + (size_t)kb * imgBytes, px, h4, l4);
     } else {
 #pragma unroll
       for (int i = 0; i < kG; i += 2) {
@@ -1137,9 +1162,9 @@ prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int W
         halves(i, h0, l0);
         halves(i + 1, h1, l1);
         uint4 const hr = swap4(oddPx ? h0 : h1), lr = kSplit ? swap4(oddPx ? l0 : l1) : hr;
-        // the even thread's row, then the odd one's
-        if (oddPx ? kbOnO : kbOn) put(oddPx ? kbO : kb, (px & ~1) % kRows, i + (oddPx ? 1 : 0), oddPx ? hr : h0, oddPx ? lr : l0);
-        if (oddPx ? kbOn : kbOnO) put(oddPx ? kb : kbO, (px | 1) % kRows, i + (oddPx ? 1 : 0), oddPx ? h1 : hr, oddPx ? l1 : lr);
+        int const mine = i + (oddPx ? 1 : 0);             // this thread's chunk of both rows
+        if (on0) put(at0, ((px & ~1) % kRows) * kG + mine, oddPx ? hr : h0, oddPx ? lr : l0);
+        if (on1) put(at1, ((px | 1) % kRows) * kG + mine, oddPx ? h1 : hr, oddPx ? l1 : lr);
       }
     }
     if (kbOn) {
@@ -1933,9 +1958,11 @@ int conv_wgrad_images(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, flo
   size_t const partBytes = p.splits > 1 ? ((sizeof(float) * nF * p.splits + 255) & ~(size_t)255) : 0;
   size_t const chunkBytes = (size_t)chunks * (split3 ? 32 : 16);
   size_t const expBytes = ((size_t)p.nGroups * g.W * (gShift == 3 ? g.H : 1) * g.C + 511) & ~(size_t)255;
-  int const octets = ceil_div(p.kbTot, p.rowBlocks) * ceil_div(g.Ho, 8);
+  // (one pixel per k-block: the columns of a plane are one long one, whose octets lie on 32-byte boundaries where P does)
+  int const oH = gShift == 3 ? g.Ho * g.Wo : g.Ho, oW = gShift == 3 ? 1 : g.Wo, oBlocks = gShift == 3 ? oH : p.rowBlocks;
+  int const octets = ceil_div(p.kbTot, oBlocks) * ceil_div(oH, 8);
   int const fBlocks = tiles * std::max(p.BN / 32, 1);
-  int const ranges = std::max(1, std::min(4 * ctx->smCount / fBlocks, octets)), per = ceil_div(octets, ranges), gx = ceil_div(octets, per);
+  int const gx = std::max(1, std::min(4 * ctx->smCount / fBlocks, octets));
   TileOut out;
   float* at = nullptr;
   ProfScope prof(ctx, kProfWgrad);
@@ -1952,7 +1979,7 @@ int conv_wgrad_images(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, flo
   dim3 const gridX((unsigned)((gShift == 3 ? ceil_div((long long)g.H * g.W, 8) : g.W) * cBlocks), (unsigned)p.nGroups, 1), gridY((unsigned)gx, (unsigned)fBlocks, 1);
 #define VLB_IM(split, G8) do { \
     vlb::launch(ctx->stream, split_images_kernel<split, G8>, gridX, 256, 0, hi, chunks, exps, zero, X, g.H, g.W, g.C, g.N, cBlocks); \
-    vlb::launch(ctx->stream, prep_image_tiles_kernel<split, G8>, gridY, 256, 0, out, dY, g.Ho, g.Wo, g.N, g.K, g.Kg, p.tilesN, p.BN, p.nGroups, p.rowBlocks, p.kbTot, octets, per, db, dbPart, tickets); \
+    vlb::launch(ctx->stream, prep_image_tiles_kernel<split, G8>, gridY, 256, 0, out, dY, oH, oW, g.N, g.K, g.Kg, p.tilesN, p.BN, p.nGroups, oBlocks, p.kbTot, octets, db, dbPart, tickets); \
   } while (0)
 #define VLB_IMS(G8) do { if (split3) VLB_IM(true, G8); else VLB_IM(false, G8); } while (0)
   if (gShift == 3) VLB_IMS(8); else if (gShift == 2) VLB_IMS(4); else if (gShift == 1) VLB_IMS(2); else VLB_IMS(1);
