@@ -779,60 +779,6 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
           xq += (long long)n * p.a.imgStride + (long long)wo * p.a.sx * p.a.H + ho * p.a.sy;
           hm = taps_inside(ho * p.a.sy - p.a.pt, p.a.FH, p.a.dy, p.a.H); wm = taps_inside(wo * p.a.sx - p.a.pl, p.a.FW, p.a.dx, p.a.W);
         }
-        if constexpr (kGen) {
-          int const grpC = (tile - tmf * p.tilesN) / p.tilesPerGroup;
-          xq += (long long)grpC * p.aGroup;
-          // A sub-block is upk units of kU channels of one tap: one table look-up and validity test per unit, kU loads a constant stride
-          // apart.  Small units are for few channels (kU = 32 would gather zeros), large ones keep the look-ups off the issue slots.
-          auto gather = [&](auto kUnitTag) {
-            constexpr int kU = decltype(kUnitTag)::value, kPer = 32 / kU;
-            for (int it = (int)((gi ^ grp) & 1); it < numIter; it += kTsGroups) {
-              float v[kTsK];
-              int const u0 = 2 * (kb0 + it) * kPer;
-              int cb = p.dTaps(u0), tap = u0 - cb * taps;
-              // First every load of the k-block, then the zeros of what is padding: a register overwritten while its load is on the way
-              // makes the thread wait for memory, once per unit.
-              uint32_t off[2] = {0, 0};
-#pragma unroll
-              for (int u = 0; u < 2 * kPer; ++u) {
-                int const at = (u / kPer) * 32 + (u % kPer) * kU;      // (kU = 3 leaves two places of a sub-block empty)
-                int2 const te = tapLut[tap];
-                uint32_t const e = (uint32_t)te.y;
-                int const left = p.a.C - cb * kU;          // channels of this unit that exist (the same for every thread)
-                bool const on = ((hm >> (e & 31u)) & (wm >> (e >> 5)) & 1u) != 0 && left > 0;
-                off[u / kPer] |= on ? 0u : 1u << (u % kPer);
-                float const* const q = on ? xq + ((long long)(cb * kU) * HW + te.x) : p.a.ptr;      // (padding reads the start of the tensor and discards it)
-                if (kU == 1 || left >= kU) {
-                  long long const step = on ? (long long)HW : 0;
-#pragma unroll
-                  for (int k = 0; k < kU; ++k) v[at + k] = __ldg(q + k * step);
-                } else {
-#pragma unroll
-                  for (int k = 0; k < kU; ++k) { v[at + k] = 0.f; ldg32_if(v[at + k], q + (long long)k * HW, on && k < left); }
-                }
-                if (++tap == taps) { tap = 0; ++cb; }
-              }
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                if (off[h] != 0) {
-#pragma unroll
-                  for (int k = 0; k < kPer * kU; ++k) v[32 * h + k] = ((off[h] >> (k / kU)) & 1u) ? 0.f : v[32 * h + k];
-                }
-#pragma unroll
-                for (int k = kPer * kU; k < 32; ++k) v[32 * h + k] = 0.f;
-              }
-              if (!hand_over(v)) { ok = false; break; }
-            }
-          };
-          switch (p.unit) {
-            case 32: gather(std::integral_constant<int, 32>{}); break;
-            case 16: gather(std::integral_constant<int, 16>{}); break;
-            case 8:  gather(std::integral_constant<int, 8>{}); break;
-            case 4:  gather(std::integral_constant<int, 4>{}); break;
-            case 3:  gather(std::integral_constant<int, 3>{}); break;
-            default: gather(std::integral_constant<int, 1>{}); break;
-          }
-        } else {
         for (int it = (int)((gi ^ grp) & 1); it < numIter; it += kTsGroups) {
           float v[kTsK];
           bool on[2];
@@ -859,7 +805,6 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
           }
           if (!hand_over(v)) { ok = false; break; }
         }
-        }
         gi += numIter;
       }
     }
@@ -879,12 +824,12 @@ conv_half_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
 
 // The same for what the plain kernel's gather does not cover: channels that are no multiple of 32, filter groups, and the residue
 // classes of a strided data gradient (several problems in one launch, so that a small layer's classes share the chip).
-template <bool kSplit, bool kNarrow, bool kChunks>
+template <bool kSplit, bool kNarrow>
 __global__ void __launch_bounds__(kTsThreads, 1) conv_half_gen_kernel(const __grid_constant__ TsProblems b)
 {
   int i = 0;
   while (i + 1 < b.n && (int)blockIdx.x >= b.p[i + 1].ctaBeg) ++i;
-  conv_half_body<kSplit, kChunks ? 3 : 0, kNarrow, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
+  conv_half_body<kSplit, 3, kNarrow, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
 }
 
 // ------------------------------------------------------------------ tile images
@@ -1235,17 +1180,17 @@ __global__ void __launch_bounds__(256) prep_dense_tiles_kernel(TileOut out, floa
   if ((int)threadIdx.x < perImage) out.exps[(size_t)blockIdx.x * perImage + threadIdx.x] = k;
 }
 
-// Filter tile images for conv_half_kernel and conv_half_gen_kernel, for the units of channels, filter groups, tap subsets
+// Filter tile images for conv_half_kernel and conv_half_gen_kernel, for filter groups, tap subsets
 // (residue classes of a strided data gradient) and shuffled columns of the general gather.  Row n of a tile is column n of its
 // group; tap (fh', fw') of the problem is tap (bh + ah*fh', bw + aw*fw') of the filter bank, zero where that does not exist; the
 // filter of (column channel n, reduction channel q) starts at F + FH*FW * (gs*group + sn*n + sq*q).
 struct PrepFilters {
   TileOut out;
   float const* f;
-  int BN, numKb, rows, tilesPerGroup, cols, unit, upk, tapsH, tapsW, C, FH, FW, bh, ah, bw, aw, shufY, shufX;
-  int whole;                        // k-block kb is tap kb % taps of the 64 channels from 64 * (kb / taps) on (kMode 3), not two sub-blocks of 32
+  int BN, numKb, rows, tilesPerGroup, cols, tapsH, tapsW, C, FH, FW, bh, ah, bw, aw, shufY, shufX;
+  int whole;                        // k-block kb is tap kb % taps of the 64 channels from 64 * (kb / taps) on (kMode 3), not two sub-blocks of one tap of 32
   long long sn, sq, gs;
-  vlb::FastDiv31 divTaps, divTapsH, divUnit;        // by tapsH * tapsW, tapsH and unit (set by launch_prep)
+  vlb::FastDiv31 divTaps, divTapsH;                 // by tapsH * tapsW and tapsH (set by launch_prep)
 };
 struct PrepBatch { PrepFilters p[kMaxTsProblems]; };
 
@@ -1270,24 +1215,12 @@ __global__ void __launch_bounds__(512) prep_filters_kernel(const __grid_constant
     int ry = 0, rx = 0, n = col;
     if (p.shufY > 0) { n = col / (p.shufY * p.shufX); int const t = col - n * p.shufY * p.shufX; rx = t / p.shufY; ry = t - rx * p.shufY; }
     float const* const fn = p.f + (long long)FT * (p.gs * grp + p.sn * n);
-    if (p.unit % 8 == 0) {
-      // the chunk's eight places are channels of one tap
-      int const kk = (chunk & 3) * 8, u = p.divUnit(kk), un = p.whole ? kb : (2 * kb + (chunk >> 2)) * p.upk + u;
-      int const cb = p.divTaps(un), tap = un - cb * taps, q0 = p.whole ? cb * 64 + chunk * 8 : cb * p.unit + (kk - u * p.unit);
-      int const tw = p.divTapsH(tap), th = tap - tw * p.tapsH, fh = p.bh + p.ah * th + ry, fw = p.bw + p.aw * tw + rx;
-      if ((unsigned)fh < (unsigned)p.FH && (unsigned)fw < (unsigned)p.FW) {
+    // the chunk's eight places are channels of one tap
+    int const un = p.whole ? kb : 2 * kb + (chunk >> 2), cb = p.divTaps(un), tap = un - cb * taps, q0 = p.whole ? cb * 64 + chunk * 8 : cb * 32 + (chunk & 3) * 8;
+    int const tw = p.divTapsH(tap), th = tap - tw * p.tapsH, fh = p.bh + p.ah * th + ry, fw = p.bw + p.aw * tw + rx;
+    if ((unsigned)fh < (unsigned)p.FH && (unsigned)fw < (unsigned)p.FW) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) if (q0 + e < p.C) v[e] = __ldg(fn + (long long)FT * p.sq * (q0 + e) + (fh + p.FH * fw));
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        int const kk = (chunk & 3) * 8 + e, u = p.divUnit(kk);
-        int const un = (2 * kb + (chunk >> 2)) * p.upk + u, cb = p.divTaps(un), tap = un - cb * taps, q = cb * p.unit + (kk - u * p.unit);
-        int const tw = p.divTapsH(tap), th = tap - tw * p.tapsH;
-        int const fh = p.bh + p.ah * th + ry, fw = p.bw + p.aw * tw + rx;
-        if (u < p.upk && q < p.C && (unsigned)fh < (unsigned)p.FH && (unsigned)fw < (unsigned)p.FW) v[e] = __ldg(fn + (long long)FT * p.sq * q + (fh + p.FH * fw));
-      }
+      for (int e = 0; e < 8; ++e) if (q0 + e < p.C) v[e] = __ldg(fn + (long long)FT * p.sq * (q0 + e) + (fh + p.FH * fw));
     }
   }
   uint32_t m = 0;
@@ -1305,7 +1238,7 @@ void launch_prep(vlb_ctx* ctx, PrepBatch& prep, int n)
   long long images = 0;
   for (int i = 0; i < n; ++i) {
     PrepFilters& q = prep.p[i];
-    q.divTaps = vlb::FastDiv31(q.tapsH * q.tapsW); q.divTapsH = vlb::FastDiv31(q.tapsH); q.divUnit = vlb::FastDiv31(q.unit);
+    q.divTaps = vlb::FastDiv31(q.tapsH * q.tapsW); q.divTapsH = vlb::FastDiv31(q.tapsH);
     images = std::max(images, (long long)q.rows / q.BN * q.numKb);
   }
   VLB_LAUNCHED(ctx, 1);
@@ -1480,15 +1413,6 @@ bool prep_dense_tiles(vlb_ctx* ctx, Params& p, float const* f, bool rows, size_t
   return true;
 }
 
-// Whether the gathered tensor (chPerGroup channels in each of `groups` groups, read once per filter tap and column tile: `readings`) is split beforehand.  A k-block
-// of the gather that splits as it goes takes 2000 cycles, one of split chunks 1150; a filter group has to be whole blocks of 64 channels, and a
-// single one may be filled up with zeros to at most half as much again.  One reading costs more to split (8 bytes per element) than it saves:
-// 1x1, 512 -> 128 channels, 28 x 28 x 64: 65 us against 60.
-bool split_pays(int chPerGroup, int groups, int readings)
-{
-  return readings >= 2 && (groups == 1 ? (chPerGroup + 63) / 64 * 128 <= 3 * chPerGroup : chPerGroup % 64 == 0);
-}
-
 // The filter bank of one group, reduction in blocks of 32 channels (conv_half_kernel): forward, or flipped and transposed for the data gradient
 // of a stride-1 convolution.
 // Where it pays, the gathered tensor is split beforehand (kMode 3).
@@ -1506,7 +1430,7 @@ bool prep_conv_tiles(vlb_ctx* ctx, Params& p, float const* f, vlb::ConvGeom cons
   if (extra) *extra = behind;
   if (chunks) split_chunks(ctx, p, (char*)behind + extraBytes, images, p.a.C);
   q.f = f; q.BN = p.BN; q.numKb = p.numKb; q.tilesPerGroup = vlb::ceil_div(p.N, p.BN); q.rows = q.tilesPerGroup * p.BN; q.cols = p.N;
-  q.unit = 32; q.upk = 1; q.tapsH = q.FH = g.FH; q.tapsW = q.FW = g.FW; q.C = dgrad ? g.K : g.C;
+  q.tapsH = q.FH = g.FH; q.tapsW = q.FW = g.FW; q.C = dgrad ? g.K : g.C;
   q.bh = dgrad ? g.FH - 1 : 0; q.bw = dgrad ? g.FW - 1 : 0; q.ah = q.aw = dgrad ? -1 : 1;
   q.sn = dgrad ? 1 : g.C; q.sq = dgrad ? g.C : 1; q.whole = p.aHi != nullptr;
   launch_prep(ctx, prep, 1);
@@ -1551,19 +1475,15 @@ template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 3, true>>() { ret
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 3, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 3, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 3, false>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, true, false>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, true, true>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, false, false>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, false, true>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, true>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 0, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 0, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 1, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 1, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 2, false>>() { return 80; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, true, false>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, true, true>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, false, false>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, false, true>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, true>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, false>>() { return 96; }
 
 // Decides whether conv_half_kernel can take its input windows from tensor-map copies and, if so, fills the box geometry in p,
 // the tensor map and the shared-memory size.  Needs: reduction in blocks of 32 channels, unit stride, input rows a multiple
@@ -1772,23 +1692,17 @@ bool wgrad_images_pay(vlb_ctx* ctx, ConvGeom const& g, bool rows, long long kbs,
   return 0.7 * tiles * (double)kbs * perSm + (x * (gShift == 3 ? 8 : 12) + y * (rows ? 3 : 0)) / 5e6 + (rows ? 3.0 : 10.0) < other;
 }
 
-// k-blocks of a reduction over `taps` filter taps of `channels` channels: whole blocks of 64 channels, or units of gen_unit channels in sub-blocks of 32.
-int gen_kblocks(int taps, int channels, bool chunks)
-{
-  if (chunks) return taps * vlb::ceil_div(channels, 64);
-  int const unit = gen_unit(channels);
-  return vlb::ceil_div(vlb::ceil_div(taps * vlb::ceil_div(channels, unit), 32 / unit), 2);
-}
+// k-blocks of a reduction over `taps` filter taps of `channels` channels.
+int gen_kblocks(int taps, int channels) { return taps * vlb::ceil_div(channels, 64); }
 
 // One contraction of conv_half_gen_kernel: the stride / pad / dilation geometry t over src, `groups` groups of chPerGroup channels
 // and `cols` output columns each.
-void gen_problem(Params& p, ConvGeom const& t, float const* src, int chPerGroup, int groups, int cols, int BN, bool chunks)
+void gen_problem(Params& p, ConvGeom const& t, float const* src, int chPerGroup, int groups, int cols, int BN)
 {
   conv_operand(p.a, t, src, chPerGroup * groups);
   p.a.C = chPerGroup; p.aGroup = (long long)t.H * t.W * chPerGroup;
   p.M = t.Ho * t.Wo * t.N; p.N = cols * groups; p.R = t.FH * t.FW * chPerGroup; p.a.rows = p.M;
-  p.unit = gen_unit(chPerGroup); p.upk = 32 / p.unit;
-  p.numKb = gen_kblocks(t.FH * t.FW, chPerGroup, chunks);
+  p.numKb = gen_kblocks(t.FH * t.FW, chPerGroup);
   p.BN = BN; p.cols = cols; p.tilesPerGroup = vlb::ceil_div(cols, BN); p.tilesN = groups * p.tilesPerGroup; p.tilesM = vlb::ceil_div(p.M, BM);
   p.splits = 1; p.kbPerSplit = p.kbTot = p.numKb;
   p.oy = p.ox = 0; p.oys = p.oxs = 1; p.outH = t.Ho; p.outW = t.Wo; p.shufY = p.shufX = 0; p.outC = cols;
@@ -1799,7 +1713,7 @@ PrepFilters gen_prep(Params const& p, ConvGeom const& g, float const* f)
 {
   PrepFilters q = {};
   q.f = f; q.BN = p.BN; q.numKb = p.numKb; q.rows = p.tilesN * p.BN; q.tilesPerGroup = p.tilesPerGroup; q.cols = p.cols;
-  q.unit = p.unit; q.upk = p.upk; q.tapsH = p.a.FH; q.tapsW = p.a.FW; q.C = p.a.C; q.FH = g.FH; q.FW = g.FW;
+  q.whole = 1; q.tapsH = p.a.FH; q.tapsW = p.a.FW; q.C = p.a.C; q.FH = g.FH; q.FW = g.FW;
   q.ah = q.aw = 1; q.shufY = p.shufY; q.shufX = p.shufX;
   return q;
 }
@@ -1808,7 +1722,7 @@ PrepFilters gen_prep(Params const& p, ConvGeom const& g, float const* f)
 // Where the problems' tiles are too few for the chip the reductions are cut, all into the same number of ranges, and `fin` (the epilogue,
 // which the problems then do not apply themselves) goes to the sum over the ranges; they cover every element of the output then
 // (`covered`).
-int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size_t nOut, vlb::SumEpilogue const& fin, bool covered, bool chunks, char const* where)
+int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size_t nOut, vlb::SumEpilogue const& fin, bool covered, char const* where)
 {
   bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
   int const BN = b.p[0].BN;
@@ -1839,15 +1753,15 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     work += (double)t * (p.kbPerSplit + 6);
     if (t >= (1LL << 31)) return VLB_Unsupported;
   }
-  // all problems gather from one tensor, which is split beforehand where its groups are whole blocks of 64 channels
+  // all problems gather from one tensor, which is split beforehand
   Operand const& a0 = b.p[0].a;
   int const images = (int)(b.p[0].M / ((long long)a0.Ho * a0.Wo)), channels = (int)(a0.imgStride / ((long long)a0.H * a0.W));
   long long const elements = (long long)a0.H * a0.W * vlb::ceil_div(channels, 64) * 64 * images;
   size_t const partBytes = splits > 1 ? (sizeof(float) * nOut * splits + 255) & ~(size_t)255 : 0;
-  char* const ws = (char*)vlb::workspace(ctx, total + partBytes + (chunks ? chunks_bytes(ctx, elements) : 0));
+  char* const ws = (char*)vlb::workspace(ctx, total + partBytes + chunks_bytes(ctx, elements));
   if (!ws) return ctx->lastError;
   float* const part = (float*)(ws + total);
-  if (chunks) split_chunks(ctx, b.p[0], ws + total + partBytes, images, channels);
+  split_chunks(ctx, b.p[0], ws + total + partBytes, images, channels);
   // CTAs per problem: one per tile when all tiles fit, else shares of the chip in proportion to the work, the rest to the longest queues
   int given = 0;
   for (int i = 0; i < b.n; ++i) {
@@ -1868,14 +1782,14 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     if (worst < 0) break;
     ++b.p[worst].ctas; ++given;
   }
-  int const stages = (int)std::min<size_t>(chunks ? 4 : kTsBStages, (227 * 1024 - kTsStatic - 1024 - patchBytes) / stageBytes);
+  int const stages = (int)std::min<size_t>(4, (227 * 1024 - kTsStatic - 1024 - patchBytes) / stageBytes);
   for (int i = 0, beg = 0; i < b.n; ++i) {
     Params& p = b.p[i];
     p.ctaBeg = beg; beg += p.ctas;
     prep.p[i].out = ts_tiles_at(ctx, ws + offset[i], p.tilesN * BN, BN, p.numKb);
     p.bTiles = (float const*)prep.p[i].out.img; p.bExp = prep.p[i].out.exps;
     if (splits > 1) p.e.out = part;
-    if (chunks) { p.c64 = b.p[0].c64; p.aHi = b.p[0].aHi; p.aLo = b.p[0].aLo; p.aExp = b.p[0].aExp; p.zero = b.p[0].zero; prep.p[i].whole = 1; prep.p[i].unit = 32; prep.p[i].upk = 1; }
+    p.c64 = b.p[0].c64; p.aHi = b.p[0].aHi; p.aLo = b.p[0].aLo; p.aExp = b.p[0].aExp; p.zero = b.p[0].zero;
     p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;
     ts_divisors(p);
     p.biasFirst = p.e.bias != nullptr && aligned16(p.e.bias) && p.cols % 4 == 0 && p.shufY == 0 && p.e.inMult == 1.f && p.e.outMult == 0.f;
@@ -1887,38 +1801,14 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     e = allow_large_smem<decltype(kernel)::value>(ctx->device);
     if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, given, kTsThreads, smemBytes, b);
   };
-#define VLB_TSG(split, nar, chunks) go(std::integral_constant<decltype(&conv_half_gen_kernel<split, nar, chunks>), &conv_half_gen_kernel<split, nar, chunks>>{})
-#define VLB_TSGN(split, nar) do { if (chunks) VLB_TSG(split, nar, true); else VLB_TSG(split, nar, false); } while (0)
-  if (split3) { if (BN <= 64) VLB_TSGN(true, true); else VLB_TSGN(true, false); }
-  else        { if (BN <= 64) VLB_TSGN(false, true); else VLB_TSGN(false, false); }
-#undef VLB_TSGN
+#define VLB_TSG(split, nar) go(std::integral_constant<decltype(&conv_half_gen_kernel<split, nar>), &conv_half_gen_kernel<split, nar>>{})
+  if (split3) { if (BN <= 64) VLB_TSG(true, true); else VLB_TSG(true, false); }
+  else        { if (BN <= 64) VLB_TSG(false, true); else VLB_TSG(false, false); }
 #undef VLB_TSG
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
   int const rc = vlb::check_launch(ctx, where);
   return rc || splits == 1 ? rc : vlb::sum_parts(ctx, out, part, nOut, nOut, splits, fin);
-}
-
-// One dimension of a data gradient's residue class: the input positions h with (h + pad) % stride == r, and the filter taps that reach
-// them.  Positions are h0 + stride * i, i < count; tap f0 + step * (taps - 1 - f') of the filter meets position i at output
-// position i + f' * dil - pad: a stride-1 convolution of the output derivative with `taps` taps.
-struct ClassDim { int h0, count, taps, f0, step, dil, pad; };
-
-ClassDim class_dim(int r, int H, int FH, int stride, int pad, int dilate)
-{
-  ClassDim c = {};
-  c.h0 = ((r - pad) % stride + stride) % stride;
-  c.count = c.h0 < H ? (H - 1 - c.h0) / stride + 1 : 0;
-  int a = stride, d = dilate;
-  while (d) { int const t = a % d; a = d; d = t; }                   // a = gcd(stride, dilate)
-  c.step = stride / a; c.dil = dilate / a;
-  c.f0 = -1;
-  for (int f = 0; f < c.step && f < FH; ++f) if ((f * dilate) % stride == r) c.f0 = f;
-  c.taps = c.f0 < 0 ? 0 : (FH - 1 - c.f0) / c.step + 1;
-  // output position of tap f0 + step*j at position h: (h + pad - (f0 + step*j)*dilate) / stride = i + first - j*dil
-  int const first = c.f0 < 0 ? 0 : (c.h0 + pad - c.f0 * dilate) / stride;          // exact: the numerator is a multiple of the stride
-  c.pad = (c.taps - 1) * c.dil - first;
-  return c;
 }
 
 }  // namespace
@@ -2035,7 +1925,7 @@ int conv_wgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float
   *dbDone = db != nullptr;
   p.e = Epilogue{};
   p.e.out = part ? part : dF; p.e.splitStride = part ? (long long)nF : 0; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.K;
-  int const rc = launch_rows(ctx, p, map, "conv_wgrad_ts");
+  int const rc = launch_rows(ctx, p, map, "conv_wgrad_half");
   if (rc) return rc;
   return part ? vlb::sum_parts(ctx, dF, part, nF, nF, p.splits) : VLB_Success;
 }
@@ -2070,7 +1960,7 @@ int fc_dgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
   p.e.out = part ? part : dX; p.e.splitStride = part ? (long long)nOut : 0; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.N;
   vlb::SumEpilogue epi;
   (part ? epi.mask : p.e.mask) = ctx->reluMask; ctx->maskDone = ctx->reluMask != nullptr;
-  int rc = launch_ts(ctx, p, "fc_dgrad_ts");
+  int rc = launch_ts(ctx, p, "fc_dgrad_half");
   return rc || !part ? rc : vlb::sum_parts(ctx, dX, part, nOut, nOut, p.splits, epi);
 }
 
@@ -2097,95 +1987,22 @@ int fc_wgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, fl
   if (chunks) split_chunks(ctx, p, behind, 1, g.N);
   p.e = Epilogue{};
   p.e.out = dF; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.K;
-  return launch_ts(ctx, p, "fc_wgrad_ts");
+  return launch_ts(ctx, p, "fc_wgrad_half");
 }
 
-// Data gradient of a strided or grouped convolution, or one whose filters are no multiple of 32, through the general gather.  Two forms:
-//   classes   one problem per residue class of the input pixel modulo the stride, each a stride-1 convolution of dY with the taps that
-//             reach the class: no product with a structural zero, but C columns each;
-//   shuffled  (dilation 1) one problem over the stride-sized blocks of input pixels whose columns are (pixel of the block, channel):
-//             the classes' taps padded to the largest class, C * strideY * strideX columns -- for few channels, whose class
-//             tiles would be mostly empty columns (11 x 11 stride 4 onto 3 channels: one 48-column problem instead of 16 with 3).
-int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
+int conv_dgrad_gen_half(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY)
 {
-  int const C = g.FC, nc = g.sy * g.sx;
-  ConvGeom t = g;
-  t.H = g.Ho; t.W = g.Wo; t.N = g.N; t.sy = t.sx = 1;
-  ClassDim ch[kMaxTsProblems], cw[kMaxTsProblems];
-  bool const classesOk = g.sy <= kMaxTsProblems && g.sx <= kMaxTsProblems && nc <= kMaxTsProblems;
-  double classCost = 1e30;
-  bool holes = false;               // classes that no tap reaches: zeros
   // dY is read once per filter tap and column tile, whichever class or column the tap belongs to
-  bool const chunks = split_pays(g.Kg, g.G, g.FH * g.FW * ceil_div(C, pick_bn(C)));
-  auto kblocks = [&](int taps) { return gen_kblocks(taps, g.Kg, chunks); };
-  if (classesOk) {
-    classCost = 0;
-    for (int r = 0; r < g.sy; ++r) ch[r] = class_dim(r, g.H, g.FH, g.sy, g.pt, g.dy);
-    for (int r = 0; r < g.sx; ++r) cw[r] = class_dim(r, g.W, g.FW, g.sx, g.pl, g.dx);
-    int const BN = pick_bn(C);
-    for (int y = 0; y < g.sy; ++y)
-      for (int x = 0; x < g.sx; ++x) {
-        int const taps = ch[y].taps * cw[x].taps, pix = ch[y].count * cw[x].count;
-        if (pix == 0) continue;
-        if (taps == 0) { holes = true; continue; }
-        classCost += gen_cost(vlb::ceil_div((long long)pix * g.N, BM) * g.G * vlb::ceil_div(C, BN), kblocks(taps), BN);
-      }
-  }
-  TsProblems ts = {};
-  PrepBatch prep = {};
-  size_t const nOut = (size_t)g.H * g.W * g.C * g.N;
-  vlb::SumEpilogue fin;
-  fin.mask = ctx->reluMask;
-  fin.bias = ctx->dgradBias; fin.P = g.H * g.W; fin.K = g.C;
-  // shuffled form
-  int const FHm = vlb::ceil_div(g.FH, g.sy), FWm = vlb::ceil_div(g.FW, g.sx);
-  int const iy = g.pt / g.sy, ix = g.pl / g.sx, Hm = (g.H - 1 + g.pt) / g.sy - iy + 1, Wm = (g.W - 1 + g.pl) / g.sx - ix + 1;
-  if (nc > 1 && g.dy == 1 && g.dx == 1 && gen_taps_ok(FHm, FWm)) {
-    int const cols = C * nc, BN = pick_bn(cols);
-    double const cost = gen_cost(vlb::ceil_div((long long)Hm * Wm * g.N, BM) * g.G * vlb::ceil_div(cols, BN), kblocks(FHm * FWm), BN);
-    if (cost < classCost) {
-      t.FH = FHm; t.FW = FWm; t.Ho = Hm; t.Wo = Wm; t.pt = FHm - 1 - iy; t.pl = FWm - 1 - ix;
-      ts.n = 1;
-      Params& p = ts.p[0];
-      gen_problem(p, t, dY, g.Kg, g.G, cols, BN, chunks);
-      p.oys = g.sy; p.oxs = g.sx; p.oy = g.sy * iy - g.pt; p.ox = g.sx * ix - g.pl; p.outH = g.H; p.outW = g.W;
-      p.shufY = g.sy; p.shufX = g.sx; p.outC = C;
-      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
-      PrepFilters& q = prep.p[0] = gen_prep(p, g, F);
-      q.bh = g.sy * (FHm - 1); q.ah = -g.sy; q.bw = g.sx * (FWm - 1); q.aw = -g.sx;
-      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
-      int const rc = launch_ts_gen(ctx, ts, prep, dX, nOut, fin, true, chunks, "conv_dgrad_gen");
-      if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true; }      // (a refused launch applies neither)
-      return rc;
-    }
-  }
-  if (!classesOk) return VLB_Unsupported;
-  for (int y = 0; y < g.sy; ++y) for (int x = 0; x < g.sx; ++x) if (ch[y].taps * cw[x].taps > 0 && !gen_taps_ok(ch[y].taps, cw[x].taps)) return VLB_Unsupported;
-  if (holes) {
-    cudaError_t const e = cudaMemsetAsync(dX, 0, sizeof(float) * (size_t)g.H * g.W * g.C * g.N, ctx->stream);
-    if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
-  }
-  ts.n = 0;
-  for (int y = 0; y < g.sy; ++y)
-    for (int x = 0; x < g.sx; ++x) {
-      ClassDim const& h = ch[y];
-      ClassDim const& w = cw[x];
-      if (h.taps * w.taps == 0 || h.count * w.count == 0) continue;
-      t.FH = h.taps; t.FW = w.taps; t.Ho = h.count; t.Wo = w.count; t.pt = h.pad; t.pl = w.pad; t.dy = h.dil; t.dx = w.dil;
-      Params& p = ts.p[ts.n];
-      gen_problem(p, t, dY, g.Kg, g.G, C, pick_bn(C), chunks);
-      p.oys = g.sy; p.oxs = g.sx; p.oy = h.h0; p.ox = w.h0; p.outH = g.H; p.outW = g.W;
-      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
-      PrepFilters& q = prep.p[ts.n] = gen_prep(p, g, F);
-      q.bh = h.f0 + h.step * (h.taps - 1); q.ah = -h.step; q.bw = w.f0 + w.step * (w.taps - 1); q.aw = -w.step;
-      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
-      ++ts.n;
-    }
-  if (holes) fin.bias = nullptr;                    // (the zeros of the classes without a tap would miss it)
-  // (ts.n == 0: no tap reaches any pixel; all zeros, written above)
-  int const rc = ts.n == 0 ? VLB_Success : launch_ts_gen(ctx, ts, prep, dX, nOut, fin, !holes, chunks, "conv_dgrad_gen");
-  if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = !holes; }
-  return rc;
+  if (!split_pays(g.Kg, g.G, g.FH * g.FW * ceil_div(g.FC, pick_bn(g.FC)))) return -1;
+  struct {
+    vlb_ctx* ctx; ConvGeom const& g; float* dX; float const* F; float const* dY;
+    int kblocks(int taps) const { return gen_kblocks(taps, g.Kg); }
+    void problem(Params& p, ConvGeom const& t, int cols, int BN) const { gen_problem(p, t, dY, g.Kg, g.G, cols, BN); }
+    PrepFilters prep(Params const& p) const { return gen_prep(p, g, F); }
+    int launch(TsProblems& ts, PrepBatch& prep, SumEpilogue const& fin, bool covered) const
+    { return launch_ts_gen(ctx, ts, prep, dX, (size_t)g.H * g.W * g.C * g.N, fin, covered, "conv_dgrad_gen_half"); }
+  } const route{ctx, g, dX, F, dY};
+  return dgrad_forms<PrepBatch>(ctx, g, dX, route);
 }
 
 // Data gradient of a stride-1 convolution: dX = conv(dY, flipped and transposed filters) with padding (F-1)*dilate - pad.  -1: not eligible.

@@ -49,10 +49,9 @@ int conv_dgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
 int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float const* X, float const* dY,
                   bool* dbDone);
 
-// The backward contractions on scaled half-precision operands (conv_half.cu), behind conv_*_tc.  -1: not eligible, the caller takes another kernel;
-// conv_dgrad_gen answers VLB_Unsupported.
+// The backward contractions on scaled half-precision operands (conv_half.cu), behind conv_*_tc.  -1: not eligible, the caller takes another kernel.
 int conv_dgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY);
-int conv_dgrad_gen(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY);
+int conv_dgrad_gen_half(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY);
 int conv_wgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float const* X, float const* dY, bool* dbDone);
 int fc_dgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, float const* dY);
 int fc_wgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, float const* dY);

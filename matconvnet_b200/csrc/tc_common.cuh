@@ -548,4 +548,122 @@ inline bool rows_map(CUtensorMap* map, float const* ptr, long long run, long lon
                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// One dimension of a data gradient's residue class: the input positions h with (h + pad) % stride == r, and the filter taps that reach
+// them.  Positions are h0 + stride * i, i < count; tap f0 + step * (taps - 1 - f') of the filter meets position i at output
+// position i + f' * dil - pad: a stride-1 convolution of the output derivative with `taps` taps.
+struct ClassDim { int h0, count, taps, f0, step, dil, pad; };
+
+inline ClassDim class_dim(int r, int H, int FH, int stride, int pad, int dilate)
+{
+  ClassDim c = {};
+  c.h0 = ((r - pad) % stride + stride) % stride;
+  c.count = c.h0 < H ? (H - 1 - c.h0) / stride + 1 : 0;
+  int a = stride, d = dilate;
+  while (d) { int const t = a % d; a = d; d = t; }                   // a = gcd(stride, dilate)
+  c.step = stride / a; c.dil = dilate / a;
+  c.f0 = -1;
+  for (int f = 0; f < c.step && f < FH; ++f) if ((f * dilate) % stride == r) c.f0 = f;
+  c.taps = c.f0 < 0 ? 0 : (FH - 1 - c.f0) / c.step + 1;
+  // output position of tap f0 + step*j at position h: (h + pad - (f0 + step*j)*dilate) / stride = i + first - j*dil
+  int const first = c.f0 < 0 ? 0 : (c.h0 + pad - c.f0 * dilate) / stride;          // exact: the numerator is a multiple of the stride
+  c.pad = (c.taps - 1) * c.dil - first;
+  return c;
+}
+
+// Whether the gathered tensor (chPerGroup channels in each of `groups` groups, read once per filter tap and column tile: `readings`) is split beforehand.  A k-block
+// of the gather that splits as it goes takes 2000 cycles, one of split chunks 1150; a filter group has to be whole blocks of 64 channels, and a
+// single one may be filled up with zeros to at most half as much again.  One reading costs more to split (8 bytes per element) than it saves:
+// 1x1, 512 -> 128 channels, 28 x 28 x 64: 65 us against 60.
+inline bool split_pays(int chPerGroup, int groups, int readings)
+{
+  return readings >= 2 && (groups == 1 ? (chPerGroup + 63) / 64 * 128 <= 3 * chPerGroup : chPerGroup % 64 == 0);
+}
+
+// Data gradient of a strided or grouped convolution, or one whose filters are no multiple of 32, through the general gather.  Two forms:
+//   classes   one problem per residue class of the input pixel modulo the stride, each a stride-1 convolution of dY with the taps that
+//             reach the class: no product with a structural zero, but C columns each;
+//   shuffled  (dilation 1) one problem over the stride-sized blocks of input pixels whose columns are (pixel of the block, channel):
+//             the classes' taps padded to the largest class, C * strideY * strideX columns -- for few channels, whose class
+//             tiles would be mostly empty columns (11 x 11 stride 4 onto 3 channels: one 48-column problem instead of 16 with 3).
+//
+// Route is the kernel: kblocks(taps), problem(p, t, columns, BN), prep(p), launch(problems, tile images' description, scalar epilogue, covered).
+template <class PrepBatch, class Route>
+int dgrad_forms(vlb_ctx* ctx, vlb::ConvGeom const& g, float* dX, Route const& route)
+{
+  int const C = g.FC, nc = g.sy * g.sx;
+  vlb::ConvGeom t = g;
+  t.H = g.Ho; t.W = g.Wo; t.N = g.N; t.sy = t.sx = 1;
+  ClassDim ch[kMaxTsProblems], cw[kMaxTsProblems];
+  bool const classesOk = g.sy <= kMaxTsProblems && g.sx <= kMaxTsProblems && nc <= kMaxTsProblems;
+  double classCost = 1e30;
+  bool holes = false;               // classes that no tap reaches: zeros
+  if (classesOk) {
+    classCost = 0;
+    for (int r = 0; r < g.sy; ++r) ch[r] = class_dim(r, g.H, g.FH, g.sy, g.pt, g.dy);
+    for (int r = 0; r < g.sx; ++r) cw[r] = class_dim(r, g.W, g.FW, g.sx, g.pl, g.dx);
+    int const BN = pick_bn(C);
+    for (int y = 0; y < g.sy; ++y)
+      for (int x = 0; x < g.sx; ++x) {
+        int const taps = ch[y].taps * cw[x].taps, pix = ch[y].count * cw[x].count;
+        if (pix == 0) continue;
+        if (taps == 0) { holes = true; continue; }
+        classCost += gen_cost(vlb::ceil_div((long long)pix * g.N, BM) * g.G * vlb::ceil_div(C, BN), route.kblocks(taps), BN);
+      }
+  }
+  TsProblems ts = {};
+  PrepBatch prep = {};
+  vlb::SumEpilogue fin;
+  fin.mask = ctx->reluMask;
+  fin.bias = ctx->dgradBias; fin.P = g.H * g.W; fin.K = g.C;
+  // shuffled form
+  int const FHm = vlb::ceil_div(g.FH, g.sy), FWm = vlb::ceil_div(g.FW, g.sx);
+  int const iy = g.pt / g.sy, ix = g.pl / g.sx, Hm = (g.H - 1 + g.pt) / g.sy - iy + 1, Wm = (g.W - 1 + g.pl) / g.sx - ix + 1;
+  if (nc > 1 && g.dy == 1 && g.dx == 1 && gen_taps_ok(FHm, FWm)) {
+    int const cols = C * nc, BN = pick_bn(cols);
+    double const cost = gen_cost(vlb::ceil_div((long long)Hm * Wm * g.N, BM) * g.G * vlb::ceil_div(cols, BN), route.kblocks(FHm * FWm), BN);
+    if (cost < classCost) {
+      t.FH = FHm; t.FW = FWm; t.Ho = Hm; t.Wo = Wm; t.pt = FHm - 1 - iy; t.pl = FWm - 1 - ix;
+      ts.n = 1;
+      Params& p = ts.p[0];
+      route.problem(p, t, cols, BN);
+      p.oys = g.sy; p.oxs = g.sx; p.oy = g.sy * iy - g.pt; p.ox = g.sx * ix - g.pl; p.outH = g.H; p.outW = g.W;
+      p.shufY = g.sy; p.shufX = g.sx; p.outC = C;
+      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
+      auto& q = prep.p[0] = route.prep(p);
+      q.bh = g.sy * (FHm - 1); q.ah = -g.sy; q.bw = g.sx * (FWm - 1); q.aw = -g.sx;
+      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
+      int const rc = route.launch(ts, prep, fin, true);
+      if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true; }      // (a refused launch applies neither)
+      return rc;
+    }
+  }
+  if (!classesOk) return VLB_Unsupported;
+  for (int y = 0; y < g.sy; ++y) for (int x = 0; x < g.sx; ++x) if (ch[y].taps * cw[x].taps > 0 && !gen_taps_ok(ch[y].taps, cw[x].taps)) return VLB_Unsupported;
+  if (holes) {
+    cudaError_t const e = cudaMemsetAsync(dX, 0, sizeof(float) * (size_t)g.H * g.W * g.C * g.N, ctx->stream);
+    if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
+  }
+  ts.n = 0;
+  for (int y = 0; y < g.sy; ++y)
+    for (int x = 0; x < g.sx; ++x) {
+      ClassDim const& h = ch[y];
+      ClassDim const& w = cw[x];
+      if (h.taps * w.taps == 0 || h.count * w.count == 0) continue;
+      t.FH = h.taps; t.FW = w.taps; t.Ho = h.count; t.Wo = w.count; t.pt = h.pad; t.pl = w.pad; t.dy = h.dil; t.dx = w.dil;
+      Params& p = ts.p[ts.n];
+      route.problem(p, t, C, pick_bn(C));
+      p.oys = g.sy; p.oxs = g.sx; p.oy = h.h0; p.ox = w.h0; p.outH = g.H; p.outW = g.W;
+      p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
+      auto& q = prep.p[ts.n] = route.prep(p);
+      q.bh = h.f0 + h.step * (h.taps - 1); q.ah = -h.step; q.bw = w.f0 + w.step * (w.taps - 1); q.aw = -w.step;
+      q.sn = 1; q.sq = C; q.gs = (long long)C * g.Kg;
+      ++ts.n;
+    }
+  if (holes) fin.bias = nullptr;                    // (the zeros of the classes without a tap would miss it)
+  // (ts.n == 0: no tap reaches any pixel; all zeros, written above)
+  int const rc = ts.n == 0 ? VLB_Success : route.launch(ts, prep, fin, !holes);
+  if (rc == VLB_Success) { ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = !holes; }
+  return rc;
+}
+
 }  // namespace
