@@ -824,11 +824,11 @@ conv_half_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
 
 // The same for what the plain kernel's gather does not cover: channels that are no multiple of 32, filter groups, and the residue
 // classes of a strided data gradient (several problems in one launch, so that a small layer's classes share the chip).
-template <bool kSplit, bool kNarrow>
-__global__ void __launch_bounds__(kTsThreads, 1) conv_half_gen_kernel(const __grid_constant__ TsProblems b)
+template <bool kSplit, bool kNarrow, int kMax>
+__global__ void __launch_bounds__(kTsThreads, 1) conv_half_gen_kernel(const __grid_constant__ Problems<kMax> b)
 {
   int i = 0;
-  while (i + 1 < b.n && (int)blockIdx.x >= b.p[i + 1].ctaBeg) ++i;
+  if constexpr (kMax > 1) while (i + 1 < b.n && (int)blockIdx.x >= b.p[i + 1].ctaBeg) ++i;
   conv_half_body<kSplit, 3, kNarrow, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
 }
 
@@ -1192,13 +1192,22 @@ struct PrepFilters {
   long long sn, sq, gs;
   vlb::FastDiv31 divTaps, divTapsH;                 // by tapsH * tapsW and tapsH (set by launch_prep)
 };
-struct PrepBatch { PrepFilters p[kMaxTsProblems]; };
+template <int kMax> struct PrepBatchOf { PrepFilters p[kMax]; };
+using PrepBatch = PrepBatchOf<kMaxTsProblems>;
+
+template <int kMax>
+PrepBatchOf<kMax> first_preps(PrepBatch const& b)
+{
+  PrepBatchOf<kMax> q;
+  std::copy(b.p, b.p + kMax, q.p);
+  return q;
+}
 
 // A block takes 64 rows of an image (all of a narrower tile), a thread eight places of one row.  Grid (tiles * numKb * blocks per image, problems).  Bound by the
 // scattered 4-byte reads, one request per place: with a block per image 7 us for 128 -> 128 channels, 3x3, with two 3.5.  (Through shared memory, in
 // runs of the taps of sixteen channels: 15 us against 13 for 512 -> 512 channels.)
-template <bool kSplit>
-__global__ void __launch_bounds__(512) prep_filters_kernel(const __grid_constant__ PrepBatch b)
+template <bool kSplit, int kMax>
+__global__ void __launch_bounds__(512) prep_filters_kernel(const __grid_constant__ PrepBatchOf<kMax> b)
 {
   vlb::pdl_wait();
   __shared__ uint32_t red[16];
@@ -1243,8 +1252,11 @@ void launch_prep(vlb_ctx* ctx, PrepBatch& prep, int n)
   }
   VLB_LAUNCHED(ctx, 1);
   dim3 const grid((unsigned)(images * std::max(prep.p[0].BN / 64, 1)), n, 1);
-  if (split3) vlb::launch(ctx->stream, prep_filters_kernel<true>, grid, 512, 0, prep);
-  else        vlb::launch(ctx->stream, prep_filters_kernel<false>, grid, 512, 0, prep);
+  with_capacity(n, [&](auto capacity) {
+    constexpr int kMax = decltype(capacity)::value;
+    if (split3) vlb::launch(ctx->stream, prep_filters_kernel<true, kMax>, grid, 512, 0, first_preps<kMax>(prep));
+    else        vlb::launch(ctx->stream, prep_filters_kernel<false, kMax>, grid, 512, 0, first_preps<kMax>(prep));
+  });
 }
 
 // dY of a filter gradient as tile images, B(n, r) = dY[pixel, n, image] with r = pixel + Pp*image (Pp: the plane's P pixels rounded up to whole
@@ -1475,15 +1487,11 @@ template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 3, true>>() { ret
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 3, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 3, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 3, false>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, true>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<true, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 0, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 0, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 1, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 1, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 2, false>>() { return 80; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, true>>() { return 96; }
-template <> constexpr int kRegsAtLaunch<conv_half_gen_kernel<false, false>>() { return 96; }
 
 // Decides whether conv_half_kernel can take its input windows from tensor-map copies and, if so, fills the box geometry in p,
 // the tensor map and the shared-memory size.  Needs: reduction in blocks of 32 channels, unit stride, input rows a multiple
@@ -1797,14 +1805,17 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
   launch_prep(ctx, prep, b.n);
   size_t const smemBytes = std::max<size_t>((size_t)stages * stageBytes + patchBytes + 1024, 120u * 1024u);      // two CTAs never share an SM
   cudaError_t e;
-  auto go = [&](auto kernel) {
-    e = allow_large_smem<decltype(kernel)::value>(ctx->device);
-    if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, given, kTsThreads, smemBytes, b);
-  };
-#define VLB_TSG(split, nar) go(std::integral_constant<decltype(&conv_half_gen_kernel<split, nar>), &conv_half_gen_kernel<split, nar>>{})
-  if (split3) { if (BN <= 64) VLB_TSG(true, true); else VLB_TSG(true, false); }
-  else        { if (BN <= 64) VLB_TSG(false, true); else VLB_TSG(false, false); }
+  with_capacity(b.n, [&](auto capacity) {
+    constexpr int kMax = decltype(capacity)::value;
+    auto go = [&](auto kernel) {
+      e = allow_large_smem<decltype(kernel)::value, 96>(ctx->device);
+      if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, given, kTsThreads, smemBytes, first_problems<kMax>(b));
+    };
+#define VLB_TSG(split, nar) go(std::integral_constant<decltype(&conv_half_gen_kernel<split, nar, kMax>), &conv_half_gen_kernel<split, nar, kMax>>{})
+    if (split3) { if (BN <= 64) VLB_TSG(true, true); else VLB_TSG(true, false); }
+    else        { if (BN <= 64) VLB_TSG(false, true); else VLB_TSG(false, false); }
 #undef VLB_TSG
+  });
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
   int const rc = vlb::check_launch(ctx, where);

@@ -1401,11 +1401,11 @@ conv_ts_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtenso
 
 // The same for what the plain kernel's gather does not cover: channels that are no multiple of 32, filter groups, and the residue
 // classes of a strided data gradient (several problems in one launch, so that a small layer's classes share the chip).
-template <bool kSplit, bool kNarrow>
-__global__ void __launch_bounds__(kTsThreads, 1) conv_ts_gen_kernel(const __grid_constant__ TsProblems b)
+template <bool kSplit, bool kNarrow, int kMax>
+__global__ void __launch_bounds__(kTsThreads, 1) conv_ts_gen_kernel(const __grid_constant__ Problems<kMax> b)
 {
   int i = 0;
-  while (i + 1 < b.n && (int)blockIdx.x >= b.p[i + 1].ctaBeg) ++i;
+  if constexpr (kMax > 1) while (i + 1 < b.n && (int)blockIdx.x >= b.p[i + 1].ctaBeg) ++i;
   conv_ts_body<kSplit, 0, kNarrow, true, true>(b.p[i], nullptr, (int)blockIdx.x - b.p[i].ctaBeg, b.p[i].ctas);
 }
 
@@ -1442,10 +1442,19 @@ struct PrepFilters {
   long long sn, sq, gs;
   vlb::FastDiv divRun, divFT;       // by 8 * FH*FW and FH*FW (set by launch_prep)
 };
-struct PrepBatch { PrepFilters p[kMaxTsProblems]; };
+template <int kMax> struct PrepBatchOf { PrepFilters p[kMax]; };
+using PrepBatch = PrepBatchOf<kMaxTsProblems>;
 
-template <bool kSplit>
-__global__ void __launch_bounds__(256) prep_filters_kernel(const __grid_constant__ PrepBatch b)
+template <int kMax>
+PrepBatchOf<kMax> first_preps(PrepBatch const& b)
+{
+  PrepBatchOf<kMax> q;
+  std::copy(b.p, b.p + kMax, q.p);
+  return q;
+}
+
+template <bool kSplit, int kMax>
+__global__ void __launch_bounds__(256) prep_filters_kernel(const __grid_constant__ PrepBatchOf<kMax> b)
 {
   vlb::pdl_wait();
   PrepFilters const& p = b.p[blockIdx.z];
@@ -1487,8 +1496,8 @@ __global__ void __launch_bounds__(256) prep_filters_kernel(const __grid_constant
 // (row, q, tap) at row * (32 * FTp + 1) + q * FTp + tap, FTp odd: the reads of a warp (four rows x eight chunks) fall into 32 banks.
 constexpr int kPrepRows = 8, kMaxPrepTaps = 45;
 
-template <bool kSplit>
-__global__ void __launch_bounds__(256) prep_filters_tile_kernel(const __grid_constant__ PrepBatch b)
+template <bool kSplit, int kMax>
+__global__ void __launch_bounds__(256) prep_filters_tile_kernel(const __grid_constant__ PrepBatchOf<kMax> b)
 {
   vlb::pdl_wait();
   extern __shared__ float prepSmem[];
@@ -1588,13 +1597,19 @@ void launch_prep(vlb_ctx* ctx, PrepBatch& prep, int n)
   if (whole && FT <= kMaxPrepTaps && elements >= 600000) {
     dim3 const grid(vlb::ceil_div(rows, kPrepRows), blocks, n);
     size_t const smem = sizeof(float) * kPrepRows * (32 * (size_t)(FT | 1) + 1);
-    if (split3) vlb::launch(ctx->stream, prep_filters_tile_kernel<true>, grid, 256, smem, prep);
-    else        vlb::launch(ctx->stream, prep_filters_tile_kernel<false>, grid, 256, smem, prep);
+    with_capacity(n, [&](auto capacity) {
+      constexpr int kMax = decltype(capacity)::value;
+      if (split3) vlb::launch(ctx->stream, prep_filters_tile_kernel<true, kMax>, grid, 256, smem, first_preps<kMax>(prep));
+      else        vlb::launch(ctx->stream, prep_filters_tile_kernel<false, kMax>, grid, 256, smem, first_preps<kMax>(prep));
+    });
     return;
   }
   dim3 const grid(vlb::ceil_div(rows, 32), groups, n);
-  if (split3) vlb::launch(ctx->stream, prep_filters_kernel<true>, grid, 256, 0, prep);
-  else        vlb::launch(ctx->stream, prep_filters_kernel<false>, grid, 256, 0, prep);
+  with_capacity(n, [&](auto capacity) {
+    constexpr int kMax = decltype(capacity)::value;
+    if (split3) vlb::launch(ctx->stream, prep_filters_kernel<true, kMax>, grid, 256, 0, first_preps<kMax>(prep));
+    else        vlb::launch(ctx->stream, prep_filters_kernel<false, kMax>, grid, 256, 0, first_preps<kMax>(prep));
+  });
 }
 
 // dY of a filter gradient as tile images, B(n, r) = dY[pixel, n, image] with r = pixel + P*image, for planes that are a multiple of
@@ -1744,10 +1759,6 @@ template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 0, true>>() { retu
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 0, false>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 1, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 1, false>>() { return 128; }
-template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<true, true>>() { return 128; }
-template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<true, false>>() { return 128; }
-template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<false, true>>() { return 128; }
-template <> constexpr int kRegsAtLaunch<conv_ts_gen_kernel<false, false>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 0, false, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 1, false, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false>>() { return 96; }
@@ -2102,14 +2113,17 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
   launch_prep(ctx, prep, b.n);
   size_t const smemBytes = std::max<size_t>((size_t)stages * stageBytes + sumBytes + 1024, 120u * 1024u);      // two CTAs never share an SM
   cudaError_t e;
-  auto go = [&](auto kernel) {
-    e = allow_large_smem<decltype(kernel)::value>(ctx->device);
-    if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, given, kTsThreads, smemBytes, b);
-  };
-#define VLB_TSG(split, nar) go(std::integral_constant<decltype(&conv_ts_gen_kernel<split, nar>), &conv_ts_gen_kernel<split, nar>>{})
-  if (split3) { if (BN <= 64) VLB_TSG(true, true); else VLB_TSG(true, false); }
-  else        { if (BN <= 64) VLB_TSG(false, true); else VLB_TSG(false, false); }
+  with_capacity(b.n, [&](auto capacity) {
+    constexpr int kMax = decltype(capacity)::value;
+    auto go = [&](auto kernel) {
+      e = allow_large_smem<decltype(kernel)::value, 128>(ctx->device);
+      if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, given, kTsThreads, smemBytes, first_problems<kMax>(b));
+    };
+#define VLB_TSG(split, nar) go(std::integral_constant<decltype(&conv_ts_gen_kernel<split, nar, kMax>), &conv_ts_gen_kernel<split, nar, kMax>>{})
+    if (split3) { if (BN <= 64) VLB_TSG(true, true); else VLB_TSG(true, false); }
+    else        { if (BN <= 64) VLB_TSG(false, true); else VLB_TSG(false, false); }
 #undef VLB_TSG
+  });
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
   int const rc = vlb::check_launch(ctx, where);

@@ -95,8 +95,31 @@ struct Params {
 };
 
 // Several contractions in one launch of conv_ts_gen_kernel (the residue classes of a strided data gradient), each with CTAs of its own.
+// Launches pass the smallest block of parameters that holds the problems (with_capacity): one of 16 is 9.7 KB, which a launch of one
+// problem then carries for nothing and reads its own through an index.  Always 16 / the smallest block: transposed convolution 35 x 47, stride 2 68.3 / 64.4 us,
+// AlexNet step of 128 images 4480 / 4356, forward and gradients of 64 -> 40 channels in 4 groups, 1x1, stride 3 43.0 / 42.0 (a process in which the
+// unchanged code took 42.0 and 43.0).
 constexpr int kMaxTsProblems = 16;
-struct TsProblems { int n; Params p[kMaxTsProblems]; };
+template <int kMax> struct Problems { int n; Params p[kMax]; };
+using TsProblems = Problems<kMaxTsProblems>;
+
+// f(std::integral_constant<int, kMax>) for the smallest capacity that holds n: one (forward, stride 1, shuffled columns), the four classes of stride 2, 16.
+template <class F>
+inline void with_capacity(int n, F const& f)
+{
+  if (n <= 1) f(std::integral_constant<int, 1>{});
+  else if (n <= 4) f(std::integral_constant<int, 4>{});
+  else f(std::integral_constant<int, kMaxTsProblems>{});
+}
+
+template <int kMax>
+inline Problems<kMax> first_problems(TsProblems const& b)
+{
+  Problems<kMax> q;
+  q.n = b.n;
+  std::copy(b.p, b.p + kMax, q.p);
+  return q;
+}
 
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(void const* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -390,18 +413,18 @@ inline bool aligned16(void const* p) { return (((uintptr_t)p) & 15) == 0; }
 template <auto kKernel> constexpr int kRegsAtLaunch() { return 0; }
 
 // The opt-in to more than 48 KB of dynamic shared memory, once per kernel and device instead of before every launch.
-template <auto kKernel>
+template <auto kKernel, int kRegs = kRegsAtLaunch<kKernel>()>
 cudaError_t allow_large_smem(int device)
 {
   static bool done[64] = {};
   if (device >= 0 && device < 64 && done[device]) return cudaSuccess;
   cudaError_t e = vlb::allow_max_dynamic_smem(kKernel);
-  if (e == cudaSuccess && kRegsAtLaunch<kKernel>() > 0) {
+  if (e == cudaSuccess && kRegs > 0) {
     // conv_ts_kernel redistributes registers between its warps (setmaxnreg) on the premise that every thread starts with
     // exactly this many; a build that gave it another count must not run (the hand-over would wait for registers for ever)
     cudaFuncAttributes attr;
     e = cudaFuncGetAttributes(&attr, kKernel);
-    if (e == cudaSuccess && attr.numRegs != kRegsAtLaunch<kKernel>()) e = cudaErrorInvalidDeviceFunction;
+    if (e == cudaSuccess && attr.numRegs != kRegs) e = cudaErrorInvalidDeviceFunction;
   }
   if (e == cudaSuccess && device >= 0 && device < 64) done[device] = true;
   return e;
