@@ -4,10 +4,10 @@
 // Every contraction on the path is D[m][n] = sum_r A(m,r) * B(n,r) with fp32 accumulation
 // in tensor memory, 128 x BN output tile, reduction in blocks of 32.  Two kernels:
 //
-//   conv_ts_kernel   convolution forward and data gradient, the filter gradient and fully connected layers where the
-//                    reduction runs along memory: the gathered operand goes to tensor memory, only the filter tiles to
-//                    shared memory (further down).  conv_ts_gen_kernel is the same body for any stride, dilation,
-//                    channel count and filter groups.
+//   conv_ts_kernel   forward convolution and fully connected layers: the gathered operand goes to tensor memory, only the
+//                    filter tiles to shared memory (further down).  conv_ts_gen_kernel is the same body for any stride, dilation,
+//                    channel count and filter groups, forward and for data gradients with few channels per group.  The
+//                    other gradients have conv_half.cu's kernels.
 //   tc_gemm_kernel   the other filter gradients and fully connected layers, and convolutions whose filter support
 //                    exceeds the tap tables: both operands in shared memory, warp-specialised:
 //     warps 0-3   fp32 drain of the accumulation chains, then epilogue: tcgen05.ld the accumulator
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(Params p)
 }
 
 // ------------------------------------------------------------------ convolution with the gathered operand in tensor memory
-// fprop and stride-1 dgrad: D[m][n] = sum_r A(m,r) B(n,r), m = output pixel (ho,wo,image), r = (fh,fw,c).
+// fprop: D[m][n] = sum_r A(m,r) B(n,r), m = output pixel (ho,wo,image), r = (fh,fw,c).
 // In tc_gemm_kernel both operands are read from shared memory by every MMA, and the shared-memory
 // banks (MMA reads + producer stores + bulk-copy writes) are the unit that saturates first.  Here the
 // gathered operand A never touches shared memory: one producer thread per output pixel (= TMEM lane)
@@ -677,8 +677,8 @@ __device__ __forceinline__ int ts_chains(int numIter, int second, int chainShift
 // (one box of boxH x boxW pixels x 32 channels per channel block and tile, zero-filled outside the image by the copy
 // engine, two buffers), instead of gathering them from global memory with per-thread loads.  xmap: the 4-D tensor map
 // (H, W, C, N) of the gathered tensor; unused otherwise.
-// kMode 2 (filter gradient): rows are (tap, channel), the reduction runs over the output pixels; the loader thread has the run of 32
-// pixels (plus up to three in front, so that the copy starts on a 16-byte boundary) of every row delivered per k-block.
+// kMode 2 (fully connected forward): the reduction index is contiguous in a row; the loader thread has the run of 32 values of every row
+// delivered per k-block.
 constexpr int kWgRowWords = 36;                         // words per row of an x run in shared memory (144 bytes: 16-byte loads of 8 rows hit 32 banks)
 constexpr int kWgRowBytes = kWgRowWords * 4;
 constexpr int kWgStageBytes = BM * kWgRowBytes;         // 18432
@@ -771,9 +771,8 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
   if (warp == kEpilogueWarps) tmem_alloc(smem_u32(&tmemBase), tmemCols);
   if ((int)threadIdx.x < p.a.FH * p.a.FW) {
     int const fh = (int)threadIdx.x % p.a.FH, fw = (int)threadIdx.x / p.a.FH;
-    if (kWg)       tapLut[threadIdx.x] = make_int2((fw * p.a.dx - p.a.pl) * p.a.H + fh * p.a.dy - p.a.pt, fh * p.a.dy - p.a.pt);   // {shift of the tap in the flattened plane, its row offset}
-    else if (kTma) tapLut[threadIdx.x] = make_int2(fw * p.a.dx * p.boxH + fh * p.a.dy, fh | (fw << 5));
-    else           tapLut[threadIdx.x] = make_int2((fw * p.a.dx - p.a.pl) * p.a.H + fh * p.a.dy - p.a.pt, fh | (fw << 5));
+    if (kTma) tapLut[threadIdx.x] = make_int2(fw * p.a.dx * p.boxH + fh * p.a.dy, fh | (fw << 5));
+    else      tapLut[threadIdx.x] = make_int2((fw * p.a.dx - p.a.pl) * p.a.H + fh * p.a.dy - p.a.pt, fh | (fw << 5));
   }
   tc_fence_before();
   vlb::pdl_wait();        // (everything above touches this CTA's own shared and tensor memory only)
@@ -1134,28 +1133,21 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
     // (the warpgroup of warps 16-19 exists in the row mode only and keeps a handful of registers, like the warps 4-7)
     if (kWg) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;" ::: "memory");
     if (kWg && warp == kTsRunWarp && lane == 0) {
-      // The run of k-block j (numbered over the CTA's life) -- 36 pixels x cPer channels per
-      // tap of the tile, from the plane of image r / P starting at pixel r % P + shift of the tap, rounded down to four pixels (P:
-      // the plane rounded up to whole k-blocks; the tile images hold zeros for the pixels added; pixels before the plane's first
-      // or past its last one -- a tap that leaves the image to the left or right, a k-block past the end of the batch -- arrive as
-      // zeros) -- goes into buffer j % xStages as soon as the producers have let go of the run of k-block j - xStages.
-      int const taps = p.a.FH * p.a.FW, P = p.plane, nX = p.xStages;
+      // The run of k-block j (numbered over the CTA's life) -- 36 words (the pitch; 32 are used) of each of the tile's 128 rows; what lies behind the
+      // rows' end, where the ranges do not divide, arrives as zeros -- goes into buffer j % xStages as soon as the producers have let go of the
+      // run of k-block j - xStages.
+      int const nX = p.xStages;
       int buf = 0; uint32_t ph = 1;                        // first use of a buffer: nothing to wait for
       bool ok = true;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
         int const tmf = (cta + ts * ctas) / p.tilesN;
-        int const split = tmf / p.tilesM, t = tmf - split * p.tilesM, cb = t / p.tapGroups, tg = t - cb * p.tapGroups;
-        int const tap0 = tg * p.tapsPerTile, nTaps = min(p.tapsPerTile, taps - tap0);
-        long long const r0 = (long long)split * numIter * BK;
-        int img = (int)(r0 / P), pix0 = (int)(r0 - (long long)img * P);
-        for (int it = 0; it < numIter; ++it) {
+        int const split = tmf / p.tilesM, t = tmf - split * p.tilesM;
+        int r = split * numIter * BK;
+        for (int it = 0; it < numIter; ++it, r += BK) {
           if (!mbar_wait(smem_u32(&emptyX[buf]), ph)) { atomicExch(p.status, 12); ok = false; break; }
-          mbar_arrive_expect_tx(smem_u32(&fullX[buf]), (uint32_t)(nTaps * p.cPer * kWgRowBytes));
-          for (int tl = 0; tl < nTaps; ++tl)
-            tma_load_3d(xTile0 + (uint32_t)buf * xTileBytes + (uint32_t)(tl * p.cPer * kWgRowBytes), xmap,
-                        pix0 + (tapLut[tap0 + tl].x & ~3), cb * p.cPer, img, smem_u32(&fullX[buf]));
+          mbar_arrive_expect_tx(smem_u32(&fullX[buf]), (uint32_t)kWgStageBytes);
+          tma_load_3d(xTile0 + (uint32_t)buf * xTileBytes, xmap, r < p.R ? r : 0, t * BM, r < p.R ? 0 : 1, smem_u32(&fullX[buf]));
           if (++buf == nX) { buf = 0; ph ^= 1u; }
-          pix0 += BK; if (pix0 >= P) { pix0 -= P; ++img; }
         }
       }
     }
@@ -1197,55 +1189,20 @@ __device__ __forceinline__ void conv_ts_body(Params const& p, CUtensorMap const*
     };
 
     if (kWg) {
-      // This thread's row: channel (row % cPer) of the tile's local tap row / cPer -- the same tap for the whole warp.  A k-block
-      // is 32 consecutive output pixels; the row's 36-pixel run lies in shared memory, the wanted 32 start `s` pixels in.
-      int const row = quarter * 32 + lane;
-      int const tl = (quarter * 32) / p.cPer;
-      int const H = p.a.H, P = p.plane, nX = p.xStages;
+      // This thread's row of the tile: the 32 values of a k-block lie in shared memory, in the run that the loader has had delivered.
+      uint32_t const rowOff = (uint32_t)((quarter * 32 + lane) * kWgRowBytes), nX = (uint32_t)p.xStages;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
-        int const tmf = (cta + ts * ctas) / p.tilesN;
-        int const split = tmf / p.tilesM, t = tmf - split * p.tilesM, tg = t % p.tapGroups;
-        int const tap = tg * p.tapsPerTile + tl;
-        bool const active = tap < taps;                                   // a tap the filter does not have: rows of zeros, never stored
-        int2 const te = tapLut[active ? tap : 0];
-        int const s = te.x & 3, dh = te.y;
-        int const itFirst = (int)((gi ^ grp) & 1);
-        int pb = (int)(((long long)split * numIter + itFirst) * BK % P);      // first pixel of the k-block inside its image
-        for (int it = itFirst; it < numIter; it += kTsGroups) {
-          uint32_t const xs = (uint32_t)(gi + it);
-          int const buf = (int)(xs % (uint32_t)nX);
-          if (!mbar_wait(smem_u32(&fullX[buf]), (xs / (uint32_t)nX) & 1u)) { atomicExch(p.status, 11); ok = false; break; }
-          uint32_t const src = xTile0 + (uint32_t)buf * xTileBytes + (uint32_t)(row * kWgRowBytes);
-          float w[kWgRowWords];
-#pragma unroll
-          for (int j = 0; j < kWgRowWords / 4; ++j) lds128(src + 16u * j, *reinterpret_cast<float(*)[4]>(&w[4 * j]));
-          // pixels whose tap row leaves the image above or below: output row ho + dh outside [0, H) -- the same for every lane's row
-          int const ho = (pb + lane) % H;
-          pb += kTsGroups * BK; while (pb >= P) pb -= P;
-          uint32_t const zm = active ? __ballot_sync(0xffffffffu, (unsigned)(ho + dh) >= (unsigned)H) : 0xffffffffu;
+        for (int it = (int)((gi ^ grp) & 1); it < numIter; it += kTsGroups) {
+          uint32_t const xs = (uint32_t)(gi + it), use = xs / nX;
+          int const buf = (int)(xs - use * nX);
+          // With an odd number of buffers the buffer's previous run belongs to the other group, which may be behind: this run's phase can be told from
+          // the one two before only once that run has been let go of.  (The run before it was this group's own.)
+          if ((use > 0 && !mbar_wait(smem_u32(&emptyX[buf]), (use - 1u) & 1u)) ||
+              !mbar_wait(smem_u32(&fullX[buf]), use & 1u)) { atomicExch(p.status, 11); ok = false; break; }
+          uint32_t const src = xTile0 + (uint32_t)buf * xTileBytes + rowOff;
           float v[32];
-          switch (s) {
-            case 0:
 #pragma unroll
-              for (int k = 0; k < 32; ++k) v[k] = w[k];
-              break;
-            case 1:
-#pragma unroll
-              for (int k = 0; k < 32; ++k) v[k] = w[k + 1];
-              break;
-            case 2:
-#pragma unroll
-              for (int k = 0; k < 32; ++k) v[k] = w[k + 2];
-              break;
-            default:
-#pragma unroll
-              for (int k = 0; k < 32; ++k) v[k] = w[k + 3];
-              break;
-          }
-          if (zm) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = ((zm >> k) & 1u) ? 0.f : v[k];
-          }
+          for (int j = 0; j < 8; ++j) lds128(src + 16u * j, *reinterpret_cast<float(*)[4]>(&v[4 * j]));
           if (!hand_over(v, it)) { ok = false; break; }
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&emptyX[buf]));     // this warp's loads from the run have completed (their values were used above)
@@ -1706,19 +1663,16 @@ size_t b_tiles_bytes(vlb_ctx* ctx, int N, int BN, int numKb)
   return (bytes + 255) & ~(size_t)255;
 }
 
-// The filter bank of one group, reduction in blocks of 32 channels (conv_ts_kernel): forward, or flipped and transposed for the data gradient
-// of a stride-1 convolution.
-float const* prep_conv_tiles(vlb_ctx* ctx, float const* f, vlb::ConvGeom const& g, int BN, int numKb, bool dgrad, size_t extraBytes)
+// The filter bank of one group, reduction in blocks of 32 channels (conv_ts_kernel).
+float const* prep_conv_tiles(vlb_ctx* ctx, float const* f, vlb::ConvGeom const& g, int BN, int numKb, size_t extraBytes)
 {
-  int const N = dgrad ? g.C : g.K;
-  float* tiles = (float*)vlb::workspace(ctx, b_tiles_bytes(ctx, N, BN, numKb) + extraBytes);
+  float* tiles = (float*)vlb::workspace(ctx, b_tiles_bytes(ctx, g.K, BN, numKb) + extraBytes);
   if (!tiles) return nullptr;
   PrepBatch prep = {};
   PrepFilters& q = prep.p[0];
-  q.out = tiles; q.f = f; q.BN = BN; q.numKb = numKb; q.tilesPerGroup = vlb::ceil_div(N, BN); q.rows = q.tilesPerGroup * BN; q.cols = N;
-  q.unit = 32; q.upk = 1; q.tapsH = q.FH = g.FH; q.tapsW = q.FW = g.FW; q.C = dgrad ? g.K : g.C;
-  q.bh = dgrad ? g.FH - 1 : 0; q.bw = dgrad ? g.FW - 1 : 0; q.ah = q.aw = dgrad ? -1 : 1;
-  q.sn = dgrad ? 1 : g.C; q.sq = dgrad ? g.C : 1; q.per = 8;
+  q.out = tiles; q.f = f; q.BN = BN; q.numKb = numKb; q.tilesPerGroup = vlb::ceil_div(g.K, BN); q.rows = q.tilesPerGroup * BN; q.cols = g.K;
+  q.unit = 32; q.upk = 1; q.tapsH = q.FH = g.FH; q.tapsW = q.FW = g.FW; q.C = g.C;
+  q.ah = q.aw = 1; q.sn = g.C; q.sq = 1; q.per = 8;
   launch_prep(ctx, prep, 1);
   return tiles;
 }
@@ -1759,8 +1713,6 @@ template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 0, true>>() { retu
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 0, false>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 1, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 1, false>>() { return 128; }
-template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 0, false, true>>() { return 128; }
-template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 1, false, true>>() { return 128; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<true, 2, false, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_ts_kernel<false, 2, false>>() { return 96; }
@@ -1858,7 +1810,7 @@ bool plan_windows(vlb_ctx* ctx, Params& p, CUtensorMap* map, size_t* smemBytes, 
   return true;
 }
 
-// fprop / stride-1 dgrad with the gathered operand in tensor memory (p.bTiles set, p.a a convolution operand).
+// Forward convolution with the gathered operand in tensor memory (p.bTiles set, p.a a convolution operand).
 int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
 {
   bool split3 = ctx->precision == VLB_PRECISION_3XTF32;
@@ -1897,15 +1849,13 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
     e = allow_large_smem<decltype(kernel)::value>(ctx->device);
     if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, grid, kTsThreads, smemBytes, p, map);
   };
-#define VLB_TS(split, mode, nar, fine) go(std::integral_constant<decltype(&conv_ts_kernel<split, mode, nar, fine>), &conv_ts_kernel<split, mode, nar, fine>>{})
-  if (split3 && p.fine && !narrow) {
-    if (windows) VLB_TS(true, 1, false, true); else VLB_TS(true, 0, false, true);
-  } else if (split3) {
-    if (windows) { if (narrow) VLB_TS(true, 1, true, false); else VLB_TS(true, 1, false, false); }
-    else         { if (narrow) VLB_TS(true, 0, true, false); else VLB_TS(true, 0, false, false); }
+#define VLB_TS(split, mode, nar) go(std::integral_constant<decltype(&conv_ts_kernel<split, mode, nar>), &conv_ts_kernel<split, mode, nar>>{})
+  if (split3) {
+    if (windows) { if (narrow) VLB_TS(true, 1, true); else VLB_TS(true, 1, false); }
+    else         { if (narrow) VLB_TS(true, 0, true); else VLB_TS(true, 0, false); }
   } else {
-    if (windows) { if (narrow) VLB_TS(false, 1, true, false); else VLB_TS(false, 1, false, false); }
-    else         { if (narrow) VLB_TS(false, 0, true, false); else VLB_TS(false, 0, false, false); }
+    if (windows) { if (narrow) VLB_TS(false, 1, true); else VLB_TS(false, 1, false); }
+    else         { if (narrow) VLB_TS(false, 0, true); else VLB_TS(false, 0, false); }
   }
 #undef VLB_TS
   if (record) { cudaEventRecord(rec.stop, ctx->stream); ctx->prof.push_back(rec); }
@@ -1927,7 +1877,7 @@ int pick_splits(vlb_ctx* ctx, int tiles, int numKb, int minKbPerSplit)
 }
 
 // conv_ts_kernel in its row mode (kMode 2): rows whose reduction index is contiguous in memory, delivered by the 3-D tensor map `map`
-// (run of 36 elements x cPer rows x 1).  p holds the tiling (cPer, tapsPerTile, tapGroups, tilesM, tilesN, splits, kbPerSplit,
+// (run of 36 elements x 128 rows x 1).  p holds the tiling (cPer, tapsPerTile, tapGroups, tilesM, tilesN, splits, kbPerSplit,
 // kbTot), the operand geometry, the tile images and the epilogue.
 int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* where)
 {
@@ -1965,7 +1915,7 @@ int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* whe
 }
 
 // Fully connected layers at small batch are bound by the one pass over the weights (fc6 of VGG-16: 411 MB against 13 GFLOP at
-// batch 64).  All three passes run through conv_ts_kernel, whose A operand goes from global memory to tensor memory without a
+// batch 64).  All three passes run through conv_ts_kernel or, backward, conv_half_kernel (conv_half.cu), whose A operand goes from global memory to tensor memory without a
 // shared-memory tile of its own, each with the weights (or their gradient) as the operand that is read or written exactly once:
 //   forward   Y(K x N) = F'(K x V) X(V x N): rows = filters, the reduction index v is contiguous in a row -> row mode, X as tile images;
 //   data      dX(V x N) = F(V x K) dY(K x N): a 1 x 1 convolution over the "plane" of V elements with K channels, dY as its N filters;
@@ -2228,7 +2178,7 @@ int conv_fprop_tc(vlb_ctx* ctx, ConvGeom const& g, float* Y, float outMult, floa
     p.splits = split_few_tiles(ctx->smCount, ceil_div(p.M, BM) * ceil_div(p.N, p.BN), p.numKb, &p.kbPerSplit, 8);
     p.numKb = p.splits * p.kbPerSplit;
     size_t const nOut = (size_t)p.M * g.K, partBytes = p.splits > 1 ? sizeof(float) * nOut * p.splits : 0;
-    p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, false, partBytes);
+    p.bTiles = prep_conv_tiles(ctx, F, g, p.BN, p.numKb, partBytes);
     if (!p.bTiles) return ctx->lastError;
     if (p.splits == 1) return launch_ts(ctx, p, "conv_fprop_ts");
     SumEpilogue epi;
