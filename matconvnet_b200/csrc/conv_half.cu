@@ -22,7 +22,7 @@ namespace {
 // existing networks the other way; a backward pass decides nothing.
 //
 // How A's rows get to tensor memory (kMode):
-//   0  a thread per row gathers fp32 values, finds their largest, converts them (few channels, 1x1 filters, general gather): 2000 cycles per k-block
+//   0  a thread per row gathers fp32 values, finds their largest, converts them (few channels, 1x1 filters): 2000 cycles per k-block
 //   1  the same from input windows that tensor-map copies brought to shared memory
 //   2  the same from runs along the planes (filter gradient; rows are (tap, channel))
 //   3  sixteen 16-byte loads from a copy of the tensor that split_chunks_kernel has converted: 1150 cycles per k-block, bound by the bandwidth of the array
@@ -822,7 +822,7 @@ conv_half_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
   conv_half_body<kSplit, kMode, kNarrow, false>(p, &xmap, (int)blockIdx.x, (int)gridDim.x);
 }
 
-// The same for what the plain kernel's gather does not cover: channels that are no multiple of 32, filter groups, and the residue
+// The same from chunks (kMode 3) for what the plain kernel does not cover: channels that are no multiple of 32, filter groups, and the residue
 // classes of a strided data gradient (several problems in one launch, so that a small layer's classes share the chip).
 template <bool kSplit, bool kNarrow, int kMax>
 __global__ void __launch_bounds__(kTsThreads, 1) conv_half_gen_kernel(const __grid_constant__ Problems<kMax> b)

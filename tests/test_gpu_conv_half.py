@@ -143,3 +143,20 @@ def test_an_odd_number_of_run_buffers_keeps_the_groups_apart(gpu):
         _, df, _ = nn.vl_nnconv(x, f, None, dy, no_der_data=True, ctx=ctx)
         assert torch.equal(df, first)
     assert ctx.device_status() == 0
+
+
+def test_run_buffers_of_a_fully_connected_forward_pass(gpu):
+    """128-column tiles with the sum in shared memory leave three run buffers to the two groups of producers there too; the sums are the same ones."""
+    import torch
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(78)
+    x, f = mat.empty((4, 4, 512, 128)).normal_(generator=g), mat.empty((4, 4, 512, 256)).normal_(generator=g)
+    y = nn.vl_nnconv(x, f, None, ctx=ctx)
+    lib = ctx.lib
+    ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 8))
+    try:
+        for _ in range(50):
+            assert torch.equal(nn.vl_nnconv(x, f, None, ctx=ctx), y)
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+    assert ctx.device_status() == 0
