@@ -27,7 +27,10 @@ namespace {
 //   2  the same from runs along the planes (filter gradient; rows are (tap, channel))
 //   3  sixteen 16-byte loads from a copy of the tensor that split_chunks_kernel has converted: 1150 cycles per k-block, bound by the bandwidth of the array
 //      that is shared memory and L1 (tiles of B written and read 48 + 32 KB, chunks of A 40 KB, 128 bytes per clock); the MMAs take 768
-//   4  the same for filter gradients, chunks of eight images
+//   4  the same for filter gradients, chunks of eight images, a k-block being 64 images of a pixel
+//   5  filter gradients of fewer images: a k-block is several rows of a column, wherever the filter tap puts them, so the chunks hold fp32 values, which a
+//      thread converts as in the modes 0 to 2.  (Split beforehand they would need one power of two for all rows that some tap may put side by side, the
+//      whole column: an infinity or a very large value in a row that a tap never reads would then cost that tap's sums their digits.)
 // Warps: 0-7 drain and epilogue; 8, 9 MMA issue (one lane each; warp 8 also allocates TMEM), issuer q takes every other k-block; 10 loader of B's tiles; 11
 // forwarder (when the tile of a k-block has landed it arrives on that k-block's A-stage barrier, so that an MMA thread waits on one barrier for both);
 // 12-19 producers, two groups of four warps (one per TMEM lane quarter), group g fills the A stages of the k-blocks g, g + 2, ...
@@ -141,7 +144,8 @@ static_assert(kTsBStages < kTsDoneRing, "the loader must not be able to fall a w
 template <bool kSplit, int kMode, bool kNarrow, bool kGen>
 __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap const* xmap, int const cta, int const ctas)
 {
-  constexpr bool kTma = kMode == 1, kWg = kMode == 2, kImages = kMode == 4;      // (0: per-thread gather, 3: gather of a tensor that was split beforehand)
+  constexpr bool kTma = kMode == 1, kWg = kMode == 2, kImages = kMode == 4 || kMode == 5;      // (0: per-thread gather, 3: gather of a tensor that was split beforehand)
+  constexpr bool kChunks = kMode == 3 || kMode == 4;      // the producers only carry
   extern __shared__ uint8_t smemRaw[];
   __shared__ __align__(8) uint64_t fullA[4], doneK[kTsDoneRing], fullB[kTsBStages];
   __shared__ __align__(8) uint64_t tFree[4], turn[2], fullX[kTsXStages], emptyX[kTsXStages];
@@ -207,7 +211,7 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
     // sum lives in registers (one TMEM lane = one output row per thread; a thread has half of the row's columns).  With four warps, each with whole
     // rows, the drain was what bounded the kernel: 1080 cycles per k-block, a quarter of them for the stores, where the MMAs take 768.
     if (kWg) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;" ::: "memory");
-    else if (kMode >= 3) asm volatile("setmaxnreg.inc.sync.aligned.u32 120;" ::: "memory");
+    else if (kChunks) asm volatile("setmaxnreg.inc.sync.aligned.u32 120;" ::: "memory");
     else     asm volatile("setmaxnreg.inc.sync.aligned.u32 112;" ::: "memory");
     uint32_t const lanes = tmemAcc + ((uint32_t)((warp & 3) * 32) << 16);
     int const row = (warp & 3) * 32 + lane, half = warp >> 2;
@@ -553,7 +557,7 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
   } else {
     // ============================== producers ==============================
     if (kWg) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;" ::: "memory");
-    else if (kMode < 3) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;" ::: "memory");      // (kMode 3, 4: the 96 of the launch)
+    else if (!kChunks) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;" ::: "memory");      // (kMode 3, 4: the 96 of the launch)
     int const grp = (warp - kTsFirstProducer) >> 2;
     int const quarter = warp & 3;                       // the TMEM lanes this warp may access
     int const row = quarter * 32 + lane;
@@ -696,9 +700,10 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
         gi += numIter;
       }
     } else if (kImages) {
-      // This warp's unit: 32 channels (a lane each) of one filter tap.  A k-block's eight 16-byte loads for hi and eight for lo are eight images at a
-      // pixel each; lanes are neighbours in memory, and which pixels exist is the same for all of them.
-      int const g = 1 << p.gShift, rows = 8 >> p.gShift, W = p.a.W, H = p.a.H;
+      // This warp's unit: 32 channels (a lane each) of one filter tap.  A k-block is eight chunks of eight images, 16 bytes for hi and 16 for lo (kMode 5:
+      // for the first four and for the other four): one pixel (kMode 4), or 8 >> gShift output rows of a column.  Lanes are neighbours in memory, and which
+      // pixels exist is the same for all of them.
+      int const gShift = kMode == 4 ? 3 : p.gShift, g = 1 << gShift, rows = 8 >> gShift, W = p.a.W, H = p.a.H;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
         int const tmf = p.dTilesN(cta + ts * ctas), split = p.dTilesM(tmf), t = tmf - split * p.tilesM, fg = t / p.tilesPerGroup;
         int const u = (t - fg * p.tilesPerGroup) * 4 + quarter, cb = p.dTaps(u), tap = u - cb * taps, c = cb * 32 + lane;
@@ -710,20 +715,34 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
           int const kb = split * numIter + it, col = p.dHo(kb), rb = kb - col * p.rowBlocks, n = p.dWo(col);      // (dHo, dWo: by rowBlocks and Wo)
           int const wx = (col - n * p.a.Wo) * p.a.sx + dw, h0 = rb * rows;
           bool const colOn = active && (unsigned)wx < (unsigned)W && n < p.nGroups;
-          uint4 h[8], l[8];
+          auto chunk = [&](int j, bool& on) -> uint4 const* {
+            int const ho = h0 + (j >> gShift), hx = ho * p.a.sy + dh;
+            on = colOn && ho < p.a.Ho && (unsigned)hx < (unsigned)H;
+            return on ? xq + (((long long)(n * g + (j & (g - 1))) * W + wx) * H + hx) * p.channels : p.zero;
+          };
+          if constexpr (kMode == 4) {
+            uint4 h[8], l[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            int const ho = h0 + (j >> p.gShift), hx = ho * p.a.sy + dh;
-            bool const on = colOn && ho < p.a.Ho && (unsigned)hx < (unsigned)H;
-            uint4 const* const q = on ? xq + (((long long)(n * g + (j & (g - 1))) * W + wx) * H + hx) * p.channels : p.zero;
-            h[j] = __ldg(q);
-            if (kSplit) l[j] = __ldg(on ? q + p.aLo : p.zero);
+            for (int j = 0; j < 8; ++j) {
+              bool on;
+              uint4 const* const q = chunk(j, on);
+              h[j] = __ldg(q);
+              if (kSplit) l[j] = __ldg(on ? q + p.aLo : p.zero);
+            }
+            int const hx = h0 * p.a.sy + dh;
+            int const ke = colOn && (unsigned)hx < (unsigned)H ? __ldg(eq + (((long long)n * W + wx) * H + hx) * p.channels) : 0;
+            ok = stage_in([&](uint32_t aAddr) { tmem_st32(aAddr, h); if (kSplit) tmem_st32(aAddr + 32u, l); }, ke);
+          } else {
+            float v[kTsK];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              bool on;
+              float4 const* const q = reinterpret_cast<float4 const*>(chunk(j, on));
+              *reinterpret_cast<float4*>(v + 8 * j) = __ldg(q);
+              *reinterpret_cast<float4*>(v + 8 * j + 4) = __ldg(on ? q + p.aLo : q);
+            }
+            ok = hand_over(v);
           }
-          int const hx0 = h0 * p.a.sy + dh;
-          int ke = 0;
-          if (rows > 1) { if (colOn) ke = __ldg(eq + ((long long)n * W + wx) * p.channels); }
-          else if (colOn && (unsigned)hx0 < (unsigned)H) ke = __ldg(eq + (((long long)n * W + wx) * H + hx0) * p.channels);
-          ok = stage_in([&](uint32_t aAddr) { tmem_st32(aAddr, h); if (kSplit) tmem_st32(aAddr + 32u, l); }, ke);
           if (!ok) break;
         }
         gi += numIter;
@@ -916,93 +935,69 @@ split_chunks_kernel(uint4* __restrict__ hi, long long loOff, int8_t* __restrict_
   exps[((long long)img * c64 + cb) * HW + pix] = (int8_t)ke;
 }
 
-// The input of a filter gradient with the images along the reduction (kMode 4), split once instead of once per filter tap and column tile: chunks of
+// The input of a filter gradient with the images along the reduction, laid out once instead of gathered per filter tap and column tile: chunks of
 // eight images of one pixel and channel, channels next to one another.  No filter tap, stride or plane size then moves a chunk off its 16-byte boundary.
-// A warp takes eight pixels of a column (rows) by four channels: 32-byte pieces in, 64-byte pieces out.
-// kG = 8: the scale exponent of a channel belongs to the 64 images of a pixel, which a thread holds in registers.  kG < 8: a k-block is several rows of
-// a column, wherever the filter tap puts them, so the exponent belongs to the whole column of the 8 * kG images; the column is read twice, the second time
-// from L2.  grid (columns of eight pixels or whole columns * channel blocks of 32, groups)
-template <bool kSplit, int kG>
+// A warp takes eight pixels by four channels: 32-byte pieces in, 64-byte pieces out.
+// split_images_kernel (kMode 4): split, with one scale exponent for the 64 images of a pixel and channel, which a thread holds in registers.
+// grid (columns of eight pixels * channel blocks of 32, groups of 64 images)
+template <bool kSplit>
 __global__ void __launch_bounds__(256, 2)
 split_images_kernel(uint4* __restrict__ hi, long long loOff, int8_t* __restrict__ exps, uint4* __restrict__ zero, float const* __restrict__ x,
-                    int H, int W, int C, int N, int cBlocks)
+                    int HW, int C, int N, int cBlocks)
 {
   vlb::pdl_wait();
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *zero = make_uint4(0, 0, 0, 0);
   int const lane = (int)threadIdx.x & 31, place = (int)blockIdx.x / cBlocks, ng = (int)blockIdx.y;
   int const c = ((int)blockIdx.x - place * cBlocks) * 32 + ((int)threadIdx.x >> 5) * 4 + (lane & 3);
-  int const HW = H * W;
-  if (kG == 8) {
-    int const pix = place * 8 + (lane >> 2);
-    if (c >= C || pix >= HW) return;
-    float const* const src = x + ((long long)ng * 64 * C + c) * HW + pix;
-    float v[64];
-    long long const step = (long long)C * HW;
-    if (ng * 64 + 64 <= N) {
+  int const pix = place * 8 + (lane >> 2);
+  if (c >= C || pix >= HW) return;
+  float const* const src = x + ((long long)ng * 64 * C + c) * HW + pix;
+  float v[64];
+  long long const step = (long long)C * HW;
+  if (ng * 64 + 64 <= N) {
 #pragma unroll
-      for (int k = 0; k < 64; ++k) v[k] = __ldg(src + k * step);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 64; ++k) v[k] = ng * 64 + k < N ? __ldg(src + k * step) : 0.f;
-    }
-    float m0 = 0.f, m1 = 0.f;
-#pragma unroll
-    for (int k = 0; k < 64; k += 4) { m0 = max3(m0, fabsf(v[k]), fabsf(v[k + 1])); m1 = max3(m1, fabsf(v[k + 2]), fabsf(v[k + 3])); }
-    float const mx = fmaxf(m0, m1);
-    int const ke = mx > 0.f ? scale_exp(mx) : 0;
-    float const s = exp2i(ke), sl = exp2i(ke + 11);
-    uint64_t const s2 = pack2(s, s), sl2 = pack2(sl, sl);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      uint32_t h[4], l[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) split_pair<kSplit>(v[8 * i + 2 * e], v[8 * i + 2 * e + 1], s2, sl2, h[e], l[e]);
-      long long const at = ((long long)(ng * 8 + i) * HW + pix) * C + c;
-      hi[at] = make_uint4(h[0], h[1], h[2], h[3]);
-      if (kSplit) hi[loOff + at] = make_uint4(l[0], l[1], l[2], l[3]);
-    }
-    exps[((long long)ng * HW + pix) * C + c] = (int8_t)ke;
+    for (int k = 0; k < 64; ++k) v[k] = __ldg(src + k * step);
   } else {
-    if (c - (lane & 3) >= C) return;                    // (the whole warp)
-    bool const real = c < C;
-    float const* const src = x + ((long long)ng * 8 * kG * C + (real ? c : 0)) * HW + place * H;
-    auto fetch = [&](int h, int i, float (&v)[8]) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { int const n = i * 8 + e; v[e] = real && h < H && ng * 8 * kG + n < N ? __ldg(src + (long long)n * C * HW + h) : 0.f; }
-    };
-    float mx = 0.f;
-    for (int h0 = 0; h0 < H; h0 += 8) {
-#pragma unroll
-      for (int i = 0; i < kG; ++i) {
-        float v[8];
-        fetch(h0 + (lane >> 2), i, v);
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) mx = max3(mx, fabsf(v[e]), fabsf(v[e + 1]));
-      }
-    }
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    int const ke = mx > 0.f ? scale_exp(mx) : 0;
-    float const s = exp2i(ke), sl = exp2i(ke + 11);
-    uint64_t const s2 = pack2(s, s), sl2 = pack2(sl, sl);
-    for (int h0 = 0; h0 < H; h0 += 8) {
-      int const h = h0 + (lane >> 2);
-#pragma unroll
-      for (int i = 0; i < kG; ++i) {
-        float v[8];
-        fetch(h, i, v);
-        uint32_t hh[4], l[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) split_pair<kSplit>(v[2 * e], v[2 * e + 1], s2, sl2, hh[e], l[e]);
-        long long const at = ((long long)(ng * kG + i) * HW + place * H + h) * C + c;
-        if (real && h < H) {
-          hi[at] = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-          if (kSplit) hi[loOff + at] = make_uint4(l[0], l[1], l[2], l[3]);
-        }
-      }
-    }
-    if (real && lane < 4) exps[((long long)ng * W + place) * C + c] = (int8_t)ke;
+    for (int k = 0; k < 64; ++k) v[k] = ng * 64 + k < N ? __ldg(src + k * step) : 0.f;
   }
+  float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+  for (int k = 0; k < 64; k += 4) { m0 = max3(m0, fabsf(v[k]), fabsf(v[k + 1])); m1 = max3(m1, fabsf(v[k + 2]), fabsf(v[k + 3])); }
+  float const mx = fmaxf(m0, m1);
+  int const ke = mx > 0.f ? scale_exp(mx) : 0;
+  float const s = exp2i(ke), sl = exp2i(ke + 11);
+  uint64_t const s2 = pack2(s, s), sl2 = pack2(sl, sl);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split_pair<kSplit>(v[8 * i + 2 * e], v[8 * i + 2 * e + 1], s2, sl2, h[e], l[e]);
+    long long const at = ((long long)(ng * 8 + i) * HW + pix) * C + c;
+    hi[at] = make_uint4(h[0], h[1], h[2], h[3]);
+    if (kSplit) hi[loOff + at] = make_uint4(l[0], l[1], l[2], l[3]);
+  }
+  exps[((long long)ng * HW + pix) * C + c] = (int8_t)ke;
+}
+
+// The same for kMode 5: fp32 values as they are, four images of a chunk at x8, the other four loOff further on.  grid (as above, groups of eight images)
+__global__ void __launch_bounds__(256)
+gather_images_kernel(float4* __restrict__ x8, long long loOff, uint4* __restrict__ zero, float const* __restrict__ x, int HW, int C, int N, int cBlocks)
+{
+  vlb::pdl_wait();
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *zero = make_uint4(0, 0, 0, 0);
+  int const lane = (int)threadIdx.x & 31, place = (int)blockIdx.x / cBlocks, n0 = (int)blockIdx.y * 8;
+  int const c = ((int)blockIdx.x - place * cBlocks) * 32 + ((int)threadIdx.x >> 5) * 4 + (lane & 3);
+  int const pix = place * 8 + (lane >> 2);
+  if (c >= C || pix >= HW) return;
+  long long const step = (long long)C * HW;
+  float const* const src = x + n0 * step + (long long)c * HW + pix;
+  float v[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = n0 + k < N ? __ldg(src + k * step) : 0.f;
+  long long const at = ((long long)blockIdx.y * HW + pix) * C + c;
+  x8[at] = make_float4(v[0], v[1], v[2], v[3]);
+  x8[loOff + at] = make_float4(v[4], v[5], v[6], v[7]);
 }
 
 // dY of such a filter gradient as tile images, and the bias gradient from the same sweep.  A block takes 32 filters of a column tile and octets -- eight
@@ -1482,6 +1477,10 @@ template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 4, true>>() { ret
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 4, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 4, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 4, false>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 5, true>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 5, false>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 5, true>>() { return 96; }
+template <> constexpr int kRegsAtLaunch<conv_half_kernel<false, 5, false>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 2, false>>() { return 80; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 3, true>>() { return 96; }
 template <> constexpr int kRegsAtLaunch<conv_half_kernel<true, 3, false>>() { return 96; }
@@ -1644,7 +1643,7 @@ int launch_rows(vlb_ctx* ctx, Params& p, CUtensorMap const& map, char const* whe
   return vlb::check_launch(ctx, where);
 }
 
-// conv_half_kernel, kMode 4: p holds the tiling, the chunks, the tile images and the epilogue.
+// conv_half_kernel, kMode 4 (64 images of a pixel per k-block) or 5: p holds the tiling, the chunks, the tile images and the epilogue.
 int launch_images(vlb_ctx* ctx, Params& p, char const* where)
 {
   bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
@@ -1665,9 +1664,13 @@ int launch_images(vlb_ctx* ctx, Params& p, char const* where)
     e = allow_large_smem<decltype(kernel)::value>(ctx->device);
     if (e == cudaSuccess) vlb::launch(ctx->stream, decltype(kernel)::value, grid, kTsThreads, smemBytes, p, map);
   };
-#define VLB_TSI(split, nar) go(std::integral_constant<decltype(&conv_half_kernel<split, 4, nar>), &conv_half_kernel<split, 4, nar>>{})
-  if (split3) { if (p.BN <= 64) VLB_TSI(true, true); else VLB_TSI(true, false); }
-  else        { if (p.BN <= 64) VLB_TSI(false, true); else VLB_TSI(false, false); }
+#define VLB_TSI(split, mode, nar) go(std::integral_constant<decltype(&conv_half_kernel<split, mode, nar>), &conv_half_kernel<split, mode, nar>>{})
+#define VLB_TSIM(mode) do { \
+    if (split3) { if (p.BN <= 64) VLB_TSI(true, mode, true); else VLB_TSI(true, mode, false); } \
+    else        { if (p.BN <= 64) VLB_TSI(false, mode, true); else VLB_TSI(false, mode, false); } \
+  } while (0)
+  if (p.gShift == 3) VLB_TSIM(4); else VLB_TSIM(5);
+#undef VLB_TSIM
 #undef VLB_TSI
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
@@ -1686,10 +1689,12 @@ bool wgrad_rows_ok(ConvGeom const& g)
 }
 
 // Whether the images along the reduction (kbs k-blocks in `tiles` output tiles, 8 << gShift images in each) beat the other route, in microseconds as measured on 148 SMs:
-// a k-block of a tile takes 0.7 here, 1.05 in planes of rows, 1.9 (per 64 pixels) in tc_gemm_kernel; splitting the input takes 8 or, with the second reading of whole
-// columns, 12 bytes per element at 5 TB/s, the tile images 3 more than the row mode's; one launch more than there 3, two more than tc_gemm_kernel with its own producers 10.
-// 3x3, 512 -> 512, 14 x 14 x 64: 215 (planes of rows 331); 256 -> 256, 56 x 56 x 64: 920 (1003); 1x1, 512 -> 128, 28 x 28 x 64: 112 (60); 13 x 13, 256 -> 384, 128
-// images: 190 (tc_gemm_kernel 260); 7 x 7, 512 -> 512, 8 images: 34 (24).
+// a k-block of a tile takes 0.7 here (0.85 with fewer than 64 images in it, whose chunks are converted as they come), 1.05 in planes of rows, 1.9 (per 64 pixels) in
+// tc_gemm_kernel; the input's chunks take 8 bytes per element at 5 TB/s, the tile images 3 more than the row mode's; one launch more than there 3 (nothing with fewer than
+// 64 images: the row mode's first runs arrive that much later), two more than tc_gemm_kernel with its own producers 10.
+// 64 images: 3x3, 512 -> 512, 14 x 14: 190 (planes of rows 331); 256 -> 256, 56 x 56: 920 (1003); 1x1, 512 -> 128, 28 x 28: 103 (62); 13 x 13, 256 -> 384, 128
+// images: 161 (tc_gemm_kernel 260).  Fewer: 3x3, 256 -> 256, 14 x 14, 8 images 48 (planes of rows 62), 16 images 56 (66), 32 images 60 (73); 512 -> 512, 7 x 7, 8 images
+// 32 (tc_gemm_kernel 28), 32 images 56 (71); 1x1, 512 -> 128, 28 x 28, 32 images 78 (planes of rows 54).
 bool wgrad_images_pay(vlb_ctx* ctx, ConvGeom const& g, bool rows, long long kbs, int tiles, int gShift)
 {
   int const V = g.FH * g.FW * g.FC;
@@ -1697,7 +1702,8 @@ bool wgrad_images_pay(vlb_ctx* ctx, ConvGeom const& g, bool rows, long long kbs,
   long long const P = (long long)g.Ho * g.Wo;
   double const other = rows ? 1.05 * vlb::ceil_div(V, BM) * vlb::ceil_div(g.K, pick_bn(g.K)) * (double)((P + kTsK - 1) / kTsK) * g.N * perSm
                             : 1.9 * vlb::ceil_div(V, BM) * vlb::ceil_div(g.Kg, pick_bn(g.Kg)) * (double)g.G * (double)P * g.N / kTsK * perSm;
-  return 0.7 * tiles * (double)kbs * perSm + (x * (gShift == 3 ? 8 : 12) + y * (rows ? 3 : 0)) / 5e6 + (rows ? 3.0 : 10.0) < other;
+  double const perKb = gShift == 3 ? 0.7 : 0.85, launches = !rows ? 10.0 : gShift == 3 ? 3.0 : 0.0;
+  return perKb * tiles * (double)kbs * perSm + (x * 8 + y * (rows ? 3 : 0)) / 5e6 + launches < other;
 }
 
 // k-blocks of a reduction over `taps` filter taps of `channels` channels.
@@ -1834,8 +1840,9 @@ int conv_wgrad_images(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, flo
   int gShift = 0;
   long long least = -1;
   for (int s = 0; s <= 3; ++s) {
-    long long const images = (long long)ceil_div(g.N, 8 << s) * (8 << s), rows = (long long)ceil_div(g.Ho, 8 >> s) * (8 >> s);
-    if (least < 0 || images * rows <= least) { least = images * rows; gShift = s; }
+    // (14 : 17, a k-block of split chunks : one of chunks that are converted as they come; 3x3, 256 -> 256, 14 x 14 maps of 100 images: 122 us in blocks of 64 images, 145 of 8)
+    long long const images = (long long)ceil_div(g.N, 8 << s) * (8 << s), rows = (long long)ceil_div(g.Ho, 8 >> s) * (8 >> s), cost = images * rows * (s == 3 ? 14 : 17);
+    if (least < 0 || cost <= least) { least = cost; gShift = s; }
   }
   if (taps > 4096 || g.K > 4096 || (g.G > 1 && g.Kg < 16)) return -1;
   Params p = {};
@@ -1852,13 +1859,13 @@ int conv_wgrad_images(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, flo
   p.M = V; p.N = g.G * p.tilesN * p.BN; p.R = (int)((long long)g.Ho * g.Wo * g.N); p.a.rows = V; p.wg = 2;
   size_t const nF = (size_t)V * g.K;
   if ((long long)nF * p.splits >= (1LL << 31)) return -1;
-  // scratch: tile images, partial results, the input's chunks and exponents, the bias gradient's partial sums
+  // scratch: tile images, partial results, the input's chunks (64 images per k-block: split, with exponents), the bias gradient's partial sums
   int const imgGroups = p.nGroups << gShift, tiles = g.G * p.tilesN;
   long long const chunks = (long long)imgGroups * g.H * g.W * g.C;
   bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
   size_t const partBytes = p.splits > 1 ? ((sizeof(float) * nF * p.splits + 255) & ~(size_t)255) : 0;
-  size_t const chunkBytes = (size_t)chunks * (split3 ? 32 : 16);
-  size_t const expBytes = ((size_t)p.nGroups * g.W * (gShift == 3 ? g.H : 1) * g.C + 511) & ~(size_t)255;
+  size_t const chunkBytes = (size_t)chunks * (split3 || gShift < 3 ? 32 : 16);
+  size_t const expBytes = gShift == 3 ? ((size_t)p.nGroups * g.W * g.H * g.C + 511) & ~(size_t)255 : 0;
   // (one pixel per k-block: the columns of a plane are one long one, whose octets lie on 32-byte boundaries where P does)
   int const oH = gShift == 3 ? g.Ho * g.Wo : g.Ho, oW = gShift == 3 ? 1 : g.Wo, oBlocks = gShift == 3 ? oH : p.rowBlocks;
   int const octets = ceil_div(p.kbTot, oBlocks) * ceil_div(oH, 8);
@@ -1876,12 +1883,12 @@ int conv_wgrad_images(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, flo
   float* const dbPart = db ? (float*)((char*)exps + expBytes) : nullptr;
   unsigned* const tickets = (unsigned*)((char*)ctx->deviceStatus + 256);
   p.aHi = hi; p.aLo = chunks; p.aExp = exps; p.zero = zero;
-  int const cBlocks = ceil_div(g.C, 32);
-  dim3 const gridX((unsigned)((gShift == 3 ? ceil_div((long long)g.H * g.W, 8) : g.W) * cBlocks), (unsigned)p.nGroups, 1), gridY((unsigned)gx, (unsigned)fBlocks, 1);
-#define VLB_IM(split, G8) do { \
-    vlb::launch(ctx->stream, split_images_kernel<split, G8>, gridX, 256, 0, hi, chunks, exps, zero, X, g.H, g.W, g.C, g.N, cBlocks); \
-    vlb::launch(ctx->stream, prep_image_tiles_kernel<split, G8>, gridY, 256, 0, out, dY, oH, oW, g.N, g.K, g.Kg, p.tilesN, p.BN, p.nGroups, oBlocks, p.kbTot, octets, db, dbPart, tickets); \
-  } while (0)
+  int const cBlocks = ceil_div(g.C, 32), HW = g.H * g.W;
+  dim3 const gridX((unsigned)(ceil_div(HW, 8) * cBlocks), (unsigned)(gShift == 3 ? p.nGroups : imgGroups), 1), gridY((unsigned)gx, (unsigned)fBlocks, 1);
+  if (gShift < 3)  vlb::launch(ctx->stream, gather_images_kernel, gridX, 256, 0, (float4*)hi, chunks, zero, X, HW, g.C, g.N, cBlocks);
+  else if (split3) vlb::launch(ctx->stream, split_images_kernel<true>, gridX, 256, 0, hi, chunks, exps, zero, X, HW, g.C, g.N, cBlocks);
+  else             vlb::launch(ctx->stream, split_images_kernel<false>, gridX, 256, 0, hi, chunks, exps, zero, X, HW, g.C, g.N, cBlocks);
+#define VLB_IM(split, G8) vlb::launch(ctx->stream, prep_image_tiles_kernel<split, G8>, gridY, 256, 0, out, dY, oH, oW, g.N, g.K, g.Kg, p.tilesN, p.BN, p.nGroups, oBlocks, p.kbTot, octets, db, dbPart, tickets)
 #define VLB_IMS(G8) do { if (split3) VLB_IM(true, G8); else VLB_IM(false, G8); } while (0)
   if (gShift == 3) VLB_IMS(8); else if (gShift == 2) VLB_IMS(4); else if (gShift == 1) VLB_IMS(2); else VLB_IMS(1);
 #undef VLB_IMS

@@ -85,9 +85,10 @@ struct Params {
   // (oy + oys * i, ox + oxs * j) of a plane of outH x outW.  shufY > 0: column n of a group is channel n / (shufY * shufX) at the
   // output pixel moved by (n % shufY, n / shufY % shufX), outC channels per group.  ctaBeg, ctas: the CTAs that walk this problem.
   int unit, upk, tilesPerGroup, cols;
-  // conv_half_kernel, kMode 4 (wg == 2): the filter gradient with the images along the reduction.  A k-block is 1 << gShift groups of eight images at 8 >> gShift
-  // consecutive output rows of one column: k-block ((group of groups * Wo + column) * rowBlocks + row block).  aHi[((n/8 * W + w) * H + h) * channels
-  // + channel] are eight images of a pixel; aExp[(group of groups * W * (per pixel ? H : 1) + pixel or column) * channels + channel].
+  // conv_half_kernel, kMode 4 and 5 (wg == 2): the filter gradient with the images along the reduction.  A k-block is 1 << gShift groups of eight images at
+  // 8 >> gShift consecutive output rows of one column: k-block ((group of groups * Wo + column) * rowBlocks + row block).  aHi[((n/8 * W + w) * H + h) *
+  // channels + channel] are eight images of a pixel (gShift < 3: four, and the other four aLo further on, fp32); aExp[(group of 64 images * W*H + pixel) *
+  // channels + channel].
   int gShift, rowBlocks, nGroups, channels;
   int groups;             // tc_gemm_kernel, filter gradient: filter groups (0 counts as one), M rows and N columns each
   long long aGroup;

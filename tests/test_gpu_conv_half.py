@@ -131,6 +131,36 @@ def test_values_that_are_not_finite_stay_where_they_are(gpu, case):
         ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 2.0 ** 60])
+@pytest.mark.parametrize("images", [8, 16, 32, 64])
+@pytest.mark.parametrize("stride", [1, 2])
+def test_a_filter_tap_knows_nothing_of_rows_that_it_does_not_read(gpu, stride, images, value):
+    """Stride 1: the last row of a padded plane, which the first filter row never reads.  Stride 2: an odd row, which the middle one never reads.  8, 16 and
+    32 images: k-blocks of 8, 4 and 2 rows.  What a tap's sums are made of has not changed, so neither may one bit of them."""
+    import torch
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(600 + images)
+    x, f = mat.empty((14, 12, 32, images)).normal_(generator=g), mat.empty((3, 3, 32, 48)).normal_(generator=g)
+    kw = dict(stride=stride, pad=1)
+    dy = mat.empty(reference(x, f, None, stride, 1, 1)).normal_(generator=g)
+    row, tap = (13, 0) if stride == 1 else (5, 1)
+    x2 = x.clone()
+    x2[row, 4, 7, 2] = value
+    lib = ctx.lib
+    try:
+        for switch in (0, 16):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            _, df, _ = nn.vl_nnconv(x, f, None, dy, no_der_data=True, ctx=ctx, **kw)
+            _, df2, _ = nn.vl_nnconv(mat.as_mat(x2), f, None, dy, no_der_data=True, ctx=ctx, **kw)
+            assert torch.equal(df2[tap], df[tap]), switch
+            read = [t for t in range(3) if t != tap and (stride == 1 or t != 1)]
+            assert not torch.equal(df2[read, :, 7], df[read, :, 7]), switch
+            other = [c for c in range(32) if c != 7]
+            assert torch.equal(df2[:, :, other], df[:, :, other]), switch
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+
+
 def test_an_odd_number_of_run_buffers_keeps_the_groups_apart(gpu):
     """128-column tiles of the row mode have three run buffers for two groups of producers: a buffer's previous run belongs to the other group.  A group that
     did not wait for it to be let go of took a run of three k-blocks before for its own, once in some thousand launches."""
