@@ -34,9 +34,10 @@ enum {
 
 /* Arithmetic of the convolution / fully-connected contractions. */
 enum {
-  VLB_PRECISION_3XTF32 = 0, /* tcgen05 kind::tf32, hi/lo split, 3 MMAs per product: fp32-faithful (default) */
-  VLB_PRECISION_TF32 = 1,   /* tcgen05 kind::tf32, single pass: fast path, the operands of every contraction on the tensor
-                               cores rounded to TF32, about 5e-4 relative error -- strided, dilated and grouped layers
+  VLB_PRECISION_3XTF32 = 0, /* operands as two parts of 11 bits, 3 MMAs per product: fp32-faithful (default).  tcgen05 kind::tf32
+                               forward, kind::f16 on scaled halves backward (see below) */
+  VLB_PRECISION_TF32 = 1,   /* the first part alone, single pass: fast path, the operands of every contraction on the tensor
+                               cores rounded to TF32's 11 bits, about 5e-4 relative error -- strided, dilated and grouped layers
                                and all their gradients included.  Exact products as in the other modes: the direct kernels of a
                                network's image end (at most 64 inputs per output pixel forward, 27 for the filter gradient,
                                4 input channels for the data gradient), fully connected forward passes of up to 8 images, and
@@ -45,6 +46,14 @@ enum {
                                groups of fewer than four channels, strided filters of more than 128 taps, more than 16
                                residue classes of a strided data gradient and reductions of more than 65535 x 32 */
 };
+
+/* Range of the scaled halves.  The gradients of convolutions and of large fully connected layers are sums over blocks of 64 products.  In each block the
+ * 64 values that enter one sum from either side share a power of two.  From the gathered side (the data, or the output derivative of a data gradient; the
+ * weights of a fully connected one) those down to 2^-28 of the largest of the 64 keep 22 bits, smaller ones are off by at most 2^-51 of the largest; from
+ * the other side (output derivative, filter bank) 2^-12 and 2^-35, or better.  VLB_PRECISION_TF32 keeps 11 bits down to 2^-29, 2^-40 at worst (2^-13, 2^-24).
+ * Such errors show only where the largest values meet zeros or cancel.  Nothing is shared beyond the 64: a filter, channel, image or pixel that is small
+ * beside others, by up to 2^100, is as exact as among its like.  Single values below about 2^-102 in magnitude lose digits as they near the subnormal
+ * range.  An infinity or a not-a-number reaches the sums that it is part of and no others. */
 
 /* ---- context: replaces vl::Context (bits/data.hpp:150-179) and the stream part of
  *      vl::CudaHelper (bits/datacu.hpp:60-158; setStream bits/datacu.cu:70-93) ---- */

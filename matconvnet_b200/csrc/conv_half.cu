@@ -9,15 +9,16 @@ namespace {
 //
 // Arithmetic: scaled half-precision pairs.  The tensor core multiplies half-precision operands twice as fast as TF32 ones, and the two
 // formats have the same 11 significant bits; what half precision lacks is range, and that is given back by scaling.  A k-block is 64
-// reduction indices.  Each row of A takes the power of two that brings the largest magnitude of its values in the k-block (or in a larger set that holds
-// them) into [2^14, 2^15), each tile of B one for 32 or 64 columns; then x * s = hi + lo / 2048 with hi = half(x*s) and lo = half((x*s - hi) * 2048): 22
-// significant bits for every value down to 2^-28 of the largest one it stands beside, below that an absolute error of 2^-51 of that one.  (Two TF32 values
-// hold 22 bits as well.)  Per k-block the accumulator T takes the small terms lo*hi + hi*lo first, which carry the 2048, then
+// reduction indices.  Each row of A takes the power of two that brings the largest magnitude of its values in the k-block into [2^14, 2^15), each tile of B one for
+// 32 or 64 columns, and a column whose own largest magnitude is more than 2^16 below theirs one of its own; then x * s = hi + lo / 2048 with hi = half(x*s)
+// and lo = half((x*s - hi) * 2048): 22 significant bits for every value of a row of A down to 2^-28 of the row's largest in the k-block, below that an absolute
+// error of 2^-51 of that one; of a column of B down to 2^-12, 2^-35 at worst.  (Two TF32 values hold 22 bits as well, whatever stands beside them.)  Per k-block the accumulator T takes the small terms lo*hi + hi*lo first, which carry the 2048, then
 // hi*hi with the accumulator scaled by 2^-11 (the MMA's scale-input-d); lo*lo (2^-22) is dropped.  Products of two halves are exact and the sums
 // are fp32, as with TF32.  The drain warps add T * 2^-(row's + tile's exponent) to the fp32 running sum: one k-block per accumulation chain, so
 // that the tensor core's truncating additions have no time to pile up (12 MMAs 16 deep; conv_ts_kernel has chains of up to 48 MMAs 8 deep).
 // 3x3, 512 -> 512 channels, 28 x 28 x 64, against float64: 2.0e-7 (conv_ts_kernel 9e-7); data gradient 956 us there, 565 here.
-// VLB_PRECISION_TF32 issues hi*hi alone: operands rounded to 11 bits, as TF32 does.
+// VLB_PRECISION_TF32 issues hi*hi alone: operands rounded to 11 bits as TF32 does, down to 2^-29 of the row's largest magnitude in the k-block (2^-13 of the
+// column's), where the subnormal halves begin; below that an absolute error of 2^-40 (2^-24) of it.
 // Why the forward passes stay where they are: their sums decide what ReLU and pooling let through.  Other sums, however near, decide some ties of
 // existing networks the other way; a backward pass decides nothing.
 //
@@ -80,6 +81,14 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, uint4 const (&r)[8])
                  "r"(r[6].x), "r"(r[6].y), "r"(r[6].z), "r"(r[6].w), "r"(r[7].x), "r"(r[7].y), "r"(r[7].z), "r"(r[7].w) : "memory");
 }
 
+// A column of B whose largest magnitude lies more than 2^kOwnScale below the tile's takes a power of two of its own, 2^c beyond the tile's.  The closer the line
+// lies to the tile's, the more k-blocks of ordinary values pay for it in the drain warps (rescale_columns; dense values never, a column with one value left by
+// ReLU and pooling once in 25000 k-blocks); the further off, the fewer digits a column just above it keeps: at 2^16 its values have 22 bits down to 2^-12
+// of its largest, 11 (VLB_PRECISION_TF32) down to 2^-13.
+constexpr int kOwnScale = 16;
+constexpr int kMaxOwnScale = 100;       // (further down 22 bits until 2^-12 of that: 2^-128 of the tile's largest magnitude)
+constexpr int kOwnFlag = 1 << 16;       // added to an exponent word of the tile images: some column has one of its own
+
 // Two fp32 values side by side in one 64-bit register pair, and the packed operations on them (one instruction for both).
 __device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ void unpack2(uint64_t r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
@@ -106,6 +115,22 @@ __device__ __forceinline__ void split_pair(float a, float b, uint64_t s2, uint64
     unpack2(fma2(pack2(h0, h1), pack2(-2048.f, -2048.f), mul2(x, sl2)), l0, l1);
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(l1), "f"(l0));
   }
+}
+
+// The columns beg .. end - 1 of an accumulator (multiples of eight) times 2^-own[column], in tensor memory, so that the drain's own loop stays as it is.
+__device__ __forceinline__ void rescale_columns(uint32_t acc, int8_t const* own, int beg, int end)
+{
+#pragma unroll 1
+  for (int c0 = beg; c0 < end; c0 += 8) {
+    uint32_t r[8];
+    tmem_ld8_issue(acc + (uint32_t)c0, r);
+    uint2 const e = __ldg(reinterpret_cast<uint2 const*>(own + c0));
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * exp2i(-(int)(((j < 4 ? e.x : e.y) >> (8 * (j & 3))) & 255u)));
+    tmem_st8(acc + (uint32_t)c0, r);
+  }
+  tmem_st_wait();
 }
 
 // kTma: the producers take the input windows from shared memory, where the loader thread has them delivered by tensor-map copies
@@ -241,7 +266,8 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
         // exponents of the tile images: one per 64 columns (this thread's, of a wide tile), per 32 where the images are along the reduction
         constexpr int kPer = kImages ? 32 : 64, kExps = kCols > kPer ? 2 : 1;
         int const perImage = max(BN / kPer, 1);
-        int const* const bExp = p.bExp + ((size_t)nt * p.kbTot + (size_t)p.dTilesM(tm) * numIter) * perImage + col0 / kPer;
+        size_t const image0 = (size_t)nt * p.kbTot + (size_t)p.dTilesM(tm) * numIter;
+        int const* const bExp = p.bExp + image0 * perImage + col0 / kPer;
         int eB[kExps];
 #pragma unroll
         for (int j = 0; j < kExps; ++j) eB[j] = __ldg(bExp + j);
@@ -289,8 +315,16 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
             odd = odd || ex[j] < -126 || ex[j] > 127;
             if (it + 1 < numIter) eB[j] = __ldg(bExp + (it + 1) * perImage + j);
           }
-          // a power of two outside the normal range (products of values around 1e-20 or 1e+20) is applied in two halves
-          bool const far = __any_sync(0xffffffffu, odd);
+          // a power of two outside the normal range (products of values around 1e-20 or 1e+20) is applied in two halves; kOwnFlag shows up here too, so that
+          // the loop has one test for both
+          bool far = __any_sync(0xffffffffu, odd);
+          if (__builtin_expect(far, 0)) {
+            int beg = kCols, end = 0;
+#pragma unroll
+            for (int j = 0; j < kExps; ++j)
+              if (ex[j] < -kOwnFlag / 2) { ex[j] += kOwnFlag; beg = min(beg, j * kPer); end = min((j + 1) * kPer, kCols); }
+            rescale_columns(lanes + (uint32_t)(t * 2 * kCols + col0), p.bOwn + (image0 + it) * BN + col0, beg, end);
+          }
 #pragma unroll
           for (int c0 = 0; c0 < kCols; c0 += kStep) {
             uint32_t t0[kStep < 16 ? 8 : kStep];
@@ -856,9 +890,11 @@ __global__ void __launch_bounds__(kTsThreads, 1) conv_half_gen_kernel(const __gr
 // shared-memory tile images -- for n-tile t and k-block kb: [hi tile BN x 64 halves][lo tile BN x 64], K-major with the 128-byte swizzle,
 // 16-byte chunk c of row r at chunk c ^ (r & 7) -- so that a stage of B is one bulk copy.  64 rows of an image share a power of two (32 of those of
 // prep_image_tiles_kernel), so that the blocks that write them need not agree on one; the exponents go to exps[(t * numKb + kb) * max(BN / 64, 1) + row / 64].
+// With kOwnFlag added to that word, own[(t * numKb + kb) * BN + row] is what each of those rows was scaled beyond it (the others' are not written).
 struct TileOut {
   uint8_t* img;
   int* exps;
+  int8_t* own;
 };
 
 // Largest finite magnitude so far (as bits): infinities and not-a-numbers spoil their own column only, not the scale of the others.
@@ -869,17 +905,36 @@ __device__ __forceinline__ void max_finite(uint32_t& m, float v)
 }
 __device__ __forceinline__ int tile_exp(uint32_t m) { return m ? scale_exp(__uint_as_float(m)) : 0; }
 
-// Maximum over a block of kWarps warps; red: kWarps words of shared memory, not touched again before the next block barrier but one.
-template <int kWarps>
-__device__ __forceinline__ uint32_t block_max(uint32_t m, uint32_t* red)
+// The exponent of a set of columns and whether some of them need their own, from the largest magnitudes of the columns: hi is the largest of them, lo
+// the smallest but for zeros, less one (all ones: none).  Both as bits.
+struct TileScale { int k; bool own; };
+__device__ __forceinline__ TileScale tile_scale(uint32_t hi, uint32_t lo)
 {
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  TileScale t;
+  t.k = tile_exp(hi);
+  t.own = lo != 0xffffffffu && scale_exp(__uint_as_float(lo + 1u)) - t.k > kOwnScale;
+  return t;
+}
+__device__ __forceinline__ int tile_word(TileScale t) { return t.k + (t.own ? kOwnFlag : 0); }
+// What a column whose largest magnitude is m is scaled beyond the tile's exponent k.
+__device__ __forceinline__ int own_exp(uint32_t m, int k)
+{
+  int const c = m ? scale_exp(__uint_as_float(m)) - k : 0;
+  return c > kOwnScale ? min(c, kMaxOwnScale) : 0;
+}
+
+// tile_scale over a block of kWarps warps whose threads hold hi and lo; red: 2 * kWarps words of shared memory, not touched again before the next block
+// barrier but one.
+template <int kWarps>
+__device__ __forceinline__ TileScale block_scale(uint32_t hi, uint32_t lo, uint32_t* red)
+{
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = hi; red[kWarps + (threadIdx.x >> 5)] = lo; }
   __syncthreads();
-  uint32_t r = red[0];
 #pragma unroll
-  for (int w = 1; w < kWarps; ++w) r = max(r, red[w]);
-  return r;
+  for (int w = 0; w < kWarps; ++w) { hi = max(hi, red[w]); lo = min(lo, red[kWarps + w]); }
+  return tile_scale(hi, lo);
 }
 
 // Eight consecutive reduction indices of one row: 16 bytes of the hi and of the lo tile.
@@ -1014,7 +1069,7 @@ prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int W
 {
   vlb::pdl_wait();
   constexpr int kRows = 8 / kG;                         // rows of a k-block
-  __shared__ uint32_t red[2][8][8];                     // [turn][warp][k-block of the octet]
+  __shared__ uint2 red[2][8][8];                        // [turn][warp][row of the octet]: largest magnitude, smallest of a filter less one
   __shared__ double sums[256][4];
   __shared__ bool last;
   int const tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31, px = lane & 7, f = warp * 4 + (lane >> 3);
@@ -1059,14 +1114,19 @@ prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int W
       for (int n = 0; n < 8 * kG; ++n) max_finite(m, v[n]);
     }
 #pragma unroll
-    for (int q = 1; q < 32; q <<= 1) if (q < kRows || q >= 8) m = max(m, __shfl_xor_sync(0xffffffffu, m, q));
-    uint32_t (&r)[8][8] = red[turn];                    // (written again two octets on, with a barrier in between)
-    if (lane < 8) r[warp][px] = m;
+    for (int q = 1; q < kRows; q <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, q));
+    uint32_t const fMax = m;                           // of this filter in the k-block
+    uint32_t lo = m - 1u;
+#pragma unroll
+    for (int q = 8; q < 32; q <<= 1) { m = max(m, __shfl_xor_sync(0xffffffffu, m, q)); lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, q)); }
+    uint2 (&r)[8][8] = red[turn];                       // (written again two octets on, with a barrier in between)
+    if (lane < 8) r[warp][px] = make_uint2(m, lo);
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 8; ++q) m = max(m, r[q][px]);
-    int const k = tile_exp(m);
-    float const s = exp2i(k), sl = exp2i(k + 11);
+    for (int q = 0; q < 8; ++q) { uint2 const u = r[q][px]; m = max(m, u.x); lo = min(lo, u.y); }
+    TileScale const ts = tile_scale(m, lo);
+    int const own = ts.own ? own_exp(fMax, ts.k) : 0;
+    float const s = exp2i(ts.k + own), sl = exp2i(ts.k + own + 11);
     uint64_t const s2 = pack2(s, s), sl2 = pack2(sl, sl);
     size_t const imgBytes = (kSplit ? 2 : 1) * (size_t)BN * kTsRowBytes;
     uint8_t* const rowAt = out.img + (size_t)tile * kbTot * imgBytes + (size_t)row * kTsRowBytes;
@@ -1107,8 +1167,10 @@ prep_image_tiles_kernel(TileOut out, float const* __restrict__ dy, int Ho, int W
         if (on1) put(at1, ((px | 1) % kRows) * kG + mine, oddPx ? h1 : hr, oddPx ? l1 : lr);
       }
     }
-    if (kbOn) {
-      if (f == 0 && px % kRows == 0) out.exps[((size_t)tile * kbTot + kb) * perTile + fb] = k;
+    if (kbOn && px % kRows == 0) {
+      size_t const image = (size_t)tile * kbTot + kb;
+      if (f == 0) out.exps[image * perTile + fb] = tile_word(ts);
+      if (ts.own) out.own[image * BN + row] = (int8_t)own;
     }
   }
   if (db == nullptr) return;
@@ -1148,31 +1210,42 @@ template <bool kSplit, bool kRows>
 __global__ void __launch_bounds__(256) prep_dense_tiles_kernel(TileOut out, float const* __restrict__ f, int N, int R, int BN, int numKb)
 {
   vlb::pdl_wait();
-  __shared__ uint32_t red[8];
-  int const tile = (int)blockIdx.x / numKb, kb = (int)blockIdx.x - tile * numKb, items = BN * 8;
+  __shared__ uint32_t colMax[BM];                       // largest magnitude of each row of the image
+  int const tid = (int)threadIdx.x, tile = (int)blockIdx.x / numKb, kb = (int)blockIdx.x - tile * numKb, items = BN * 8;
+  if (tid < BM) colMax[tid] = 0u;
   float v[4][8];
-  uint32_t m = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    int const it = (int)threadIdx.x + 256 * i;
+    int const it = tid + 256 * i;
     int const row = kRows ? it >> 3 : it % BN, chunk = kRows ? it & 7 : it / BN, n = tile * BN + row, r0 = kb * kTsK + chunk * 8;
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[i][e] = it < items && n < N && r0 + e < R ? __ldg(f + (kRows ? (size_t)n * R + r0 + e : (size_t)(r0 + e) * N + n)) : 0.f;
   }
+  __syncthreads();
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
+    int const it = tid + 256 * i;
+    uint32_t m = 0;
 #pragma unroll
     for (int e = 0; e < 8; ++e) max_finite(m, v[i][e]);
+    if (it < items && m) atomicMax(&colMax[kRows ? it >> 3 : it % BN], m);
   }
-  int const k = tile_exp(block_max<8>(m, red));
+  __syncthreads();
+  uint32_t hi = 0, lo = 0xffffffffu;
+  for (int c = tid & 31; c < BN; c += 32) { uint32_t const m = colMax[c]; hi = max(hi, m); lo = min(lo, m - 1u); }
+  TileScale const ts = tile_scale(__reduce_max_sync(0xffffffffu, hi), __reduce_min_sync(0xffffffffu, lo));
   uint8_t* const img = out.img + (size_t)blockIdx.x * ((kSplit ? 2 : 1) * (size_t)BN * kTsRowBytes);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    int const it = (int)threadIdx.x + 256 * i;
-    if (it < items) store_chunk8<kSplit>(img, BN, kRows ? it >> 3 : it % BN, kRows ? it & 7 : it / BN, v[i], k);
+    int const it = tid + 256 * i;
+    if (it < items) {
+      int const row = kRows ? it >> 3 : it % BN, chunk = kRows ? it & 7 : it / BN, own = ts.own ? own_exp(colMax[row], ts.k) : 0;
+      store_chunk8<kSplit>(img, BN, row, chunk, v[i], ts.k + own);
+      if (ts.own && chunk == 0) out.own[(size_t)blockIdx.x * BN + row] = (int8_t)own;
+    }
   }
   int const perImage = max(BN / 64, 1);
-  if ((int)threadIdx.x < perImage) out.exps[(size_t)blockIdx.x * perImage + threadIdx.x] = k;
+  if (tid < perImage) out.exps[(size_t)blockIdx.x * perImage + tid] = tile_word(ts);
 }
 
 // Filter tile images for conv_half_kernel and conv_half_gen_kernel, for filter groups, tap subsets
@@ -1205,7 +1278,7 @@ template <bool kSplit, int kMax>
 __global__ void __launch_bounds__(512) prep_filters_kernel(const __grid_constant__ PrepBatchOf<kMax> b)
 {
   vlb::pdl_wait();
-  __shared__ uint32_t red[16];
+  __shared__ uint32_t red[32];
   PrepFilters const& p = b.p[blockIdx.y];
   int const per = max(p.BN / 64, 1), img = (int)blockIdx.x / per, tile = img / p.numKb, kb = img - tile * p.numKb;
   if (tile * p.BN >= p.rows) return;
@@ -1230,9 +1303,15 @@ __global__ void __launch_bounds__(512) prep_filters_kernel(const __grid_constant
   uint32_t m = 0;
 #pragma unroll
   for (int e = 0; e < 8; ++e) max_finite(m, v[e]);
-  int const k = tile_exp(block_max<16>(m, red));
-  if (row < p.BN) store_chunk8<kSplit>(p.out.img + (size_t)img * ((kSplit ? 2 : 1) * (size_t)p.BN * kTsRowBytes), p.BN, row, chunk, v, k);
-  if (threadIdx.x == 0) p.out.exps[blockIdx.x] = k;
+#pragma unroll
+  for (int q = 1; q < 8; q <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, q));      // (the eight threads of a row are neighbours)
+  TileScale const ts = block_scale<16>(m, m - 1u, red);
+  int const own = ts.own ? own_exp(m, ts.k) : 0;
+  if (row < p.BN) {
+    store_chunk8<kSplit>(p.out.img + (size_t)img * ((kSplit ? 2 : 1) * (size_t)p.BN * kTsRowBytes), p.BN, row, chunk, v, ts.k + own);
+    if (ts.own && chunk == 0) p.out.own[(size_t)img * p.BN + row] = (int8_t)own;
+  }
+  if (threadIdx.x == 0) p.out.exps[blockIdx.x] = tile_word(ts);
 }
 
 // Launches the tile-image kernel for n problems whose output pointers are set.  The problems share the tile width.
@@ -1268,7 +1347,7 @@ prep_pixel_tiles_kernel(TileOut out, float const* __restrict__ dy, int N, int im
 {
   vlb::pdl_wait();
   constexpr int BN = 16 * kPasses;
-  __shared__ uint32_t red[2][8];
+  __shared__ uint32_t red[2][16];
   __shared__ double sums[256][4];
   __shared__ bool last;
   int const tid = (int)threadIdx.x, tile = (int)blockIdx.y, row0 = tid >> 4, c4 = tid & 15;
@@ -1293,31 +1372,52 @@ prep_pixel_tiles_kernel(TileOut out, float const* __restrict__ dy, int N, int im
 #pragma unroll
     for (int i = 0; i < kPasses; ++i) v[i] = w[i];
     if (kb + 1 < kbEnd) fetch(w);
-    uint32_t m = 0;
+    uint32_t hi = 0, lo = 0xffffffffu;
+    auto largest = [&](float4 const& a) { uint32_t m = 0; max_finite(m, a.x); max_finite(m, a.y); max_finite(m, a.z); max_finite(m, a.w); return m; };
 #pragma unroll
     for (int i = 0; i < kPasses; ++i) {
-      max_finite(m, v[i].x); max_finite(m, v[i].y); max_finite(m, v[i].z); max_finite(m, v[i].w);
+      uint32_t const m = largest(v[i]);
+      hi = max(hi, m); lo = min(lo, m - 1u);
       inner[i] += (v[i].x + v[i].y) + (v[i].z + v[i].w);
     }
     if (((kb - kbBeg) & 7) == 7) {      // (sums of eight, then of those: a long range keeps its digits)
 #pragma unroll
       for (int i = 0; i < kPasses; ++i) { outer[i] += inner[i]; inner[i] = 0.f; }
     }
-    int const k = tile_exp(block_max<8>(m, red[kb & 1]));
-    float const s = exp2i(k), sl = exp2i(k + 11);
-    uint64_t const s2 = pack2(s, s), sl2 = pack2(sl, sl);
+    // (four values of a row are the least: where they call for powers of their own, the rows' largest magnitudes decide)
+    TileScale ts = block_scale<8>(hi, lo, red[kb & 1]);
+    unsigned long long own = 0;                         // a byte for each pass
+    if (ts.own) {
+#pragma unroll
+      for (int i = 0; i < kPasses; ++i) {
+        uint32_t m = largest(v[i]);
+        for (int o = 8; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        own |= (unsigned long long)own_exp(m, ts.k) << (8 * i);
+      }
+      ts.own = __syncthreads_or(own != 0) != 0;
+      if (ts.own && c4 == 0) {
+#pragma unroll
+        for (int i = 0; i < kPasses; ++i) out.own[((size_t)tile * numKb + kb) * BN + row0 + 16 * i] = (int8_t)(own >> (8 * i));
+      }
+    }
+    float const s = exp2i(ts.k), sl = exp2i(ts.k + 11);
+    uint64_t s2 = pack2(s, s), sl2 = pack2(sl, sl);
     uint8_t* const at = out.img + ((size_t)tile * numKb + kb) * ((kSplit ? 2 : 1) * (size_t)BN * kTsRowBytes) + (size_t)row0 * kTsRowBytes +
                         (((c4 >> 1) ^ (row0 & 7)) << 4) + (c4 & 1) * 8;      // (rows 16 apart share the swizzle)
 #pragma unroll
     for (int i = 0; i < kPasses; ++i) {
       uint2 h, l;
+      if (ts.own) {
+        int const k = ts.k + (int)((own >> (8 * i)) & 255u);
+        s2 = pack2(exp2i(k), exp2i(k)); sl2 = pack2(exp2i(k + 11), exp2i(k + 11));
+      }
       split_pair<kSplit>(v[i].x, v[i].y, s2, sl2, h.x, l.x);
       split_pair<kSplit>(v[i].z, v[i].w, s2, sl2, h.y, l.y);
       *reinterpret_cast<uint2*>(at + (size_t)(16 * i) * kTsRowBytes) = h;
       if (kSplit) *reinterpret_cast<uint2*>(at + (size_t)(BN + 16 * i) * kTsRowBytes) = l;
     }
     constexpr int kPerImage = BN >= 64 ? BN / 64 : 1;
-    if (tid < kPerImage) out.exps[((size_t)tile * numKb + kb) * kPerImage + tid] = k;
+    if (tid < kPerImage) out.exps[((size_t)tile * numKb + kb) * kPerImage + tid] = tile_word(ts);
   }
   if (db == nullptr) return;
   int const rows = (int)gridDim.y * BN;
@@ -1355,12 +1455,16 @@ prep_pixel_tiles_kernel(TileOut out, float const* __restrict__ dy, int N, int im
   if (tid == 0) tickets[tile] = 0;      // ready for the next call
 }
 
-// The tile images of conv_half_kernel in the context's scratch: images, then exponents, then the caller's bytes.
+// The tile images of conv_half_kernel in the context's scratch: images, exponents, the columns' own ones, then the caller's bytes.
+size_t ts_images_bytes(vlb_ctx* ctx, size_t images, int BN)      // (a multiple of 2048)
+{ return images * (ctx->precision == VLB_PRECISION_3XTF32 ? 2 : 1) * (size_t)BN * kTsRowBytes; }
+
+size_t ts_exps_bytes(size_t images, int BN) { return (images * std::max(BN / 32, 1) * sizeof(int) + 255) & ~(size_t)255; }
+
 size_t ts_tiles_bytes(vlb_ctx* ctx, int rows, int BN, int numKb)
 {
   size_t const images = (size_t)vlb::ceil_div(rows, BN) * (size_t)numKb;
-  size_t const bytes = images * (ctx->precision == VLB_PRECISION_3XTF32 ? 2 : 1) * (size_t)BN * kTsRowBytes;      // (a multiple of 2048)
-  return bytes + ((images * std::max(BN / 32, 1) * sizeof(int) + 255) & ~(size_t)255);
+  return ts_images_bytes(ctx, images, BN) + ts_exps_bytes(images, BN) + ((images * BN + 255) & ~(size_t)255);
 }
 
 TileOut ts_tiles_at(vlb_ctx* ctx, void* at, int rows, int BN, int numKb)
@@ -1368,7 +1472,8 @@ TileOut ts_tiles_at(vlb_ctx* ctx, void* at, int rows, int BN, int numKb)
   size_t const images = (size_t)vlb::ceil_div(rows, BN) * (size_t)numKb;
   TileOut out;
   out.img = (uint8_t*)at;
-  out.exps = (int*)(out.img + images * (ctx->precision == VLB_PRECISION_3XTF32 ? 2 : 1) * (size_t)BN * kTsRowBytes);
+  out.exps = (int*)(out.img + ts_images_bytes(ctx, images, BN));
+  out.own = (int8_t*)out.exps + ts_exps_bytes(images, BN);
   return out;
 }
 
@@ -1402,7 +1507,7 @@ bool ts_tiles(vlb_ctx* ctx, Params& p, size_t extraBytes, TileOut* out, float** 
   char* const ws = (char*)vlb::workspace(ctx, bytes + extraBytes);
   if (!ws) return false;
   *out = ts_tiles_at(ctx, ws, p.N, p.BN, p.numKb);
-  p.bTiles = (float const*)out->img; p.bExp = out->exps;
+  p.bTiles = (float const*)out->img; p.bExp = out->exps; p.bOwn = out->own;
   if (extra) *extra = (float*)(ws + bytes);
   return true;
 }
@@ -1801,7 +1906,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     Params& p = b.p[i];
     p.ctaBeg = beg; beg += p.ctas;
     prep.p[i].out = ts_tiles_at(ctx, ws + offset[i], p.tilesN * BN, BN, p.numKb);
-    p.bTiles = (float const*)prep.p[i].out.img; p.bExp = prep.p[i].out.exps;
+    p.bTiles = (float const*)prep.p[i].out.img; p.bExp = prep.p[i].out.exps; p.bOwn = prep.p[i].out.own;
     if (splits > 1) p.e.out = part;
     p.c64 = b.p[0].c64; p.aHi = b.p[0].aHi; p.aLo = b.p[0].aLo; p.aExp = b.p[0].aExp; p.zero = b.p[0].zero;
     p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;

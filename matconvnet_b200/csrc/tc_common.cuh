@@ -72,6 +72,7 @@ struct Params {
   long long aLo;
   int c64;                // blocks of 64 channels per image
   int const* bExp;        // conv_half_kernel: scale exponents of the tile images, [column tile][k-block]
+  int8_t const* bOwn;     // and what single columns were scaled beyond them, [column tile][k-block][column]
   int chainShift;         // conv_ts_gen_kernel: 1 << chainShift own k-blocks per accumulation chain
   int fine;               // conv_ts_kernel, 128-column tiles: chains half as long, small terms first (kFine)
   int smemSum;            // conv_ts_kernel, kMode 0 / 1: keep the running sum of a tile in shared memory even for the tile widths that fit the

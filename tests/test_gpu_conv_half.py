@@ -161,6 +161,73 @@ def test_a_filter_tap_knows_nothing_of_rows_that_it_does_not_read(gpu, stride, i
         ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
 
 
+# input, filters, images whose tiles are 16, 32, 64 and two of 128 columns wide: K filters for the filter gradient, C channels for the data gradient
+SMALL = [((8, 8, 64, 8), (3, 3, 64, 64)), ((8, 12, 32, 64), (3, 3, 32, 200)), ((14, 14, 16, 16), (1, 1, 16, 32)), ((10, 10, 200, 32), (3, 3, 200, 16)),
+         ((9, 7, 40, 24), (3, 3, 40, 96)), ((8, 8, 128, 5), (3, 3, 128, 128))]
+
+
+def columns_apart(got, want, axis, bound):
+    got, want = (t.double().movedim(axis, 0).reshape(t.shape[axis], -1) for t in (got, want))
+    off = (got - want).norm(dim=1) / want.norm(dim=1)
+    assert float(off.max()) < bound, (int(off.argmax()), float(off.max()))
+
+
+@pytest.mark.parametrize("precision,bound", [(0, 1e-6), (1, 5e-4)])
+@pytest.mark.parametrize("e", [-15, -18, -30, -44, -70, -100])
+@pytest.mark.parametrize("case", range(len(SMALL)))
+def test_a_filter_or_channel_is_as_exact_beside_far_larger_ones(gpu, case, e, precision, bound):
+    """Filters with small derivatives, channels with small weights, among ordinary ones: each one's gradient by itself against float64, within the bounds of
+    ordinary ones.  At 2^-15 a column still has the tile's power of two, beyond 2^-16 its own."""
+    nn, mat, ctx = gpu
+    import torch
+    xs, fs = SMALL[case]
+    g = torch.Generator(device="cuda").manual_seed(700 + case)
+    x, f = mat.empty(xs).normal_(generator=g), mat.empty(fs).normal_(generator=g)
+    dy = mat.empty(reference(x, f, None, 1, 1, 1)).normal_(generator=g)
+    dy[:, :, 1::3] *= 2.0 ** e
+    f[:, :, 2::5] *= 2.0 ** e
+    dxr, dfr, _ = reference(x, f, dy, 1, 1, 1)
+    lib = ctx.lib
+    ctx.set_precision(precision)
+    try:
+        for switch in (0, 16):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            dx, df, _ = nn.vl_nnconv(x, f, None, dy, pad=1, ctx=ctx)
+            columns_apart(df, dfr, 3, 1e-3 if precision == 1 and switch == 0 else bound)
+            # (16 filters fill too little of a block of 64: the gather that splits as it goes, whose plain TF32 filters are cut off)
+            columns_apart(dx, dxr, 2, 1e-3 if precision == 1 and fs[3] == 16 else bound)
+        assert ctx.device_status() == 0
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+        ctx.set_precision(0)
+
+
+@pytest.mark.parametrize("precision,bound", [(0, 1e-6), (1, 5e-4)])
+@pytest.mark.parametrize("e", [-15, -18, -30, -44, -70, -100])
+@pytest.mark.parametrize("images", [32, 64, 160])
+def test_an_image_is_as_exact_beside_far_larger_ones(gpu, images, e, precision, bound):
+    """Fully connected: images, and filters, whose derivatives are small among ordinary ones."""
+    nn, mat, ctx = gpu
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(800 + images)
+    x, f = mat.empty((4, 4, 512, images)).normal_(generator=g), mat.empty((4, 4, 512, 1024)).normal_(generator=g)
+    dy = mat.empty((1, 1, 1024, images)).normal_(generator=g)
+    X, F, D = x.double().reshape(-1, images), f.double().reshape(-1, 1024), dy.double().reshape(1024, images)
+    small = torch.ones(images, device="cuda", dtype=torch.float64)
+    small[1::3] = 2.0 ** e
+    few = torch.ones(1024, device="cuda", dtype=torch.float64)
+    few[::7] = 2.0 ** e
+    ctx.set_precision(precision)
+    try:
+        dx, _, _ = nn.vl_nnconv(x, f, None, mat.as_mat(dy * small.float()), no_der_filters=True, ctx=ctx)
+        columns_apart(dx.reshape(-1, images), F @ (D * small), 1, bound)
+        _, df, _ = nn.vl_nnconv(x, f, None, mat.as_mat(dy * few.float()[:, None]), no_der_data=True, ctx=ctx)
+        columns_apart(df.reshape(-1, 1024), X @ (D * few[:, None]).T, 1, bound)
+        assert ctx.device_status() == 0
+    finally:
+        ctx.set_precision(0)
+
+
 def test_an_odd_number_of_run_buffers_keeps_the_groups_apart(gpu):
     """128-column tiles of the row mode have three run buffers for two groups of producers: a buffer's previous run belongs to the other group.  A group that
     did not wait for it to be let go of took a run of three k-blocks before for its own, once in some thousand launches."""
