@@ -646,7 +646,7 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
       // This thread's row: channel (row % cPer) of the tile's local tap row / cPer -- the same tap for the whole warp.  A k-block
       // is 64 consecutive output pixels; the row's 68-pixel run lies in shared memory, the wanted 64 start `s` pixels in.
       int const tl = (quarter * 32) / p.cPer;
-      int const H = p.a.H, P = p.plane, nX = p.xStages;
+      int const H = p.a.H, P = p.plane, real = p.a.Ho * p.a.Wo, nX = p.xStages;
       for (int ts = 0; ts < myTiles && ok; ++ts) {
         int const tmf = (cta + ts * ctas) / p.tilesN;
         int const split = tmf / p.tilesM, t = tmf - split * p.tilesM, tg = t % p.tapGroups;
@@ -667,11 +667,12 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
           float w[kWgRowWords];
 #pragma unroll
           for (int j = 0; j < kWgRowWords / 4; ++j) lds128(src + 16u * j, *reinterpret_cast<float(*)[4]>(&w[4 * j]));
-          // pixels whose tap row leaves the image above or below: output row ho + dh outside [0, H) -- the same for every lane's row
-          int const ho0 = (pb + lane) % H, ho1 = (pb + 32 + lane) % H;
+          // pixels whose tap row leaves the image above or below: output row ho + dh outside [0, H) -- the same for every lane's row -- and those that fill
+          // the plane up to whole k-blocks, whose taps to the left still lie inside it (an infinity there times dY's zeros would be none)
+          int const p0 = pb + lane, p1 = p0 + 32, ho0 = p0 % H, ho1 = p1 % H;
           pb += kTsGroups * kTsK; while (pb >= P) pb -= P;
-          uint32_t const zm0 = active ? __ballot_sync(0xffffffffu, (unsigned)(ho0 + dh) >= (unsigned)H) : 0xffffffffu;
-          uint32_t const zm1 = active ? __ballot_sync(0xffffffffu, (unsigned)(ho1 + dh) >= (unsigned)H) : 0xffffffffu;
+          uint32_t const zm0 = active ? __ballot_sync(0xffffffffu, (unsigned)(ho0 + dh) >= (unsigned)H || p0 >= real) : 0xffffffffu;
+          uint32_t const zm1 = active ? __ballot_sync(0xffffffffu, (unsigned)(ho1 + dh) >= (unsigned)H || p1 >= real) : 0xffffffffu;
           // the wanted 64, by two rounds of selects (s is uniform; a copy of the code per shift runs at the speed of instruction fetches)
           if (s != 0) {
             bool const s1 = (s & 1) != 0, s2 = (s & 2) != 0;

@@ -131,6 +131,29 @@ def test_values_that_are_not_finite_stay_where_they_are(gpu, case):
         ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("shape", [(10, 10), (14, 12), (8, 12)])
+@pytest.mark.parametrize("images", [4, 8])
+def test_a_filter_tap_knows_nothing_of_columns_that_it_does_not_read(gpu, images, shape, value):
+    """The last column of a padded plane, which the first filter column never reads -- also where the plane's pixels are filled up to whole k-blocks."""
+    import torch
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(900 + images)
+    x, f, dy = (mat.empty(s).normal_(generator=g) for s in (shape + (32, images), (3, 3, 32, 48), shape + (48, images)))
+    x2 = x.clone()
+    x2[5, shape[1] - 1, 7, images - 1] = value
+    lib = ctx.lib
+    try:
+        for switch in (0, 16):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            _, df, _ = nn.vl_nnconv(x, f, None, dy, pad=1, no_der_data=True, ctx=ctx)
+            _, df2, _ = nn.vl_nnconv(mat.as_mat(x2), f, None, dy, pad=1, no_der_data=True, ctx=ctx)
+            assert torch.equal(df2[:, 0], df[:, 0]), switch
+            assert not torch.isfinite(df2[:, 1:, 7]).any(), switch
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 2.0 ** 60])
 @pytest.mark.parametrize("images", [8, 16, 32, 64])
 @pytest.mark.parametrize("stride", [1, 2])
