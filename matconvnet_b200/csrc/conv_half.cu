@@ -1478,6 +1478,8 @@ TileOut ts_tiles_at(vlb_ctx* ctx, void* at, int rows, int BN, int numKb)
   return out;
 }
 
+constexpr int kMaxGridY = 65535;      // (blocks of 64 channels, groups of images; fully connected layers that fit 32-bit counting have 2^14 at most, the general gather 2^15)
+
 // Scratch of the split form of a tensor of `elements` values in whole blocks of 64 channels.
 size_t chunks_bytes(vlb_ctx* ctx, long long elements)
 {
@@ -1535,7 +1537,7 @@ bool prep_conv_tiles(vlb_ctx* ctx, Params& p, float const* f, vlb::ConvGeom cons
   PrepFilters& q = prep.p[0];
   extraBytes = (extraBytes + 255) & ~(size_t)255;
   int const images = p.M / (p.a.Ho * p.a.Wo);
-  bool const chunks = split_pays(p.a.C, 1, p.a.FH * p.a.FW * vlb::ceil_div(p.N, p.BN));
+  bool const chunks = split_pays(p.a.C, 1, p.a.FH * p.a.FW * vlb::ceil_div(p.N, p.BN)) && vlb::ceil_div(p.a.C, 64) <= kMaxGridY;
   if (chunks) p.numKb = p.splits * (p.kbPerSplit = vlb::ceil_div(p.a.FH * p.a.FW * vlb::ceil_div(p.a.C, 64), p.splits));
   long long const elements = (long long)p.a.H * p.a.W * vlb::ceil_div(p.a.C, 64) * 64 * images;
   float* behind = nullptr;
@@ -1965,6 +1967,8 @@ int conv_wgrad_images(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, flo
   p.M = V; p.N = g.G * p.tilesN * p.BN; p.R = (int)((long long)g.Ho * g.Wo * g.N); p.a.rows = V; p.wg = 2;
   size_t const nF = (size_t)V * g.K;
   if ((long long)nF * p.splits >= (1LL << 31)) return -1;
+  // (a block of the input's preparation per group of images on gridDim.y)
+  if ((gShift == 3 ? p.nGroups : p.nGroups << gShift) > kMaxGridY) return -1;
   // scratch: tile images, partial results, the input's chunks (64 images per k-block: split, with exponents), the bias gradient's partial sums
   int const imgGroups = p.nGroups << gShift, tiles = g.G * p.tilesN;
   long long const chunks = (long long)imgGroups * g.H * g.W * g.C;

@@ -251,6 +251,37 @@ def test_an_image_is_as_exact_beside_far_larger_ones(gpu, images, e, precision, 
         ctx.set_precision(0)
 
 
+def test_more_groups_of_images_than_a_grid_is_high(gpu):
+    """65537 groups of eight images: a launch takes 65535 along y, so the filter gradient has to come from a kernel that counts them otherwise."""
+    import torch
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(79)
+    images = 8 * 65537
+    x, f, dy = mat.empty((8, 1, 32, images)).normal_(generator=g), mat.empty((1, 1, 32, 16)).normal_(generator=g), mat.empty((8, 1, 16, images)).normal_(generator=g)
+    want = torch.einsum("hwcn,hwkn->ck", x.double(), dy.double())
+    lib = ctx.lib
+    try:
+        for switch in (0, 16):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            _, df, db = nn.vl_nnconv(x, f, mat.zeros((1, 16)), dy, no_der_data=True, ctx=ctx)
+            assert rel(df[0, 0], want) < 1e-6 and rel(db.reshape(-1), dy.double().sum((0, 1, 3))) < 1e-5
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+
+
+def test_more_blocks_of_channels_than_a_grid_is_high(gpu):
+    """The data gradient of 65537 blocks of 64 filters, two column tiles.  The reduction is cut into at least 74 ranges (two tiles on 148 SMs); the running sum
+    of one has 886 k-blocks, whose rounding, 2^-24 each at random, comes to 1.8e-6 at most."""
+    import torch
+    nn, mat, ctx = gpu
+    g = torch.Generator(device="cuda").manual_seed(80)
+    k = 64 * 65537
+    f, dy = mat.empty((1, 1, 130, k)).normal_(generator=g), mat.empty((2, 2, k, 1)).normal_(generator=g)
+    dx, _, _ = nn.vl_nnconv(mat.zeros((2, 2, 130, 1)), f, None, dy, no_der_filters=True, ctx=ctx)
+    assert rel(dx[..., 0], torch.einsum("ck,hwk->hwc", f[0, 0].double(), dy[..., 0].double())) < 2e-6
+    ctx.check(ctx.lib.vlb_ctx_clear_workspace(ctx.handle))
+
+
 def test_an_odd_number_of_run_buffers_keeps_the_groups_apart(gpu):
     """128-column tiles of the row mode have three run buffers for two groups of producers: a buffer's previous run belongs to the other group.  A group that
     did not wait for it to be let go of took a run of three k-blocks before for its own, once in some thousand launches."""
