@@ -87,6 +87,8 @@ int vlb_ctx_set_wait_limit(vlb_ctx* ctx, long long cycles);
  * Bit 2: the filter gradient of a convolution takes the kernel with both operands in shared memory even where the
  * tensor-memory kernel applies (the two differ in the order of the sums; a test checks both against the CPU checker).
  * Bit 4: the filter gradient takes the form with the images along the reduction wherever that is possible, not only where it pays.
+ * Bit 5: scratch that a call can do without is refused, as where the device's memory does not hold it: gradients come from the kernels that need no copy
+ * of the data or of the output derivative.
  * Bit 3: the tensor-memory convolution kernel keeps the running sum of an output tile in shared memory even for the tile
  * widths (64 and 128 columns) whose sum fits the registers of its drain warps; same additions in the same order, so the
  * results are equal, which is what a test compares. */

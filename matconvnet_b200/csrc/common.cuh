@@ -56,6 +56,8 @@ int pass_error(vlb_ctx* ctx, int code, char const* where);
 // Scratch of at least `bytes`; contents belong to whichever op asked last
 // (reference Context::getWorkspace, bits/data.cu:395-404).  nullptr on failure.
 void* workspace(vlb_ctx* ctx, size_t bytes);
+// The same for a route that has another to fall back on: nullptr, and no error, where so much cannot be had.
+void* try_workspace(vlb_ctx* ctx, size_t bytes);
 // cudaPeekAtLastError after a launch, as the reference does (bits/datacu.cu:356-371).
 int check_launch(vlb_ctx* ctx, char const* where);
 

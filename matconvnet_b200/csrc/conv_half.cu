@@ -1530,16 +1530,18 @@ bool prep_dense_tiles(vlb_ctx* ctx, Params& p, float const* f, bool rows, size_t
 
 // The filter bank of one group, reduction in blocks of 32 channels (conv_half_kernel): forward, or flipped and transposed for the data gradient
 // of a stride-1 convolution.
-// Where it pays, the gathered tensor is split beforehand (kMode 3).
+// Where it pays and there is room for the chunks, the gathered tensor is split beforehand (kMode 3).
 bool prep_conv_tiles(vlb_ctx* ctx, Params& p, float const* f, vlb::ConvGeom const& g, bool dgrad, size_t extraBytes, float** extra)
 {
   PrepBatch prep = {};
   PrepFilters& q = prep.p[0];
   extraBytes = (extraBytes + 255) & ~(size_t)255;
   int const images = p.M / (p.a.Ho * p.a.Wo);
-  bool const chunks = split_pays(p.a.C, 1, p.a.FH * p.a.FW * vlb::ceil_div(p.N, p.BN)) && vlb::ceil_div(p.a.C, 64) <= kMaxGridY;
-  if (chunks) p.numKb = p.splits * (p.kbPerSplit = vlb::ceil_div(p.a.FH * p.a.FW * vlb::ceil_div(p.a.C, 64), p.splits));
   long long const elements = (long long)p.a.H * p.a.W * vlb::ceil_div(p.a.C, 64) * 64 * images;
+  int const chunkKb = vlb::ceil_div(p.a.FH * p.a.FW * vlb::ceil_div(p.a.C, 64), p.splits);
+  bool const chunks = split_pays(p.a.C, 1, p.a.FH * p.a.FW * vlb::ceil_div(p.N, p.BN)) && vlb::ceil_div(p.a.C, 64) <= kMaxGridY &&
+                      vlb::try_workspace(ctx, ts_tiles_bytes(ctx, p.N, p.BN, p.splits * chunkKb) + extraBytes + chunks_bytes(ctx, elements));
+  if (chunks) p.numKb = p.splits * (p.kbPerSplit = chunkKb);
   float* behind = nullptr;
   if (!ts_tiles(ctx, p, extraBytes + (chunks ? chunks_bytes(ctx, elements) : 0), &q.out, &behind)) return false;
   if (extra) *extra = behind;
@@ -1843,7 +1845,7 @@ PrepFilters gen_prep(Params const& p, ConvGeom const& g, float const* f)
 // Builds the tile images of all problems (one launch) and runs them (one launch).  The problems share the tile width.
 // Where the problems' tiles are too few for the chip the reductions are cut, all into the same number of ranges, and `fin` (the epilogue,
 // which the problems then do not apply themselves) goes to the sum over the ranges; they cover every element of the output then
-// (`covered`).
+// (`covered`).  -1: the gather that splits as it goes has it (a reduction too long; no room for the chunks).
 int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size_t nOut, vlb::SumEpilogue const& fin, bool covered, char const* where)
 {
   bool const split3 = ctx->precision == VLB_PRECISION_3XTF32;
@@ -1869,7 +1871,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     else { p.e.bias = fin.bias; p.e.inMult = fin.inMult; p.e.outMult = fin.outMult; p.e.relu = fin.relu; p.e.mask = fin.mask; }
     offset[i] = total;
     total += ts_tiles_bytes(ctx, p.tilesN * BN, BN, p.numKb);
-    if (p.numKb > 32767) return VLB_Unsupported;
+    if (p.numKb > 32767) return -1;
     long long const t = (long long)p.tilesM * p.tilesN * p.splits;
     tiles += t;
     work += (double)t * (p.kbPerSplit + 6);
@@ -1880,8 +1882,8 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
   int const images = (int)(b.p[0].M / ((long long)a0.Ho * a0.Wo)), channels = (int)(a0.imgStride / ((long long)a0.H * a0.W));
   long long const elements = (long long)a0.H * a0.W * vlb::ceil_div(channels, 64) * 64 * images;
   size_t const partBytes = splits > 1 ? (sizeof(float) * nOut * splits + 255) & ~(size_t)255 : 0;
-  char* const ws = (char*)vlb::workspace(ctx, total + partBytes + chunks_bytes(ctx, elements));
-  if (!ws) return ctx->lastError;
+  char* const ws = (char*)vlb::try_workspace(ctx, total + partBytes + chunks_bytes(ctx, elements));
+  if (!ws) return -1;
   float* const part = (float*)(ws + total);
   split_chunks(ctx, b.p[0], ws + total + partBytes, images, channels);
   // CTAs per problem: one per tile when all tiles fit, else shares of the chip in proportion to the work, the rest to the longest queues
@@ -1981,11 +1983,13 @@ int conv_wgrad_images(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, flo
   int const octets = ceil_div(p.kbTot, oBlocks) * ceil_div(oH, 8);
   int const fBlocks = tiles * std::max(p.BN / 32, 1);
   int const gx = std::max(1, std::min(4 * ctx->smCount / fBlocks, octets));
+  size_t const extraBytes = partBytes + ((chunkBytes + 255) & ~(size_t)255) + 256 + expBytes + (db ? sizeof(float) * (size_t)gx * fBlocks * 32 : 0);
+  if (!try_workspace(ctx, ts_tiles_bytes(ctx, p.N, p.BN, p.numKb) + extraBytes)) return -1;      // (the other kernels need no copy of the input)
   TileOut out;
   float* at = nullptr;
   ProfScope prof(ctx, kProfWgrad);
   prof.rec.flops = 2.0 * (double)V * (double)g.Kg * g.G * (double)p.R;
-  if (!ts_tiles(ctx, p, partBytes + ((chunkBytes + 255) & ~(size_t)255) + 256 + expBytes + (db ? sizeof(float) * (size_t)gx * fBlocks * 32 : 0), &out, &at)) return ctx->lastError;
+  if (!ts_tiles(ctx, p, extraBytes, &out, &at)) return ctx->lastError;
   float* const part = at;
   uint4* const hi = (uint4*)((char*)at + partBytes);
   uint4* const zero = (uint4*)((char*)hi + ((chunkBytes + 255) & ~(size_t)255));
@@ -2078,10 +2082,10 @@ int fc_dgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, fl
   prof.rec.flops = 2.0 * (double)V * (double)g.N * (double)g.K;
   // more than 128 images: several column tiles read the weights, from chunks then (256 images, V = 25088, K = 4096: 322 us -> 264, of
   // which 122 are the split, at the copy rate)
-  bool const chunks = split_pays(g.K, 1, vlb::ceil_div(p.N, p.BN));
-  size_t const partRoom = (partBytes + 255) & ~(size_t)255;
+  size_t const partRoom = (partBytes + 255) & ~(size_t)255, chunkBytes = chunks_bytes(ctx, (long long)V * vlb::ceil_div(g.K, 64) * 64);
+  bool const chunks = split_pays(g.K, 1, vlb::ceil_div(p.N, p.BN)) && try_workspace(ctx, ts_tiles_bytes(ctx, p.N, p.BN, p.numKb) + partRoom + chunkBytes);
   float* behind = nullptr;
-  if (!prep_dense_tiles(ctx, p, dY, true, partRoom + (chunks ? chunks_bytes(ctx, (long long)V * vlb::ceil_div(g.K, 64) * 64) : 0), &behind)) return ctx->lastError;      // B(n, k) = dY[k + K n]
+  if (!prep_dense_tiles(ctx, p, dY, true, partRoom + (chunks ? chunkBytes : 0), &behind)) return ctx->lastError;      // B(n, k) = dY[k + K n]
   float* const part = p.splits > 1 ? behind : nullptr;
   if (chunks) split_chunks(ctx, p, (char*)behind + partRoom, 1, g.K);
   p.e = Epilogue{};
@@ -2109,9 +2113,10 @@ int fc_wgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dF, float const* X, fl
   prof.rec.flops = 2.0 * (double)V * (double)g.K * (double)g.N;
   // the column tiles of the filters all read X, from chunks (eight images of an input) where the images fill blocks of 64 (V = 25088, K = 4096, 256 images:
   // 335 us -> 220; 64 images 207 -> 133, where the gradient's 411 MB take 63)
-  bool const chunks = split_pays(g.N, 1, vlb::ceil_div(p.N, p.BN));
+  size_t const chunkBytes = chunks_bytes(ctx, (long long)V * vlb::ceil_div(g.N, 64) * 64);
+  bool const chunks = split_pays(g.N, 1, vlb::ceil_div(p.N, p.BN)) && try_workspace(ctx, ts_tiles_bytes(ctx, p.N, p.BN, p.numKb) + chunkBytes);
   float* behind = nullptr;
-  if (!prep_dense_tiles(ctx, p, dY, false, chunks ? chunks_bytes(ctx, (long long)V * vlb::ceil_div(g.N, 64) * 64) : 0, &behind)) return ctx->lastError;      // B(k, n) = dY[k + K n]
+  if (!prep_dense_tiles(ctx, p, dY, false, chunks ? chunkBytes : 0, &behind)) return ctx->lastError;      // B(k, n) = dY[k + K n]
   if (chunks) split_chunks(ctx, p, behind, 1, g.N);
   p.e = Epilogue{};
   p.e.out = dF; p.e.inMult = 1.f; p.e.P = V; p.e.Ktot = g.K;

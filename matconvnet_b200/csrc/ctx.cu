@@ -27,10 +27,8 @@ int pass_error(vlb_ctx* ctx, int code, char const* where)
   return code;
 }
 
-void* workspace(vlb_ctx* ctx, size_t bytes)
+static cudaError_t grow_workspace(vlb_ctx* ctx, size_t bytes)
 {
-  if (bytes <= ctx->workspaceBytes && ctx->workspace) return ctx->workspace;
-  if (bytes == 0) bytes = 256;
   if (ctx->workspace) {
     // Work enqueued earlier may still be using the old buffer.
     cudaStreamSynchronize(ctx->stream);
@@ -39,15 +37,34 @@ void* workspace(vlb_ctx* ctx, size_t bytes)
     ctx->workspaceBytes = 0;
   }
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    set_error(ctx, VLB_OutOfGPUMemeory, cudaGetErrorString(e));
-    return nullptr;
-  }
+  cudaError_t const e = cudaMalloc(&p, bytes);
+  if (e != cudaSuccess) { cudaGetLastError(); return e; }
   ctx->workspace = p;
   ctx->workspaceBytes = bytes;
-  return p;
+  return cudaSuccess;
+}
+
+void* workspace(vlb_ctx* ctx, size_t bytes)
+{
+  if (bytes <= ctx->workspaceBytes && ctx->workspace) return ctx->workspace;
+  cudaError_t const e = grow_workspace(ctx, bytes == 0 ? 256 : bytes);
+  if (e != cudaSuccess) set_error(ctx, VLB_OutOfGPUMemeory, cudaGetErrorString(e));
+  return ctx->workspace;
+}
+
+void* try_workspace(vlb_ctx* ctx, size_t bytes)
+{
+  if (ctx->testSwitch & 32) return nullptr;
+  if (bytes <= ctx->workspaceBytes && ctx->workspace) return ctx->workspace;
+  // a stream that is being captured can neither wait nor allocate: the scratch that was reserved has to do
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (capture != cudaStreamCaptureStatusNone) return nullptr;
+  // what the device cannot hold leaves the buffer that is there, so that a program which lives with the smaller one does not pay for it on every call
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) cudaGetLastError();
+  else if (bytes > free + ctx->workspaceBytes) return nullptr;
+  return grow_workspace(ctx, bytes == 0 ? 256 : bytes) == cudaSuccess ? ctx->workspace : nullptr;
 }
 
 int check_launch(vlb_ctx* ctx, char const* where)

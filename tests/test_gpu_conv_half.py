@@ -311,3 +311,123 @@ def test_run_buffers_of_a_fully_connected_forward_pass(gpu):
     finally:
         ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
     assert ctx.device_status() == 0
+
+
+# data, filters, stride: a data gradient in one piece, one by residue classes, one in filter groups; filter gradients of 64 images per k-block, of fewer, of planes
+# that the row mode does not take
+SCRATCH = [((28, 28, 64, 70), (3, 3, 64, 128), 1), ((14, 14, 64, 16), (3, 3, 64, 64), 2), ((13, 13, 128, 9), (3, 3, 64, 128), 1), ((7, 7, 512, 32), (3, 3, 512, 512), 1)]
+
+
+@pytest.mark.parametrize("case", range(len(SCRATCH)))
+def test_gradients_without_room_for_chunks(gpu, case):
+    """Test switch bit 5: the kernels that need no copy of the data or of dY, in less scratch, as near to float64."""
+    nn, mat, ctx = gpu
+    import torch
+    xs, fs, stride = SCRATCH[case]
+    g = torch.Generator(device="cuda").manual_seed(1000 + case)
+    x, f = mat.empty(xs).normal_(generator=g), mat.empty(fs).normal_(generator=g)
+    dy = mat.empty(reference(x, f, None, stride, 1, 1)).normal_(generator=g)
+    dxr, dfr, dbr = reference(x, f, dy, stride, 1, 1)
+    lib = ctx.lib
+    needs = {}
+    try:
+        for switch in (0, 16, 32, 48):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            needs[switch] = []
+            for kw in (dict(no_der_filters=True, no_der_biases=True), dict(no_der_data=True)):
+                ctx.check(lib.vlb_ctx_clear_workspace(ctx.handle))
+                dx, df, db = nn.vl_nnconv(x, f, mat.zeros((1, fs[3])), dy, stride=stride, pad=1, ctx=ctx, **kw)
+                needs[switch].append(lib.vlb_ctx_workspace_bytes(ctx.handle))
+                if "no_der_data" in kw:
+                    # (tc_gemm_kernel's chains: the bound of its own tests)
+                    assert rel(df, dfr) < 1e-5 and rel(db.reshape(-1), dbr) < 1e-5, switch
+                else:
+                    assert rel(dx, dxr) < 1e-5, switch
+        assert ctx.device_status() == 0
+        assert needs[32] == needs[48] and needs[32][0] < needs[0][0] and needs[32][1] != needs[16][1]
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+
+
+@pytest.mark.parametrize("images", [256, 640])
+def test_fully_connected_gradients_without_room_for_chunks(gpu, images):
+    nn, mat, ctx = gpu
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1100 + images)
+    x, f, dy = mat.empty((4, 4, 512, images)).normal_(generator=g), mat.empty((4, 4, 512, 512)).normal_(generator=g), mat.empty((1, 1, 512, images)).normal_(generator=g)
+    X, F, D = x.double().reshape(-1, images), f.double().reshape(-1, 512), dy.double().reshape(512, images)
+    lib = ctx.lib
+    needs = {}
+    try:
+        for switch in (0, 32):
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, switch))
+            ctx.check(lib.vlb_ctx_clear_workspace(ctx.handle))
+            dx, df, _ = nn.vl_nnconv(x, f, None, dy, ctx=ctx)
+            needs[switch] = lib.vlb_ctx_workspace_bytes(ctx.handle)
+            assert rel(dx.reshape(-1, images), F @ D) < 1e-6 and rel(df.reshape(-1, 512), X @ D.T) < 1e-6, switch
+        assert needs[32] < needs[0]
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+
+
+def test_a_device_without_room_for_chunks(gpu):
+    """No switch: so little of the device's memory left that the 0.5 GB of dY's chunks, and 0.5 GB of the data's beside the tile images of dY, do not fit.  The
+    same kernels as with the switch, so the same bits."""
+    nn, mat, ctx = gpu
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1200)
+    x, f, dy = mat.empty((56, 56, 64, 640)).normal_(generator=g), mat.empty((3, 3, 64, 64)).normal_(generator=g), mat.empty((56, 56, 64, 640)).normal_(generator=g)
+    lib = ctx.lib
+    taken = None
+    try:
+        for kw, which, left in ((dict(no_der_filters=True), 0, 256), (dict(no_der_data=True), 1, 768)):
+            ctx.check(lib.vlb_ctx_clear_workspace(ctx.handle))
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 32))
+            want = nn.vl_nnconv(x, f, None, dy, pad=1, ctx=ctx, **kw)[which]
+            need = lib.vlb_ctx_workspace_bytes(ctx.handle)
+            again = nn.vl_nnconv(x, f, None, dy, pad=1, ctx=ctx, **kw)[which]
+            del again                                         # (torch keeps the room of a second output)
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+            ctx.check(lib.vlb_ctx_clear_workspace(ctx.handle))
+            torch.cuda.synchronize()
+            taken = torch.empty(torch.cuda.mem_get_info()[0] - (left << 20), dtype=torch.uint8, device="cuda")
+            for _ in range(2):
+                got = nn.vl_nnconv(x, f, None, dy, pad=1, ctx=ctx, **kw)[which]
+                assert torch.equal(got, want)
+                del got
+            assert lib.vlb_ctx_workspace_bytes(ctx.handle) == need
+            del taken
+            taken = None
+            torch.cuda.empty_cache()
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+        ctx.check(lib.vlb_ctx_clear_workspace(ctx.handle))
+
+
+def test_a_captured_call_makes_do_with_the_scratch_that_is_there(gpu):
+    """A stream that is being captured can neither wait nor allocate."""
+    nn, mat, ctx = gpu
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1300)
+    x, f, dy = mat.empty((14, 14, 64, 64)).normal_(generator=g), mat.empty((3, 3, 64, 64)).normal_(generator=g), mat.empty((14, 14, 64, 64)).normal_(generator=g)
+    lib = ctx.lib
+    try:
+        for kw, which in ((dict(no_der_filters=True), 0), (dict(no_der_data=True), 1)):
+            ctx.check(lib.vlb_ctx_clear_workspace(ctx.handle))
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 32))
+            want = nn.vl_nnconv(x, f, None, dy, pad=1, ctx=ctx, **kw)[which]
+            need = lib.vlb_ctx_workspace_bytes(ctx.handle)
+            ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                got = nn.vl_nnconv(x, f, None, dy, pad=1, ctx=ctx, **kw)[which]
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(got, want) and lib.vlb_ctx_workspace_bytes(ctx.handle) == need
+            graph.reset()
+    finally:
+        ctx.check(lib.vlb_ctx_set_test_switch(ctx.handle, 0))
+        nn.vl_nnrelu(x, ctx=ctx)            # (the context follows torch's current stream again)
+        ctx.check(lib.vlb_ctx_clear_workspace(ctx.handle))
