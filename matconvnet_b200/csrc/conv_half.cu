@@ -363,7 +363,7 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
         // thread, coalesced along the rows: nothing here waits for anything.  (Every load of this phase -- a patch of shared memory, a
         // bias -- cost the drain warps its full latency plus a queue behind the producers' gathers: 4.4k cycles per 128-column tile through
         // 16-byte stores from a patch, 13k to 20k where planes of 13 x 13 or 27 x 27 pixels rule those out.)
-        bool const direct = p.e.inMult == 1.f && p.e.outMult == 0.f && (p.e.bias == nullptr || p.biasFirst) && (p.e.mask == nullptr || preMask) && !(kGen && p.shufY > 0);
+        bool const direct = (p.e.bias == nullptr || p.biasFirst) && (p.e.mask == nullptr || preMask) && !(kGen && p.shufY > 0);
         if (preMask) {
 #pragma unroll
           for (int j = 0; j < kCols; j += 2) {
@@ -378,7 +378,6 @@ __device__ __forceinline__ void conv_half_body(Params const& p, CUtensorMap cons
           for (int j = 0; j < kCols; j += 2) {
             float a, b;
             unpack2(P2[j / 2], a, b);
-            if (p.e.relu) { a = a > 0.f ? a : 0.f; b = b > 0.f ? b : 0.f; }
             if (dst.valid && j < nEndT) *o = a;
             o += p.e.P;
             if (dst.valid && j + 1 < nEndT) *o = b;
@@ -1528,10 +1527,9 @@ bool prep_dense_tiles(vlb_ctx* ctx, Params& p, float const* f, bool rows, size_t
   return true;
 }
 
-// The filter bank of one group, reduction in blocks of 32 channels (conv_half_kernel): forward, or flipped and transposed for the data gradient
-// of a stride-1 convolution.
+// The filter bank of one group flipped and transposed, for the data gradient of a stride-1 convolution (conv_half_kernel).
 // Where it pays and there is room for the chunks, the gathered tensor is split beforehand (kMode 3).
-bool prep_conv_tiles(vlb_ctx* ctx, Params& p, float const* f, vlb::ConvGeom const& g, bool dgrad, size_t extraBytes, float** extra)
+bool prep_flipped_tiles(vlb_ctx* ctx, Params& p, float const* f, vlb::ConvGeom const& g, size_t extraBytes, float** extra)
 {
   PrepBatch prep = {};
   PrepFilters& q = prep.p[0];
@@ -1547,9 +1545,9 @@ bool prep_conv_tiles(vlb_ctx* ctx, Params& p, float const* f, vlb::ConvGeom cons
   if (extra) *extra = behind;
   if (chunks) split_chunks(ctx, p, (char*)behind + extraBytes, images, p.a.C);
   q.f = f; q.BN = p.BN; q.numKb = p.numKb; q.tilesPerGroup = vlb::ceil_div(p.N, p.BN); q.rows = q.tilesPerGroup * p.BN; q.cols = p.N;
-  q.tapsH = q.FH = g.FH; q.tapsW = q.FW = g.FW; q.C = dgrad ? g.K : g.C;
-  q.bh = dgrad ? g.FH - 1 : 0; q.bw = dgrad ? g.FW - 1 : 0; q.ah = q.aw = dgrad ? -1 : 1;
-  q.sn = dgrad ? 1 : g.C; q.sq = dgrad ? g.C : 1; q.whole = p.aHi != nullptr;
+  q.tapsH = q.FH = g.FH; q.tapsW = q.FW = g.FW; q.C = g.K;
+  q.bh = g.FH - 1; q.bw = g.FW - 1; q.ah = q.aw = -1;
+  q.sn = 1; q.sq = g.C; q.whole = p.aHi != nullptr;
   launch_prep(ctx, prep, 1);
   return true;
 }
@@ -1659,7 +1657,7 @@ bool plan_windows(vlb_ctx* ctx, Params& p, CUtensorMap* map, size_t* smemBytes, 
   return true;
 }
 
-// fprop / stride-1 dgrad with the gathered operand in tensor memory (p.bTiles set, p.a a convolution operand).
+// Stride-1 and fully connected gradients with the gathered operand in tensor memory (p.bTiles set, p.a a convolution operand).
 int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
 {
   bool split3 = ctx->precision == VLB_PRECISION_3XTF32;
@@ -1677,7 +1675,7 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   bool const windows = p.aHi == nullptr && plan_windows(ctx, p, &map, &smemBytes, split3);
-  p.biasFirst = p.e.bias != nullptr && aligned16(p.e.bias) && p.N % 4 == 0 && p.e.inMult == 1.f && p.e.outMult == 0.f;
+  p.biasFirst = p.e.bias != nullptr && aligned16(p.e.bias) && p.N % 4 == 0;
   ts_divisors(p);
   if (smemBytes < 120u * 1024u) smemBytes = 120u * 1024u;
   long long const numTiles = (long long)p.tilesM * p.tilesN * p.splits;
@@ -1686,13 +1684,6 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
   // while the next one is computed.
   dim3 grid((unsigned)std::min<long long>(numTiles, ctx->smCount), 1, 1);
   cudaError_t e;
-  vlb_ctx::ProfRec rec;
-  bool const record = ctx->profiling && ctx->profDepth == 0;
-  if (record) {
-    cudaEventCreate(&rec.start); cudaEventCreate(&rec.stop);
-    rec.flops = 2.0 * (double)p.M * (double)p.N * (double)p.R; rec.kind = -1;
-    cudaEventRecord(rec.start, ctx->stream);
-  }
   bool const narrow = p.BN <= 64;
   auto go = [&](auto kernel) {
     e = allow_large_smem<decltype(kernel)::value>(ctx->device);
@@ -1710,7 +1701,6 @@ int launch_ts(vlb_ctx* ctx, Params& p, char const* where)
     else         { if (narrow) VLB_TS(false, 0, true); else VLB_TS(false, 0, false); }
   }
 #undef VLB_TS
-  if (record) { cudaEventRecord(rec.stop, ctx->stream); ctx->prof.push_back(rec); }
   if (e != cudaSuccess) { cudaGetLastError(); return vlb::set_error(ctx, VLB_Cuda, cudaGetErrorString(e)); }
   VLB_LAUNCHED(ctx, 1);
   return vlb::check_launch(ctx, where);
@@ -1868,7 +1858,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     prep.p[i].numKb = p.numKb;
     p.e.out = out;
     if (splits > 1) p.e.splitStride = (long long)nOut;
-    else { p.e.bias = fin.bias; p.e.inMult = fin.inMult; p.e.outMult = fin.outMult; p.e.relu = fin.relu; p.e.mask = fin.mask; }
+    else { p.e.bias = fin.bias; p.e.mask = fin.mask; }
     offset[i] = total;
     total += ts_tiles_bytes(ctx, p.tilesN * BN, BN, p.numKb);
     if (p.numKb > 32767) return -1;
@@ -1916,7 +1906,7 @@ int launch_ts_gen(vlb_ctx* ctx, TsProblems& b, PrepBatch& prep, float* out, size
     p.c64 = b.p[0].c64; p.aHi = b.p[0].aHi; p.aLo = b.p[0].aLo; p.aExp = b.p[0].aExp; p.zero = b.p[0].zero;
     p.status = ctx->deviceStatus; p.testSwitch = ctx->testSwitch; p.chanFast = 1; p.bStages = stages;
     ts_divisors(p);
-    p.biasFirst = p.e.bias != nullptr && aligned16(p.e.bias) && p.cols % 4 == 0 && p.shufY == 0 && p.e.inMult == 1.f && p.e.outMult == 0.f;
+    p.biasFirst = p.e.bias != nullptr && aligned16(p.e.bias) && p.cols % 4 == 0 && p.shufY == 0;
   }
   launch_prep(ctx, prep, b.n);
   size_t const smemBytes = std::max<size_t>((size_t)stages * stageBytes + patchBytes + 1024, 120u * 1024u);      // two CTAs never share an SM
@@ -2159,7 +2149,7 @@ int conv_dgrad_half(vlb_ctx* ctx, ConvGeom const& g, float* dX, float const* F, 
   p.numKb = p.splits * p.kbPerSplit;
   size_t const nOut = (size_t)p.M * g.C;
   float* part = nullptr;
-  if (!prep_conv_tiles(ctx, p, F, g, true, p.splits > 1 ? sizeof(float) * nOut * p.splits : 0, &part)) return ctx->lastError;
+  if (!prep_flipped_tiles(ctx, p, F, g, p.splits > 1 ? sizeof(float) * nOut * p.splits : 0, &part)) return ctx->lastError;
   p.e = Epilogue{}; p.e.out = dX; p.e.inMult = 1.f; p.e.P = g.H * g.W; p.e.Ktot = g.C;
   ctx->maskDone = ctx->reluMask != nullptr; ctx->biasDone = true;
   if (p.splits == 1) { p.e.mask = ctx->reluMask; p.e.bias = ctx->dgradBias; return launch_ts(ctx, p, "conv_dgrad_half"); }

@@ -1581,7 +1581,7 @@ constexpr int kPrepThreads = 256, kPrepIters = 4;
 // kVec: planes of a multiple of four pixels on a 16-byte boundary; otherwise (13 x 13, 27 x 27 maps) four scalar loads.
 template <bool kSplit, bool kVec>
 __global__ void __launch_bounds__(kPrepThreads)
-prep_dy_tiles_kernel(float* __restrict__ out, float const* __restrict__ dy, int N, int R, int P, int Pp, int BN, int numKb,
+prep_dy_tiles_kernel(float* __restrict__ out, float const* __restrict__ dy, int N, int R, int P, int BN, int numKb,
                      float* __restrict__ db, float* __restrict__ dbPart, unsigned* __restrict__ tickets, int Kg, int tilesPerGroup)
 {
   vlb::pdl_wait();
@@ -1597,12 +1597,11 @@ prep_dy_tiles_kernel(float* __restrict__ out, float const* __restrict__ dy, int 
     int const r = ((int)blockIdx.x * kPrepIters + u) * (kPrepThreads * 4) + (int)threadIdx.x * 4;
     if (r < Rp) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      // reduction index r = pixel + Pp * image (Pp >= P: planes padded to whole k-blocks read as zeros); R = P * images
-      int const img = r / Pp, pix = r - img * Pp;
+      // reduction index r = pixel + P * image; R = P * images
+      int const img = r / P, pix = r - img * P;
       if (kVec) {
-        if (n < N && pix < P && img * P + pix < R) v = *reinterpret_cast<float4 const*>(dy + ((size_t)img * N + n) * P + pix);
+        if (n < N && r < R) v = *reinterpret_cast<float4 const*>(dy + ((size_t)img * N + n) * P + pix);
       } else if (n < N) {
-        // (planes that are no multiple of four pixels are never padded: Pp == P)
         float w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -1679,10 +1678,8 @@ float const* prep_conv_tiles(vlb_ctx* ctx, float const* f, vlb::ConvGeom const& 
 
 // dY tile images and, when db is given, the bias gradient from the same sweep; K channels in `groups` filter groups.
 // Scratch layout: [tiles][extraBytes for the caller][per-block partial sums of db].
-float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, int BN, int numKb, size_t extraBytes, float* db, int Pp = 0,
-                           int groups = 1)
+float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, int BN, int numKb, size_t extraBytes, float* db, int groups = 1)
 {
-  if (Pp == 0) Pp = P;
   bool split3 = ctx->precision == VLB_PRECISION_3XTF32;
   int const Kg = K / groups, tpg = vlb::ceil_div(Kg, BN), rows = groups * tpg * BN;
   bool const vec = P % 4 == 0 && (((uintptr_t)dY) & 15) == 0;
@@ -1697,7 +1694,7 @@ float const* prep_dy_tiles(vlb_ctx* ctx, float const* dY, int K, int R, int P, i
   float* dbPart = db ? (float*)(ws + tileBytes + extraBytes) : nullptr;
   unsigned* tickets = (unsigned*)((char*)ctx->deviceStatus + 256);
   dim3 grid(bx, (unsigned)rows);
-#define VLB_PDY(split, v) vlb::launch(ctx->stream, prep_dy_tiles_kernel<split, v>, grid, kPrepThreads, 0, tiles, dY, K, R, P, Pp, BN, numKb, db, dbPart, tickets, Kg, tpg)
+#define VLB_PDY(split, v) vlb::launch(ctx->stream, prep_dy_tiles_kernel<split, v>, grid, kPrepThreads, 0, tiles, dY, K, R, P, BN, numKb, db, dbPart, tickets, Kg, tpg)
   if (split3) { if (vec) VLB_PDY(true, true); else VLB_PDY(true, false); }
   else        { if (vec) VLB_PDY(false, true); else VLB_PDY(false, false); }
 #undef VLB_PDY
@@ -2324,7 +2321,7 @@ int conv_wgrad_tc(vlb_ctx* ctx, ConvGeom const& g, float* dF, float* db, float c
   // dY is split into hi / lo once and laid out as tile images, like the filters of fprop
   size_t const tileBytes = b_tiles_bytes(ctx, tpg * p.BN * g.G, p.BN, p.numKb);
   float* const dbHere = g.K <= 4096 ? db : nullptr;      // (a ticket counter per channel)
-  p.bTiles = prep_dy_tiles(ctx, dY, g.K, p.R, P, p.BN, p.numKb, partBytes, dbHere, 0, g.G);
+  p.bTiles = prep_dy_tiles(ctx, dY, g.K, p.R, P, p.BN, p.numKb, partBytes, dbHere, g.G);
   if (!p.bTiles) return ctx->lastError;
   *dbDone = dbHere != nullptr;
   if (splits == 1) {
