@@ -155,7 +155,7 @@ def contraction_kernels(ctx, passes, peak_tf32):
     names = ["conv fprop (conv_ts_kernel; conv1_1 runs on CUDA cores and is not in this sum)",
              "conv dgrad (dY split into chunks + conv_half_kernel, ReLU mask fused)",
              "conv wgrad + dbias (x split into chunks, dY tile images, conv_half_kernel, sum of the reduction ranges; conv1_1 on CUDA cores)",
-             "fully connected fprop/dgrad/wgrad (fc6 on conv_ts_kernel and conv_half_kernel: weights read or written once; fc7, fc8 on tc_gemm_kernel)"]
+             "fully connected fprop/dgrad/wgrad (fc6 on conv_ts_kernel and conv_half_kernel: weights read or written once; the others on conv_half_kernel and tc_gemm_kernel)"]
     out = []
     for kind, name in enumerate(names):
         ms, fl, n = ctx.profile_kind(kind)
@@ -356,7 +356,7 @@ def main():
                 "traffic": None,
                 "traffic_note": "DRAM bytes are captured per kernel on single layers (one kernel, a few launches) and kept under "
                                 "profiles/; no whole-step counter capture is made",
-                "kernel": "conv_ts_kernel (conv fprop, fc6), conv_half_kernel (conv dgrad / wgrad, fc6) + tc_gemm_kernel (fc7, fc8), operand "
+                "kernel": "conv_ts_kernel (conv fprop, fc6), conv_half_kernel (conv dgrad / wgrad, fc6) + tc_gemm_kernel (fc7 fprop, fc8), operand "
                           "preparation and the sums over reduction ranges included",
                 "contractions_per_step": tc_count, "ms_per_step": tc_ms, "mma_passes": passes,
                 "tensor_work_frac": passes * achieved / peak, "peak_source": peak_src,

@@ -49,8 +49,8 @@ enum {
 
 /* Range of the scaled halves.  The gradients of convolutions and of large fully connected layers are sums over blocks of 64 products.  In each block the
  * 64 values that enter one sum from either side share a power of two.  From the gathered side (the data, or the output derivative of a data gradient; the
- * weights of a fully connected one) those down to 2^-28 of the largest of the 64 keep 22 bits, smaller ones are off by at most 2^-51 of the largest; from
- * the other side (output derivative, filter bank) 2^-12 and 2^-35, or better.  VLB_PRECISION_TF32 keeps 11 bits down to 2^-29, 2^-40 at worst (2^-13, 2^-24).
+ * weights of a fully connected one) those down to 2^-28 of the largest of the 64 keep 22 bits, smaller ones are off by at most 2^-50 of the largest; from
+ * the other side (output derivative, filter bank) 2^-12 and 2^-34, or better.  VLB_PRECISION_TF32 keeps 11 bits down to 2^-28, 2^-39 at worst (2^-12, 2^-23).
  * Such errors show only where the largest values meet zeros or cancel.  Nothing is shared beyond the 64: a filter, channel, image or pixel that is small
  * beside others, by up to 2^100, is as exact as among its like.  Single values below about 2^-102 in magnitude lose digits as they near the subnormal
  * range.  An infinity or a not-a-number reaches the sums that it is part of and no others. */

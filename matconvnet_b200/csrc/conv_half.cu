@@ -12,13 +12,13 @@ namespace {
 // reduction indices.  Each row of A takes the power of two that brings the largest magnitude of its values in the k-block into [2^14, 2^15), each tile of B one for
 // 32 or 64 columns, and a column whose own largest magnitude is more than 2^16 below theirs one of its own; then x * s = hi + lo / 2048 with hi = half(x*s)
 // and lo = half((x*s - hi) * 2048): 22 significant bits for every value of a row of A down to 2^-28 of the row's largest in the k-block, below that an absolute
-// error of 2^-51 of that one; of a column of B down to 2^-12, 2^-35 at worst.  (Two TF32 values hold 22 bits as well, whatever stands beside them.)  Per k-block the accumulator T takes the small terms lo*hi + hi*lo first, which carry the 2048, then
+// error of 2^-50 of that one; of a column of B down to 2^-12, 2^-34 at worst.  (Two TF32 values hold 22 bits as well, whatever stands beside them.)  Per k-block the accumulator T takes the small terms lo*hi + hi*lo first, which carry the 2048, then
 // hi*hi with the accumulator scaled by 2^-11 (the MMA's scale-input-d); lo*lo (2^-22) is dropped.  Products of two halves are exact and the sums
 // are fp32, as with TF32.  The drain warps add T * 2^-(row's + tile's exponent) to the fp32 running sum: one k-block per accumulation chain, so
 // that the tensor core's truncating additions have no time to pile up (12 MMAs 16 deep; conv_ts_kernel has chains of up to 48 MMAs 8 deep).
 // 3x3, 512 -> 512 channels, 28 x 28 x 64, against float64: 2.0e-7 (conv_ts_kernel 9e-7); data gradient 956 us there, 565 here.
-// VLB_PRECISION_TF32 issues hi*hi alone: operands rounded to 11 bits as TF32 does, down to 2^-29 of the row's largest magnitude in the k-block (2^-13 of the
-// column's), where the subnormal halves begin; below that an absolute error of 2^-40 (2^-24) of it.
+// VLB_PRECISION_TF32 issues hi*hi alone: operands rounded to 11 bits as TF32 does, down to 2^-28 of the row's largest magnitude in the k-block (2^-12 of the
+// column's), where the subnormal halves begin; below that an absolute error of 2^-39 (2^-23) of it.
 // Why the forward passes stay where they are: their sums decide what ReLU and pooling let through.  Other sums, however near, decide some ties of
 // existing networks the other way; a backward pass decides nothing.
 //
@@ -26,8 +26,8 @@ namespace {
 //   0  a thread per row gathers fp32 values, finds their largest, converts them (few channels, 1x1 filters): 2000 cycles per k-block
 //   1  the same from input windows that tensor-map copies brought to shared memory
 //   2  the same from runs along the planes (filter gradient; rows are (tap, channel))
-//   3  sixteen 16-byte loads from a copy of the tensor that split_chunks_kernel has converted: 1150 cycles per k-block, bound by the bandwidth of the array
-//      that is shared memory and L1 (tiles of B written and read 48 + 32 KB, chunks of A 40 KB, 128 bytes per clock); the MMAs take 768
+//   3  sixteen 16-byte loads from a copy of the tensor that split_chunks_kernel has converted: 1150 cycles per k-block where the MMAs take 768.  No unit is saturated
+//      (tensor pipe 73-77%, L2 24-30%, data banks of shared memory and L1 24-29%); by elimination it is the chain from a freed A stage over the loads to the next MMA
 //   4  the same for filter gradients, chunks of eight images, a k-block being 64 images of a pixel
 //   5  filter gradients of fewer images: a k-block is several rows of a column, wherever the filter tap puts them, so the chunks hold fp32 values, which a
 //      thread converts as in the modes 0 to 2.  (Split beforehand they would need one power of two for all rows that some tap may put side by side, the
@@ -83,10 +83,10 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, uint4 const (&r)[8])
 
 // A column of B whose largest magnitude lies more than 2^kOwnScale below the tile's takes a power of two of its own, 2^c beyond the tile's.  The closer the line
 // lies to the tile's, the more k-blocks of ordinary values pay for it in the drain warps (rescale_columns; dense values never, a column with one value left by
-// ReLU and pooling once in 25000 k-blocks); the further off, the fewer digits a column just above it keeps: at 2^16 its values have 22 bits down to 2^-12
-// of its largest, 11 (VLB_PRECISION_TF32) down to 2^-13.
+// ReLU and pooling once in 25000 k-blocks, the cross terms of a normalisation layer in a fifth: AlexNet's filter gradients 522 -> 618 us); the further off, the fewer digits a column just above it keeps: at 2^16 its values have 22 bits (VLB_PRECISION_TF32:
+// 11) down to 2^-12 of its largest.
 constexpr int kOwnScale = 16;
-constexpr int kMaxOwnScale = 100;       // (further down 22 bits until 2^-12 of that: 2^-128 of the tile's largest magnitude)
+constexpr int kMaxOwnScale = 100;       // (further down 22 bits until 2^-128 of the tile's largest magnitude)
 constexpr int kOwnFlag = 1 << 16;       // added to an exponent word of the tile images: some column has one of its own
 
 // Two fp32 values side by side in one 64-bit register pair, and the packed operations on them (one instruction for both).
